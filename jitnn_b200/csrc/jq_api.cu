@@ -385,15 +385,16 @@ int jq_weight_upload_rows(int device, int type, const void* host_blocks, int64_t
     w->n = rows;
     w->k = k;
     const bool tiled = tiled_layout(type) || tiled_planes(type);
-    w->q_bytes = tiled ? tiled_rows(rows) * (k / qk) * plane_q_bytes(type) : blocks * plane_q_bytes(type);
-    w->aux_bytes = (tiled_planes(type) ? tiled_rows(rows) * (k / qk) : blocks) * plane_aux_bytes(type);
+    const int64_t held = tiled_steps(k) * 256 / qk;  // blocks per row as stored: 32-element blocks fill up whole 256-wide steps
+    w->q_bytes = tiled ? tiled_rows(rows) * held * plane_q_bytes(type) : blocks * plane_q_bytes(type);
+    w->aux_bytes = (tiled_planes(type) ? tiled_rows(rows) * held : blocks) * plane_aux_bytes(type);
     w->q = nullptr;
     w->aux = nullptr;
 
     int rc = JQ_OK;
     uint8_t* tmp = nullptr;
     // PAD_ROWS rows of zeros follow each plane, so that 16-row tiles may read past the last row
-    const int64_t pad_q = (int64_t)PAD_ROWS * (k / qk) * plane_q_bytes(type), pad_aux = (int64_t)PAD_ROWS * (k / qk) * plane_aux_bytes(type);
+    const int64_t pad_q = (int64_t)PAD_ROWS * held * plane_q_bytes(type), pad_aux = (int64_t)PAD_ROWS * held * plane_aux_bytes(type);
     cudaError_t e = cudaMalloc(&w->q, (size_t)(w->q_bytes + pad_q + 16));
     if (e == cudaSuccess) {
         // a tiled weight is zeroed as a whole (the rows that pad its last tile), the others behind their last row

@@ -83,14 +83,25 @@ inline int plane_aux_bytes(int type) {
 // The last tile is padded with zero rows. No byte of a block changes; jq_weight_download restores GGUF's order.
 constexpr int TILE_ROWS = 128;
 __host__ __device__ inline bool tiled_layout(int type) { return type == JQ_TYPE_Q4_K || type == JQ_TYPE_Q5_K; }
-// Q6_K keeps its two planes (208 bytes of quants and scales, one fp16 d per block) and orders the blocks of each plane the
-// same way, so that 16 rows x one super-block are 3328 contiguous bytes of the quant plane and 32 of the d plane.
-__host__ __device__ inline bool tiled_planes(int type) { return type == JQ_TYPE_Q6_K; }
+// The formats with two planes (quants; fp16 scales) order the blocks of each plane the same way. Q6_K: 16 rows x one super-block are
+// 3328 contiguous bytes of the quant plane and 32 of the d plane. The formats with 32-element blocks take eight blocks (256 values
+// of k) where the K-quants have a super-block; a k that is no multiple of 256 is padded with zero blocks, and the 16-byte pieces of
+// a row's eight blocks are stored with the low three bits of their number XORed by (row & 7), so that eight rows read at the same
+// place of their rows fall into different shared-memory banks after a plain copy.
+__host__ __device__ inline bool tiled_planes(int type) {
+    return type == JQ_TYPE_Q6_K || type == JQ_TYPE_Q8_0 || type == JQ_TYPE_Q4_0 || type == JQ_TYPE_Q4_1;
+}
 __host__ __device__ inline int64_t tiled_rows(int64_t n) { return (n + TILE_ROWS - 1) / TILE_ROWS * TILE_ROWS; }
-// Position of block b of `row` among the blocks of a tiled plane with kb blocks per row.
+// 256-wide steps of k of a tiled weight.
+__host__ __device__ inline int64_t tiled_steps(int64_t k) { return (k + 255) >> 8; }
+// Position of super-block b of `row` among the super-blocks of a tiled plane with kb of them per row.
 __host__ __device__ inline int64_t tiled_index(int64_t row, int64_t b, int64_t kb) {
     return ((row >> 7) * kb + b) * TILE_ROWS + (row & (TILE_ROWS - 1));
 }
+// Position of 32-element block b of `row` in a tiled plane of kb 256-wide steps per row.
+__host__ __device__ inline int64_t tiled_index32(int64_t row, int64_t b, int64_t kb) { return tiled_index(row, b >> 3, kb) * 8 + (b & 7); }
+// Where 16-byte piece c of a row's 256-wide step lies within that row's run of the quant plane.
+__host__ __device__ inline int swizzle_piece(int c, int64_t row) { return (c & ~7) | ((c ^ (int)row) & 7); }
 // Byte offset of block b of `row` in a tiled weight with kb blocks of `bytes` bytes per row.
 __host__ __device__ inline int64_t tiled_offset(int64_t row, int64_t b, int64_t kb, int bytes) {
     return ((row >> 7) * kb + b) * (int64_t)(TILE_ROWS * bytes) + (row & (TILE_ROWS - 1)) * bytes;
@@ -111,7 +122,7 @@ struct View {
 };
 
 // ---- kernel launchers (one translation unit each) ----------------------------------------------
-// kb: blocks per row; the planes of a type with tiled_planes() hold their blocks in tiled order (tiled_rows(n) rows).
+// kb: blocks per row; the planes hold their blocks in tiled order (tiled_rows(n) rows).
 int launch_repack(int type, const uint8_t* verbatim, uint8_t* q, uint8_t* aux, int64_t blocks, int64_t kb, cudaStream_t s);
 int launch_unpack(int type, const uint8_t* q, const uint8_t* aux, uint8_t* verbatim, int64_t blocks, int64_t kb, cudaStream_t s);
 // Verbatim blocks [n, kb] <-> the tiled layout of Q4_K and Q5_K (`tiled` holds tiled_rows(n) rows).

@@ -15,6 +15,7 @@
 //   Q8_0  q: 32 int8 per block; aux: fp16 d per block
 //   Q4_0  q: 16 nibble bytes per block; aux: fp16 d per block
 //   Q4_1  q: 16 nibble bytes per block; aux: fp16 d, fp16 m per block
+//         (all planes in tiled order; the 32-element formats eight blocks at a time, 16-byte pieces swizzled by the row)
 #pragma once
 
 #include <cuda_fp16.h>
@@ -34,6 +35,16 @@ __device__ __forceinline__ const uint8_t* tiled_block(const View& v, int64_t blo
     const uint32_t kb = (uint32_t)(v.k >> 8);
     const uint32_t row = (uint32_t)block / kb, b = (uint32_t)block - row * kb;  // fewer than 2^23 blocks: weights have fewer than 2^31 elements
     return v.q + tiled_offset(row, b, kb, bytes);
+}
+
+// The same for the planes of the 32-element formats: where the block's scale lies (in blocks) and the address of its 16-byte piece `u`.
+template <int PIECES>
+__device__ __forceinline__ const uint8_t* tiled_piece32(const View& v, int64_t block, int u, int64_t& at) {
+    const uint32_t per_row = (uint32_t)(v.k >> 5);
+    const uint32_t row = (uint32_t)block / per_row, b = (uint32_t)block - row * per_row;  // fewer than 2^26 blocks
+    at = tiled_index32(row, b, tiled_steps(v.k));
+    const int piece = (int)(b & 7) * PIECES + u;
+    return v.q + (at - (b & 7)) * (PIECES * 16) + swizzle_piece(piece, row) * 16;
 }
 
 __device__ __forceinline__ uint32_t byte_of(uint32_t w, int i) { return (w >> (8 * i)) & 0xffu; }
@@ -68,8 +79,9 @@ struct Fmt<JQ_TYPE_Q8_0> {
         uint32_t d;
     };
     __device__ static void load(const View& v, int64_t block, int unit, Raw& r) {
-        r.q = ld16(v.q + block * 32 + unit * 16);
-        r.d = __ldg(reinterpret_cast<const unsigned short*>(v.aux) + block);
+        int64_t at;
+        r.q = ld16(tiled_piece32<2>(v, block, unit, at));
+        r.d = __ldg(reinterpret_cast<const unsigned short*>(v.aux) + at);
     }
     __device__ static void decode(const View& v, int64_t block, int unit, float (&out)[RUNS][16], int (&pos)[RUNS]) {
         Raw r;
@@ -98,8 +110,9 @@ struct Fmt<JQ_TYPE_Q4_0> {
         uint32_t d;
     };
     __device__ static void load(const View& v, int64_t block, int, Raw& r) {
-        r.q = ld16(v.q + block * 16);
-        r.d = __ldg(reinterpret_cast<const unsigned short*>(v.aux) + block);
+        int64_t at;
+        r.q = ld16(tiled_piece32<1>(v, block, 0, at));
+        r.d = __ldg(reinterpret_cast<const unsigned short*>(v.aux) + at);
     }
     __device__ static void decode(const View& v, int64_t block, int unit, float (&out)[RUNS][16], int (&pos)[RUNS]) {
         Raw r;
@@ -130,8 +143,9 @@ struct Fmt<JQ_TYPE_Q4_1> {
         uint32_t dm;
     };
     __device__ static void load(const View& v, int64_t block, int, Raw& r) {
-        r.q = ld16(v.q + block * 16);
-        r.dm = __ldg(reinterpret_cast<const uint32_t*>(v.aux) + block);
+        int64_t at;
+        r.q = ld16(tiled_piece32<1>(v, block, 0, at));
+        r.dm = __ldg(reinterpret_cast<const uint32_t*>(v.aux) + at);
     }
     __device__ static void decode(const View& v, int64_t block, int unit, float (&out)[RUNS][16], int (&pos)[RUNS]) {
         Raw r;

@@ -17,9 +17,9 @@
 //
 // Work split as in the Q4_K kernel: a CTA of 8 warps owns 16 output rows at a time, warp p takes the 256-blocks of k
 // with index p (mod 8); per tile the warps' partial sums meet in shared memory in a fixed order that depends on k only
-// (row shards are bitwise equal to the whole weight). Quant and scale planes are separate on the device
-// (jq_formats.cuh); both are padded by 16 rows. Shared-memory rows are swizzled by (row & 7) so that ldmatrix's eight
-// row reads fall into different banks.
+// (row shards are bitwise equal to the whole weight). Quant and scale planes are separate on the device (jq_formats.cuh), in tiled
+// order, so that a step is one contiguous run of each; its rows are stored swizzled by (row & 7), so that ldmatrix's eight row
+// reads fall into different banks.
 #include "jq_formats.cuh"
 
 namespace jq {
@@ -77,8 +77,7 @@ struct Geo {
     static constexpr int QC = QROW / 16, AC = AROW / 16;           // 16-byte chunks per row
     static constexpr int AUX_OFF = 16 * QROW;
     static constexpr int SLOT = 16 * (QROW + AROW);
-    static constexpr int CHUNKS = 16 * (QC + AC);
-    static constexpr int PER_LANE = (CHUNKS + 31) / 32;
+    static_assert(16 * AC <= 32, "one scale piece per lane");
 };
 
 // Image of one row group of x per 256 values of k: digit fragments of the 8 blocks (two blocks side by side per
@@ -196,26 +195,6 @@ __global__ void __launch_bounds__(THREADS, 2) gemv_blk32_i8_kernel(View v, const
     float* red = reinterpret_cast<float*>(smem_raw + (size_t)KB * I::PB);  // [2][NW][16][MT]
     uint8_t* ring = reinterpret_cast<uint8_t*>(red + 2 * NW * 16 * MT) + (size_t)warp * RING_BYTES;
     const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring);
-    const int64_t qrow = (int64_t)KB * G::QROW, arow = (int64_t)KB * G::AROW;  // plane bytes per weight row
-
-    // ---- weight stream: chunk c = lane + 32 i of a slot's chunks (quant chunks of the 16 rows, then their scale chunks) ----
-    uint32_t src_off[G::PER_LANE], dst_off[G::PER_LANE];
-    bool is_aux[G::PER_LANE], live[G::PER_LANE];
-#pragma unroll
-    for (int i = 0; i < G::PER_LANE; i++) {
-        const int c = lane + 32 * i;
-        live[i] = c < G::CHUNKS;
-        is_aux[i] = c >= 16 * G::QC;
-        if (!is_aux[i]) {
-            const int r = c / G::QC, ch = c % G::QC;
-            src_off[i] = (uint32_t)(r * (int)qrow + ch * 16);
-            dst_off[i] = (uint32_t)(r * G::QROW + (((ch & 8) | ((ch & 7) ^ (r & 7))) << 4));
-        } else {
-            const int ca = c - 16 * G::QC, r = ca / G::AC, ch = ca % G::AC;
-            src_off[i] = (uint32_t)(r * (int)arow + ch * 16);
-            dst_off[i] = (uint32_t)(G::AUX_OFF + r * G::AROW + ch * 16);
-        }
-    }
     const int nb = warp < KB ? (KB - warp + NW - 1) / NW : 0;
     const int my_tiles = (int)blockIdx.x < tiles ? (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
     int iss_left = nb * my_tiles, iss_ti = 0, iss_j = 0;
@@ -225,13 +204,16 @@ __global__ void __launch_bounds__(THREADS, 2) gemv_blk32_i8_kernel(View v, const
             iss_left--;
             const int tile = (int)blockIdx.x + iss_ti * (int)gridDim.x;
             const int sb = warp + NW * iss_j;
-            const uint8_t* qb = v.q + (int64_t)tile * 16 * qrow + (int64_t)sb * G::QROW;
-            const uint8_t* ab = v.aux + (int64_t)tile * 16 * arow + (int64_t)sb * G::AROW;
-            const uint32_t slot = ring_s + iss_slot;
+            // 16 rows x 256 k are one contiguous run of each plane, already in the slot's (swizzled) order
+            const int64_t at = (int64_t)(tile >> 3) * KB * 8 + (int64_t)sb * 8 + (tile & 7);  // in steps of 16 rows
+            const uint8_t* qb = v.q + at * 16 * G::QROW + lane * 16;
+            const uint8_t* ab = v.aux + at * 16 * G::AROW + lane * 16;
+            const uint32_t slot = ring_s + iss_slot + (uint32_t)lane * 16u;
 #pragma unroll
-            for (int i = 0; i < G::PER_LANE; i++) {
-                cp_async16_if(slot + dst_off[i], (is_aux[i] ? ab : qb) + src_off[i], live[i]);
+            for (int i = 0; i < 16 * G::QC / 32; i++) {
+                cp_async16(slot + i * 512u, qb + i * 512);
             }
+            cp_async16_if(slot + (uint32_t)G::AUX_OFF, ab, lane < 16 * G::AC);
             if (++iss_j == nb) {
                 iss_j = 0;
                 iss_ti++;

@@ -26,7 +26,7 @@ static Split split_of(int type) {
 
 // One thread per 2 bytes of a block (every block size and field offset here is even).
 __global__ void repack_kernel(Split sp, const uint16_t* __restrict__ src, uint16_t* __restrict__ q, uint16_t* __restrict__ aux,
-                              int64_t blocks, int64_t kb, bool tiled, bool inverse) {
+                              int64_t blocks, int64_t kb, bool inverse) {
     int64_t halves_per_block = sp.block / 2;
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= blocks * halves_per_block) {
@@ -34,15 +34,20 @@ __global__ void repack_kernel(Split sp, const uint16_t* __restrict__ src, uint16
     }
     int64_t b = i / halves_per_block;
     int off = (int)(i % halves_per_block) * 2;
-    if (tiled) {
-        b = tiled_index(b / kb, b % kb, kb);  // where the block sits in the planes
-    }
+    const int64_t row = b / kb, col = b % kb;
+    const bool small = sp.q_bytes < 64;  // 32-element blocks: eight per 256-wide step, their 16-byte pieces swizzled by the row
+    b = small ? tiled_index32(row, col, (kb + 7) >> 3) : tiled_index(row, col, kb);  // where the block sits in the planes
     uint16_t* verbatim = const_cast<uint16_t*>(src) + i;
     uint16_t* plane;
     if (off >= sp.aux_off && off < sp.aux_off + sp.aux_bytes) {
         plane = aux + (b * sp.aux_bytes + (off - sp.aux_off)) / 2;
     } else {
-        plane = q + (b * sp.q_bytes + (off - sp.q_off)) / 2;
+        int64_t at = off - sp.q_off;
+        if (small) {
+            const int per_block = sp.q_bytes / 16, piece = (int)(col & 7) * per_block + (int)(at >> 4);
+            at = (int64_t)(swizzle_piece(piece, row) - (int)(col & 7) * per_block) * 16 + (at & 15);
+        }
+        plane = q + (b * sp.q_bytes + at) / 2;
     }
     if (inverse) {
         *verbatim = *plane;
@@ -60,7 +65,7 @@ int launch_repack(int type, const uint8_t* verbatim, uint8_t* q, uint8_t* aux, i
     if (total == 0) {
         return JQ_OK;
     }
-    repack_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(sp, (const uint16_t*)verbatim, (uint16_t*)q, (uint16_t*)aux, blocks, kb, tiled_planes(type), false);
+    repack_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(sp, (const uint16_t*)verbatim, (uint16_t*)q, (uint16_t*)aux, blocks, kb, false);
     count_launch();
     return check_launch("repack_kernel");
 }
@@ -74,7 +79,7 @@ int launch_unpack(int type, const uint8_t* q, const uint8_t* aux, uint8_t* verba
     if (total == 0) {
         return JQ_OK;
     }
-    repack_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(sp, (const uint16_t*)verbatim, (uint16_t*)q, (uint16_t*)aux, blocks, kb, tiled_planes(type), true);
+    repack_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(sp, (const uint16_t*)verbatim, (uint16_t*)q, (uint16_t*)aux, blocks, kb, true);
     count_launch();
     return check_launch("repack_kernel");
 }
