@@ -73,7 +73,7 @@ class GgufFile:
         lo, hi = (0, -1) if rows is None else rows
         _lib.check(self._lib.jq_gguf_upload(self._live(), t.index, device, lo, hi, ctypes.byref(h)))
         n = t.shape[0] if rows is None else hi - lo
-        return Tensor(h, DType(t.ggml_type), (n, t.shape[1]))
+        return Tensor(h, DType(t.ggml_type), (n, t.shape[1]), device)
 
     def close(self):
         if self._h is not None:

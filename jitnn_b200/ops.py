@@ -60,10 +60,11 @@ def _is_torch(x):
 class Tensor:
     """A persistent quantised weight on one GPU (the handle behind ``jq_weight``)."""
 
-    def __init__(self, handle, dtype, dims):
+    def __init__(self, handle, dtype, dims, device=0):
         self._h = handle
         self._dtype = dtype
         self._dims = tuple(dims)
+        self._device = device
 
     @staticmethod
     def quantized(dtype, blocks, *dims, device=0, rows=None):
@@ -89,7 +90,7 @@ class Tensor:
             check(L.jq_weight_upload_rows(device, dtype.value, raw.ctypes.data, raw.size, n, k, int(rows[0]), int(rows[1]),
                                           _lib.JQ_LAYOUT_AUTO, ctypes.byref(out)))
             shape = (int(rows[1]) - int(rows[0]), k)
-        return Tensor(out, dtype, shape)
+        return Tensor(out, dtype, shape, device)
 
     def _handle(self):
         if self._h is None:
@@ -112,9 +113,8 @@ class Tensor:
         return self._dims[0] * self._dims[1]
 
     def device(self):
-        info = (ctypes.c_int64 * 8)()
-        check(_lib.load().jq_weight_info(self._handle(), info))
-        return int(info[4])
+        self._handle()  # a released tensor is on no device
+        return self._device
 
     def deviceBytes(self):
         info = (ctypes.c_int64 * 8)()
@@ -146,34 +146,60 @@ class Tensor:
             pass
 
 
-def _stream_of(t):
-    import torch
-    return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+# Calls on torch tensors. A decode linear takes a few microseconds on the GPU, less than the host needs for an ordinary chain of torch calls
+# around it, so these paths ask each tensor for as little as the checks need, take torch's raw current stream, and leave making the
+# weight's device current to the library.
+_torch = None
+
+
+def _t():
+    global _torch
+    if _torch is None:
+        import torch
+        _torch = torch
+    return _torch
+
+
+def _raw_stream(torch, index):
+    get = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return get(index) if get is not None else torch.cuda.current_stream(index).cuda_stream
+
+
+def _check_torch(x, dtype, name, last, w, what):
+    """The shape of a CUDA tensor x of `dtype` with `last` values per row on w's device, or the reference's error."""
+    if x.dtype is not dtype:
+        raise ValueError("needs %s tensor, got %s" % (name, x.dtype))  # Checks.f32
+    shape = x.shape
+    if len(shape) == 0 or shape[-1] != last:
+        raise ValueError("%s %s %s and weight %s" % (w._dtype.name, what, list(shape), list(w._dims)))
+    if x.get_device() != w._device:
+        raise ValueError("%s %s on %s, weight on cuda:%d" % (w._dtype.name, what, x.device, w._device))
+    return shape
+
+
+def _checked_bias(torch, bias, x, n, w):
+    b = bias.contiguous()
+    if b.dtype is not torch.float32 or b.numel() != n or b.device != x.device:
+        raise ValueError("%s linear: bias %s for %d outputs" % (w._dtype.name, list(bias.shape), n))
+    return b
 
 
 def _linear(x, w, bias, who):
     L = _lib.load()
     if not isinstance(w, Tensor):
         raise ValueError("%s: weight is not a quantised tensor" % who)
-    n, k = w.shape()
+    n, k = w._dims
     if _is_torch(x):
-        import torch
-        if x.dtype != torch.float32:
-            raise ValueError("needs an FP32 tensor, got %s" % x.dtype)  # Checks.f32
-        if x.dim() == 0 or x.shape[-1] != k:
-            raise ValueError("%s linear: input %s and weight %s" % (w.dtype().name, list(x.shape), list(w.shape())))
-        if not x.is_cuda or x.device.index != w.device():
-            raise ValueError("%s linear: input on %s, weight on cuda:%d" % (w.dtype().name, x.device, w.device()))
-        xc = x.contiguous()
+        torch = _t()
+        h = w._handle()
+        shape = _check_torch(x, torch.float32, "an FP32", k, w, "linear: input")
+        xc = x if x.is_contiguous() else x.contiguous()
         m = xc.numel() // k if k else 0
-        y = torch.empty(list(x.shape[:-1]) + [n], dtype=torch.float32, device=x.device)
-        b = None
-        if bias is not None:
-            b = bias.contiguous()
-            if b.dtype != torch.float32 or b.numel() != n or b.device != x.device:
-                raise ValueError("%s linear: bias %s for %d outputs" % (w.dtype().name, list(bias.shape), n))
-        with torch.cuda.device(x.device):
-            check(L.jq_linear_f32(w._handle(), xc.data_ptr(), m, None if b is None else b.data_ptr(), y.data_ptr(), JQ_MEM_DEVICE, _stream_of(x)))
+        y = xc.new_empty((*shape[:-1], n))
+        b = None if bias is None else _checked_bias(torch, bias, x, n, w)
+        rc = L.jq_linear_f32(h, xc.data_ptr(), m, None if b is None else b.data_ptr(), y.data_ptr(), JQ_MEM_DEVICE, _raw_stream(torch, w._device))
+        if rc:
+            check(rc)
         return y
     x = np.asarray(x)
     if x.dtype != np.float32:
@@ -196,20 +222,17 @@ def _linear_backward(g, w):
     L = _lib.load()
     if not isinstance(w, Tensor):
         raise ValueError("linear backward: weight is not a quantised tensor")
-    n, k = w.shape()
+    n, k = w._dims
     if _is_torch(g):
-        import torch
-        if g.dtype != torch.float32:
-            raise ValueError("needs an FP32 tensor, got %s" % g.dtype)
-        if g.dim() == 0 or g.shape[-1] != n:
-            raise ValueError("%s linear backward: gradient %s and weight %s" % (w.dtype().name, list(g.shape), list(w.shape())))
-        if not g.is_cuda or g.device.index != w.device():
-            raise ValueError("%s linear backward: gradient on %s, weight on cuda:%d" % (w.dtype().name, g.device, w.device()))
-        gc = g.contiguous()
-        m = gc.numel() // n if n else int(np.prod(g.shape[:-1]))
-        gx = torch.empty(list(g.shape[:-1]) + [k], dtype=torch.float32, device=g.device)
-        with torch.cuda.device(g.device):
-            check(L.jq_linear_backward_f32(w._handle(), gc.data_ptr(), m, gx.data_ptr(), JQ_MEM_DEVICE, _stream_of(g)))
+        torch = _t()
+        h = w._handle()
+        shape = _check_torch(g, torch.float32, "an FP32", n, w, "linear backward: gradient")
+        gc = g if g.is_contiguous() else g.contiguous()
+        m = gc.numel() // n if n else int(np.prod(shape[:-1]))
+        gx = gc.new_empty((*shape[:-1], k))
+        rc = L.jq_linear_backward_f32(h, gc.data_ptr(), m, gx.data_ptr(), JQ_MEM_DEVICE, _raw_stream(torch, w._device))
+        if rc:
+            check(rc)
         return gx
     g = np.asarray(g)
     if g.dtype != np.float32:
@@ -227,7 +250,7 @@ def _dequantize(w, out=None):
     L = _lib.load()
     n, k = w.shape()
     if out is not None and _is_torch(out):
-        check(L.jq_dequantize(w._handle(), out.data_ptr(), JQ_MEM_DEVICE, _stream_of(out)))
+        check(L.jq_dequantize(w._handle(), out.data_ptr(), JQ_MEM_DEVICE, _raw_stream(_t(), out.get_device())))
         return out
     y = np.empty((n, k), dtype=np.float32)
     check(L.jq_dequantize(w._handle(), y.ctypes.data, JQ_MEM_HOST, None))
@@ -259,19 +282,18 @@ class Gguf:
         L = _lib.load()
         if not isinstance(w, Tensor):
             raise ValueError("Gguf.linearBf16: weight is not a quantised tensor")
-        n, k = w.shape()
+        n, k = w._dims
         if _is_torch(x):
-            import torch
-            if x.dtype != torch.bfloat16:
-                raise ValueError("needs a BF16 tensor, got %s" % x.dtype)
-            if x.dim() == 0 or x.shape[-1] != k:
-                raise ValueError("%s linear: input %s and weight %s" % (w.dtype().name, list(x.shape), list(w.shape())))
-            xc = x.contiguous()
+            torch = _t()
+            h = w._handle()
+            shape = _check_torch(x, torch.bfloat16, "a BF16", k, w, "linear: input")
+            xc = x if x.is_contiguous() else x.contiguous()
             m = xc.numel() // k if k else 0
-            y = torch.empty(list(x.shape[:-1]) + [n], dtype=torch.float32, device=x.device)
-            b = None if bias is None else bias.contiguous()
-            with torch.cuda.device(x.device):
-                check(L.jq_linear_bf16(w._handle(), xc.data_ptr(), m, None if b is None else b.data_ptr(), y.data_ptr(), JQ_MEM_DEVICE, _stream_of(x)))
+            y = xc.new_empty((*shape[:-1], n), dtype=torch.float32)
+            b = None if bias is None else _checked_bias(torch, bias, x, n, w)
+            rc = L.jq_linear_bf16(h, xc.data_ptr(), m, None if b is None else b.data_ptr(), y.data_ptr(), JQ_MEM_DEVICE, _raw_stream(torch, w._device))
+            if rc:
+                check(rc)
             return y
         x = np.asarray(x)
         if x.dtype != np.uint16:
@@ -321,15 +343,15 @@ class Quant:
         """FP32 values (last axis a multiple of 32) to raw Q8_0 block bytes (numpy uint8)."""
         L = _lib.load()
         if _is_torch(x):
-            import torch
-            if x.dtype != torch.float32:
+            torch = _t()
+            if x.dtype is not torch.float32:
                 raise ValueError("needs an FP32 tensor, got %s" % x.dtype)
             if x.shape[-1] % 32 != 0:
                 raise ValueError("Q8_0 needs a last axis that is a multiple of 32, got %s" % list(x.shape))
-            xc = x.contiguous()
-            out = torch.empty(xc.numel() // 32 * 34, dtype=torch.uint8, device=x.device)
-            with torch.cuda.device(x.device):
-                check(L.jq_quantize_q8_0(x.device.index, xc.data_ptr(), xc.numel(), out.data_ptr(), JQ_MEM_DEVICE, _stream_of(x)))
+            xc = x if x.is_contiguous() else x.contiguous()
+            index = x.get_device()
+            out = xc.new_empty((xc.numel() // 32 * 34,), dtype=torch.uint8)
+            check(L.jq_quantize_q8_0(index, xc.data_ptr(), xc.numel(), out.data_ptr(), JQ_MEM_DEVICE, _raw_stream(torch, index)))
             return out
         x = np.asarray(x)
         if x.dtype != np.float32:
