@@ -119,8 +119,9 @@ JQ_API int jq_dequantize(const jq_weight* w, float* dst, int dst_mem, void* stre
  * non-finite outputs (Q4_K, Q5_K: NaN in every output of that row of x). Stands in for Gguf.linear(x, w, bias) (ops/Gguf.java:76-98) and
  * Quant.linear / F.linearQ8 (ops/Quant.java:66-80): any m >= 0 (leading axes of x flattened by the
  * caller as ops/Gguf.java:86-93 does), bias may be NULL. Rows are dispatched like the reference
- * dispatches them (ops/Gguf.java:90): m <= 16 to the fused dequantise-GEMV kernels, larger m in
- * groups of up to 16 rows through the same kernels unless the tensor-core prefill path is selected with
+ * dispatches them (ops/Gguf.java:90): m <= 16 to the fused dequantise-GEMV kernels, larger m to the tensor-core matrix
+ * kernel, which takes x and the weights as sums of two half-precision numbers (22 significant bits, relative to the largest
+ * magnitude of a 256-element block) and adds up in FP32, unless the bfloat16 prefill path is selected with
  * jq_set_option. `mem` says where x, bias and y live (all three alike); with JQ_MEM_DEVICE they must
  * be 16-byte aligned and `stream` is the CUDA stream (cudaStream_t, NULL = default stream).
  */
@@ -140,8 +141,8 @@ JQ_API int jq_linear_bf16(const jq_weight* w, const uint16_t* x_bf16, int64_t m,
 /*
  * Input gradient of the linear: gx[m, k] = g[m, n] . dequant(W), float32 (the backward of Gguf.linear and Quant.linear,
  * ops/Gguf.java:208-212 and ops/Quant.java:191-197: the quantised weight gets no gradient, the bias gradient is the
- * column sum of g and needs no weight). The weight is read once per four (Q6_K: one, 4-bit formats: two) rows of g, in
- * its quantised form, with FP32 accumulation (the reference accumulates in double; results agree within 1e-3 relative).
+ * column sum of g and needs no weight). Runs on the matrix kernel with the same two-part operands as jq_linear_f32 of many
+ * rows and FP32 accumulation (the reference accumulates in double; results agree within 1e-3 relative).
  * `mem` as for jq_linear_f32; device pointers must be 16-byte aligned.
  */
 JQ_API int jq_linear_backward_f32(const jq_weight* w, const float* g, int64_t m, float* gx, int mem, void* stream);

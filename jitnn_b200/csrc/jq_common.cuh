@@ -130,7 +130,7 @@ int launch_tile(int type, const uint8_t* verbatim, uint8_t* tiled, int64_t n, in
 int launch_dequantize(const View& v, float* dst, cudaStream_t s);
 // x_remote: x lies in host memory that the GPU reads across PCIe; kernels then read it once instead of once per thread block.
 int launch_gemv(const View& v, const float* x, int rows, const float* bias, float* y, cudaStream_t s, bool x_remote = false);
-// gx [m, k] = g [m, n] . dequant(W) (jq_backward.cu).
+// gx [m, k] = g [m, n] . dequant(W) (jq_matmul.cu).
 int launch_linear_backward(const View& v, const float* g, int64_t m, float* gx, cudaStream_t s);
 int launch_quantize_q8_0(const float* x, int64_t blocks, uint8_t* out, cudaStream_t s);
 // Where a GEMV's outputs go besides (or instead of) y when the linear is sharded by rows over several GPUs: every
@@ -211,7 +211,8 @@ extern std::atomic<int64_t> g_opt_peer_wait_us;  // microseconds a thread waits 
 // Rows of zero padding behind every uploaded weight plane: kernels that work on 16-row tiles read past n.
 constexpr int PAD_ROWS = 16;
 
-// Tensor-core prefill (jq_prefill.cu).
+// The matrix kernel (jq_matmul.cu): the FP32 product with many rows of x, and the bfloat16 product.
+int launch_matmul_f32(const View& v, const float* x, int64_t m, const float* bias, float* y, cudaStream_t s);
 bool prefill_supported(const View& v);
 int launch_prefill_bf16(const View& v, const uint16_t* x_bf16, int64_t m, const float* bias, float* y, cudaStream_t s);
 int launch_f32_to_bf16(const float* x, uint16_t* out, int64_t count, cudaStream_t s);

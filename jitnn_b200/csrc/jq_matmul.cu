@@ -1,0 +1,389 @@
+// Host side of the matrix kernel (jq_matmul.cuh): the split of FP32 activations, the choice of tiles, the launches.
+#include <cuda_bf16.h>
+
+#include <mutex>
+
+#include "jq_matmul_launch.cuh"
+
+namespace jq {
+
+static __device__ int g_matmul_status;
+
+namespace mm {
+
+// x [m, k] FP32 -> two planes of halves [2][m][width] (hi, lo) and a scale per (BLK values of k, row of x): the block's values times a power of
+// two that brings the largest to [2^9, 2^10), hi = that rounded to half precision, lo = the rest rounded to half precision: 22
+// significant bits for everything down to 2^-13 of the largest. A block that holds a NaN or an Inf gets the scale NaN, which reaches
+// every output of that row. One warp per 256 values of a row; memory bound (8 bytes moved per value, 4 of them to L2).
+// EXT: 64 more columns follow every 256, of which the first 16 hold the sums over the eight runs of 32 values, twice (hi plane: their
+// hi parts, lo plane: their lo parts); the others are never used.
+template <int BLK, bool EXT>
+__global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ x, int m, int64_t k, int per_row, uint4* __restrict__ planes,
+                                                    float* __restrict__ scales, int stride, int vec) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t task = (int64_t)blockIdx.x * 8 + warp;
+    const int row = (int)(task / per_row), b = (int)(task - (int64_t)row * per_row);
+    if (row >= m) {
+        return;
+    }
+    const int64_t i0 = (int64_t)b * 256 + lane * 8;
+    const float* src = x + (int64_t)row * k + i0;
+    float v[8];
+    if (vec && i0 + 8 <= k) {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(src)), c = __ldg(reinterpret_cast<const float4*>(src) + 1);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        v[4] = c.x; v[5] = c.y; v[6] = c.z; v[7] = c.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            v[i] = i0 + i < k ? __ldg(src + i) : 0.0f;
+        }
+    }
+    uint32_t am = 0;  // the largest magnitude as bits: an Inf or a NaN is larger than any number
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        am = max(am, __float_as_uint(v[i]) & 0x7fffffffu);
+    }
+#pragma unroll
+    for (int o = BLK / 16; o > 0; o >>= 1) {
+        am = max(am, __shfl_xor_sync(0xffffffffu, am, o));
+    }
+    const bool bad = am >= 0x7f800000u;
+    uint32_t e = am >> 23;
+    e = e < 14u ? 14u : (e > 254u ? 254u : e);
+    const float f = __uint_as_float((263u - e) << 23);
+    uint32_t hi[4], lo[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        split_pair(v[2 * i] * f, v[2 * i + 1] * f, hi[i], lo[i]);
+    }
+    constexpr int BLOCK = EXT ? 320 : 256;
+    const int64_t row_at = ((int64_t)row * per_row + b) * BLOCK, at = (row_at >> 3) + lane, plane = ((int64_t)m * per_row * BLOCK) >> 3;
+    planes[at] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    planes[at + plane] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    if constexpr (EXT) {
+        float sum = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&hi[i])), c = __half22float2(*reinterpret_cast<const __half2*>(&lo[i]));
+            sum += (a.x + c.x) + (a.y + c.y);
+        }
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        const __half h = __float2half_rn(sum), l = __float2half_rn(sum - __half2float(h));
+        if ((lane & 3) == 0) {  // sums of up to 2^15
+            __half* to = reinterpret_cast<__half*>(planes) + row_at + 256 + (lane >> 2);
+            to[0] = h;
+            to[8] = h;
+            to[plane * 8] = l;
+            to[plane * 8 + 8] = l;
+        }
+    }
+    if ((lane & (BLK / 8 - 1)) == 0) {
+        scales[(int64_t)(i0 / BLK) * stride + row] = bad ? __uint_as_float(0x7fc00000u) : __uint_as_float((e - 9u) << 23);
+    }
+}
+
+static int status_word(int** out) {
+    static std::atomic<int*> known[64];
+    int dev = 0;
+    JQ_CUDA(cudaGetDevice(&dev));
+    int* p = known[dev & 63].load(std::memory_order_acquire);
+    if (p == nullptr) {
+        void* a = nullptr;
+        JQ_CUDA(cudaGetSymbolAddress(&a, g_matmul_status));
+        p = static_cast<int*>(a);
+        known[dev & 63].store(p, std::memory_order_release);
+    }
+    *out = p;
+    return JQ_OK;
+}
+
+static int unit_bytes(int type) { return TILE_ROWS * (plane_q_bytes(type) + plane_aux_bytes(type)) * 256 / block_values(type); }
+
+// Ring depths: at least as many weight operands as there are groups of dequantiser warps, two activation tiles and two raw units; then the
+// activations' ring grows first. False if not even those fit.
+static bool rings(int type, bool fp32, bool bwd, int nt, int groups, Args& a, Plan& plan) {
+    const int at = a_bytes(bwd), bt = b_bytes(fp32, nt), rb = unit_bytes(type), room = 227 * 1024 - 1024 - TAIL_BYTES;
+    // weight operands: backward at most four, for the fold's ring of factors; forward what tensor memory holds behind one accumulator, or two
+    // where they fit beside the groups' operands
+    int max_a = 4;
+    if (!bwd) {
+        const int cols = ((plan.narrow ? 2 * nt : nt) + 31) / 32 * 32, per = a_columns(type, fp32, false);
+        const int bufs = 2 * cols + groups * per <= 512 ? 2 : 1;
+        max_a = (512 - bufs * cols) / per;
+        max_a = max_a > MAX_A ? MAX_A : max_a;
+    }
+    a.sa = bwd ? groups : max_a;
+    a.sb = 2;
+    a.raw = 2;
+    int left = room - a.sa * at - a.sb * bt - a.raw * rb;
+    if (left < 0) {
+        return false;
+    }
+    auto grow = [&](int& depth, int most, int bytes) {
+        while (depth < most && left >= bytes) {
+            depth++;
+            left -= bytes;
+        }
+    };
+    grow(a.sb, bwd ? 3 : 6, bt);
+    if (at > 0) {
+        grow(a.sa, max_a, at);
+    }
+    grow(a.raw, 3, rb);
+    grow(a.sb, MAX_B, bt);
+    grow(a.raw, MAX_RAW, rb);
+    plan.smem = (size_t)(room - left) + TAIL_BYTES + 1024;
+    return true;
+}
+
+// A tile width: the instance that can run it and its rings.
+static bool configure(int type, bool fp32, bool bwd, int nt, Args& a, Plan& plan) {
+    plan.fp32 = fp32;
+    plan.bwd = bwd;
+    plan.narrow = fp32 && nt <= 32;
+    a.nt = nt;
+    if (plan.narrow && rings(type, fp32, bwd, nt, Warps<true, 32>::GROUPS, a, plan)) {
+        return true;
+    }
+    plan.narrow = false;
+    return rings(type, fp32, bwd, nt, fp32 ? Warps<true, 128>::GROUPS : Warps<false, 16>::GROUPS, a, plan);
+}
+
+// What one unit of the contraction takes a CTA in nanoseconds, by the tile's width (measured on long contractions): the dequantiser warps and
+// the barriers between the roles up to a width, the tensor pipe beyond it.
+static double unit_ns(int type, bool fp32, bool bwd, int nt) {
+    if (bwd) {
+        return nt < 64 ? 940.0 : 430.0 + 7.9 * nt;
+    }
+    if (!fp32) {
+        const double t = 6.4 * ((nt + 63) / 64 * 64);  // (a tile of 208 or 240 is no faster than one of 256)
+        return t < 1200.0 ? 1200.0 : t;
+    }
+    const bool one_part = type == JQ_TYPE_Q4_K || type == JQ_TYPE_Q5_K;
+    const double t = one_part ? 450.0 + 9.9 * nt : 300.0 + 14.7 * nt;
+    return t < 1320.0 ? 1320.0 : t;
+}
+
+// Tile width and ranges of the contraction for a product of `features` x m over `units` units.
+static void choose(int type, bool fp32, bool bwd, int64_t features, int units, int m, Args& a, Plan& plan) {
+    const int nmax = fp32 ? 128 : 256;
+    double best = 1e30;
+    int best_nt = 16, best_ks = 1;
+    const int64_t ftiles = (features + 127) / 128;
+    int last_nt = 0;
+    for (int tt = (m + nmax - 1) / nmax; tt <= (m + nmax - 1) / nmax + 6; tt++) {
+        const int nt = ((m + tt - 1) / tt + 15) / 16 * 16;
+        if (nt == last_nt || !configure(type, fp32, bwd, nt, a, plan)) {
+            continue;
+        }
+        last_nt = nt;
+        const int64_t tiles = ftiles * ((m + nt - 1) / nt);
+        const double unit = unit_ns(type, fp32, bwd, nt);
+        for (int ks = 1; ks <= 8; ks *= 2) {
+            if (ks > 1 && units < 2 * ks) {
+                break;
+            }
+            const int slots = (ks <= 2 ? 148 : (ks == 4 ? 144 : 128)) / ks;  // clusters at a time
+            if (ks > 1 && tiles > slots) {
+                break;  // more than one wave of whole tiles: nothing to gain
+            }
+            const double waves = (double)((tiles + slots - 1) / slots);
+            const double cost = waves * (((units + ks - 1) / ks) * unit + 1500.0 + 12.0 * nt) + (ks > 1 ? 1500.0 + 6.0 * nt : 0.0);
+            if (cost < best) {
+                best = cost;
+                best_nt = nt;
+                best_ks = ks;
+            }
+        }
+    }
+    configure(type, fp32, bwd, best_nt, a, plan);
+    a.ksplit = best_ks;
+    a.ftiles = (int)ftiles;
+    a.ttiles = (m + best_nt - 1) / best_nt;
+    const int tiles = a.ftiles * a.ttiles;
+    plan.ctas = best_ks > 1 || tiles < 148 ? tiles * best_ks : 148;
+    a.units = units;
+    a.m = m;
+    a.cols = ((plan.narrow ? 2 * a.nt : a.nt) + 31) / 32 * 32;
+    const int ring = a.sa * a_columns(type, fp32, bwd);
+    a.bufs = 2 * a.cols + ring <= 512 ? 2 : 1;
+    a.tmem = 32;
+    while (a.tmem < a.bufs * a.cols + ring) {
+        a.tmem *= 2;
+    }
+}
+
+static int launch_any(int type, const Plan& plan, const Args& args, const CUtensorMap& map, cudaStream_t s) {
+    switch (type) {
+        case JQ_TYPE_Q4_K: return launch_q4_k(plan, args, map, s);
+        case JQ_TYPE_Q5_K: return launch_q5_k(plan, args, map, s);
+        case JQ_TYPE_Q6_K: return launch_q6_k(plan, args, map, s);
+        case JQ_TYPE_Q8_0: return launch_q8_0(plan, args, map, s);
+        case JQ_TYPE_Q4_0: return launch_q4_0(plan, args, map, s);
+        case JQ_TYPE_Q4_1: return launch_q4_1(plan, args, map, s);
+        default: return fail(JQ_ERR_UNSUPPORTED, "matrix product: type %d has no kernel", type);
+    }
+}
+
+// The activations as a tensor of [planes][rows][width] 16-bit values.
+static int activation_map(CUtensorMap* map, bool bf16, const void* x, int64_t width, int64_t rows, int planes, int box_rows) {
+    EncodeTiledFn enc = encode_tiled();
+    if (enc == nullptr) {
+        return fail(JQ_ERR_CUDA, "matrix product: cuTensorMapEncodeTiled is not available from this driver");
+    }
+    const cuuint64_t dims[3] = {(cuuint64_t)width, (cuuint64_t)rows, (cuuint64_t)planes};
+    const cuuint64_t strides[2] = {(cuuint64_t)width * 2, (cuuint64_t)width * 2 * (cuuint64_t)rows};
+    const cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = enc(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(x), dims, strides, box, estr,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? JQ_OK : fail(JQ_ERR_CUDA, "matrix product: cuTensorMapEncodeTiled failed with code %d", (int)r);
+}
+
+static void weight_args(const View& v, Args& a) {
+    a.q = v.q;
+    a.aux = v.aux;
+    a.kb = (int)tiled_steps(v.k);
+    a.rows128 = (int)(tiled_rows(v.n) / TILE_ROWS);
+}
+
+constexpr int SPLIT_SLOT = 6;  // scratch slot of the split activations
+
+// out [m, features] = the FP32 product in either direction; x has `width` values per row.
+static int product_f32(const View& v, bool bwd, const float* x, int64_t m, const float* bias, float* out, cudaStream_t s) {
+    const int64_t width = bwd ? v.n : v.k, features = bwd ? v.k : v.n;
+    const int per_row = (int)((width + 255) / 256);
+    const bool ext = unit_stages(v.type, true, bwd) == 5;
+    const int64_t wpad = (int64_t)per_row * (ext ? 320 : 256);
+    constexpr int64_t GROUP = 4096;  // rows at a time: bounds the scratch
+    int* status = nullptr;
+    int rc = status_word(&status);
+    for (int64_t m0 = 0; m0 < m && rc == JQ_OK; m0 += GROUP) {
+        const int rows = (int)(m - m0 < GROUP ? m - m0 : GROUP);
+        Args a = {};
+        Plan plan = {};
+        weight_args(v, a);
+        choose(v.type, true, bwd, features, bwd ? a.rows128 : a.kb, rows, a, plan);
+        const int stride = a.ttiles * a.nt, blk = bwd ? 128 : 256;
+        const size_t plane_bytes = (size_t)2 * rows * wpad * 2;
+        uint8_t* scratch = nullptr;
+        rc = scratch_for_slot(s, SPLIT_SLOT, plane_bytes + (size_t)(per_row * 256 / blk) * stride * sizeof(float), &scratch);
+        if (rc != JQ_OK) {
+            break;
+        }
+        float* scales = reinterpret_cast<float*>(scratch + plane_bytes);
+        const float* xg = x + m0 * width;
+        const int vec = width % 4 == 0 && ((uintptr_t)xg & 15) == 0;
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        cfg.stream = s;
+        cfg.gridDim = dim3((unsigned)(((int64_t)rows * per_row + 7) / 8));
+        cfg.blockDim = dim3(256);
+        auto split = bwd ? split_kernel<128, false> : (ext ? split_kernel<256, true> : split_kernel<256, false>);
+        JQ_CUDA(cudaLaunchKernelEx(&cfg, split, xg, rows, width, per_row, reinterpret_cast<uint4*>(scratch), scales, stride, vec));
+        count_launch();
+        CUtensorMap map;
+        rc = activation_map(&map, false, scratch, wpad, rows, 2, a.nt);
+        if (rc != JQ_OK) {
+            break;
+        }
+        a.features = features;
+        a.xscale = scales;
+        a.xstride = stride;
+        a.bias = bias;
+        a.y = out + m0 * features;
+        a.status = status;
+        rc = launch_any(v.type, plan, a, map, s);
+    }
+    return rc;
+}
+
+}  // namespace mm
+
+int launch_matmul_f32(const View& v, const float* x, int64_t m, const float* bias, float* y, cudaStream_t s) {
+    return mm::product_f32(v, false, x, m, bias, y, s);
+}
+
+// gx [m, k] = g [m, n] . dequant(W) (ops/Gguf.java:208-212, ops/Quant.java:191-197); device pointers; n >= 1, m >= 1.
+int launch_linear_backward(const View& v, const float* g, int64_t m, float* gx, cudaStream_t s) { return mm::product_f32(v, true, g, m, nullptr, gx, s); }
+
+bool prefill_supported(const View& v) { return has_linear_kernel(v.type) && v.k % 64 == 0 && v.n > 0 && v.k > 0; }
+
+// y[m, n] = x_bf16[m, k] . W^T (+ bias); x 16-byte aligned device memory.
+int launch_prefill_bf16(const View& v, const uint16_t* x_bf16, int64_t m, const float* bias, float* y, cudaStream_t s) {
+    using namespace mm;
+    if (!prefill_supported(v)) {
+        return fail(JQ_ERR_UNSUPPORTED, "prefill: the tensor-core kernel needs k to be a multiple of 64 (k = %lld)", (long long)v.k);
+    }
+    Args a = {};
+    Plan plan = {};
+    weight_args(v, a);
+    choose(v.type, false, false, v.n, a.kb, (int)m, a, plan);
+    int rc = status_word(&a.status);
+    CUtensorMap map;
+    if (rc == JQ_OK) {
+        rc = activation_map(&map, true, x_bf16, v.k, m, 1, a.nt);
+    }
+    if (rc != JQ_OK) {
+        return rc;
+    }
+    a.features = v.n;
+    a.bias = bias;
+    a.y = y;
+    return launch_any(v.type, plan, a, map, s);
+}
+
+EncodeTiledFn encode_tiled() {
+    static EncodeTiledFn fn = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess) {
+            fn = reinterpret_cast<EncodeTiledFn>(p);
+        }
+    });
+    return fn;
+}
+
+// fp32 -> bf16 (round to nearest even, as the reference's LowPrecision.java:36-46), for jq_linear_f32's prefill option
+static __global__ void f32_to_bf16_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ out, int64_t count) {
+    int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    if (i + 3 < count) {
+        const float4 v = *reinterpret_cast<const float4*>(x + i);
+        __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+        *reinterpret_cast<uint2*>(out + i) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
+    } else {
+        for (; i < count; i++) {
+            out[i] = __float2bfloat16_rn(x[i]);
+        }
+    }
+}
+
+int launch_f32_to_bf16(const float* x, uint16_t* out, int64_t count, cudaStream_t s) {
+    if (count == 0) {
+        return JQ_OK;
+    }
+    const int64_t threads = (count + 3) / 4;
+    f32_to_bf16_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(x, reinterpret_cast<__nv_bfloat16*>(out), count);
+    count_launch();
+    return check_launch("f32_to_bf16_kernel");
+}
+
+// Reads and clears the status word of the matrix kernel on the current device (0 = no wait ever gave up).
+int prefill_status(int* status) {
+    int zero = 0;
+    JQ_CUDA(cudaMemcpyFromSymbol(status, g_matmul_status, sizeof(int)));
+    JQ_CUDA(cudaMemcpyToSymbol(g_matmul_status, &zero, sizeof(int)));
+    return JQ_OK;
+}
+
+}  // namespace jq

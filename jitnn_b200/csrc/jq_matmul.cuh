@@ -1,0 +1,846 @@
+// The matrix kernel: products of a quantised weight with many rows of activations on the 5th-generation tensor cores.
+//
+//   forward   y[m, n]  = x[m, k] . W[n, k]^T (+ bias)     features = rows of W,  contraction over k
+//   backward  gx[m, k] = g[m, n] . W[n, k]                features = k,          contraction over the rows of W
+//
+// Two operand precisions. BF16: x is bfloat16, weights are rounded to bfloat16, one product. FP32: x is split into two halves (hi + lo, 22
+// significant bits), and so are weights that one half cannot hold (jq_matmul_dequant.cuh); the products hi.hi + hi.lo + lo.hi (or
+// the first two) are taken, so that results keep FP32's accuracy; sums leave the tensor core every 256 (backward: 128) terms and are added
+// up in registers, rounded to nearest.
+//
+// A CTA owns 128 features and a tile of up to 256 (FP32: 128) rows of x and walks the contraction in stages of 64. (Pairs of CTAs under one
+// tcgen05.mma, cta_group::2, read each activation tile from L2 once for 256 features; measured equal within 3 % on every shape and
+// dearer to synchronise, so not kept.) Roles:
+//   warp 0       one thread brings activation tiles in by TMA (128-byte swizzle, no multicast). From "free" to "full" a tile takes more than a
+//                microsecond (L2), several stages' worth, so this ring is deeper than that of the weight operands
+//   warp 1       issues tcgen05.mma
+//   warp 2       one thread brings raw units in (128 rows x 256 k, one contiguous run of the tiled weight, cp.async.bulk)
+//   then         groups of four warps that dequantise. The groups take stages in turn, so that what a stage costs a warp besides its
+//                instructions (barrier round trips) overlaps with the other groups' work. Forward: a thread turns 64 weights of its
+//                row into 32 columns of its lane of the operand in tensor memory. In shared memory, writing and reading the weights took
+//                more of its 128 bytes per clock than the rest together, and bound the kernel. Backward: the weights are the transposed
+//                operand, which only shared memory can hold: a thread makes a 128-byte row of 64 features of one contraction index
+//   last         four or eight warps take finished accumulators from tensor memory (double buffered where that fits), add them up, store y
+// A cluster may also split the contraction (ksplit ranges); the ranges' sums then meet through distributed shared memory, in range
+// order. Grid: one cluster per tile and range, or, without ranges, as many CTAs as the GPU has SMs walking the tiles.
+//
+// What bounds it: the tensor pipe for tiles of 200 and more rows of x (BF16, 0.84 of its rate at 256), else the chain of barriers and the
+// dequantiser warps' issue slots (a stage of 128 x 64 weights takes 230 to 260 ns whatever the number of rows).
+//
+// Every wait is bounded: one that runs out records a code, raises the CTA's abort flag and all roles fall through to the exit.
+#pragma once
+
+#include <cuda_bf16.h>
+
+#include "jq_matmul_dequant.cuh"
+#include "jq_tc.cuh"
+
+namespace jq {
+namespace mm {
+
+// Four groups of dequantiser warps where the registers allow it (80 a thread with 23 warps); the FP32 kernel for more than 32 rows of x adds up
+// 64 columns per thread and has two.
+template <bool FP32, int NMAX>
+struct Warps {
+    static constexpr int GROUPS = FP32 && NMAX > 32 ? 2 : 4, FOLD = FP32 && NMAX > 32 ? 8 : 4, THREADS = (3 + 4 * GROUPS + FOLD) * 32;
+};
+constexpr int A_TILE = 128 * 128;  // 128 rows of 128 bytes
+constexpr long long WAIT_CLOCKS = 4000000000ll;  // about two seconds
+constexpr int MAX_A = 6, MAX_B = 12, MAX_RAW = 4;
+
+struct Args {
+    const uint8_t* q;
+    const uint8_t* aux;
+    int kb;           // 256-wide steps of k in the weight
+    int rows128;      // 128-row tiles of the weight
+    int units;        // units along the contraction
+    int ftiles;       // tiles of 128 features
+    int ttiles, nt;   // tiles of nt rows of x
+    int m;
+    int ksplit;
+    int sa, sb, raw;  // ring depths: weight operands, activation tiles, raw units
+    int cols;         // tensor-memory columns of one accumulator
+    int bufs;         // accumulators: 2, or 1 where a second one does not fit
+    int tmem;         // columns to allocate
+    int64_t features; // valid features, and the row length of y
+    const float* xscale;  // FP32: scale of (contraction block, row of x): [block][xstride]
+    int xstride;
+    const float* bias;
+    float* y;
+    int* status;      // 0, or the code of the first wait that gave up: 1 operand free, 2 weights ready, 3 activations ready or their tile free,
+                      // 4 accumulator ready, 5 accumulator free, 6 raw blocks, 8 raw blocks read by all
+};
+
+// Shared-memory matrix descriptors, 128-byte swizzle (layout type 2), descriptor version 1 (sm_100). The high word is the same for all: 1024
+// bytes from one group of eight 128-byte rows to the next. K-major rows hold 64 values of the contraction; feature-major rows 64 features
+// of one contraction index, and the next 64 features follow 8 KB further.
+constexpr uint32_t DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t desc_k(uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | (1u << 16); }
+__device__ __forceinline__ uint32_t desc_mn(uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | ((8192u >> 4) << 16); }
+
+// D (tensor memory, lane = feature) = or += A (shared memory) . B (shared memory); descriptors by their low words
+__device__ __forceinline__ void mma(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}" ::"r"(d),
+        "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "r"(DESC_HI)
+        : "memory");
+}
+
+// The same with the A operand in tensor memory (lane = feature, two values of the contraction per column).
+__device__ __forceinline__ void mma_ta(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 db, {%2, %5};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t}" ::"r"(d),
+        "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "r"(DESC_HI)
+        : "memory");
+}
+
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// A bounded wait, as tc::mbar_wait. (A try_wait with a time limit of its own becomes a sleep in software that wakes late.)
+__device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+    if (tc::mbar_try(bar, parity)) {
+        return true;
+    }
+    const long long t0 = clock64();
+    for (;;) {
+        if (tc::mbar_try(bar, parity)) {
+            return true;
+        }
+        if (*abort_flag != 0) {
+            return false;
+        }
+        if (clock64() - t0 > WAIT_CLOCKS) {
+            break;
+        }
+    }
+    atomicCAS(status, 0, code);
+    *abort_flag = 1;
+    return false;
+}
+
+// The same for a whole warp that goes on to warp-wide instructions: all lanes or none.
+__device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+    return __all_sync(0xffffffffu, wait(bar, parity, abort_flag, status, code));
+}
+
+__device__ __forceinline__ void tma_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst), "l"(map), "r"(bar), "r"(c0),
+                 "r"(c1), "r"(c2)
+                 : "memory");
+}
+
+__device__ __forceinline__ void ld_tmem8(float (&r)[8], uint32_t addr) {
+    uint32_t u[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7])
+                 : "r"(addr)
+                 : "memory");
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        r[i] = __uint_as_float(u[i]);
+    }
+}
+__device__ __forceinline__ void ld_tmem_done() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+__device__ __forceinline__ void st_tmem8(uint32_t addr, const uint32_t (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]),
+                 "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+
+__device__ __forceinline__ void sts16(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+// A run of 16 weights as operand values: bfloat16 (hi), or halves hi and lo.
+template <bool FP32>
+__device__ __forceinline__ void operand_run(const f2 (&w)[8], uint32_t (&hi)[8], uint32_t (&lo)[8]) {
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        float a, b;
+        unpack2(w[i], a, b);
+        if constexpr (FP32) {
+            const __half2 h = __floats2half2_rn(a, b);
+            hi[i] = *reinterpret_cast<const uint32_t*>(&h);
+            float c, d;  // what is left: exact
+            asm("{\n\t.reg .f16 l, h, m;\n\t.reg .b16 minus_one;\n\tmov.b32 {l, h}, %2;\n\tmov.b16 minus_one, 0xBC00;\n\tmov.b16 m, minus_one;\n\t"
+                "fma.rn.f32.f16 %0, l, m, %3;\n\tfma.rn.f32.f16 %1, h, m, %4;\n\t}"
+                : "=f"(c), "=f"(d)
+                : "r"(hi[i]), "f"(a), "f"(b));
+            const __half2 l = __floats2half2_rn(c, d);
+            lo[i] = *reinterpret_cast<const uint32_t*>(&l);
+        } else {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+            hi[i] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+    }
+}
+
+// A run into this lane's row of an operand in tensor memory: pieces p, p + 1 of the row's eight are columns 4 p .. 4 p + 7.
+__device__ __forceinline__ void run_to_tmem(const f2 (&w)[8], uint32_t a, int p) {
+    uint32_t hi[8], lo[8];
+    operand_run<false>(w, hi, lo);
+    st_tmem8(a + 4 * p, hi);
+}
+
+// A run into the row at `row_addr` of an operand in shared memory (pieces p, p + 1, swizzled by row & 7; lo A_TILE further).
+template <bool FP32>
+__device__ __forceinline__ void run_to_smem(const f2 (&w)[8], uint32_t row_addr, int p, int swz) {
+    uint32_t hi[8], lo[8];
+    operand_run<FP32>(w, hi, lo);
+    const uint32_t at0 = row_addr + (uint32_t)((p ^ swz) << 4), at1 = row_addr + (uint32_t)(((p + 1) ^ swz) << 4);
+    sts16(at0, hi[0], hi[1], hi[2], hi[3]);
+    sts16(at1, hi[4], hi[5], hi[6], hi[7]);
+    if constexpr (FP32) {
+        sts16(at0 + A_TILE, lo[0], lo[1], lo[2], lo[3]);
+        sts16(at1 + A_TILE, lo[4], lo[5], lo[6], lo[7]);
+    }
+}
+
+// Bytes of the parts of a CTA's shared memory.
+template <int TYPE>
+__host__ __device__ constexpr int raw_bytes() {
+    return Dq<TYPE>::UNIT_Q + Dq<TYPE>::UNIT_A;
+}
+__host__ __device__ inline int a_bytes(bool bwd) { return bwd ? 2 * A_TILE : 0; }  // the forward product's weights go to tensor memory
+// tensor-memory columns of a stage's weights, and stages of 64 per unit of the contraction
+__host__ __device__ constexpr int a_columns(int type, bool fp32, bool bwd) {
+    return bwd ? 0 : (fp32 && type != JQ_TYPE_Q4_K && type != JQ_TYPE_Q5_K ? 64 : 32);
+}
+__host__ __device__ constexpr int unit_stages(int type, bool fp32, bool bwd) {
+    return bwd ? 2 : (fp32 && (type == JQ_TYPE_Q4_K || type == JQ_TYPE_Q5_K || type == JQ_TYPE_Q4_1) ? 5 : 4);
+}
+__host__ __device__ inline int b_bytes(bool fp32, int nt) { return (fp32 ? 2 * nt : nt) * 128; }
+constexpr int TAIL_BYTES = 4 * 128 * 4 + 8 * 2 * 64 * 4 + 768;  // row factors, the fold warps' scales, barriers
+
+// NMAX: largest tile of rows of x an FP32 instance adds up in registers.
+template <int TYPE, bool FP32, bool BWD, int NMAX>
+__global__ void __launch_bounds__(Warps<FP32, NMAX>::THREADS, 1) matmul_kernel(const __grid_constant__ Args p, const __grid_constant__ CUtensorMap xmap) {
+    using D = Dq<TYPE>;
+    using W = Warps<FP32, NMAX>;
+    using H = Half<TYPE>;
+    static_assert(FP32 || !BWD, "the backward product is FP32");
+    constexpr bool HALF = FP32 && !BWD;                                 // weights by half arithmetic, see there
+    constexpr bool EXT = HALF && H::EXT;                                // a fifth stage with 16 more columns
+    constexpr int UNIT_STAGES = unit_stages(TYPE, FP32, BWD);           // stages of 64 per unit of the contraction
+    constexpr int A_COLS = a_columns(TYPE, FP32, BWD);
+    static_assert(BWD || A_COLS == (HALF ? 32 * H::TILES : 32), "");
+    static_assert(UNIT_STAGES == (BWD ? 2 : 4) + (EXT ? 1 : 0), "");
+    constexpr int G = W::GROUPS;
+    constexpr bool JOINED = FP32 && NMAX <= 32;  // x's hi and lo rows as one operand of 2 nt columns: fewer of the small MMAs, whose issue would bound
+    extern __shared__ uint8_t smem_unaligned[];
+    const uint32_t base = (tc::smem_u32(smem_unaligned) + 1023u) & ~1023u;  // swizzled tiles start on 1024-byte boundaries
+    const int SA = p.sa, SB = p.sb, R = p.raw, nt = p.nt;
+    const uint32_t a_st = (uint32_t)a_bytes(BWD), b_st = (uint32_t)b_bytes(FP32, nt);
+    const uint32_t a0 = base, b0 = a0 + (uint32_t)SA * a_st, raw0 = b0 + (uint32_t)SB * b_st;
+    const uint32_t fac0 = raw0 + (uint32_t)R * raw_bytes<TYPE>();
+    const uint32_t scl0 = fac0 + 4 * 128 * 4, full_a = scl0 + 8 * 2 * 64 * 4, free_a = full_a + 8 * MAX_A, full_b = free_a + 8 * MAX_A, free_b = full_b + 8 * MAX_B;
+    const uint32_t raw_full = free_b + 8 * MAX_B, raw_read = raw_full + 8 * MAX_RAW;
+    const uint32_t acc_full = raw_read + 8 * MAX_RAW, acc_empty = acc_full + 16, fac_full = acc_empty + 16, max_full = fac_full + 32, slot_s = max_full + 64;
+    uint8_t* const generic = smem_unaligned + (slot_s - tc::smem_u32(smem_unaligned));
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(generic);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(generic + 4);
+    volatile uint32_t* unit_max = reinterpret_cast<volatile uint32_t*>(generic + 16);  // backward: [8 units][4 warps] largest bounds
+
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int range = p.ksplit == 1 ? 0 : (int)cluster_rank();  // which range of the contraction
+    const int cluster_id = (int)blockIdx.x / p.ksplit, clusters = (int)gridDim.x / p.ksplit;
+    const int u0 = (int)((int64_t)range * p.units / p.ksplit), u1 = (int)((int64_t)(range + 1) * p.units / p.ksplit);
+    const int tiles = p.ftiles * p.ttiles;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < SA; s++) {
+            tc::mbar_init(full_a + 8 * s, 4);  // a group's four warps
+            tc::mbar_init(free_a + 8 * s, 1);
+        }
+        for (int s = 0; s < SB; s++) {
+            tc::mbar_init(full_b + 8 * s, 1);
+            tc::mbar_init(free_b + 8 * s, 1);
+        }
+        for (int r = 0; r < R; r++) {
+            tc::mbar_init(raw_full + 8 * r, 1);
+            tc::mbar_init(raw_read + 8 * r, 4 * G);
+        }
+        for (int i = 0; i < 2; i++) {
+            tc::mbar_init(acc_full + 8 * i, 1);
+            tc::mbar_init(acc_empty + 8 * i, W::FOLD);
+        }
+        for (int i = 0; i < 4; i++) {
+            tc::mbar_init(fac_full + 8 * i, BWD ? 1 : 4);
+        }
+        for (int i = 0; i < 8; i++) {
+            tc::mbar_init(max_full + 8 * i, 4);
+        }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_s), "r"(p.tmem) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    if (p.ksplit > 1) {
+        cluster_sync();
+    }
+    tc::fence_after_sync();
+    asm volatile("griddepcontrol.launch_dependents;");
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    const uint32_t tmem_a = tmem + (uint32_t)(p.bufs * p.cols);  // the ring of weight operands behind the accumulators
+
+    if (warp == 0) {
+        // ---- activation tiles -------------------------------------------------------------------------------------------------
+        if (lane == 0) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");  // x is written by the kernel in front
+            int s = 0;
+            uint32_t ph = 1;
+            bool ok = true;
+            for (int tile = cluster_id; tile < tiles && ok; tile += clusters) {
+                const int t0 = (tile % p.ttiles) * nt;
+                for (int it = u0 * UNIT_STAGES; it < u1 * UNIT_STAGES; it++) {
+                    if (!(ok = wait(free_b + 8 * s, ph, abort_flag, p.status, 3))) {
+                        break;
+                    }
+                    const uint32_t bar = full_b + 8 * s, dst = b0 + (uint32_t)s * b_st;
+                    tc::mbar_expect_tx(bar, b_st);
+                    tma_3d(dst, &xmap, bar, it * 64, t0, 0);
+                    if constexpr (FP32) {  // hi rows, then lo rows
+                        tma_3d(dst + (uint32_t)nt * 128, &xmap, bar, it * 64, t0, 1);
+                    }
+                    if (++s == SB) {
+                        s = 0;
+                        ph ^= 1;
+                    }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ---- MMA issue: the warp goes through the loop together, so that addresses and descriptors stay in uniform registers, and one elected
+        // lane issues. (A lone lane's loop, converting every operand, took 300 clocks a stage beside busy dequantiser warps.)
+        const uint32_t fmt = FP32 ? 0u : ((1u << 7) | (1u << 10));  // halves or bfloat16
+        const uint32_t id = (1u << 4) | fmt | (BWD ? 1u << 15 : 0u) | ((uint32_t)(128 >> 4) << 24);
+        const uint32_t id_n = id | ((uint32_t)(nt >> 3) << 17), id_2n = id | ((uint32_t)(2 * nt >> 3) << 17);
+        const uint32_t lo_rows = (uint32_t)(nt * 128) >> 4;  // from x's hi rows to its lo rows, in descriptor units
+        int s = 0, sb = 0, buf = 0;
+        uint32_t ph = 0, phb = 0, aph = 0;
+        bool ok = true, ready = false, ready_b = false;
+        for (int tile = cluster_id; tile < tiles && ok; tile += clusters) {
+            uint32_t acc = 0;
+            for (int u = u0; u < u1 && ok; u++) {
+                const uint32_t d = tmem + (uint32_t)(buf * p.cols);
+                if (FP32 || u == u0) {
+                    if (!(ok = wait_warp(acc_empty + 8 * buf, aph ^ 1u, abort_flag, p.status, 5))) {
+                        break;
+                    }
+                    acc = 0;
+                }
+#pragma unroll
+                for (int st = 0; st < UNIT_STAGES; st++) {
+                    ok = (__all_sync(0xffffffffu, ready) || wait_warp(full_a + 8 * s, ph, abort_flag, p.status, 2)) &&
+                         (__all_sync(0xffffffffu, ready_b) || wait_warp(full_b + 8 * sb, phb, abort_flag, p.status, 3));
+                    if (!ok) {
+                        break;
+                    }
+                    // asked before this stage's MMAs are issued: the answer takes over a hundred clocks even when it is yes
+                    const int sn = s + 1 == SA ? 0 : s + 1, sbn = sb + 1 == SB ? 0 : sb + 1;
+                    const uint32_t phn = sn == 0 ? ph ^ 1 : ph, phbn = sbn == 0 ? phb ^ 1 : phb;
+                    ready = tc::mbar_test(full_a + 8 * sn, phn);
+                    ready_b = tc::mbar_test(full_b + 8 * sbn, phbn);
+                    tc::fence_after_sync();
+                    const uint32_t bd = desc_k(b0 + (uint32_t)sb * b_st), bl = bd + lo_rows;  // x: hi, lo; 16 of the contraction are 32 bytes
+                    if (elect_one()) {
+                        if constexpr (BWD) {
+                            // feature-major weights: 16 of the contraction are two 1024-byte groups
+                            const uint32_t ad = desc_mn(a0 + (uint32_t)s * a_st), al = ad + (A_TILE >> 4);
+#pragma unroll
+                            for (uint32_t ks = 0; ks < 4; ks++) {
+                                if constexpr (JOINED) {
+                                    mma(d, ad + 128 * ks, bd + 2 * ks, id_2n, acc | ks);  // hi x (hi | lo)
+                                    mma(d, al + 128 * ks, bd + 2 * ks, id_n, 1u);         // lo x hi
+                                } else {
+                                    mma(d, ad + 128 * ks, bd + 2 * ks, id_n, acc | ks);
+                                    mma(d, ad + 128 * ks, bl + 2 * ks, id_n, 1u);
+                                    mma(d, al + 128 * ks, bd + 2 * ks, id_n, 1u);
+                                }
+                            }
+                        } else {
+                            const uint32_t ta = tmem_a + (uint32_t)(s * A_COLS);  // 16 of the contraction are 8 columns
+                            constexpr bool TWO = HALF && H::TILES == 2;            // the weights have a lo part
+#pragma unroll
+                            for (uint32_t ks = 0; ks < (EXT && st == 4 ? 1 : 4); ks++) {
+                                if constexpr (JOINED) {
+                                    mma_ta(d, ta + 8 * ks, bd + 2 * ks, id_2n, acc | ks);  // hi x (hi | lo)
+                                } else {
+                                    mma_ta(d, ta + 8 * ks, bd + 2 * ks, id_n, acc | ks);
+                                    if constexpr (FP32) {
+                                        mma_ta(d, ta + 8 * ks, bl + 2 * ks, id_n, 1u);
+                                    }
+                                }
+                                if constexpr (TWO) {
+                                    if (!(EXT && st == 4)) {
+                                        mma_ta(d, ta + 32 + 8 * ks, bd + 2 * ks, id_n, 1u);
+                                    }
+                                }
+                            }
+                        }
+                        tc::umma_commit(free_a + 8 * s);
+                        tc::umma_commit(free_b + 8 * sb);
+                        if (st == UNIT_STAGES - 1 && (FP32 || u == u1 - 1)) {
+                            tc::umma_commit(acc_full + 8 * buf);
+                        }
+                    }
+                    __syncwarp();
+                    acc = 1;
+                    s = sn;
+                    ph = phn;
+                    sb = sbn;
+                    phb = phbn;
+                }
+                if (FP32 || u == u1 - 1) {
+                    if (++buf == p.bufs) {
+                        buf = 0;
+                        aph ^= 1;
+                    }
+                }
+            }
+        }
+    } else if (warp == 2) {
+        // ---- raw units, in the order in which they are used: tile after tile, u0 .. u1 - 1 ---------------------------------------
+        if (lane == 0) {
+            int r = 0;
+            uint32_t ph = 1;
+            bool ok = true;
+            for (int tile = cluster_id; tile < tiles && ok; tile += clusters) {
+                const int ft = tile / p.ttiles;
+                for (int u = u0; u < u1; u++) {
+                    const int64_t at = BWD ? (int64_t)u * p.kb + (ft >> 1) : (int64_t)ft * p.kb + u;
+                    if (!(ok = wait(raw_read + 8 * r, ph, abort_flag, p.status, 8))) {
+                        break;
+                    }
+                    const uint32_t dst = raw0 + (uint32_t)r * raw_bytes<TYPE>(), bar = raw_full + 8 * r;
+                    tc::mbar_expect_tx(bar, raw_bytes<TYPE>());
+                    tc::bulk_load(dst, p.q + at * D::UNIT_Q, D::UNIT_Q, bar);
+                    if constexpr (D::UNIT_A > 0) {
+                        tc::bulk_load(dst + D::UNIT_Q, p.aux + at * D::UNIT_A, D::UNIT_A, bar);
+                    }
+                    if (++r == R) {
+                        r = 0;
+                        ph ^= 1;
+                    }
+                }
+            }
+        }
+    } else if (warp < 3 + 4 * G) {
+        // ---- dequantise ------------------------------------------------------------------------------------------------------------
+        const int tid = (threadIdx.x - 96) & 127, group = (warp - 3) >> 2;
+        // forward: a thread has one row of the unit; backward: 64 rows x the two 64-feature halves of this CTA's 128 features
+        // (the warp's place among tensor memory's lanes, 32 (warp % 4) .., decides which)
+        const int row0 = BWD ? (tid & 63) : (warp & 3) * 32 + lane;
+        const uint32_t my_lanes = (uint32_t)((warp & 3) * 32) << 16;
+        const uint32_t row_at = (BWD ? (uint32_t)(tid >> 6) * 8192u : 0u) + (uint32_t)row0 * 128u;  // of the thread's row in the operand tile
+        int s = group, r = 0, at_unit = 0;
+        uint32_t ph = 1, rph = 0;  // SA >= G: the barrier of a group's next stage is never two phases behind
+        bool ok = true, raw_ready = false;
+        int first = group;  // the group's first stage of the unit, or of a later one
+        for (int tile = cluster_id; tile < tiles && ok; tile += clusters) {
+            const int h = (tile / p.ttiles) & 1;  // backward: which 128 of the super-block's features
+            for (int u = u0; u < u1; u++, at_unit++) {
+                // every group waits for and gives back every unit: no group is a whole turn of the ring away from a barrier it tests
+                if (!__all_sync(0xffffffffu, raw_ready) && !(ok = wait_warp(raw_full + 8 * r, rph, abort_flag, p.status, 6))) {
+                    break;
+                }
+                const int rn = r + 1 == R ? 0 : r + 1;
+                const uint32_t rphn = rn == 0 ? rph ^ 1 : rph;
+                raw_ready = tc::mbar_test(raw_full + 8 * rn, rphn);
+                if (first >= UNIT_STAGES) {
+                    __syncwarp();
+                    if (lane == 0) {
+                        tc::mbar_arrive(raw_read + 8 * r);
+                    }
+                } else {
+                    const uint32_t uq = raw0 + (uint32_t)r * raw_bytes<TYPE>(), ua = uq + D::UNIT_Q;
+                    typename D::Head head;
+                    float fac = 1.0f;
+                    uint32_t unit_factor = 0;  // what the fold multiplies the unit's sums by
+                    if constexpr (!BWD) {
+                        head = D::head(uq, ua, row0);
+                    }
+                    if constexpr (HALF) {
+                        unit_factor = __float_as_uint(H::factor(head));
+                    }
+                    if constexpr (BWD) {
+                        // a power of two brings the largest weight that the unit's blocks can hold to [2^13, 2^14); the fold multiplies by its inverse
+                        const int slot = at_unit & 7;  // a group is at most four stages, so fewer than eight units, ahead of another
+                        if (first == 0) {
+                            const uint32_t b = __reduce_max_sync(0xffffffffu, __float_as_uint(D::bound(D::head(uq, ua, tid))));
+                            if (lane == 0) {
+                                unit_max[slot * 4 + (tid >> 5)] = b;
+                                tc::mbar_arrive(max_full + 8 * slot);
+                            }
+                        }
+                        if (!(ok = wait_warp(max_full + 8 * slot, (uint32_t)(at_unit >> 3) & 1u, abort_flag, p.status, 8))) {
+                            break;
+                        }
+                        uint32_t e = max(max(unit_max[slot * 4], unit_max[slot * 4 + 1]), max(unit_max[slot * 4 + 2], unit_max[slot * 4 + 3])) >> 23;
+                        e = e < 40u ? 40u : (e > 254u ? 254u : e);
+                        fac = __uint_as_float((267u - e) << 23);
+                        unit_factor = (e - 13u) << 23;
+                    }
+                    for (int st = first; st < UNIT_STAGES; st += G) {
+                        const int row = BWD ? row0 + 64 * st : row0, c = BWD ? 2 * h + (tid >> 6) : st;
+                        if constexpr (BWD) {
+                            head = D::head(uq, ua, row);
+                        }
+                        const bool ext = EXT && st == 4;
+                        const typename D::Raw raw = D::load(uq, row, ext ? 0 : c);
+                        if (st + G >= UNIT_STAGES) {  // this warp has read all it needs of the unit
+                            __syncwarp();
+                            if (lane == 0) {
+                                tc::mbar_arrive(raw_read + 8 * r);
+                            }
+                        }
+                        const bool ready = tc::mbar_test(free_a + 8 * s, ph);  // asked early: the answer takes longer than it looks
+                        // the first values while it is on its way
+                        f2 w0[8], w1[8];
+                        uint32_t hi[8], lo[8];
+                        typename H::Scales sc;
+                        if constexpr (HALF) {
+                            sc = H::scales(head, ext ? 0 : c);
+                            if (ext) {
+                                H::ext(head, hi);
+                            } else {
+                                H::values(head, raw, sc, c, 0, 0, hi, lo);
+                            }
+                        } else {
+                            D::values(head, raw, c, 0, fac, w0, w1);
+                        }
+                        if (!__all_sync(0xffffffffu, ready) && !(ok = wait_warp(free_a + 8 * s, ph, abort_flag, p.status, 1))) {
+                            break;
+                        }
+                        if (FP32 && st == 0) {
+                            // The unit's factors for the fold. Not before the unit's first stage is this group's: the accumulator four
+                            // units back has then been taken, and the fold is done with what this ring of four held.
+                            const uint32_t fa = fac0 + (uint32_t)(at_unit & 3) * 512u;
+                            if (!BWD || tid == 0) {
+                                asm volatile("st.shared.u32 [%0], %1;" ::"r"(fa + (BWD ? 0u : 4u * (uint32_t)row0)), "r"(unit_factor) : "memory");
+                            }
+                            __syncwarp();
+                            if (lane == 0 && (!BWD || tid == 0)) {
+                                tc::mbar_arrive(fac_full + 8 * (at_unit & 3));
+                            }
+                        }
+                        if constexpr (BWD) {  // operand row = contraction index, 64 features a row
+                            const uint32_t to = a0 + (uint32_t)s * a_st + row_at;
+                            run_to_smem<FP32>(w0, to, D::piece(0, 0), row0 & 7);
+                            run_to_smem<FP32>(w1, to, D::piece(0, 1), row0 & 7);
+                            D::values(head, raw, c, 1, fac, w0, w1);
+                            run_to_smem<FP32>(w0, to, D::piece(1, 0), row0 & 7);
+                            run_to_smem<FP32>(w1, to, D::piece(1, 1), row0 & 7);
+                            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic stores -> visible to the tensor core
+                        } else {
+                            const uint32_t to = tmem_a + my_lanes + (uint32_t)(s * A_COLS);
+                            tc::fence_after_sync();
+                            if constexpr (HALF) {
+                                if (ext) {
+                                    st_tmem8(to, hi);
+                                } else {
+#pragma unroll
+                                    for (int i = 0; i < 4; i++) {
+                                        if (i > 0) {
+                                            H::values(head, raw, sc, c, i >> 1, i & 1, hi, lo);
+                                        }
+                                        st_tmem8(to + 4 * D::piece(i >> 1, i & 1), hi);
+                                        if constexpr (H::TILES == 2) {
+                                            st_tmem8(to + 32 + 4 * D::piece(i >> 1, i & 1), lo);
+                                        }
+                                    }
+                                }
+                            } else {
+                                run_to_tmem(w0, to, D::piece(0, 0));
+                                run_to_tmem(w1, to, D::piece(0, 1));
+                                D::values(head, raw, c, 1, fac, w0, w1);
+                                run_to_tmem(w0, to, D::piece(1, 0));
+                                run_to_tmem(w1, to, D::piece(1, 1));
+                            }
+                            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                            tc::fence_before_sync();
+                        }
+                        __syncwarp();
+                        if (lane == 0) {
+                            tc::mbar_arrive(full_a + 8 * s);
+                        }
+                        if ((s += G) >= SA) {
+                            s -= SA;
+                            ph ^= 1;
+                        }
+                        first += G;
+                    }
+                    if (!ok) {
+                        break;
+                    }
+                }
+                first -= UNIT_STAGES;
+                r = rn;
+                rph = rphn;
+            }
+        }
+    } else {
+        // ---- accumulators to y -----------------------------------------------------------------------------------------------------
+        asm volatile("griddepcontrol.wait;" ::: "memory");  // the scales of x; and y may be read by the kernel in front
+        constexpr int PARTS = W::FOLD / 4;
+        const int group = warp & 3, part = (warp - 3 - 4 * G) >> 2;  // a warp may only read lanes 32 (warp % 4) .. of tensor memory
+        const int lane_row = group * 32 + lane;
+        const uint32_t lanes = (uint32_t)(group * 32) << 16;
+        const int cols = nt / PARTS, c0 = part * cols;  // this warp's columns of the tile: a multiple of 8
+        int chunk = 0, buf = 0;
+        uint32_t aph = 0;
+        bool ok = true;
+        auto release = [&] {  // the accumulator is read: the next one
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) {
+                tc::mbar_arrive(acc_empty + 8 * buf);
+            }
+            if (++buf == p.bufs) {
+                buf = 0;
+                aph ^= 1;
+            }
+        };
+        for (int tile = cluster_id; tile < tiles && ok; tile += clusters) {
+            const int ft = tile / p.ttiles, t0 = (tile % p.ttiles) * nt;
+            const int64_t feature = (int64_t)ft * 128 + lane_row;
+            const bool valid = feature < p.features;
+            const float bias = p.bias != nullptr && valid ? __ldg(p.bias + feature) : 0.0f;
+            // Columns c .. c + 7 of the tile are finished: to y, or (contraction split over the cluster) to this CTA's own partial tile
+            // [column][128]. One warp per scheduler does this, so it is kept short: no test per value where the tile is whole.
+            const int64_t row_bytes = p.features * 4;
+            uint8_t* const yt = reinterpret_cast<uint8_t*>(p.y + (int64_t)t0 * p.features + feature);
+            const bool whole = t0 + nt <= p.m;
+            auto emit8 = [&](int c, const float (&v)[8]) {
+                if (p.ksplit > 1) {
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + (uint32_t)((c + i) * 128 + lane_row) * 4u), "f"(v[i]) : "memory");
+                    }
+                } else if (valid) {
+                    uint8_t* at = yt + (int64_t)c * row_bytes;
+                    if (whole) {
+#pragma unroll
+                        for (int i = 0; i < 8; i++) {
+                            *reinterpret_cast<float*>(at) = v[i] + bias;
+                            at += row_bytes;
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 8; i++) {
+                            if (t0 + c + i < p.m) {
+                                *reinterpret_cast<float*>(at) = v[i] + bias;
+                            }
+                            at += row_bytes;
+                        }
+                    }
+                }
+            };
+            if constexpr (FP32) {
+                constexpr int C = NMAX / PARTS;  // columns per thread
+                f2 sum[C / 2];
+#pragma unroll
+                for (int i = 0; i < C / 2; i++) {
+                    sum[i] = 0;
+                }
+                // the scales of a unit's columns: fetched by the lanes a unit ahead, read back as broadcasts
+                const uint32_t scl = scl0 + (uint32_t)(warp - 3 - 4 * G) * 512u;
+                const float* xs = p.xscale + (int64_t)u0 * p.xstride + t0 + c0;
+                float next[(C + 31) / 32];
+#pragma unroll
+                for (int i = 0; i < (C + 31) / 32; i++) {
+                    next[i] = lane + 32 * i < cols ? __ldg(xs + lane + 32 * i) : 0.0f;
+                }
+                for (int u = u0; u < u1; u++, chunk++) {
+                    const uint32_t sb = scl + (uint32_t)(chunk & 1) * 256u;
+                    __syncwarp();
+#pragma unroll
+                    for (int i = 0; i < (C + 31) / 32; i++) {
+                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(sb + (uint32_t)(lane + 32 * i) * 4u), "f"(next[i]) : "memory");
+                    }
+                    xs += p.xstride;
+                    if (u + 1 < u1) {
+#pragma unroll
+                        for (int i = 0; i < (C + 31) / 32; i++) {
+                            next[i] = lane + 32 * i < cols ? __ldg(xs + lane + 32 * i) : 0.0f;
+                        }
+                    }
+                    __syncwarp();
+                    ok = wait_warp(fac_full + 8 * (chunk & 3), (uint32_t)(chunk >> 2) & 1u, abort_flag, p.status, 6) &&
+                         wait_warp(acc_full + 8 * buf, aph, abort_flag, p.status, 4);
+                    if (!ok) {
+                        break;
+                    }
+                    tc::fence_after_sync();
+                    float f;
+                    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"(fac0 + (uint32_t)(chunk & 3) * 512u + (BWD ? 0u : 4u * (uint32_t)lane_row)));
+                    const f2 ff = pack2(f, f);
+                    const uint32_t d = tmem + lanes + (uint32_t)(buf * p.cols + c0);
+#pragma unroll
+                    for (int c = 0; c < C / 8; c++) {
+                        if (c * 8 < cols) {
+                            float hi[8], lo[8];
+                            ld_tmem8(hi, d + c * 8);
+                            if constexpr (JOINED) {
+                                ld_tmem8(lo, d + nt + c * 8);
+                            }
+                            const uint4 s0 = lds16(sb + c * 32), s1 = lds16(sb + c * 32 + 16);
+                            const uint32_t sc[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+                            ld_tmem_done();
+#pragma unroll
+                            for (int i = 0; i < 4; i++) {
+                                f2 v = mul2(pack2(hi[2 * i], hi[2 * i + 1]), ff);
+                                if constexpr (JOINED) {
+                                    v = fma2(pack2(lo[2 * i], lo[2 * i + 1]), ff, v);
+                                }
+                                sum[c * 4 + i] = fma2(v, pack2(__uint_as_float(sc[2 * i]), __uint_as_float(sc[2 * i + 1])), sum[c * 4 + i]);
+                            }
+                        }
+                    }
+                    release();
+                }
+                if (!ok) {
+                    break;
+                }
+                // (the last accumulator is complete: every tile in shared memory is used up and may hold the partial tile)
+#pragma unroll
+                for (int c = 0; c < C / 8; c++) {
+                    if (c * 8 < cols) {
+                        float v[8];
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            unpack2(sum[c * 4 + i], v[2 * i], v[2 * i + 1]);
+                        }
+                        emit8(c0 + c * 8, v);
+                    }
+                }
+            } else {
+                if (!(ok = wait_warp(acc_full + 8 * buf, aph, abort_flag, p.status, 4))) {
+                    break;
+                }
+                tc::fence_after_sync();
+                const uint32_t d = tmem + lanes + (uint32_t)(buf * p.cols + c0);
+                for (int c = 0; c < cols; c += 16) {
+                    float v[8], w[8];
+                    ld_tmem8(v, d + c);
+                    ld_tmem8(w, d + c + 8);
+                    ld_tmem_done();
+                    emit8(c0 + c, v);
+                    emit8(c0 + c + 8, w);
+                }
+                release();
+            }
+        }
+    }
+
+    // ---- exit -----------------------------------------------------------------------------------------------------------------------
+    tc::fence_before_sync();
+    __syncthreads();
+    if (*abort_flag != 0) {
+        for (int i = 0; i < 1000; i++) {
+            __nanosleep(1000);  // copies that may still be in flight land long before this millisecond is over
+        }
+    }
+    __syncthreads();
+    if (p.ksplit > 1) {
+        cluster_sync();  // partial tiles are complete
+    }
+    if (p.ksplit > 1 && *abort_flag == 0) {
+        // columns range, range + ksplit, .. of the tile: the ranges' sums in range order
+        const int ft = cluster_id / p.ttiles, t0 = (cluster_id % p.ttiles) * nt;
+        const int64_t f0 = (int64_t)ft * 128;
+        const int mine = (nt - range + p.ksplit - 1) / p.ksplit * 32;  // pieces of four features of a column
+        constexpr int BATCH = 2, MOST = 4;  // pieces and ranges in flight: another CTA's memory is most of a microsecond away
+        for (int i0 = threadIdx.x; i0 < mine; i0 += BATCH * W::THREADS) {
+            float4 sum[BATCH];
+#pragma unroll
+            for (int j = 0; j < BATCH; j++) {
+                sum[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+            for (int g0 = 0; g0 < p.ksplit; g0 += MOST) {
+                float4 v[MOST][BATCH];
+#pragma unroll
+                for (int g = 0; g < MOST; g++) {
+                    const uint32_t from = map_rank(base, (uint32_t)(g0 + g < p.ksplit ? g0 + g : 0));
+#pragma unroll
+                    for (int j = 0; j < BATCH; j++) {
+                        const int i = i0 + j * W::THREADS, col = range + (i >> 5) * p.ksplit;
+                        v[g][j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // a missing range adds an exact zero
+                        if (g0 + g < p.ksplit && i < mine) {
+                            asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];"
+                                         : "=f"(v[g][j].x), "=f"(v[g][j].y), "=f"(v[g][j].z), "=f"(v[g][j].w)
+                                         : "r"(from + (uint32_t)(col * 128 + (i & 31) * 4) * 4u));
+                        }
+                    }
+                }
+#pragma unroll
+                for (int g = 0; g < MOST; g++) {
+#pragma unroll
+                    for (int j = 0; j < BATCH; j++) {
+                        sum[j].x += v[g][j].x; sum[j].y += v[g][j].y; sum[j].z += v[g][j].z; sum[j].w += v[g][j].w;
+                    }
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < BATCH; j++) {
+                const int i = i0 + j * W::THREADS, col = range + (i >> 5) * p.ksplit;
+                const int64_t f = f0 + (i & 31) * 4;
+                if (i >= mine || t0 + col >= p.m) {
+                    continue;
+                }
+                float* const at = p.y + (int64_t)(t0 + col) * p.features + f;
+                const float one[4] = {sum[j].x, sum[j].y, sum[j].z, sum[j].w};
+                if (f + 4 <= p.features && ((uintptr_t)at & 15) == 0) {
+                    float4 b = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (p.bias != nullptr) {
+                        b = make_float4(__ldg(p.bias + f), __ldg(p.bias + f + 1), __ldg(p.bias + f + 2), __ldg(p.bias + f + 3));
+                    }
+                    *reinterpret_cast<float4*>(at) = make_float4(one[0] + b.x, one[1] + b.y, one[2] + b.z, one[3] + b.w);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        if (f + q < p.features) {
+                            at[q] = one[q] + (p.bias != nullptr ? __ldg(p.bias + f + q) : 0.0f);
+                        }
+                    }
+                }
+            }
+        }
+    }
+    if (p.ksplit > 1) {
+        __syncthreads();
+        cluster_sync();  // no CTA leaves while another still reads its partial tile
+    }
+    if (warp == 1) {
+        tc::fence_after_sync();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(p.tmem) : "memory");
+    }
+}
+
+}  // namespace mm
+}  // namespace jq

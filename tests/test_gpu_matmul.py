@@ -1,0 +1,100 @@
+"""The tensor-core matrix kernel (FP32 products with many rows of x, and the input gradient) where its tiles, ranges and rings end.
+
+The reference is the product of the oracle's dequantised weights in double. Both operands of the kernel keep 22 significant bits (2^-22 each),
+and sums of at most 272 terms are taken in FP32 by the tensor core before they are added up in FP32 registers: about sqrt(272) 2^-24 = 1e-6
+of the result's norm at random, and 1e-5 leaves room for cancellation.
+"""
+import numpy as np
+import pytest
+import torch
+
+from conftest import LINEAR_TYPES
+from jitnn_b200 import Gguf, Tensor, device_status, synth
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+REL = 1e-5
+
+
+def weight(t, n, k, seed, edit=None):
+    raw = synth.random_valid_blocks(t, n, k, seed=seed).numpy().reshape(-1)
+    if edit is not None:
+        edit(raw)
+    return Tensor.quantized(t, raw, n, k), torch.from_numpy(oracle.dequantize(t, raw).reshape(n, k)).cuda().double()
+
+
+def close(y, ref):
+    assert device_status(0) == 0
+    err = float((y.double() - ref).norm() / ref.norm())
+    assert err <= REL, err
+
+
+# one feature; one row of a second 128-feature tile; one unit of k and more units than rings hold; the widths of the two instances (32 rows of
+# x) and of a tile (128); few enough tiles for k in ranges (1, 2, 4 of them); more tiles than SMs (persistent CTAs)
+SHAPES = [(1, 256, 17), (129, 512, 32), (128, 2816, 33), (257, 4096, 128), (640, 1024, 129), (4096, 4096, 40), (20000, 512, 150)]
+
+
+@pytest.mark.parametrize("n,k,m", SHAPES)
+@pytest.mark.parametrize("t", LINEAR_TYPES)
+def test_linear(t, n, k, m):
+    w, wd = weight(t, n, k, seed=n + m)
+    g = torch.Generator().manual_seed(k)
+    x, b = torch.randn(m, k, generator=g).cuda(), torch.randn(n, generator=g).cuda()
+    close(Gguf.linear(x, w, b), x.double() @ wd.T + b.double())
+    close(Gguf.linear(x, w), x.double() @ wd.T)
+
+
+@pytest.mark.parametrize("n,k,m", [(1, 256, 1), (130, 256, 3), (64, 2816, 32), (4096, 512, 33), (200, 4096, 128), (512, 1024, 300), (300, 20480, 65)])
+@pytest.mark.parametrize("t", LINEAR_TYPES)
+def test_backward(t, n, k, m):
+    w, wd = weight(t, n, k, seed=n + m)
+    g = torch.randn(m, n, generator=torch.Generator().manual_seed(k)).cuda()
+    close(Gguf.linearBackward(g, w), g.double() @ wd)
+
+
+# 32-element formats: k that does not fill a step of 256, or not even a multiple of 4 x 32
+@pytest.mark.parametrize("k", [32, 96, 224, 288, 1056])
+@pytest.mark.parametrize("t", ["Q8_0", "Q4_0", "Q4_1"])
+def test_partial_steps(t, k):
+    n, m = 150, 20
+    w, wd = weight(t, n, k, seed=k)
+    g = torch.Generator().manual_seed(k)
+    x, gy = torch.randn(m, k, generator=g).cuda(), torch.randn(m, n, generator=g).cuda()
+    close(Gguf.linear(x, w), x.double() @ wd.T)
+    close(Gguf.linearBackward(gy, w), gy.double() @ wd)
+
+
+def test_wide_ranges():
+    """Scales and mins of very different sizes within a row's block and across rows, zero and subnormal scales, x over 80 powers of two."""
+    n, k, m = 256, 512, 64
+    for t in LINEAR_TYPES:
+        block = {"Q8_0": 34, "Q4_0": 18, "Q4_1": 20, "Q4_K": 144, "Q5_K": 176, "Q6_K": 210}[t]
+        fields = {"Q8_0": [0], "Q4_0": [0], "Q4_1": [0, 2], "Q4_K": [0, 2], "Q5_K": [0, 2], "Q6_K": [208]}[t]
+
+        def edit(raw):
+            blocks = raw.reshape(-1, block)
+            rng = np.random.default_rng(1)
+            for f in fields:
+                v = (2.0 ** rng.uniform(-24, 4, len(blocks))).astype(np.float16)
+                v[rng.random(len(blocks)) < 0.1] = 0
+                blocks[:, f:f + 2] = v.view(np.uint8).reshape(-1, 2)
+
+        w, wd = weight(t, n, k, 7, edit)
+        x = torch.randn(m, k, generator=torch.Generator().manual_seed(3)).cuda() * (2.0 ** torch.linspace(-40, 40, m))[:, None].cuda()
+        y = Gguf.linear(x, w)
+        ref = x.double() @ wd.T
+        # per output: relative to the sum of the magnitudes of what is added up
+        assert float(((y.double() - ref).abs() / (x.double().abs() @ wd.abs().T + 1e-300)).max()) <= REL
+        assert device_status(0) == 0
+
+
+def test_nan_and_inf_reach_their_rows():
+    w, wd = weight("Q4_K", 256, 1024, 5)
+    x = torch.randn(40, 1024, generator=torch.Generator().manual_seed(3)).cuda()
+    x[3, 17], x[20, 1000] = float("nan"), float("inf")
+    y = Gguf.linear(x, w)
+    bad = ~torch.isfinite(y)
+    assert bool(bad[3].all()) and bool(bad[20].all())
+    rows = [r for r in range(40) if r not in (3, 20)]
+    close(y[rows], x[rows].double() @ wd.T)
