@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "jq_common.cuh"
+#include "jq_prompt.cuh"
 #include "jq_q4k_image.cuh"
 #include "jq_q6k_image.cuh"
 #include "jq_peer_device.cuh"
@@ -91,18 +92,29 @@ __global__ void embed_kernel(const int* __restrict__ tokens, const float* __rest
     }
 }
 
+// Element i, or elements 4 i .. 4 i + 3, of a float or bfloat16 (round to nearest even) array.
+__device__ __forceinline__ void store1(float* o, int64_t i, float v) { o[i] = v; }
+__device__ __forceinline__ void store1(__nv_bfloat16* o, int64_t i, float v) { o[i] = __float2bfloat16_rn(v); }
+__device__ __forceinline__ void store4(float* o, int64_t i, float4 v) { reinterpret_cast<float4*>(o)[i] = v; }
+__device__ __forceinline__ void store4(__nv_bfloat16* o, int64_t i, float4 v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    reinterpret_cast<uint2*>(o)[i] = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+
 // If delta != nullptr: x += delta (the residual add). Then out = x * rsqrt(mean(x^2) + eps) * w (RMSNorm).
 // One CTA of NORM_THREADS threads per row: with few rows the kernel is bound by the latency of its loads, so every thread has
 // all of its row's values in flight at once (128-bit loads) and keeps up to 16 of them in registers for the second pass.
+// Out: float, or bfloat16 for a linear that rounds its input to it.
 constexpr int NORM_THREADS = 1024;
+template <typename Out>
 __global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ delta, const float* __restrict__ w,
-                                                                   float eps, float* __restrict__ out, int dim) {
+                                                                   float eps, Out* __restrict__ out, int dim) {
     asm volatile("griddepcontrol.launch_dependents;");  // launched programmatically, the kernel behind this one may be scheduled now ...
     asm volatile("griddepcontrol.wait;" ::: "memory");  // ... and this one touches memory only when the kernel before it has finished
     __shared__ float scratch[32];
     float* xr = x + (int64_t)blockIdx.x * dim;
     const float* dr = delta != nullptr ? delta + (int64_t)blockIdx.x * dim : nullptr;
-    float* o = out + (int64_t)blockIdx.x * dim;
+    Out* o = out + (int64_t)blockIdx.x * dim;
     constexpr int HOLD = 4;
     const int nv = (dim & 3) == 0 ? dim >> 2 : 0;  // 128-bit pieces; a dim that is no multiple of 4 takes the scalar loops below
     float4 held[HOLD];
@@ -138,11 +150,11 @@ __global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_kernel(float* __rest
         const int i = threadIdx.x + h * NORM_THREADS;
         if (i < nv) {
             const float4 wv = reinterpret_cast<const float4*>(w)[i];
-            reinterpret_cast<float4*>(o)[i] = make_float4(held[h].x * inv * wv.x, held[h].y * inv * wv.y, held[h].z * inv * wv.z, held[h].w * inv * wv.w);
+            store4(o, i, make_float4(held[h].x * inv * wv.x, held[h].y * inv * wv.y, held[h].z * inv * wv.z, held[h].w * inv * wv.w));
         }
     }
     for (int i = rest + threadIdx.x; i < dim; i += NORM_THREADS) {
-        o[i] = xr[i] * inv * w[i];
+        store1(o, i, xr[i] * inv * w[i]);
     }
 }
 
@@ -316,152 +328,20 @@ __global__ void attention_combine_kernel(const float* __restrict__ part, float* 
     }
 }
 
-// Causal attention for a long run of consecutive tokens (the prompt path): CTA (head h, group of PA_Q queries) walks the keys
-// 0 .. (its last query's position) in tiles of PA_KEYS. A tile of keys and values is loaded into shared memory once and
-// serves all PA_Q queries; per query a running maximum m, a running sum l and the output row are carried from tile to
-// tile (the usual streaming softmax: out = sum_j exp(s_j - m) v_j / sum_j exp(s_j - m)). Thread (query, key) pairs compute
-// the scores, two queries per warp the softmax statistics, thread d the output dimension d of every query.
-constexpr int PA_Q = 8;
-constexpr int PA_KEYS = 64;
-constexpr int PA_THREADS = 128;
-
-template <int HD>
-constexpr size_t prompt_attention_smem() {
-    return (size_t)(PA_Q * HD + PA_KEYS * (HD + 4) + PA_KEYS * HD + PA_Q * PA_KEYS + 3 * PA_Q) * sizeof(float);
-}
-
-template <int HD>
-__global__ void __launch_bounds__(PA_THREADS) attention_prompt_kernel(const float* __restrict__ q, const float* __restrict__ k_cache,
-                                                                       const float* __restrict__ v_cache, float* __restrict__ out,
-                                                                       const int* __restrict__ pos0p, int heads, int kv_heads, int T, float scale) {
-    static_assert(HD == 64 || HD == 128, "head sizes of the prompt path");
-    extern __shared__ __align__(16) float pa_smem[];
-    float* qs = pa_smem;                          // [PA_Q][HD]
-    float* ks = qs + PA_Q * HD;                   // [PA_KEYS][HD + 4]: the pad spreads a key's 16-byte pieces over the banks
-    float* vs = ks + PA_KEYS * (HD + 4);          // [PA_KEYS][HD]
-    float* ps = vs + PA_KEYS * HD;                // [PA_Q][PA_KEYS] scores, then exp(score - m)
-    float* m_s = ps + PA_Q * PA_KEYS;             // [PA_Q] running maximum
-    float* l_s = m_s + PA_Q;                      // [PA_Q] running sum
-    float* a_s = l_s + PA_Q;                      // [PA_Q] exp(m before - m after) of the tile
-    const int h = blockIdx.x, t0 = blockIdx.y * PA_Q, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nq = T - t0 < PA_Q ? T - t0 : PA_Q;
-    const int pos0 = *pos0p;
-    const int kv_dim = kv_heads * HD;
-    const int kvh = h / (heads / kv_heads);
-    const int keys_all = pos0 + t0 + nq;  // keys the last query of the group sees
-    for (int i = tid; i < PA_Q * HD; i += PA_THREADS) {
-        const int qi = i / HD, d = i % HD;
-        qs[i] = qi < nq ? q[((int64_t)(t0 + qi) * heads + h) * HD + d] : 0.0f;
-    }
-    if (tid < PA_Q) {
-        m_s[tid] = -INFINITY;
-        l_s[tid] = 0.0f;
-    }
-    float acc[PA_Q];
-#pragma unroll
-    for (int i = 0; i < PA_Q; i++) {
-        acc[i] = 0.0f;
-    }
-    for (int kc = 0; kc < keys_all; kc += PA_KEYS) {
-        const int cnt = keys_all - kc < PA_KEYS ? keys_all - kc : PA_KEYS;
-        __syncthreads();  // the tile before is used up (first pass: qs, m_s, l_s are written)
-        // ---- the tile's keys and values
-        constexpr int V4 = HD / 4;
-        for (int i = tid; i < PA_KEYS * V4; i += PA_THREADS) {
-            const int r = i / V4, c = i % V4;
-            float4 kv4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), vv4 = kv4;
-            if (r < cnt) {
-                const int64_t off = (int64_t)(kc + r) * kv_dim + kvh * HD + 4 * c;
-                kv4 = *reinterpret_cast<const float4*>(k_cache + off);
-                vv4 = *reinterpret_cast<const float4*>(v_cache + off);
-            }
-            *reinterpret_cast<float4*>(ks + r * (HD + 4) + 4 * c) = kv4;
-            *reinterpret_cast<float4*>(vs + r * HD + 4 * c) = vv4;
-        }
-        __syncthreads();
-        // ---- scores: pair p = (query p / PA_KEYS, key p % PA_KEYS)
-        for (int p = tid; p < PA_Q * PA_KEYS; p += PA_THREADS) {
-            const int qi = p / PA_KEYS, j = p % PA_KEYS;
-            const float4* kr = reinterpret_cast<const float4*>(ks + j * (HD + 4));
-            const float4* qr = reinterpret_cast<const float4*>(qs + qi * HD);
-            float d0 = 0.0f, d1 = 0.0f, d2 = 0.0f, d3 = 0.0f;
-#pragma unroll 8
-            for (int c = 0; c < V4; c++) {
-                const float4 a = qr[c], b = kr[c];
-                d0 = fmaf(a.x, b.x, d0);
-                d1 = fmaf(a.y, b.y, d1);
-                d2 = fmaf(a.z, b.z, d2);
-                d3 = fmaf(a.w, b.w, d3);
-            }
-            const bool seen = qi < nq && j < cnt && kc + j <= pos0 + t0 + qi;
-            ps[p] = seen ? ((d0 + d1) + (d2 + d3)) * scale : -INFINITY;
-        }
-        __syncthreads();
-        // ---- statistics: warp w takes queries w and w + 4
-#pragma unroll
-        for (int u = 0; u < PA_Q / 4; u++) {
-            const int qi = warp + 4 * u;
-            const float s0 = ps[qi * PA_KEYS + lane], s1 = ps[qi * PA_KEYS + lane + 32];
-            float mx = fmaxf(s0, s1);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-            }
-            const float m_old = m_s[qi];
-            const float m_new = fmaxf(m_old, mx);
-            const float e0 = s0 == -INFINITY ? 0.0f : expf(s0 - m_new), e1 = s1 == -INFINITY ? 0.0f : expf(s1 - m_new);
-            float sum = e0 + e1;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                sum += __shfl_xor_sync(0xffffffffu, sum, o);
-            }
-            ps[qi * PA_KEYS + lane] = e0;
-            ps[qi * PA_KEYS + lane + 32] = e1;
-            __syncwarp();
-            if (lane == 0) {
-                const float alpha = m_old == -INFINITY ? 0.0f : expf(m_old - m_new);  // no key seen so far: nothing to carry
-                a_s[qi] = alpha;
-                l_s[qi] = fmaf(l_s[qi], alpha, sum);
-                m_s[qi] = m_new;
-            }
-        }
-        __syncthreads();
-        // ---- weighted values: thread d, every query
-        if (tid < HD) {
-#pragma unroll
-            for (int qi = 0; qi < PA_Q; qi++) {
-                acc[qi] *= a_s[qi];
-            }
-            for (int j = 0; j < PA_KEYS; j += 4) {
-                const float v0 = vs[j * HD + tid], v1 = vs[(j + 1) * HD + tid], v2 = vs[(j + 2) * HD + tid], v3 = vs[(j + 3) * HD + tid];
-#pragma unroll
-                for (int qi = 0; qi < PA_Q; qi++) {
-                    const float4 pr = *reinterpret_cast<const float4*>(ps + qi * PA_KEYS + j);
-                    acc[qi] = fmaf(pr.w, v3, fmaf(pr.z, v2, fmaf(pr.y, v1, fmaf(pr.x, v0, acc[qi]))));
-                }
-            }
-        }
-    }
-    if (tid < HD) {
-#pragma unroll
-        for (int qi = 0; qi < PA_Q; qi++) {
-            if (qi < nq) {
-                out[((int64_t)(t0 + qi) * heads + h) * HD + tid] = acc[qi] / l_s[qi];
-            }
-        }
-    }
-}
-
-__global__ void set_pos_kernel(int pos0, int* __restrict__ pos) { *pos = pos0; }
-
-// act = silu(gate) * up
-__global__ void swiglu_kernel(const float* __restrict__ gate, const float* __restrict__ up, float* __restrict__ act, int64_t count) {
+// act = silu(gate) * up, four elements per thread
+template <typename Out>
+__global__ void __launch_bounds__(256) swiglu_kernel(const float* __restrict__ gate, const float* __restrict__ up, Out* __restrict__ act, int64_t count) {
     asm volatile("griddepcontrol.launch_dependents;");  // launched programmatically, the kernel behind this one may be scheduled now ...
     asm volatile("griddepcontrol.wait;" ::: "memory");  // ... and this one touches memory only when the kernel before it has finished
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < count) {
-        const float g = gate[i];
-        act[i] = (g / (1.0f + expf(-g))) * up[i];
+    auto one = [](float g, float u) { return (g / (1.0f + expf(-g))) * u; };
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (4 * i + 3 < count) {
+        const float4 g = reinterpret_cast<const float4*>(gate)[i], u = reinterpret_cast<const float4*>(up)[i];
+        store4(act, i, make_float4(one(g.x, u.x), one(g.y, u.y), one(g.z, u.z), one(g.w, u.w)));
+    } else {
+        for (int64_t j = 4 * i; j < count; j++) {
+            store1(act, j, one(gate[j], up[j]));
+        }
     }
 }
 
@@ -1524,7 +1404,7 @@ static int enqueue_forward(jq_decoder* d, int T, int max_keys, const TokenArgs* 
         float* kc = d->k_cache + seq_base + (size_t)l * d->max_seq * kv_dim;
         float* vc = d->v_cache + seq_base + (size_t)l * d->max_seq * kv_dim;
         // attention block; the residual add of the previous block's feed-forward output is fused into this norm
-        if (rc == JQ_OK) pdl_err = launch_pdl(add_rmsnorm_kernel, dim3(T), dim3(NORM_THREADS), 0, s, true, d->x, l == 0 ? nullptr : d->proj, d->norms + (size_t)(2 * l) * dim, d->eps, d->xn, dim);
+        if (rc == JQ_OK) pdl_err = launch_pdl(add_rmsnorm_kernel<float>, dim3(T), dim3(NORM_THREADS), 0, s, true, d->x, l == 0 ? nullptr : d->proj, d->norms + (size_t)(2 * l) * dim, d->eps, d->xn, dim);
         LAUNCHED("add_rmsnorm_kernel");
         {
             float* const qkv[3] = {d->q, d->k, d->v};
@@ -1543,7 +1423,7 @@ static int enqueue_forward(jq_decoder* d, int T, int max_keys, const TokenArgs* 
         LIN(L[3], d->att, d->proj);
         if (rc != JQ_OK) break;
         // feed-forward block
-        if (rc == JQ_OK) pdl_err = launch_pdl(add_rmsnorm_kernel, dim3(T), dim3(NORM_THREADS), 0, s, true, d->x, d->proj, d->norms + (size_t)(2 * l + 1) * dim, d->eps, d->xn, dim);
+        if (rc == JQ_OK) pdl_err = launch_pdl(add_rmsnorm_kernel<float>, dim3(T), dim3(NORM_THREADS), 0, s, true, d->x, d->proj, d->norms + (size_t)(2 * l + 1) * dim, d->eps, d->xn, dim);
         LAUNCHED("add_rmsnorm_kernel");
         {
             float* const gu[2] = {d->gate, d->up};
@@ -1551,12 +1431,12 @@ static int enqueue_forward(jq_decoder* d, int T, int max_keys, const TokenArgs* 
         }
         if (rc != JQ_OK) break;
         const int64_t cnt = (int64_t)T * d->hidden;
-        if (rc == JQ_OK) pdl_err = launch_pdl(swiglu_kernel, dim3((unsigned)((cnt + 255) / 256)), dim3(256), 0, s, true, d->gate, d->up, d->act, cnt);
+        if (rc == JQ_OK) pdl_err = launch_pdl(swiglu_kernel<float>, dim3((unsigned)((cnt + 1023) / 1024)), dim3(256), 0, s, true, d->gate, d->up, d->act, cnt);
         LAUNCHED("swiglu_kernel");
         LIN(L[6], d->act, d->proj);
     }
     if (rc == JQ_OK) {
-        if (rc == JQ_OK) pdl_err = launch_pdl(add_rmsnorm_kernel, dim3(T), dim3(NORM_THREADS), 0, s, true, d->x, d->proj, d->norms + (size_t)(2 * d->layers) * dim, d->eps, d->xn, dim);
+        if (rc == JQ_OK) pdl_err = launch_pdl(add_rmsnorm_kernel<float>, dim3(T), dim3(NORM_THREADS), 0, s, true, d->x, d->proj, d->norms + (size_t)(2 * d->layers) * dim, d->eps, d->xn, dim);
         LAUNCHED("add_rmsnorm_kernel");
         LIN(d->output, d->xn, d->logits);
     }
@@ -1689,7 +1569,7 @@ static int enqueue_forward_sharded(jq_decoder* d, int T, int max_keys, const Tok
                 rc = decoder_gemv_imaged3(d, L[0], d->q, L[1], d->k, L[2], d->v, s);
             }
         } else {
-            add_rmsnorm_kernel<<<T, NORM_THREADS, 0, s>>>(d->x, l == 0 ? nullptr : D, d->norms + (size_t)(2 * l) * dim, d->eps, d->xn, dim);
+            add_rmsnorm_kernel<float><<<T, NORM_THREADS, 0, s>>>(d->x, l == 0 ? nullptr : D, d->norms + (size_t)(2 * l) * dim, d->eps, d->xn, dim);
             LAUNCHED("add_rmsnorm_kernel");
             float* const qkv[3] = {d->q, d->k, d->v};
             if (rc == JQ_OK) rc = linear_device_multi(L, 3, d->xn, T, qkv, s);
@@ -1727,7 +1607,7 @@ static int enqueue_forward_sharded(jq_decoder* d, int T, int max_keys, const Tok
             NORM_IMAGE(B, d->norms + (size_t)(2 * l + 1) * dim, {L[4], L[5]});
             GEMV_IMAGED(L[4], d->gate, L[5], d->up);
         } else {
-            add_rmsnorm_kernel<<<T, NORM_THREADS, 0, s>>>(d->x, B, d->norms + (size_t)(2 * l + 1) * dim, d->eps, d->xn, dim);
+            add_rmsnorm_kernel<float><<<T, NORM_THREADS, 0, s>>>(d->x, B, d->norms + (size_t)(2 * l + 1) * dim, d->eps, d->xn, dim);
             LAUNCHED("add_rmsnorm_kernel");
             float* const gu[2] = {d->gate, d->up};
             if (rc == JQ_OK) rc = linear_device_multi(L + 4, 2, d->xn, T, gu, s);
@@ -1744,14 +1624,14 @@ static int enqueue_forward_sharded(jq_decoder* d, int T, int max_keys, const Tok
             if (rc == JQ_OK) rc = peer_linear_q4k_imaged(L[6], shard_image(d, 6), dim, d->rank * dim_l, d->peer_buf, d->area[3], d->stage[3], d->rank, G, s, true, false);
         } else {
             const int64_t cnt = (int64_t)T * hidden_l;
-            swiglu_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, s>>>(d->gate, d->up, d->act, cnt);
+            swiglu_kernel<float><<<(unsigned)((cnt + 1023) / 1024), 256, 0, s>>>(d->gate, d->up, d->act, cnt);
             LAUNCHED("swiglu_kernel");
             GATHER(d->act, d->hidden, hidden_l, 2);
             PEER_LIN(L[6], C, dim, dim_l, 3);
         }
     }
     if (rc == JQ_OK) {
-        add_rmsnorm_kernel<<<T, NORM_THREADS, 0, s>>>(d->x, D, d->norms + (size_t)(2 * d->layers) * dim, d->eps, d->xn, dim);
+        add_rmsnorm_kernel<float><<<T, NORM_THREADS, 0, s>>>(d->x, D, d->norms + (size_t)(2 * d->layers) * dim, d->eps, d->xn, dim);
         LAUNCHED("add_rmsnorm_kernel");
         PEER_LIN(d->output, d->xn, d->vocab, vocab_l, 4);
     }
@@ -1901,8 +1781,8 @@ JQ_API int jq_decoder_forward_batch(jq_decoder* d, const int32_t* tokens_host, i
 
 // ---- the prompt path ---------------------------------------------------------------------------------------------------------
 // A long run of consecutive tokens in one pass over the weights: the general path's operators on T rows, with every linear
-// on the tensor-core prefill kernel (its input rounded to bfloat16, FP32 accumulation) and the attention of all T queries by
-// attention_prompt_kernel. Only the last token's logits are computed.
+// on the tensor-core matrix kernel (its input rounded to bfloat16, FP32 accumulation) and the attention of all T queries by
+// jq_prompt_attention.cu. Only the last token's logits are computed.
 constexpr int PROMPT_MAX_TOKENS = 4096;
 
 static int ensure_prompt_workspace(jq_decoder* d, int rows) {
@@ -1917,9 +1797,10 @@ static int ensure_prompt_workspace(jq_decoder* d, int rows) {
     d->prompt_tokens = nullptr;
     d->prompt_rows = 0;
     const size_t kv_dim = (size_t)d->kv_heads * d->head_dim;
-    const size_t per_row = (size_t)5 * d->dim + 2 * kv_dim + 3 * (size_t)d->hidden;  // x, xn, q, att, proj; k, v; gate, up, act
+    const size_t per_row = (size_t)3 * d->dim + 2 * kv_dim + 2 * (size_t)d->hidden;  // x, q, proj; k, v; gate, up
     const size_t widest = (size_t)(d->dim > d->hidden ? d->dim : d->hidden);
-    cudaError_t e = cudaMalloc(&d->prompt_buf, (size_t)rows * per_row * sizeof(float));
+    // the attention's workspace: queries of the run, keys and values of the whole cache
+    cudaError_t e = cudaMalloc(&d->prompt_buf, (size_t)rows * per_row * sizeof(float) + prompt_attention_bytes(rows, d->max_seq, d->heads, d->kv_heads, d->head_dim) + 256);
     if (e == cudaSuccess) e = cudaMalloc(&d->prompt_bf16, (size_t)rows * widest * sizeof(uint16_t));
     if (e == cudaSuccess) e = cudaMalloc(&d->prompt_tokens, (size_t)rows * sizeof(int));
     if (e != cudaSuccess) {
@@ -1989,84 +1870,69 @@ JQ_API int jq_decoder_prompt(jq_decoder* d, int seq, const int32_t* tokens_host,
     if (rc == JQ_OK) {
         float* p = d->prompt_buf;
         float* x = p; p += (size_t)T * dim;
-        float* xn = p; p += (size_t)T * dim;
         float* q = p; p += (size_t)T * dim;
-        float* att = p; p += (size_t)T * dim;
         float* proj = p; p += (size_t)T * dim;
         float* k = p; p += (size_t)T * kv_dim;
         float* v = p; p += (size_t)T * kv_dim;
         float* gate = p; p += (size_t)T * hidden;
         float* up = p; p += (size_t)T * hidden;
-        float* act = p;
-        uint16_t* xb = d->prompt_bf16;
-        // a linear on all T rows: the input rounded to bfloat16 once (`fresh`), then the tensor-core kernel
-        auto LIN = [&](const jq_weight* w, const float* in, float* out_, bool fresh) {
-            if (rc == JQ_OK && fresh) {
-                rc = launch_f32_to_bf16(in, xb, (int64_t)T * w->k, s);
-            }
+        // the input of every linear, rounded to bfloat16 by the kernel that makes it; each linear's is used up before the next is written
+        __nv_bfloat16* xb = reinterpret_cast<__nv_bfloat16*>(d->prompt_bf16);
+        PromptAttention att = {};
+        att.q = q; att.k = k; att.v = v;
+        att.cos_t = d->cos_t; att.sin_t = d->sin_t;
+        att.out = xb;
+        att.T = T; att.pos0 = pos0; att.heads = d->heads; att.kv_heads = d->kv_heads;
+        att.scale = (float)(1.0 / std::sqrt((double)hd));
+        prompt_attention_layout(att, reinterpret_cast<uint8_t*>(((uintptr_t)p + 255) / 256 * 256), hd);
+        auto LIN = [&](const jq_weight* w, float* out_) {
             if (rc == JQ_OK) {
-                rc = launch_prefill_bf16(View{w->q, w->aux, w->n, w->k, w->type}, xb, T, nullptr, out_, s);
+                rc = launch_prefill_bf16(View{w->q, w->aux, w->n, w->k, w->type}, d->prompt_bf16, T, nullptr, out_, s);
             }
+        };
+        auto KERNEL = [&](cudaError_t e, const char* name) {
+            count_launch(1);
+            CK(e, name);
         };
         // the copy out of pageable host memory is staged before the call returns: the caller's buffer is free afterwards
         CK(cudaMemcpyAsync(d->prompt_tokens, tokens_host, (size_t)T * sizeof(int), cudaMemcpyHostToDevice, s), "prompt tokens");
         if (rc == JQ_OK) {
-            set_pos_kernel<<<1, 1, 0, s>>>(pos0, d->pos);
-            LAUNCHED("set_pos_kernel");
-        }
-        if (rc == JQ_OK) {
             embed_kernel<<<T, 256, 0, s>>>(d->prompt_tokens, d->embed, x, dim, d->vocab);
             LAUNCHED("embed_kernel");
         }
-        const float scale = (float)(1.0 / std::sqrt((double)hd));
         const size_t seq_elems = (size_t)d->layers * d->max_seq * kv_dim, seq_base = (size_t)seq * seq_elems;
-        static std::atomic<uint64_t> configured{0};  // the opt-in for large dynamic shared memory is per device
-        if (rc == JQ_OK && (configured.load() >> (d->device & 63) & 1) == 0) {
-            CK(cudaFuncSetAttribute(attention_prompt_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prompt_attention_smem<64>()), "attention_prompt_kernel");
-            CK(cudaFuncSetAttribute(attention_prompt_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prompt_attention_smem<128>()), "attention_prompt_kernel");
-            configured.fetch_or((uint64_t)1 << (d->device & 63));
-        }
+        const int64_t cnt = (int64_t)T * hidden;
         for (int l = 0; l < d->layers && rc == JQ_OK; l++) {
             const jq_weight* const* L = &d->lin[(size_t)l * 7];
-            float* kc = d->k_cache + seq_base + (size_t)l * d->max_seq * kv_dim;
-            float* vc = d->v_cache + seq_base + (size_t)l * d->max_seq * kv_dim;
-            add_rmsnorm_kernel<<<T, NORM_THREADS, 0, s>>>(x, l == 0 ? nullptr : proj, d->norms + (size_t)(2 * l) * dim, d->eps, xn, dim);
-            LAUNCHED("add_rmsnorm_kernel");
-            LIN(L[0], xn, q, true);
-            LIN(L[1], xn, k, false);
-            LIN(L[2], xn, v, false);
+            KERNEL(launch_pdl(add_rmsnorm_kernel<__nv_bfloat16>, dim3(T), dim3(NORM_THREADS), 0, s, true, x, l == 0 ? nullptr : proj,
+                              d->norms + (size_t)(2 * l) * dim, d->eps, xb, dim), "add_rmsnorm_kernel");
+            LIN(L[0], q);
+            LIN(L[1], k);
+            LIN(L[2], v);
             if (rc != JQ_OK) break;
-            rope_store_kernel<<<dim3(T, d->heads + 2 * d->kv_heads), hd / 2, 0, s>>>(q, k, v, kc, vc, d->cos_t, d->sin_t, d->pos, d->heads, d->kv_heads, hd, 1, 0);
-            LAUNCHED("rope_store_kernel");
-            const dim3 agrid((unsigned)d->heads, (unsigned)((T + PA_Q - 1) / PA_Q));
-            if (hd == 128) {
-                attention_prompt_kernel<128><<<agrid, PA_THREADS, prompt_attention_smem<128>(), s>>>(q, kc, vc, att, d->pos, d->heads, d->kv_heads, T, scale);
-            } else {
-                attention_prompt_kernel<64><<<agrid, PA_THREADS, prompt_attention_smem<64>(), s>>>(q, kc, vc, att, d->pos, d->heads, d->kv_heads, T, scale);
-            }
-            LAUNCHED("attention_prompt_kernel");
-            LIN(L[3], att, proj, true);
+            att.k_cache = d->k_cache + seq_base + (size_t)l * d->max_seq * kv_dim;
+            att.v_cache = d->v_cache + seq_base + (size_t)l * d->max_seq * kv_dim;
+            rc = launch_prompt_attention(att, hd, s);
+            LIN(L[3], proj);
             if (rc != JQ_OK) break;
-            add_rmsnorm_kernel<<<T, NORM_THREADS, 0, s>>>(x, proj, d->norms + (size_t)(2 * l + 1) * dim, d->eps, xn, dim);
-            LAUNCHED("add_rmsnorm_kernel");
-            LIN(L[4], xn, gate, true);
-            LIN(L[5], xn, up, false);
+            KERNEL(launch_pdl(add_rmsnorm_kernel<__nv_bfloat16>, dim3(T), dim3(NORM_THREADS), 0, s, true, x, proj, d->norms + (size_t)(2 * l + 1) * dim,
+                              d->eps, xb, dim), "add_rmsnorm_kernel");
+            LIN(L[4], gate);
+            LIN(L[5], up);
             if (rc != JQ_OK) break;
-            const int64_t cnt = (int64_t)T * hidden;
-            swiglu_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, s>>>(gate, up, act, cnt);
-            LAUNCHED("swiglu_kernel");
-            LIN(L[6], act, proj, true);
+            KERNEL(launch_pdl(swiglu_kernel<__nv_bfloat16>, dim3((unsigned)((cnt + 1023) / 1024)), dim3(256), 0, s, true, gate, up, xb, cnt), "swiglu_kernel");
+            LIN(L[6], proj);
         }
         if (rc == JQ_OK) {
             // the last token alone goes on: final residual add and norm, output projection (FP32 path), first index of the maximum
             const size_t last = (size_t)(T - 1) * dim;
-            add_rmsnorm_kernel<<<1, NORM_THREADS, 0, s>>>(x + last, proj + last, d->norms + (size_t)(2 * d->layers) * dim, d->eps, d->xn, dim);
-            LAUNCHED("add_rmsnorm_kernel");
+            KERNEL(launch_pdl(add_rmsnorm_kernel<float>, dim3(1), dim3(NORM_THREADS), 0, s, true, x + last, proj + last, d->norms + (size_t)(2 * d->layers) * dim, d->eps,
+                              d->xn, dim), "add_rmsnorm_kernel");
             if (rc == JQ_OK) rc = linear_device(d->output, d->xn, 1, nullptr, d->logits, s);
         }
         if (rc == JQ_OK) {
-            argmax_kernel<<<1, 1024, 0, s>>>(d->logits, d->argmax, d->vocab);
-            LAUNCHED("argmax_kernel");
+            KERNEL(launch_pdl(argmax_split_kernel, dim3(ARGMAX_CTAS), dim3(256), 0, s, true, d->logits, d->vocab, d->argmax_v, d->argmax_i,
+                              d->counters + d->dim / 256 + 1, d->argmax), "argmax_split_kernel");
         }
     }
     if (rc == JQ_OK && (logits_host != nullptr || next_host != nullptr)) {
