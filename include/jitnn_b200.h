@@ -119,8 +119,8 @@ JQ_API int jq_dequantize(const jq_weight* w, float* dst, int dst_mem, void* stre
  * non-finite outputs (Q4_K, Q5_K: NaN in every output of that row of x). Stands in for Gguf.linear(x, w, bias) (ops/Gguf.java:76-98) and
  * Quant.linear / F.linearQ8 (ops/Quant.java:66-80): any m >= 0 (leading axes of x flattened by the
  * caller as ops/Gguf.java:86-93 does), bias may be NULL. Rows are dispatched like the reference
- * dispatches them (ops/Gguf.java:90): m <= 16 to the fused dequantise-GEMV kernels, larger m to the tensor-core matrix
- * kernel, which takes x and the weights as sums of two half-precision numbers (22 significant bits, relative to the largest
+ * dispatches them (ops/Gguf.java:90): few rows to the fused dequantise-GEMV kernels, more (from 5 to 12 on, by format;
+ * always above 16) to the tensor-core matrix kernel, which takes x and the weights as sums of two half-precision numbers (22 significant bits, relative to the largest
  * magnitude of a 256-element block) and adds up in FP32, unless the bfloat16 prefill path is selected with
  * jq_set_option. `mem` says where x, bias and y live (all three alike); with JQ_MEM_DEVICE they must
  * be 16-byte aligned and `stream` is the CUDA stream (cudaStream_t, NULL = default stream).
@@ -217,10 +217,9 @@ JQ_API int jq_quantize_q8_0(int device, const float* x, int64_t count, void* blo
  *   "decoder_graph"     zero: the decoder issues its single-token step kernel by kernel instead of replaying a CUDA graph.
  *   "decoder_fused"     zero: the decoder's single-token step uses the general kernels (one per operator) instead of the
  *                       fused ones that hand activations to the next linear as its activation image.
- *   "gemv_tcgen05"      which Q4_K and Q5_K decode GEMVs run on the tcgen05 kernel (1 to 16 rows of x in one pass over the weights)
- *                       instead of the mma.sync one (up to 8 rows per pass). 0 (default): those where it is the faster of the
- *                       two, 11 or more rows of x on a weight of at least one 128-row tile per SM, and the shapes the mma.sync
- *                       kernel declines; 1: all; 2: none.
+ *   "gemv_tcgen05"      which Q4_K and Q5_K decode GEMVs run on the tcgen05 GEMV (1 to 16 rows of x in one pass over the weights)
+ *                       instead of the mma.sync one (up to 8 rows) and the matrix kernel (more). 0 (default): the shapes the
+ *                       mma.sync kernel declines; 1: all; 2: none.
  *   "wait_limit_us"     microseconds after which a bounded device-side wait of the tcgen05 GEMV gives up (default 2 000 000; a
  *                       wait that gives up makes jq_device_status report 64 + the waiting role, and the outputs of that call
  *                       are undefined).

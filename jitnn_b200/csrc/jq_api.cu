@@ -206,21 +206,18 @@ int linear_device(const jq_weight* w, const float* x, int64_t m, const float* bi
         }
         return rc;
     }
-    // The integer tensor-core kernel of Q4_K and Q5_K takes up to 8 activation rows per pass (the tcgen05 one, where it is chosen, 16),
-    // Q6_K's 4, the generic kernel 16.
     const bool tc = g_opt_gemv_generic.load() == 0;
-    // Q8_0, Q4_0 and Q4_1 (k a multiple of 256) go two rows at a time through their tensor-core kernel: re-reading the weights
-    // (mostly from L2) per pair of rows is far cheaper than the generic kernel's arithmetic.
-    const bool blk32 = tc && gemv_blk32_i8_scratch_bytes(w->type, w->k, 2) > 0;
-    const int64_t group = (tc && (w->type == JQ_TYPE_Q4_K || w->type == JQ_TYPE_Q5_K)) ? 8 : ((tc && w->type == JQ_TYPE_Q6_K) ? 4 : (blk32 ? 2 : 16));
-    // More than 16 rows: the matrix kernel reads the weight once for all of them (200 rows of Q4_K 11008 x 4096: 55 us, in groups of eight
-    // rows 360 us).
-    if (tc && m > 16) {
+    // (under option gemv_tcgen05 = 1 up to 16 rows of Q4_K and Q5_K go to the tcgen05 GEMV)
+    if (tc && matmul_takes(v, m) && !(m <= 16 && gemv_umma_takes(w->type, w->k, (int)m))) {
         return launch_matmul_f32(v, x, m, bias, y, s);
     }
+    // The integer tensor-core kernel of Q4_K and Q5_K takes up to 8 activation rows per pass, Q6_K's 4, the one of Q8_0, Q4_0 and Q4_1 2, the
+    // generic kernel 16.
+    const bool blk32 = tc && gemv_blk32_i8_scratch_bytes(w->type, w->k, 2) > 0;
+    const int64_t group = (tc && (w->type == JQ_TYPE_Q4_K || w->type == JQ_TYPE_Q5_K)) ? 8 : ((tc && w->type == JQ_TYPE_Q6_K) ? 4 : (blk32 ? 2 : 16));
     for (int64_t m0 = 0; m0 < m;) {
         const int left = (int)(m - m0 < 16 ? m - m0 : 16);
-        const int rows = gemv_umma_takes(w->type, w->k, left, w->n) ? left : (int)(left < group ? left : group);
+        const int rows = gemv_umma_takes(w->type, w->k, left) ? left : (int)(left < group ? left : group);
         int rc = launch_gemv(v, x + m0 * w->k, rows, bias, y + m0 * w->n, s, x_remote);
         if (rc != JQ_OK) {
             return rc;
@@ -239,10 +236,8 @@ int linear_device_multi(const jq_weight* const* ws, int count, const float* x, i
     }
     const int64_t min_rows = g_prefill_min_rows.load();
     bool same = count >= 1;
-    int64_t n_all = 0;
     for (int i = 0; i < count && same; i++) {
         same = ws[i]->type == ws[0]->type && ws[i]->k == ws[0]->k && ws[i]->n > 0;
-        n_all += ws[i]->n;
     }
     if (!same && count >= 2 && count <= 3) {
         // mixed formats (a Q6_K wv beside Q4_K wq and wk): those like the first go together, the others alone
@@ -263,7 +258,14 @@ int linear_device_multi(const jq_weight* const* ws, int count, const float* x, i
         return n_like > 0 ? linear_device_multi(like, n_like, x, m, like_y, s) : JQ_OK;
     }
     const bool together = same && count >= 2 && count <= 3 && m >= 1 && m <= 16 && !(min_rows > 0 && m >= min_rows);
-    if (together && gemv_umma_takes(ws[0]->type, ws[0]->k, (int)m, n_all)) {
+    if (together && g_opt_gemv_generic.load() == 0 && matmul_takes(view_of(ws[0]), m) && !gemv_umma_takes(ws[0]->type, ws[0]->k, (int)m)) {
+        View vs[3];
+        for (int i = 0; i < count; i++) {
+            vs[i] = view_of(ws[i]);
+        }
+        return launch_matmul_f32_multi(vs, count, x, m, ys, s);
+    }
+    if (together && gemv_umma_takes(ws[0]->type, ws[0]->k, (int)m)) {
         View vs[3];
         for (int i = 0; i < count; i++) {
             vs[i] = view_of(ws[i]);

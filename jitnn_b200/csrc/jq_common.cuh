@@ -191,7 +191,7 @@ int scratch_for_slot(cudaStream_t s, int slot, size_t bytes, uint8_t** out);
 int scratch_zeroed_for_slot(cudaStream_t s, int slot, size_t bytes, uint8_t** out);
 
 // Decode GEMV on tcgen05 (jq_gemv_umma.cu): Q4_K and Q5_K, 1 to 16 rows of x in one pass over the weights.
-bool gemv_umma_takes(int type, int64_t k, int rows, int64_t n = 0);
+bool gemv_umma_takes(int type, int64_t k, int rows);  // under option gemv_tcgen05 = 1
 bool gemv_umma_fallback(int type, int64_t k, int rows);  // may stand in for the mma.sync kernel on a shape that one declines
 size_t gemv_umma_image_bytes(int64_t k, int rows);
 inline size_t gemv_umma_image_bytes_one_row(int64_t k) { return gemv_umma_image_bytes(k, 1); }
@@ -201,8 +201,7 @@ int launch_gemv_umma(const View& v, const View* v2, const float* x, uint8_t* ima
 int launch_gemv_umma_multi(const View* vs, int count, const float* x, uint8_t* image, int rows, const float* bias, float* const* ys, cudaStream_t s,
                            const PeerOut* peer = nullptr, bool no_scratch = false);
 int gemv_umma_status(int* status);
-// Option "gemv_tcgen05": 1 sends Q4_K and Q5_K decode (1 to 16 rows) to the tcgen05 kernel instead of the mma.sync one, 2 never,
-// 0 where it is faster (many rows of x, many rows of the weight).
+// Option "gemv_tcgen05": 1 sends Q4_K and Q5_K decode (1 to 16 rows) to the tcgen05 GEMV, 2 never, 0 where the mma.sync kernel declines.
 extern std::atomic<int64_t> g_opt_gemv_umma;
 // Option "wait_limit_us": microseconds after which a bounded device-side wait of the tcgen05 GEMV gives up.
 extern std::atomic<int64_t> g_opt_wait_limit_us;
@@ -213,6 +212,9 @@ constexpr int PAD_ROWS = 16;
 
 // The matrix kernel (jq_matmul.cu): the FP32 product with many rows of x, and the bfloat16 product.
 int launch_matmul_f32(const View& v, const float* x, int64_t m, const float* bias, float* y, cudaStream_t s);
+// Several weights of one k on the same x: the split of x into halves is shared (formats may differ in whether they need its sums).
+int launch_matmul_f32_multi(const View* vs, int count, const float* x, int64_t m, float* const* ys, cudaStream_t s);
+bool matmul_takes(const View& v, int64_t rows);  // where it is the fastest of the FP32 kernels
 bool prefill_supported(const View& v);
 int launch_prefill_bf16(const View& v, const uint16_t* x_bf16, int64_t m, const float* bias, float* y, cudaStream_t s);
 int launch_f32_to_bf16(const float* x, uint16_t* out, int64_t count, cudaStream_t s);

@@ -297,29 +297,191 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_partial_kernel(const fl
     }
 }
 
-// out[t, h, :] = sum_s exp(m_s - M) acc_s / sum_s exp(m_s - M) l_s over the splits of (t, h), in split order.
+// The same for head sizes 64 and 128, all query heads that share a key/value head in one CTA: CTA (kv head, split, t) has its 64 keys and values
+// in registers (warp w keys 8w .. 8w + 7, a lane HD / 32 neighbouring dimensions of each) and goes through the group's query heads. With one CTA
+// per query head, a group of eight read every cached byte eight times, and the dot products' shuffles, five per key, bound it (16 sequences of
+// 64 heads at position 256: 55 us).
+constexpr int GROUP_THREADS = 256;
+template <int HD>
+__global__ void __launch_bounds__(GROUP_THREADS) attention_group_kernel(const float* __restrict__ q, const float* __restrict__ k_cache,
+                                                                       const float* __restrict__ v_cache, float* __restrict__ part,
+                                                                       const int* __restrict__ pos0, int heads, int kv_heads, int splits, float scale,
+                                                                       int pos_step, int64_t tok_stride) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    static_assert(HD == 64 || HD == 128, "head sizes");
+    constexpr int V = HD / 32;
+    __shared__ float red[2][8][HD];
+    __shared__ float stat[2][16];
+    const int kvh = blockIdx.x, sp = blockIdx.y, t = blockIdx.z, group = heads / kv_heads;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int keys = *pos0 + t * pos_step + 1, k0 = sp * ATT_CHUNK;
+    float* const out0 = part + (((int64_t)t * heads + (int64_t)kvh * group) * splits + sp) * (HD + 2);
+    const int64_t head_stride = (int64_t)splits * (HD + 2);
+    if (k0 >= keys) {
+        for (int hh = tid; hh < group; hh += GROUP_THREADS) {
+            out0[hh * head_stride + HD] = -INFINITY;  // m
+            out0[hh * head_stride + HD + 1] = 0.0f;   // l
+        }
+        return;
+    }
+    const int cnt = keys - k0 < ATT_CHUNK ? keys - k0 : ATT_CHUNK;
+    const int kv_dim = kv_heads * HD;
+    const float* kb = k_cache + t * tok_stride + (int64_t)(k0 + warp * 8) * kv_dim + kvh * HD + lane * V;
+    const float* vb = v_cache + t * tok_stride + (int64_t)(k0 + warp * 8) * kv_dim + kvh * HD + lane * V;
+    auto get = [](const float* p, float (&r)[V]) {
+        if constexpr (V == 4) {
+            const float4 x = *reinterpret_cast<const float4*>(p);
+            r[0] = x.x; r[1] = x.y; r[2] = x.z; r[3] = x.w;
+        } else {
+            const float2 x = *reinterpret_cast<const float2*>(p);
+            r[0] = x.x; r[1] = x.y;
+        }
+    };
+    float kr[8][V], vr[8][V];
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+#pragma unroll
+        for (int i = 0; i < V; i++) {
+            kr[u][i] = vr[u][i] = 0.0f;
+        }
+        if (warp * 8 + u < cnt) {
+            get(kb + (int64_t)u * kv_dim, kr[u]);
+            get(vb + (int64_t)u * kv_dim, vr[u]);
+        }
+    }
+    const float* qp = q + ((int64_t)t * heads + (int64_t)kvh * group) * HD + lane * V;
+    float qn[V];
+    get(qp, qn);
+    // after the halving exchange below a lane holds the score of key (lane >> 2), every key in four lanes
+    const int my_key = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+    const bool seen = warp * 8 + my_key < cnt;
+    for (int hh = 0; hh < group; hh++) {
+        float qv[V];
+#pragma unroll
+        for (int i = 0; i < V; i++) {
+            qv[i] = qn[i];
+        }
+        if (hh + 1 < group) {
+            get(qp + (hh + 1) * HD, qn);
+        }
+        float d[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            d[u] = 0.0f;
+#pragma unroll
+            for (int i = 0; i < V; i++) {
+                d[u] = fmaf(qv[i], kr[u][i], d[u]);
+            }
+        }
+        // eight sums over 32 lanes in nine shuffles: exchange halves of the keys, then sum the last two bits of the lane
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float mine = (lane & 16) ? d[i + 4] : d[i], other = (lane & 16) ? d[i] : d[i + 4];
+            d[i] = mine + __shfl_xor_sync(0xffffffffu, other, 16);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const float mine = (lane & 8) ? d[i + 2] : d[i], other = (lane & 8) ? d[i] : d[i + 2];
+            d[i] = mine + __shfl_xor_sync(0xffffffffu, other, 8);
+        }
+        {
+            const float mine = (lane & 4) ? d[1] : d[0], other = (lane & 4) ? d[0] : d[1];
+            d[0] = mine + __shfl_xor_sync(0xffffffffu, other, 4);
+        }
+        d[0] += __shfl_xor_sync(0xffffffffu, d[0], 2);
+        d[0] += __shfl_xor_sync(0xffffffffu, d[0], 1);
+        const float sco = seen ? d[0] * scale : -INFINITY;
+        float mw = sco;
+#pragma unroll
+        for (int o = 16; o >= 4; o >>= 1) {
+            mw = fmaxf(mw, __shfl_xor_sync(0xffffffffu, mw, o));
+        }
+        const float pj = mw == -INFINITY ? 0.0f : expf(sco - mw);  // 0 for the keys beyond the chunk's count
+        float lw = pj;
+#pragma unroll
+        for (int o = 16; o >= 4; o >>= 1) {
+            lw += __shfl_xor_sync(0xffffffffu, lw, o);
+        }
+        float acc[V];
+#pragma unroll
+        for (int i = 0; i < V; i++) {
+            acc[i] = 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const float w = __shfl_sync(0xffffffffu, pj, (u >> 2) * 16 + ((u >> 1) & 1) * 8 + (u & 1) * 4);
+#pragma unroll
+            for (int i = 0; i < V; i++) {
+                acc[i] = fmaf(w, vr[u][i], acc[i]);
+            }
+        }
+        const int buf = hh & 1;  // (a buffer is written again only behind the next head's barrier)
+#pragma unroll
+        for (int i = 0; i < V; i++) {
+            red[buf][warp][lane * V + i] = acc[i];
+        }
+        if (lane == 0) {
+            stat[buf][warp] = mw;
+            stat[buf][8 + warp] = lw;
+        }
+        __syncthreads();
+        // the 8 warps' results in warp order
+        if (tid <= HD) {
+            float M = stat[buf][0];  // warp 0 always has a key
+#pragma unroll
+            for (int wv = 1; wv < 8; wv++) {
+                M = fmaxf(M, stat[buf][wv]);
+            }
+            float sum = 0.0f, l = 0.0f;
+#pragma unroll
+            for (int wv = 0; wv < 8; wv++) {
+                const float wgt = expf(stat[buf][wv] - M);  // 0 for a warp without keys
+                l = fmaf(wgt, stat[buf][8 + wv], l);
+                sum = fmaf(wgt, red[buf][wv][tid & (HD - 1)], sum);
+            }
+            float* const out = out0 + hh * head_stride;
+            if (tid < HD) {
+                out[tid] = sum;
+            } else {
+                out[HD] = M;
+                out[HD + 1] = l;
+            }
+        }
+    }
+}
+
+// out[t, h, :] = sum_s exp(m_s - M) acc_s / sum_s exp(m_s - M) l_s over the splits of (t, h), in split order. The splits' maxima and sums are
+// read at once, one per thread; chunks without a visible key (those of a captured step beyond the position) have weight zero and are not read.
+constexpr int MAX_SPLITS = 128;  // 8192 positions
 __global__ void attention_combine_kernel(const float* __restrict__ part, float* __restrict__ out, int heads, int head_dim, int stride_splits,
                                          int splits) {
     asm volatile("griddepcontrol.launch_dependents;");  // launched programmatically, the kernel behind this one may be scheduled now ...
     asm volatile("griddepcontrol.wait;" ::: "memory");  // ... and this one touches memory only when the kernel before it has finished
     // stride_splits = chunks the partial buffer was laid out for, splits = chunks written by this call
+    __shared__ float wm[MAX_SPLITS], wl[MAX_SPLITS];
     const int h = blockIdx.x, t = blockIdx.y;
     const float* p = part + ((int64_t)t * heads + h) * stride_splits * (head_dim + 2);
+    for (int s = threadIdx.x; s < splits; s += blockDim.x) {
+        wm[s] = p[(int64_t)s * (head_dim + 2) + head_dim];
+        wl[s] = p[(int64_t)s * (head_dim + 2) + head_dim + 1];
+    }
+    __syncthreads();
     float M = -INFINITY;
     for (int s = 0; s < splits; s++) {
-        M = fmaxf(M, p[(int64_t)s * (head_dim + 2) + head_dim]);
+        M = fmaxf(M, wm[s]);
     }
     float L = 0.0f;
     for (int s = 0; s < splits; s++) {
-        const float m = p[(int64_t)s * (head_dim + 2) + head_dim];
-        if (m != -INFINITY) {
-            L = fmaf(expf(m - M), p[(int64_t)s * (head_dim + 2) + head_dim + 1], L);
+        if (wm[s] != -INFINITY) {
+            L = fmaf(expf(wm[s] - M), wl[s], L);
         }
     }
     for (int d = threadIdx.x; d < head_dim; d += blockDim.x) {
         float acc = 0.0f;
+#pragma unroll 4
         for (int s = 0; s < splits; s++) {
-            const float m = p[(int64_t)s * (head_dim + 2) + head_dim];
+            const float m = wm[s];
             if (m != -INFINITY) {
                 acc = fmaf(expf(m - M), p[(int64_t)s * (head_dim + 2) + d], acc);
             }
@@ -344,48 +506,6 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const float* __restrict__ g
         }
     }
 }
-
-// First index of the maximum of each row (ops/Reduce.java:201). grid = rows, 1024 threads.
-__global__ void __launch_bounds__(1024) argmax_kernel(const float* __restrict__ logits, int* __restrict__ out, int vocab) {
-    asm volatile("griddepcontrol.launch_dependents;");  // launched programmatically, the kernel behind this one may be scheduled now ...
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // ... and this one touches memory only when the kernel before it has finished
-    __shared__ float bv[32];
-    __shared__ int bi[32];
-    const float* row = logits + (int64_t)blockIdx.x * vocab;
-    float best = -INFINITY;
-    int idx = 0x7fffffff;
-    for (int i = threadIdx.x; i < vocab; i += blockDim.x) {
-        const float v = row[i];
-        if (v > best || (v == best && i < idx)) {
-            best = v;
-            idx = i;
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-        if (ov > best || (ov == best && oi < idx)) {
-            best = ov;
-            idx = oi;
-        }
-    }
-    if ((threadIdx.x & 31) == 0) {
-        bv[threadIdx.x >> 5] = best;
-        bi[threadIdx.x >> 5] = idx;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); w++) {
-            if (bv[w] > best || (bv[w] == best && bi[w] < idx)) {
-                best = bv[w];
-                idx = bi[w];
-            }
-        }
-        out[blockIdx.x] = idx;
-    }
-}
-
 
 // ---- the single-token step with fewer, fused kernels --------------------------------------------------------------
 // For one token and Q4_K / Q6_K linears the kernels that produce an activation vector (norm, attention, SwiGLU) write
@@ -709,8 +829,8 @@ __global__ void __launch_bounds__(256) swiglu_image_kernel(const float* __restri
     }
 }
 
-// First index of the maximum (ops/Reduce.java:201) of one row, over ARGMAX_CTAS CTAs: each leaves its best (value,
-// index), the CTA that finishes last picks among them.
+// First index of the maximum (ops/Reduce.java:201) of each row (grid y), over ARGMAX_CTAS CTAs: each leaves its best (value,
+// index), the CTA of a row that finishes last picks among them.
 constexpr int ARGMAX_CTAS = 64;
 __global__ void __launch_bounds__(256) argmax_split_kernel(const float* __restrict__ logits, int vocab, float* __restrict__ best_v, int* __restrict__ best_i,
                                                            int* __restrict__ counter, int* __restrict__ out) {
@@ -718,6 +838,10 @@ __global__ void __launch_bounds__(256) argmax_split_kernel(const float* __restri
     __shared__ int bi[8];
     __shared__ int last_flag;
     pdl_enter();
+    logits += (int64_t)blockIdx.y * vocab;
+    best_v += blockIdx.y * ARGMAX_CTAS;
+    best_i += blockIdx.y * ARGMAX_CTAS;
+    counter += blockIdx.y;
     float best = -INFINITY;
     int idx = 0x7fffffff;
     for (int i = blockIdx.x * 256 + threadIdx.x; i < vocab; i += ARGMAX_CTAS * 256) {
@@ -783,7 +907,7 @@ __global__ void __launch_bounds__(256) argmax_split_kernel(const float* __restri
         }
     }
     if (threadIdx.x == 0) {
-        out[0] = idx == 0x7fffffff ? 0 : idx;
+        out[blockIdx.y] = idx == 0x7fffffff ? 0 : idx;
     }
 }
 
@@ -837,6 +961,7 @@ int decoder_peer_status(int* status) {
 }  // namespace jq
 
 #define JQ_DECODER_MAGIC 0x4a514443u
+constexpr int GRAPHS = 6;  // 256 << 5 = 8192 positions
 
 struct jq_decoder {
     uint32_t magic;
@@ -854,16 +979,16 @@ struct jq_decoder {
     int splits;          // key chunks of ATT_CHUNK positions covering max_seq
     int *tokens, *pos, *argmax;
     uint8_t *img_q4k, *img_q6k;  // activation images of the fused single-token step
-    int* counters;               // [dim / 256 attention merge counters][1 argmax counter], zero between launches
-    float* argmax_v;             // [ARGMAX_CTAS] per-CTA best value
-    int* argmax_i;               // [ARGMAX_CTAS] per-CTA best index
+    int* counters;               // [dim / 256 attention merge counters][one argmax counter per row], zero between launches
+    float* argmax_v;             // [rows][ARGMAX_CTAS] per-CTA best value
+    int* argmax_i;               // [rows][ARGMAX_CTAS] per-CTA best index
     int* host_stage;     // pinned: [0..7] tokens in, [8] position in, [9..16] argmax out
     int sequences;       // key/value caches held (jq_decoder_set_sequences)
     int cur_seq;         // the sequence the call being enqueued works on
     bool cur_batch;      // the call being enqueued runs one token of each of the first T sequences
-    int graph_T, graph_seq;  // what the captured step was captured for (batch: graph_seq = -1)
+    int graph_T, graph_seq;  // what the captured steps were captured for (batch: graph_seq = -1)
     int warm_calls;      // decode steps of that kind issued so far
-    cudaGraphExec_t graph;  // the decode step, captured on its second call
+    cudaGraphExec_t graphs[GRAPHS];  // the decode step, captured on its second call, for up to 256, 512, 1024 ... cached positions
     cudaStream_t own_stream;  // used when the caller passes no stream (the legacy default stream cannot be captured)
     // Row-sharded form (jq_decoder_set_shard): this rank holds rows [rank * n / world, (rank + 1) * n / world) of every
     // linear, that is heads / world query heads, kv_heads / world key/value heads and hidden / world feed-forward
@@ -882,6 +1007,15 @@ struct jq_decoder {
 };
 
 using namespace jq;
+
+static void drop_graphs(jq_decoder* d) {
+    for (cudaGraphExec_t& g : d->graphs) {
+        if (g != nullptr) {
+            cudaGraphExecDestroy(g);
+            g = nullptr;
+        }
+    }
+}
 
 static int check_decoder(const jq_decoder* d, const char* who) {
     if (d == nullptr || d->magic != JQ_DECODER_MAGIC) {
@@ -920,9 +1054,7 @@ JQ_API int jq_decoder_destroy(jq_decoder* d) {
     cudaFree(d->prompt_buf);
     cudaFree(d->prompt_bf16);
     cudaFree(d->prompt_tokens);
-    if (d->graph != nullptr) {
-        cudaGraphExecDestroy(d->graph);
-    }
+    drop_graphs(d);
     if (d->own_stream != nullptr) {
         cudaStreamSynchronize(d->own_stream);
         cudaStreamDestroy(d->own_stream);
@@ -968,7 +1100,9 @@ JQ_API int jq_decoder_create(int device, int layers, int dim, int heads, int kv_
     d->lin.assign((size_t)layers * 7, nullptr);
     d->output = nullptr;
     d->warm_calls = 0;
-    d->graph = nullptr;
+    for (cudaGraphExec_t& g : d->graphs) {
+        g = nullptr;
+    }
     d->sequences = 1;
     d->cur_seq = 0;
     d->cur_batch = false;
@@ -1032,13 +1166,13 @@ JQ_API int jq_decoder_create(int device, int layers, int dim, int heads, int kv_
     if (e == cudaSuccess) e = cudaMallocHost(&d->host_stage, (2 * T + 1) * sizeof(int));
     {
         const int64_t kmax = dim > hidden ? dim : hidden;
-        const size_t ncount = (size_t)(dim / 256 + 2);
+        const size_t ncount = (size_t)(dim / 256 + 1 + T);
         if (e == cudaSuccess) e = cudaMalloc(&d->img_q4k, q4k_image_bytes_one_row(kmax) + 256);
         if (e == cudaSuccess) e = cudaMalloc(&d->img_q6k, q6k_image_bytes_one_row(kmax) + 256);
         if (e == cudaSuccess) e = cudaMalloc(&d->counters, ncount * sizeof(int));
         if (e == cudaSuccess) e = cudaMemset(d->counters, 0, ncount * sizeof(int));
-        if (e == cudaSuccess) e = cudaMalloc(&d->argmax_v, ARGMAX_CTAS * sizeof(float));
-        if (e == cudaSuccess) e = cudaMalloc(&d->argmax_i, ARGMAX_CTAS * sizeof(int));
+        if (e == cudaSuccess) e = cudaMalloc(&d->argmax_v, T * ARGMAX_CTAS * sizeof(float));
+        if (e == cudaSuccess) e = cudaMalloc(&d->argmax_i, T * ARGMAX_CTAS * sizeof(int));
     }
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&d->own_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) {
@@ -1104,10 +1238,7 @@ JQ_API int jq_decoder_set_shard(jq_decoder* d, int rank, int world, void* const*
             return fail(JQ_ERR_INVALID, "jq_decoder_set_shard: the buffer of rank %d is null", r);
         }
     }
-    if (d->graph != nullptr) {
-        cudaGraphExecDestroy(d->graph);
-        d->graph = nullptr;
-    }
+    drop_graphs(d);
     d->world = world;
     d->rank = rank;
     for (int r = 0; r < 8; r++) {
@@ -1139,10 +1270,7 @@ JQ_API int jq_decoder_set_linear(jq_decoder* d, int layer, int which, const jq_w
         return fail(JQ_ERR_INVALID, "jq_decoder_set_linear: layer %d slot %d needs a [%lld, %lld] weight, got [%lld, %lld]", layer, which, (long long)n,
                     (long long)k, (long long)w->n, (long long)w->k);
     }
-    if (d->graph != nullptr) {
-        cudaGraphExecDestroy(d->graph);  // the captured forward holds the old weight
-        d->graph = nullptr;
-    }
+    drop_graphs(d);  // the captured forward holds the old weight
     if (layer == -1) {
         d->output = w;
     } else {
@@ -1350,6 +1478,21 @@ static int enqueue_forward_fused(jq_decoder* d, int max_keys, const TokenArgs* t
 
 static int enqueue_forward_sharded(jq_decoder* d, int T, int max_keys, const TokenArgs* ta, cudaStream_t s);
 
+// The general path's attention of T tokens over `splits_now` chunks of keys, into the decoder's partial results.
+static cudaError_t launch_attention(jq_decoder* d, int heads, int kv_heads, int T, int splits_now, const float* kc, const float* vc, float scale, int pos_step,
+                                    int64_t tok_stride, bool programmatic, cudaStream_t s) {
+    if (d->head_dim == 128) {
+        return launch_pdl(attention_group_kernel<128>, dim3(kv_heads, splits_now, T), dim3(GROUP_THREADS), 0, s, programmatic, d->q, kc, vc, d->att_part, d->pos, heads,
+                          kv_heads, d->splits, scale, pos_step, tok_stride);
+    }
+    if (d->head_dim == 64) {
+        return launch_pdl(attention_group_kernel<64>, dim3(kv_heads, splits_now, T), dim3(GROUP_THREADS), 0, s, programmatic, d->q, kc, vc, d->att_part, d->pos, heads,
+                          kv_heads, d->splits, scale, pos_step, tok_stride);
+    }
+    return launch_pdl(attention_partial_kernel, dim3(heads, splits_now, T), dim3(ATT_THREADS), 0, s, programmatic, d->q, kc, vc, d->att_part, d->pos, heads, kv_heads,
+                      d->head_dim, d->splits, scale, pos_step, tok_stride);
+}
+
 // Enqueues the forward of T tokens on s. Tokens and position come either from kernel arguments (ta != nullptr) or, for
 // the captured single-token graph, from the pinned staging words through a host-to-device copy.
 static int enqueue_forward(jq_decoder* d, int T, int max_keys, const TokenArgs* ta, cudaStream_t s) {
@@ -1415,9 +1558,8 @@ static int enqueue_forward(jq_decoder* d, int T, int max_keys, const TokenArgs* 
         LAUNCHED("rope_store_kernel");
         // only the key chunks that can hold a position of this call are launched (all of them inside the captured graph)
         const int splits_now = (max_keys + ATT_CHUNK - 1) / ATT_CHUNK;
-        if (rc == JQ_OK) pdl_err = launch_pdl(attention_partial_kernel, dim3(d->heads, splits_now, T), dim3(ATT_THREADS), 0, s, true, d->q, kc, vc, d->att_part, d->pos, d->heads, d->kv_heads, hd,
-                                                                                 d->splits, scale, pos_step, tok_stride);
-        LAUNCHED("attention_partial_kernel");
+        if (rc == JQ_OK) pdl_err = launch_attention(d, d->heads, d->kv_heads, T, splits_now, kc, vc, scale, pos_step, tok_stride, true, s);
+        LAUNCHED("attention_group_kernel");
         if (rc == JQ_OK) pdl_err = launch_pdl(attention_combine_kernel, dim3(d->heads, T), dim3(hd < 128 ? hd : 128), 0, s, true, d->att_part, d->att, d->heads, hd, d->splits, splits_now);
         LAUNCHED("attention_combine_kernel");
         LIN(L[3], d->att, d->proj);
@@ -1441,8 +1583,9 @@ static int enqueue_forward(jq_decoder* d, int T, int max_keys, const TokenArgs* 
         LIN(d->output, d->xn, d->logits);
     }
     if (rc == JQ_OK) {
-        if (rc == JQ_OK) pdl_err = launch_pdl(argmax_kernel, dim3(T), dim3(1024), 0, s, true, d->logits, d->argmax, d->vocab);
-        LAUNCHED("argmax_kernel");
+        if (rc == JQ_OK) pdl_err = launch_pdl(argmax_split_kernel, dim3(ARGMAX_CTAS, T), dim3(256), 0, s, true, d->logits, d->vocab, d->argmax_v, d->argmax_i,
+                                               d->counters + d->dim / 256 + 1, d->argmax);
+        LAUNCHED("argmax_split_kernel");
     }
     return rc;
 }
@@ -1594,9 +1737,11 @@ static int enqueue_forward_sharded(jq_decoder* d, int T, int max_keys, const Tok
             rope_store_kernel<<<dim3(T, heads + 2 * kv_heads), hd / 2, 0, s>>>(d->q, d->k, d->v, kc, vc, d->cos_t, d->sin_t, d->pos, heads, kv_heads, hd, pos_step,
                                                                                tok_stride);
             LAUNCHED("rope_store_kernel");
-            attention_partial_kernel<<<dim3(heads, splits_now, T), ATT_THREADS, 0, s>>>(d->q, kc, vc, d->att_part, d->pos, heads, kv_heads, hd, d->splits,
-                                                                                  scale, pos_step, tok_stride);
-            LAUNCHED("attention_partial_kernel");
+            if (rc == JQ_OK) {
+                const cudaError_t e = launch_attention(d, heads, kv_heads, T, splits_now, kc, vc, scale, pos_step, tok_stride, false, s);
+                if (e != cudaSuccess) rc = cuda_fail(e, "attention_group_kernel");
+            }
+            LAUNCHED("attention_group_kernel");
             attention_combine_kernel<<<dim3(heads, T), hd < 128 ? hd : 128, 0, s>>>(d->att_part, d->att, heads, hd, d->splits, splits_now);
             LAUNCHED("attention_combine_kernel");
             GATHER(d->att, dim, dim_l, 0);
@@ -1636,8 +1781,8 @@ static int enqueue_forward_sharded(jq_decoder* d, int T, int max_keys, const Tok
         PEER_LIN(d->output, d->xn, d->vocab, vocab_l, 4);
     }
     if (rc == JQ_OK) {
-        argmax_kernel<<<T, 1024, 0, s>>>(E, d->argmax, d->vocab);
-        LAUNCHED("argmax_kernel");
+        argmax_split_kernel<<<dim3(ARGMAX_CTAS, T), 256, 0, s>>>(E, d->vocab, d->argmax_v, d->argmax_i, d->counters + d->dim / 256 + 1, d->argmax);
+        LAUNCHED("argmax_split_kernel");
     }
     return rc;
 }
@@ -1684,10 +1829,7 @@ static int decoder_forward(jq_decoder* d, int seq, bool batch, const int32_t* to
     d->cur_batch = batch && T > 1;  // a batch of one is the single-token step of sequence 0
     if (decode_step && (d->graph_T != T || d->graph_seq != (d->cur_batch ? -1 : d->cur_seq))) {
         // another kind of step than the one counted (and perhaps captured) so far
-        if (d->graph != nullptr) {
-            cudaGraphExecDestroy(d->graph);
-            d->graph = nullptr;
-        }
+        drop_graphs(d);
         d->warm_calls = 0;
         d->graph_T = T;
         d->graph_seq = d->cur_batch ? -1 : d->cur_seq;
@@ -1703,25 +1845,31 @@ static int decoder_forward(jq_decoder* d, int seq, bool batch, const int32_t* to
             d->host_stage[i] = tokens_host[i];
         }
         d->host_stage[MAX_TOKENS] = pos0;
-        if (d->graph == nullptr) {
+        // the launches of a captured step cover a fixed number of key chunks: the smallest power of two that reaches this position
+        int bucket = 0;
+        while (bucket < GRAPHS - 1 && (256 << bucket) < pos0 + 1) {
+            bucket++;
+        }
+        cudaGraphExec_t& graph = d->graphs[bucket];
+        if (graph == nullptr) {
             cudaGraph_t g = nullptr;
             CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
             if (rc == JQ_OK) {
-                rc = enqueue_forward(d, T, d->max_seq, nullptr, s);
+                rc = enqueue_forward(d, T, (256 << bucket) < d->max_seq ? 256 << bucket : d->max_seq, nullptr, s);
                 cudaError_t e = cudaMemcpyAsync(d->host_stage + MAX_TOKENS + 1, d->argmax, T * sizeof(int), cudaMemcpyDeviceToHost, s);
                 cudaError_t e2 = cudaStreamEndCapture(s, &g);
                 CK(e, "argmax copy");
                 CK(e2, "cudaStreamEndCapture");
             }
             if (rc == JQ_OK) {
-                CK(cudaGraphInstantiate(&d->graph, g, 0), "cudaGraphInstantiate");
+                CK(cudaGraphInstantiate(&graph, g, 0), "cudaGraphInstantiate");
             }
             if (g != nullptr) {
                 cudaGraphDestroy(g);
             }
         }
         if (rc == JQ_OK) {
-            CK(cudaGraphLaunch(d->graph, s), "cudaGraphLaunch");
+            CK(cudaGraphLaunch(graph, s), "cudaGraphLaunch");
         }
     } else {
         TokenArgs ta;
@@ -1973,10 +2121,7 @@ JQ_API int jq_decoder_set_sequences(jq_decoder* d, int sequences) {
     cudaGetDevice(&prev);
     JQ_CUDA(cudaSetDevice(d->device));
     JQ_CUDA(cudaDeviceSynchronize());
-    if (d->graph != nullptr) {
-        cudaGraphExecDestroy(d->graph);  // the captured step holds the old cache addresses
-        d->graph = nullptr;
-    }
+    drop_graphs(d);  // the captured step holds the old cache addresses
     d->warm_calls = 0;
     d->graph_T = 0;
     const size_t elems = (size_t)sequences * d->layers * d->max_seq * d->kv_heads * d->head_dim;

@@ -92,7 +92,7 @@ int launch_gemv(const View& v, const float* x, int rows, const float* bias, floa
     if (v.n == 0) {
         return JQ_OK;
     }
-    if (gemv_umma_takes(v.type, v.k, rows, v.n)) {
+    if (gemv_umma_takes(v.type, v.k, rows)) {
         // Q4_K, Q5_K: the tcgen05 kernel, one pass over the weights for up to 16 rows
         uint8_t* image = nullptr;
         int rc = scratch_for(s, gemv_umma_image_bytes(v.k, rows), &image);

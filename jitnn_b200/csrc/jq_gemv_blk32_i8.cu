@@ -378,16 +378,24 @@ int sm_count() {
     return g_sms;
 }
 
+constexpr int stages_of(int type) { return type == JQ_TYPE_Q8_0 ? 2 : 3; }
+template <int TYPE, int MT>
+size_t smem_bytes(int KB) {
+    return (size_t)KB * Img<MT>::PB + (size_t)(2 * NW * 16 * MT) * sizeof(float) + (size_t)NW * stages_of(TYPE) * Geo<TYPE>::SLOT;
+}
+template <int TYPE>
+bool image_fits(int64_t k, int rows) {
+    return (rows == 1 ? smem_bytes<TYPE, 1>((int)(k / 256)) : smem_bytes<TYPE, 2>((int)(k / 256))) <= SMEM_MAX;
+}
+
 template <int TYPE, int MT>
 int run(const View& v, const float* x, int rows, const float* bias, float* y, cudaStream_t s, uint8_t* image, bool* handled) {
-    constexpr int STAGES = TYPE == JQ_TYPE_Q8_0 ? 2 : 3;
+    constexpr int STAGES = stages_of(TYPE);
     const int KB = (int)(v.k / 256);
     const int tiles = (int)((v.n + 15) / 16);
-    const size_t smem = (size_t)KB * Img<MT>::PB + (size_t)(2 * NW * 16 * MT) * sizeof(float) + (size_t)NW * STAGES * Geo<TYPE>::SLOT;
-    if (smem > SMEM_MAX / 2 - 1024) {
-        *handled = false;  // the image of the whole k does not fit beside the ring
-        return JQ_OK;
-    }
+    const size_t smem = smem_bytes<TYPE, MT>(KB);
+    // two CTAs per SM, or one where the image of the whole k leaves no room for two (Q8_0, one row of x: from k = 11008 on)
+    const int per_sm = smem > SMEM_MAX / 2 - 1024 ? 1 : 2;
     *handled = true;
     static std::atomic<uint64_t> configured{0};  // the opt-in for large dynamic shared memory is per device
     int dev = 0;
@@ -409,7 +417,7 @@ int run(const View& v, const float* x, int rows, const float* bias, float* y, cu
     icfg.blockDim = dim3(PREP_WARPS * 32);
     JQ_CUDA(cudaLaunchKernelEx(&icfg, blk32_image_kernel<MT>, x, rows, (int64_t)v.k, image));
     count_launch();
-    const int grid = tiles < sm_count() * 2 ? tiles : sm_count() * 2;
+    const int grid = tiles < sm_count() * per_sm ? tiles : sm_count() * per_sm;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(THREADS);
@@ -436,6 +444,9 @@ int by_rows(const View& v, const float* x, int rows, const float* bias, float* y
 // Bytes of scratch (activation image) the kernel needs; 0 if the shape is not handled.
 size_t gemv_blk32_i8_scratch_bytes(int type, int64_t k, int rows) {
     if ((type != JQ_TYPE_Q8_0 && type != JQ_TYPE_Q4_0 && type != JQ_TYPE_Q4_1) || rows < 1 || rows > 2 || k <= 0 || k % 256 != 0) {
+        return 0;
+    }
+    if (!(type == JQ_TYPE_Q8_0 ? image_fits<JQ_TYPE_Q8_0>(k, rows) : (type == JQ_TYPE_Q4_0 ? image_fits<JQ_TYPE_Q4_0>(k, rows) : image_fits<JQ_TYPE_Q4_1>(k, rows)))) {
         return 0;
     }
     return (size_t)(k / 256) * (rows == 1 ? Img<1>::PB : Img<2>::PB);

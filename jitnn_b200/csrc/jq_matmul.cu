@@ -15,8 +15,8 @@ namespace mm {
 // two that brings the largest to [2^9, 2^10), hi = that rounded to half precision, lo = the rest rounded to half precision: 22
 // significant bits for everything down to 2^-13 of the largest. A block that holds a NaN or an Inf gets the scale NaN, which reaches
 // every output of that row. One warp per 256 values of a row; memory bound (8 bytes moved per value, 4 of them to L2).
-// EXT: 64 more columns follow every 256, of which the first 16 hold the sums over the eight runs of 32 values, twice (hi plane: their
-// hi parts, lo plane: their lo parts); the others are never used.
+// EXT: 16 more columns follow every 256, the sums over the eight runs of 32 values, twice (hi plane: their hi parts, lo plane: their lo
+// parts).
 template <int BLK, bool EXT>
 __global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ x, int m, int64_t k, int per_row, uint4* __restrict__ planes,
                                                     float* __restrict__ scales, int stride, int vec) {
@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ x,
     for (int i = 0; i < 4; i++) {
         split_pair(v[2 * i] * f, v[2 * i + 1] * f, hi[i], lo[i]);
     }
-    constexpr int BLOCK = EXT ? 320 : 256;
+    constexpr int BLOCK = EXT ? 272 : 256;
     const int64_t row_at = ((int64_t)row * per_row + b) * BLOCK, at = (row_at >> 3) + lane, plane = ((int64_t)m * per_row * BLOCK) >> 3;
     planes[at] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
     planes[at + plane] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
@@ -103,54 +103,64 @@ static int status_word(int** out) {
 
 static int unit_bytes(int type) { return TILE_ROWS * (plane_q_bytes(type) + plane_aux_bytes(type)) * 256 / block_values(type); }
 
-// Ring depths: at least as many weight operands as there are groups of dequantiser warps, two activation tiles and two raw units; then the
-// activations' ring grows first. False if not even those fit.
-static bool rings(int type, bool fp32, bool bwd, int nt, int groups, Args& a, Plan& plan) {
-    const int at = a_bytes(bwd), bt = b_bytes(fp32, nt), rb = unit_bytes(type), room = 227 * 1024 - 1024 - TAIL_BYTES;
-    // weight operands: backward at most four, for the fold's ring of factors; forward what tensor memory holds behind one accumulator, or two
-    // where they fit beside the groups' operands
-    int max_a = 4;
-    if (!bwd) {
-        const int cols = ((plan.narrow ? 2 * nt : nt) + 31) / 32 * 32, per = a_columns(type, fp32, false);
-        const int bufs = 2 * cols + groups * per <= 512 ? 2 : 1;
-        max_a = (512 - bufs * cols) / per;
-        max_a = max_a > MAX_A ? MAX_A : max_a;
+static Facts facts(int type, bool fp32, bool bwd, int nmax) {
+    switch (type) {
+        case JQ_TYPE_Q4_K: return facts_format<JQ_TYPE_Q4_K>(fp32, bwd, nmax);
+        case JQ_TYPE_Q5_K: return facts_format<JQ_TYPE_Q5_K>(fp32, bwd, nmax);
+        case JQ_TYPE_Q6_K: return facts_format<JQ_TYPE_Q6_K>(fp32, bwd, nmax);
+        case JQ_TYPE_Q8_0: return facts_format<JQ_TYPE_Q8_0>(fp32, bwd, nmax);
+        case JQ_TYPE_Q4_0: return facts_format<JQ_TYPE_Q4_0>(fp32, bwd, nmax);
+        default: return facts_format<JQ_TYPE_Q4_1>(fp32, bwd, nmax);
     }
-    a.sa = bwd ? groups : max_a;
-    a.sb = 2;
-    a.raw = 2;
-    int left = room - a.sa * at - a.sb * bt - a.raw * rb;
-    if (left < 0) {
-        return false;
-    }
-    auto grow = [&](int& depth, int most, int bytes) {
-        while (depth < most && left >= bytes) {
-            depth++;
-            left -= bytes;
-        }
-    };
-    grow(a.sb, bwd ? 3 : 6, bt);
-    if (at > 0) {
-        grow(a.sa, max_a, at);
-    }
-    grow(a.raw, 3, rb);
-    grow(a.sb, MAX_B, bt);
-    grow(a.raw, MAX_RAW, rb);
-    plan.smem = (size_t)(room - left) + TAIL_BYTES + 1024;
-    return true;
 }
 
-// A tile width: the instance that can run it and its rings.
-static bool configure(int type, bool fp32, bool bwd, int nt, Args& a, Plan& plan) {
+// Ring depths for a tile of nt rows of x: at least as many weight operands as there are groups of dequantiser warps, two activation entries and
+// two raw units (or one per group); then the activations' ring grows first. False if not even those fit.
+static bool configure(int type, bool fp32, bool bwd, int nt, int ksplit, Args& a, Plan& plan) {
     plan.fp32 = fp32;
     plan.bwd = bwd;
-    plan.narrow = fp32 && nt <= 32;
+    plan.nmax = !fp32 ? (nt <= 128 ? 128 : 256) : (nt <= 16 && !bwd ? 16 : (nt <= 32 ? 32 : 128));
     a.nt = nt;
-    if (plan.narrow && rings(type, fp32, bwd, nt, Warps<true, 32>::GROUPS, a, plan)) {
-        return true;
+    a.ksplit = ksplit;
+    const Facts f = facts(type, fp32, bwd, plan.nmax);
+    // sums of a CTA's virtual ranges (instances for 16 rows of x), kept apart from the rings, which are still in use
+    a.part_bytes = fp32 && !bwd && nt <= 16 && ksplit > 1 ? VIRTUAL / ksplit * nt * 512 : 0;
+    const int at = a_bytes(bwd), bt = f.b_tiles * tile_bytes(fp32, nt), rb = unit_bytes(type), room = 227 * 1024 - 1024 - TAIL_BYTES - a.part_bytes;
+    // tensor memory: two accumulators where they fit beside the groups' operands, else one; operands behind them
+    a.cols = (f.columns * nt + 31) / 32 * 32;
+    a.bufs = 2 * a.cols + f.groups * f.a_cols <= 512 ? 2 : 1;
+    int max_a = 4;
+    if (!bwd) {
+        max_a = (512 - a.bufs * a.cols) / f.a_cols;
+        max_a = max_a > MAX_A ? MAX_A : max_a;
     }
-    plan.narrow = false;
-    return rings(type, fp32, bwd, nt, fp32 ? Warps<true, 128>::GROUPS : Warps<false, 16>::GROUPS, a, plan);
+    const int raw_step = f.owned ? f.groups : 1;
+    a.sa = bwd ? f.groups : max_a;
+    a.sb = 2;
+    a.raw = f.owned ? f.groups : 2;
+    int left = room - a.sa * at - a.sb * bt - a.raw * rb;
+    if (left < 0 || a.sa < f.groups) {
+        return false;
+    }
+    auto grow = [&](int& depth, int most, int bytes, int step) {
+        while (depth + step <= most && left >= bytes * step) {
+            depth += step;
+            left -= bytes * step;
+        }
+    };
+    grow(a.sb, bwd ? 3 : (f.b_tiles > 1 ? 3 : 6), bt, 1);
+    if (at > 0) {
+        grow(a.sa, max_a, at, 1);
+    }
+    grow(a.raw, f.owned ? MAX_RAW : 3, rb, raw_step);
+    grow(a.sb, f.b_tiles > 1 ? 6 : MAX_B, bt, 1);
+    grow(a.raw, f.owned ? MAX_RAW : 4, rb, raw_step);
+    a.tmem = 32;
+    while (a.tmem < a.bufs * a.cols + (bwd ? 0 : a.sa * f.a_cols)) {
+        a.tmem *= 2;
+    }
+    plan.smem = (size_t)(room - left) + a.part_bytes + TAIL_BYTES + 1024;
+    return true;
 }
 
 // What one unit of the contraction takes a CTA in nanoseconds, by the tile's width (measured on long contractions): the dequantiser warps and
@@ -160,11 +170,12 @@ static double unit_ns(int type, bool fp32, bool bwd, int nt) {
         return nt < 64 ? 940.0 : 430.0 + 7.9 * nt;
     }
     if (!fp32) {
-        const double t = 6.4 * ((nt + 63) / 64 * 64);  // (a tile of 208 or 240 is no faster than one of 256)
-        return t < 1200.0 ? 1200.0 : t;
+        return nt <= 128 ? 950.0 : 350.0 + 4.5 * ((nt + 63) / 64 * 64);  // (a tile of 208 or 240 is no faster than one of 256)
     }
-    const bool one_part = type == JQ_TYPE_Q4_K || type == JQ_TYPE_Q5_K;
-    const double t = one_part ? 450.0 + 9.9 * nt : 300.0 + 14.7 * nt;
+    if (nt <= 32) {
+        return one_part(type) ? (nt <= 16 ? 830.0 : 1060.0) : 1300.0;
+    }
+    const double t = one_part(type) ? 450.0 + 9.9 * nt : 300.0 + 14.7 * nt;
     return t < 1320.0 ? 1320.0 : t;
 }
 
@@ -177,7 +188,7 @@ static void choose(int type, bool fp32, bool bwd, int64_t features, int units, i
     int last_nt = 0;
     for (int tt = (m + nmax - 1) / nmax; tt <= (m + nmax - 1) / nmax + 6; tt++) {
         const int nt = ((m + tt - 1) / tt + 15) / 16 * 16;
-        if (nt == last_nt || !configure(type, fp32, bwd, nt, a, plan)) {
+        if (nt == last_nt) {
             continue;
         }
         last_nt = nt;
@@ -191,6 +202,9 @@ static void choose(int type, bool fp32, bool bwd, int64_t features, int units, i
             if (ks > 1 && tiles > slots) {
                 break;  // more than one wave of whole tiles: nothing to gain
             }
+            if (!configure(type, fp32, bwd, nt, ks, a, plan)) {
+                continue;
+            }
             const double waves = (double)((tiles + slots - 1) / slots);
             const double cost = waves * (((units + ks - 1) / ks) * unit + 1500.0 + 12.0 * nt) + (ks > 1 ? 1500.0 + 6.0 * nt : 0.0);
             if (cost < best) {
@@ -200,21 +214,13 @@ static void choose(int type, bool fp32, bool bwd, int64_t features, int units, i
             }
         }
     }
-    configure(type, fp32, bwd, best_nt, a, plan);
-    a.ksplit = best_ks;
+    configure(type, fp32, bwd, best_nt, best_ks, a, plan);
     a.ftiles = (int)ftiles;
     a.ttiles = (m + best_nt - 1) / best_nt;
     const int tiles = a.ftiles * a.ttiles;
     plan.ctas = best_ks > 1 || tiles < 148 ? tiles * best_ks : 148;
     a.units = units;
     a.m = m;
-    a.cols = ((plan.narrow ? 2 * a.nt : a.nt) + 31) / 32 * 32;
-    const int ring = a.sa * a_columns(type, fp32, bwd);
-    a.bufs = 2 * a.cols + ring <= 512 ? 2 : 1;
-    a.tmem = 32;
-    while (a.tmem < a.bufs * a.cols + ring) {
-        a.tmem *= 2;
-    }
 }
 
 static int launch_any(int type, const Plan& plan, const Args& args, const CUtensorMap& map, cudaStream_t s) {
@@ -237,7 +243,7 @@ static int activation_map(CUtensorMap* map, bool bf16, const void* x, int64_t wi
     }
     const cuuint64_t dims[3] = {(cuuint64_t)width, (cuuint64_t)rows, (cuuint64_t)planes};
     const cuuint64_t strides[2] = {(cuuint64_t)width * 2, (cuuint64_t)width * 2 * (cuuint64_t)rows};
-    const cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
+    const cuuint32_t box[3] = {64, (cuuint32_t)box_rows, (cuuint32_t)planes};
     const cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = enc(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(x), dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -251,57 +257,69 @@ static void weight_args(const View& v, Args& a) {
     a.rows128 = (int)(tiled_rows(v.n) / TILE_ROWS);
 }
 
-constexpr int SPLIT_SLOT = 6;  // scratch slot of the split activations
+constexpr int SPLIT_SLOT = 6;  // scratch slots 6 and 7: split activations without and with the 16 more columns
 
-// out [m, features] = the FP32 product in either direction; x has `width` values per row.
-static int product_f32(const View& v, bool bwd, const float* x, int64_t m, const float* bias, float* out, cudaStream_t s) {
-    const int64_t width = bwd ? v.n : v.k, features = bwd ? v.k : v.n;
-    const int per_row = (int)((width + 255) / 256);
-    const bool ext = unit_stages(v.type, true, bwd) == 5;
-    const int64_t wpad = (int64_t)per_row * (ext ? 320 : 256);
+// ys[i] [m, features_i] = the FP32 products of `count` weights with the same x (backward: one weight); x has `width` values per row.
+static int product_f32(const View* vs, int count, bool bwd, const float* x, int64_t m, const float* bias, float* const* ys, cudaStream_t s) {
+    const int64_t width = bwd ? vs[0].n : vs[0].k;
+    const int per_row = (int)((width + 255) / 256), blk = bwd ? 128 : 256;
     constexpr int64_t GROUP = 4096;  // rows at a time: bounds the scratch
     int* status = nullptr;
     int rc = status_word(&status);
     for (int64_t m0 = 0; m0 < m && rc == JQ_OK; m0 += GROUP) {
         const int rows = (int)(m - m0 < GROUP ? m - m0 : GROUP);
-        Args a = {};
-        Plan plan = {};
-        weight_args(v, a);
-        choose(v.type, true, bwd, features, bwd ? a.rows128 : a.kb, rows, a, plan);
-        const int stride = a.ttiles * a.nt, blk = bwd ? 128 : 256;
-        const size_t plane_bytes = (size_t)2 * rows * wpad * 2;
-        uint8_t* scratch = nullptr;
-        rc = scratch_for_slot(s, SPLIT_SLOT, plane_bytes + (size_t)(per_row * 256 / blk) * stride * sizeof(float), &scratch);
-        if (rc != JQ_OK) {
-            break;
-        }
-        float* scales = reinterpret_cast<float*>(scratch + plane_bytes);
+        const int stride = (rows + 128 + 15) / 16 * 16;  // tiles of rows reach at most this far
         const float* xg = x + m0 * width;
         const int vec = width % 4 == 0 && ((uintptr_t)xg & 15) == 0;
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        cfg.stream = s;
-        cfg.gridDim = dim3((unsigned)(((int64_t)rows * per_row + 7) / 8));
-        cfg.blockDim = dim3(256);
-        auto split = bwd ? split_kernel<128, false> : (ext ? split_kernel<256, true> : split_kernel<256, false>);
-        JQ_CUDA(cudaLaunchKernelEx(&cfg, split, xg, rows, width, per_row, reinterpret_cast<uint4*>(scratch), scales, stride, vec));
-        count_launch();
-        CUtensorMap map;
-        rc = activation_map(&map, false, scratch, wpad, rows, 2, a.nt);
-        if (rc != JQ_OK) {
-            break;
+        // weights with the 16 more columns per unit and weights without: one split each
+        for (int ext = 0; ext < 2 && rc == JQ_OK; ext++) {
+            const int64_t wpad = (int64_t)per_row * (ext ? 272 : 256);
+            const size_t plane_bytes = (size_t)2 * rows * wpad * 2;
+            uint8_t* scratch = nullptr;
+            float* scales = nullptr;
+            for (int i = 0; i < count && rc == JQ_OK; i++) {
+                const View& v = vs[i];
+                if (facts(v.type, true, bwd, 16).ext != (ext != 0)) {
+                    continue;
+                }
+                if (scratch == nullptr) {
+                    rc = scratch_for_slot(s, SPLIT_SLOT + ext, plane_bytes + (size_t)(per_row * 256 / blk) * stride * sizeof(float), &scratch);
+                    if (rc != JQ_OK) {
+                        break;
+                    }
+                    scales = reinterpret_cast<float*>(scratch + plane_bytes);
+                    cudaLaunchConfig_t cfg = {};
+                    cudaLaunchAttribute attr[1];
+                    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+                    attr[0].val.programmaticStreamSerializationAllowed = 1;
+                    cfg.attrs = attr;
+                    cfg.numAttrs = 1;
+                    cfg.stream = s;
+                    cfg.gridDim = dim3((unsigned)(((int64_t)rows * per_row + 7) / 8));
+                    cfg.blockDim = dim3(256);
+                    auto split = bwd ? split_kernel<128, false> : (ext ? split_kernel<256, true> : split_kernel<256, false>);
+                    JQ_CUDA(cudaLaunchKernelEx(&cfg, split, xg, rows, width, per_row, reinterpret_cast<uint4*>(scratch), scales, stride, vec));
+                    count_launch();
+                }
+                const int64_t features = bwd ? v.k : v.n;
+                Args a = {};
+                Plan plan = {};
+                weight_args(v, a);
+                choose(v.type, true, bwd, features, bwd ? a.rows128 : a.kb, rows, a, plan);
+                CUtensorMap map;
+                rc = activation_map(&map, false, scratch, wpad, rows, 2, a.nt);
+                if (rc != JQ_OK) {
+                    break;
+                }
+                a.features = features;
+                a.xscale = scales;
+                a.xstride = stride;
+                a.bias = bias;
+                a.y = ys[i] + m0 * features;
+                a.status = status;
+                rc = launch_any(v.type, plan, a, map, s);
+            }
         }
-        a.features = features;
-        a.xscale = scales;
-        a.xstride = stride;
-        a.bias = bias;
-        a.y = out + m0 * features;
-        a.status = status;
-        rc = launch_any(v.type, plan, a, map, s);
     }
     return rc;
 }
@@ -309,11 +327,36 @@ static int product_f32(const View& v, bool bwd, const float* x, int64_t m, const
 }  // namespace mm
 
 int launch_matmul_f32(const View& v, const float* x, int64_t m, const float* bias, float* y, cudaStream_t s) {
-    return mm::product_f32(v, false, x, m, bias, y, s);
+    return mm::product_f32(&v, 1, false, x, m, bias, &y, s);
+}
+
+int launch_matmul_f32_multi(const View* vs, int count, const float* x, int64_t m, float* const* ys, cudaStream_t s) {
+    return mm::product_f32(vs, count, false, x, m, nullptr, ys, s);
+}
+
+// More than 16 rows of x always: the weight is read once for all of them. Up to 16 rows take the same time as one (Q4_K 32000 x 4096: 27 us,
+// Q6_K 41, 4096 x 4096: 11), so the line lies where the decode kernels need another pass: Q4_K and Q5_K take up to eight rows in one
+// (25 us), Q6_K four (35), the 32-element formats two (24 and 16). It does not depend on the number of output rows, and neither do
+// the sums, so a row shard gives bitwise the outputs of the whole weight. Where k is no multiple of 256 there is only the CUDA-core
+// kernel besides, which is the faster one up to about eight million products (4096 x 1056, one row: 4.5 us against 8.9).
+bool matmul_takes(const View& v, int64_t rows) {
+    if (rows > 16) {
+        return true;
+    }
+    if (v.type == JQ_TYPE_Q4_K || v.type == JQ_TYPE_Q5_K) {
+        return rows >= (v.k <= 1024 ? 12 : 9);
+    }
+    if (v.type == JQ_TYPE_Q6_K) {
+        return rows >= 5;
+    }
+    if (gemv_blk32_i8_scratch_bytes(v.type, v.k, rows < 2 ? 1 : 2) > 0) {
+        return rows >= 5;
+    }
+    return rows * v.n * v.k > 8000000;
 }
 
 // gx [m, k] = g [m, n] . dequant(W) (ops/Gguf.java:208-212, ops/Quant.java:191-197); device pointers; n >= 1, m >= 1.
-int launch_linear_backward(const View& v, const float* g, int64_t m, float* gx, cudaStream_t s) { return mm::product_f32(v, true, g, m, nullptr, gx, s); }
+int launch_linear_backward(const View& v, const float* g, int64_t m, float* gx, cudaStream_t s) { return mm::product_f32(&v, 1, true, g, m, nullptr, &gx, s); }
 
 bool prefill_supported(const View& v) { return has_linear_kernel(v.type) && v.k % 64 == 0 && v.n > 0 && v.k > 0; }
 

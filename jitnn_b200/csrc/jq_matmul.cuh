@@ -38,15 +38,30 @@
 namespace jq {
 namespace mm {
 
-// Four groups of dequantiser warps where the registers allow it (80 a thread with 23 warps); the FP32 kernel for more than 32 rows of x adds up
-// 64 columns per thread and has two.
-template <bool FP32, int NMAX>
-struct Warps {
-    static constexpr int GROUPS = FP32 && NMAX > 32 ? 2 : 4, FOLD = FP32 && NMAX > 32 ? 8 : 4, THREADS = (3 + 4 * GROUPS + FOLD) * 32;
+// How an instance splits its work. TURN: chunks of 64 k that a group of dequantiser warps makes at a time, one operand in tensor memory; what a
+// turn costs besides its instructions (barrier round trips, stores' completion) is several hundred clocks, so longer turns pay wherever
+// tensor memory holds an operand for every group beside the accumulator. JOINED: x's hi and lo rows are one operand of 2 nt columns
+// (fewer of the small MMAs, whose issue would bound), and an operand's activation tiles arrive together.
+// The FP32 instance for more than 32 rows of x adds up 64 columns per thread and has registers for two groups only.
+__host__ __device__ constexpr bool one_part(int type) { return type == JQ_TYPE_Q4_K || type == JQ_TYPE_Q5_K; }
+template <int TYPE, bool FP32, bool BWD, int NMAX>
+struct Shape {
+    static constexpr bool JOINED = FP32 && NMAX <= 32;
+    static constexpr int TURN = BWD ? 1 : (!FP32 ? (NMAX <= 128 ? 4 : 1) : (!JOINED ? (one_part(TYPE) ? 2 : 1) : (NMAX <= 16 && one_part(TYPE) ? 4 : 2)));
+    static constexpr int GROUPS = FP32 && !JOINED ? 2 : (BWD || (!FP32 && NMAX > 128) ? 4 : 3), FOLD = FP32 && !JOINED ? 8 : 4, THREADS = (3 + 4 * GROUPS + FOLD) * 32;
+    static constexpr int CHUNKS = BWD ? 2 : 4;                           // chunks of 64 of the contraction in a unit
+    static constexpr int TURNS = CHUNKS / TURN;
+    static constexpr bool EXT = FP32 && !BWD && (one_part(TYPE) || TYPE == JQ_TYPE_Q4_1);  // 16 more columns of the contraction per unit
+    static constexpr int PARTS = FP32 && !BWD && !one_part(TYPE) ? 2 : 1;                    // operand columns per value
+    static constexpr int A_COLS = BWD ? 0 : 32 * PARTS * TURN + (EXT ? 8 : 0);              // tensor-memory columns of an operand
+    static constexpr int B_TILES = JOINED && !BWD ? TURN + (EXT ? 1 : 0) : 1;               // activation tiles of 64 that arrive together
+    static constexpr bool OWNED = TURNS == 1;                           // a raw unit is one group's own
 };
 constexpr int A_TILE = 128 * 128;  // 128 rows of 128 bytes
 constexpr long long WAIT_CLOCKS = 4000000000ll;  // about two seconds
-constexpr int MAX_A = 6, MAX_B = 12, MAX_RAW = 4;
+constexpr int MAX_A = 6, MAX_B = 12, MAX_RAW = 6;
+constexpr int FACTORS = 8;   // units whose factors the fold may still need: operands in flight and accumulators, see where they are written
+constexpr int VIRTUAL = 8;   // ranges of the contraction whose sums are added up in order, whatever the cluster (instances for 16 rows of x)
 
 struct Args {
     const uint8_t* q;
@@ -58,6 +73,7 @@ struct Args {
     int ttiles, nt;   // tiles of nt rows of x
     int m;
     int ksplit;
+    int part_bytes;   // shared memory for the sums of this CTA's virtual ranges
     int sa, sb, raw;  // ring depths: weight operands, activation tiles, raw units
     int cols;         // tensor-memory columns of one accumulator
     int bufs;         // accumulators: 2, or 1 where a second one does not fit
@@ -223,40 +239,31 @@ __host__ __device__ constexpr int raw_bytes() {
     return Dq<TYPE>::UNIT_Q + Dq<TYPE>::UNIT_A;
 }
 __host__ __device__ inline int a_bytes(bool bwd) { return bwd ? 2 * A_TILE : 0; }  // the forward product's weights go to tensor memory
-// tensor-memory columns of a stage's weights, and stages of 64 per unit of the contraction
-__host__ __device__ constexpr int a_columns(int type, bool fp32, bool bwd) {
-    return bwd ? 0 : (fp32 && type != JQ_TYPE_Q4_K && type != JQ_TYPE_Q5_K ? 64 : 32);
-}
-__host__ __device__ constexpr int unit_stages(int type, bool fp32, bool bwd) {
-    return bwd ? 2 : (fp32 && (type == JQ_TYPE_Q4_K || type == JQ_TYPE_Q5_K || type == JQ_TYPE_Q4_1) ? 5 : 4);
-}
-__host__ __device__ inline int b_bytes(bool fp32, int nt) { return (fp32 ? 2 * nt : nt) * 128; }
-constexpr int TAIL_BYTES = 4 * 128 * 4 + 8 * 2 * 64 * 4 + 768;  // row factors, the fold warps' scales, barriers
+__host__ __device__ inline int tile_bytes(bool fp32, int nt) { return (fp32 ? 2 * nt : nt) * 128; }
+constexpr int TAIL_BYTES = FACTORS * 128 * 4 + 8 * 2 * 64 * 4 + 1024;  // row factors, the fold warps' scales, barriers
 
 // NMAX: largest tile of rows of x an FP32 instance adds up in registers.
 template <int TYPE, bool FP32, bool BWD, int NMAX>
-__global__ void __launch_bounds__(Warps<FP32, NMAX>::THREADS, 1) matmul_kernel(const __grid_constant__ Args p, const __grid_constant__ CUtensorMap xmap) {
+__global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) matmul_kernel(const __grid_constant__ Args p, const __grid_constant__ CUtensorMap xmap) {
     using D = Dq<TYPE>;
-    using W = Warps<FP32, NMAX>;
+    using W = Shape<TYPE, FP32, BWD, NMAX>;
     using H = Half<TYPE>;
     static_assert(FP32 || !BWD, "the backward product is FP32");
-    constexpr bool HALF = FP32 && !BWD;                                 // weights by half arithmetic, see there
-    constexpr bool EXT = HALF && H::EXT;                                // a fifth stage with 16 more columns
-    constexpr int UNIT_STAGES = unit_stages(TYPE, FP32, BWD);           // stages of 64 per unit of the contraction
-    constexpr int A_COLS = a_columns(TYPE, FP32, BWD);
-    static_assert(BWD || A_COLS == (HALF ? 32 * H::TILES : 32), "");
-    static_assert(UNIT_STAGES == (BWD ? 2 : 4) + (EXT ? 1 : 0), "");
-    constexpr int G = W::GROUPS;
-    constexpr bool JOINED = FP32 && NMAX <= 32;  // x's hi and lo rows as one operand of 2 nt columns: fewer of the small MMAs, whose issue would bound
+    constexpr bool HALF = FP32 && !BWD;  // weights by half arithmetic, see there
+    constexpr bool EXT = W::EXT, JOINED = W::JOINED, OWNED = W::OWNED;
+    constexpr bool CANON = HALF && NMAX <= 16;  // sums depend on k alone, not on how many CTAs share it
+    constexpr int G = W::GROUPS, TURN = W::TURN, TURNS = W::TURNS, A_COLS = W::A_COLS, BT = W::B_TILES;
+    static_assert(!HALF || (W::PARTS == H::TILES && EXT == H::EXT), "");
+    constexpr int X_UNIT = BWD ? 128 : 256 + (EXT ? 16 : 0);  // columns of the activations per unit
     extern __shared__ uint8_t smem_unaligned[];
     const uint32_t base = (tc::smem_u32(smem_unaligned) + 1023u) & ~1023u;  // swizzled tiles start on 1024-byte boundaries
     const int SA = p.sa, SB = p.sb, R = p.raw, nt = p.nt;
-    const uint32_t a_st = (uint32_t)a_bytes(BWD), b_st = (uint32_t)b_bytes(FP32, nt);
-    const uint32_t a0 = base, b0 = a0 + (uint32_t)SA * a_st, raw0 = b0 + (uint32_t)SB * b_st;
+    const uint32_t tile_st = (uint32_t)tile_bytes(FP32, nt), a_st = (uint32_t)a_bytes(BWD), b_st = (uint32_t)BT * tile_st;
+    const uint32_t a0 = base + (uint32_t)p.part_bytes, b0 = a0 + (uint32_t)SA * a_st, raw0 = b0 + (uint32_t)SB * b_st;
     const uint32_t fac0 = raw0 + (uint32_t)R * raw_bytes<TYPE>();
-    const uint32_t scl0 = fac0 + 4 * 128 * 4, full_a = scl0 + 8 * 2 * 64 * 4, free_a = full_a + 8 * MAX_A, full_b = free_a + 8 * MAX_A, free_b = full_b + 8 * MAX_B;
+    const uint32_t scl0 = fac0 + FACTORS * 128 * 4, full_a = scl0 + 8 * 2 * 64 * 4, free_a = full_a + 8 * MAX_A, full_b = free_a + 8 * MAX_A, free_b = full_b + 8 * MAX_B;
     const uint32_t raw_full = free_b + 8 * MAX_B, raw_read = raw_full + 8 * MAX_RAW;
-    const uint32_t acc_full = raw_read + 8 * MAX_RAW, acc_empty = acc_full + 16, fac_full = acc_empty + 16, max_full = fac_full + 32, slot_s = max_full + 64;
+    const uint32_t acc_full = raw_read + 8 * MAX_RAW, acc_empty = acc_full + 16, fac_full = acc_empty + 16, max_full = fac_full + 8 * FACTORS, slot_s = max_full + 64;
     uint8_t* const generic = smem_unaligned + (slot_s - tc::smem_u32(smem_unaligned));
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(generic);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(generic + 4);
@@ -279,13 +286,13 @@ __global__ void __launch_bounds__(Warps<FP32, NMAX>::THREADS, 1) matmul_kernel(c
         }
         for (int r = 0; r < R; r++) {
             tc::mbar_init(raw_full + 8 * r, 1);
-            tc::mbar_init(raw_read + 8 * r, 4 * G);
+            tc::mbar_init(raw_read + 8 * r, OWNED ? 4 : 4 * G);
         }
         for (int i = 0; i < 2; i++) {
             tc::mbar_init(acc_full + 8 * i, 1);
             tc::mbar_init(acc_empty + 8 * i, W::FOLD);
         }
-        for (int i = 0; i < 4; i++) {
+        for (int i = 0; i < FACTORS; i++) {
             tc::mbar_init(fac_full + 8 * i, BWD ? 1 : 4);
         }
         for (int i = 0; i < 8; i++) {
@@ -317,19 +324,23 @@ __global__ void __launch_bounds__(Warps<FP32, NMAX>::THREADS, 1) matmul_kernel(c
             bool ok = true;
             for (int tile = cluster_id; tile < tiles && ok; tile += clusters) {
                 const int t0 = (tile % p.ttiles) * nt;
-                for (int it = u0 * UNIT_STAGES; it < u1 * UNIT_STAGES; it++) {
-                    if (!(ok = wait(free_b + 8 * s, ph, abort_flag, p.status, 3))) {
-                        break;
-                    }
-                    const uint32_t bar = full_b + 8 * s, dst = b0 + (uint32_t)s * b_st;
-                    tc::mbar_expect_tx(bar, b_st);
-                    tma_3d(dst, &xmap, bar, it * 64, t0, 0);
-                    if constexpr (FP32) {  // hi rows, then lo rows
-                        tma_3d(dst + (uint32_t)nt * 128, &xmap, bar, it * 64, t0, 1);
-                    }
-                    if (++s == SB) {
-                        s = 0;
-                        ph ^= 1;
+                for (int u = u0; u < u1 && ok; u++) {
+                    constexpr int ALL = W::CHUNKS + (EXT ? 1 : 0);  // tiles per unit; the last one is the 16 more columns
+                    for (int i = 0; i < ALL;) {
+                        const int last = BT > 1 ? (i + TURN == W::CHUNKS ? ALL : i + TURN) : i + 1;
+                        if (!(ok = wait(free_b + 8 * s, ph, abort_flag, p.status, 3))) {
+                            break;
+                        }
+                        const uint32_t bar = full_b + 8 * s;
+                        uint32_t dst = b0 + (uint32_t)s * b_st;
+                        tc::mbar_expect_tx(bar, (uint32_t)(last - i) * tile_st);
+                        for (; i < last; i++, dst += tile_st) {  // FP32: hi rows, then lo rows
+                            tma_3d(dst, &xmap, bar, u * X_UNIT + i * 64, t0, 0);
+                        }
+                        if (++s == SB) {
+                            s = 0;
+                            ph ^= 1;
+                        }
                     }
                 }
             }
@@ -345,76 +356,100 @@ __global__ void __launch_bounds__(Warps<FP32, NMAX>::THREADS, 1) matmul_kernel(c
         uint32_t ph = 0, phb = 0, aph = 0;
         bool ok = true, ready = false, ready_b = false;
         for (int tile = cluster_id; tile < tiles && ok; tile += clusters) {
-            uint32_t acc = 0;
+            bool first = true;
             for (int u = u0; u < u1 && ok; u++) {
                 const uint32_t d = tmem + (uint32_t)(buf * p.cols);
                 if (FP32 || u == u0) {
                     if (!(ok = wait_warp(acc_empty + 8 * buf, aph ^ 1u, abort_flag, p.status, 5))) {
                         break;
                     }
-                    acc = 0;
+                    first = true;
                 }
 #pragma unroll
-                for (int st = 0; st < UNIT_STAGES; st++) {
-                    ok = (__all_sync(0xffffffffu, ready) || wait_warp(full_a + 8 * s, ph, abort_flag, p.status, 2)) &&
-                         (__all_sync(0xffffffffu, ready_b) || wait_warp(full_b + 8 * sb, phb, abort_flag, p.status, 3));
+                for (int turn = 0; turn < TURNS; turn++) {
+                    if (!(ok = __all_sync(0xffffffffu, ready) || wait_warp(full_a + 8 * s, ph, abort_flag, p.status, 2))) {
+                        break;
+                    }
+                    // asked before this operand's MMAs are issued: the answer takes over a hundred clocks even when it is yes
+                    const int sn = s + 1 == SA ? 0 : s + 1;
+                    const uint32_t phn = sn == 0 ? ph ^ 1 : ph;
+                    ready = tc::mbar_test(full_a + 8 * sn, phn);
+                    constexpr int LAST = TURN + (EXT ? 1 : 0);
+#pragma unroll
+                    for (int c = 0; c < LAST; c++) {
+                        const bool ext = c == TURN;
+                        if (ext && turn < TURNS - 1) {
+                            break;
+                        }
+                        if (BT == 1 || c == 0) {
+                            if (!(ok = __all_sync(0xffffffffu, ready_b) || wait_warp(full_b + 8 * sb, phb, abort_flag, p.status, 3))) {
+                                break;
+                            }
+                            ready_b = tc::mbar_test(full_b + 8 * (sb + 1 == SB ? 0 : sb + 1), sb + 1 == SB ? phb ^ 1 : phb);
+                            tc::fence_after_sync();
+                        }
+                        // x: hi, lo; 16 of the contraction are 32 bytes
+                        const uint32_t bd = desc_k(b0 + (uint32_t)sb * b_st + (BT == 1 ? 0u : (uint32_t)c * tile_st)), bl = bd + lo_rows;
+                        const bool b_done = BT == 1 || c == LAST - 1 || (turn < TURNS - 1 && c == TURN - 1);
+                        const bool a_done = turn < TURNS - 1 ? c == TURN - 1 : c == LAST - 1;
+                        if (elect_one()) {
+                            const uint32_t acc = first ? 0u : 1u;
+                            if constexpr (BWD) {
+                                // feature-major weights: 16 of the contraction are two 1024-byte groups
+                                const uint32_t ad = desc_mn(a0 + (uint32_t)s * a_st), al = ad + (A_TILE >> 4);
+#pragma unroll
+                                for (uint32_t ks = 0; ks < 4; ks++) {
+                                    if constexpr (JOINED) {
+                                        mma(d, ad + 128 * ks, bd + 2 * ks, id_2n, acc | ks);  // hi x (hi | lo)
+                                        mma(d, al + 128 * ks, bd + 2 * ks, id_n, 1u);         // lo x hi
+                                    } else {
+                                        mma(d, ad + 128 * ks, bd + 2 * ks, id_n, acc | ks);
+                                        mma(d, ad + 128 * ks, bl + 2 * ks, id_n, 1u);
+                                        mma(d, al + 128 * ks, bd + 2 * ks, id_n, 1u);
+                                    }
+                                }
+                            } else {
+                                constexpr bool TWO = W::PARTS == 2;                                        // the weights have a lo part
+                                const uint32_t ta = tmem_a + (uint32_t)(s * A_COLS + c * 32 * W::PARTS);  // 16 of the contraction are 8 columns
+#pragma unroll
+                                for (uint32_t ks = 0; ks < (ext ? 1 : 4); ks++) {
+                                    if constexpr (JOINED) {
+                                        mma_ta(d, ta + 8 * ks, bd + 2 * ks, id_2n, acc | ks);  // hi x (hi | lo)
+                                    } else {
+                                        mma_ta(d, ta + 8 * ks, bd + 2 * ks, id_n, acc | ks);
+                                        if constexpr (FP32) {
+                                            mma_ta(d, ta + 8 * ks, bl + 2 * ks, id_n, 1u);
+                                        }
+                                    }
+                                    if constexpr (TWO) {
+                                        if (!ext) {
+                                            mma_ta(d, ta + 32 + 8 * ks, bd + 2 * ks, id_n, 1u);
+                                        }
+                                    }
+                                }
+                            }
+                            if (b_done) {
+                                tc::umma_commit(free_b + 8 * sb);
+                            }
+                            if (a_done) {
+                                tc::umma_commit(free_a + 8 * s);
+                                if (turn == TURNS - 1 && (FP32 || u == u1 - 1)) {
+                                    tc::umma_commit(acc_full + 8 * buf);
+                                }
+                            }
+                        }
+                        __syncwarp();
+                        first = false;
+                        if (b_done && ++sb == SB) {
+                            sb = 0;
+                            phb ^= 1;
+                        }
+                    }
                     if (!ok) {
                         break;
                     }
-                    // asked before this stage's MMAs are issued: the answer takes over a hundred clocks even when it is yes
-                    const int sn = s + 1 == SA ? 0 : s + 1, sbn = sb + 1 == SB ? 0 : sb + 1;
-                    const uint32_t phn = sn == 0 ? ph ^ 1 : ph, phbn = sbn == 0 ? phb ^ 1 : phb;
-                    ready = tc::mbar_test(full_a + 8 * sn, phn);
-                    ready_b = tc::mbar_test(full_b + 8 * sbn, phbn);
-                    tc::fence_after_sync();
-                    const uint32_t bd = desc_k(b0 + (uint32_t)sb * b_st), bl = bd + lo_rows;  // x: hi, lo; 16 of the contraction are 32 bytes
-                    if (elect_one()) {
-                        if constexpr (BWD) {
-                            // feature-major weights: 16 of the contraction are two 1024-byte groups
-                            const uint32_t ad = desc_mn(a0 + (uint32_t)s * a_st), al = ad + (A_TILE >> 4);
-#pragma unroll
-                            for (uint32_t ks = 0; ks < 4; ks++) {
-                                if constexpr (JOINED) {
-                                    mma(d, ad + 128 * ks, bd + 2 * ks, id_2n, acc | ks);  // hi x (hi | lo)
-                                    mma(d, al + 128 * ks, bd + 2 * ks, id_n, 1u);         // lo x hi
-                                } else {
-                                    mma(d, ad + 128 * ks, bd + 2 * ks, id_n, acc | ks);
-                                    mma(d, ad + 128 * ks, bl + 2 * ks, id_n, 1u);
-                                    mma(d, al + 128 * ks, bd + 2 * ks, id_n, 1u);
-                                }
-                            }
-                        } else {
-                            const uint32_t ta = tmem_a + (uint32_t)(s * A_COLS);  // 16 of the contraction are 8 columns
-                            constexpr bool TWO = HALF && H::TILES == 2;            // the weights have a lo part
-#pragma unroll
-                            for (uint32_t ks = 0; ks < (EXT && st == 4 ? 1 : 4); ks++) {
-                                if constexpr (JOINED) {
-                                    mma_ta(d, ta + 8 * ks, bd + 2 * ks, id_2n, acc | ks);  // hi x (hi | lo)
-                                } else {
-                                    mma_ta(d, ta + 8 * ks, bd + 2 * ks, id_n, acc | ks);
-                                    if constexpr (FP32) {
-                                        mma_ta(d, ta + 8 * ks, bl + 2 * ks, id_n, 1u);
-                                    }
-                                }
-                                if constexpr (TWO) {
-                                    if (!(EXT && st == 4)) {
-                                        mma_ta(d, ta + 32 + 8 * ks, bd + 2 * ks, id_n, 1u);
-                                    }
-                                }
-                            }
-                        }
-                        tc::umma_commit(free_a + 8 * s);
-                        tc::umma_commit(free_b + 8 * sb);
-                        if (st == UNIT_STAGES - 1 && (FP32 || u == u1 - 1)) {
-                            tc::umma_commit(acc_full + 8 * buf);
-                        }
-                    }
-                    __syncwarp();
-                    acc = 1;
                     s = sn;
                     ph = phn;
-                    sb = sbn;
-                    phb = phbn;
                 }
                 if (FP32 || u == u1 - 1) {
                     if (++buf == p.bufs) {
@@ -459,20 +494,32 @@ __global__ void __launch_bounds__(Warps<FP32, NMAX>::THREADS, 1) matmul_kernel(c
         const uint32_t my_lanes = (uint32_t)((warp & 3) * 32) << 16;
         const uint32_t row_at = (BWD ? (uint32_t)(tid >> 6) * 8192u : 0u) + (uint32_t)row0 * 128u;  // of the thread's row in the operand tile
         int s = group, r = 0, at_unit = 0;
-        uint32_t ph = 1, rph = 0;  // SA >= G: the barrier of a group's next stage is never two phases behind
+        uint32_t ph = 1, rph = 0;  // SA >= G: the barrier of a group's next operand is never two phases behind
         bool ok = true, raw_ready = false;
-        int first = group;  // the group's first stage of the unit, or of a later one
+        int first = OWNED ? 0 : group;  // the group's first turn of the unit, or of a later one
         for (int tile = cluster_id; tile < tiles && ok; tile += clusters) {
             const int h = (tile / p.ttiles) & 1;  // backward: which 128 of the super-block's features
             for (int u = u0; u < u1; u++, at_unit++) {
-                // every group waits for and gives back every unit: no group is a whole turn of the ring away from a barrier it tests
+                // Units of the whole ring in turn, where they are the group's own (R is a multiple of G, so a slot belongs to one group); else
+                // every group waits for and gives back every unit. Either way no group is a turn of the ring away from a barrier it tests.
+                const int rn = r + 1 == R ? 0 : r + 1;
+                const uint32_t rphn = rn == 0 ? rph ^ 1 : rph;
+                const bool mine = OWNED ? at_unit % G == group : first < TURNS;
+                if (OWNED && !mine) {
+                    r = rn;
+                    rph = rphn;
+                    continue;
+                }
                 if (!__all_sync(0xffffffffu, raw_ready) && !(ok = wait_warp(raw_full + 8 * r, rph, abort_flag, p.status, 6))) {
                     break;
                 }
-                const int rn = r + 1 == R ? 0 : r + 1;
-                const uint32_t rphn = rn == 0 ? rph ^ 1 : rph;
-                raw_ready = tc::mbar_test(raw_full + 8 * rn, rphn);
-                if (first >= UNIT_STAGES) {
+                if constexpr (OWNED) {
+                    const int ro = r + G >= R ? r + G - R : r + G;  // the group's next unit
+                    raw_ready = tc::mbar_test(raw_full + 8 * ro, r + G >= R ? rph ^ 1 : rph);
+                } else {
+                    raw_ready = tc::mbar_test(raw_full + 8 * rn, rphn);
+                }
+                if (!mine) {
                     __syncwarp();
                     if (lane == 0) {
                         tc::mbar_arrive(raw_read + 8 * r);
@@ -490,7 +537,7 @@ __global__ void __launch_bounds__(Warps<FP32, NMAX>::THREADS, 1) matmul_kernel(c
                     }
                     if constexpr (BWD) {
                         // a power of two brings the largest weight that the unit's blocks can hold to [2^13, 2^14); the fold multiplies by its inverse
-                        const int slot = at_unit & 7;  // a group is at most four stages, so fewer than eight units, ahead of another
+                        const int slot = at_unit & 7;  // a group is at most four turns, so fewer than eight units, ahead of another
                         if (first == 0) {
                             const uint32_t b = __reduce_max_sync(0xffffffffu, __float_as_uint(D::bound(D::head(uq, ua, tid))));
                             if (lane == 0) {
@@ -506,81 +553,86 @@ __global__ void __launch_bounds__(Warps<FP32, NMAX>::THREADS, 1) matmul_kernel(c
                         fac = __uint_as_float((267u - e) << 23);
                         unit_factor = (e - 13u) << 23;
                     }
-                    for (int st = first; st < UNIT_STAGES; st += G) {
-                        const int row = BWD ? row0 + 64 * st : row0, c = BWD ? 2 * h + (tid >> 6) : st;
+                    for (int turn = first; turn < TURNS; turn += G) {
+                        const bool ready = tc::mbar_test(free_a + 8 * s, ph);  // asked early: the answer takes longer than it looks
+                        const int row = BWD ? row0 + 64 * turn : row0, c0 = BWD ? 2 * h + (tid >> 6) : turn * TURN;
                         if constexpr (BWD) {
                             head = D::head(uq, ua, row);
                         }
-                        const bool ext = EXT && st == 4;
-                        const typename D::Raw raw = D::load(uq, row, ext ? 0 : c);
-                        if (st + G >= UNIT_STAGES) {  // this warp has read all it needs of the unit
+                        typename D::Raw raw[TURN];
+#pragma unroll
+                        for (int j = 0; j < TURN; j++) {
+                            raw[j] = D::load(uq, row, c0 + j);
+                        }
+                        if (OWNED || turn + G >= TURNS) {  // this warp has read all it needs of the unit
                             __syncwarp();
                             if (lane == 0) {
                                 tc::mbar_arrive(raw_read + 8 * r);
                             }
                         }
-                        const bool ready = tc::mbar_test(free_a + 8 * s, ph);  // asked early: the answer takes longer than it looks
                         // the first values while it is on its way
                         f2 w0[8], w1[8];
-                        uint32_t hi[8], lo[8];
-                        typename H::Scales sc;
-                        if constexpr (HALF) {
-                            sc = H::scales(head, ext ? 0 : c);
-                            if (ext) {
-                                H::ext(head, hi);
-                            } else {
-                                H::values(head, raw, sc, c, 0, 0, hi, lo);
-                            }
-                        } else {
-                            D::values(head, raw, c, 0, fac, w0, w1);
+                        if constexpr (!HALF) {
+                            D::values(head, raw[0], c0, 0, fac, w0, w1);
                         }
                         if (!__all_sync(0xffffffffu, ready) && !(ok = wait_warp(free_a + 8 * s, ph, abort_flag, p.status, 1))) {
                             break;
                         }
-                        if (FP32 && st == 0) {
-                            // The unit's factors for the fold. Not before the unit's first stage is this group's: the accumulator four
-                            // units back has then been taken, and the fold is done with what this ring of four held.
-                            const uint32_t fa = fac0 + (uint32_t)(at_unit & 3) * 512u;
+                        if (FP32 && turn == 0) {
+                            // The unit's factors for the fold, into a ring of FACTORS units. This operand's slot is free, so what it held SA
+                            // operands ago went through the tensor core, into an accumulator that the fold had emptied: the fold is done
+                            // with the unit at least that far and `bufs` accumulators back, SA + bufs <= FACTORS.
+                            const uint32_t fa = fac0 + (uint32_t)(at_unit & (FACTORS - 1)) * 512u;
                             if (!BWD || tid == 0) {
                                 asm volatile("st.shared.u32 [%0], %1;" ::"r"(fa + (BWD ? 0u : 4u * (uint32_t)row0)), "r"(unit_factor) : "memory");
                             }
                             __syncwarp();
                             if (lane == 0 && (!BWD || tid == 0)) {
-                                tc::mbar_arrive(fac_full + 8 * (at_unit & 3));
+                                tc::mbar_arrive(fac_full + 8 * (at_unit & (FACTORS - 1)));
                             }
                         }
                         if constexpr (BWD) {  // operand row = contraction index, 64 features a row
                             const uint32_t to = a0 + (uint32_t)s * a_st + row_at;
                             run_to_smem<FP32>(w0, to, D::piece(0, 0), row0 & 7);
                             run_to_smem<FP32>(w1, to, D::piece(0, 1), row0 & 7);
-                            D::values(head, raw, c, 1, fac, w0, w1);
+                            D::values(head, raw[0], c0, 1, fac, w0, w1);
                             run_to_smem<FP32>(w0, to, D::piece(1, 0), row0 & 7);
                             run_to_smem<FP32>(w1, to, D::piece(1, 1), row0 & 7);
                             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic stores -> visible to the tensor core
                         } else {
                             const uint32_t to = tmem_a + my_lanes + (uint32_t)(s * A_COLS);
                             tc::fence_after_sync();
-                            if constexpr (HALF) {
-                                if (ext) {
-                                    st_tmem8(to, hi);
-                                } else {
+#pragma unroll
+                            for (int j = 0; j < TURN; j++) {
+                                const uint32_t tj = to + (uint32_t)(j * 32 * W::PARTS);
+                                if constexpr (HALF) {
+                                    const typename H::Scales sc = H::scales(head, c0 + j);
 #pragma unroll
                                     for (int i = 0; i < 4; i++) {
-                                        if (i > 0) {
-                                            H::values(head, raw, sc, c, i >> 1, i & 1, hi, lo);
-                                        }
-                                        st_tmem8(to + 4 * D::piece(i >> 1, i & 1), hi);
-                                        if constexpr (H::TILES == 2) {
-                                            st_tmem8(to + 32 + 4 * D::piece(i >> 1, i & 1), lo);
+                                        uint32_t hi[8], lo[8];
+                                        H::values(head, raw[j], sc, c0 + j, i >> 1, i & 1, hi, lo);
+                                        st_tmem8(tj + 4 * D::piece(i >> 1, i & 1), hi);
+                                        if constexpr (W::PARTS == 2) {
+                                            st_tmem8(tj + 32 + 4 * D::piece(i >> 1, i & 1), lo);
                                         }
                                     }
+                                } else {
+                                    if (j > 0) {
+                                        D::values(head, raw[j], c0 + j, 0, fac, w0, w1);
+                                    }
+                                    run_to_tmem(w0, tj, D::piece(0, 0));
+                                    run_to_tmem(w1, tj, D::piece(0, 1));
+                                    D::values(head, raw[j], c0 + j, 1, fac, w0, w1);
+                                    run_to_tmem(w0, tj, D::piece(1, 0));
+                                    run_to_tmem(w1, tj, D::piece(1, 1));
                                 }
-                            } else {
-                                run_to_tmem(w0, to, D::piece(0, 0));
-                                run_to_tmem(w1, to, D::piece(0, 1));
-                                D::values(head, raw, c, 1, fac, w0, w1);
-                                run_to_tmem(w0, to, D::piece(1, 0));
-                                run_to_tmem(w1, to, D::piece(1, 1));
+                            }
+                            if constexpr (EXT) {
+                                if (turn == TURNS - 1) {
+                                    uint32_t v[8];
+                                    H::ext(head, v);
+                                    st_tmem8(to + TURN * 32 * W::PARTS, v);
+                                }
                             }
                             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                             tc::fence_before_sync();
@@ -599,7 +651,7 @@ __global__ void __launch_bounds__(Warps<FP32, NMAX>::THREADS, 1) matmul_kernel(c
                         break;
                     }
                 }
-                first -= UNIT_STAGES;
+                first = OWNED ? 0 : first - TURNS;
                 r = rn;
                 rph = rphn;
             }
@@ -663,10 +715,22 @@ __global__ void __launch_bounds__(Warps<FP32, NMAX>::THREADS, 1) matmul_kernel(c
             };
             if constexpr (FP32) {
                 constexpr int C = NMAX / PARTS;  // columns per thread
-                f2 sum[C / 2];
+                f2 sum[C / 2], total[CANON ? C / 2 : 1];
 #pragma unroll
                 for (int i = 0; i < C / 2; i++) {
                     sum[i] = 0;
+                    if constexpr (CANON) {
+                        total[i] = 0;
+                    }
+                }
+                // CANON: the end of the virtual range that unit u0 belongs to; its sum is added to the total, or kept apart for the cluster
+                int virt = 0, slot = 0;
+                auto virt_end = [&](int v) { return (int)((int64_t)(v + 1) * p.units / VIRTUAL); };
+                if constexpr (CANON) {
+                    while (virt < VIRTUAL - 1 && virt_end(virt) <= u0) {
+                        virt++;
+                    }
+                    slot = virt - range * (VIRTUAL / p.ksplit);
                 }
                 // the scales of a unit's columns: fetched by the lanes a unit ahead, read back as broadcasts
                 const uint32_t scl = scl0 + (uint32_t)(warp - 3 - 4 * G) * 512u;
@@ -691,14 +755,14 @@ __global__ void __launch_bounds__(Warps<FP32, NMAX>::THREADS, 1) matmul_kernel(c
                         }
                     }
                     __syncwarp();
-                    ok = wait_warp(fac_full + 8 * (chunk & 3), (uint32_t)(chunk >> 2) & 1u, abort_flag, p.status, 6) &&
+                    ok = wait_warp(fac_full + 8 * (chunk & (FACTORS - 1)), (uint32_t)(chunk / FACTORS) & 1u, abort_flag, p.status, 6) &&
                          wait_warp(acc_full + 8 * buf, aph, abort_flag, p.status, 4);
                     if (!ok) {
                         break;
                     }
                     tc::fence_after_sync();
                     float f;
-                    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"(fac0 + (uint32_t)(chunk & 3) * 512u + (BWD ? 0u : 4u * (uint32_t)lane_row)));
+                    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"(fac0 + (uint32_t)(chunk & (FACTORS - 1)) * 512u + (BWD ? 0u : 4u * (uint32_t)lane_row)));
                     const f2 ff = pack2(f, f);
                     const uint32_t d = tmem + lanes + (uint32_t)(buf * p.cols + c0);
 #pragma unroll
@@ -723,9 +787,45 @@ __global__ void __launch_bounds__(Warps<FP32, NMAX>::THREADS, 1) matmul_kernel(c
                         }
                     }
                     release();
+                    if constexpr (CANON) {
+                        if (u + 1 == virt_end(virt)) {
+                            if (p.ksplit > 1) {
+#pragma unroll
+                                for (int i = 0; i < C / 2; i++) {
+                                    float a, b;
+                                    unpack2(sum[i], a, b);
+                                    const uint32_t to = base + (uint32_t)(((slot * nt + c0 + 2 * i) * 128 + lane_row) * 4);
+                                    asm volatile("st.shared.f32 [%0], %1;" ::"r"(to), "f"(a) : "memory");
+                                    asm volatile("st.shared.f32 [%0], %1;" ::"r"(to + 512u), "f"(b) : "memory");
+                                }
+                            } else {
+#pragma unroll
+                                for (int i = 0; i < C / 2; i++) {
+                                    total[i] = add2(total[i], sum[i]);
+                                }
+                            }
+#pragma unroll
+                            for (int i = 0; i < C / 2; i++) {
+                                sum[i] = 0;
+                            }
+                            do {
+                                virt++;
+                                slot++;
+                            } while (virt < VIRTUAL - 1 && virt_end(virt) <= u + 1);
+                        }
+                    }
                 }
                 if (!ok) {
                     break;
+                }
+                if constexpr (CANON) {
+                    if (p.ksplit > 1) {
+                        continue;  // (one tile per cluster)
+                    }
+#pragma unroll
+                    for (int i = 0; i < C / 2; i++) {
+                        sum[i] = total[i];
+                    }
                 }
                 // (the last accumulator is complete: every tile in shared memory is used up and may hold the partial tile)
 #pragma unroll
@@ -771,27 +871,30 @@ __global__ void __launch_bounds__(Warps<FP32, NMAX>::THREADS, 1) matmul_kernel(c
         cluster_sync();  // partial tiles are complete
     }
     if (p.ksplit > 1 && *abort_flag == 0) {
-        // columns range, range + ksplit, .. of the tile: the ranges' sums in range order
+        // columns range, range + ksplit, .. of the tile: the (virtual) ranges' sums in order
         const int ft = cluster_id / p.ttiles, t0 = (cluster_id % p.ttiles) * nt;
         const int64_t f0 = (int64_t)ft * 128;
         const int mine = (nt - range + p.ksplit - 1) / p.ksplit * 32;  // pieces of four features of a column
         constexpr int BATCH = 2, MOST = 4;  // pieces and ranges in flight: another CTA's memory is most of a microsecond away
+        const int parts = CANON ? VIRTUAL : p.ksplit, per_cta = parts / p.ksplit;
         for (int i0 = threadIdx.x; i0 < mine; i0 += BATCH * W::THREADS) {
             float4 sum[BATCH];
 #pragma unroll
             for (int j = 0; j < BATCH; j++) {
                 sum[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             }
-            for (int g0 = 0; g0 < p.ksplit; g0 += MOST) {
+            for (int g0 = 0; g0 < parts; g0 += MOST) {
                 float4 v[MOST][BATCH];
 #pragma unroll
                 for (int g = 0; g < MOST; g++) {
-                    const uint32_t from = map_rank(base, (uint32_t)(g0 + g < p.ksplit ? g0 + g : 0));
+                    const int part = g0 + g;
+                    const bool there = part < parts && (!CANON || (int64_t)part * p.units / VIRTUAL < (int64_t)(part + 1) * p.units / VIRTUAL);
+                    const uint32_t from = map_rank(base + (uint32_t)(part % per_cta * nt * 512), (uint32_t)(there ? part / per_cta : 0));
 #pragma unroll
                     for (int j = 0; j < BATCH; j++) {
                         const int i = i0 + j * W::THREADS, col = range + (i >> 5) * p.ksplit;
                         v[g][j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // a missing range adds an exact zero
-                        if (g0 + g < p.ksplit && i < mine) {
+                        if (there && i < mine) {
                             asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];"
                                          : "=f"(v[g][j].x), "=f"(v[g][j].y), "=f"(v[g][j].z), "=f"(v[g][j].w)
                                          : "r"(from + (uint32_t)(col * 128 + (i & 31) * 4) * 4u));

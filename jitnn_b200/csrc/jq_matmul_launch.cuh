@@ -9,10 +9,31 @@ namespace mm {
 
 struct Plan {
     bool fp32, bwd;
-    bool narrow;  // the FP32 instance for tiles of up to 32 rows of x
-    int ctas;     // grid
+    int nmax;  // the instance, by the widest tile of rows of x it takes
+    int ctas;  // grid
     size_t smem;
 };
+
+// What the host has to know of an instance's Shape.
+struct Facts {
+    int groups, turn, turns, a_cols, b_tiles, columns;  // columns: accumulator columns per row of x
+    bool owned, ext;
+};
+template <int TYPE, bool FP32, bool BWD, int NMAX>
+constexpr Facts facts_of() {
+    using W = Shape<TYPE, FP32, BWD, NMAX>;
+    return Facts{W::GROUPS, W::TURN, W::TURNS, W::A_COLS, W::B_TILES, W::JOINED ? 2 : 1, W::OWNED, W::EXT};
+}
+template <int TYPE>
+Facts facts_format(bool fp32, bool bwd, int nmax) {
+    if (!fp32) {
+        return nmax <= 128 ? facts_of<TYPE, false, false, 128>() : facts_of<TYPE, false, false, 256>();
+    }
+    if (bwd) {
+        return nmax <= 32 ? facts_of<TYPE, true, true, 32>() : facts_of<TYPE, true, true, 128>();
+    }
+    return nmax <= 16 ? facts_of<TYPE, true, false, 16>() : (nmax <= 32 ? facts_of<TYPE, true, false, 32>() : facts_of<TYPE, true, false, 128>());
+}
 
 template <int TYPE, bool FP32, bool BWD, int NMAX>
 int launch_instance(const Plan& plan, const Args& args, const CUtensorMap& map, cudaStream_t s) {
@@ -26,7 +47,7 @@ int launch_instance(const Plan& plan, const Args& args, const CUtensorMap& map, 
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)plan.ctas);
-    cfg.blockDim = dim3((Warps<FP32, NMAX>::THREADS));
+    cfg.blockDim = dim3((Shape<TYPE, FP32, BWD, NMAX>::THREADS));
     cfg.dynamicSmemBytes = plan.smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
@@ -46,12 +67,14 @@ int launch_instance(const Plan& plan, const Args& args, const CUtensorMap& map, 
 template <int TYPE>
 int launch_format(const Plan& plan, const Args& args, const CUtensorMap& map, cudaStream_t s) {
     if (!plan.fp32) {
-        return launch_instance<TYPE, false, false, 16>(plan, args, map, s);
+        return plan.nmax <= 128 ? launch_instance<TYPE, false, false, 128>(plan, args, map, s) : launch_instance<TYPE, false, false, 256>(plan, args, map, s);
     }
     if (plan.bwd) {
-        return plan.narrow ? launch_instance<TYPE, true, true, 32>(plan, args, map, s) : launch_instance<TYPE, true, true, 128>(plan, args, map, s);
+        return plan.nmax <= 32 ? launch_instance<TYPE, true, true, 32>(plan, args, map, s) : launch_instance<TYPE, true, true, 128>(plan, args, map, s);
     }
-    return plan.narrow ? launch_instance<TYPE, true, false, 32>(plan, args, map, s) : launch_instance<TYPE, true, false, 128>(plan, args, map, s);
+    return plan.nmax <= 16   ? launch_instance<TYPE, true, false, 16>(plan, args, map, s)
+           : plan.nmax <= 32 ? launch_instance<TYPE, true, false, 32>(plan, args, map, s)
+                             : launch_instance<TYPE, true, false, 128>(plan, args, map, s);
 }
 
 int launch_q4_k(const Plan& plan, const Args& args, const CUtensorMap& map, cudaStream_t s);

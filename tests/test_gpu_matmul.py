@@ -53,6 +53,23 @@ def test_backward(t, n, k, m):
     close(Gguf.linearBackward(g, w), g.double() @ wd)
 
 
+# up to 16 rows the sums are taken in eight ranges of k whatever the number of thread blocks that share it: a row shard, whose k is split over a
+# larger cluster, gives bitwise the outputs of the whole weight. k: fewer units than ranges, more, and not a multiple
+@pytest.mark.parametrize("k", [768, 2048, 2816, 11008])
+@pytest.mark.parametrize("t", LINEAR_TYPES)
+def test_row_shards_are_bitwise_equal(t, k):
+    n, m = 5000, 13
+    raw = synth.random_valid_blocks(t, n, k, seed=k).numpy().reshape(-1)
+    whole = Tensor.quantized(t, raw, n, k)
+    x = torch.randn(m, k, generator=torch.Generator().manual_seed(k)).cuda()
+    y = Gguf.linear(x, whole)
+    for lo, hi in [(0, 100), (2048, 2560), (3000, 5000)]:
+        shard = Tensor.quantized(t, raw, n, k, rows=(lo, hi))
+        assert torch.equal(Gguf.linear(x, shard), y[:, lo:hi])
+    wd = torch.from_numpy(oracle.dequantize(t, raw).reshape(n, k)).cuda().double()
+    close(y, x.double() @ wd.T)
+
+
 # 32-element formats: k that does not fill a step of 256, or not even a multiple of 4 x 32
 @pytest.mark.parametrize("k", [32, 96, 224, 288, 1056])
 @pytest.mark.parametrize("t", ["Q8_0", "Q4_0", "Q4_1"])
