@@ -61,9 +61,27 @@ struct Staging {
     uint8_t* dev = nullptr;
     size_t bytes = 0;
     cudaStream_t stream = nullptr;
+    uint8_t* pinned = nullptr;      // PINNED_BYTES of page-locked memory that the device can address
+    uint8_t* pinned_dev = nullptr;  // its address on the device
 };
+// Pageable arrays up to this size in all take the way through page-locked memory of the thread, which the kernels then read and write
+// themselves: a copy by the host of some kilobytes costs less than setting up a copy engine for it (one row of Q8_0 4096 x 4096 with bias,
+// from and to numpy arrays: 36 us with three engine copies).
+constexpr size_t PINNED_BYTES = (size_t)512 << 10;
 
-static thread_local std::vector<Staging> t_staging;
+// What a thread holds is given back when it ends (a driver that is shutting down has released it already and says so).
+struct ThreadStaging {
+    std::vector<Staging> devices;
+    ~ThreadStaging() {
+        for (Staging& st : devices) {
+            if (st.pinned != nullptr) {
+                cudaFreeHost(st.pinned);
+            }
+        }
+    }
+};
+static thread_local ThreadStaging t_staging_owner;
+#define t_staging t_staging_owner.devices
 
 static int staging_for(int device, size_t bytes, Staging** out) {
     if ((size_t)device >= t_staging.size()) {
@@ -144,6 +162,26 @@ int scratch_for_slot(cudaStream_t s, int slot, size_t bytes, uint8_t** out) { re
 int scratch_zeroed_for_slot(cudaStream_t s, int slot, size_t bytes, uint8_t** out) { return scratch_impl(s, slot, bytes, true, out); }
 
 static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
+
+// The thread's page-locked staging memory, nullptr where there is none to be had.
+static uint8_t* pinned_staging(Staging* st) {
+    if (st->pinned == nullptr) {
+        void* host = nullptr;
+        void* dev = nullptr;
+        if (cudaHostAlloc(&host, PINNED_BYTES, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        if (cudaHostGetDevicePointer(&dev, host, 0) != cudaSuccess) {
+            cudaGetLastError();
+            cudaFreeHost(host);
+            return nullptr;
+        }
+        st->pinned = static_cast<uint8_t*>(host);
+        st->pinned_dev = static_cast<uint8_t*>(dev);
+    }
+    return st->pinned;
+}
 
 // The device-side address of a host buffer that kernels may use directly: page-locked, 16-byte aligned, at most `limit`
 // bytes. nullptr otherwise (pageable memory, or a driver that cannot say).
@@ -602,7 +640,32 @@ int jq_linear_f32(const jq_weight* w, const float* x, int64_t m, const float* bi
     const float* dx = pinned_device_pointer(x, (size_t)m * w->k * 4, direct_limit << 2);
     const float* db = bias != nullptr ? pinned_device_pointer(bias, (size_t)w->n * 4, direct_limit) : nullptr;
     float* dy = const_cast<float*>(pinned_device_pointer(y, (size_t)m * w->n * 4, direct_limit));
+    const size_t x_bytes = (size_t)m * w->k * 4, b_bytes = (size_t)w->n * 4, y_bytes = (size_t)m * w->n * 4;
+    float* y_staged = nullptr;  // where y lies in page-locked staging memory
+    if ((dx == nullptr || dy == nullptr) && xb + bb + yb <= PINNED_BYTES && y_bytes <= direct_limit && pinned_staging(st) != nullptr) {
+        if (dx == nullptr) {
+            memcpy(st->pinned, x, x_bytes);
+            // (the CUDA-core kernel reads x once per output row: that one gets a copy on the device)
+            const bool once = g_opt_gemv_generic.load() == 0 &&
+                              (w->type == JQ_TYPE_Q4_K || w->type == JQ_TYPE_Q5_K || w->type == JQ_TYPE_Q6_K || gemv_blk32_i8_scratch_bytes(w->type, w->k, 1) > 0);
+            if (once) {
+                dx = reinterpret_cast<const float*>(st->pinned_dev);
+            } else {
+                JQ_CUDA(cudaMemcpyAsync(st->dev, st->pinned, x_bytes, cudaMemcpyHostToDevice, st->stream));
+                dx = (const float*)st->dev;
+            }
+        }
+        if (bias != nullptr && db == nullptr) {
+            memcpy(st->pinned + xb, bias, b_bytes);
+            db = reinterpret_cast<const float*>(st->pinned_dev + xb);
+        }
+        if (dy == nullptr) {
+            y_staged = reinterpret_cast<float*>(st->pinned + xb + bb);
+            dy = reinterpret_cast<float*>(st->pinned_dev + xb + bb);
+        }
+    }
     const bool copy_y = dy == nullptr;
+    const bool x_remote = dx != nullptr;
     if (dx == nullptr) {
         JQ_CUDA(cudaMemcpyAsync(st->dev, x, (size_t)m * w->k * 4, cudaMemcpyHostToDevice, st->stream));
         dx = (const float*)st->dev;
@@ -614,7 +677,7 @@ int jq_linear_f32(const jq_weight* w, const float* x, int64_t m, const float* bi
     if (copy_y) {
         dy = (float*)(st->dev + xb + bb);
     }
-    rc = linear_device(w, dx, m, db, dy, st->stream, dx == x);  // x in host memory: read it once, not once per thread block
+    rc = linear_device(w, dx, m, db, dy, st->stream, x_remote);  // x in host memory: read it once, not once per thread block
     if (rc != JQ_OK) {
         return rc;
     }
@@ -622,6 +685,9 @@ int jq_linear_f32(const jq_weight* w, const float* x, int64_t m, const float* bi
         JQ_CUDA(cudaMemcpyAsync(y, dy, (size_t)m * w->n * 4, cudaMemcpyDeviceToHost, st->stream));
     }
     JQ_CUDA(cudaStreamSynchronize(st->stream));
+    if (y_staged != nullptr) {
+        memcpy(y, y_staged, y_bytes);
+    }
     return JQ_OK;
 }
 
