@@ -273,6 +273,19 @@ int linear_device_multi(const jq_weight* const* ws, int count, const float* x, i
         return JQ_OK;
     }
     const int64_t min_rows = g_prefill_min_rows.load();
+    const bool tc = g_opt_gemv_generic.load() == 0;
+    // more rows of x than the decode kernels take in a pass: one split of x, one launch per format
+    bool matrix = count >= 2 && count <= 3 && tc && !(min_rows > 0 && m >= min_rows);
+    for (int i = 0; i < count && matrix; i++) {
+        matrix = ws[i]->n > 0 && ws[i]->k == ws[0]->k && matmul_takes(view_of(ws[i]), m) && !(m <= 16 && gemv_umma_takes(ws[i]->type, ws[i]->k, (int)m));
+    }
+    if (matrix) {
+        View vs[3];
+        for (int i = 0; i < count; i++) {
+            vs[i] = view_of(ws[i]);
+        }
+        return launch_matmul_f32_multi(vs, count, x, m, ys, s);
+    }
     bool same = count >= 1;
     for (int i = 0; i < count && same; i++) {
         same = ws[i]->type == ws[0]->type && ws[i]->k == ws[0]->k && ws[i]->n > 0;
@@ -296,13 +309,6 @@ int linear_device_multi(const jq_weight* const* ws, int count, const float* x, i
         return n_like > 0 ? linear_device_multi(like, n_like, x, m, like_y, s) : JQ_OK;
     }
     const bool together = same && count >= 2 && count <= 3 && m >= 1 && m <= 16 && !(min_rows > 0 && m >= min_rows);
-    if (together && g_opt_gemv_generic.load() == 0 && matmul_takes(view_of(ws[0]), m) && !gemv_umma_takes(ws[0]->type, ws[0]->k, (int)m)) {
-        View vs[3];
-        for (int i = 0; i < count; i++) {
-            vs[i] = view_of(ws[i]);
-        }
-        return launch_matmul_f32_multi(vs, count, x, m, ys, s);
-    }
     if (together && gemv_umma_takes(ws[0]->type, ws[0]->k, (int)m)) {
         View vs[3];
         for (int i = 0; i < count; i++) {

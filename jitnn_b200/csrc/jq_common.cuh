@@ -212,11 +212,12 @@ constexpr int PAD_ROWS = 16;
 
 // The matrix kernel (jq_matmul.cu): the FP32 product with many rows of x, and the bfloat16 product.
 int launch_matmul_f32(const View& v, const float* x, int64_t m, const float* bias, float* y, cudaStream_t s);
-// Several weights of one k on the same x: the split of x into halves is shared (formats may differ in whether they need its sums).
+// Up to three weights of one k on the same x: the split of x into halves is shared, weights of one format are one launch.
 int launch_matmul_f32_multi(const View* vs, int count, const float* x, int64_t m, float* const* ys, cudaStream_t s);
 bool matmul_takes(const View& v, int64_t rows);  // where it is the fastest of the FP32 kernels
 bool prefill_supported(const View& v);
 int launch_prefill_bf16(const View& v, const uint16_t* x_bf16, int64_t m, const float* bias, float* y, cudaStream_t s);
+int launch_prefill_bf16_multi(const View* vs, int count, const uint16_t* x_bf16, int64_t m, const float* bias, float* const* ys, cudaStream_t s);
 int launch_f32_to_bf16(const float* x, uint16_t* out, int64_t count, cudaStream_t s);
 int prefill_status(int* status);
 // Same for the bounded waits of the peer gather (jq_peer.cu): 0, or 32 + the rank whose slice did not arrive.

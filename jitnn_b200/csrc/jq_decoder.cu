@@ -2033,11 +2033,18 @@ JQ_API int jq_decoder_prompt(jq_decoder* d, int seq, const int32_t* tokens_host,
         att.T = T; att.pos0 = pos0; att.heads = d->heads; att.kv_heads = d->kv_heads;
         att.scale = (float)(1.0 / std::sqrt((double)hd));
         prompt_attention_layout(att, reinterpret_cast<uint8_t*>(((uintptr_t)p + 255) / 256 * 256), hd);
-        auto LIN = [&](const jq_weight* w, float* out_) {
+        // up to three linears on what is in xb
+        auto LIN = [&](const jq_weight* const* w, int count, float* const* out_) {
+            View vs[3];
+            for (int i = 0; i < count; i++) {
+                vs[i] = View{w[i]->q, w[i]->aux, w[i]->n, w[i]->k, w[i]->type};
+            }
             if (rc == JQ_OK) {
-                rc = launch_prefill_bf16(View{w->q, w->aux, w->n, w->k, w->type}, d->prompt_bf16, T, nullptr, out_, s);
+                rc = launch_prefill_bf16_multi(vs, count, d->prompt_bf16, T, nullptr, out_, s);
             }
         };
+        float* const qkv[3] = {q, k, v};
+        float* const gate_up[2] = {gate, up};
         auto KERNEL = [&](cudaError_t e, const char* name) {
             count_launch(1);
             CK(e, name);
@@ -2054,22 +2061,19 @@ JQ_API int jq_decoder_prompt(jq_decoder* d, int seq, const int32_t* tokens_host,
             const jq_weight* const* L = &d->lin[(size_t)l * 7];
             KERNEL(launch_pdl(add_rmsnorm_kernel<__nv_bfloat16>, dim3(T), dim3(NORM_THREADS), 0, s, true, x, l == 0 ? nullptr : proj,
                               d->norms + (size_t)(2 * l) * dim, d->eps, xb, dim), "add_rmsnorm_kernel");
-            LIN(L[0], q);
-            LIN(L[1], k);
-            LIN(L[2], v);
+            LIN(L, 3, qkv);
             if (rc != JQ_OK) break;
             att.k_cache = d->k_cache + seq_base + (size_t)l * d->max_seq * kv_dim;
             att.v_cache = d->v_cache + seq_base + (size_t)l * d->max_seq * kv_dim;
             rc = launch_prompt_attention(att, hd, s);
-            LIN(L[3], proj);
+            LIN(L + 3, 1, &proj);
             if (rc != JQ_OK) break;
             KERNEL(launch_pdl(add_rmsnorm_kernel<__nv_bfloat16>, dim3(T), dim3(NORM_THREADS), 0, s, true, x, proj, d->norms + (size_t)(2 * l + 1) * dim,
                               d->eps, xb, dim), "add_rmsnorm_kernel");
-            LIN(L[4], gate);
-            LIN(L[5], up);
+            LIN(L + 4, 2, gate_up);
             if (rc != JQ_OK) break;
             KERNEL(launch_pdl(swiglu_kernel<__nv_bfloat16>, dim3((unsigned)((cnt + 1023) / 1024)), dim3(256), 0, s, true, gate, up, xb, cnt), "swiglu_kernel");
-            LIN(L[6], proj);
+            LIN(L + 6, 1, &proj);
         }
         if (rc == JQ_OK) {
             // the last token alone goes on: final residual add and norm, output projection (FP32 path), first index of the maximum

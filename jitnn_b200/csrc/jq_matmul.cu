@@ -179,12 +179,11 @@ static double unit_ns(int type, bool fp32, bool bwd, int nt) {
     return t < 1320.0 ? 1320.0 : t;
 }
 
-// Tile width and ranges of the contraction for a product of `features` x m over `units` units.
-static void choose(int type, bool fp32, bool bwd, int64_t features, int units, int m, Args& a, Plan& plan) {
+// Tile width and ranges of the contraction for a product of `ftiles` tiles of features x m over `units` units.
+static void choose(int type, bool fp32, bool bwd, int64_t ftiles, int units, int m, Args& a, Plan& plan) {
     const int nmax = fp32 ? 128 : 256;
     double best = 1e30;
     int best_nt = 16, best_ks = 1;
-    const int64_t ftiles = (features + 127) / 128;
     int last_nt = 0;
     for (int tt = (m + nmax - 1) / nmax; tt <= (m + nmax - 1) / nmax + 6; tt++) {
         const int nt = ((m + tt - 1) / tt + 15) / 16 * 16;
@@ -250,11 +249,20 @@ static int activation_map(CUtensorMap* map, bool bf16, const void* x, int64_t wi
     return r == CUDA_SUCCESS ? JQ_OK : fail(JQ_ERR_CUDA, "matrix product: cuTensorMapEncodeTiled failed with code %d", (int)r);
 }
 
-static void weight_args(const View& v, Args& a) {
-    a.q = v.q;
-    a.aux = v.aux;
-    a.kb = (int)tiled_steps(v.k);
-    a.rows128 = (int)(tiled_rows(v.n) / TILE_ROWS);
+// Puts `count` weights (one format and k) into the arguments; returns their tiles of features.
+static int weight_args(const View* vs, int count, bool bwd, float* const* ys, Args& a) {
+    int end = 0;
+    for (int i = 0; i < MAX_WEIGHTS; i++) {
+        const View& v = vs[i < count ? i : 0];
+        a.q[i] = v.q;
+        a.aux[i] = v.aux;
+        a.y[i] = ys[i < count ? i : 0];
+        a.features[i] = bwd ? v.k : v.n;
+        end += i < count ? (int)((a.features[i] + 127) / 128) : 0;
+        a.ft_end[i] = end;
+    }
+    a.kb = (int)tiled_steps(vs[0].k);
+    return end;
 }
 
 constexpr int SPLIT_SLOT = 6;  // scratch slots 6 and 7: split activations without and with the 16 more columns
@@ -278,8 +286,20 @@ static int product_f32(const View* vs, int count, bool bwd, const float* x, int6
             uint8_t* scratch = nullptr;
             float* scales = nullptr;
             for (int i = 0; i < count && rc == JQ_OK; i++) {
-                const View& v = vs[i];
-                if (facts(v.type, true, bwd, 16).ext != (ext != 0)) {
+                // the weights of one format in one launch, with the first of them
+                const int type = vs[i].type;
+                View like[MAX_WEIGHTS];
+                float* like_y[MAX_WEIGHTS];
+                int n_like = 0;
+                bool first = true;
+                for (int j = 0; j < count; j++) {
+                    if (vs[j].type == type) {
+                        first = first && j >= i;
+                        like[n_like] = vs[j];
+                        like_y[n_like++] = ys[j] + m0 * (bwd ? vs[j].k : vs[j].n);
+                    }
+                }
+                if (!first || facts(type, true, bwd, 16).ext != (ext != 0)) {
                     continue;
                 }
                 if (scratch == nullptr) {
@@ -301,23 +321,20 @@ static int product_f32(const View* vs, int count, bool bwd, const float* x, int6
                     JQ_CUDA(cudaLaunchKernelEx(&cfg, split, xg, rows, width, per_row, reinterpret_cast<uint4*>(scratch), scales, stride, vec));
                     count_launch();
                 }
-                const int64_t features = bwd ? v.k : v.n;
                 Args a = {};
                 Plan plan = {};
-                weight_args(v, a);
-                choose(v.type, true, bwd, features, bwd ? a.rows128 : a.kb, rows, a, plan);
+                const int ftiles = weight_args(like, n_like, bwd, like_y, a);
+                choose(type, true, bwd, ftiles, bwd ? (int)(tiled_rows(vs[i].n) / TILE_ROWS) : a.kb, rows, a, plan);
                 CUtensorMap map;
                 rc = activation_map(&map, false, scratch, wpad, rows, 2, a.nt);
                 if (rc != JQ_OK) {
                     break;
                 }
-                a.features = features;
                 a.xscale = scales;
                 a.xstride = stride;
                 a.bias = bias;
-                a.y = ys[i] + m0 * features;
                 a.status = status;
-                rc = launch_any(v.type, plan, a, map, s);
+                rc = launch_any(type, plan, a, map, s);
             }
         }
     }
@@ -360,28 +377,47 @@ int launch_linear_backward(const View& v, const float* g, int64_t m, float* gx, 
 
 bool prefill_supported(const View& v) { return has_linear_kernel(v.type) && v.k % 64 == 0 && v.n > 0 && v.k > 0; }
 
-// y[m, n] = x_bf16[m, k] . W^T (+ bias); x 16-byte aligned device memory.
-int launch_prefill_bf16(const View& v, const uint16_t* x_bf16, int64_t m, const float* bias, float* y, cudaStream_t s) {
+// ys[i] [m, n_i] = x_bf16[m, k] . W_i^T (+ bias for the first) for up to three weights of one k; x 16-byte aligned device memory.
+int launch_prefill_bf16_multi(const View* vs, int count, const uint16_t* x_bf16, int64_t m, const float* bias, float* const* ys, cudaStream_t s) {
     using namespace mm;
-    if (!prefill_supported(v)) {
-        return fail(JQ_ERR_UNSUPPORTED, "prefill: the tensor-core kernel needs k to be a multiple of 64 (k = %lld)", (long long)v.k);
+    int* status = nullptr;
+    int rc = status_word(&status);
+    for (int i = 0; i < count && rc == JQ_OK; i++) {
+        if (!prefill_supported(vs[i])) {
+            return fail(JQ_ERR_UNSUPPORTED, "prefill: the tensor-core kernel needs k to be a multiple of 64 (k = %lld)", (long long)vs[i].k);
+        }
+        // the weights of one format in one launch, with the first of them
+        View like[MAX_WEIGHTS];
+        float* like_y[MAX_WEIGHTS];
+        int n_like = 0;
+        bool first = true;
+        for (int j = 0; j < count; j++) {
+            if (vs[j].type == vs[i].type) {
+                first = first && j >= i;
+                like[n_like] = vs[j];
+                like_y[n_like++] = ys[j];
+            }
+        }
+        if (!first) {
+            continue;
+        }
+        Args a = {};
+        Plan plan = {};
+        const int ftiles = weight_args(like, n_like, false, like_y, a);
+        choose(vs[i].type, false, false, ftiles, a.kb, (int)m, a, plan);
+        CUtensorMap map;
+        rc = activation_map(&map, true, x_bf16, vs[i].k, m, 1, a.nt);
+        if (rc == JQ_OK) {
+            a.bias = i == 0 ? bias : nullptr;
+            a.status = status;
+            rc = launch_any(vs[i].type, plan, a, map, s);
+        }
     }
-    Args a = {};
-    Plan plan = {};
-    weight_args(v, a);
-    choose(v.type, false, false, v.n, a.kb, (int)m, a, plan);
-    int rc = status_word(&a.status);
-    CUtensorMap map;
-    if (rc == JQ_OK) {
-        rc = activation_map(&map, true, x_bf16, v.k, m, 1, a.nt);
-    }
-    if (rc != JQ_OK) {
-        return rc;
-    }
-    a.features = v.n;
-    a.bias = bias;
-    a.y = y;
-    return launch_any(v.type, plan, a, map, s);
+    return rc;
+}
+
+int launch_prefill_bf16(const View& v, const uint16_t* x_bf16, int64_t m, const float* bias, float* y, cudaStream_t s) {
+    return launch_prefill_bf16_multi(&v, 1, x_bf16, m, bias, &y, s);
 }
 
 EncodeTiledFn encode_tiled() {

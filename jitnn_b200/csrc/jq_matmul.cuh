@@ -63,11 +63,18 @@ constexpr int MAX_A = 6, MAX_B = 12, MAX_RAW = 6;
 constexpr int FACTORS = 8;   // units whose factors the fold may still need: operands in flight and accumulators, see where they are written
 constexpr int VIRTUAL = 8;   // ranges of the contraction whose sums are added up in order, whatever the cluster (instances for 16 rows of x)
 
+constexpr int MAX_WEIGHTS = 3;
+
 struct Args {
-    const uint8_t* q;
-    const uint8_t* aux;
+    // Up to three weights of one format and k, whose tiles of features follow one another. Linears on one x (q, k and v; gate and up) leave
+    // the chip partly idle one by one: 32 or 86 tiles of features on 148 SMs, each launch with a fill and a drain. Together: prompt of 512
+    // tokens, 8 layers of the 7B width, 2529 -> 2437 us; 16 sequences at the 70B width, 626 -> 588 us.
+    const uint8_t* q[MAX_WEIGHTS];
+    const uint8_t* aux[MAX_WEIGHTS];
+    float* y[MAX_WEIGHTS];
+    int64_t features[MAX_WEIGHTS];  // valid features, and the row length of y
+    int ft_end[MAX_WEIGHTS];        // tiles of features up to and including each weight
     int kb;           // 256-wide steps of k in the weight
-    int rows128;      // 128-row tiles of the weight
     int units;        // units along the contraction
     int ftiles;       // tiles of 128 features
     int ttiles, nt;   // tiles of nt rows of x
@@ -78,11 +85,9 @@ struct Args {
     int cols;         // tensor-memory columns of one accumulator
     int bufs;         // accumulators: 2, or 1 where a second one does not fit
     int tmem;         // columns to allocate
-    int64_t features; // valid features, and the row length of y
     const float* xscale;  // FP32: scale of (contraction block, row of x): [block][xstride]
     int xstride;
-    const float* bias;
-    float* y;
+    const float* bias;    // of the first weight, or null
     int* status;      // 0, or the code of the first wait that gave up: 1 operand free, 2 weights ready, 3 activations ready or their tile free,
                       // 4 accumulator ready, 5 accumulator free, 6 raw blocks, 8 raw blocks read by all
 };
@@ -110,6 +115,17 @@ __device__ __forceinline__ void mma_ta(uint32_t d, uint32_t a, uint32_t b, uint3
         "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t}" ::"r"(d),
         "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "r"(DESC_HI)
         : "memory");
+}
+
+// Which weight a tile of features belongs to, and the first tile of that weight.
+__device__ __forceinline__ int weight_of(const Args& p, int ft, int& ft0) {
+    const int w = ft < p.ft_end[0] ? 0 : (ft < p.ft_end[1] ? 1 : 2);
+    ft0 = w == 0 ? 0 : (w == 1 ? p.ft_end[0] : p.ft_end[1]);
+    return w;
+}
+template <typename T>
+__device__ __forceinline__ T pick(const T (&v)[MAX_WEIGHTS], int w) {
+    return w == 0 ? v[0] : (w == 1 ? v[1] : v[2]);
 }
 
 __device__ __forceinline__ bool elect_one() {
@@ -467,16 +483,20 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
             bool ok = true;
             for (int tile = cluster_id; tile < tiles && ok; tile += clusters) {
                 const int ft = tile / p.ttiles;
+                int ft0;
+                const int wi = weight_of(p, ft, ft0);
+                const uint8_t* const wq = pick(p.q, wi);
+                const uint8_t* const wa = pick(p.aux, wi);
                 for (int u = u0; u < u1; u++) {
-                    const int64_t at = BWD ? (int64_t)u * p.kb + (ft >> 1) : (int64_t)ft * p.kb + u;
+                    const int64_t at = BWD ? (int64_t)u * p.kb + (ft >> 1) : (int64_t)(ft - ft0) * p.kb + u;
                     if (!(ok = wait(raw_read + 8 * r, ph, abort_flag, p.status, 8))) {
                         break;
                     }
                     const uint32_t dst = raw0 + (uint32_t)r * raw_bytes<TYPE>(), bar = raw_full + 8 * r;
                     tc::mbar_expect_tx(bar, raw_bytes<TYPE>());
-                    tc::bulk_load(dst, p.q + at * D::UNIT_Q, D::UNIT_Q, bar);
+                    tc::bulk_load(dst, wq + at * D::UNIT_Q, D::UNIT_Q, bar);
                     if constexpr (D::UNIT_A > 0) {
-                        tc::bulk_load(dst + D::UNIT_Q, p.aux + at * D::UNIT_A, D::UNIT_A, bar);
+                        tc::bulk_load(dst + D::UNIT_Q, wa + at * D::UNIT_A, D::UNIT_A, bar);
                     }
                     if (++r == R) {
                         r = 0;
@@ -680,13 +700,15 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
         };
         for (int tile = cluster_id; tile < tiles && ok; tile += clusters) {
             const int ft = tile / p.ttiles, t0 = (tile % p.ttiles) * nt;
-            const int64_t feature = (int64_t)ft * 128 + lane_row;
-            const bool valid = feature < p.features;
-            const float bias = p.bias != nullptr && valid ? __ldg(p.bias + feature) : 0.0f;
+            int ft0;
+            const int wi = weight_of(p, ft, ft0);
+            const int64_t feature = (int64_t)(ft - ft0) * 128 + lane_row, features = pick(p.features, wi);
+            const bool valid = feature < features;
+            const float bias = p.bias != nullptr && wi == 0 && valid ? __ldg(p.bias + feature) : 0.0f;
             // Columns c .. c + 7 of the tile are finished: to y, or (contraction split over the cluster) to this CTA's own partial tile
             // [column][128]. One warp per scheduler does this, so it is kept short: no test per value where the tile is whole.
-            const int64_t row_bytes = p.features * 4;
-            uint8_t* const yt = reinterpret_cast<uint8_t*>(p.y + (int64_t)t0 * p.features + feature);
+            const int64_t row_bytes = features * 4;
+            uint8_t* const yt = reinterpret_cast<uint8_t*>(pick(p.y, wi) + (int64_t)t0 * features + feature);
             const bool whole = t0 + nt <= p.m;
             auto emit8 = [&](int c, const float (&v)[8]) {
                 if (p.ksplit > 1) {
@@ -873,7 +895,11 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
     if (p.ksplit > 1 && *abort_flag == 0) {
         // columns range, range + ksplit, .. of the tile: the (virtual) ranges' sums in order
         const int ft = cluster_id / p.ttiles, t0 = (cluster_id % p.ttiles) * nt;
-        const int64_t f0 = (int64_t)ft * 128;
+        int ft0;
+        const int wi = weight_of(p, ft, ft0);
+        const int64_t f0 = (int64_t)(ft - ft0) * 128, features = pick(p.features, wi);
+        float* const y = pick(p.y, wi);
+        const float* const bias = wi == 0 ? p.bias : nullptr;
         const int mine = (nt - range + p.ksplit - 1) / p.ksplit * 32;  // pieces of four features of a column
         constexpr int BATCH = 2, MOST = 4;  // pieces and ranges in flight: another CTA's memory is most of a microsecond away
         const int parts = CANON ? VIRTUAL : p.ksplit, per_cta = parts / p.ksplit;
@@ -916,19 +942,19 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                 if (i >= mine || t0 + col >= p.m) {
                     continue;
                 }
-                float* const at = p.y + (int64_t)(t0 + col) * p.features + f;
+                float* const at = y + (int64_t)(t0 + col) * features + f;
                 const float one[4] = {sum[j].x, sum[j].y, sum[j].z, sum[j].w};
-                if (f + 4 <= p.features && ((uintptr_t)at & 15) == 0) {
+                if (f + 4 <= features && ((uintptr_t)at & 15) == 0) {
                     float4 b = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    if (p.bias != nullptr) {
-                        b = make_float4(__ldg(p.bias + f), __ldg(p.bias + f + 1), __ldg(p.bias + f + 2), __ldg(p.bias + f + 3));
+                    if (bias != nullptr) {
+                        b = make_float4(__ldg(bias + f), __ldg(bias + f + 1), __ldg(bias + f + 2), __ldg(bias + f + 3));
                     }
                     *reinterpret_cast<float4*>(at) = make_float4(one[0] + b.x, one[1] + b.y, one[2] + b.z, one[3] + b.w);
                 } else {
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
-                        if (f + q < p.features) {
-                            at[q] = one[q] + (p.bias != nullptr ? __ldg(p.bias + f + q) : 0.0f);
+                        if (f + q < features) {
+                            at[q] = one[q] + (bias != nullptr ? __ldg(bias + f + q) : 0.0f);
                         }
                     }
                 }

@@ -1,0 +1,61 @@
+"""The captured decode steps where one range of cached positions ends and the next begins, and the page-locked logits arrays."""
+import numpy as np
+import pytest
+
+import jitnn_b200
+from jitnn_b200 import LlamaDecoder
+from oracle import llama_oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def build(heads, kv_heads, head_dim, max_seq, seed=5):
+    dim = heads * head_dim
+    cfg = llama_oracle.Config(layers=2, dim=dim, heads=heads, kv_heads=kv_heads, hidden=2 * dim, vocab=8192, max_seq=max_seq)
+    dec = LlamaDecoder(cfg.layers, cfg.dim, cfg.heads, cfg.kv_heads, cfg.hidden, cfg.vocab, cfg.max_seq, cfg.eps, cfg.rope_base)
+    dec.load(llama_oracle.random_model(cfg, seed))
+    return dec
+
+
+# a graph covers up to 256, 512, ... positions; one, two, four and eight query heads per key/value head; both head sizes; one row and several
+@pytest.mark.parametrize("heads,kv_heads,head_dim,n_seqs", [(2, 2, 128, 1), (4, 2, 128, 1), (4, 2, 128, 3), (4, 1, 64, 2), (8, 1, 128, 2)])
+def test_captured_steps_across_ranges(heads, kv_heads, head_dim, n_seqs):
+    toks = np.random.default_rng(1).integers(0, 8192, (516, n_seqs)).astype(np.int32)
+    out = []
+    for graph in (0, 1):
+        jitnn_b200.load().jq_set_option(b"decoder_graph", graph)
+        try:
+            dec = build(heads, kv_heads, head_dim, 516)
+            if n_seqs > 1:
+                dec.set_sequences(n_seqs)
+            got = []
+            for pos in range(516):
+                lg, nxt = dec.forward(toks[pos], pos) if n_seqs == 1 else dec.forward_batch(toks[pos], pos)
+                if pos in (0, 63, 64, 254, 255, 256, 257, 511, 512, 515):
+                    got.append(np.array(lg))
+                    assert np.array_equal(nxt, np.argmax(lg, axis=1))
+            out.append(got)
+            dec.close()
+        finally:
+            jitnn_b200.load().jq_set_option(b"decoder_graph", 1)
+    # The two forms cut the keys into chunks alike but launch a different number of them; merging an empty chunk multiplies by one and adds
+    # zero, so only FP32 rounding in the merge may differ: 2e-4 of the largest logit is the decoder's own bar.
+    for a, b in zip(*out):
+        assert np.abs(a - b).max() <= 2e-4 * np.abs(a).max()
+
+
+def test_logits_arrays_stay_valid():
+    """More arrays held than page-locked blocks exist; each keeps its step's values, also after the decoder is closed."""
+    dec = build(4, 2, 64, 32)
+    held, copies = [], []
+    for pos in range(9):
+        lg, _ = dec.forward([pos + 1], pos)
+        held.append(lg)
+        copies.append(lg.copy())
+    del held[2], copies[2]  # its block is free for the next step
+    lg, _ = dec.forward([3], 9)
+    held.append(lg)
+    copies.append(lg.copy())
+    dec.close()
+    for a, b in zip(held, copies):
+        assert np.array_equal(a, b)
