@@ -1436,16 +1436,43 @@ static int enqueue_forward_fused(jq_decoder* d, int max_keys, const TokenArgs* t
     const size_t norm_smem = (size_t)(dim / norm_ctas) * sizeof(float);
     const dim3 norm_block((unsigned)(dim / norm_ctas / 4));
     const int splits_now = (max_keys + ATT_CHUNK - 1) / ATT_CHUNK;
+    // The residual stream. A norm whose linears' first is Q4_K is made inside that launch, which leaves x + delta in the other buffer.
+    float *x = d->x, *x_other = d->xn;
+    auto NORMED = [&](const float* norm_w, const jq_weight* const* w, int count, float* const* ys, uint8_t* q6k) {
+        View vs[3];
+        for (int i = 0; i < count; i++) {
+            vs[i] = View{w[i]->q, w[i]->aux, w[i]->n, w[i]->k, w[i]->type};
+        }
+        const NormInput in{x, d->proj, norm_w, d->eps, x_other, d->att, q6k};
+        bool handled = false;
+        if (rc == JQ_OK) {
+            rc = launch_gemv_q4k_i8_normed(vs, count, in, ys, s, &handled);
+        }
+        if (handled) {
+            std::swap(x, x_other);
+        }
+        return handled;
+    };
+    float* const qkv[3] = {d->q, d->k, d->v};
+    float* const gate_up[2] = {d->gate, d->up};
     for (int l = 0; l < d->layers && rc == JQ_OK; l++) {
         const jq_weight* const* L = &d->lin[(size_t)l * 7];
         float* kc = d->k_cache + seq_base + (size_t)l * d->max_seq * kv_dim;
         float* vc = d->v_cache + seq_base + (size_t)l * d->max_seq * kv_dim;
         // attention block: x = embedding (first layer) or x += feed-forward output of the layer before; norm -> images
-        CKL(launch_cluster_pdl(norm_image_kernel, norm_ctas, norm_block, norm_smem, s, l > 0 || first_programmatic, d->x, l == 0 ? nullptr : d->proj,
-                       l == 0 ? d->embed : nullptr, d->tokens, d->vocab, d->norms + (size_t)(2 * l) * dim, d->eps, dim, images_for({L[0], L[1], L[2]}), (const uint32_t*)nullptr, 0),
-            "norm_image_kernel");
-        if (rc == JQ_OK) {
-            rc = decoder_gemv_imaged3(d, L[0], d->q, L[1], d->k, L[2], d->v, s);
+        const bool all_q4k = L[2]->type == JQ_TYPE_Q4_K;
+        if (l > 0 && NORMED(d->norms + (size_t)(2 * l) * dim, L, all_q4k ? 3 : 2, qkv, all_q4k ? nullptr : d->img_q6k)) {
+            if (!all_q4k) {
+                GEMV(L[2], d->v, nullptr, nullptr, s);
+            }
+        } else {
+            CKL(launch_cluster_pdl(norm_image_kernel, norm_ctas, norm_block, norm_smem, s, l > 0 || first_programmatic, x, l == 0 ? nullptr : d->proj,
+                                   l == 0 ? d->embed : nullptr, d->tokens, d->vocab, d->norms + (size_t)(2 * l) * dim, d->eps, dim,
+                                   images_for({L[0], L[1], L[2]}), (const uint32_t*)nullptr, 0),
+                "norm_image_kernel");
+            if (rc == JQ_OK) {
+                rc = decoder_gemv_imaged3(d, L[0], d->q, L[1], d->k, L[2], d->v, s);
+            }
         }
         if (rc != JQ_OK) break;
         CKL(launch_pdl(attention_image_kernel<false>, dim3(d->heads, splits_now), dim3(ATTF_THREADS), 0, s, true, d->q, d->k, d->v, kc, vc, d->cos_t, d->sin_t, d->pos,
@@ -1454,16 +1481,18 @@ static int enqueue_forward_fused(jq_decoder* d, int max_keys, const TokenArgs* t
         GEMV(L[3], d->proj, nullptr, nullptr, s);
         if (rc != JQ_OK) break;
         // feed-forward block
-        CKL(launch_cluster_pdl(norm_image_kernel, norm_ctas, norm_block, norm_smem, s, true, d->x, d->proj, nullptr, d->tokens, d->vocab,
-                       d->norms + (size_t)(2 * l + 1) * dim, d->eps, dim, images_for({L[4], L[5]}), (const uint32_t*)nullptr, 0),
-            "norm_image_kernel");
-        GEMV(L[4], d->gate, L[5], d->up, s);
+        if (!NORMED(d->norms + (size_t)(2 * l + 1) * dim, L + 4, 2, gate_up, nullptr)) {
+            CKL(launch_cluster_pdl(norm_image_kernel, norm_ctas, norm_block, norm_smem, s, true, x, d->proj, nullptr, d->tokens, d->vocab,
+                                   d->norms + (size_t)(2 * l + 1) * dim, d->eps, dim, images_for({L[4], L[5]}), (const uint32_t*)nullptr, 0),
+                "norm_image_kernel");
+            GEMV(L[4], d->gate, L[5], d->up, s);
+        }
         if (rc != JQ_OK) break;
         CKL(launch_pdl(swiglu_image_kernel<false>, dim3(d->hidden / 256), dim3(256), 0, s, true, d->gate, d->up, images_for({L[6]}), PeerImage{}, d->hidden / 256), "swiglu_image_kernel");
         GEMV(L[6], d->proj, nullptr, nullptr, s);
     }
     if (rc == JQ_OK) {
-        CKL(launch_cluster_pdl(norm_image_kernel, norm_ctas, norm_block, norm_smem, s, true, d->x, d->proj, nullptr, d->tokens, d->vocab,
+        CKL(launch_cluster_pdl(norm_image_kernel, norm_ctas, norm_block, norm_smem, s, true, x, d->proj, nullptr, d->tokens, d->vocab,
                        d->norms + (size_t)(2 * d->layers) * dim, d->eps, dim, images_for({d->output}), (const uint32_t*)nullptr, 0),
             "norm_image_kernel");
         GEMV(d->output, d->logits, nullptr, nullptr, s);

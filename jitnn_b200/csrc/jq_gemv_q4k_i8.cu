@@ -38,6 +38,7 @@
 #include "jq_formats.cuh"
 #include "jq_peer_device.cuh"
 #include "jq_q4k_image.cuh"
+#include "jq_q6k_image.cuh"
 #include "jq_tc.cuh"
 
 namespace jq {
@@ -137,14 +138,21 @@ struct Second {
     int second_tiles;  // tiles of the first and the second weight
 };
 
+// Where the image comes from: written by a kernel earlier in the stream; made by every warp for its own super-blocks from x as floats; or
+// (one row) from the RMSNorm of x + delta, which every CTA computes for itself.
+enum From { FROM_IMAGE, FROM_FLOATS, FROM_NORM };
+
 // PEER: the outputs go into every rank's y of a row-sharded linear (jq_peer.cu) instead of y. A template flag, not a
 // run-time branch: the mere presence of the peer stores in the epilogue cost the ordinary kernel a fifth of its speed.
-// FUSED: `xin` holds the rows of x as floats and every warp builds the image of its own super-blocks; otherwise `image`
-// holds the image, written by a kernel earlier in the stream.
-template <int MT, int STAGES, int NW, int OCC, bool Q5, bool PEER, bool FUSED>
+// FROM_FLOATS: `xin` holds the rows of x as floats; FROM_IMAGE: `image` holds the image; FROM_NORM: `norm` says what to read.
+// The norm in here costs a CTA the load of two vectors and a barrier, about what the load of the image costs it, and saves a kernel whose
+// only work is 16 KB, on a chain where every kernel takes more than four microseconds whatever its size (one token, 8 layers of the 7B width
+// at position 576: 530 -> 493 us). Up to NORM_MAX super-blocks a warp, that is k <= 8192; their values stay in registers.
+constexpr int NORM_MAX = 4;
+template <int MT, int STAGES, int NW, int OCC, bool Q5, bool PEER, From SRC>
 __global__ void __launch_bounds__(NW * 32, OCC) gemv_q4k_i8_kernel(View v, Second w2, const PeerOut* __restrict__ peerp, const uint8_t* __restrict__ image,
                                                                   const float* __restrict__ xin, int rows, const float* __restrict__ bias, float* __restrict__ y,
-                                                                  int tiles, int KS, int max_tiles, long long wait_clocks) {
+                                                                  int tiles, int KS, int max_tiles, long long wait_clocks, NormInput norm) {
     // Tiles 0 .. w2.first_tiles - 1 are rows of v, the tiles from w2.first_tiles on rows of the second weight w2 (same k,
     // same x, its own output), if there is one.
     // KS = super-blocks of k per slice: the activation image of one slice is resident in shared memory at a time;
@@ -231,6 +239,15 @@ __global__ void __launch_bounds__(NW * 32, OCC) gemv_q4k_i8_kernel(View v, Secon
 #pragma unroll
     for (int s = 0; s < STAGES - 1; s++) {
         issue();  // the first weights are on their way before x or the activation image is complete
+    }
+
+    float norm_w[SRC == FROM_NORM ? NORM_MAX : 1][8];
+    if constexpr (SRC == FROM_NORM) {  // the norm's weights never change
+#pragma unroll
+        for (int j = 0; j < NORM_MAX; j++) {
+            const int b = warp + NW * j;
+            q4k::load_image_values(b < KB ? norm.w + b * 256 : nullptr, lane, norm_w[j]);
+        }
     }
 
     // ---- x (or the image made from it) is complete once the kernel before this one has finished --------------------------
@@ -397,7 +414,60 @@ __global__ void __launch_bounds__(NW * 32, OCC) gemv_q4k_i8_kernel(View v, Secon
         // ---- this slice of the activation image in shared memory ---------------------------------------------------------
         const int len = sl == nslices - 1 ? len_last : KS;
         const int nb = sl == nslices - 1 ? nb_last : nb_full;
-        if constexpr (FUSED) {
+        if constexpr (SRC == FROM_NORM) {  // one slice
+            float a[NORM_MAX][8], sq = 0.0f;
+#pragma unroll
+            for (int j = 0; j < NORM_MAX; j++) {
+                const int b = warp + NW * j;
+                float dl[8];
+                q4k::load_image_values(b < KB ? norm.x + b * 256 : nullptr, lane, a[j]);
+                q4k::load_image_values(b < KB ? norm.delta + b * 256 : nullptr, lane, dl);
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    a[j][i] += dl[i];
+                    sq = fmaf(a[j][i], a[j][i], sq);
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                sq += __shfl_xor_sync(0xffffffffu, sq, o);
+            }
+            float* const partial = red + NW * 16 * MT;  // (the half that the second tile is the first to use)
+            if (lane == 0) {
+                partial[warp] = sq;
+            }
+            __syncthreads();
+            float total = 0.0f;
+#pragma unroll
+            for (int i = 0; i < NW; i++) {
+                total += partial[i];
+            }
+            const float inv = 1.0f / sqrtf(total / (float)(int)v.k + norm.eps);
+            const bool keeps = blockIdx.x == gridDim.x - 1;  // this CTA writes what others need (it is among those with the fewest tiles)
+#pragma unroll
+            for (int j = 0; j < NORM_MAX; j++) {
+                const int b = warp + NW * j;
+                if (b < KB) {
+                    if (keeps) {
+                        float4* const to = reinterpret_cast<float4*>(norm.x_out + b * 256) + 2 * lane;
+                        to[0] = make_float4(a[j][0], a[j][1], a[j][2], a[j][3]);
+                        to[1] = make_float4(a[j][4], a[j][5], a[j][6], a[j][7]);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        a[j][i] = a[j][i] * inv * norm_w[j][i];
+                    }
+                    q4k::build_image_from<MT>(a[j], true, 0, img + (size_t)b * C::PB, lane);
+                    if (keeps && norm.q6k != nullptr) {
+                        float4* const to = reinterpret_cast<float4*>(norm.scratch + b * 256) + 2 * lane;
+                        to[0] = make_float4(a[j][0], a[j][1], a[j][2], a[j][3]);
+                        to[1] = make_float4(a[j][4], a[j][5], a[j][6], a[j][7]);
+                        q6k::build_image<1>(norm.scratch + b * 256, 0, norm.q6k + (size_t)b * q6k::Cfg<1>::PB, lane);  // (a lane reads what it wrote)
+                    }
+                }
+            }
+            __syncwarp();
+        } else if constexpr (SRC == FROM_FLOATS) {
             // a warp only ever reads the image of its own super-blocks, so it makes just those and waits for nobody
             __syncwarp();  // the warp's lanes are done with the previous slice
             // two (super-block, row) parts at a time, so that the loads of the second are in flight while the first is made
@@ -580,14 +650,14 @@ int sm_count() {
     return g_sms;
 }
 
-template <int MT, int STAGES, int NW, int OCC, bool Q5, bool PEER, bool FUSED>
+template <int MT, int STAGES, int NW, int OCC, bool Q5, bool PEER, From SRC>
 int launch(const View& v, const Second& w2, const PeerOut& peer, const uint8_t* image, const float* x, int rows, const float* bias, float* y, cudaStream_t s,
-           int KS, int grid, int max_tiles, size_t smem) {
+           int KS, int grid, int max_tiles, size_t smem, const NormInput& norm) {
     static std::atomic<uint64_t> configured{0};  // the opt-in for large dynamic shared memory is per device
     int dev = 0;
     JQ_CUDA(cudaGetDevice(&dev));
     if ((configured.load() >> (dev & 63) & 1) == 0) {
-        JQ_CUDA(cudaFuncSetAttribute(gemv_q4k_i8_kernel<MT, STAGES, NW, OCC, Q5, PEER, FUSED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
+        JQ_CUDA(cudaFuncSetAttribute(gemv_q4k_i8_kernel<MT, STAGES, NW, OCC, Q5, PEER, SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
         configured.fetch_or((uint64_t)1 << (dev & 63));
     }
     const int tiles = (int)((v.n + 15) / 16) + (w2.q != nullptr ? (int)((w2.n + 15) / 16) : 0) + (w2.q3 != nullptr ? (int)((w2.n3 + 15) / 16) : 0);
@@ -602,8 +672,8 @@ int launch(const View& v, const Second& w2, const PeerOut& peer, const uint8_t* 
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const long long wait_clocks = (long long)g_opt_wait_limit_us.load(std::memory_order_relaxed) * 2000;  // about 2 GHz
-    JQ_CUDA(cudaLaunchKernelEx(&cfg, gemv_q4k_i8_kernel<MT, STAGES, NW, OCC, Q5, PEER, FUSED>, v, w2, (const PeerOut*)(PEER ? peer.table : nullptr), image, x, rows,
-                               bias, y, tiles, KS, max_tiles, wait_clocks));
+    JQ_CUDA(cudaLaunchKernelEx(&cfg, gemv_q4k_i8_kernel<MT, STAGES, NW, OCC, Q5, PEER, SRC>, v, w2, (const PeerOut*)(PEER ? peer.table : nullptr), image, x, rows,
+                               bias, y, tiles, KS, max_tiles, wait_clocks, norm));
     count_launch();
     return JQ_OK;
 }
@@ -624,7 +694,7 @@ struct Shape {
 
 template <int MT, bool Q5>
 int run(const View& v, const Second& w2, const PeerOut& peer, const float* x, int rows, const float* bias, float* y, cudaStream_t s, uint8_t* image,
-        bool* handled, bool may_fuse) {
+        bool* handled, bool may_fuse, const NormInput* norm = nullptr) {
     // x == nullptr: the image is already in `image` (written by a kernel earlier in the stream)
     const int KB = (int)(v.k / 256);
     const int tiles = (int)((v.n + 15) / 16) + (w2.q != nullptr ? (int)((w2.n + 15) / 16) : 0) + (w2.q3 != nullptr ? (int)((w2.n3 + 15) / 16) : 0);
@@ -670,7 +740,11 @@ int run(const View& v, const Second& w2, const PeerOut& peer, const float* x, in
     // x lies in host memory: the image kernel reads it once, the thread blocks of the GEMV would each read it across PCIe.
     // With three to eight rows a warp would build eight parts for k = 4096, each behind a load of x from L2 (about 0.7
     // microseconds, two in flight): measured 3 microseconds slower per launch than the image kernel, so those rows keep it.
-    constexpr bool CAN_FUSE = !WIDE;
+    constexpr bool CAN_FUSE = !WIDE, CAN_NORM = MT == 1 && !Q5;
+    if (norm != nullptr && (!CAN_NORM || is_sliced || KB > NORM_MAX * sh.nw || peer.world != 0)) {
+        *handled = false;
+        return JQ_OK;
+    }
     const bool fuse = CAN_FUSE && may_fuse && x != nullptr && KB <= 4 * sh.nw;
     if (x != nullptr && !fuse) {
         // launched programmatically as well: it is scheduled while the kernel before it still runs (it waits for that kernel
@@ -687,14 +761,20 @@ int run(const View& v, const Second& w2, const PeerOut& peer, const float* x, in
         JQ_CUDA(cudaLaunchKernelEx(&icfg, q4k_activation_image_kernel<MT>, x, rows, (int64_t)v.k, image));
         count_launch();
     }
+    const NormInput no_norm{};
 #define JQ_VARIANT(NWV, OCCV, STV, PEERV)                                                                                               \
-    if constexpr (CAN_FUSE) {                                                                                                            \
-        if (fuse) {                                                                                                                      \
-            return launch<MT, STV, NWV, OCCV, Q5, PEERV, true>(v, w2, peer, image, x, rows, bias, y, s, KS, grid, max_tiles, smem);      \
-        }                                                                                                                                \
-    }                                                                                                                                    \
-    if constexpr (true) {                                                                                                                \
-        return launch<MT, STV, NWV, OCCV, Q5, PEERV, false>(v, w2, peer, image, nullptr, rows, bias, y, s, KS, grid, max_tiles, smem);   \
+    if constexpr (CAN_NORM && !PEERV) {                                                                                                                  \
+        if (norm != nullptr) {                                                                                                                           \
+            return launch<MT, STV, NWV, OCCV, Q5, PEERV, FROM_NORM>(v, w2, peer, image, nullptr, rows, bias, y, s, KS, grid, max_tiles, smem, *norm);    \
+        }                                                                                                                                                \
+    }                                                                                                                                                    \
+    if constexpr (CAN_FUSE) {                                                                                                                            \
+        if (fuse) {                                                                                                                                      \
+            return launch<MT, STV, NWV, OCCV, Q5, PEERV, FROM_FLOATS>(v, w2, peer, image, x, rows, bias, y, s, KS, grid, max_tiles, smem, no_norm);      \
+        }                                                                                                                                                \
+    }                                                                                                                                                    \
+    if constexpr (true) {                                                                                                                                \
+        return launch<MT, STV, NWV, OCCV, Q5, PEERV, FROM_IMAGE>(v, w2, peer, image, nullptr, rows, bias, y, s, KS, grid, max_tiles, smem, no_norm);     \
     }
 #define JQ_SHAPE(NWV, OCCV, STV)                                   \
     if (sh.nw == NWV && sh.occ == OCCV && sh.stages == STV) {       \
@@ -817,6 +897,22 @@ int launch_gemv_q4k_i8_imaged(const View& v, const View* v2, const uint8_t* imag
         return JQ_OK;  // a second weight has no place in a peer's y
     }
     return run<1, false>(v, w2, peer != nullptr ? *peer : local, nullptr, 1, bias, y, s, const_cast<uint8_t*>(image), handled, false);
+}
+
+// One row of x that is the RMSNorm of a vector and a delta (NormInput), up to three Q4_K weights of one k <= 8192.
+int launch_gemv_q4k_i8_normed(const View* vs, int count, const NormInput& norm, float* const* ys, cudaStream_t s, bool* handled) {
+    *handled = false;
+    const View& v = vs[0];
+    for (int i = 0; i < count; i++) {
+        if (vs[i].type != JQ_TYPE_Q4_K || vs[i].k != v.k || vs[i].n == 0 || vs[i].k == 0 || vs[i].k > 8192) {
+            return JQ_OK;
+        }
+    }
+    const int t1 = (int)((v.n + 15) / 16), t2 = count > 1 ? t1 + (int)((vs[1].n + 15) / 16) : 0;
+    const Second w2{count > 1 ? vs[1].q : nullptr, count > 1 ? vs[1].n : 0, count > 1 ? ys[1] : nullptr, count > 1 ? t1 : 0x7fffffff,
+                    count > 2 ? vs[2].q : nullptr, count > 2 ? vs[2].n : 0, count > 2 ? ys[2] : nullptr, count > 2 ? t2 : 0x7fffffff};
+    const PeerOut local{};
+    return run<1, false>(v, w2, local, nullptr, 1, nullptr, ys[0], s, nullptr, handled, false, &norm);
 }
 
 }  // namespace jq
