@@ -300,8 +300,9 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_partial_kernel(const fl
 // The same for head sizes 64 and 128, all query heads that share a key/value head in one CTA: CTA (kv head, split, t) has its 64 keys and values
 // in registers (warp w keys 8w .. 8w + 7, a lane HD / 32 neighbouring dimensions of each) and goes through the group's query heads. With one CTA
 // per query head, a group of eight read every cached byte eight times, and the dot products' shuffles, five per key, bound it (16 sequences of
-// 64 heads at position 256: 55 us).
-constexpr int GROUP_THREADS = 256;
+// 64 heads at position 256: 55 us). The warps go through up to GROUP_HEADS heads on their own and meet once for all of them: with a barrier and
+// a merge for each head the kernel was a chain of those (587.5 us against 582.9 for a step of 16 sequences, 2 layers of the 70B width).
+constexpr int GROUP_THREADS = 256, GROUP_HEADS = 8;
 template <int HD>
 __global__ void __launch_bounds__(GROUP_THREADS) attention_group_kernel(const float* __restrict__ q, const float* __restrict__ k_cache,
                                                                        const float* __restrict__ v_cache, float* __restrict__ part,
@@ -311,8 +312,8 @@ __global__ void __launch_bounds__(GROUP_THREADS) attention_group_kernel(const fl
     asm volatile("griddepcontrol.wait;" ::: "memory");
     static_assert(HD == 64 || HD == 128, "head sizes");
     constexpr int V = HD / 32;
-    __shared__ float red[2][8][HD];
-    __shared__ float stat[2][16];
+    __shared__ __align__(16) float red[GROUP_HEADS][8][HD];
+    __shared__ float stat[GROUP_HEADS][16];  // the warps' maxima, later their weights; their sums
     const int kvh = blockIdx.x, sp = blockIdx.y, t = blockIdx.z, group = heads / kv_heads;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int keys = *pos0 + t * pos_step + 1, k0 = sp * ATT_CHUNK;
@@ -416,37 +417,55 @@ __global__ void __launch_bounds__(GROUP_THREADS) attention_group_kernel(const fl
                 acc[i] = fmaf(w, vr[u][i], acc[i]);
             }
         }
-        const int buf = hh & 1;  // (a buffer is written again only behind the next head's barrier)
-#pragma unroll
-        for (int i = 0; i < V; i++) {
-            red[buf][warp][lane * V + i] = acc[i];
+        const int at = hh % GROUP_HEADS;
+        if constexpr (V == 4) {
+            reinterpret_cast<float4*>(red[at][warp])[lane] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        } else {
+            reinterpret_cast<float2*>(red[at][warp])[lane] = make_float2(acc[0], acc[1]);
         }
         if (lane == 0) {
-            stat[buf][warp] = mw;
-            stat[buf][8 + warp] = lw;
+            stat[at][warp] = mw;
+            stat[at][8 + warp] = lw;
+        }
+        if (at < GROUP_HEADS - 1 && hh < group - 1) {
+            continue;
+        }
+        // the 8 warps' results of heads hh - at .. hh, added up in warp order
+        __syncthreads();
+        float* const out = out0 + (hh - at) * head_stride;
+        if (tid < GROUP_HEADS * 8) {  // (whole warps; what lies in the places of heads beyond `at` goes nowhere)
+            const int w = tid & 7;
+            float* const st = stat[tid >> 3];
+            const float m = st[w];
+            float M = m;
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) {
+                M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+            }
+            const float wgt = expf(m - M);  // 0 for a warp without keys (warp 0 always has one)
+            float l = wgt * st[8 + w];
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) {
+                l += __shfl_xor_sync(0xffffffffu, l, o);
+            }
+            st[w] = wgt;
+            if (w == 0 && (tid >> 3) <= at) {
+                out[(tid >> 3) * head_stride + HD] = M;
+                out[(tid >> 3) * head_stride + HD + 1] = l;
+            }
         }
         __syncthreads();
-        // the 8 warps' results in warp order
-        if (tid <= HD) {
-            float M = stat[buf][0];  // warp 0 always has a key
-#pragma unroll
-            for (int wv = 1; wv < 8; wv++) {
-                M = fmaxf(M, stat[buf][wv]);
-            }
-            float sum = 0.0f, l = 0.0f;
+        for (int i = tid; i < (at + 1) * HD; i += GROUP_THREADS) {
+            const int head = i / HD, dd = i % HD;
+            float sum = 0.0f;
 #pragma unroll
             for (int wv = 0; wv < 8; wv++) {
-                const float wgt = expf(stat[buf][wv] - M);  // 0 for a warp without keys
-                l = fmaf(wgt, stat[buf][8 + wv], l);
-                sum = fmaf(wgt, red[buf][wv][tid & (HD - 1)], sum);
+                sum = fmaf(stat[head][wv], red[head][wv][dd], sum);
             }
-            float* const out = out0 + hh * head_stride;
-            if (tid < HD) {
-                out[tid] = sum;
-            } else {
-                out[HD] = M;
-                out[HD + 1] = l;
-            }
+            out[head * head_stride + dd] = sum;
+        }
+        if (hh < group - 1) {
+            __syncthreads();  // read by all before the next heads' results come
         }
     }
 }
