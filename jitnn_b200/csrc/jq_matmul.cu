@@ -1,6 +1,8 @@
 // Host side of the matrix kernel (jq_matmul.cuh): the split of FP32 activations, the choice of tiles, the launches.
 #include <cuda_bf16.h>
 
+#include <cstring>
+#include <memory>
 #include <mutex>
 
 #include "jq_matmul_launch.cuh"
@@ -179,8 +181,11 @@ static double unit_ns(int type, bool fp32, bool bwd, int nt) {
     return t < 1320.0 ? 1320.0 : t;
 }
 
+// Clusters of ks CTAs that run at a time, one CTA per SM (cudaOccupancyMaxActiveClusters; the SMs of a GPC are not all a multiple of 4 or 8).
+static int clusters_of(int ks) { return ks == 1 ? 148 : (ks == 2 ? 74 : (ks == 4 ? 33 : 15)); }
+
 // Tile width and ranges of the contraction for a product of `ftiles` tiles of features x m over `units` units.
-static void choose(int type, bool fp32, bool bwd, int64_t ftiles, int units, int m, Args& a, Plan& plan) {
+static double choose(int type, bool fp32, bool bwd, int64_t ftiles, int units, int m, Args& a, Plan& plan) {
     const int nmax = fp32 ? 128 : 256;
     double best = 1e30;
     int best_nt = 16, best_ks = 1;
@@ -197,14 +202,15 @@ static void choose(int type, bool fp32, bool bwd, int64_t ftiles, int units, int
             if (ks > 1 && units < 2 * ks) {
                 break;
             }
-            const int slots = (ks <= 2 ? 148 : (ks == 4 ? 144 : 128)) / ks;  // clusters at a time
+            const int slots = clusters_of(ks);  // clusters at a time
             if (ks > 1 && tiles > slots) {
                 break;  // more than one wave of whole tiles: nothing to gain
             }
             if (!configure(type, fp32, bwd, nt, ks, a, plan)) {
                 continue;
             }
-            const double waves = (double)((tiles + slots - 1) / slots);
+            // (a last wave that leaves SMs idle is a little faster: there is more of L2 and of the power for each CTA)
+            const double part = (double)(tiles % slots) / slots, waves = (double)(tiles / slots) + (part > 0.0 ? 0.9 + 0.1 * part : 0.0);
             const double cost = waves * (((units + ks - 1) / ks) * unit + 1500.0 + 12.0 * nt) + (ks > 1 ? 1500.0 + 6.0 * nt : 0.0);
             if (cost < best) {
                 best = cost;
@@ -220,6 +226,80 @@ static void choose(int type, bool fp32, bool bwd, int64_t ftiles, int units, int
     plan.ctas = best_ks > 1 || tiles < 148 ? tiles * best_ks : 148;
     a.units = units;
     a.m = m;
+    return best;
+}
+
+// A product may be cut by features into up to three launches, each with its own tiles: whole waves first, then what is left, which alone would
+// leave most of the chip idle for a whole contraction, with its contraction split over clusters. (57344 x 8192, 16 rows: 448 tiles are three
+// waves and four tiles: 93.8 us in one launch, 80.8 in two. Q4_K 11008 x 4096, 200 rows: 49.5 and 44.6; backward 4096 x 11008, 128 rows: 54.1 and
+// 51.0.) The launch behind waits for the one in front, fills and drains: GAP_NS, measured at 5 to 7 us. Finding the cut takes 10 to 35 us.
+constexpr int MAX_PARTS = 3;
+constexpr double GAP_NS = 7000.0;
+struct Part {
+    Args a;
+    Plan plan;
+};
+struct Parts {
+    int count;
+    Part part[MAX_PARTS];
+};
+static double cut(int type, bool fp32, bool bwd, int first_ft, int ftiles, int units, int m, int most, Parts& out) {
+    Parts best;
+    best.count = 1;
+    best.part[0] = Part{};
+    double cost = choose(type, fp32, bwd, ftiles, units, m, best.part[0].a, best.part[0].plan);
+    best.part[0].a.first_ft = first_ft;
+    if (most > 1) {
+        const int nmax = fp32 ? 128 : 256, least = (m + nmax - 1) / nmax;
+        for (int tt = least; tt <= least + 2; tt++) {  // tiles of rows of x in front
+            for (int ks = 1; ks <= 4; ks *= 2) {
+                const int slots = clusters_of(ks), waves = ks == 1 ? ftiles * tt / slots : 1, front = waves * slots / tt;
+                if (front < 1 || front >= ftiles) {
+                    continue;
+                }
+                Parts rest;
+                Part lead{};
+                const double c = choose(type, fp32, bwd, front, units, m, lead.a, lead.plan) + GAP_NS +
+                                 cut(type, fp32, bwd, first_ft + front, ftiles - front, units, m, most - 1, rest);
+                if (c < cost) {
+                    cost = c;
+                    lead.a.first_ft = first_ft;
+                    best.count = 1 + rest.count;
+                    best.part[0] = lead;
+                    for (int i = 0; i < rest.count; i++) {
+                        best.part[1 + i] = rest.part[i];
+                    }
+                }
+            }
+        }
+    }
+    out = best;
+    return cost;
+}
+
+// The same from a small table of the thread: a user's program asks for the same shapes again and again.
+static const Parts& parts_of(int type, bool fp32, bool bwd, int ftiles, int units, int m) {
+    struct Entry {
+        int key[6];
+        Parts parts;
+    };
+    constexpr int ENTRIES = 64;
+    static thread_local std::unique_ptr<Entry[]> table;
+    if (table == nullptr) {
+        table.reset(new Entry[ENTRIES]());
+    }
+    const int key[6] = {type + 1, fp32, bwd, ftiles, units, m};
+    uint32_t h = 0;
+    for (int v : key) {
+        h = (h ^ (uint32_t)v) * 0x9E3779B1u;
+        h ^= h >> 15;
+    }
+    Entry& e = table[h % ENTRIES];
+    if (memcmp(e.key, key, sizeof(key)) != 0) {
+        cut(type, fp32, bwd, 0, ftiles, units, m, MAX_PARTS, e.parts);
+        memcpy(e.key, key, sizeof(key));
+    }
+    return e.parts;
 }
 
 static int launch_any(int type, const Plan& plan, const Args& args, const CUtensorMap& map, cudaStream_t s) {
@@ -321,20 +401,22 @@ static int product_f32(const View* vs, int count, bool bwd, const float* x, int6
                     JQ_CUDA(cudaLaunchKernelEx(&cfg, split, xg, rows, width, per_row, reinterpret_cast<uint4*>(scratch), scales, stride, vec));
                     count_launch();
                 }
-                Args a = {};
-                Plan plan = {};
-                const int ftiles = weight_args(like, n_like, bwd, like_y, a);
-                choose(type, true, bwd, ftiles, bwd ? (int)(tiled_rows(vs[i].n) / TILE_ROWS) : a.kb, rows, a, plan);
-                CUtensorMap map;
-                rc = activation_map(&map, false, scratch, wpad, rows, 2, a.nt);
-                if (rc != JQ_OK) {
-                    break;
+                Args w = {};
+                const int ftiles = weight_args(like, n_like, bwd, like_y, w);
+                const Parts& parts = parts_of(type, true, bwd, ftiles, bwd ? (int)(tiled_rows(vs[i].n) / TILE_ROWS) : w.kb, rows);
+                for (int c = 0; c < parts.count && rc == JQ_OK; c++) {
+                    Args a = parts.part[c].a;
+                    weight_args(like, n_like, bwd, like_y, a);
+                    CUtensorMap map;
+                    rc = activation_map(&map, false, scratch, wpad, rows, 2, a.nt);
+                    if (rc == JQ_OK) {
+                        a.xscale = scales;
+                        a.xstride = stride;
+                        a.bias = bias;
+                        a.status = status;
+                        rc = launch_any(type, parts.part[c].plan, a, map, s);
+                    }
                 }
-                a.xscale = scales;
-                a.xstride = stride;
-                a.bias = bias;
-                a.status = status;
-                rc = launch_any(type, plan, a, map, s);
             }
         }
     }
@@ -401,16 +483,19 @@ int launch_prefill_bf16_multi(const View* vs, int count, const uint16_t* x_bf16,
         if (!first) {
             continue;
         }
-        Args a = {};
-        Plan plan = {};
-        const int ftiles = weight_args(like, n_like, false, like_y, a);
-        choose(vs[i].type, false, false, ftiles, a.kb, (int)m, a, plan);
-        CUtensorMap map;
-        rc = activation_map(&map, true, x_bf16, vs[i].k, m, 1, a.nt);
-        if (rc == JQ_OK) {
-            a.bias = i == 0 ? bias : nullptr;
-            a.status = status;
-            rc = launch_any(vs[i].type, plan, a, map, s);
+        Args w = {};
+        const int ftiles = weight_args(like, n_like, false, like_y, w);
+        const Parts& parts = parts_of(vs[i].type, false, false, ftiles, w.kb, (int)m);
+        for (int c = 0; c < parts.count && rc == JQ_OK; c++) {
+            Args a = parts.part[c].a;
+            weight_args(like, n_like, false, like_y, a);
+            CUtensorMap map;
+            rc = activation_map(&map, true, x_bf16, vs[i].k, m, 1, a.nt);
+            if (rc == JQ_OK) {
+                a.bias = i == 0 ? bias : nullptr;
+                a.status = status;
+                rc = launch_any(vs[i].type, parts.part[c].plan, a, map, s);
+            }
         }
     }
     return rc;

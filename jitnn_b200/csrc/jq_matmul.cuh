@@ -76,7 +76,7 @@ struct Args {
     int ft_end[MAX_WEIGHTS];        // tiles of features up to and including each weight
     int kb;           // 256-wide steps of k in the weight
     int units;        // units along the contraction
-    int ftiles;       // tiles of 128 features
+    int first_ft, ftiles;  // tiles of 128 features: those of this launch
     int ttiles, nt;   // tiles of nt rows of x
     int m;
     int ksplit;
@@ -482,7 +482,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
             uint32_t ph = 1;
             bool ok = true;
             for (int tile = cluster_id; tile < tiles && ok; tile += clusters) {
-                const int ft = tile / p.ttiles;
+                const int ft = p.first_ft + tile / p.ttiles;
                 int ft0;
                 const int wi = weight_of(p, ft, ft0);
                 const uint8_t* const wq = pick(p.q, wi);
@@ -518,7 +518,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
         bool ok = true, raw_ready = false;
         int first = OWNED ? 0 : group;  // the group's first turn of the unit, or of a later one
         for (int tile = cluster_id; tile < tiles && ok; tile += clusters) {
-            const int h = (tile / p.ttiles) & 1;  // backward: which 128 of the super-block's features
+            const int h = (p.first_ft + tile / p.ttiles) & 1;  // backward: which 128 of the super-block's features
             for (int u = u0; u < u1; u++, at_unit++) {
                 // Units of the whole ring in turn, where they are the group's own (R is a multiple of G, so a slot belongs to one group); else
                 // every group waits for and gives back every unit. Either way no group is a turn of the ring away from a barrier it tests.
@@ -699,7 +699,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
             }
         };
         for (int tile = cluster_id; tile < tiles && ok; tile += clusters) {
-            const int ft = tile / p.ttiles, t0 = (tile % p.ttiles) * nt;
+            const int ft = p.first_ft + tile / p.ttiles, t0 = (tile % p.ttiles) * nt;
             int ft0;
             const int wi = weight_of(p, ft, ft0);
             const int64_t feature = (int64_t)(ft - ft0) * 128 + lane_row, features = pick(p.features, wi);
@@ -894,7 +894,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
     }
     if (p.ksplit > 1 && *abort_flag == 0) {
         // columns range, range + ksplit, .. of the tile: the (virtual) ranges' sums in order
-        const int ft = cluster_id / p.ttiles, t0 = (cluster_id % p.ttiles) * nt;
+        const int ft = p.first_ft + cluster_id / p.ttiles, t0 = (cluster_id % p.ttiles) * nt;
         int ft0;
         const int wi = weight_of(p, ft, ft0);
         const int64_t f0 = (int64_t)(ft - ft0) * 128, features = pick(p.features, wi);

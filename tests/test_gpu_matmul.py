@@ -53,6 +53,21 @@ def test_backward(t, n, k, m):
     close(Gguf.linearBackward(g, w), g.double() @ wd)
 
 
+# products cut by features into several launches, each with its own tiles: 150 tiles for 9 rows (two more than a wave), 86 x 2 for 200 rows, and the
+# backward form, with an even and an odd first tile of features
+@pytest.mark.parametrize("t,n,k,m,bwd", [("Q4_K", 19100, 8192, 9, False), ("Q6_K", 19100, 8192, 9, False), ("Q4_K", 11000, 4096, 200, False),
+                                         ("Q6_K", 11000, 4096, 500, False), ("Q8_0", 4096, 11008, 128, True), ("Q4_K", 16384, 5120, 128, True)])
+def test_cut_by_features(t, n, k, m, bwd):
+    w, wd = weight(t, n, k, seed=m)
+    g = torch.Generator().manual_seed(k)
+    if bwd:
+        x = torch.randn(m, n, generator=g).cuda()
+        close(Gguf.linearBackward(x, w), x.double() @ wd)
+    else:
+        x, b = torch.randn(m, k, generator=g).cuda(), torch.randn(n, generator=g).cuda()
+        close(Gguf.linear(x, w, b), x.double() @ wd.T + b.double())
+
+
 # up to 16 rows the sums are taken in eight ranges of k whatever the number of thread blocks that share it: a row shard, whose k is split over a
 # larger cluster, gives bitwise the outputs of the whole weight. k: fewer units than ranges, more, and not a multiple
 @pytest.mark.parametrize("k", [768, 2048, 2816, 11008])
