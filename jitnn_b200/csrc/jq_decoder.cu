@@ -102,21 +102,26 @@ __device__ __forceinline__ void store4(__nv_bfloat16* o, int64_t i, float4 v) {
 }
 
 // If delta != nullptr: x += delta (the residual add). Then out = x * rsqrt(mean(x^2) + eps) * w (RMSNorm).
-// One CTA of NORM_THREADS threads per row: with few rows the kernel is bound by the latency of its loads, so every thread has
-// all of its row's values in flight at once (128-bit loads) and keeps up to 16 of them in registers for the second pass.
+// One CTA of THREADS threads per row: with few rows the kernel is bound by the latency of its loads, so every thread has
+// all of its row's values in flight at once (128-bit loads) and keeps up to HOLD of them in registers for the second pass. 1024 threads a row
+// while each row can have an SM; with more rows 256 or 512, so that more of them are in flight at once.
 // Out: float, or bfloat16 for a linear that rounds its input to it.
-constexpr int NORM_THREADS = 1024;
-template <typename Out>
+template <typename Out, int NORM_THREADS, int HOLD>
 __global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ delta, const float* __restrict__ w,
                                                                    float eps, Out* __restrict__ out, int dim) {
     asm volatile("griddepcontrol.launch_dependents;");  // launched programmatically, the kernel behind this one may be scheduled now ...
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // ... and this one touches memory only when the kernel before it has finished
+    const int nv = (dim & 3) == 0 ? dim >> 2 : 0;  // 128-bit pieces; a dim that is no multiple of 4 takes the scalar loops below
+    float4 wv[HOLD];
+#pragma unroll
+    for (int h = 0; h < HOLD; h++) {  // the weights never change
+        const int i = threadIdx.x + h * NORM_THREADS;
+        wv[h] = i < nv ? __ldg(reinterpret_cast<const float4*>(w) + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // ... and this one touches what others write only when the kernel before it has finished
     __shared__ float scratch[32];
     float* xr = x + (int64_t)blockIdx.x * dim;
     const float* dr = delta != nullptr ? delta + (int64_t)blockIdx.x * dim : nullptr;
     Out* o = out + (int64_t)blockIdx.x * dim;
-    constexpr int HOLD = 4;
-    const int nv = (dim & 3) == 0 ? dim >> 2 : 0;  // 128-bit pieces; a dim that is no multiple of 4 takes the scalar loops below
     float4 held[HOLD];
     float sq = 0.0f;
 #pragma unroll
@@ -149,8 +154,7 @@ __global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_kernel(float* __rest
     for (int h = 0; h < HOLD; h++) {
         const int i = threadIdx.x + h * NORM_THREADS;
         if (i < nv) {
-            const float4 wv = reinterpret_cast<const float4*>(w)[i];
-            store4(o, i, make_float4(held[h].x * inv * wv.x, held[h].y * inv * wv.y, held[h].z * inv * wv.z, held[h].w * inv * wv.w));
+            store4(o, i, make_float4(held[h].x * inv * wv[h].x, held[h].y * inv * wv[h].y, held[h].z * inv * wv[h].z, held[h].w * inv * wv[h].w));
         }
     }
     for (int i = rest + threadIdx.x; i < dim; i += NORM_THREADS) {
@@ -947,6 +951,17 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+template <typename Out>
+cudaError_t launch_add_rmsnorm(int rows, cudaStream_t s, bool programmatic, float* x, const float* delta, const float* w, float eps, Out* out, int dim) {
+    if (rows <= 148) {
+        return launch_pdl(add_rmsnorm_kernel<Out, 1024, 4>, dim3((unsigned)rows), dim3(1024), 0, s, programmatic, x, delta, w, eps, out, dim);
+    }
+    if (dim <= 4096) {
+        return launch_pdl(add_rmsnorm_kernel<Out, 256, 4>, dim3((unsigned)rows), dim3(256), 0, s, programmatic, x, delta, w, eps, out, dim);
+    }
+    return launch_pdl(add_rmsnorm_kernel<Out, 512, 4>, dim3((unsigned)rows), dim3(512), 0, s, programmatic, x, delta, w, eps, out, dim);
+}
+
 // The same for a kernel whose whole grid is one thread-block cluster.
 template <typename... KArgs, typename... Args>
 cudaError_t launch_cluster_pdl(void (*kernel)(KArgs...), int ctas, dim3 block, size_t smem, cudaStream_t s, bool programmatic, Args... args) {
@@ -1595,7 +1610,7 @@ static int enqueue_forward(jq_decoder* d, int T, int max_keys, const TokenArgs* 
         float* kc = d->k_cache + seq_base + (size_t)l * d->max_seq * kv_dim;
         float* vc = d->v_cache + seq_base + (size_t)l * d->max_seq * kv_dim;
         // attention block; the residual add of the previous block's feed-forward output is fused into this norm
-        if (rc == JQ_OK) pdl_err = launch_pdl(add_rmsnorm_kernel<float>, dim3(T), dim3(NORM_THREADS), 0, s, true, d->x, l == 0 ? nullptr : d->proj, d->norms + (size_t)(2 * l) * dim, d->eps, d->xn, dim);
+        if (rc == JQ_OK) pdl_err = launch_add_rmsnorm<float>(T, s, true, d->x, l == 0 ? nullptr : d->proj, d->norms + (size_t)(2 * l) * dim, d->eps, d->xn, dim);
         LAUNCHED("add_rmsnorm_kernel");
         {
             float* const qkv[3] = {d->q, d->k, d->v};
@@ -1613,7 +1628,7 @@ static int enqueue_forward(jq_decoder* d, int T, int max_keys, const TokenArgs* 
         LIN(L[3], d->att, d->proj);
         if (rc != JQ_OK) break;
         // feed-forward block
-        if (rc == JQ_OK) pdl_err = launch_pdl(add_rmsnorm_kernel<float>, dim3(T), dim3(NORM_THREADS), 0, s, true, d->x, d->proj, d->norms + (size_t)(2 * l + 1) * dim, d->eps, d->xn, dim);
+        if (rc == JQ_OK) pdl_err = launch_add_rmsnorm<float>(T, s, true, d->x, d->proj, d->norms + (size_t)(2 * l + 1) * dim, d->eps, d->xn, dim);
         LAUNCHED("add_rmsnorm_kernel");
         {
             float* const gu[2] = {d->gate, d->up};
@@ -1626,7 +1641,7 @@ static int enqueue_forward(jq_decoder* d, int T, int max_keys, const TokenArgs* 
         LIN(L[6], d->act, d->proj);
     }
     if (rc == JQ_OK) {
-        if (rc == JQ_OK) pdl_err = launch_pdl(add_rmsnorm_kernel<float>, dim3(T), dim3(NORM_THREADS), 0, s, true, d->x, d->proj, d->norms + (size_t)(2 * d->layers) * dim, d->eps, d->xn, dim);
+        if (rc == JQ_OK) pdl_err = launch_add_rmsnorm<float>(T, s, true, d->x, d->proj, d->norms + (size_t)(2 * d->layers) * dim, d->eps, d->xn, dim);
         LAUNCHED("add_rmsnorm_kernel");
         LIN(d->output, d->xn, d->logits);
     }
@@ -1760,7 +1775,7 @@ static int enqueue_forward_sharded(jq_decoder* d, int T, int max_keys, const Tok
                 rc = decoder_gemv_imaged3(d, L[0], d->q, L[1], d->k, L[2], d->v, s);
             }
         } else {
-            add_rmsnorm_kernel<float><<<T, NORM_THREADS, 0, s>>>(d->x, l == 0 ? nullptr : D, d->norms + (size_t)(2 * l) * dim, d->eps, d->xn, dim);
+            launch_add_rmsnorm<float>(T, s, false, d->x, l == 0 ? nullptr : D, d->norms + (size_t)(2 * l) * dim, d->eps, d->xn, dim);
             LAUNCHED("add_rmsnorm_kernel");
             float* const qkv[3] = {d->q, d->k, d->v};
             if (rc == JQ_OK) rc = linear_device_multi(L, 3, d->xn, T, qkv, s);
@@ -1800,7 +1815,7 @@ static int enqueue_forward_sharded(jq_decoder* d, int T, int max_keys, const Tok
             NORM_IMAGE(B, d->norms + (size_t)(2 * l + 1) * dim, {L[4], L[5]});
             GEMV_IMAGED(L[4], d->gate, L[5], d->up);
         } else {
-            add_rmsnorm_kernel<float><<<T, NORM_THREADS, 0, s>>>(d->x, B, d->norms + (size_t)(2 * l + 1) * dim, d->eps, d->xn, dim);
+            launch_add_rmsnorm<float>(T, s, false, d->x, B, d->norms + (size_t)(2 * l + 1) * dim, d->eps, d->xn, dim);
             LAUNCHED("add_rmsnorm_kernel");
             float* const gu[2] = {d->gate, d->up};
             if (rc == JQ_OK) rc = linear_device_multi(L + 4, 2, d->xn, T, gu, s);
@@ -1824,7 +1839,7 @@ static int enqueue_forward_sharded(jq_decoder* d, int T, int max_keys, const Tok
         }
     }
     if (rc == JQ_OK) {
-        add_rmsnorm_kernel<float><<<T, NORM_THREADS, 0, s>>>(d->x, D, d->norms + (size_t)(2 * d->layers) * dim, d->eps, d->xn, dim);
+        launch_add_rmsnorm<float>(T, s, false, d->x, D, d->norms + (size_t)(2 * d->layers) * dim, d->eps, d->xn, dim);
         LAUNCHED("add_rmsnorm_kernel");
         PEER_LIN(d->output, d->xn, d->vocab, vocab_l, 4);
     }
@@ -2107,7 +2122,7 @@ JQ_API int jq_decoder_prompt(jq_decoder* d, int seq, const int32_t* tokens_host,
         const int64_t cnt = (int64_t)T * hidden;
         for (int l = 0; l < d->layers && rc == JQ_OK; l++) {
             const jq_weight* const* L = &d->lin[(size_t)l * 7];
-            KERNEL(launch_pdl(add_rmsnorm_kernel<__nv_bfloat16>, dim3(T), dim3(NORM_THREADS), 0, s, true, x, l == 0 ? nullptr : proj,
+            KERNEL(launch_add_rmsnorm<__nv_bfloat16>(T, s, true, x, l == 0 ? nullptr : proj,
                               d->norms + (size_t)(2 * l) * dim, d->eps, xb, dim), "add_rmsnorm_kernel");
             LIN(L, 3, qkv);
             if (rc != JQ_OK) break;
@@ -2116,7 +2131,7 @@ JQ_API int jq_decoder_prompt(jq_decoder* d, int seq, const int32_t* tokens_host,
             rc = launch_prompt_attention(att, hd, s);
             LIN(L + 3, 1, &proj);
             if (rc != JQ_OK) break;
-            KERNEL(launch_pdl(add_rmsnorm_kernel<__nv_bfloat16>, dim3(T), dim3(NORM_THREADS), 0, s, true, x, proj, d->norms + (size_t)(2 * l + 1) * dim,
+            KERNEL(launch_add_rmsnorm<__nv_bfloat16>(T, s, true, x, proj, d->norms + (size_t)(2 * l + 1) * dim,
                               d->eps, xb, dim), "add_rmsnorm_kernel");
             LIN(L + 4, 2, gate_up);
             if (rc != JQ_OK) break;
@@ -2126,7 +2141,7 @@ JQ_API int jq_decoder_prompt(jq_decoder* d, int seq, const int32_t* tokens_host,
         if (rc == JQ_OK) {
             // the last token alone goes on: final residual add and norm, output projection (FP32 path), first index of the maximum
             const size_t last = (size_t)(T - 1) * dim;
-            KERNEL(launch_pdl(add_rmsnorm_kernel<float>, dim3(1), dim3(NORM_THREADS), 0, s, true, x + last, proj + last, d->norms + (size_t)(2 * d->layers) * dim, d->eps,
+            KERNEL(launch_add_rmsnorm<float>(1, s, true, x + last, proj + last, d->norms + (size_t)(2 * d->layers) * dim, d->eps,
                               d->xn, dim), "add_rmsnorm_kernel");
             if (rc == JQ_OK) rc = linear_device(d->output, d->xn, 1, nullptr, d->logits, s);
         }
