@@ -228,6 +228,18 @@ std::atomic<int64_t> g_opt_gemv_generic{0};
 std::atomic<int64_t> g_opt_decoder_graph{1};
 std::atomic<int64_t> g_opt_decoder_fused{1};
 
+// Whether a product with m rows of x goes to the matrix kernel in FP32 (under option gemv_tcgen05 = 1 up to 16 rows of Q4_K and Q5_K go to the
+// tcgen05 GEMV).
+static bool to_matrix_kernel(const jq_weight* w, int64_t m) {
+    return g_opt_gemv_generic.load() == 0 && matmul_takes(view_of(w), m) && !(m <= 16 && gemv_umma_takes(w->type, w->k, (int)m));
+}
+
+// Whether the linear behind a SwiGLU of m rows can take gate and up instead of their product.
+bool linear_takes_swiglu(const jq_weight* w, int64_t m) {
+    const int64_t min_rows = g_prefill_min_rows.load();
+    return w->n > 0 && !(min_rows > 0 && m >= min_rows) && to_matrix_kernel(w, m);
+}
+
 // ---- linear on device pointers --------------------------------------------------------------------
 int linear_device(const jq_weight* w, const float* x, int64_t m, const float* bias, float* y, cudaStream_t s, bool x_remote) {
     View v = view_of(w);
@@ -245,8 +257,7 @@ int linear_device(const jq_weight* w, const float* x, int64_t m, const float* bi
         return rc;
     }
     const bool tc = g_opt_gemv_generic.load() == 0;
-    // (under option gemv_tcgen05 = 1 up to 16 rows of Q4_K and Q5_K go to the tcgen05 GEMV)
-    if (tc && matmul_takes(v, m) && !(m <= 16 && gemv_umma_takes(w->type, w->k, (int)m))) {
+    if (to_matrix_kernel(w, m)) {
         return launch_matmul_f32(v, x, m, bias, y, s);
     }
     // The integer tensor-core kernel of Q4_K and Q5_K takes up to 8 activation rows per pass, Q6_K's 4, the one of Q8_0, Q4_0 and Q4_1 2, the
@@ -273,11 +284,10 @@ int linear_device_multi(const jq_weight* const* ws, int count, const float* x, i
         return JQ_OK;
     }
     const int64_t min_rows = g_prefill_min_rows.load();
-    const bool tc = g_opt_gemv_generic.load() == 0;
     // more rows of x than the decode kernels take in a pass: one split of x, one launch per format
-    bool matrix = count >= 2 && count <= 3 && tc && !(min_rows > 0 && m >= min_rows);
+    bool matrix = count >= 2 && count <= 3 && !(min_rows > 0 && m >= min_rows);
     for (int i = 0; i < count && matrix; i++) {
-        matrix = ws[i]->n > 0 && ws[i]->k == ws[0]->k && matmul_takes(view_of(ws[i]), m) && !(m <= 16 && gemv_umma_takes(ws[i]->type, ws[i]->k, (int)m));
+        matrix = ws[i]->n > 0 && ws[i]->k == ws[0]->k && to_matrix_kernel(ws[i], m);
     }
     if (matrix) {
         View vs[3];

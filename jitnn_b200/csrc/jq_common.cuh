@@ -221,6 +221,8 @@ constexpr int PAD_ROWS = 16;
 
 // The matrix kernel (jq_matmul.cu): the FP32 product with many rows of x, and the bfloat16 product.
 int launch_matmul_f32(const View& v, const float* x, int64_t m, const float* bias, float* y, cudaStream_t s);
+// The same for x = silu(gate) * up, made where x is split into halves.
+int launch_matmul_f32_swiglu(const View& v, const float* gate, const float* up, int64_t m, float* y, cudaStream_t s);
 // Up to three weights of one k on the same x: the split of x into halves is shared, weights of one format are one launch.
 int launch_matmul_f32_multi(const View* vs, int count, const float* x, int64_t m, float* const* ys, cudaStream_t s);
 bool matmul_takes(const View& v, int64_t rows);  // where it is the fastest of the FP32 kernels

@@ -22,6 +22,7 @@ namespace jq {
 
 int linear_device(const jq_weight* w, const float* x, int64_t m, const float* bias, float* y, cudaStream_t s, bool x_remote = false);
 int linear_device_multi(const jq_weight* const* ws, int count, const float* x, int64_t m, float* const* ys, cudaStream_t s);
+bool linear_takes_swiglu(const jq_weight* w, int64_t m);
 
 namespace {
 
@@ -1635,10 +1636,14 @@ static int enqueue_forward(jq_decoder* d, int T, int max_keys, const TokenArgs* 
             if (rc == JQ_OK) rc = linear_device_multi(L + 4, 2, d->xn, T, gu, s);
         }
         if (rc != JQ_OK) break;
-        const int64_t cnt = (int64_t)T * d->hidden;
-        if (rc == JQ_OK) pdl_err = launch_pdl(swiglu_kernel<float>, dim3((unsigned)((cnt + 1023) / 1024)), dim3(256), 0, s, true, d->gate, d->up, d->act, cnt);
-        LAUNCHED("swiglu_kernel");
-        LIN(L[6], d->act, d->proj);
+        if (linear_takes_swiglu(L[6], T)) {
+            rc = launch_matmul_f32_swiglu(View{L[6]->q, L[6]->aux, L[6]->n, L[6]->k, L[6]->type}, d->gate, d->up, T, d->proj, s);
+        } else {
+            const int64_t cnt = (int64_t)T * d->hidden;
+            pdl_err = launch_pdl(swiglu_kernel<float>, dim3((unsigned)((cnt + 1023) / 1024)), dim3(256), 0, s, true, d->gate, d->up, d->act, cnt);
+            LAUNCHED("swiglu_kernel");
+            LIN(L[6], d->act, d->proj);
+        }
     }
     if (rc == JQ_OK) {
         if (rc == JQ_OK) pdl_err = launch_add_rmsnorm<float>(T, s, true, d->x, d->proj, d->norms + (size_t)(2 * d->layers) * dim, d->eps, d->xn, dim);

@@ -13,14 +13,14 @@ static __device__ int g_matmul_status;
 
 namespace mm {
 
-// x [m, k] FP32 -> two planes of halves [2][m][width] (hi, lo) and a scale per (BLK values of k, row of x): the block's values times a power of
+// x [m, k] FP32 (or silu(x) * up) -> two planes of halves [2][m][width] (hi, lo) and a scale per (BLK values of k, row of x): the block's values times a power of
 // two that brings the largest to [2^9, 2^10), hi = that rounded to half precision, lo = the rest rounded to half precision: 22
 // significant bits for everything down to 2^-13 of the largest. A block that holds a NaN or an Inf gets the scale NaN, which reaches
 // every output of that row. One warp per 256 values of a row; memory bound (8 bytes moved per value, 4 of them to L2).
 // EXT: 16 more columns follow every 256, the sums over the eight runs of 32 values, twice (hi plane: their hi parts, lo plane: their lo
 // parts).
 template <int BLK, bool EXT>
-__global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ x, int m, int64_t k, int per_row, uint4* __restrict__ planes,
+__global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ x, const float* __restrict__ up, int m, int64_t k, int per_row, uint4* __restrict__ planes,
                                                     float* __restrict__ scales, int stride, int vec) {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -41,6 +41,24 @@ __global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ x,
 #pragma unroll
         for (int i = 0; i < 8; i++) {
             v[i] = i0 + i < k ? __ldg(src + i) : 0.0f;
+        }
+    }
+    if (up != nullptr) {  // x is the gate of a feed-forward block
+        const float* us = up + (src - x);
+        float u[8];
+        if (vec && i0 + 8 <= k) {
+            const float4 a = __ldg(reinterpret_cast<const float4*>(us)), c = __ldg(reinterpret_cast<const float4*>(us) + 1);
+            u[0] = a.x; u[1] = a.y; u[2] = a.z; u[3] = a.w;
+            u[4] = c.x; u[5] = c.y; u[6] = c.z; u[7] = c.w;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                u[i] = i0 + i < k ? __ldg(us + i) : 0.0f;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            v[i] = (v[i] / (1.0f + expf(-v[i]))) * u[i];
         }
     }
     uint32_t am = 0;  // the largest magnitude as bits: an Inf or a NaN is larger than any number
@@ -348,7 +366,7 @@ static int weight_args(const View* vs, int count, bool bwd, float* const* ys, Ar
 constexpr int SPLIT_SLOT = 6;  // scratch slots 6 and 7: split activations without and with the 16 more columns
 
 // ys[i] [m, features_i] = the FP32 products of `count` weights with the same x (backward: one weight); x has `width` values per row.
-static int product_f32(const View* vs, int count, bool bwd, const float* x, int64_t m, const float* bias, float* const* ys, cudaStream_t s) {
+static int product_f32(const View* vs, int count, bool bwd, const float* x, const float* up, int64_t m, const float* bias, float* const* ys, cudaStream_t s) {
     const int64_t width = bwd ? vs[0].n : vs[0].k;
     const int per_row = (int)((width + 255) / 256), blk = bwd ? 128 : 256;
     constexpr int64_t GROUP = 4096;  // rows at a time: bounds the scratch
@@ -358,7 +376,8 @@ static int product_f32(const View* vs, int count, bool bwd, const float* x, int6
         const int rows = (int)(m - m0 < GROUP ? m - m0 : GROUP);
         const int stride = (rows + 128 + 15) / 16 * 16;  // tiles of rows reach at most this far
         const float* xg = x + m0 * width;
-        const int vec = width % 4 == 0 && ((uintptr_t)xg & 15) == 0;
+        const float* ug = up != nullptr ? up + m0 * width : nullptr;
+        const int vec = width % 4 == 0 && (((uintptr_t)xg | (uintptr_t)ug) & 15) == 0;
         // weights with the 16 more columns per unit and weights without: one split each
         for (int ext = 0; ext < 2 && rc == JQ_OK; ext++) {
             const int64_t wpad = (int64_t)per_row * (ext ? 272 : 256);
@@ -398,7 +417,7 @@ static int product_f32(const View* vs, int count, bool bwd, const float* x, int6
                     cfg.gridDim = dim3((unsigned)(((int64_t)rows * per_row + 7) / 8));
                     cfg.blockDim = dim3(256);
                     auto split = bwd ? split_kernel<128, false> : (ext ? split_kernel<256, true> : split_kernel<256, false>);
-                    JQ_CUDA(cudaLaunchKernelEx(&cfg, split, xg, rows, width, per_row, reinterpret_cast<uint4*>(scratch), scales, stride, vec));
+                    JQ_CUDA(cudaLaunchKernelEx(&cfg, split, xg, ug, rows, width, per_row, reinterpret_cast<uint4*>(scratch), scales, stride, vec));
                     count_launch();
                 }
                 Args w = {};
@@ -426,11 +445,15 @@ static int product_f32(const View* vs, int count, bool bwd, const float* x, int6
 }  // namespace mm
 
 int launch_matmul_f32(const View& v, const float* x, int64_t m, const float* bias, float* y, cudaStream_t s) {
-    return mm::product_f32(&v, 1, false, x, m, bias, &y, s);
+    return mm::product_f32(&v, 1, false, x, nullptr, m, bias, &y, s);
+}
+
+int launch_matmul_f32_swiglu(const View& v, const float* gate, const float* up, int64_t m, float* y, cudaStream_t s) {
+    return mm::product_f32(&v, 1, false, gate, up, m, nullptr, &y, s);
 }
 
 int launch_matmul_f32_multi(const View* vs, int count, const float* x, int64_t m, float* const* ys, cudaStream_t s) {
-    return mm::product_f32(vs, count, false, x, m, nullptr, ys, s);
+    return mm::product_f32(vs, count, false, x, nullptr, m, nullptr, ys, s);
 }
 
 // More than 16 rows of x always: the weight is read once for all of them. Up to 16 rows take the same time as one (Q4_K 32000 x 4096: 27 us,
@@ -455,7 +478,7 @@ bool matmul_takes(const View& v, int64_t rows) {
 }
 
 // gx [m, k] = g [m, n] . dequant(W) (ops/Gguf.java:208-212, ops/Quant.java:191-197); device pointers; n >= 1, m >= 1.
-int launch_linear_backward(const View& v, const float* g, int64_t m, float* gx, cudaStream_t s) { return mm::product_f32(&v, 1, true, g, m, nullptr, &gx, s); }
+int launch_linear_backward(const View& v, const float* g, int64_t m, float* gx, cudaStream_t s) { return mm::product_f32(&v, 1, true, g, nullptr, m, nullptr, &gx, s); }
 
 bool prefill_supported(const View& v) { return has_linear_kernel(v.type) && v.k % 64 == 0 && v.n > 0 && v.k > 0; }
 
