@@ -250,7 +250,15 @@ def _dequantize(w, out=None):
     L = _lib.load()
     n, k = w.shape()
     if out is not None and _is_torch(out):
-        check(L.jq_dequantize(w._handle(), out.data_ptr(), JQ_MEM_DEVICE, _raw_stream(_t(), out.get_device())))
+        torch = _t()
+        # a kernel writes n k floats from the tensor's address on: nothing else may reach the library
+        if out.dtype is not torch.float32:
+            raise ValueError("needs an FP32 tensor, got %s" % out.dtype)
+        if not out.is_contiguous() or out.numel() < n * k:
+            raise ValueError("%s dequantize: %s tensor %s for %d values" % (w._dtype.name, "contiguous" if out.is_contiguous() else "strided", list(out.shape), n * k))
+        if out.get_device() != w._device:
+            raise ValueError("%s dequantize: output on %s, weight on cuda:%d" % (w._dtype.name, out.device, w._device))
+        check(L.jq_dequantize(w._handle(), out.data_ptr(), JQ_MEM_DEVICE, _raw_stream(torch, w._device)))
         return out
     y = np.empty((n, k), dtype=np.float32)
     check(L.jq_dequantize(w._handle(), y.ctypes.data, JQ_MEM_HOST, None))
@@ -348,8 +356,10 @@ class Quant:
                 raise ValueError("needs an FP32 tensor, got %s" % x.dtype)
             if x.shape[-1] % 32 != 0:
                 raise ValueError("Q8_0 needs a last axis that is a multiple of 32, got %s" % list(x.shape))
-            xc = x if x.is_contiguous() else x.contiguous()
             index = x.get_device()
+            if index < 0:
+                raise ValueError("Q8_0 quantiser: input on %s, not on a GPU" % x.device)
+            xc = x if x.is_contiguous() else x.contiguous()
             out = xc.new_empty((xc.numel() // 32 * 34,), dtype=torch.uint8)
             check(L.jq_quantize_q8_0(index, xc.data_ptr(), xc.numel(), out.data_ptr(), JQ_MEM_DEVICE, _raw_stream(torch, index)))
             return out
