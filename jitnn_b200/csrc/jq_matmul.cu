@@ -458,9 +458,11 @@ int launch_matmul_f32_multi(const View* vs, int count, const float* x, int64_t m
 
 // More than 16 rows of x always: the weight is read once for all of them. Up to 16 rows take the same time as one (Q4_K 32000 x 4096: 27 us,
 // Q6_K 41, 4096 x 4096: 11), so the line lies where the decode kernels need another pass: Q4_K and Q5_K take up to eight rows in one
-// (25 us), Q6_K four (35), the 32-element formats two (24 and 16). It does not depend on the number of output rows, and neither do
-// the sums, so a row shard gives bitwise the outputs of the whole weight. Where k is no multiple of 256 there is only the CUDA-core
-// kernel besides, which is the faster one up to about eight million products (4096 x 1056, one row: 4.5 us against 8.9).
+// (25 us), Q6_K four (35), the 32-element formats two (24 and 16). It must not depend on the number of output rows, and neither do
+// the sums, so a row shard gives bitwise the outputs of the whole weight. Where the decode kernels decline (k no multiple of 256, or too
+// wide) there is only the CUDA-core kernel besides, whose time grows with rows x k: with 4096 output rows it meets the matrix kernel near
+// rows k = 4096 for Q8_0 (k = 1056: 16.4 us at 4 rows against 17.4; 2080: 16.4 at 2 rows and 24.6 at 4 against 19.2) and near 2048 for Q4_0 and
+// Q4_1 (1056: 16.4 at 2 rows and 32.8 at 4 against 17.4; 2080: 16.4 at one row against 17.4).
 bool matmul_takes(const View& v, int64_t rows) {
     if (rows > 16) {
         return true;
@@ -474,7 +476,7 @@ bool matmul_takes(const View& v, int64_t rows) {
     if (gemv_blk32_i8_scratch_bytes(v.type, v.k, rows < 2 ? 1 : 2) > 0) {
         return rows >= 5;
     }
-    return rows * v.n * v.k > 8000000;
+    return rows * v.k >= (v.type == JQ_TYPE_Q8_0 ? 4096 : 2048);
 }
 
 // gx [m, k] = g [m, n] . dequant(W) (ops/Gguf.java:208-212, ops/Quant.java:191-197); device pointers; n >= 1, m >= 1.

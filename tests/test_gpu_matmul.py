@@ -130,3 +130,19 @@ def test_nan_and_inf_reach_their_rows():
     assert bool(bad[3].all()) and bool(bad[20].all())
     rows = [r for r in range(40) if r not in (3, 20)]
     close(y[rows], x[rows].double() @ wd.T)
+
+
+# 32-element formats with a k that the decode kernels decline: up to 16 rows the choice of the kernel must not depend on the number of output rows
+# either, or a shard would add up in another order than the whole weight (5000 x 1056 and 100 x 1056 lie on both sides of any line in products)
+@pytest.mark.parametrize("k", [288, 1056, 2080])
+@pytest.mark.parametrize("t", ["Q8_0", "Q4_0", "Q4_1"])
+def test_row_shards_are_bitwise_equal_for_partial_steps(t, k):
+    n = 5000
+    raw = synth.random_valid_blocks(t, n, k, seed=k).numpy().reshape(-1)
+    whole = Tensor.quantized(t, raw, n, k)
+    shards = [(lo, hi, Tensor.quantized(t, raw, n, k, rows=(lo, hi))) for lo, hi in [(0, 100), (2048, 2560), (2500, 5000)]]
+    for m in range(1, 17):
+        x = torch.randn(m, k, generator=torch.Generator().manual_seed(k + m)).cuda()
+        y = Gguf.linear(x, whole)
+        for lo, hi, shard in shards:
+            assert torch.equal(Gguf.linear(x, shard), y[:, lo:hi]), (m, lo, hi)
