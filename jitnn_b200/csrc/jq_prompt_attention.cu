@@ -20,7 +20,7 @@ namespace {
 // The largest magnitude of a row goes to [2^9, 2^10): the lo halves of values down to 2^-13 of it stay normal numbers.
 __device__ __forceinline__ void row_scale(float amax, float& up, float& down) {
     uint32_t e = __float_as_uint(amax) >> 23;
-    const bool bad = e == 255u;  // a NaN or an Inf: the row's scale becomes NaN and reaches every result that uses it
+    const bool bad = e == 255u;  // a NaN or an Inf: the row's scale becomes NaN and reaches every result that uses it (its halves are zeros)
     e = e < 20u ? 20u : (e > 250u ? 250u : e);
     up = __uint_as_float((263u - e) << 23);
     down = bad ? __uint_as_float(0x7fc00000u) : __uint_as_float((e - 9u) << 23);
@@ -106,6 +106,12 @@ __global__ void __launch_bounds__(256) rope_split_kernel(PromptAttention p) {
     am = __reduce_max_sync(0xffffffffu, am);
     float up, down;
     row_scale(__uint_as_float(am), up, down);
+    if (am >= 0x7f800000u) {  // the scale says it: a NaN among the halves of a value row would reach queries that do not see the key, as 0 x NaN
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            a[i] = b[i] = 0.0f;
+        }
+    }
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         __half hv[N], lv[N];
@@ -223,7 +229,7 @@ __global__ void __launch_bounds__(THREADS, 2) prompt_attention_kernel(PromptAtte
         acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
     }
     float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.0f, l1 = 0.0f;
-    float vmax = 7.8886091e-31f;  // 2^-100; acc is in units of this power of two, the largest value scale of the tiles so far
+    float vmax0 = 7.8886091e-31f, vmax1 = vmax0;  // 2^-100; a query's acc is in units of this power of two, the largest scale of the values it has seen
     // ldmatrix rows: K fragments of 16 keys (two n-blocks) x 16 d; V fragments of 16 keys x 16 d (transposed)
     const int k_row = (lane & 7) + ((lane >> 4) << 3), k_ch = (lane >> 3) & 1;
     const int v_row = (lane & 7) + (((lane >> 3) & 1) << 3), v_ch = lane >> 4;
@@ -289,11 +295,29 @@ __global__ void __launch_bounds__(THREADS, 2) prompt_attention_kernel(PromptAtte
         l1 *= al1;
         cp_wait<1>();
         __syncthreads();  // the tile's values are here
-        // every value row has a scale of its own, which goes into the weights, relative to the largest one so far
-        const float vm = fmaxf(vmax, warp_max(fmaxf(vs_s[lane], vs_s[lane + 32])));
-        const float turn = vmax / vm, inv = 1024.0f / vm;  // powers of two; weights of up to 2^10
-        vmax = vm;
-        const float b0 = al0 * turn, b1 = al1 * turn;
+        // every value row has a scale of its own, which goes into the weights, relative to the largest one that the query has seen so far
+        float vm0 = vmax0, vm1 = vmax1;
+        if (!edge) {
+            const float vm = warp_max(fmaxf(vs_s[lane], vs_s[lane + 32]));
+            vm0 = fmaxf(vm0, vm);
+            vm1 = fmaxf(vm1, vm);
+        } else {
+#pragma unroll
+            for (int nb = 0; nb < KT / 8; nb++) {
+                const float2 sv = *reinterpret_cast<const float2*>(vs_s + nb * 8 + 2 * t);
+                const int key = key0 + nb * 8 + 2 * t;
+                vm0 = fmaxf(vm0, fmaxf(key <= p.pos0 + r0 ? sv.x : 0.0f, key + 1 <= p.pos0 + r0 ? sv.y : 0.0f));
+                vm1 = fmaxf(vm1, fmaxf(key <= p.pos0 + r1 ? sv.x : 0.0f, key + 1 <= p.pos0 + r1 ? sv.y : 0.0f));
+            }
+            vm0 = fmaxf(vm0, __shfl_xor_sync(0xffffffffu, vm0, 1));
+            vm0 = fmaxf(vm0, __shfl_xor_sync(0xffffffffu, vm0, 2));
+            vm1 = fmaxf(vm1, __shfl_xor_sync(0xffffffffu, vm1, 1));
+            vm1 = fmaxf(vm1, __shfl_xor_sync(0xffffffffu, vm1, 2));
+        }
+        const float inv0 = 1024.0f / vm0, inv1 = 1024.0f / vm1;  // powers of two; weights of up to 2^10
+        const float b0 = al0 * (vmax0 / vm0), b1 = al1 * (vmax1 / vm1);
+        vmax0 = vm0;
+        vmax1 = vm1;
 #pragma unroll
         for (int i = 0; i < HD / 8; i++) {
             acc[i][0] *= b0; acc[i][1] *= b0;
@@ -306,13 +330,21 @@ __global__ void __launch_bounds__(THREADS, 2) prompt_attention_kernel(PromptAtte
             for (int j = 0; j < 2; j++) {
                 float(&e)[4] = s[2 * kb + j];
                 const float2 sv = *reinterpret_cast<const float2*>(vs_s + kb * 16 + j * 8 + 2 * t);
-                const float w0 = sv.x * inv, w1 = sv.y * inv;
                 e[0] = expf(e[0] - m0); e[1] = expf(e[1] - m0);
                 e[2] = expf(e[2] - m1); e[3] = expf(e[3] - m1);
                 l0 += e[0] + e[1];
                 l1 += e[2] + e[3];
-                split2(e[0] * w0, e[1] * w1, pa[2 * j], pb[2 * j]);
-                split2(e[2] * w0, e[3] * w1, pa[2 * j + 1], pb[2 * j + 1]);
+                e[0] *= sv.x * inv0; e[1] *= sv.y * inv0;
+                e[2] *= sv.x * inv1; e[3] *= sv.y * inv1;
+                if (edge) {  // a key that the query does not see has the weight zero, and its scale may be a NaN
+                    const int key = key0 + kb * 16 + j * 8 + 2 * t;
+                    e[0] = key <= p.pos0 + r0 ? e[0] : 0.0f;
+                    e[1] = key + 1 <= p.pos0 + r0 ? e[1] : 0.0f;
+                    e[2] = key <= p.pos0 + r1 ? e[2] : 0.0f;
+                    e[3] = key + 1 <= p.pos0 + r1 ? e[3] : 0.0f;
+                }
+                split2(e[0], e[1], pa[2 * j], pb[2 * j]);
+                split2(e[2], e[3], pa[2 * j + 1], pb[2 * j + 1]);
             }
             const int row = kb * 16 + v_row;
 #pragma unroll
@@ -341,7 +373,7 @@ __global__ void __launch_bounds__(THREADS, 2) prompt_attention_kernel(PromptAtte
     l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
     l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
     l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-    const float f0 = vmax * 0.0009765625f / l0, f1 = vmax * 0.0009765625f / l1;
+    const float f0 = vmax0 * 0.0009765625f / l0, f1 = vmax1 * 0.0009765625f / l1;
     __nv_bfloat16* const o0 = p.out + ((int64_t)r0 * p.heads + h) * HD + 2 * t;
     __nv_bfloat16* const o1 = p.out + ((int64_t)r1 * p.heads + h) * HD + 2 * t;
 #pragma unroll
