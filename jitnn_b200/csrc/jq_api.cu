@@ -69,15 +69,28 @@ struct Staging {
 // from and to numpy arrays: 36 us with three engine copies).
 constexpr size_t PINNED_BYTES = (size_t)512 << 10;
 
+void scratch_release(cudaStream_t s);
+
 // What a thread holds is given back when it ends (a driver that is shutting down has released it already and says so).
 struct ThreadStaging {
     std::vector<Staging> devices;
     ~ThreadStaging() {
-        for (Staging& st : devices) {
-            if (st.pinned != nullptr) {
-                cudaFreeHost(st.pinned);
-            }
+        int prev = -1;
+        if (devices.empty() || cudaGetDevice(&prev) != cudaSuccess) {
+            return;
         }
+        for (size_t device = 0; device < devices.size(); device++) {
+            Staging& st = devices[device];
+            if (st.stream == nullptr || cudaSetDevice((int)device) != cudaSuccess) {
+                continue;
+            }
+            cudaStreamSynchronize(st.stream);  // (a call that failed half-way may have left work)
+            scratch_release(st.stream);
+            cudaFree(st.dev);
+            cudaFreeHost(st.pinned);
+            cudaStreamDestroy(st.stream);
+        }
+        cudaSetDevice(prev);
     }
 };
 static thread_local ThreadStaging t_staging_owner;
@@ -109,7 +122,7 @@ static int staging_for(int device, size_t bytes, Staging** out) {
 // ---- per (device, stream) scratch ------------------------------------------------------------------
 // A buffer that has been handed out may be baked into a captured CUDA graph (the decoder's step, a caller's own capture
 // of jq_linear_*), so it is never freed or moved: a request that outgrows it gets a new allocation and the old one stays
-// where it is until the process ends.
+// where it is until the process ends, or until the library gives up a stream of its own (scratch_release).
 struct Scratch {
     int device;
     cudaStream_t stream;
@@ -119,7 +132,7 @@ struct Scratch {
 };
 static std::mutex g_scratch_mu;
 static std::vector<Scratch> g_scratch;
-static std::vector<uint8_t*> g_scratch_retired;
+constexpr int RETIRED = -1;  // the slot of a buffer that was outgrown
 
 int scratch_for(cudaStream_t s, size_t bytes, uint8_t** out) { return scratch_for_slot(s, 0, bytes, out); }
 
@@ -146,14 +159,31 @@ static int scratch_impl(cudaStream_t s, int slot, size_t bytes, bool zeroed, uin
         if (zeroed) {
             JQ_CUDA(cudaMemsetAsync(fresh, 0, want, s));  // in stream order before the first kernel that uses it
         }
-        if (hit->buf != nullptr) {
-            g_scratch_retired.push_back(hit->buf);
-        }
+        const Scratch old{dev, s, RETIRED, hit->buf, hit->bytes};
         hit->buf = fresh;
         hit->bytes = want;
+        *out = fresh;
+        if (old.buf != nullptr) {
+            g_scratch.push_back(old);
+        }
+        return JQ_OK;
     }
     *out = hit->buf;
     return JQ_OK;
+}
+
+// Frees the scratch of a stream that the library made itself and is about to destroy: nothing runs on it, and no graph that used it is left.
+void scratch_release(cudaStream_t s) {
+    std::lock_guard<std::mutex> lock(g_scratch_mu);
+    size_t kept = 0;
+    for (const Scratch& sc : g_scratch) {
+        if (sc.stream == s) {
+            cudaFree(sc.buf);
+        } else {
+            g_scratch[kept++] = sc;
+        }
+    }
+    g_scratch.resize(kept);
 }
 
 int scratch_for_slot(cudaStream_t s, int slot, size_t bytes, uint8_t** out) { return scratch_impl(s, slot, bytes, false, out); }

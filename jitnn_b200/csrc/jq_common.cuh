@@ -198,6 +198,8 @@ int scratch_for_slot(cudaStream_t s, int slot, size_t bytes, uint8_t** out);
 
 // The same for words that kernels use as counters and leave at zero: a new allocation starts out zeroed (in stream order).
 int scratch_zeroed_for_slot(cudaStream_t s, int slot, size_t bytes, uint8_t** out);
+// For a stream of the library's own that is about to be destroyed.
+void scratch_release(cudaStream_t s);
 
 // Decode GEMV on tcgen05 (jq_gemv_umma.cu): Q4_K and Q5_K, 1 to 16 rows of x in one pass over the weights.
 bool gemv_umma_takes(int type, int64_t k, int rows);  // under option gemv_tcgen05 = 1
