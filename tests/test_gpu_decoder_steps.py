@@ -59,3 +59,21 @@ def test_logits_arrays_stay_valid():
     dec.close()
     for a, b in zip(held, copies):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n_seqs", [1, 2])
+def test_the_next_range_is_captured_before_it_is_reached(n_seqs):
+    """A step past the end of a range finds its graph there: capturing counts the step's launches, replaying does not."""
+    dec = build(4, 2, 128, 520)
+    if n_seqs > 1:
+        dec.set_sequences(n_seqs)
+    L = jitnn_b200.load()
+    toks = np.zeros(n_seqs, np.int32)
+    counts = [L.jq_launch_count()]
+    for pos in range(236, 520):
+        dec.forward(toks, pos) if n_seqs == 1 else dec.forward_batch(toks, pos)
+        counts.append(L.jq_launch_count())
+    per_step = np.diff(counts)
+    assert per_step[256 - 236] == 0 and per_step[512 - 236] == 0
+    assert (per_step > 0).sum() == 2 + 2  # the first step is issued kernel by kernel; one capture each for up to 256, 512 and 520 positions
+    dec.close()
