@@ -149,9 +149,10 @@ JQ_API int jq_linear_backward_f32(const jq_weight* w, const float* g, int64_t m,
 
 /*
  * Waits for the work enqueued on `device` and reports, then clears, the status word of its kernels: 0, or the code of
- * the first bounded device-side wait that gave up (the prefill kernel's barrier waits are bounded instead of being
- * able to hang). Calls with host memory check this themselves and return JQ_ERR_TIMEOUT; callers that enqueue with
- * device memory can poll it at a synchronisation point of their own. (No counterpart in the reference.)
+ * a bounded device-side wait that gave up (barrier waits are bounded instead of being able to hang). For callers that enqueue
+ * with device memory, at a synchronisation point of their own. Calls with host memory and decoder calls that return a
+ * result have status words of their own and return JQ_ERR_TIMEOUT for their own kernels (a decoder call also for the
+ * calls that were only enqueued before it); what they report is not reported here. (No counterpart in the reference.)
  */
 JQ_API int jq_device_status(int device, int* status);
 
@@ -220,9 +221,10 @@ JQ_API int jq_quantize_q8_0(int device, const float* x, int64_t count, void* blo
  *   "gemv_tcgen05"      which Q4_K and Q5_K decode GEMVs run on the tcgen05 GEMV (1 to 16 rows of x in one pass over the weights)
  *                       instead of the mma.sync one (up to 8 rows) and the matrix kernel (more). 0 (default): the shapes the
  *                       mma.sync kernel declines; 1: all; 2: none.
- *   "wait_limit_us"     microseconds after which a bounded device-side wait of the tcgen05 GEMV gives up (default 2 000 000; a
- *                       wait that gives up makes jq_device_status report 64 + the waiting role, and the outputs of that call
- *                       are undefined).
+ *   "wait_limit_us"     microseconds after which a kernel's wait for its own copies and tensor-core work gives up (default 2 000 000,
+ *                       in the matrix kernel counted from the end of the kernel in front): the call returns JQ_ERR_TIMEOUT or
+ *                       jq_device_status reports a code (1 to 8 matrix kernel, 24 and 25 decode GEMVs, 64 + role tcgen05
+ *                       GEMV), its outputs are undefined.
  */
 JQ_API int jq_set_option(const char* name, int64_t value);
 JQ_API int jq_get_option(const char* name, int64_t* value);

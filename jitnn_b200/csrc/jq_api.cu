@@ -63,6 +63,7 @@ struct Staging {
     cudaStream_t stream = nullptr;
     uint8_t* pinned = nullptr;      // PINNED_BYTES of page-locked memory that the device can address
     uint8_t* pinned_dev = nullptr;  // its address on the device
+    int* status = nullptr;          // of the calls' kernels
 };
 // Pageable arrays up to this size in all take the way through page-locked memory of the thread, which the kernels then read and write
 // themselves: a copy by the host of some kilobytes costs less than setting up a copy engine for it (one row of Q8_0 4096 x 4096 with bias,
@@ -88,6 +89,7 @@ struct ThreadStaging {
             scratch_release(st.stream);
             cudaFree(st.dev);
             cudaFreeHost(st.pinned);
+            give_status_word(st.status);
             cudaStreamDestroy(st.stream);
         }
         cudaSetDevice(prev);
@@ -96,11 +98,24 @@ struct ThreadStaging {
 static thread_local ThreadStaging t_staging_owner;
 #define t_staging t_staging_owner.devices
 
+// Waits for what a host call enqueued on its thread's stream.
+static int staging_wait(Staging* st, const char* who) {
+    JQ_CUDA(cudaStreamSynchronize(st->stream));
+    const int code = read_status(st->status);
+    return code == 0 ? JQ_OK : fail(JQ_ERR_TIMEOUT, "%s: a bounded wait on the device gave up (code %d)", who, code);
+}
+
 static int staging_for(int device, size_t bytes, Staging** out) {
     if ((size_t)device >= t_staging.size()) {
         t_staging.resize(device + 1);
     }
     Staging& st = t_staging[device];
+    if (st.status == nullptr) {
+        const int rc = take_status_word(&st.status);
+        if (rc != JQ_OK) {
+            return rc;
+        }
+    }
     if (st.stream == nullptr) {
         JQ_CUDA(cudaStreamCreateWithFlags(&st.stream, cudaStreamNonBlocking));
     }
@@ -190,6 +205,67 @@ int scratch_for_slot(cudaStream_t s, int slot, size_t bytes, uint8_t** out) { re
 
 // The same, for words that kernels use as counters and leave at zero: a new allocation starts out zeroed.
 int scratch_zeroed_for_slot(cudaStream_t s, int slot, size_t bytes, uint8_t** out) { return scratch_impl(s, slot, bytes, true, out); }
+
+// ---- status words ----------------------------------------------------------------------------------------------
+static std::mutex g_status_mu;
+static std::vector<int*> g_status_free;
+static std::atomic<int*> g_device_status[64];
+static thread_local int* t_status = nullptr;
+
+int take_status_word(int** word) {
+    std::lock_guard<std::mutex> lock(g_status_mu);
+    if (g_status_free.empty()) {
+        constexpr int WORDS = 1024;
+        void* slab = nullptr;  // kept until the process ends: devices keep their words
+        JQ_CUDA(cudaHostAlloc(&slab, WORDS * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+        memset(slab, 0, WORDS * sizeof(int));
+        for (int i = 0; i < WORDS; i++) {
+            g_status_free.push_back(static_cast<int*>(slab) + i);  // (one address on host and devices)
+        }
+    }
+    *word = g_status_free.back();
+    g_status_free.pop_back();
+    read_status(*word);
+    return JQ_OK;
+}
+
+void give_status_word(int* word) {
+    if (word != nullptr) {
+        std::lock_guard<std::mutex> lock(g_status_mu);
+        g_status_free.push_back(word);
+    }
+}
+
+int* device_status_word(int device) { return g_device_status[device & 63].load(std::memory_order_acquire); }
+
+// Made when a weight comes to the device, so that no launch has to allocate it.
+static int make_device_status_word(int device) {
+    if (device_status_word(device) != nullptr) {
+        return JQ_OK;
+    }
+    int* word = nullptr;
+    const int rc = take_status_word(&word);
+    int* expected = nullptr;
+    if (rc == JQ_OK && !g_device_status[device & 63].compare_exchange_strong(expected, word)) {
+        give_status_word(word);
+    }
+    return rc;
+}
+
+int status_word(int** word) {
+    if (t_status != nullptr) {
+        *word = t_status;
+        return JQ_OK;
+    }
+    int device = 0;
+    JQ_CUDA(cudaGetDevice(&device));
+    const int rc = make_device_status_word(device);
+    *word = device_status_word(device);
+    return rc;
+}
+
+StatusScope::StatusScope(int* word) : before(t_status) { t_status = word; }
+StatusScope::~StatusScope() { t_status = before; }
 
 static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
@@ -460,6 +536,10 @@ int jq_weight_upload_rows(int device, int type, const void* host_blocks, int64_t
     if (!guard.ok) {
         return fail(JQ_ERR_CUDA, "weight upload: cannot select device %d", device);
     }
+    const int status_rc = make_device_status_word(device);
+    if (status_rc != JQ_OK) {
+        return status_rc;
+    }
     int64_t rows = row_end - row_begin;
     int64_t blocks = rows * (k / qk);
     const uint8_t* src = (const uint8_t*)host_blocks + row_begin * row_bytes;
@@ -723,6 +803,7 @@ int jq_linear_f32(const jq_weight* w, const float* x, int64_t m, const float* bi
     if (copy_y) {
         dy = (float*)(st->dev + xb + bb);
     }
+    const StatusScope scope(st->status);
     rc = linear_device(w, dx, m, db, dy, st->stream, x_remote);  // x in host memory: read it once, not once per thread block
     if (rc != JQ_OK) {
         return rc;
@@ -730,11 +811,11 @@ int jq_linear_f32(const jq_weight* w, const float* x, int64_t m, const float* bi
     if (copy_y) {
         JQ_CUDA(cudaMemcpyAsync(y, dy, (size_t)m * w->n * 4, cudaMemcpyDeviceToHost, st->stream));
     }
-    JQ_CUDA(cudaStreamSynchronize(st->stream));
-    if (y_staged != nullptr) {
+    rc = staging_wait(st, "jq_linear_f32");
+    if (rc == JQ_OK && y_staged != nullptr) {
         memcpy(y, y_staged, y_bytes);
     }
-    return JQ_OK;
+    return rc;
 }
 
 int jq_linear_backward_f32(const jq_weight* w, const float* g, int64_t m, float* gx, int mem, void* stream) {
@@ -780,14 +861,14 @@ int jq_linear_backward_f32(const jq_weight* w, const float* g, int64_t m, float*
         JQ_CUDA(cudaMemsetAsync(dgx, 0, xb, st->stream));
     } else {
         JQ_CUDA(cudaMemcpyAsync(st->dev, g, (size_t)m * w->n * 4, cudaMemcpyHostToDevice, st->stream));
+        const StatusScope scope(st->status);
         rc = launch_linear_backward(view_of(w), (const float*)st->dev, m, dgx, st->stream);
         if (rc != JQ_OK) {
             return rc;
         }
     }
     JQ_CUDA(cudaMemcpyAsync(gx, dgx, xb, cudaMemcpyDeviceToHost, st->stream));
-    JQ_CUDA(cudaStreamSynchronize(st->stream));
-    return JQ_OK;
+    return staging_wait(st, "jq_linear_backward_f32");
 }
 
 int jq_linear_bf16(const jq_weight* w, const uint16_t* x, int64_t m, const float* bias, float* y, int mem, void* stream) {
@@ -832,18 +913,13 @@ int jq_linear_bf16(const jq_weight* w, const uint16_t* x, int64_t m, const float
     if (bias != nullptr) {
         JQ_CUDA(cudaMemcpyAsync(db, bias, (size_t)w->n * 4, cudaMemcpyHostToDevice, st->stream));
     }
+    const StatusScope scope(st->status);
     rc = launch_prefill_bf16(v, dx, m, bias != nullptr ? db : nullptr, dy, st->stream);
     if (rc != JQ_OK) {
         return rc;
     }
     JQ_CUDA(cudaMemcpyAsync(y, dy, (size_t)m * w->n * 4, cudaMemcpyDeviceToHost, st->stream));
-    JQ_CUDA(cudaStreamSynchronize(st->stream));
-    int status = 0;
-    rc = prefill_status(&status);
-    if (rc == JQ_OK && status != 0) {
-        rc = fail(JQ_ERR_TIMEOUT, "prefill kernel: a bounded wait gave up (code %d)", status);
-    }
-    return rc;
+    return staging_wait(st, "jq_linear_bf16");
 }
 
 int jq_device_status(int device, int* status) {
@@ -857,17 +933,12 @@ int jq_device_status(int device, int* status) {
     }
     DeviceGuard guard(device);
     JQ_CUDA(cudaDeviceSynchronize());
-    int rc = prefill_status(status);
-    int peer = 0;
-    if (rc == JQ_OK) {
-        rc = peer_status(&peer);
-    }
-    if (rc == JQ_OK && *status == 0) {
-        *status = peer;
-    }
+    int* const word = device_status_word(device);
+    *status = word != nullptr ? read_status(word) : 0;
+    int rc = JQ_OK;
     for (int part = 0; part < 4 && rc == JQ_OK; part++) {
         int other = 0;
-        rc = part == 0 ? gemv_peer_status(&other) : (part == 1 ? decoder_peer_status(&other) : (part == 2 ? gemv_umma_status(&other) : gemv_q6k_status(&other)));
+        rc = part == 0 ? peer_status(&other) : (part == 1 ? gemv_peer_status(&other) : (part == 2 ? decoder_peer_status(&other) : gemv_umma_peer_status(&other)));
         if (rc == JQ_OK && *status == 0) {
             *status = other;
         }

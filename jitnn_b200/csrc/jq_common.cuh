@@ -170,7 +170,6 @@ int launch_gemv_q4k_i8_imaged(const View& v, const View* v2, const uint8_t* imag
                               const PeerOut* peer = nullptr, const View* v3 = nullptr, float* y3 = nullptr);
 // Status word of the waits a GEMV makes itself for a peer exchange (peer_wait_inline): 0 or 32 + rank, cleared by the call.
 int gemv_peer_status(int* status);
-int gemv_q6k_status(int* status);  // the same for the Q6_K kernel's weight-ring waits (0 or 25)
 // Pieces of the peer exchange (jq_peer.cu) for the row-sharded decoder: the bounded wait for all ranks' flags of this
 // rank's latest exchange, and a Q4_K row shard applied to an activation image that is already complete, its outputs
 // stored into every rank's y [1, n_total] at payload_offset, followed by that wait.
@@ -200,6 +199,27 @@ int scratch_for_slot(cudaStream_t s, int slot, size_t bytes, uint8_t** out);
 int scratch_zeroed_for_slot(cudaStream_t s, int slot, size_t bytes, uint8_t** out);
 // For a stream of the library's own that is about to be destroyed.
 void scratch_release(cudaStream_t s);
+// Status words: where kernels record that a bounded wait gave up. Page-locked host memory that the device writes, so that reading one costs
+// no copy. A call that waits for its own result gives its kernels a word of its own (StatusScope) and learns of its own failures alone; the
+// kernels of calls that only enqueue work write to the word of their device, which jq_device_status reads.
+int status_word(int** word);          // for the kernels launched now, on the current device
+int take_status_word(int** word);     // a zeroed word; give_status_word returns it
+void give_status_word(int* word);
+int* device_status_word(int device);  // nullptr before the first weight of that device
+// The code in a word (0: no wait gave up), which is cleared. After the work that may write it has ended.
+inline int read_status(int* word) {
+    volatile int* v = word;
+    const int code = *v;
+    if (code != 0) {
+        *v = 0;
+    }
+    return code;
+}
+struct StatusScope {
+    int* before;
+    explicit StatusScope(int* word);
+    ~StatusScope();
+};
 
 // Decode GEMV on tcgen05 (jq_gemv_umma.cu): Q4_K and Q5_K, 1 to 16 rows of x in one pass over the weights.
 bool gemv_umma_takes(int type, int64_t k, int rows);  // under option gemv_tcgen05 = 1
@@ -211,7 +231,7 @@ int launch_gemv_umma(const View& v, const View* v2, const float* x, uint8_t* ima
                      const PeerOut* peer = nullptr, bool no_scratch = false);
 int launch_gemv_umma_multi(const View* vs, int count, const float* x, uint8_t* image, int rows, const float* bias, float* const* ys, cudaStream_t s,
                            const PeerOut* peer = nullptr, bool no_scratch = false);
-int gemv_umma_status(int* status);
+int gemv_umma_peer_status(int* status);  // 0, or 32 + rank once a wait of its peer exchange has given up
 // Option "gemv_tcgen05": 1 sends Q4_K and Q5_K decode (1 to 16 rows) to the tcgen05 GEMV, 2 never, 0 where the mma.sync kernel declines.
 extern std::atomic<int64_t> g_opt_gemv_umma;
 // Option "wait_limit_us": microseconds after which a bounded device-side wait of the tcgen05 GEMV gives up.
@@ -232,7 +252,6 @@ bool prefill_supported(const View& v);
 int launch_prefill_bf16(const View& v, const uint16_t* x_bf16, int64_t m, const float* bias, float* y, cudaStream_t s);
 int launch_prefill_bf16_multi(const View* vs, int count, const uint16_t* x_bf16, int64_t m, const float* bias, float* const* ys, cudaStream_t s);
 int launch_f32_to_bf16(const float* x, uint16_t* out, int64_t count, cudaStream_t s);
-int prefill_status(int* status);
 // Same for the bounded waits of the peer gather (jq_peer.cu): 0, or 32 + the rank whose slice did not arrive.
 int peer_status(int* status);
 

@@ -1026,6 +1026,7 @@ struct jq_decoder {
     int* counters;               // [dim / 256 attention merge counters][one argmax counter per row], zero between launches
     float* argmax_v;             // [rows][ARGMAX_CTAS] per-CTA best value
     int* argmax_i;               // [rows][ARGMAX_CTAS] per-CTA best index
+    int* status;         // status word of this decoder's kernels
     int* host_stage;     // pinned: [0..7] tokens in, [8] position in, [9..16] argmax out
     int sequences;       // key/value caches held (jq_decoder_set_sequences)
     int cur_seq;         // the sequence the call being enqueued works on
@@ -1095,6 +1096,7 @@ JQ_API int jq_decoder_destroy(jq_decoder* d) {
     cudaFree(d->argmax_v);
     cudaFree(d->argmax_i);
     cudaFreeHost(d->host_stage);
+    give_status_word(d->status);
     cudaFree(d->prompt_buf);
     cudaFree(d->prompt_bf16);
     cudaFree(d->prompt_tokens);
@@ -1196,6 +1198,7 @@ JQ_API int jq_decoder_create(int device, int layers, int dim, int heads, int kv_
     }
     d->tokens = d->pos = d->argmax = nullptr;
     d->host_stage = nullptr;
+    d->status = nullptr;
     d->img_q4k = d->img_q6k = nullptr;
     d->counters = nullptr;
     d->argmax_v = nullptr;
@@ -1220,6 +1223,7 @@ JQ_API int jq_decoder_create(int device, int layers, int dim, int heads, int kv_
         if (e == cudaSuccess) e = cudaMalloc(&d->argmax_i, T * ARGMAX_CTAS * sizeof(int));
     }
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&d->own_stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess && take_status_word(&d->status) != JQ_OK) e = cudaErrorMemoryAllocation;
     if (e == cudaSuccess) {
         // cos / sin tables in double, stored as float (ops/Rope.java:84-101)
         const int half = head_dim / 2;
@@ -1865,6 +1869,12 @@ static int enqueue_forward_sharded(jq_decoder* d, int T, int max_keys, const Tok
     return rc;
 }
 
+// Whether a bounded wait has given up in this call, or in those since the last one that waited for the GPU.
+static int decoder_status(jq_decoder* d, const char* who) {
+    const int code = read_status(d->status);
+    return code == 0 ? JQ_OK : fail(JQ_ERR_TIMEOUT, "%s: a bounded wait on the device gave up (code %d)", who, code);
+}
+
 // Captures the decode step of T tokens for up to 256 << bucket cached positions.
 static int capture_step(jq_decoder* d, int T, int bucket, cudaStream_t s) {
     cudaGraph_t g = nullptr;
@@ -1931,6 +1941,7 @@ static int decoder_forward(jq_decoder* d, int seq, bool batch, const int32_t* to
     if (prev != d->device) {
         JQ_CUDA(cudaSetDevice(d->device));
     }
+    const StatusScope scope(d->status);
     // all state of a decoder is private to it and its inputs come from the host, so its own stream is as good as any
     cudaStream_t s = stream != nullptr ? (cudaStream_t)stream : d->own_stream;
     const int T = n_tokens;
@@ -1992,6 +2003,9 @@ static int decoder_forward(jq_decoder* d, int seq, bool batch, const int32_t* to
             CK(cudaMemcpyAsync(logits_host, src, (size_t)T * d->vocab * sizeof(float), cudaMemcpyDeviceToHost, s), "logits");
         }
         CK(cudaStreamSynchronize(s), "jq_decoder_forward");
+        if (rc == JQ_OK) {
+            rc = decoder_status(d, "jq_decoder_forward");
+        }
         if (rc == JQ_OK && d->world > 1) {
             int status = 0, part = 0;
             rc = peer_status(&status);
@@ -2101,6 +2115,7 @@ JQ_API int jq_decoder_prompt(jq_decoder* d, int seq, const int32_t* tokens_host,
     if (prev != d->device) {
         JQ_CUDA(cudaSetDevice(d->device));
     }
+    const StatusScope scope(d->status);
     cudaStream_t s = stream != nullptr ? (cudaStream_t)stream : d->own_stream;
     const int T = n_tokens, dim = d->dim, hd = d->head_dim, hidden = d->hidden;
     const int64_t kv_dim = (int64_t)d->kv_heads * hd;
@@ -2197,11 +2212,7 @@ JQ_API int jq_decoder_prompt(jq_decoder* d, int seq, const int32_t* tokens_host,
         }
         CK(cudaStreamSynchronize(s), "jq_decoder_prompt");
         if (rc == JQ_OK) {
-            int status = 0;
-            rc = prefill_status(&status);
-            if (rc == JQ_OK && status != 0) {
-                rc = fail(JQ_ERR_TIMEOUT, "jq_decoder_prompt: a bounded wait of the tensor-core kernel gave up (code %d)", status);
-            }
+            rc = decoder_status(d, "jq_decoder_prompt");
         }
         if (rc == JQ_OK && next_host != nullptr) {
             next_host[0] = d->host_stage[MAX_TOKENS + 1];

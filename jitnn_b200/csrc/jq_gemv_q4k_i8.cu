@@ -152,7 +152,7 @@ constexpr int NORM_MAX = 4;
 template <int MT, int STAGES, int NW, int OCC, bool Q5, bool PEER, From SRC>
 __global__ void __launch_bounds__(NW * 32, OCC) gemv_q4k_i8_kernel(View v, Second w2, const PeerOut* __restrict__ peerp, const uint8_t* __restrict__ image,
                                                                   const float* __restrict__ xin, int rows, const float* __restrict__ bias, float* __restrict__ y,
-                                                                  int tiles, int KS, int max_tiles, long long wait_clocks, NormInput norm) {
+                                                                  int tiles, int KS, int max_tiles, long long wait_clocks, int* status, NormInput norm) {
     // Tiles 0 .. w2.first_tiles - 1 are rows of v, the tiles from w2.first_tiles on rows of the second weight w2 (same k,
     // same x, its own output), if there is one.
     // KS = super-blocks of k per slice: the activation image of one slice is resident in shared memory at a time;
@@ -526,7 +526,7 @@ __global__ void __launch_bounds__(NW * 32, OCC) gemv_q4k_i8_kernel(View v, Secon
                         const long long t0 = clock64();
                         while (!tc::mbar_try(bar, cmp_phase)) {
                             if (clock64() - t0 > wait_clocks) {
-                                atomicCAS(&g_gemv_peer_status, 0, 24);
+                                tc::record_status(status, 24);
                                 gave_up = true;
                                 break;
                             }
@@ -626,6 +626,11 @@ __global__ void __launch_bounds__(NW * 32, OCC) gemv_q4k_i8_kernel(View v, Secon
             parity ^= 1;
         }
     }
+    if (gave_up) {
+        for (int i = 0; i < 1000; i++) {
+            __nanosleep(1000);  // copies that may still be in flight land long before this millisecond is over
+        }
+    }
     QT(5);
     if constexpr (PEER) {
         if (peer_marks) {
@@ -672,8 +677,13 @@ int launch(const View& v, const Second& w2, const PeerOut& peer, const uint8_t* 
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const long long wait_clocks = (long long)g_opt_wait_limit_us.load(std::memory_order_relaxed) * 2000;  // about 2 GHz
+    int* status = nullptr;
+    const int rc = status_word(&status);
+    if (rc != JQ_OK) {
+        return rc;
+    }
     JQ_CUDA(cudaLaunchKernelEx(&cfg, gemv_q4k_i8_kernel<MT, STAGES, NW, OCC, Q5, PEER, SRC>, v, w2, (const PeerOut*)(PEER ? peer.table : nullptr), image, x, rows,
-                               bias, y, tiles, KS, max_tiles, wait_clocks, norm));
+                               bias, y, tiles, KS, max_tiles, wait_clocks, status, norm));
     count_launch();
     return JQ_OK;
 }

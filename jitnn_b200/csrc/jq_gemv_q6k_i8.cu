@@ -99,7 +99,6 @@ __device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {
 // ---- activations -> image (scratch buffer in global memory) ---------------------------------------------------
 // One warp per (super-block of k, row of x).
 constexpr int PREP_WARPS = 4;
-__device__ int g_q6k_status;  // 0, or 25 once a wait for the weight ring has given up
 
 template <int MT>
 __global__ void __launch_bounds__(PREP_WARPS * 32) q6k_activation_image_kernel(const float* __restrict__ x, int rows, int64_t k,
@@ -117,7 +116,7 @@ __global__ void __launch_bounds__(PREP_WARPS * 32) q6k_activation_image_kernel(c
 template <int MT, int STAGES, int OCC>
 __global__ void __launch_bounds__(THREADS, OCC) gemv_q6k_i8_kernel(View v, const uint8_t* __restrict__ image, int rows,
                                                                   const float* __restrict__ bias, float* __restrict__ y, int tiles,
-                                                                  int KS, int max_tiles, long long wait_clocks) {
+                                                                  int KS, int max_tiles, long long wait_clocks, int* status) {
     // KS = super-blocks of k per slice: the activation image of one slice is resident in shared memory at a time;
     // with more than one slice the per-tile sums are carried in shared memory (max_tiles tiles per CTA).
     using C = Cfg<MT>;
@@ -344,7 +343,7 @@ __global__ void __launch_bounds__(THREADS, OCC) gemv_q6k_i8_kernel(View v, const
                         const long long t0 = clock64();
                         while (!tc::mbar_try(bar, cmp_phase)) {
                             if (clock64() - t0 > wait_clocks) {
-                                atomicCAS(&g_q6k_status, 0, 25);
+                                tc::record_status(status, 25);
                                 gave_up = true;
                                 break;
                             }
@@ -405,6 +404,11 @@ __global__ void __launch_bounds__(THREADS, OCC) gemv_q6k_i8_kernel(View v, const
             parity ^= 1;
         }
     }
+    if (gave_up) {
+        for (int i = 0; i < 1000; i++) {
+            __nanosleep(1000);  // copies that may still be in flight land long before this millisecond is over
+        }
+    }
 }
 
 int g_sms = 0;
@@ -441,7 +445,12 @@ int launch(const View& v, const uint8_t* image, int rows, const float* bias, flo
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const long long wait_clocks = (long long)g_opt_wait_limit_us.load(std::memory_order_relaxed) * 2000;  // about 2 GHz
-    JQ_CUDA(cudaLaunchKernelEx(&cfg, gemv_q6k_i8_kernel<MT, STAGES, OCC>, v, image, rows, bias, y, tiles, KS, max_tiles, wait_clocks));
+    int* status = nullptr;
+    const int rc = status_word(&status);
+    if (rc != JQ_OK) {
+        return rc;
+    }
+    JQ_CUDA(cudaLaunchKernelEx(&cfg, gemv_q6k_i8_kernel<MT, STAGES, OCC>, v, image, rows, bias, y, tiles, KS, max_tiles, wait_clocks, status));
     count_launch();
     return JQ_OK;
 }
@@ -537,14 +546,6 @@ int launch_gemv_q6k_i8(const View& v, const float* x, int rows, const float* bia
     if (rows == 1) return run<1>(v, x, rows, bias, y, s, image, handled);
     if (rows == 2) return run<2>(v, x, rows, bias, y, s, image, handled);
     return run<4>(v, x, rows, bias, y, s, image, handled);
-}
-
-// Reads and clears the status of the weight-ring waits on the current device.
-int gemv_q6k_status(int* status) {
-    const int zero = 0;
-    JQ_CUDA(cudaMemcpyFromSymbol(status, g_q6k_status, sizeof(int)));
-    JQ_CUDA(cudaMemcpyToSymbol(g_q6k_status, &zero, sizeof(int)));
-    return JQ_OK;
 }
 
 size_t q6k_image_bytes_one_row(int64_t k) { return (size_t)(k / 256) * Cfg<1>::PB; }

@@ -37,8 +37,7 @@
 
 namespace jq {
 
-// 0, or 64 + the role whose wait gave up first (1 copy issue, 2 MMA issue, 3 unpack, 4 epilogue) since the last read.
-static __device__ int g_umma_status;
+// Status codes: 64 + the role whose wait gave up (1 copy issue, 2 MMA issue, 3 unpack, 4 epilogue).
 static __device__ int g_umma_peer_status;
 
 // Development aid, compiled in with -DJQ_UMMA_TRACE: CTA 0 records clock64() at the hand-over points of every role for
@@ -113,6 +112,7 @@ struct UArgs {
     int max_pieces;
     int whole_tiles;        // non-zero: every CTA's run is whole tiles (partial is not used)
     long long wait_clocks;  // clocks after which a bounded wait gives up
+    int* status;
     uint32_t lbo, sbo;      // byte offsets of the image's shared-memory descriptor
     const PeerOut* peer;
 };
@@ -183,24 +183,25 @@ __device__ __forceinline__ uint64_t smem_desc_plain(uint32_t addr, uint32_t lbo,
 struct Phase {
     uint32_t bar, parity;
 };
-__device__ __forceinline__ bool wait_phases(const Phase& p0, const Phase& p1, const Phase& p2, bool use2, volatile int* abort_flag, int code, long long limit) {
+__device__ __forceinline__ bool wait_phases(const Phase& p0, const Phase& p1, const Phase& p2, bool use2, volatile int* abort_flag, int* status, int code,
+                                            long long limit) {
     const bool r0 = tc::mbar_try(p0.bar, p0.parity);
     const bool r1 = tc::mbar_try(p1.bar, p1.parity);
     const bool r2 = use2 ? tc::mbar_try(p2.bar, p2.parity) : true;
     if (r0 && r1 && r2) {
         return true;
     }
-    return (r0 || tc::mbar_wait(p0.bar, p0.parity, abort_flag, &g_umma_status, code, limit)) &&
-           (r1 || tc::mbar_wait(p1.bar, p1.parity, abort_flag, &g_umma_status, code, limit)) &&
-           (r2 || tc::mbar_wait(p2.bar, p2.parity, abort_flag, &g_umma_status, code, limit));
+    return (r0 || tc::mbar_wait(p0.bar, p0.parity, abort_flag, status, code, limit)) &&
+           (r1 || tc::mbar_wait(p1.bar, p1.parity, abort_flag, status, code, limit)) &&
+           (r2 || tc::mbar_wait(p2.bar, p2.parity, abort_flag, status, code, limit));
 }
 // The same on behalf of a whole warp: lane 0 polls (32 lanes polling one word would serialise), the outcome goes to the other
 // lanes, and __shfl_sync orders their later reads behind lane 0's acquire.
-__device__ __forceinline__ bool warp_wait_phases(const Phase& p0, const Phase& p1, const Phase& p2, bool use2, volatile int* abort_flag, int code,
+__device__ __forceinline__ bool warp_wait_phases(const Phase& p0, const Phase& p1, const Phase& p2, bool use2, volatile int* abort_flag, int* status, int code,
                                                  long long limit, int lane) {
     int ok = 1;
     if (lane == 0) {
-        ok = wait_phases(p0, p1, p2, use2, abort_flag, code, limit) ? 1 : 0;
+        ok = wait_phases(p0, p1, p2, use2, abort_flag, status, code, limit) ? 1 : 0;
     }
     return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
@@ -491,7 +492,7 @@ __global__ void __launch_bounds__(Roles<MR>::THREADS, 1) gemv_umma_kernel(const 
                 } else if (idle_since == 0) {
                     idle_since = clock64();
                 } else if (clock64() - idle_since > limit) {
-                    atomicCAS(&g_umma_status, 0, 64 + 1);
+                    tc::record_status(a.status, 64 + 1);
                     *abort_flag = 1;
                     break;
                 }
@@ -533,7 +534,7 @@ __global__ void __launch_bounds__(Roles<MR>::THREADS, 1) gemv_umma_kernel(const 
                         return false;
                     }
                     if (clock64() - t0 > limit) {
-                        atomicCAS(&g_umma_status, 0, 64 + 2);
+                        tc::record_status(a.status, 64 + 2);
                         *abort_flag = 1;
                         return false;
                     }
@@ -553,7 +554,7 @@ __global__ void __launch_bounds__(Roles<MR>::THREADS, 1) gemv_umma_kernel(const 
             }
             for (int i = first; i < units && ok; i += 2) {
                 ok = my_turn(dr.s, filling[dr.s]) &&
-                     wait_phases(Phase{full_a(ar.s), ar.ph}, Phase{empty_d(dr.s), dr.ph ^ 1u}, Phase{full_x(xr.s), xr.ph}, !RES, abort_flag, 64 + 2, limit);
+                     wait_phases(Phase{full_a(ar.s), ar.ph}, Phase{empty_d(dr.s), dr.ph ^ 1u}, Phase{full_x(xr.s), xr.ph}, !RES, abort_flag, a.status, 64 + 2, limit);
                 if (!ok) {
                     break;
                 }
@@ -606,7 +607,7 @@ __global__ void __launch_bounds__(Roles<MR>::THREADS, 1) gemv_umma_kernel(const 
         for (int i = 0; i < units; i++) {
             const int ws = wr.s, as = ar.s, ps = pr.s;
             // the weights have landed, the MMAs that read the A stage before have finished, the epilogue has read the parameter slot
-            if (!warp_wait_phases(Phase{full_w(ws), wr.ph}, Phase{empty_a(as), ar.ph ^ 1u}, Phase{empty_p(ps), pr.ph ^ 1u}, true, abort_flag, 64 + 3, limit,
+            if (!warp_wait_phases(Phase{full_w(ws), wr.ph}, Phase{empty_a(as), ar.ph ^ 1u}, Phase{empty_p(ps), pr.ph ^ 1u}, true, abort_flag, a.status, 64 + 3, limit,
                                   lane)) {
                 break;
             }
@@ -780,7 +781,7 @@ __global__ void __launch_bounds__(Roles<MR>::THREADS, 1) gemv_umma_kernel(const 
                             if (t0 == 0) {
                                 t0 = clock64();
                             } else if (*abort_flag != 0 || clock64() - t0 > limit) {
-                                atomicCAS(&g_umma_status, 0, 64 + 5);
+                                tc::record_status(a.status, 64 + 5);
                                 *abort_flag = 1;
                                 good = false;
                                 break;
@@ -826,7 +827,7 @@ __global__ void __launch_bounds__(Roles<MR>::THREADS, 1) gemv_umma_kernel(const 
                     break;
                 }
             }
-            if (!warp_wait_phases(Phase{full_p(ps), pr.ph}, Phase{full_d(dr.s), dr.ph}, Phase{full_x(xs), xr.ph}, !RES, abort_flag, 64 + 4, limit, lane)) {
+            if (!warp_wait_phases(Phase{full_p(ps), pr.ph}, Phase{full_d(dr.s), dr.ph}, Phase{full_x(xs), xr.ph}, !RES, abort_flag, a.status, 64 + 4, limit, lane)) {
                 ok = false;
                 break;
             }
@@ -1157,6 +1158,10 @@ int launch_gemv_umma_multi(const View* vs, int count, const float* x, uint8_t* i
     a.SW = sw > MAX_SW ? MAX_SW : sw;
     const size_t smem = fixed + (size_t)a.SW * ROWS * bb;
     a.wait_clocks = g_opt_wait_limit_us.load(std::memory_order_relaxed) * 2000;  // about 2 GHz
+    const int status_rc = status_word(&a.status);
+    if (status_rc != JQ_OK) {
+        return status_rc;
+    }
     a.lbo = (uint32_t)(ncols / 8) * 128u;
     a.sbo = 128u;
     a.peer = peer != nullptr ? peer->table : nullptr;
@@ -1202,17 +1207,11 @@ extern "C" JQ_API int jq_debug_umma_cta(long long* out) {
 }
 namespace jq {
 #endif
-// Reads and clears the status words of the tcgen05 GEMV on the current device (0 = no wait ever gave up).
-int gemv_umma_status(int* status) {
+// Reads and clears the status of the peer exchange's waits on the current device.
+int gemv_umma_peer_status(int* status) {
     const int zero = 0;
-    int peer = 0;
-    JQ_CUDA(cudaMemcpyFromSymbol(status, g_umma_status, sizeof(int)));
-    JQ_CUDA(cudaMemcpyToSymbol(g_umma_status, &zero, sizeof(int)));
-    JQ_CUDA(cudaMemcpyFromSymbol(&peer, g_umma_peer_status, sizeof(int)));
+    JQ_CUDA(cudaMemcpyFromSymbol(status, g_umma_peer_status, sizeof(int)));
     JQ_CUDA(cudaMemcpyToSymbol(g_umma_peer_status, &zero, sizeof(int)));
-    if (*status == 0) {
-        *status = peer;
-    }
     return JQ_OK;
 }
 

@@ -9,8 +9,6 @@
 
 namespace jq {
 
-static __device__ int g_matmul_status;
-
 namespace mm {
 
 // x [m, k] FP32 (or silu(x) * up) -> two planes of halves [2][m][width] (hi, lo) and a scale per (BLK values of k, row of x): the block's values times a power of
@@ -106,20 +104,7 @@ __global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ x,
     }
 }
 
-static int status_word(int** out) {
-    static std::atomic<int*> known[64];
-    int dev = 0;
-    JQ_CUDA(cudaGetDevice(&dev));
-    int* p = known[dev & 63].load(std::memory_order_acquire);
-    if (p == nullptr) {
-        void* a = nullptr;
-        JQ_CUDA(cudaGetSymbolAddress(&a, g_matmul_status));
-        p = static_cast<int*>(a);
-        known[dev & 63].store(p, std::memory_order_release);
-    }
-    *out = p;
-    return JQ_OK;
-}
+static long long wait_clocks() { return (long long)g_opt_wait_limit_us.load(std::memory_order_relaxed) * 2000; }  // about 2 GHz
 
 static int unit_bytes(int type) { return TILE_ROWS * (plane_q_bytes(type) + plane_aux_bytes(type)) * 256 / block_values(type); }
 
@@ -433,6 +418,7 @@ static int product_f32(const View* vs, int count, bool bwd, const float* x, cons
                         a.xstride = stride;
                         a.bias = bias;
                         a.status = status;
+                        a.wait_clocks = wait_clocks();
                         rc = launch_any(type, parts.part[c].plan, a, map, s);
                     }
                 }
@@ -519,6 +505,7 @@ int launch_prefill_bf16_multi(const View* vs, int count, const uint16_t* x_bf16,
             if (rc == JQ_OK) {
                 a.bias = i == 0 ? bias : nullptr;
                 a.status = status;
+                a.wait_clocks = wait_clocks();
                 rc = launch_any(vs[i].type, parts.part[c].plan, a, map, s);
             }
         }
@@ -565,14 +552,6 @@ int launch_f32_to_bf16(const float* x, uint16_t* out, int64_t count, cudaStream_
     f32_to_bf16_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(x, reinterpret_cast<__nv_bfloat16*>(out), count);
     count_launch();
     return check_launch("f32_to_bf16_kernel");
-}
-
-// Reads and clears the status word of the matrix kernel on the current device (0 = no wait ever gave up).
-int prefill_status(int* status) {
-    int zero = 0;
-    JQ_CUDA(cudaMemcpyFromSymbol(status, g_matmul_status, sizeof(int)));
-    JQ_CUDA(cudaMemcpyToSymbol(g_matmul_status, &zero, sizeof(int)));
-    return JQ_OK;
 }
 
 }  // namespace jq

@@ -58,7 +58,6 @@ struct Shape {
     static constexpr bool OWNED = TURNS == 1;                           // a raw unit is one group's own
 };
 constexpr int A_TILE = 128 * 128;  // 128 rows of 128 bytes
-constexpr long long WAIT_CLOCKS = 4000000000ll;  // about two seconds
 constexpr int MAX_A = 6, MAX_B = 12, MAX_RAW = 6;
 constexpr int FACTORS = 8;   // units whose factors the fold may still need: operands in flight and accumulators, see where they are written
 constexpr int VIRTUAL = 8;   // ranges of the contraction whose sums are added up in order, whatever the cluster (instances for 16 rows of x)
@@ -88,8 +87,9 @@ struct Args {
     const float* xscale;  // FP32: scale of (contraction block, row of x): [block][xstride]
     int xstride;
     const float* bias;    // of the first weight, or null
-    int* status;      // 0, or the code of the first wait that gave up: 1 operand free, 2 weights ready, 3 activations ready or their tile free,
+    int* status;      // receives the code of a wait that gives up: 1 operand free, 2 weights ready, 3 activations ready or their tile free,
                       // 4 accumulator ready, 5 accumulator free, 6 raw blocks, 8 raw blocks read by all
+    long long wait_clocks;  // after which a wait gives up
 };
 
 // Shared-memory matrix descriptors, 128-byte swizzle (layout type 2), descriptor version 1 (sm_100). The high word is the same for all: 1024
@@ -148,31 +148,37 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// A bounded wait, as tc::mbar_wait. (A try_wait with a time limit of its own becomes a sleep in software that wakes late.)
-__device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+// A bounded wait, as tc::mbar_wait. (A try_wait with a time limit of its own becomes a sleep in software that wakes late.) Most roles start
+// before the kernel in front of this one has ended, and in the end all of them wait for what it writes: the limit counts from its end on. The
+// roles that have waited for it already (AFTER) need no second turn.
+template <bool AFTER = false>
+__device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, const Args& p, int code) {
     if (tc::mbar_try(bar, parity)) {
         return true;
     }
-    const long long t0 = clock64();
-    for (;;) {
-        if (tc::mbar_try(bar, parity)) {
-            return true;
-        }
-        if (*abort_flag != 0) {
-            return false;
-        }
-        if (clock64() - t0 > WAIT_CLOCKS) {
-            break;
+    for (int turn = AFTER ? 1 : 0; turn < 2; turn++) {
+        const long long t0 = clock64();
+        do {
+            if (tc::mbar_try(bar, parity)) {
+                return true;
+            }
+            if (*abort_flag != 0) {
+                return false;
+            }
+        } while (clock64() - t0 <= p.wait_clocks);
+        if (turn == 0) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");
         }
     }
-    atomicCAS(status, 0, code);
+    tc::record_status(p.status, code);
     *abort_flag = 1;
     return false;
 }
 
 // The same for a whole warp that goes on to warp-wide instructions: all lanes or none.
-__device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
-    return __all_sync(0xffffffffu, wait(bar, parity, abort_flag, status, code));
+template <bool AFTER = false>
+__device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, const Args& p, int code) {
+    return __all_sync(0xffffffffu, wait<AFTER>(bar, parity, abort_flag, p, code));
 }
 
 __device__ __forceinline__ void tma_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
@@ -344,7 +350,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                     constexpr int ALL = W::CHUNKS + (EXT ? 1 : 0);  // tiles per unit; the last one is the 16 more columns
                     for (int i = 0; i < ALL;) {
                         const int last = BT > 1 ? (i + TURN == W::CHUNKS ? ALL : i + TURN) : i + 1;
-                        if (!(ok = wait(free_b + 8 * s, ph, abort_flag, p.status, 3))) {
+                        if (!(ok = wait<true>(free_b + 8 * s, ph, abort_flag, p, 3))) {
                             break;
                         }
                         const uint32_t bar = full_b + 8 * s;
@@ -376,14 +382,14 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
             for (int u = u0; u < u1 && ok; u++) {
                 const uint32_t d = tmem + (uint32_t)(buf * p.cols);
                 if (FP32 || u == u0) {
-                    if (!(ok = wait_warp(acc_empty + 8 * buf, aph ^ 1u, abort_flag, p.status, 5))) {
+                    if (!(ok = wait_warp(acc_empty + 8 * buf, aph ^ 1u, abort_flag, p, 5))) {
                         break;
                     }
                     first = true;
                 }
 #pragma unroll
                 for (int turn = 0; turn < TURNS; turn++) {
-                    if (!(ok = __all_sync(0xffffffffu, ready) || wait_warp(full_a + 8 * s, ph, abort_flag, p.status, 2))) {
+                    if (!(ok = __all_sync(0xffffffffu, ready) || wait_warp(full_a + 8 * s, ph, abort_flag, p, 2))) {
                         break;
                     }
                     // asked before this operand's MMAs are issued: the answer takes over a hundred clocks even when it is yes
@@ -398,7 +404,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                             break;
                         }
                         if (BT == 1 || c == 0) {
-                            if (!(ok = __all_sync(0xffffffffu, ready_b) || wait_warp(full_b + 8 * sb, phb, abort_flag, p.status, 3))) {
+                            if (!(ok = __all_sync(0xffffffffu, ready_b) || wait_warp(full_b + 8 * sb, phb, abort_flag, p, 3))) {
                                 break;
                             }
                             ready_b = tc::mbar_test(full_b + 8 * (sb + 1 == SB ? 0 : sb + 1), sb + 1 == SB ? phb ^ 1 : phb);
@@ -489,7 +495,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                 const uint8_t* const wa = pick(p.aux, wi);
                 for (int u = u0; u < u1; u++) {
                     const int64_t at = BWD ? (int64_t)u * p.kb + (ft >> 1) : (int64_t)(ft - ft0) * p.kb + u;
-                    if (!(ok = wait(raw_read + 8 * r, ph, abort_flag, p.status, 8))) {
+                    if (!(ok = wait(raw_read + 8 * r, ph, abort_flag, p, 8))) {
                         break;
                     }
                     const uint32_t dst = raw0 + (uint32_t)r * raw_bytes<TYPE>(), bar = raw_full + 8 * r;
@@ -530,7 +536,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                     rph = rphn;
                     continue;
                 }
-                if (!__all_sync(0xffffffffu, raw_ready) && !(ok = wait_warp(raw_full + 8 * r, rph, abort_flag, p.status, 6))) {
+                if (!__all_sync(0xffffffffu, raw_ready) && !(ok = wait_warp(raw_full + 8 * r, rph, abort_flag, p, 6))) {
                     break;
                 }
                 if constexpr (OWNED) {
@@ -565,7 +571,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                                 tc::mbar_arrive(max_full + 8 * slot);
                             }
                         }
-                        if (!(ok = wait_warp(max_full + 8 * slot, (uint32_t)(at_unit >> 3) & 1u, abort_flag, p.status, 8))) {
+                        if (!(ok = wait_warp(max_full + 8 * slot, (uint32_t)(at_unit >> 3) & 1u, abort_flag, p, 8))) {
                             break;
                         }
                         uint32_t e = max(max(unit_max[slot * 4], unit_max[slot * 4 + 1]), max(unit_max[slot * 4 + 2], unit_max[slot * 4 + 3])) >> 23;
@@ -595,7 +601,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                         if constexpr (!HALF) {
                             D::values(head, raw[0], c0, 0, fac, w0, w1);
                         }
-                        if (!__all_sync(0xffffffffu, ready) && !(ok = wait_warp(free_a + 8 * s, ph, abort_flag, p.status, 1))) {
+                        if (!__all_sync(0xffffffffu, ready) && !(ok = wait_warp(free_a + 8 * s, ph, abort_flag, p, 1))) {
                             break;
                         }
                         if (FP32 && turn == 0) {
@@ -777,8 +783,8 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                         }
                     }
                     __syncwarp();
-                    ok = wait_warp(fac_full + 8 * (chunk & (FACTORS - 1)), (uint32_t)(chunk / FACTORS) & 1u, abort_flag, p.status, 6) &&
-                         wait_warp(acc_full + 8 * buf, aph, abort_flag, p.status, 4);
+                    ok = wait_warp<true>(fac_full + 8 * (chunk & (FACTORS - 1)), (uint32_t)(chunk / FACTORS) & 1u, abort_flag, p, 6) &&
+                         wait_warp<true>(acc_full + 8 * buf, aph, abort_flag, p, 4);
                     if (!ok) {
                         break;
                     }
@@ -862,7 +868,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                     }
                 }
             } else {
-                if (!(ok = wait_warp(acc_full + 8 * buf, aph, abort_flag, p.status, 4))) {
+                if (!(ok = wait_warp<true>(acc_full + 8 * buf, aph, abort_flag, p, 4))) {
                     break;
                 }
                 tc::fence_after_sync();

@@ -41,9 +41,15 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 
+// A wait gave up: `status` is a status word (page-locked host memory); of several codes written at a time any one will do.
+__device__ __forceinline__ void record_status(int* status, int code) {
+    *reinterpret_cast<volatile int*>(status) = code;
+    __threadfence_system();
+}
+
 // Waits for the phase with the given parity, for at most `limit` clocks of the SM (a poll may suspend the thread for a time the
 // hardware chooses, so the bound counts time, not polls). Gives up earlier when another role of the CTA has given up (abort
-// flag in shared memory); the first wait that runs out records `code` in *status (global memory).
+// flag in shared memory); a wait that runs out records `code` in the status word.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code, long long limit) {
     if (mbar_try(bar, parity)) {
         return true;
@@ -57,7 +63,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
             return false;
         }
         if (clock64() - t0 > limit) {
-            atomicCAS(status, 0, code);
+            record_status(status, code);
             *abort_flag = 1;
             return false;
         }

@@ -6,6 +6,7 @@ hanging anything: two peer buffers are allocated on the same device as "rank 0" 
 ever calls. Its exchange stores its slice into its own y and, as marked words, into the other buffer's staging area, then waits
 for rank 1's words in its own staging area, which nothing writes: the wait gives up after its limit (option "peer_wait_us",
 0.4 s by default), records 32 + 1 and the kernel returns.
+The matrix kernel's waits run out by themselves under a limit of a microsecond ("wait_limit_us"): its first accumulator takes longer.
 After a timeout the ranks' exchange numbers on those buffers are out of step: the buffers are to be freed and allocated anew
 (jq_peer_free / jq_peer_alloc), which is what the test does before it checks that the device still works.
 """
@@ -18,6 +19,7 @@ import torch
 
 import jitnn_b200
 from jitnn_b200 import Gguf, Tensor, _lib, synth
+from oracle import llama_oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -113,3 +115,76 @@ def test_a_table_slot_is_never_reused_for_another_target():
     torch.cuda.synchronize()
     assert status(L) == 0
     _lib.check(L.jq_peer_free(p))
+
+
+@pytest.fixture()
+def short_waits():
+    L = jitnn_b200.load()
+    torch.cuda.synchronize()
+    assert status(L) == 0
+    _lib.check(L.jq_set_option(b"wait_limit_us", 1))
+    yield L
+    _lib.check(L.jq_set_option(b"wait_limit_us", 2000000))
+
+
+def gives_up(call):
+    """Whether one of a few calls does: an FP32 product's first accumulator takes one to three microseconds. (A bfloat16 one adds up the whole k
+    before anybody gets it.)"""
+    for _ in range(30):
+        try:
+            call()
+        except TimeoutError as e:
+            assert "gave up" in str(e)
+            return True
+    return False
+
+
+def test_the_matrix_kernel_gives_up(short_waits):
+    """Host calls report their own waits, and nobody else's; calls with device memory leave a code for jq_device_status."""
+    L = short_waits
+    n, k, m = 11008, 4096, 200
+    w = Tensor.quantized("Q4_0", synth.random_valid_blocks("Q4_0", n, k, seed=2).numpy().reshape(-1), n, k)
+    rng = np.random.default_rng(1)
+    x, g = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((m, n)).astype(np.float32)
+    xb = torch.from_numpy(x).to(torch.bfloat16).view(torch.uint16).numpy()
+    calls = [lambda: Gguf.linear(x, w), lambda: Gguf.linear(x[:9], w), lambda: Gguf.linearBackward(g, w), lambda: Gguf.linearBf16(xb, w)]
+    for call in calls:
+        assert gives_up(call)
+        assert status(L) == 0
+    # with device memory: a code for whoever asks, and none of the host call's business
+    xd = torch.from_numpy(x).cuda()
+    Gguf.linearBf16(xd.to(torch.bfloat16), w)
+    torch.cuda.synchronize()
+    _lib.check(L.jq_set_option(b"wait_limit_us", 2000000))
+    done = [call() for call in calls]
+    assert 1 <= status(L) <= 8 and status(L) == 0
+    for got, want in zip(done, (Gguf.linear(xd, w), Gguf.linear(xd[:9], w), Gguf.linearBackward(torch.from_numpy(g).cuda(), w),
+                                Gguf.linearBf16(torch.from_numpy(x).cuda().to(torch.bfloat16), w))):
+        assert np.array_equal(got, want.cpu().numpy())
+    assert status(L) == 0
+
+
+def test_a_decoder_reports_its_own_waits(short_waits):
+    L = short_waits
+    cfg = llama_oracle.Config(layers=1, dim=2048, heads=16, kv_heads=16, hidden=5632, vocab=8192, max_seq=256)
+    model = llama_oracle.random_model(cfg, 1, formats={name: "Q8_0" for name in ("wq", "wk", "wv", "wo", "w1", "w2", "w3", "output")})
+    dec = jitnn_b200.LlamaDecoder(cfg.layers, cfg.dim, cfg.heads, cfg.kv_heads, cfg.hidden, cfg.vocab, cfg.max_seq, cfg.eps, cfg.rope_base)
+    dec.load(model)
+    dec.set_sequences(16)
+    toks = np.arange(200, dtype=np.int32)
+    with pytest.raises(TimeoutError, match="gave up"):
+        dec.prompt(toks, 0)
+    _lib.check(L.jq_set_option(b"decoder_graph", 0))  # a captured step would keep the short limit
+    try:
+        assert gives_up(lambda: dec.forward_batch(toks[:16], 0))
+    finally:
+        _lib.check(L.jq_set_option(b"decoder_graph", 1))
+    for _ in range(30):
+        dec.enqueue(toks[:16], 0)  # reported by the next call that waits
+    _lib.check(L.jq_set_option(b"wait_limit_us", 2000000))
+    with pytest.raises(TimeoutError, match="gave up"):
+        dec.forward_batch(toks[:16], 0)
+    got, _ = dec.forward_batch(toks[:16], 0)
+    assert np.isfinite(got).all()
+    assert status(L) == 0
+    dec.close()
