@@ -289,7 +289,6 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
     uint8_t* const generic = smem_unaligned + (slot_s - tc::smem_u32(smem_unaligned));
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(generic);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(generic + 4);
-    volatile uint32_t* unit_max = reinterpret_cast<volatile uint32_t*>(generic + 16);  // backward: [8 units][4 warps] largest bounds
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int range = p.ksplit == 1 ? 0 : (int)cluster_rank();  // which range of the contraction
@@ -315,7 +314,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
             tc::mbar_init(acc_empty + 8 * i, W::FOLD);
         }
         for (int i = 0; i < FACTORS; i++) {
-            tc::mbar_init(fac_full + 8 * i, BWD ? 1 : 4);
+            tc::mbar_init(fac_full + 8 * i, BWD ? 2 : 4);
         }
         for (int i = 0; i < 8; i++) {
             tc::mbar_init(max_full + 8 * i, 4);
@@ -553,8 +552,8 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                 } else {
                     const uint32_t uq = raw0 + (uint32_t)r * raw_bytes<TYPE>(), ua = uq + D::UNIT_Q;
                     typename D::Head head;
-                    float fac = 1.0f;
-                    uint32_t unit_factor = 0;  // what the fold multiplies the unit's sums by
+                    float f0 = 1.0f, f1 = 1.0f;
+                    uint32_t unit_factor = 0, unit_factor1 = 0;  // what the fold multiplies the unit's sums by
                     if constexpr (!BWD) {
                         head = D::head(uq, ua, row0);
                     }
@@ -562,22 +561,38 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                         unit_factor = __float_as_uint(H::factor(head));
                     }
                     if constexpr (BWD) {
-                        // a power of two brings the largest weight that the unit's blocks can hold to [2^13, 2^14); the fold multiplies by its inverse
+                        // For every 32 features a power of two brings the largest weight that their blocks can hold to [2^13, 2^14); the fold
+                        // multiplies by its inverse. (Features are outputs of their own: with one power of two for all 128, blocks 2^-20 times
+                        // their neighbours' lost bits.) The unit's maxima [block][warp] lie behind its factors.
                         const int slot = at_unit & 7;  // a group is at most four turns, so fewer than eight units, ahead of another
+                        const uint32_t maxima = fac0 + (uint32_t)slot * 512u + 64u;
                         if (first == 0) {
-                            const uint32_t b = __reduce_max_sync(0xffffffffu, __float_as_uint(D::bound(D::head(uq, ua, tid))));
+                            float b[4];
+                            D::bounds(D::head(uq, ua, tid), h, b);
+#pragma unroll
+                            for (int i = 0; i < 4; i++) {
+                                const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(b[i]));
+                                if (lane == 0) {
+                                    asm volatile("st.shared.u32 [%0], %1;" ::"r"(maxima + 16u * i + 4u * (uint32_t)(tid >> 5)), "r"(m) : "memory");
+                                }
+                            }
                             if (lane == 0) {
-                                unit_max[slot * 4 + (tid >> 5)] = b;
                                 tc::mbar_arrive(max_full + 8 * slot);
                             }
                         }
                         if (!(ok = wait_warp(max_full + 8 * slot, (uint32_t)(at_unit >> 3) & 1u, abort_flag, p, 8))) {
                             break;
                         }
-                        uint32_t e = max(max(unit_max[slot * 4], unit_max[slot * 4 + 1]), max(unit_max[slot * 4 + 2], unit_max[slot * 4 + 3])) >> 23;
-                        e = e < 40u ? 40u : (e > 254u ? 254u : e);
-                        fac = __uint_as_float((267u - e) << 23);
-                        unit_factor = (e - 13u) << 23;
+                        auto exponent = [&](int block) {
+                            const uint4 m = lds16(maxima + 16u * (uint32_t)block);
+                            const uint32_t e = max(max(m.x, m.y), max(m.z, m.w)) >> 23;
+                            return e < 40u ? 40u : (e > 254u ? 254u : e);
+                        };
+                        const uint32_t e0 = exponent(2 * (tid >> 6)), e1 = exponent(2 * (tid >> 6) + 1);
+                        f0 = __uint_as_float((267u - e0) << 23);
+                        f1 = __uint_as_float((267u - e1) << 23);
+                        unit_factor = (e0 - 13u) << 23;
+                        unit_factor1 = (e1 - 13u) << 23;
                     }
                     for (int turn = first; turn < TURNS; turn += G) {
                         const bool ready = tc::mbar_test(free_a + 8 * s, ph);  // asked early: the answer takes longer than it looks
@@ -599,7 +614,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                         // the first values while it is on its way
                         f2 w0[8], w1[8];
                         if constexpr (!HALF) {
-                            D::values(head, raw[0], c0, 0, fac, w0, w1);
+                            D::values(head, raw[0], c0, 0, f0, f1, w0, w1);
                         }
                         if (!__all_sync(0xffffffffu, ready) && !(ok = wait_warp(free_a + 8 * s, ph, abort_flag, p, 1))) {
                             break;
@@ -609,11 +624,13 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                             // operands ago went through the tensor core, into an accumulator that the fold had emptied: the fold is done
                             // with the unit at least that far and `bufs` accumulators back, SA + bufs <= FACTORS.
                             const uint32_t fa = fac0 + (uint32_t)(at_unit & (FACTORS - 1)) * 512u;
-                            if (!BWD || tid == 0) {
-                                asm volatile("st.shared.u32 [%0], %1;" ::"r"(fa + (BWD ? 0u : 4u * (uint32_t)row0)), "r"(unit_factor) : "memory");
+                            if constexpr (!BWD) {
+                                asm volatile("st.shared.u32 [%0], %1;" ::"r"(fa + 4u * (uint32_t)row0), "r"(unit_factor) : "memory");
+                            } else if ((tid & 63) == 0) {  // one for every 32 features
+                                asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(fa + 8u * (uint32_t)(tid >> 6)), "r"(unit_factor), "r"(unit_factor1) : "memory");
                             }
                             __syncwarp();
-                            if (lane == 0 && (!BWD || tid == 0)) {
+                            if (lane == 0 && (!BWD || (tid & 63) == 0)) {
                                 tc::mbar_arrive(fac_full + 8 * (at_unit & (FACTORS - 1)));
                             }
                         }
@@ -621,7 +638,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                             const uint32_t to = a0 + (uint32_t)s * a_st + row_at;
                             run_to_smem<FP32>(w0, to, D::piece(0, 0), row0 & 7);
                             run_to_smem<FP32>(w1, to, D::piece(0, 1), row0 & 7);
-                            D::values(head, raw[0], c0, 1, fac, w0, w1);
+                            D::values(head, raw[0], c0, 1, f0, f1, w0, w1);
                             run_to_smem<FP32>(w0, to, D::piece(1, 0), row0 & 7);
                             run_to_smem<FP32>(w1, to, D::piece(1, 1), row0 & 7);
                             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic stores -> visible to the tensor core
@@ -644,11 +661,11 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                                     }
                                 } else {
                                     if (j > 0) {
-                                        D::values(head, raw[j], c0 + j, 0, fac, w0, w1);
+                                        D::values(head, raw[j], c0 + j, 0, f0, f1, w0, w1);
                                     }
                                     run_to_tmem(w0, tj, D::piece(0, 0));
                                     run_to_tmem(w1, tj, D::piece(0, 1));
-                                    D::values(head, raw[j], c0 + j, 1, fac, w0, w1);
+                                    D::values(head, raw[j], c0 + j, 1, f0, f1, w0, w1);
                                     run_to_tmem(w0, tj, D::piece(1, 0));
                                     run_to_tmem(w1, tj, D::piece(1, 1));
                                 }
@@ -790,7 +807,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                     }
                     tc::fence_after_sync();
                     float f;
-                    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"(fac0 + (uint32_t)(chunk & (FACTORS - 1)) * 512u + (BWD ? 0u : 4u * (uint32_t)lane_row)));
+                    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"(fac0 + (uint32_t)(chunk & (FACTORS - 1)) * 512u + 4u * (uint32_t)(BWD ? group : lane_row)));
                     const f2 ff = pack2(f, f);
                     const uint32_t d = tmem + lanes + (uint32_t)(buf * p.cols + c0);
 #pragma unroll

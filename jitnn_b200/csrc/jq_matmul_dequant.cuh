@@ -8,7 +8,8 @@
 // quarter of the rate), and one packed FMA applies scale and offset to two weights: a (P + q) + (c - P a) with P = 16, 32, 64 or
 // 32768. For Q8_0, Q4_0 and Q6_K every operand and result is exact, so the value is the reference's; for Q4_K, Q5_K and Q4_1 the
 // constant is rounded once, at most 2^-24 of the largest weight that the block can hold, which is what FP32 keeps anyway.
-// `fac` is a power of two that all values are multiplied by (exactly).
+// f0 and f1 are powers of two that the values of the chunk's first and second 32 are multiplied by (exactly). bounds(): the sizes that no
+// weight of blocks 4 h .. 4 h + 3 of 32 values exceeds (the backward product's powers of two).
 #pragma once
 
 #include "jq_formats.cuh"
@@ -94,22 +95,27 @@ struct DqK45 {
         const uint32_t at = uq + (uint32_t)row * ROW + (Q5 ? 48 : 16) + 32 * c;
         return Raw{{lds16(at), lds16(at + 16)}};
     }
-    // No weight of the row's 256 is larger.
-    __device__ static __forceinline__ float bound(const Head& r) {
-        return fmaf(fabsf(half_bits_to_float(r.h.x)), Q5 ? 1953.0f : 945.0f, 63.0f * fabsf(half_bits_to_float(r.h.x >> 16)));
+    __device__ static __forceinline__ void bounds(const Head& r, int h, float (&b)[4]) {
+        const float d = fabsf(half_bits_to_float(r.h.x)) * (Q5 ? 31.0f : 15.0f), dmin = fabsf(half_bits_to_float(r.h.x >> 16));
+        uint32_t sc, mn;  // sub-blocks 4 h .. 4 h + 3
+        scale_min_words(r.h, 2 * h, sc, mn);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            b[i] = fmaf(d, (float)byte_of(sc, i), dmin * (float)byte_of(mn, i));
+        }
     }
-    __device__ static __forceinline__ void values(const Head& r, const Raw& raw, int c, int part, float fac, f2 (&w0)[8], f2 (&w1)[8]) {
+    __device__ static __forceinline__ void values(const Head& r, const Raw& raw, int c, int part, float f0, float f1, f2 (&w0)[8], f2 (&w1)[8]) {
         const uint4 q = raw.q[part];
-        const float d = half_bits_to_float(r.h.x) * fac, dmin = half_bits_to_float(r.h.x >> 16) * fac;
+        const float d = half_bits_to_float(r.h.x), dmin = half_bits_to_float(r.h.x >> 16);
         uint32_t sc, mn;  // sub-blocks 2c and 2c + 1
         scale_min_words(r.h, c, sc, mn);
         sc >>= 16 * (c & 1);
         mn >>= 16 * (c & 1);
         // exact: 11 + 6 bits
-        const float a0 = d * (under2(sc, 0x47000000u, 0) - 32768.0f), a1 = d * (under2(sc, 0x47000000u, 1) - 32768.0f);
+        const float a0 = d * f0 * (under2(sc, 0x47000000u, 0) - 32768.0f), a1 = d * f1 * (under2(sc, 0x47000000u, 1) - 32768.0f);
         const float m0 = under2(mn, 0x47000000u, 0) - 32768.0f, m1 = under2(mn, 0x47000000u, 1) - 32768.0f;
         constexpr float P = Q5 ? 32.0f : 16.0f;
-        const float k0 = -fmaf(P, a0, dmin * m0), k1 = -fmaf(P, a1, dmin * m1);
+        const float k0 = -fmaf(P, a0, dmin * f0 * m0), k1 = -fmaf(P, a1, dmin * f1 * m1);
         const f2 A0 = pack2(a0, a0), A1 = pack2(a1, a1), K0 = pack2(k0, k0), K1 = pack2(k1, k1);
         const uint32_t w[4] = {q.x, q.y, q.z, q.w};
         const uint32_t g[4] = {r.hi[part].x, r.hi[part].y, r.hi[part].z, r.hi[part].w};
@@ -163,14 +169,20 @@ struct Dq<JQ_TYPE_Q6_K> {
         const uint32_t l = uq + (uint32_t)row * ROW + 64 * (c >> 1), h = uq + (uint32_t)row * ROW + 128 + 32 * (c >> 1);
         return Raw{{lds16(l), lds16(l + 16)}, {lds16(l + 32), lds16(l + 48)}, {lds16(h), lds16(h + 16)}};
     }
-    __device__ static __forceinline__ float bound(const Head& r) { return 4096.0f * fabsf(r.d); }
-    __device__ static __forceinline__ void values(const Head& r, const Raw& raw, int c, int part, float fac, f2 (&w0)[8], f2 (&w1)[8]) {
+    __device__ static __forceinline__ void bounds(const Head& r, int h, float (&b)[4]) {
+        const float d = 32.0f * fabsf(r.d);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {  // the scales of 32 values are two bytes
+            const uint32_t s = (h == 0 ? (i < 2 ? r.sv.x : r.sv.y) : (i < 2 ? r.sv.z : r.sv.w)) >> (16 * (i & 1));
+            b[i] = d * (float)max(abs((int)(int8_t)(s & 0xff)), abs((int)(int8_t)((s >> 8) & 0xff)));
+        }
+    }
+    __device__ static __forceinline__ void values(const Head& r, const Raw& raw, int c, int part, float f0, float f1, f2 (&w0)[8], f2 (&w1)[8]) {
         // 64 values: pair p of half n of the super-block (jq_formats.cuh)
         const int n = c >> 1, p = c & 1;
         const uint4 la = raw.la[part], lb = raw.lb[part], hq = raw.hq[part];
         const uint32_t sw = n == 0 ? (p == 0 ? r.sv.x : r.sv.y) : (p == 0 ? r.sv.z : r.sv.w);
-        const float d = r.d * fac;
-        const float a0 = d * (float)(int)(int8_t)byte_of(sw, part), a1 = d * (float)(int)(int8_t)byte_of(sw, part + 2);
+        const float a0 = r.d * f0 * (float)(int)(int8_t)byte_of(sw, part), a1 = r.d * f1 * (float)(int)(int8_t)byte_of(sw, part + 2);
         const f2 A0 = pack2(a0, a0), A1 = pack2(a1, a1), K0 = pack2(-96.0f * a0, -96.0f * a0), K1 = pack2(-96.0f * a1, -96.0f * a1);
         const uint32_t wa[4] = {la.x, la.y, la.z, la.w}, wb[4] = {lb.x, lb.y, lb.z, lb.w}, wh[4] = {hq.x, hq.y, hq.z, hq.w};
 #pragma unroll
@@ -205,11 +217,16 @@ struct Dq<JQ_TYPE_Q8_0> {
         return Raw{{lds16(base + 16 * swizzle_piece(4 * c, row)), lds16(base + 16 * swizzle_piece(4 * c + 1, row)), lds16(base + 16 * swizzle_piece(4 * c + 2, row)),
                     lds16(base + 16 * swizzle_piece(4 * c + 3, row))}};
     }
-    __device__ static __forceinline__ float bound(const Head& r) { return 128.0f * half_bits_to_float(max_half8(r.d)); }
-    __device__ static __forceinline__ void values(const Head& r, const Raw& raw, int c, int part, float fac, f2 (&w0)[8], f2 (&w1)[8]) {
+    __device__ static __forceinline__ void bounds(const Head& r, int h, float (&b)[4]) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            b[i] = 128.0f * fabsf(half_bits_to_float((h == 0 ? (i < 2 ? r.d.x : r.d.y) : (i < 2 ? r.d.z : r.d.w)) >> (16 * (i & 1))));
+        }
+    }
+    __device__ static __forceinline__ void values(const Head& r, const Raw& raw, int c, int part, float f0, float f1, f2 (&w0)[8], f2 (&w1)[8]) {
         const uint4 qa = raw.q[2 * part], qb = raw.q[2 * part + 1];
         const uint32_t dw = c == 0 ? r.d.x : (c == 1 ? r.d.y : (c == 2 ? r.d.z : r.d.w));
-        const float d = half_bits_to_float(dw >> (16 * part)) * fac;
+        const float d = half_bits_to_float(dw >> (16 * part)) * (part == 0 ? f0 : f1);
         const f2 D = pack2(d, d), K = pack2(-32896.0f * d, -32896.0f * d);  // 32768 + 128
         const uint32_t w[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
 #pragma unroll
@@ -250,14 +267,24 @@ struct DqN {
         const uint32_t base = uq + (uint32_t)row * ROW;
         return Raw{{lds16(base + 16 * swizzle_piece(2 * c, row)), lds16(base + 16 * swizzle_piece(2 * c + 1, row))}};
     }
-    __device__ static __forceinline__ float bound(const Head& r) {
-        if constexpr (HAS_MIN) {  // 15 |d| + |m| <= 16 max(|d|, |m|)
-            return 16.0f * half_bits_to_float(max(max_half8(r.d), max_half8(r.d2)));
+    __device__ static __forceinline__ void bounds(const Head& r, int h, float (&b)[4]) {
+        if constexpr (HAS_MIN) {
+            const uint4 four = h == 0 ? r.d : r.d2;
+            const uint32_t dm[4] = {four.x, four.y, four.z, four.w};
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                b[i] = fmaf(15.0f, fabsf(half_bits_to_float(dm[i])), fabsf(half_bits_to_float(dm[i] >> 16)));
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                b[i] = 8.0f * fabsf(half_bits_to_float((h == 0 ? (i < 2 ? r.d.x : r.d.y) : (i < 2 ? r.d.z : r.d.w)) >> (16 * (i & 1))));
+            }
         }
-        return 8.0f * half_bits_to_float(max_half8(r.d));
     }
-    __device__ static __forceinline__ void values(const Head& r, const Raw& raw, int c, int part, float fac, f2 (&w0)[8], f2 (&w1)[8]) {
+    __device__ static __forceinline__ void values(const Head& r, const Raw& raw, int c, int part, float f0, float f1, f2 (&w0)[8], f2 (&w1)[8]) {
         const uint4 q = raw.q[part];
+        const float fac = part == 0 ? f0 : f1;
         float d, k;
         if constexpr (HAS_MIN) {
             const uint4 four = c < 2 ? r.d : r.d2;

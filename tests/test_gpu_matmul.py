@@ -146,3 +146,23 @@ def test_row_shards_are_bitwise_equal_for_partial_steps(t, k):
         y = Gguf.linear(x, whole)
         for lo, hi, shard in shards:
             assert torch.equal(Gguf.linear(x, shard), y[:, lo:hi]), (m, lo, hi)
+
+
+def test_wide_ranges_backward():
+    """Features whose blocks are far smaller than their neighbours' in the same 128 rows: outputs of their own, to their own precision."""
+    n, k, m = 300, 512, 40
+    for t in ["Q8_0", "Q4_0", "Q4_1"]:
+        block, fields = {"Q8_0": (34, [0]), "Q4_0": (18, [0]), "Q4_1": (20, [0, 2])}[t]
+
+        def edit(raw):
+            blocks = raw.reshape(n, k // 32, block)
+            for f in fields:
+                for b in range(k // 32):
+                    blocks[:, b, f:f + 2] = np.full(n, 1.25 * 2.0 ** (3 - 3 * (b % 8)), np.float16).view(np.uint8).reshape(-1, 2)
+
+        w, wd = weight(t, n, k, 7, edit)
+        g = torch.randn(m, n, generator=torch.Generator().manual_seed(3)).cuda() * (2.0 ** torch.linspace(-40, 40, m))[:, None].cuda()
+        y, ref = Gguf.linearBackward(g, w), g.double() @ wd
+        # 2^-22 of each operand and what the tensor cores cut off
+        assert float(((y.double() - ref).abs() / (g.double().abs() @ wd.abs() + 1e-300)).max()) <= 2e-6
+        assert device_status(0) == 0
