@@ -317,7 +317,7 @@ struct Dq<JQ_TYPE_Q4_1> : DqN<JQ_TYPE_Q4_1> {};
 // ---- the forward FP32 product's weights: half arithmetic ------------------------------------------------------------------------------
 // A row's 256 weights of a unit are a factor (applied in FP32 when the unit's sums are folded) times values that halves hold exactly, in one
 // part or two:
-//   Q4_K, Q5_K  d x (scale q - r min), r = dmin / d: scale q <= 1953 is a half. The mins are the same for 32 values, so they are not
+//   Q4_K, Q5_K  d x (scale q - r min), r = dmin / d: scale q <= 1953 is a half (see factor for a dmin far above d). The mins are the same for 32 values, so they are not
 //               subtracted from each value but multiplied with the sum of x over the 32 (EXT: 16 more columns of the contraction per unit,
 //               -r min_j as hi and lo halves, against the sums that split_kernel wrote there).
 //   Q6_K        d x scale (q - 32): 13 bits, hi = the product rounded to a half, lo = fma(scale, q - 32, -hi), which is exact
@@ -370,11 +370,23 @@ struct HalfK45 {
     static constexpr bool Q5 = TYPE == JQ_TYPE_Q5_K;
     static constexpr int TILES = 1;
     static constexpr bool EXT = true;
-    // d, except where a min's weight -r min would not fit a half (dmin above 1000 d: all 32 values of a sub-block are then nearly equal, and
-    // the values are rounded relative to the mins instead).
+    // d; where a min's weight -r min might not fit a half (dmin above 952 d), d 2^p with the smallest p that brings the block's mins below 2^15. The
+    // scales are then divided by 2^p, which is exact: sub-blocks whose min is 0 or 1 keep their values beside others whose min is 63.
     __device__ static __forceinline__ float factor(const typename D::Head& h) {
         const float d = half_bits_to_float(h.h.x), dmin = half_bits_to_float(h.h.x >> 16);
-        return fabsf(dmin) > 1000.0f * fabsf(d) ? dmin * 0.001953125f : d;
+        if (!(63.0f * fabsf(dmin) > 60000.0f * fabsf(d))) {
+            return d;
+        }
+        if (d == 0.0f) {
+            return dmin;  // the mins alone
+        }
+        uint32_t sc, m0, m1;
+        scale_min_words(h.h, 0, sc, m0);
+        scale_min_words(h.h, 2, sc, m1);
+        m0 = __vmaxu4(m0, m1);
+        m0 = max(max(m0 & 0xffu, (m0 >> 8) & 0xffu), max((m0 >> 16) & 0xffu, m0 >> 24));
+        const int p = (int)(__float_as_uint(fabsf(dmin) / fabsf(d) * (float)m0) >> 23) - (127 + 14);
+        return p <= 0 ? d : d * __uint_as_float((uint32_t)(127 + p) << 23);
     }
     struct Scales {
         uint32_t s0, c0, s1, c1;  // as pairs of halves: scale and -1024 scale (sub-block 2c); scale / 16 and -64 scale (2c + 1), Q5_K as the first
@@ -386,8 +398,9 @@ struct HalfK45 {
         uint32_t a = hadd2(__byte_perm(sc, 0x64646464u, (c & 1) ? 0x4242u : 0x4040u), 0xe400e400u);
         uint32_t b = hadd2(__byte_perm(sc, 0x64646464u, (c & 1) ? 0x4343u : 0x4141u), 0xe400e400u);
         const float d = half_bits_to_float(h.h.x), f = factor(h);
-        if (f != d) {  // rare (see factor)
-            const uint32_t ratio = h2_dup(d / f);
+        if (f != d) {  // rare (see factor). Beyond 2^20 the scales' part of a weight is below 2^-25 of the block's largest, and halves would round it
+            const float inverse = d / f;
+            const uint32_t ratio = h2_dup(fabsf(inverse) < 9.5367431640625e-7f ? 0.0f : inverse);
             a = hmul2(a, ratio);
             b = hmul2(b, ratio);
         }

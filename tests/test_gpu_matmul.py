@@ -166,3 +166,46 @@ def test_wide_ranges_backward():
         # 2^-22 of each operand and what the tensor cores cut off
         assert float(((y.double() - ref).abs() / (g.double().abs() @ wd.abs() + 1e-300)).max()) <= 2e-6
         assert device_status(0) == 0
+
+
+def k_scales(sc, mn):
+    """The 12 bytes of a Q4_K or Q5_K block that hold eight 6-bit scales and mins (GgufKernels.java:74-83)."""
+    b = [sc[j] | (sc[j + 4] >> 4) << 6 for j in range(4)] + [mn[j] | (mn[j + 4] >> 4) << 6 for j in range(4)]
+    return np.array(b + [(sc[j + 4] & 15) | (mn[j + 4] & 15) << 4 for j in range(4)], np.uint8)
+
+
+# mins far above the scales beside sub-blocks whose min is 0 or 1: every weight keeps its own 22 bits. All quants of a sub-block are equal and x is
+# positive, so an error of a weight does not average out. ratio = dmin / d, 0: d is zero
+@pytest.mark.parametrize("ratio", [30.0, 900.0, 1001.0, 1100.0, 20000.0, 1.0e6, 0.0])
+@pytest.mark.parametrize("t", ["Q4_K", "Q5_K"])
+def test_mins_far_above_the_scales(t, ratio):
+    n, k, m = 64, 512, 20
+    block, quants = {"Q4_K": (144, 16), "Q5_K": (176, 16)}[t]
+    d = 0.0 if ratio == 0.0 else (2.0 ** -14 if ratio > 30000 else 2.0 ** -9)
+    dmin = float(np.float16(d * ratio if ratio else 0.37))
+    parts = np.empty((n * k // 256, 8))  # of a sub-block's weights: d scale q + dmin min
+
+    def edit(raw):
+        rng = np.random.default_rng(int(ratio))
+        for i, b in enumerate(raw.reshape(-1, block)):
+            scales, mins = rng.integers(1, 64, 8), rng.integers(0, 2, 8) * (i % 3 != 0)
+            if i % 3 == 2:
+                mins[i % 8] = 63
+            b[0:4] = np.array([d, dmin], np.float16).view(np.uint8)
+            b[4:16] = k_scales([int(v) for v in scales], [int(v) for v in mins])
+            b[quants:] = 0xff if i % 2 == 0 else 0x77  # Q5_K: the fifth bits too
+            q = np.full(8, 15 if i % 2 == 0 else 7) + (0 if t == "Q4_K" else 16 * np.array([(b[quants] >> j) & 1 for j in range(8)]))
+            parts[i] = d * scales * q + dmin * mins
+
+    w, wd = weight(t, n, k, 3, edit)
+    size = torch.from_numpy(np.repeat(parts, 32, axis=1).reshape(n, k)).cuda()
+    assert bool((wd.abs() <= size * 1.0000001).all())
+    x = torch.rand(m, k, generator=torch.Generator().manual_seed(9)).cuda() + 0.5
+    # one sub-block at a time, so that the large ones do not hide the small ones
+    for sub in range(16):
+        part = torch.zeros_like(x)
+        part[:, 32 * sub:32 * sub + 32] = x[:, 32 * sub:32 * sub + 32]
+        y, ref = Gguf.linear(part, w).double(), part.double() @ wd.T
+        # 2^-22 of the two parts of each weight, 2^-22 of x, and what the tensor cores cut off: some 2^-23 a step
+        assert float(((y - ref).abs() / (part.double() @ size.T + 1e-30)).max()) <= 2e-6, (sub, ratio)
+    assert device_status(0) == 0
