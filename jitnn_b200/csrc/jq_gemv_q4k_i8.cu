@@ -909,14 +909,22 @@ int launch_gemv_q4k_i8_imaged(const View& v, const View* v2, const uint8_t* imag
     return run<1, false>(v, w2, peer != nullptr ? *peer : local, nullptr, 1, bias, y, s, const_cast<uint8_t*>(image), handled, false);
 }
 
-// One row of x that is the RMSNorm of a vector and a delta (NormInput), up to three Q4_K weights of one k <= 8192.
+// One row of x that is the RMSNorm of a vector and a delta (NormInput), up to three Q4_K weights of one k <= 8192; above 7168 only up to 20000 rows
+// in all. Up to there the norm kernel costs more than it does in here (steps of 10 layers, norm kernel and this: k = 5120, hidden 13824 637
+// and 600 us, 7168 / 20480 845 and 825), at 8192 with 57344 rows less (1079 and 1092; with wq|wk|wv alone in this form 1080, with Q6_K wv
+// and w2 1301 against 1315 and 1318).
 int launch_gemv_q4k_i8_normed(const View* vs, int count, const NormInput& norm, float* const* ys, cudaStream_t s, bool* handled) {
     *handled = false;
     const View& v = vs[0];
+    int64_t rows = 0;
     for (int i = 0; i < count; i++) {
         if (vs[i].type != JQ_TYPE_Q4_K || vs[i].k != v.k || vs[i].n == 0 || vs[i].k == 0 || vs[i].k > 8192) {
             return JQ_OK;
         }
+        rows += vs[i].n;
+    }
+    if (v.k > 7168 && rows > 20000) {
+        return JQ_OK;
     }
     const int t1 = (int)((v.n + 15) / 16), t2 = count > 1 ? t1 + (int)((vs[1].n + 15) / 16) : 0;
     const Second w2{count > 1 ? vs[1].q : nullptr, count > 1 ? vs[1].n : 0, count > 1 ? ys[1] : nullptr, count > 1 ? t1 : 0x7fffffff,

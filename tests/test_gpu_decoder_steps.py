@@ -1,9 +1,10 @@
 """The captured decode steps where one range of cached positions ends and the next begins, and the page-locked logits arrays."""
 import numpy as np
 import pytest
+import torch
 
 import jitnn_b200
-from jitnn_b200 import LlamaDecoder
+from jitnn_b200 import LlamaDecoder, synth
 from oracle import llama_oracle
 
 pytestmark = pytest.mark.gpu
@@ -76,4 +77,35 @@ def test_the_next_range_is_captured_before_it_is_reached(n_seqs):
     per_step = np.diff(counts)
     assert per_step[256 - 236] == 0 and per_step[512 - 236] == 0
     assert (per_step > 0).sum() == 2 + 2  # the first step is issued kernel by kernel; one capture each for up to 256, 512 and 520 positions
+    dec.close()
+
+
+# where the norm in front of gate and up stops being made inside their launch: by width, and at 8192 by the rows of both
+@pytest.mark.parametrize("dim,hidden", [(7168, 12544), (7424, 9984), (8192, 9984), (8192, 10240)])
+def test_norms_inside_and_in_front(dim, hidden):
+    """The fused single-token step against the general kernels."""
+    heads, vocab = dim // 128, 512
+    g = torch.Generator(device="cuda").manual_seed(hidden)
+
+    def lin(n, k):
+        return ("Q4_K", synth.quantize_q4_k(torch.randn(n, k, generator=g, device="cuda") * 0.02).cpu().numpy().reshape(-1), n, k)
+
+    w = {"tok_embeddings": torch.randn(vocab, dim, generator=g, device="cuda").cpu().numpy(), "norm": np.ones(dim, np.float32), "output": lin(vocab, dim)}
+    for layer in range(2):
+        p = "layers.%d." % layer
+        w[p + "attention_norm"] = (1.0 + 0.1 * torch.randn(dim, generator=g, device="cuda")).cpu().numpy()
+        w[p + "ffn_norm"] = (1.0 + 0.1 * torch.randn(dim, generator=g, device="cuda")).cpu().numpy()
+        w.update({p + "wq": lin(dim, dim), p + "wk": lin(128, dim), p + "wv": lin(128, dim), p + "wo": lin(dim, dim), p + "w1": lin(hidden, dim),
+                  p + "w3": lin(hidden, dim), p + "w2": lin(dim, hidden)})
+    dec = LlamaDecoder(2, dim, heads, 1, hidden, vocab, 8)
+    dec.load(w)
+    out = []
+    for fused in (0, 1):
+        jitnn_b200.load().jq_set_option(b"decoder_fused", fused)
+        try:
+            out.append([np.array(dec.forward([7 * pos + 1], pos)[0]) for pos in range(3)])
+        finally:
+            jitnn_b200.load().jq_set_option(b"decoder_fused", 1)
+    for a, b in zip(*out):
+        assert np.abs(a - b).max() <= 1e-5 * np.abs(a).max()  # FP32 throughout, sums in other orders
     dec.close()
