@@ -131,9 +131,15 @@ static bool configure(int type, bool fp32, bool bwd, int nt, int ksplit, Args& a
     // sums of a CTA's virtual ranges (instances for 16 rows of x), kept apart from the rings, which are still in use
     a.part_bytes = fp32 && !bwd && nt <= 16 && ksplit > 1 ? VIRTUAL / ksplit * nt * 512 : 0;
     const int at = a_bytes(bwd), bt = f.b_tiles * tile_bytes(fp32, nt), rb = unit_bytes(type), room = 227 * 1024 - 1024 - TAIL_BYTES - a.part_bytes;
-    // tensor memory: two accumulators where they fit beside the groups' operands, else one; operands behind them
-    a.cols = (f.columns * nt + 31) / 32 * 32;
-    a.bufs = 2 * a.cols + f.groups * f.a_cols <= 512 ? 2 : 1;
+    // tensor memory: as many accumulators as fit beside the groups' operands; operands behind them
+    a.cols = f.columns * nt;
+    a.bufs = fp32 ? MAX_BUFS : 2;
+    while (a.bufs > 1 && a.bufs * a.cols + f.operands * f.a_cols > 512) {
+        a.bufs--;
+    }
+    if (f.paired && a.bufs < 2) {
+        return false;  // (two parts and the 16 more columns: tiles of up to 112 rows)
+    }
     int max_a = 4;
     if (!bwd) {
         max_a = (512 - a.bufs * a.cols) / f.a_cols;
@@ -172,16 +178,16 @@ static bool configure(int type, bool fp32, bool bwd, int nt, int ksplit, Args& a
 // the barriers between the roles up to a width, the tensor pipe beyond it.
 static double unit_ns(int type, bool fp32, bool bwd, int nt) {
     if (bwd) {
-        return nt < 64 ? 940.0 : 430.0 + 7.9 * nt;
+        return nt < 64 ? 1040.0 : 570.0 + 8.6 * nt;
     }
     if (!fp32) {
         return nt <= 128 ? 950.0 : 350.0 + 4.5 * ((nt + 63) / 64 * 64);  // (a tile of 208 or 240 is no faster than one of 256)
     }
     if (nt <= 32) {
-        return one_part(type) ? (nt <= 16 ? 830.0 : 1060.0) : 1300.0;
+        return one_part(type) ? (nt <= 16 ? 950.0 : 1270.0) : 1430.0;
     }
-    const double t = one_part(type) ? 450.0 + 9.9 * nt : 300.0 + 14.7 * nt;
-    return t < 1320.0 ? 1320.0 : t;
+    const double t = one_part(type) ? 1330.0 + 6.5 * nt : 1450.0 + 8.6 * nt;
+    return one_part(type) || t > 1960.0 ? t : 1960.0;
 }
 
 // Clusters of ks CTAs that run at a time, one CTA per SM (cudaOccupancyMaxActiveClusters; the SMs of a GPC are not all a multiple of 4 or 8).

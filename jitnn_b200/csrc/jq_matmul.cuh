@@ -5,8 +5,8 @@
 //
 // Two operand precisions. BF16: x is bfloat16, weights are rounded to bfloat16, one product. FP32: x is split into two halves (hi + lo, 22
 // significant bits), and so are weights that one half cannot hold (jq_matmul_dequant.cuh); the products hi.hi + hi.lo + lo.hi (or
-// the first two) are taken, so that results keep FP32's accuracy; sums leave the tensor core every 256 (backward: 128) terms and are added
-// up in registers, rounded to nearest.
+// the first two) are taken, so that results keep FP32's accuracy; sums leave the tensor core every 128 (backward: 64) terms and are added
+// up in registers, rounded to nearest (see Shape::ACC).
 //
 // A CTA owns 128 features and a tile of up to 256 (FP32: 128) rows of x and walks the contraction in stages of 64. (Pairs of CTAs under one
 // tcgen05.mma, cta_group::2, read each activation tile from L2 once for 256 features; measured equal within 3 % on every shape and
@@ -48,7 +48,7 @@ template <int TYPE, bool FP32, bool BWD, int NMAX>
 struct Shape {
     static constexpr bool JOINED = FP32 && NMAX <= 32;
     static constexpr int TURN = BWD ? 1 : (!FP32 ? (NMAX <= 128 ? 4 : 1) : (!JOINED ? (one_part(TYPE) ? 2 : 1) : (NMAX <= 16 && one_part(TYPE) ? 4 : 2)));
-    static constexpr int GROUPS = FP32 && !JOINED ? 2 : (BWD || (!FP32 && NMAX > 128) ? 4 : 3), FOLD = FP32 && !JOINED ? 8 : 4, THREADS = (3 + 4 * GROUPS + FOLD) * 32;
+    static constexpr int GROUPS = FP32 && !JOINED ? 2 : (BWD || (!FP32 && NMAX > 128) ? 4 : 3), FOLD = FP32 && !JOINED ? 16 : 4, THREADS = (3 + 4 * GROUPS + FOLD) * 32;
     static constexpr int CHUNKS = BWD ? 2 : 4;                           // chunks of 64 of the contraction in a unit
     static constexpr int TURNS = CHUNKS / TURN;
     static constexpr bool EXT = FP32 && !BWD && (one_part(TYPE) || TYPE == JQ_TYPE_Q4_1);  // 16 more columns of the contraction per unit
@@ -56,10 +56,21 @@ struct Shape {
     static constexpr int A_COLS = BWD ? 0 : 32 * PARTS * TURN + (EXT ? 8 : 0);              // tensor-memory columns of an operand
     static constexpr int B_TILES = JOINED && !BWD ? TURN + (EXT ? 1 : 0) : 1;               // activation tiles of 64 that arrive together
     static constexpr bool OWNED = TURNS == 1;                           // a raw unit is one group's own
+    // FP32: ACC chunks' products go into one accumulator before the fold adds it up. The tensor core cuts every sum off towards zero, so the error
+    // grows with the MMAs that add to an accumulator of full size. Products with a lo part are small: they go first (PAIRED: two chunks' operands
+    // and activation tiles are waited for and used together) or into columns of their own (JOINED); then 4 (backward), 8 or 16 are left.
+    // Relative to the result's norm at k = 4096: 1.5e-7 (backward) and 1.8 to 2.3e-7 with 4 and 8; 3.0e-7, which is what the decode kernels
+    // have, with 16 (Q4_K up to 16 rows, whose second hand-over a unit would take 11 % longer). All products of 256 terms as they come left
+    // 4e-7 to 2.4e-6.
+    static constexpr int ACC = BWD ? 1 : (TYPE == JQ_TYPE_Q4_K && JOINED && TURN == 4 ? 4 : 2), ACCS = CHUNKS / ACC;
+    static constexpr bool PAIRED = FP32 && !BWD && !JOINED;
+    static constexpr int OPERANDS = PAIRED ? 2 / TURN + 2 : GROUPS;     // to have at least
+    static_assert(!FP32 || PAIRED || TURN % ACC == 0, "");
 };
 constexpr int A_TILE = 128 * 128;  // 128 rows of 128 bytes
 constexpr int MAX_A = 6, MAX_B = 12, MAX_RAW = 6;
-constexpr int FACTORS = 8;   // units whose factors the fold may still need: operands in flight and accumulators, see where they are written
+constexpr int MAX_BUFS = 4;
+constexpr int FACTORS = 8;   // units whose factors the fold may still need, see where they are written
 constexpr int VIRTUAL = 8;   // ranges of the contraction whose sums are added up in order, whatever the cluster (instances for 16 rows of x)
 
 constexpr int MAX_WEIGHTS = 3;
@@ -82,7 +93,7 @@ struct Args {
     int part_bytes;   // shared memory for the sums of this CTA's virtual ranges
     int sa, sb, raw;  // ring depths: weight operands, activation tiles, raw units
     int cols;         // tensor-memory columns of one accumulator
-    int bufs;         // accumulators: 2, or 1 where a second one does not fit
+    int bufs;         // accumulators: as many as fit, up to MAX_BUFS
     int tmem;         // columns to allocate
     const float* xscale;  // FP32: scale of (contraction block, row of x): [block][xstride]
     int xstride;
@@ -181,6 +192,14 @@ __device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, volatil
     return __all_sync(0xffffffffu, wait<AFTER>(bar, parity, abort_flag, p, code));
 }
 
+// Different barriers for lanes 0 .. n - 1 of a warp: one round trip for all of them (a poll takes over a hundred clocks even when the phase is
+// complete, and more when all lanes poll the same barrier).
+__device__ __forceinline__ bool wait_lanes(int n, int lane, uint32_t bar, uint32_t parity, volatile int* abort_flag, const Args& p, int code) {
+    const bool ok = __all_sync(0xffffffffu, lane < n ? wait(bar, parity, abort_flag, p, code) : true);
+    __syncwarp();
+    return ok;
+}
+
 __device__ __forceinline__ void tma_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst), "l"(map), "r"(bar), "r"(c0),
                  "r"(c1), "r"(c2)
@@ -195,6 +214,18 @@ __device__ __forceinline__ void ld_tmem8(float (&r)[8], uint32_t addr) {
                  : "memory");
 #pragma unroll
     for (int i = 0; i < 8; i++) {
+        r[i] = __uint_as_float(u[i]);
+    }
+}
+__device__ __forceinline__ void ld_tmem16(float (&r)[16], uint32_t addr) {
+    uint32_t u[16];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]), "=r"(u[9]), "=r"(u[10]), "=r"(u[11]),
+                   "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
+                 : "r"(addr)
+                 : "memory");
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
         r[i] = __uint_as_float(u[i]);
     }
 }
@@ -285,7 +316,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
     const uint32_t fac0 = raw0 + (uint32_t)R * raw_bytes<TYPE>();
     const uint32_t scl0 = fac0 + FACTORS * 128 * 4, full_a = scl0 + 8 * 2 * 64 * 4, free_a = full_a + 8 * MAX_A, full_b = free_a + 8 * MAX_A, free_b = full_b + 8 * MAX_B;
     const uint32_t raw_full = free_b + 8 * MAX_B, raw_read = raw_full + 8 * MAX_RAW;
-    const uint32_t acc_full = raw_read + 8 * MAX_RAW, acc_empty = acc_full + 16, fac_full = acc_empty + 16, max_full = fac_full + 8 * FACTORS, slot_s = max_full + 64;
+    const uint32_t acc_full = raw_read + 8 * MAX_RAW, acc_empty = acc_full + 8 * MAX_BUFS, fac_full = acc_empty + 8 * MAX_BUFS, max_full = fac_full + 8 * FACTORS, slot_s = max_full + 64;
     uint8_t* const generic = smem_unaligned + (slot_s - tc::smem_u32(smem_unaligned));
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(generic);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(generic + 4);
@@ -309,7 +340,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
             tc::mbar_init(raw_full + 8 * r, 1);
             tc::mbar_init(raw_read + 8 * r, OWNED ? 4 : 4 * G);
         }
-        for (int i = 0; i < 2; i++) {
+        for (int i = 0; i < MAX_BUFS; i++) {
             tc::mbar_init(acc_full + 8 * i, 1);
             tc::mbar_init(acc_empty + 8 * i, W::FOLD);
         }
@@ -376,11 +407,106 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
         int s = 0, sb = 0, buf = 0;
         uint32_t ph = 0, phb = 0, aph = 0;
         bool ok = true, ready = false, ready_b = false;
-        for (int tile = cluster_id; tile < tiles && ok; tile += clusters) {
+        if constexpr (W::PAIRED) {
+            constexpr int OPS = 2 / TURN;        // operands of two chunks
+            constexpr bool TWO = W::PARTS == 2;  // the weights have a lo part
+            for (int tile = cluster_id; tile < tiles && ok; tile += clusters) {
+                for (int u = u0; u < u1 && ok; u++) {
+#pragma unroll
+                    for (int pair = 0; pair < 2; pair++) {
+                        // lane 0 (and 1) waits for the operand(s), the next two for an activation tile each, the last one for the accumulator
+                        uint32_t a_at[OPS], a_bar[OPS], b_at[2], b_bar[2], bar = 0, parity = 0;
+#pragma unroll
+                        for (int o = 0; o < OPS; o++) {
+                            a_at[o] = tmem_a + (uint32_t)(s * A_COLS);
+                            a_bar[o] = free_a + 8 * s;
+                            bar = lane == o ? full_a + 8 * s : bar;
+                            parity = lane == o ? ph : parity;
+                            if (++s == SA) {
+                                s = 0;
+                                ph ^= 1;
+                            }
+                        }
+#pragma unroll
+                        for (int b = 0; b < 2; b++) {
+                            b_at[b] = desc_k(b0 + (uint32_t)sb * b_st);
+                            b_bar[b] = free_b + 8 * sb;
+                            bar = lane == OPS + b ? full_b + 8 * sb : bar;
+                            parity = lane == OPS + b ? phb : parity;
+                            if (++sb == SB) {
+                                sb = 0;
+                                phb ^= 1;
+                            }
+                        }
+                        bar = lane == OPS + 2 ? acc_empty + 8 * buf : bar;
+                        parity = lane == OPS + 2 ? aph ^ 1u : parity;
+                        if (!(ok = wait_lanes(OPS + 3, lane, bar, parity, abort_flag, p, lane < OPS ? 2 : (lane < OPS + 2 ? 3 : 5)))) {
+                            break;
+                        }
+                        tc::fence_after_sync();
+                        const uint32_t d = tmem + (uint32_t)(buf * p.cols), d_bar = acc_full + 8 * buf;
+                        if (++buf == p.bufs) {
+                            buf = 0;
+                            aph ^= 1;
+                        }
+                        if (elect_one()) {
+                            // first all products with a lo part
+#pragma unroll
+                            for (int c = 0; c < 2; c++) {
+                                const uint32_t ta = a_at[c / TURN] + (uint32_t)(c % TURN * 32 * W::PARTS);  // 16 of the contraction are 8 columns
+#pragma unroll
+                                for (uint32_t ks = 0; ks < 4; ks++) {
+                                    mma_ta(d, ta + 8 * ks, b_at[c] + lo_rows + 2 * ks, id_n, (uint32_t)c | ks);
+                                    if constexpr (TWO) {
+                                        mma_ta(d, ta + 32 + 8 * ks, b_at[c] + 2 * ks, id_n, 1u);
+                                    }
+                                }
+                            }
+#pragma unroll
+                            for (int c = 0; c < 2; c++) {
+                                const uint32_t ta = a_at[c / TURN] + (uint32_t)(c % TURN * 32 * W::PARTS);
+#pragma unroll
+                                for (uint32_t ks = 0; ks < 4; ks++) {
+                                    mma_ta(d, ta + 8 * ks, b_at[c] + 2 * ks, id_n, 1u);
+                                }
+                                tc::umma_commit(b_bar[c]);
+                            }
+                        }
+                        __syncwarp();
+                        if (EXT && pair == 1) {  // the 16 more columns; their tile is not waited for with the others, which it would keep from being refilled
+                            const uint32_t bd = desc_k(b0 + (uint32_t)sb * b_st), be = free_b + 8 * sb;
+                            if (!(ok = wait_lanes(1, lane, full_b + 8 * sb, phb, abort_flag, p, 3))) {
+                                break;
+                            }
+                            tc::fence_after_sync();
+                            if (++sb == SB) {
+                                sb = 0;
+                                phb ^= 1;
+                            }
+                            if (elect_one()) {
+                                const uint32_t te = a_at[OPS - 1] + TURN * 32 * W::PARTS;
+                                mma_ta(d, te, bd + lo_rows, id_n, 1u);
+                                mma_ta(d, te, bd, id_n, 1u);
+                                tc::umma_commit(be);
+                            }
+                            __syncwarp();
+                        }
+                        if (elect_one()) {
+#pragma unroll
+                            for (int o = 0; o < OPS; o++) {
+                                tc::umma_commit(a_bar[o]);
+                            }
+                            tc::umma_commit(d_bar);
+                        }
+                        __syncwarp();
+                    }
+                }
+            }
+        }
+        for (int tile = cluster_id; !W::PAIRED && tile < tiles && ok; tile += clusters) {
             bool first = true;
             for (int u = u0; u < u1 && ok; u++) {
-                const uint32_t d = tmem + (uint32_t)(buf * p.cols);
-                if (FP32 || u == u0) {
+                if (!FP32 && u == u0) {
                     if (!(ok = wait_warp(acc_empty + 8 * buf, aph ^ 1u, abort_flag, p, 5))) {
                         break;
                     }
@@ -388,6 +514,9 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                 }
 #pragma unroll
                 for (int turn = 0; turn < TURNS; turn++) {
+                    if (FP32 && !(ok = wait_warp(acc_empty + 8 * buf, aph ^ 1u, abort_flag, p, 5))) {
+                        break;
+                    }
                     if (!(ok = __all_sync(0xffffffffu, ready) || wait_warp(full_a + 8 * s, ph, abort_flag, p, 2))) {
                         break;
                     }
@@ -409,10 +538,20 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                             ready_b = tc::mbar_test(full_b + 8 * (sb + 1 == SB ? 0 : sb + 1), sb + 1 == SB ? phb ^ 1 : phb);
                             tc::fence_after_sync();
                         }
+                        if (FP32 && !ext && c % W::ACC == 0) {  // the next accumulator (the turn's first one is waited for above)
+                            if (c > 0 && !(ok = wait_warp(acc_empty + 8 * buf, aph ^ 1u, abort_flag, p, 5))) {
+                                break;
+                            }
+                            first = true;
+                            tc::fence_after_sync();
+                        }
+                        const uint32_t d = tmem + (uint32_t)(buf * p.cols), d_lo = d + (uint32_t)nt;  // JOINED: sums with a lo part in columns of their own
                         // x: hi, lo; 16 of the contraction are 32 bytes
                         const uint32_t bd = desc_k(b0 + (uint32_t)sb * b_st + (BT == 1 ? 0u : (uint32_t)c * tile_st)), bl = bd + lo_rows;
                         const bool b_done = BT == 1 || c == LAST - 1 || (turn < TURNS - 1 && c == TURN - 1);
                         const bool a_done = turn < TURNS - 1 ? c == TURN - 1 : c == LAST - 1;
+                        const bool d_done = FP32 ? (ext || ((c + 1) % W::ACC == 0 && !(EXT && turn == TURNS - 1 && c == TURN - 1)))
+                                                 : a_done && turn == TURNS - 1 && u == u1 - 1;
                         if (elect_one()) {
                             const uint32_t acc = first ? 0u : 1u;
                             if constexpr (BWD) {
@@ -422,11 +561,16 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                                 for (uint32_t ks = 0; ks < 4; ks++) {
                                     if constexpr (JOINED) {
                                         mma(d, ad + 128 * ks, bd + 2 * ks, id_2n, acc | ks);  // hi x (hi | lo)
-                                        mma(d, al + 128 * ks, bd + 2 * ks, id_n, 1u);         // lo x hi
+                                        mma(d_lo, al + 128 * ks, bd + 2 * ks, id_n, 1u);      // lo x hi
                                     } else {
-                                        mma(d, ad + 128 * ks, bd + 2 * ks, id_n, acc | ks);
+                                        mma(d, al + 128 * ks, bd + 2 * ks, id_n, acc | ks);
                                         mma(d, ad + 128 * ks, bl + 2 * ks, id_n, 1u);
-                                        mma(d, al + 128 * ks, bd + 2 * ks, id_n, 1u);
+                                    }
+                                }
+                                if constexpr (!JOINED) {
+#pragma unroll
+                                    for (uint32_t ks = 0; ks < 4; ks++) {
+                                        mma(d, ad + 128 * ks, bd + 2 * ks, id_n, 1u);
                                     }
                                 }
                             } else {
@@ -436,16 +580,11 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                                 for (uint32_t ks = 0; ks < (ext ? 1 : 4); ks++) {
                                     if constexpr (JOINED) {
                                         mma_ta(d, ta + 8 * ks, bd + 2 * ks, id_2n, acc | ks);  // hi x (hi | lo)
+                                        if (TWO && !ext) {
+                                            mma_ta(d_lo, ta + 32 + 8 * ks, bd + 2 * ks, id_n, 1u);
+                                        }
                                     } else {
                                         mma_ta(d, ta + 8 * ks, bd + 2 * ks, id_n, acc | ks);
-                                        if constexpr (FP32) {
-                                            mma_ta(d, ta + 8 * ks, bl + 2 * ks, id_n, 1u);
-                                        }
-                                    }
-                                    if constexpr (TWO) {
-                                        if (!ext) {
-                                            mma_ta(d, ta + 32 + 8 * ks, bd + 2 * ks, id_n, 1u);
-                                        }
                                     }
                                 }
                             }
@@ -454,13 +593,17 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                             }
                             if (a_done) {
                                 tc::umma_commit(free_a + 8 * s);
-                                if (turn == TURNS - 1 && (FP32 || u == u1 - 1)) {
-                                    tc::umma_commit(acc_full + 8 * buf);
-                                }
+                            }
+                            if (d_done) {
+                                tc::umma_commit(acc_full + 8 * buf);
                             }
                         }
                         __syncwarp();
                         first = false;
+                        if (d_done && ++buf == p.bufs) {
+                            buf = 0;
+                            aph ^= 1;
+                        }
                         if (b_done && ++sb == SB) {
                             sb = 0;
                             phb ^= 1;
@@ -471,12 +614,6 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                     }
                     s = sn;
                     ph = phn;
-                }
-                if (FP32 || u == u1 - 1) {
-                    if (++buf == p.bufs) {
-                        buf = 0;
-                        aph ^= 1;
-                    }
                 }
             }
         }
@@ -621,8 +758,9 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                         }
                         if (FP32 && turn == 0) {
                             // The unit's factors for the fold, into a ring of FACTORS units. This operand's slot is free, so what it held SA
-                            // operands ago went through the tensor core, into an accumulator that the fold had emptied: the fold is done
-                            // with the unit at least that far and `bufs` accumulators back, SA + bufs <= FACTORS.
+                            // operands ago went through the tensor core, into an accumulator that the fold had emptied: the fold has
+                            // finished the accumulator `bufs` before that one, and with it the unit eight before this one as
+                            // SA TURN / ACC + bufs <= 7 ACCS + 1 (at most 6 + 4 and 15; Q4_K up to 16 rows 3 + 4 and 8).
                             const uint32_t fa = fac0 + (uint32_t)(at_unit & (FACTORS - 1)) * 512u;
                             if constexpr (!BWD) {
                                 asm volatile("st.shared.u32 [%0], %1;" ::"r"(fa + 4u * (uint32_t)row0), "r"(unit_factor) : "memory");
@@ -706,7 +844,8 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
         const int group = warp & 3, part = (warp - 3 - 4 * G) >> 2;  // a warp may only read lanes 32 (warp % 4) .. of tensor memory
         const int lane_row = group * 32 + lane;
         const uint32_t lanes = (uint32_t)(group * 32) << 16;
-        const int cols = nt / PARTS, c0 = part * cols;  // this warp's columns of the tile: a multiple of 8
+        // this warp's columns of the tile, a multiple of 16: up to NMAX / PARTS in registers (BF16: all)
+        const int c0 = part * (FP32 ? NMAX / PARTS : nt / PARTS), cols = FP32 ? max(0, min(NMAX / PARTS, nt - c0)) : nt / PARTS;
         int chunk = 0, buf = 0;
         uint32_t aph = 0;
         bool ok = true;
@@ -759,7 +898,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                 }
             };
             if constexpr (FP32) {
-                constexpr int C = NMAX / PARTS;  // columns per thread
+                constexpr int C = NMAX / PARTS, C32 = C < 32 ? 32 : C;  // columns per thread
                 f2 sum[C / 2], total[CANON ? C / 2 : 1];
 #pragma unroll
                 for (int i = 0; i < C / 2; i++) {
@@ -778,7 +917,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                     slot = virt - range * (VIRTUAL / p.ksplit);
                 }
                 // the scales of a unit's columns: fetched by the lanes a unit ahead, read back as broadcasts
-                const uint32_t scl = scl0 + (uint32_t)(warp - 3 - 4 * G) * 512u;
+                const uint32_t scl = scl0 + (uint32_t)(warp - 3 - 4 * G) * (8u * C32);
                 const float* xs = p.xscale + (int64_t)u0 * p.xstride + t0 + c0;
                 float next[(C + 31) / 32];
 #pragma unroll
@@ -786,7 +925,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                     next[i] = lane + 32 * i < cols ? __ldg(xs + lane + 32 * i) : 0.0f;
                 }
                 for (int u = u0; u < u1; u++, chunk++) {
-                    const uint32_t sb = scl + (uint32_t)(chunk & 1) * 256u;
+                    const uint32_t sb = scl + (uint32_t)(chunk & 1) * (4u * C32);
                     __syncwarp();
 #pragma unroll
                     for (int i = 0; i < (C + 31) / 32; i++) {
@@ -800,38 +939,48 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                         }
                     }
                     __syncwarp();
-                    ok = wait_warp<true>(fac_full + 8 * (chunk & (FACTORS - 1)), (uint32_t)(chunk / FACTORS) & 1u, abort_flag, p, 6) &&
-                         wait_warp<true>(acc_full + 8 * buf, aph, abort_flag, p, 4);
-                    if (!ok) {
+                    if (!(ok = wait_warp<true>(fac_full + 8 * (chunk & (FACTORS - 1)), (uint32_t)(chunk / FACTORS) & 1u, abort_flag, p, 6))) {
                         break;
                     }
-                    tc::fence_after_sync();
                     float f;
                     asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"(fac0 + (uint32_t)(chunk & (FACTORS - 1)) * 512u + 4u * (uint32_t)(BWD ? group : lane_row)));
                     const f2 ff = pack2(f, f);
-                    const uint32_t d = tmem + lanes + (uint32_t)(buf * p.cols + c0);
+#pragma unroll 1
+                    for (int a = 0; a < W::ACCS; a++) {
+                        if (!(ok = wait_warp<true>(acc_full + 8 * buf, aph, abort_flag, p, 4))) {
+                            break;
+                        }
+                        tc::fence_after_sync();
+                        const uint32_t d = tmem + lanes + (uint32_t)(buf * p.cols + c0);
 #pragma unroll
-                    for (int c = 0; c < C / 8; c++) {
-                        if (c * 8 < cols) {
-                            float hi[8], lo[8];
-                            ld_tmem8(hi, d + c * 8);
-                            if constexpr (JOINED) {
-                                ld_tmem8(lo, d + nt + c * 8);
-                            }
-                            const uint4 s0 = lds16(sb + c * 32), s1 = lds16(sb + c * 32 + 16);
-                            const uint32_t sc[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-                            ld_tmem_done();
-#pragma unroll
-                            for (int i = 0; i < 4; i++) {
-                                f2 v = mul2(pack2(hi[2 * i], hi[2 * i + 1]), ff);
+                        for (int c = 0; c < C / 16; c++) {
+                            if (c * 16 < cols) {
+                                float hi[16], lo[16];
+                                ld_tmem16(hi, d + c * 16);
                                 if constexpr (JOINED) {
-                                    v = fma2(pack2(lo[2 * i], lo[2 * i + 1]), ff, v);
+                                    ld_tmem16(lo, d + nt + c * 16);
                                 }
-                                sum[c * 4 + i] = fma2(v, pack2(__uint_as_float(sc[2 * i]), __uint_as_float(sc[2 * i + 1])), sum[c * 4 + i]);
+                                ld_tmem_done();
+#pragma unroll
+                                for (int j = 0; j < 4; j++) {
+                                    const uint4 x4 = lds16(sb + c * 64 + j * 16);
+                                    const f2 sc[2] = {pack2(__uint_as_float(x4.x), __uint_as_float(x4.y)), pack2(__uint_as_float(x4.z), __uint_as_float(x4.w))};
+#pragma unroll
+                                    for (int i = 2 * j; i < 2 * j + 2; i++) {
+                                        f2 v = mul2(pack2(hi[2 * i], hi[2 * i + 1]), ff);
+                                        if constexpr (JOINED) {
+                                            v = fma2(pack2(lo[2 * i], lo[2 * i + 1]), ff, v);
+                                        }
+                                        sum[c * 8 + i] = fma2(v, sc[i & 1], sum[c * 8 + i]);
+                                    }
+                                }
                             }
                         }
+                        release();
                     }
-                    release();
+                    if (!ok) {
+                        break;
+                    }
                     if constexpr (CANON) {
                         if (u + 1 == virt_end(virt)) {
                             if (p.ksplit > 1) {

@@ -317,11 +317,12 @@ struct Dq<JQ_TYPE_Q4_1> : DqN<JQ_TYPE_Q4_1> {};
 // ---- the forward FP32 product's weights: half arithmetic ------------------------------------------------------------------------------
 // A row's 256 weights of a unit are a factor (applied in FP32 when the unit's sums are folded) times values that halves hold exactly, in one
 // part or two:
-//   Q4_K, Q5_K  d x (scale q - r min), r = dmin / d: scale q <= 1953 is a half (see factor for a dmin far above d). The mins are the same for 32 values, so they are not
-//               subtracted from each value but multiplied with the sum of x over the 32 (EXT: 16 more columns of the contraction per unit,
-//               -r min_j as hi and lo halves, against the sums that split_kernel wrote there).
+//   Q4_K, Q5_K  d x (scale (q - mid) + scale mid - r min), r = dmin / d, mid = 8 or 16: scale (q - mid) <= 1008 is a half (see factor for a dmin far
+//               above d). The rest is the same for 32 values, so it is not added to each value but multiplied with the sum of x over the 32 (EXT:
+//               16 more columns of the contraction per unit, scale_j mid - r min_j as hi and lo halves, against the sums that split_kernel
+//               wrote there). With q - mid in the place of q the accumulators hold smaller sums, of which less is cut off.
 //   Q6_K        d x scale (q - 32): 13 bits, hi = the product rounded to a half, lo = fma(scale, q - 32, -hi), which is exact
-//   Q8_0, Q4_0  2^e x d' q with d' = 2^-e d exact: hi and lo in the same way; Q4_1 likewise, its m' through the 16 more columns
+//   Q8_0, Q4_0  2^e x d' q with d' = 2^-e d exact: hi and lo in the same way; Q4_1 likewise with q - 8, its m' + 8 d' through the 16 more columns
 // The quants become halves with one byte permute per pair (1024 + q under the exponent 0x64). About 1.3 (K-quants) to 2.3 instructions per
 // weight; going through FP32 and splitting the result takes 5 and was issue bound at twice the time.
 
@@ -388,8 +389,14 @@ struct HalfK45 {
         const int p = (int)(__float_as_uint(fabsf(dmin) / fabsf(d) * (float)m0) >> 23) - (127 + 14);
         return p <= 0 ? d : d * __uint_as_float((uint32_t)(127 + p) << 23);
     }
+    static constexpr float MID = Q5 ? 16.0f : 8.0f;
+    // 1 / 2^p, see factor. Beyond 2^20 the scales' part of a weight is below 2^-25 of the block's largest, and halves would round it
+    __device__ static __forceinline__ float scale_by(float d, float f) {
+        const float by = f == d ? 1.0f : d / f;
+        return fabsf(by) < 9.5367431640625e-7f ? 0.0f : by;
+    }
     struct Scales {
-        uint32_t s0, c0, s1, c1;  // as pairs of halves: scale and -1024 scale (sub-block 2c); scale / 16 and -64 scale (2c + 1), Q5_K as the first
+        uint32_t s0, c0, s1, c1;  // as pairs of halves, for sub-blocks 2c and 2c + 1: what 1024 + 16 q (Q5_K: 8 q) is multiplied by, and what is added
     };
     __device__ static __forceinline__ Scales scales(const typename D::Head& h, int c) {
         uint32_t sc, mn;
@@ -398,18 +405,14 @@ struct HalfK45 {
         uint32_t a = hadd2(__byte_perm(sc, 0x64646464u, (c & 1) ? 0x4242u : 0x4040u), 0xe400e400u);
         uint32_t b = hadd2(__byte_perm(sc, 0x64646464u, (c & 1) ? 0x4343u : 0x4141u), 0xe400e400u);
         const float d = half_bits_to_float(h.h.x), f = factor(h);
-        if (f != d) {  // rare (see factor). Beyond 2^20 the scales' part of a weight is below 2^-25 of the block's largest, and halves would round it
-            const float inverse = d / f;
-            const uint32_t ratio = h2_dup(fabsf(inverse) < 9.5367431640625e-7f ? 0.0f : inverse);
+        if (f != d) {  // rare
+            const uint32_t ratio = h2_dup(scale_by(d, f));
             a = hmul2(a, ratio);
             b = hmul2(b, ratio);
         }
-        Scales r;
-        r.s0 = a;
-        r.c0 = hmul2(a, 0xe400e400u);  // x -1024
-        r.s1 = Q5 ? b : hmul2(b, 0x2c002c00u);  // / 16
-        r.c1 = Q5 ? hmul2(b, 0xe400e400u) : hmul2(b, 0xd400d400u);  // x -64
-        return r;
+        // / 16 and x -(1024 / 16 + 8); / 8 and x -(1024 / 8 + 16): all exact
+        constexpr uint32_t BY = Q5 ? 0x30003000u : 0x2c002c00u, OFF = Q5 ? 0xd880d880u : 0xd480d480u;
+        return Scales{hmul2(a, BY), hmul2(a, OFF), hmul2(b, BY), hmul2(b, OFF)};
     }
     __device__ static __forceinline__ void values(const typename D::Head& h, const typename D::Raw& raw, const Scales& s, int c, int part, int run, uint32_t (&hi)[8],
                                                   uint32_t (&)[8]) {
@@ -422,17 +425,17 @@ struct HalfK45 {
             uint32_t v;
             if constexpr (Q5) {
                 const uint32_t bit = g[x] >> (2 * c + run);
-                v = ((run == 0 ? w[x] : w[x] >> 4) & 0x0f0f0f0fu) | ((bit << 4) & 0x10101010u);
+                v = ((run == 0 ? w[x] << 3 : w[x] >> 1) & 0x78787878u) | ((bit << 7) & 0x80808080u);
             } else {
-                v = run == 0 ? w[x] & 0x0f0f0f0fu : w[x] & 0xf0f0f0f0u;  // high nibbles stay in place: 16 q against scale / 16
+                v = (run == 0 ? w[x] << 4 : w[x]) & 0xf0f0f0f0u;
             }
             hi[2 * x] = hfma2(bytes_to_halves(v, 0), run == 0 ? s.s0 : s.s1, run == 0 ? s.c0 : s.c1);
             hi[2 * x + 1] = hfma2(bytes_to_halves(v, 1), run == 0 ? s.s0 : s.s1, run == 0 ? s.c0 : s.c1);
         }
     }
-    // The 16 more columns: -r min of the eight sub-blocks, hi then lo.
+    // The 16 more columns: scale mid - r min of the eight sub-blocks, hi then lo.
     __device__ static __forceinline__ void ext(const typename D::Head& h, uint32_t (&v)[8]) {
-        const float f = factor(h), r = f != 0.0f ? half_bits_to_float(h.h.x >> 16) / f : 0.0f;
+        const float d = half_bits_to_float(h.h.x), f = factor(h), r = f != 0.0f ? half_bits_to_float(h.h.x >> 16) / f : 0.0f, mid = MID * scale_by(d, f);
 #pragma unroll
         for (int c = 0; c < 4; c += 2) {
             uint32_t sc, mn;
@@ -440,7 +443,8 @@ struct HalfK45 {
 #pragma unroll
             for (int i = 0; i < 2; i++) {
                 const float a = under2(mn, 0x47000000u, 2 * i) - 32768.0f, b = under2(mn, 0x47000000u, 2 * i + 1) - 32768.0f;
-                split_pair(-r * a, -r * b, v[c + i], v[4 + c + i]);
+                const float sa = under2(sc, 0x47000000u, 2 * i) - 32768.0f, sb = under2(sc, 0x47000000u, 2 * i + 1) - 32768.0f;
+                split_pair(fmaf(-r, a, mid * sa), fmaf(-r, b, mid * sb), v[c + i], v[4 + c + i]);
             }
         }
     }
@@ -528,7 +532,7 @@ struct Half32 {
                                                   uint32_t (&lo)[8]) {
         const uint4 q = Q8 ? raw.q[(2 * part + run) % (Q8 ? 4 : 2)] : raw.q[part];
         const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-        const uint32_t offset = Q8 ? 0xe480e480u : (EXT ? 0xe400e400u : 0xe408e408u);  // -(1024 + 128), -1024, -(1024 + 8)
+        const uint32_t offset = Q8 ? 0xe480e480u : 0xe408e408u;  // -(1024 + 128), -(1024 + 8)
 #pragma unroll
         for (int x = 0; x < 4; x++) {
             const uint32_t v = Q8 ? w[x] ^ 0x80808080u : ((run == 0 ? w[x] : w[x] >> 4) & 0x0f0f0f0fu);
@@ -544,7 +548,8 @@ struct Half32 {
             const uint32_t a[8] = {h.d.x, h.d.y, h.d.z, h.d.w, h.d2.x, h.d2.y, h.d2.z, h.d2.w};
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                split_pair(half_bits_to_float(a[2 * i] >> 16) * inv, half_bits_to_float(a[2 * i + 1] >> 16) * inv, v[i], v[4 + i]);
+                split_pair(fmaf(8.0f, half_bits_to_float(a[2 * i]), half_bits_to_float(a[2 * i] >> 16)) * inv,
+                           fmaf(8.0f, half_bits_to_float(a[2 * i + 1]), half_bits_to_float(a[2 * i + 1] >> 16)) * inv, v[i], v[4 + i]);
             }
         }
     }
