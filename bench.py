@@ -795,10 +795,10 @@ def decode_70b_leg(torch, device, rank, world, shape=None):
                         "frac": round((weight_bytes + kv16) / world / dt16 / 1e9 / peak, 4)},
             "prompt_tokens_per_s": round(seqs * prompt_len / t_prompt, 1), "weight_bytes_per_token": int(weight_bytes), "peak_source": "of " + which,
             "config": "70B shape, %d layers, all Q4_K, rows split over %d GPU(s), 16 prompts of %d tokens in groups of 16, %d timed greedy steps "
-                      "per batch size, fp32 KV cache; batch 1: the fused single-token step (8 launches per layer; with several GPUs the attention and "
+                      "per batch size, fp32 KV cache; batch 1: the fused single-token step (7 launches per layer on one GPU; with several GPUs the attention and "
                       "SwiGLU kernels store the next linear's activation image into every rank, wo / w2 store their rows into every rank's "
-                      "vector, the consumers wait for the flags themselves); batch 16: general kernels, the linears of enough weight rows on the tcgen05 "
-                      "GEMV (16 rows of x in one pass), the others in two passes of 8; both replayed as CUDA graphs" % (layers, world, prompt_len, gen - 2),
+                      "vector, the consumers wait for the flags themselves); batch 16: general kernels, the linears on the tcgen05 matrix kernel in FP32 "
+                      "precision (16 rows of x in one pass); both replayed as CUDA graphs" % (layers, world, prompt_len, gen - 2),
             "first_tokens": {"batch16_seq0": out16[:6], "batch1": out1[:6]}, "parity_check": parity}
 
 
@@ -924,7 +924,7 @@ def decode_leg(torch, device, shape=None):
     return {"tokens_per_s": round(1.0 / dt, 1), "ms_per_token": round(dt * 1e3, 4), "prompt_tokens_per_s": round(prompt_len / t_prompt, 1),
             "prompt_tokens_per_s_tensor_core": round(prompt_len / t_prompt_bf16, 1),
             "prompt_note": "prompt_tokens_per_s: FP32 operands, groups of 8 tokens through the decode kernels; ..._tensor_core: jq_decoder_prompt, the whole "
-                           "prompt in one pass, linears on the tcgen05 prefill kernel with bfloat16 operands (next token %s the FP32 path's)"
+                           "prompt in one pass, linears on the tcgen05 matrix kernel with bfloat16 operands (next token %s the FP32 path's)"
                            % ("equals" if int(nxt_bf16) == int(nxt[-1]) else "differs from"),
             "weight_bytes_per_token": int(weight_bytes), "kv_cache_bytes_per_token": int(kv_bytes),
             "hbm_roofline_tokens_per_s": round(peak * 1e9 / (weight_bytes + kv_bytes), 1),

@@ -121,8 +121,8 @@ JQ_API int jq_dequantize(const jq_weight* w, float* dst, int dst_mem, void* stre
  * caller as ops/Gguf.java:86-93 does), bias may be NULL. Rows are dispatched like the reference
  * dispatches them (ops/Gguf.java:90): few rows to the fused dequantise-GEMV kernels, more (from 5 to 12 on, by format;
  * always above 16) to the tensor-core matrix kernel, which takes x and the weights as sums of two half-precision numbers (22 significant bits, relative to the largest
- * magnitude of a 256-element block) and adds up in FP32, unless the bfloat16 prefill path is selected with
- * jq_set_option. `mem` says where x, bias and y live (all three alike); with JQ_MEM_DEVICE they must
+ * magnitude of a 256-element block) and adds up in FP32 (errors of 2e-7 to 3e-7 of the result's norm, the decode kernels' own),
+ * unless the bfloat16 prefill path is selected with jq_set_option. `mem` says where x, bias and y live (all three alike); with JQ_MEM_DEVICE they must
  * be 16-byte aligned and `stream` is the CUDA stream (cudaStream_t, NULL = default stream).
  */
 JQ_API int jq_linear_f32(const jq_weight* w, const float* x, int64_t m, const float* bias, float* y, int mem,
@@ -141,8 +141,9 @@ JQ_API int jq_linear_bf16(const jq_weight* w, const uint16_t* x_bf16, int64_t m,
 /*
  * Input gradient of the linear: gx[m, k] = g[m, n] . dequant(W), float32 (the backward of Gguf.linear and Quant.linear,
  * ops/Gguf.java:208-212 and ops/Quant.java:191-197: the quantised weight gets no gradient, the bias gradient is the
- * column sum of g and needs no weight). Runs on the matrix kernel with the same two-part operands as jq_linear_f32 of many
- * rows and FP32 accumulation (the reference accumulates in double; results agree within 1e-3 relative).
+ * column sum of g and needs no weight). Runs on the matrix kernel with two-part operands and FP32 accumulation (1.5e-7 of the
+ * result's norm; the reference accumulates in double): 22 significant bits, g relative to the largest magnitude of 128 of a row's
+ * values, weights relative to the largest that their block of 32 columns can hold in 128 rows.
  * `mem` as for jq_linear_f32; device pointers must be 16-byte aligned.
  */
 JQ_API int jq_linear_backward_f32(const jq_weight* w, const float* g, int64_t m, float* gx, int mem, void* stream);

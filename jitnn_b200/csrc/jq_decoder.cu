@@ -1978,7 +1978,9 @@ static int decoder_forward(jq_decoder* d, int seq, bool batch, const int32_t* to
             CK(cudaGraphLaunch(d->graphs[bucket], s), "cudaGraphLaunch");
         }
         // The next range's graph is captured while the GPU is busy with a step shortly before it: in line, the step that crosses over took twice its
-        // time (32 layers of the 7B width: 3.0 ms against 1.56, 16 sequences 8.3 against 3.1). If that fails, the crossing step tries again.
+        // time (32 layers of the 7B width: 3.0 ms against 1.56, eight sequences 8.3 and 5.7 against 3.1 and 3.6). Behind a step of one sequence
+        // it is hidden (1.61 ms at most); with eight, the first time took 6.4 ms, later ones 3.7 against 3.6. If it fails, the crossing step
+        // tries again.
         constexpr int AHEAD = 16;
         if (rc == JQ_OK && (256 << bucket) < d->max_seq && pos0 + 1 + AHEAD > (256 << bucket) && d->graphs[bucket + 1] == nullptr) {
             (void)capture_step(d, T, bucket + 1, s);

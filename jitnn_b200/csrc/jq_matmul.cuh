@@ -20,12 +20,13 @@
 //                row into 32 columns of its lane of the operand in tensor memory. In shared memory, writing and reading the weights took
 //                more of its 128 bytes per clock than the rest together, and bound the kernel. Backward: the weights are the transposed
 //                operand, which only shared memory can hold: a thread makes a 128-byte row of 64 features of one contraction index
-//   last         four or eight warps take finished accumulators from tensor memory (double buffered where that fits), add them up, store y
+//   last         four or sixteen warps take finished accumulators from tensor memory (up to four buffers), add them up, store y
 // A cluster may also split the contraction (ksplit ranges); the ranges' sums then meet through distributed shared memory, in range
 // order. Grid: one cluster per tile and range, or, without ranges, as many CTAs as the GPU has SMs walking the tiles.
 //
-// What bounds it: the tensor pipe for tiles of 200 and more rows of x (BF16, 0.84 of its rate at 256), else the chain of barriers and the
-// dequantiser warps' issue slots (a stage of 128 x 64 weights takes 230 to 260 ns whatever the number of rows).
+// What bounds it: the tensor pipe for BF16 tiles of 200 and more rows of x (1.5 us per unit at 256, the measured rate of a dense BF16 product). Below
+// that a BF16 unit takes 0.95 us whatever the number of rows. FP32, one unit: 0.95 us for 17 MMAs (Q4_K, up to 16 rows), 1.4 for 32 (two parts,
+// up to 32 rows), 1.3 us + 6.5 ns a row for 34 (Q4_K), which is 80 to 110 clocks an MMA and what the hand-over of an accumulator takes besides.
 //
 // Every wait is bounded: one that runs out records a code, raises the CTA's abort flag and all roles fall through to the exit.
 #pragma once
@@ -42,7 +43,8 @@ namespace mm {
 // turn costs besides its instructions (barrier round trips, stores' completion) is several hundred clocks, so longer turns pay wherever
 // tensor memory holds an operand for every group beside the accumulator. JOINED: x's hi and lo rows are one operand of 2 nt columns
 // (fewer of the small MMAs, whose issue would bound), and an operand's activation tiles arrive together.
-// The FP32 instance for more than 32 rows of x adds up 64 columns per thread and has registers for two groups only.
+// The FP32 instance for more than 32 rows of x reads its accumulators with sixteen warps, 32 columns per thread (with eight, their loads' latency
+// bound the kernel: Q4_K 32000 x 4096, 128 rows 114 us, now 87), and has registers for two groups only.
 __host__ __device__ constexpr bool one_part(int type) { return type == JQ_TYPE_Q4_K || type == JQ_TYPE_Q5_K; }
 template <int TYPE, bool FP32, bool BWD, int NMAX>
 struct Shape {
