@@ -240,8 +240,8 @@ static double choose(int type, bool fp32, bool bwd, int64_t ftiles, int units, i
 
 // A product may be cut by features into up to three launches, each with its own tiles: whole waves first, then what is left, which alone would
 // leave most of the chip idle for a whole contraction, with its contraction split over clusters. (57344 x 8192, 16 rows: 448 tiles are three
-// waves and four tiles: 93.8 us in one launch, 80.8 in two. Q4_K 11008 x 4096, 200 rows: 49.5 and 44.6; backward 4096 x 11008, 128 rows: 54.1 and
-// 51.0.) The launch behind waits for the one in front, fills and drains: GAP_NS, measured at 5 to 7 us. Finding the cut takes 10 to 35 us.
+// waves and four tiles: 107.4 us in one launch, 92.2 in two. Q4_K 11008 x 4096, 200 rows: 63.3 and 56.5; backward 4096 x 11008, 128 rows: 67.9
+// and 57.9.) The launch behind waits for the one in front, fills and drains: GAP_NS, measured at 5 to 7 us. Finding the cut takes 10 to 35 us.
 constexpr int MAX_PARTS = 3;
 constexpr double GAP_NS = 7000.0;
 struct Part {
@@ -448,9 +448,9 @@ int launch_matmul_f32_multi(const View* vs, int count, const float* x, int64_t m
     return mm::product_f32(vs, count, false, x, nullptr, m, nullptr, ys, s);
 }
 
-// More than 16 rows of x always: the weight is read once for all of them. Up to 16 rows take the same time as one (Q4_K 32000 x 4096: 27 us,
-// Q6_K 41, 4096 x 4096: 11), so the line lies where the decode kernels need another pass: Q4_K and Q5_K take up to eight rows in one
-// (25 us), Q6_K four (35), the 32-element formats two (24 and 16). It must not depend on the number of output rows, and neither do
+// More than 16 rows of x always: the weight is read once for all of them. Up to 16 rows take the same time as one (Q4_K 32000 x 4096: 32 us, Q6_K
+// 45, the others 44, Q4_K 4096 x 4096 12), so the line lies where the decode kernels need another pass: Q4_K and Q5_K take up to eight rows in
+// one (25 us), Q6_K four (34), the 32-element formats two (24 and 16). It must not depend on the number of output rows, and neither do
 // the sums, so a row shard gives bitwise the outputs of the whole weight. Where the decode kernels decline (k no multiple of 256, or too
 // wide) there is only the CUDA-core kernel besides, whose time grows with rows x k: with 4096 output rows it meets the matrix kernel near
 // rows k = 4096 for Q8_0 (k = 1056: 16.4 us at 4 rows against 17.4; 2080: 16.4 at 2 rows and 24.6 at 4 against 19.2) and near 2048 for Q4_0 and
