@@ -744,8 +744,18 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                         for (int j = 0; j < TURN; j++) {
                             raw[j] = D::load(uq, row, c0 + j);
                         }
-                        if (OWNED || turn + G >= TURNS) {  // this warp has read all it needs of the unit
-                            __syncwarp();
+                        if (OWNED || turn + G >= TURNS) {
+                            // This warp has read all it needs of the unit once the values are in registers. Program order alone does not see to that: the
+                            // arrival overtook loads whose values were used later, and the next unit was copied over what they had yet to read (backward,
+                            // 11008 x 4096 Q4_0, 128 rows: wrong weights in 179 of 200 calls). A vote on a word of every load waits for them.
+                            uint32_t seen = D::seen(head);
+#pragma unroll
+                            for (int j = 0; j < TURN; j++) {
+                                seen ^= words_seen(raw[j]);
+                            }
+                            if (__any_sync(0xffffffffu, seen == 0x9E3779B9u)) {
+                                __threadfence_block();  // (nothing more to wait for)
+                            }
                             if (lane == 0) {
                                 tc::mbar_arrive(raw_read + 8 * r);
                             }

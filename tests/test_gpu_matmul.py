@@ -229,3 +229,23 @@ def test_error_is_no_larger_than_the_decode_kernels(t):
             worst[name, m] = float((y.double() - ref).norm() / ref.norm())
     assert max(v for (name, _), v in worst.items() if name == "forward") <= 3.2e-7, worst
     assert max(v for (name, _), v in worst.items() if name == "backward") <= 1.8e-7, worst
+
+
+# Many units through the ring of raw blocks, back to back: a unit that is copied over while a warp still reads it shows as weights of another unit
+# (so did the backward form of every format but Q4_K and Q4_1, and the bfloat16 one of Q8_0, in up to nine calls of ten).
+@pytest.mark.parametrize("t,n,k,m,kind", [("Q4_0", 11008, 4096, 128, "backward"), ("Q8_0", 11008, 4096, 128, "backward"), ("Q5_K", 11008, 4096, 128, "backward"),
+                                          ("Q6_K", 11008, 4096, 128, "backward"), ("Q4_1", 11008, 4096, 100, "backward"), ("Q4_K", 11008, 4096, 128, "backward"),
+                                          ("Q8_0", 4096, 4096, 512, "bf16"), ("Q6_K", 4096, 4096, 512, "bf16"), ("Q4_K", 11008, 4096, 200, "forward"),
+                                          ("Q8_0", 11008, 4096, 16, "forward")])
+def test_repeated_calls_give_the_same_bits(t, n, k, m, kind):
+    w, _ = weight(t, n, k, seed=2)
+    x = torch.randn(m, n if kind == "backward" else k, generator=torch.Generator().manual_seed(4)).cuda()
+    call = {"backward": lambda: Gguf.linearBackward(x, w), "forward": lambda: Gguf.linear(x, w), "bf16": lambda: Gguf.linearBf16(x.to(torch.bfloat16), w)}[kind]
+    call()
+    torch.cuda.synchronize()
+    alone = call()  # with nothing before or behind it
+    torch.cuda.synchronize()
+    for _ in range(5):
+        ys = [call() for _ in range(20)]
+        assert all(torch.equal(y, alone) for y in ys)
+    assert device_status(0) == 0
