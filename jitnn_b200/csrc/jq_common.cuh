@@ -247,6 +247,8 @@ int launch_matmul_f32(const View& v, const float* x, int64_t m, const float* bia
 int launch_matmul_f32_swiglu(const View& v, const float* gate, const float* up, int64_t m, float* y, cudaStream_t s);
 // Up to three weights of one k on the same x: the split of x into halves is shared, weights of one format are one launch.
 int launch_matmul_f32_multi(const View* vs, int count, const float* x, int64_t m, float* const* ys, cudaStream_t s);
+// The rows kernel (jq_rows.cu): the same for up to 16 rows of x (up: x is silu(x) * up).
+int launch_rows(const View* vs, int count, const float* x, const float* up, int m, const float* bias, float* const* ys, cudaStream_t s);
 bool matmul_takes(const View& v, int64_t rows);  // where it is the fastest of the FP32 kernels
 bool prefill_supported(const View& v);
 int launch_prefill_bf16(const View& v, const uint16_t* x_bf16, int64_t m, const float* bias, float* y, cudaStream_t s);

@@ -368,6 +368,14 @@ static int product_f32(const View* vs, int count, bool bwd, const float* x, cons
         const int stride = (rows + 128 + 15) / 16 * 16;  // tiles of rows reach at most this far
         const float* xg = x + m0 * width;
         const float* ug = up != nullptr ? up + m0 * width : nullptr;
+        if (!bwd && rows <= 16) {
+            float* at[MAX_WEIGHTS];
+            for (int i = 0; i < count; i++) {
+                at[i] = ys[i] + m0 * vs[i].n;
+            }
+            rc = launch_rows(vs, count, xg, ug, rows, bias, at, s);
+            continue;
+        }
         const int vec = width % 4 == 0 && (((uintptr_t)xg | (uintptr_t)ug) & 15) == 0;
         // weights with the 16 more columns per unit and weights without: one split each
         for (int ext = 0; ext < 2 && rc == JQ_OK; ext++) {

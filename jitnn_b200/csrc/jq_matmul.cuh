@@ -164,8 +164,8 @@ __device__ __forceinline__ void cluster_sync() {
 // A bounded wait, as tc::mbar_wait. (A try_wait with a time limit of its own becomes a sleep in software that wakes late.) Most roles start
 // before the kernel in front of this one has ended, and in the end all of them wait for what it writes: the limit counts from its end on. The
 // roles that have waited for it already (AFTER) need no second turn.
-template <bool AFTER = false>
-__device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, const Args& p, int code) {
+template <bool AFTER = false, typename A>
+__device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, const A& p, int code) {
     if (tc::mbar_try(bar, parity)) {
         return true;
     }
@@ -189,8 +189,8 @@ __device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, volatile int
 }
 
 // The same for a whole warp that goes on to warp-wide instructions: all lanes or none.
-template <bool AFTER = false>
-__device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, const Args& p, int code) {
+template <bool AFTER = false, typename A>
+__device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, const A& p, int code) {
     return __all_sync(0xffffffffu, wait<AFTER>(bar, parity, abort_flag, p, code));
 }
 

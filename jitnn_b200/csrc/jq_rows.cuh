@@ -1,0 +1,746 @@
+// The rows kernel: y[m, n] = x[m, k] . W[n, k]^T (+ bias) in FP32 for up to 16 rows of x on the 5th-generation tensor cores, every weight read once.
+//
+// What bounds it. At 6.5 TB/s an SM gets a unit of 128 rows x 256 k of Q4_K (18 KB) in 770 clocks. The tensor core needs 270 of them: an MMA of 128
+// weights' rows x 32 columns x 16 k whose weights lie in tensor memory takes 16 clocks. What is scarce is instructions: a unit is 64 KB of halves to
+// be made by the warps, and with 1050 instructions per scheduler and unit, a fifth of the time without the next instruction at hand (long unrolled
+// code of five roles), the same product as an instance of the matrix kernel (jq_matmul.cuh) took 1800 clocks a unit. So the roles here are small loops,
+// and the weights are made with as few instructions as there are:
+// * A quant in the low bits of a half IS the subnormal half q 2^-24: 1.1 logic operations a pair and one fused multiply-add that
+//   multiplies by the scale and takes off the middle of the quants' range, exactly (Q4_K, Q5_K: (q - 8) scale <= 1008 is a half). Bits 4 .. 7
+//   stay in place, as 16 q. The pairs are values 0 and 2, 1 and 3 of four; x's image has the same order.
+// * d and dmin go to the sums: the mins, times the sums of x over 32 values, have columns of their own in tensor memory.
+// * Formats whose products do not fit a half (Q6_K 13 bits, 32-element formats 15 to 18) have two: hi = scale q rounded, lo = the rest, exact.
+//
+// x is split into halves hi + lo, 22 bits a value, times a power of two per row and 256 values (image_kernel in jq_rows.cu): 16 + 16 columns of one B
+// operand; a unit's part of the image is one contiguous copy. An accumulator holds 256 (two-part formats and Q5_K: 128) terms before its sums are
+// added up in registers, rounded to nearest: the tensor core cuts sums off towards zero.
+//
+// Roles: warp 0 brings in raw units, warp 2 the image, one bulk copy each; warp 1 issues the MMAs; warps 4 .. 11 add up (a warp may only read its
+// quarter of tensor memory's lanes; two share it, eight rows of x each); warps 12 .. 19 are two groups that turn raw units into operands in tensor memory (three of them), thread = row of W.
+//
+// k is cut into eight ranges whatever the grid is; a range's units are added up in order, then the ranges. So a row shard gives bitwise what the whole
+// weight gives, and a cluster of 2, 4 or 8 thread blocks may share the ranges (their sums meet through distributed shared memory) where there
+// are too few tiles of rows to fill the chip.
+//
+// Every wait is bounded: one that runs out records a code (as jq_matmul.cuh's), raises the thread block's abort flag, and all roles leave their loops.
+#pragma once
+
+#include "jq_matmul.cuh"
+
+namespace jq {
+namespace rows {
+
+using mm::add2;
+using mm::elect_one;
+using mm::f2;
+using mm::fma2;
+using mm::hadd2;
+using mm::hfma2;
+using mm::hmul2;
+using mm::lds16;
+using mm::mul2;
+using mm::pack2;
+using mm::unpack2;
+
+constexpr int NT = 16, N = 32;       // rows of x, columns
+constexpr int RANGES = 8;
+constexpr int MAX_WEIGHTS = 3;
+constexpr int GROUPS = 2, FOLD = 8, THREADS = (4 + FOLD + 4 * GROUPS) * 32;
+constexpr int C = NT / (FOLD / 4);   // columns (rows of x) of a fold warp
+constexpr int STEP = N * 32;         // bytes of 16 k of the image: [8 k][8 columns][8 rows of 16 bytes]
+constexpr int IMAGE = 17 * STEP;     // of a unit: 256 k, then the sums of x over its runs of 32, twice, as 16 more k
+constexpr int MAX_RAW = 6, MAX_IMG = 6, OPERANDS = 3, MAX_ACC = 4, FACTORS = 8;
+
+struct Args {
+    const uint8_t* q[MAX_WEIGHTS];
+    const uint8_t* aux[MAX_WEIGHTS];
+    float* y[MAX_WEIGHTS];
+    int64_t n[MAX_WEIGHTS];
+    int ft_end[MAX_WEIGHTS];  // tiles of 128 rows up to and including each weight
+    const uint8_t* image;     // [units][IMAGE]
+    const float* scales;      // [units][NT]
+    const float* bias;        // of the first weight, or null
+    int units, ftiles, m;
+    int ksplit;               // thread blocks that share a tile's ranges
+    int raw, img;             // ring depths
+    int* status;
+    long long wait_clocks;
+};
+
+__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+    return r;
+}
+__device__ __forceinline__ uint32_t lds4(uint32_t at) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(at));
+    return v;
+}
+__device__ __forceinline__ void sts_pair(uint32_t at, float a, float b) { asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(at), "f"(a), "f"(b) : "memory"); }
+__device__ __forceinline__ void st_tmem16(uint32_t addr, const uint32_t (&v)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+                 "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+                 : "memory");
+}
+// D (tensor memory) = or += A (tensor memory) . B (shared memory, K-major core matrices without swizzle)
+__device__ __forceinline__ void mma(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 db, {%2, %5};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t}" ::"r"(d),
+        "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "r"((128u >> 4) | (1u << 14))  // 128 bytes between groups of 8 columns
+        : "memory");
+}
+__device__ __forceinline__ uint32_t desc(uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | ((uint32_t)(N * 16) >> 4 << 16); }  // between the two halves of a step
+constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(128 >> 4) << 24);
+constexpr uint32_t ID_N = IDESC | ((uint32_t)(N >> 3) << 17), ID_NT = IDESC | ((uint32_t)(NT >> 3) << 17);
+
+constexpr uint32_t dup(uint32_t half_bits) { return half_bits * 0x10001u; }
+
+// Several barriers at once for a whole warp. A poll that finds its phase complete takes a warp among four busy ones 200 clocks and more, one after the
+// other; the answers to several polls come back together. What is not complete is waited for in turn, by a wait that suspends the warp: a loop
+// of polls takes issue slots from the very warps it waits for.
+struct Phase {
+    uint32_t bar, parity;
+    int code;
+};
+template <typename... P>
+__device__ __forceinline__ bool wait_all(volatile int* abort_flag, const Args& p, const P&... phases) {
+    constexpr int COUNT = sizeof...(P);
+    bool ready[COUNT];
+    int i = 0;
+    ((ready[i++] = tc::mbar_test(phases.bar, phases.parity)), ...);
+    i = 0;
+    return ((__all_sync(0xffffffffu, ready[i++]) || mm::wait_warp(phases.bar, phases.parity, abort_flag, p, phases.code)) && ...);
+}
+
+// ---- the formats -------------------------------------------------------------------------------------------------------------------
+// PARTS: operand values per weight; MINS: the sums of x have a part (what is the same for 32 weights, the middle of the quants and the min: 8 more columns
+// of an operand, the eight values' hi parts and lo parts, whose products have an accumulator of their own); HALVES: operands per unit; ACCS: accumulators per unit.
+// make(): operand `half` of the row's unit into this lane's columns from `to` on, and (with the first) what the fold multiplies the sums by into `fac`.
+template <int TYPE>
+struct Rw;
+
+// Eight values of at most `bound` as columns of halves, hi then lo, times a power of two; the fold multiplies by its inverse.
+__device__ __forceinline__ float sums_part(const float (&e)[8], float bound, uint32_t to) {
+    const uint32_t ex = min(max(__float_as_uint(bound) >> 23, 40u), 250u);
+    const float by = __uint_as_float((267u - ex) << 23);  // below 2^14
+    uint32_t v[8];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        mm::split_pair(e[2 * i] * by, e[2 * i + 1] * by, v[i], v[4 + i]);
+    }
+    mm::st_tmem8(to, v);
+    return __uint_as_float((ex - 13u) << 23);
+}
+
+// Q4_K and Q5_K: values scale (q - mid) 2^-14.
+template <bool FIVE>
+struct RwK45 {
+    static constexpr int ROW = FIVE ? 176 : 144, AUX = 0, PARTS = 1, HALVES = 1, ACCS = FIVE ? 2 : 1;
+    static constexpr bool MINS = true;
+    __device__ static __forceinline__ void make(uint32_t uq, uint32_t, int row, int, uint32_t to, uint32_t fac) {
+        const uint32_t at = uq + (uint32_t)(row * ROW);
+        const uint4 h = lds16(at);
+        uint4 q0 = lds16(at + (FIVE ? 48 : 16)), q1 = lds16(at + (FIVE ? 64 : 32));
+        uint4 b0 = make_uint4(0, 0, 0, 0), b1 = b0;
+        if constexpr (FIVE) {
+            b0 = lds16(at + 16);
+            b1 = lds16(at + 32);
+        }
+        const uint32_t sc0 = h.y & 0x3f3f3f3fu, sc1 = and_or(h.y >> 2, 0x30303030u, h.w & 0x0f0f0f0fu);
+        const uint32_t mn0 = h.z & 0x3f3f3f3fu, mn1 = and_or(h.z >> 2, 0x30303030u, (h.w >> 4) & 0x0f0f0f0fu);
+        {
+            const float d = half_bits_to_float(h.x), dmin = half_bits_to_float(h.x >> 16), mid = d * (FIVE ? 16.0f : 8.0f);
+            float e[8];  // mid d scale - dmin min; a byte in the mantissa of 2^23
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const float sc = __uint_as_float(__byte_perm(i < 4 ? sc0 : sc1, 0x4B000000u, 0x7540u + (uint32_t)(i & 3))) - 8388608.0f;
+                const float mn = __uint_as_float(__byte_perm(i < 4 ? mn0 : mn1, 0x4B000000u, 0x7540u + (uint32_t)(i & 3))) - 8388608.0f;
+                e[i] = fmaf(-dmin, mn, mid * sc);
+            }
+            const float f1 = sums_part(e, fmaxf(63.0f * fabsf(mid), 63.0f * fabsf(dmin)) * 2.0f, to + 128);
+            sts_pair(fac, d * 16384.0f, f1);
+        }
+#pragma unroll 1
+        for (int j = 0; j < 4; j++) {
+            const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+            const uint32_t g[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+            if (j < 3) {
+                q0 = lds16(at + (FIVE ? 80 : 48) + 32 * (uint32_t)j);
+                q1 = lds16(at + (FIVE ? 96 : 64) + 32 * (uint32_t)j);
+            }
+            const uint32_t sc = j < 2 ? sc0 : sc1, pick = 0x4040u + 0x0202u * (uint32_t)(j & 1);
+            const uint32_t a = hadd2(__byte_perm(sc, 0x64646464u, pick), 0xE400E400u), b = hadd2(__byte_perm(sc, 0x64646464u, pick + 0x0101u), 0xE400E400u);
+            // q 2^-24 x scale 2^10 and 16 q 2^-24 x scale 2^6, minus mid scale 2^-14
+            const uint32_t sa = hmul2(a, dup(0x6400)), sb = hmul2(b, dup(0x5400)), ca = hmul2(a, FIVE ? dup(0x9400) : dup(0x9000)),
+                           cb = hmul2(b, FIVE ? dup(0x9400) : dup(0x9000));
+            uint32_t lo[16], hi[16];
+#pragma unroll
+            for (int x = 0; x < 8; x++) {
+                const uint32_t v = w[x], u = v >> 8;
+                uint32_t l0 = v & 0x000F000Fu, l1 = u & 0x000F000Fu, h0 = v & 0x00F000F0u, h1 = u & 0x00F000F0u;
+                if constexpr (FIVE) {
+                    const uint32_t t = g[x] >> (2 * j);  // bits 2 j and 2 j + 1 of every byte, to bit 4 and bit 8
+                    l0 = and_or(t << 4, 0x00100010u, l0);
+                    l1 = and_or(t >> 4, 0x00100010u, l1);
+                    h0 = and_or(t << 7, 0x01000100u, h0);
+                    h1 = and_or(t >> 1, 0x01000100u, h1);
+                }
+                lo[2 * x] = hfma2(l0, sa, ca);
+                lo[2 * x + 1] = hfma2(l1, sa, ca);
+                hi[2 * x] = hfma2(h0, sb, cb);
+                hi[2 * x + 1] = hfma2(h1, sb, cb);
+            }
+            st_tmem16(to + 32 * (uint32_t)j, lo);
+            st_tmem16(to + 32 * (uint32_t)j + 16, hi);
+        }
+    }
+};
+template <>
+struct Rw<JQ_TYPE_Q4_K> : RwK45<false> {};
+template <>
+struct Rw<JQ_TYPE_Q5_K> : RwK45<true> {};
+
+// hi and lo of the products of two pairs of quants
+__device__ __forceinline__ void product(uint32_t q, uint32_t s, uint32_t& hi, uint32_t& lo) {
+    hi = hmul2(q, s);
+    lo = hfma2(q, s, hi ^ 0x80008000u);
+}
+
+template <>
+struct Rw<JQ_TYPE_Q6_K> {
+    static constexpr int ROW = 208, AUX = 2, PARTS = 2, HALVES = 2, ACCS = 2;
+    static constexpr bool MINS = false;
+    __device__ static __forceinline__ void make(uint32_t uq, uint32_t ua, int row, int half, uint32_t to, uint32_t fac) {
+        const uint32_t at = uq + (uint32_t)(row * ROW), l = at + 64u * (uint32_t)half, h = at + 128u + 32u * (uint32_t)half;
+        const uint32_t s0 = lds4(at + 192u + 8u * (uint32_t)half) ^ 0x80808080u, s1 = lds4(at + 196u + 8u * (uint32_t)half) ^ 0x80808080u;
+        const uint32_t dw = lds4(ua + 4u * (uint32_t)(row >> 1));
+        if (half == 0) {
+            sts_pair(fac, half_bits_to_float((row & 1) != 0 ? dw >> 16 : dw), 0.0f);
+        }
+#pragma unroll 1
+        for (int p = 0; p < 2; p++) {  // bytes 16 p .. 16 p + 15 of the half's runs of 32
+            const uint4 qa = lds16(l + 16u * (uint32_t)p), qb = lds16(l + 32u + 16u * (uint32_t)p), qh = lds16(h + 16u * (uint32_t)p);
+            const uint32_t wa[4] = {qa.x, qa.y, qa.z, qa.w}, wb[4] = {qb.x, qb.y, qb.z, qb.w}, wh[4] = {qh.x, qh.y, qh.z, qh.w};
+            // runs 0 .. 3: low nibbles of a and b, high nibbles of a and b; their scales are bytes p, p + 2, p + 4, p + 6
+#pragma unroll
+            for (int run = 0; run < 4; run++) {
+                const uint32_t pick = 0x4040u + 0x0101u * (uint32_t)(2 * (run & 1) + p);
+                const uint32_t s = hadd2(__byte_perm(run < 2 ? s0 : s1, 0x64646464u, pick), 0xE480E480u);  // 1024 + 128 + scale
+                uint32_t hi[8], lo[8];
+#pragma unroll
+                for (int x = 0; x < 4; x++) {
+#pragma unroll
+                    for (int odd = 0; odd < 2; odd++) {
+                        const uint32_t v = (run & 1 ? wb[x] : wa[x]) >> (8 * odd), b = wh[x] >> (8 * odd);
+                        uint32_t q;  // 1024 + q, and 1024 + 16 q; minus 32
+                        if (run < 2) {
+                            q = hadd2(and_or(v, 0x000F000Fu, and_or(run == 0 ? b << 4 : b << 2, 0x00300030u, 0x64006400u)), 0xE420E420u);
+                        } else {
+                            q = hfma2(and_or(v, 0x00F000F0u, and_or(run == 2 ? b << 4 : b << 2, 0x03000300u, 0x64006400u)), 0x2C002C00u, 0xD600D600u);
+                        }
+                        product(q, s, hi[2 * x + odd], lo[2 * x + odd]);
+                    }
+                }
+                const uint32_t col = to + (uint32_t)(16 * run) + 8u * (uint32_t)p;
+                mm::st_tmem8(col, hi);
+                mm::st_tmem8(col + 64, lo);
+            }
+        }
+    }
+};
+
+// The 32-element formats: block scales d' = d 2^-e in [2^4, 2^5) at the largest of the row's eight; the fold multiplies by 2^e.
+template <int TYPE>
+struct Rw32 {
+    static constexpr bool Q8 = TYPE == JQ_TYPE_Q8_0, MINS = TYPE == JQ_TYPE_Q4_1;
+    static constexpr int ROW = Q8 ? 256 : 128, AUX = MINS ? 32 : 16, PARTS = 2, HALVES = 2, ACCS = 2;
+    __device__ static __forceinline__ void make(uint32_t uq, uint32_t ua, int row, int half, uint32_t to, uint32_t fac) {
+        const uint32_t at = uq + (uint32_t)(row * ROW), au = ua + (uint32_t)(row * AUX);
+        const uint4 d0 = lds16(au), d1 = MINS ? lds16(au + 16) : d0;
+        uint32_t ds[4];  // the eight d
+        if constexpr (MINS) {
+            ds[0] = __byte_perm(d0.x, d0.y, 0x5410), ds[1] = __byte_perm(d0.z, d0.w, 0x5410), ds[2] = __byte_perm(d1.x, d1.y, 0x5410), ds[3] = __byte_perm(d1.z, d1.w, 0x5410);
+        } else {
+            ds[0] = d0.x, ds[1] = d0.y, ds[2] = d0.z, ds[3] = d0.w;
+        }
+        const uint32_t e = mm::scale_exponent(mm::max_half8(make_uint4(ds[0], ds[1], ds[2], ds[3])));
+        const float inv = __uint_as_float((258u - e) << 23);  // 2^(4 + 127 - e)
+        // (the second half's group knows the sums' part, the first half's has to know its factor)
+        float bound = 0.0f;
+        if constexpr (MINS) {
+            const uint32_t a[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+            float c[8];  // 8 d + m
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                c[i] = fmaf(8.0f, half_bits_to_float(a[i]), half_bits_to_float(a[i] >> 16));
+                bound = fmaxf(bound, fabsf(c[i]));
+            }
+            if (half == 1) {
+                sums_part(c, bound, to + 128);
+            }
+        }
+        if (half == 0) {
+            const uint32_t ex = min(max(__float_as_uint(bound) >> 23, 40u), 250u);
+            sts_pair(fac, __uint_as_float((e - 4u) << 23), __uint_as_float((ex - 13u) << 23));
+        }
+        const uint32_t dp[2] = {half ? ds[2] : ds[0], half ? ds[3] : ds[1]};
+#pragma unroll 1
+        for (int b = 0; b < 4; b++) {  // blocks of 32 of the half
+            const uint32_t dw = b < 2 ? dp[0] : dp[1];
+            const uint32_t s = mm::h2_dup(half_bits_to_float((b & 1) != 0 ? dw >> 16 : dw) * inv);
+            const uint32_t col = to + 16u * (uint32_t)b;
+            uint32_t hi[8], lo[8];
+            if constexpr (Q8) {
+#pragma unroll
+                for (int c = 0; c < 2; c++) {
+                    const uint4 q = lds16(at + 16u * (uint32_t)swizzle_piece(8 * half + 2 * b + c, row));
+                    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                    for (int x = 0; x < 4; x++) {
+                        const uint32_t u = w[x] ^ 0x80808080u;  // q + 128 under 0x64: 1024 + that
+                        product(hadd2(__byte_perm(u, 0x64646464u, 0x4240), 0xE480E480u), s, hi[2 * x], lo[2 * x]);
+                        product(hadd2(__byte_perm(u, 0x64646464u, 0x4341), 0xE480E480u), s, hi[2 * x + 1], lo[2 * x + 1]);
+                    }
+                    mm::st_tmem8(col + 8u * (uint32_t)c, hi);
+                    mm::st_tmem8(col + 8u * (uint32_t)c + 64u, lo);
+                }
+            } else {
+                const uint4 q = lds16(at + 16u * (uint32_t)swizzle_piece(4 * half + b, row));
+                const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                for (int c = 0; c < 2; c++) {  // low nibbles, high nibbles: 1024 + q, 1024 + 16 q; minus 8
+#pragma unroll
+                    for (int x = 0; x < 4; x++) {
+#pragma unroll
+                        for (int odd = 0; odd < 2; odd++) {
+                            const uint32_t v = w[x] >> (8 * odd);
+                            const uint32_t n = c == 0 ? hadd2(and_or(v, 0x000F000Fu, 0x64006400u), 0xE408E408u) : hfma2(and_or(v, 0x00F000F0u, 0x64006400u), 0x2C002C00u, 0xD480D480u);
+                            product(n, s, hi[2 * x + odd], lo[2 * x + odd]);
+                        }
+                    }
+                    mm::st_tmem8(col + 8u * (uint32_t)c, hi);
+                    mm::st_tmem8(col + 8u * (uint32_t)c + 64u, lo);
+                }
+            }
+        }
+    }
+};
+template <>
+struct Rw<JQ_TYPE_Q8_0> : Rw32<JQ_TYPE_Q8_0> {};
+template <>
+struct Rw<JQ_TYPE_Q4_0> : Rw32<JQ_TYPE_Q4_0> {};
+template <>
+struct Rw<JQ_TYPE_Q4_1> : Rw32<JQ_TYPE_Q4_1> {};
+
+// Tensor memory: accumulators (32 columns each, then 16 each for the mins' sums), behind them the operands.
+template <int TYPE>
+struct Shape {
+    using F = Rw<TYPE>;
+    static constexpr int UNIT_Q = 128 * F::ROW, UNIT_A = 128 * F::AUX, UNIT = UNIT_Q + UNIT_A;
+    static constexpr int A_COLS = 128 + (F::MINS ? 8 : 0);
+    static constexpr int ACC = F::MINS ? 2 : 4, ACC_COLS = ACC * (N + (F::MINS ? NT : 0));  // accumulators
+    static_assert(ACC_COLS + OPERANDS * A_COLS <= 512, "tensor memory");
+};
+constexpr int TAIL = FACTORS * 128 * 8 + 4 * 1024 + 1024;  // factors, the fold warps' scales of x, barriers
+constexpr int part_bytes(int ksplit) { return ksplit > 1 ? RANGES / ksplit * NT * 512 : 0; }
+
+template <int TYPE>
+__global__ void __launch_bounds__(THREADS, 1) rows_kernel(const __grid_constant__ Args p) {
+    using F = Rw<TYPE>;
+    using S = Shape<TYPE>;
+    extern __shared__ uint8_t smem_unaligned[];
+    const uint32_t base = (tc::smem_u32(smem_unaligned) + 127u) & ~127u;  // sums of this thread block's ranges (ksplit > 1), then the rings
+    const uint32_t img0 = base + (uint32_t)(p.ksplit > 1 ? RANGES / p.ksplit * NT * 512 : 0), raw0 = img0 + (uint32_t)(p.img * IMAGE), fac0 = raw0 + (uint32_t)(p.raw * S::UNIT);
+    const uint32_t scl0 = fac0 + FACTORS * 128 * 8, bars = scl0 + 4 * 1024;
+    const uint32_t img_full = bars, img_free = img_full + 8 * MAX_IMG, raw_full = img_free + 8 * MAX_IMG, raw_free = raw_full + 8 * MAX_RAW;
+    const uint32_t full_a = raw_free + 8 * MAX_RAW, free_a = full_a + 8 * OPERANDS, acc_full = free_a + 8 * OPERANDS, acc_free = acc_full + 8 * MAX_ACC;
+    const uint32_t fac_full = acc_free + 8 * MAX_ACC, slot_s = fac_full + 8 * FACTORS;
+    uint8_t* const generic = smem_unaligned + (slot_s - tc::smem_u32(smem_unaligned));
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(generic);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(generic + 4);
+
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int range = p.ksplit == 1 ? 0 : (int)mm::cluster_rank();
+    const int cluster_id = (int)blockIdx.x / p.ksplit, clusters = (int)gridDim.x / p.ksplit;
+    const int u0 = (int)((int64_t)range * p.units / p.ksplit), u1 = (int)((int64_t)(range + 1) * p.units / p.ksplit);
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < MAX_IMG; i++) {
+            tc::mbar_init(img_full + 8 * i, 1);
+            tc::mbar_init(img_free + 8 * i, 1);
+        }
+        for (int i = 0; i < MAX_RAW; i++) {
+            tc::mbar_init(raw_full + 8 * i, 1);
+            tc::mbar_init(raw_free + 8 * i, 4 * F::HALVES);
+        }
+        for (int i = 0; i < OPERANDS; i++) {
+            tc::mbar_init(full_a + 8 * i, 4);
+            tc::mbar_init(free_a + 8 * i, 1);
+        }
+        for (int i = 0; i < MAX_ACC; i++) {
+            tc::mbar_init(acc_full + 8 * i, 1);
+            tc::mbar_init(acc_free + 8 * i, FOLD);
+        }
+        for (int i = 0; i < FACTORS; i++) {
+            tc::mbar_init(fac_full + 8 * i, 4);
+        }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(slot_s) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    if (p.ksplit > 1) {
+        mm::cluster_sync();
+    }
+    tc::fence_after_sync();
+    asm volatile("griddepcontrol.launch_dependents;");
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    const uint32_t tmem_m = tmem + S::ACC * N, tmem_a = tmem + S::ACC_COLS;
+
+    auto weight_of = [&](int ft, int& ft0) {
+        const int w = ft < p.ft_end[0] ? 0 : (ft < p.ft_end[1] ? 1 : 2);
+        ft0 = w == 0 ? 0 : (w == 1 ? p.ft_end[0] : p.ft_end[1]);
+        return w;
+    };
+    bool ok = true;
+    if (warp == 0) {
+        // ---- raw units -------------------------------------------------------------------------------------------------------------
+        if (lane == 0) {
+            int r = 0;
+            uint32_t ph = 1;
+            for (int ft = cluster_id; ft < p.ftiles && ok; ft += clusters) {
+                int ft0;
+                const int w = weight_of(ft, ft0);
+                const int64_t first = (int64_t)(ft - ft0) * p.units;
+                const uint8_t* const q = mm::pick(p.q, w) + first * S::UNIT_Q;
+                const uint8_t* const a = mm::pick(p.aux, w) + first * S::UNIT_A;
+                for (int u = u0; u < u1; u++) {
+                    if (!(ok = mm::wait(raw_free + 8 * r, ph, abort_flag, p, 8))) {
+                        break;
+                    }
+                    const uint32_t to = raw0 + (uint32_t)(r * S::UNIT), bar = raw_full + 8 * r;
+                    tc::mbar_expect_tx(bar, S::UNIT);
+                    tc::bulk_load(to, q + (int64_t)u * S::UNIT_Q, S::UNIT_Q, bar);
+                    if constexpr (F::AUX > 0) {
+                        tc::bulk_load(to + S::UNIT_Q, a + (int64_t)u * S::UNIT_A, S::UNIT_A, bar);
+                    }
+                    if (++r == p.raw) {
+                        r = 0;
+                        ph ^= 1;
+                    }
+                }
+            }
+        }
+    } else if (warp == 2) {
+        // ---- the image ---------------------------------------------------------------------------------------------------------------
+        if (lane == 0) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");  // the kernel in front writes it
+            int s = 0;
+            uint32_t ph = 1;
+            for (int ft = cluster_id; ft < p.ftiles && ok; ft += clusters) {
+                for (int u = u0; u < u1; u++) {
+                    if (!(ok = mm::wait<true>(img_free + 8 * s, ph, abort_flag, p, 3))) {
+                        break;
+                    }
+                    tc::mbar_expect_tx(img_full + 8 * s, IMAGE);
+                    tc::bulk_load(img0 + (uint32_t)(s * IMAGE), p.image + (int64_t)u * IMAGE, IMAGE, img_full + 8 * s);
+                    if (++s == p.img) {
+                        s = 0;
+                        ph ^= 1;
+                    }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ---- MMAs: an operand's in one go (an election between them costs as much as several) --------------------------------------------
+        int a = 0, s = 0, buf = 0;
+        uint32_t pa = 0, ps = 0, pb = 1;
+        for (int ft = cluster_id; ft < p.ftiles && ok; ft += clusters) {
+            for (int u = u0; u < u1 && ok; u++) {
+                const uint32_t img = desc(img0 + (uint32_t)(s * IMAGE));
+#pragma unroll
+                for (int half = 0; half < F::HALVES; half++) {
+                    constexpr int BUFS = F::ACCS / F::HALVES, STEPS = 16 / F::HALVES;  // accumulators and steps of 16 k of an operand
+                    uint32_t d[BUFS], d_bar[BUFS], dm = 0;
+                    Phase free[BUFS];
+#pragma unroll
+                    for (int i = 0; i < BUFS; i++) {
+                        d[i] = tmem + (uint32_t)(buf * N);
+                        dm = tmem_m + (uint32_t)(buf * NT);
+                        d_bar[i] = acc_full + 8 * buf;
+                        free[i] = Phase{acc_free + 8 * buf, pb, 5};
+                        if (++buf == S::ACC) {
+                            buf = 0;
+                            pb ^= 1;
+                        }
+                    }
+                    if (!(ok = wait_all(abort_flag, p, Phase{img_full + 8 * s, ps, 3}, Phase{full_a + 8 * a, pa, 2}, free[0], free[BUFS - 1]))) {
+                        break;
+                    }
+                    tc::fence_after_sync();
+                    const uint32_t ta = tmem_a + (uint32_t)(a * S::A_COLS), bd = img + (uint32_t)(half * STEPS * (STEP >> 4)), a_bar = free_a + 8 * a, s_bar = img_free + 8 * s;
+                    if (elect_one()) {
+#pragma unroll
+                        for (int i = 0; i < STEPS; i++) {
+                            const int b = i / (STEPS / BUFS);
+                            mma(d[b], ta + 8 * i, bd + i * (STEP >> 4), ID_N, i % (STEPS / BUFS) == 0 ? 0u : 1u);  // hi x (hi | lo)
+                            if constexpr (F::PARTS == 2) {
+                                mma(d[b] + NT, ta + 64 + 8 * i, bd + i * (STEP >> 4), ID_NT, 1u);  // lo x hi, beside the other small products
+                            }
+                            if (F::MINS && half == F::HALVES - 1 && i == STEPS - 1) {
+                                mma(dm, ta + 128, img + 16 * (STEP >> 4) + (NT * 16 >> 4), ID_NT, 0u);
+                                mma(dm, ta + 128, img + 16 * (STEP >> 4), ID_NT, 1u);
+                            }
+                            if ((i + 1) % (STEPS / BUFS) == 0) {
+                                tc::umma_commit(d_bar[b]);
+                            }
+                        }
+                        tc::umma_commit(a_bar);
+                        if (half == F::HALVES - 1) {
+                            tc::umma_commit(s_bar);
+                        }
+                    }
+                    __syncwarp();
+                    if (++a == OPERANDS) {
+                        a = 0;
+                        pa ^= 1;
+                    }
+                }
+                if (++s == p.img) {
+                    s = 0;
+                    ps ^= 1;
+                }
+            }
+        }
+    } else if (warp >= 4 + FOLD) {
+        // ---- weights -------------------------------------------------------------------------------------------------------------------
+        const int group = (warp - 4 - FOLD) >> 2, row = (warp & 3) * 32 + lane;
+        const uint32_t to0 = tmem_a + ((uint32_t)((warp & 3) * 32) << 16);
+        const int units = (p.ftiles - cluster_id + clusters - 1) / clusters * (u1 - u0);
+        // One operand per unit: the groups take units in turn, and places in the ring of raw units too (its depth is even), so no group tests a barrier
+        // that is a turn of the ring behind. Two: each group makes its half of every unit.
+        constexpr bool OWN = F::HALVES == 1;
+        int r = OWN ? group : 0, o = group;
+        uint32_t pr = 0, po = 1;
+        for (int unit = OWN ? group : 0; unit < units; unit += OWN ? GROUPS : 1) {
+            if (!(ok = wait_all(abort_flag, p, Phase{raw_full + 8 * r, pr, 6}, Phase{free_a + 8 * o, po, 1}))) {
+                break;
+            }
+            tc::fence_after_sync();
+            const int half = OWN ? 0 : group;
+            const uint32_t uq = raw0 + (uint32_t)(r * S::UNIT), fac = fac0 + (uint32_t)((unit & (FACTORS - 1)) * 1024 + row * 8);
+            F::make(uq, uq + S::UNIT_Q, row, half, to0 + (uint32_t)(o * S::A_COLS), fac);
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) {
+                tc::mbar_arrive(full_a + 8 * o);
+                if (half == 0) {
+                    tc::mbar_arrive(fac_full + 8 * (unit & (FACTORS - 1)));
+                }
+                tc::mbar_arrive(raw_free + 8 * r);  // (all that was read of the unit has been used)
+            }
+            if ((r += OWN ? GROUPS : 1) >= p.raw) {
+                r -= p.raw;
+                pr ^= 1;
+            }
+            if ((o += GROUPS) >= OPERANDS) {
+                o -= OPERANDS;
+                po ^= 1;
+            }
+        }
+    } else if (warp >= 4) {
+        // ---- sums ----------------------------------------------------------------------------------------------------------------------
+        asm volatile("griddepcontrol.wait;" ::: "memory");  // x's scales; and y may be read by the kernel in front
+        const int lane_row = (warp & 3) * 32 + lane;
+        const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+        const int c0 = (warp - 4) / 4 * C;  // this warp's columns
+        const uint32_t scl = scl0 + (uint32_t)(warp - 4) * (16 * C * 4);
+        int chunk = 0, buf = 0;
+        uint32_t pb = 0;
+        // The scales of x of 16 units at a time: a load takes up to 2000 clocks while the weights stream, so it is asked for a whole block ahead.
+        constexpr int NEXT = 16 * C / 32;
+        float next[NEXT];
+        auto fetch = [&](int u) {
+#pragma unroll
+            for (int i = 0; i < NEXT; i++) {
+                const int at = lane + 32 * i, on = at / C;
+                next[i] = u + on < u1 ? __ldg(p.scales + (int64_t)(u + on) * NT + c0 + at % C) : 0.0f;
+            }
+        };
+        const bool keep = u1 - u0 <= 16;  // (a short contraction's stay for the next tile)
+        fetch(u0);
+        for (int ft = cluster_id; ft < p.ftiles && ok; ft += clusters) {
+            f2 sum[C / 2], total[C / 2];
+#pragma unroll
+            for (int i = 0; i < C / 2; i++) {
+                sum[i] = total[i] = 0;
+            }
+            int v = 0;  // the range that the unit belongs to
+            while (v < RANGES - 1 && (int)((int64_t)(v + 1) * p.units / RANGES) <= u0) {
+                v++;
+            }
+            int v_end = (int)((int64_t)(v + 1) * p.units / RANGES);
+            for (int u = u0; u < u1; u++, chunk++) {
+                if (((u - u0) & 15) == 0 && (!keep || ft == cluster_id)) {
+                    __syncwarp();
+#pragma unroll
+                    for (int i = 0; i < NEXT; i++) {
+                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(scl + (uint32_t)(lane + 32 * i) * 4u), "f"(next[i]) : "memory");
+                    }
+                    __syncwarp();
+                    if (!keep) {
+                        fetch(u + 16 < u1 ? u + 16 : u0);
+                    }
+                }
+                const uint32_t xs = scl + (uint32_t)((u - u0) & 15) * (C * 4);
+                uint4 x4[C / 4];
+#pragma unroll
+                for (int j = 0; j < C / 4; j++) {
+                    x4[j] = lds16(xs + 16u * (uint32_t)j);
+                }
+                if (!(ok = wait_all(abort_flag, p, Phase{fac_full + 8 * (chunk & (FACTORS - 1)), (uint32_t)(chunk / FACTORS) & 1u, 6}, Phase{acc_full + 8 * buf, pb, 4}))) {
+                    break;
+                }
+                float f0, f1;
+                asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(f0), "=f"(f1) : "r"(fac0 + (uint32_t)((chunk & (FACTORS - 1)) * 1024 + lane_row * 8)));
+                const f2 ff0 = pack2(f0, f0), ff1 = pack2(f1, f1);
+#pragma unroll
+                for (int acc = 0; acc < F::ACCS; acc++) {
+                    if (acc > 0 && !(ok = mm::wait_warp<true>(acc_full + 8 * buf, pb, abort_flag, p, 4))) {
+                        break;
+                    }
+                    tc::fence_after_sync();
+                    float hi[C], lo[C], mn[C];
+                    mm::ld_tmem8(hi, tmem + lanes + (uint32_t)(buf * N + c0));
+                    mm::ld_tmem8(lo, tmem + lanes + (uint32_t)(buf * N + NT + c0));
+                    const bool mins = F::MINS && acc == F::ACCS - 1;
+                    if (mins) {
+                        mm::ld_tmem8(mn, tmem_m + lanes + (uint32_t)(buf * NT + c0));
+                    }
+                    mm::ld_tmem_done();
+                    tc::fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) {
+                        tc::mbar_arrive(acc_free + 8 * buf);
+                    }
+                    if (++buf == S::ACC) {
+                        buf = 0;
+                        pb ^= 1;
+                    }
+#pragma unroll
+                    for (int j = 0; j < C / 4; j++) {
+                        const f2 sc[2] = {pack2(__uint_as_float(x4[j].x), __uint_as_float(x4[j].y)), pack2(__uint_as_float(x4[j].z), __uint_as_float(x4[j].w))};
+#pragma unroll
+                        for (int i = 2 * j; i < 2 * j + 2; i++) {
+                            f2 t = mul2(add2(pack2(hi[2 * i], hi[2 * i + 1]), pack2(lo[2 * i], lo[2 * i + 1])), ff0);
+                            if (mins) {
+                                t = fma2(pack2(mn[2 * i], mn[2 * i + 1]), ff1, t);
+                            }
+                            sum[i] = fma2(t, sc[i & 1], sum[i]);
+                        }
+                    }
+                }
+                if (!ok) {
+                    break;
+                }
+                if (u + 1 == v_end) {  // the end of a range
+                    const int slot = v - range * (RANGES / p.ksplit);
+#pragma unroll
+                    for (int i = 0; i < C / 2; i++) {
+                        if (p.ksplit > 1) {
+                            float a, b;
+                            unpack2(sum[i], a, b);
+                            const uint32_t at = base + (uint32_t)(((slot * NT + c0 + 2 * i) * 128 + lane_row) * 4);
+                            asm volatile("st.shared.f32 [%0], %1;" ::"r"(at), "f"(a) : "memory");
+                            asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + 512u), "f"(b) : "memory");
+                        } else {
+                            total[i] = add2(total[i], sum[i]);
+                        }
+                        sum[i] = 0;
+                    }
+                    do {
+                        v++;
+                        v_end = (int)((int64_t)(v + 1) * p.units / RANGES);
+                    } while (v < RANGES - 1 && v_end <= u + 1);
+                }
+            }
+            if (!ok || p.ksplit > 1) {
+                break;  // (one tile per cluster)
+            }
+            int ft0;
+            const int w = weight_of(ft, ft0);
+            const int64_t row = (int64_t)(ft - ft0) * 128 + lane_row, n = mm::pick(p.n, w);
+            if (row < n) {
+                const float b = w == 0 && p.bias != nullptr ? __ldg(p.bias + row) : 0.0f;
+                float* at = mm::pick(p.y, w) + (int64_t)c0 * n + row;
+#pragma unroll
+                for (int i = 0; i < C; i++, at += n) {
+                    float v[2];
+                    unpack2(total[i / 2], v[0], v[1]);
+                    if (c0 + i < p.m) {
+                        *at = v[i % 2] + b;
+                    }
+                }
+            }
+        }
+    }
+
+    // ---- exit -----------------------------------------------------------------------------------------------------------------------
+    __syncwarp();
+    tc::fence_before_sync();
+    __syncthreads();
+    if (*abort_flag != 0) {
+        for (int i = 0; i < 1000; i++) {
+            __nanosleep(1000);  // copies that may still be in flight land long before this millisecond is over
+        }
+    }
+    __syncthreads();
+    if (p.ksplit > 1) {
+        mm::cluster_sync();  // the sums of all ranges are there
+        if (*abort_flag == 0) {
+            int ft0;
+            const int w = weight_of(cluster_id, ft0);
+            const int64_t f0 = (int64_t)(cluster_id - ft0) * 128, n = mm::pick(p.n, w);
+            float* const y = mm::pick(p.y, w);
+            const int per = RANGES / p.ksplit;
+            // columns range, range + ksplit, ... of the tile; a thread adds up one row's eight ranges
+            for (int i = threadIdx.x; i < NT / p.ksplit * 128; i += THREADS) {
+                const int col = range + (i >> 7) * p.ksplit, row = i & 127;
+                float e[RANGES];
+#pragma unroll
+                for (int g = 0; g < RANGES; g++) {
+                    const bool there = (int64_t)g * p.units / RANGES < (int64_t)(g + 1) * p.units / RANGES;  // (a range without units has no sums)
+                    const uint32_t from = mm::map_rank(base + (uint32_t)(((g % per * NT + col) * 128 + row) * 4), (uint32_t)(g / per));
+                    e[g] = 0.0f;
+                    if (there) {
+                        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(e[g]) : "r"(from));
+                    }
+                }
+                float t = 0.0f;
+#pragma unroll
+                for (int g = 0; g < RANGES; g++) {
+                    t += e[g];
+                }
+                if (f0 + row < n && col < p.m) {
+                    y[(int64_t)col * n + f0 + row] = t + (w == 0 && p.bias != nullptr ? __ldg(p.bias + f0 + row) : 0.0f);
+                }
+            }
+        }
+        __syncthreads();
+        mm::cluster_sync();  // no thread block ends while others read its sums
+    }
+    if (warp == 1) {
+        tc::fence_after_sync();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+    }
+}
+
+}  // namespace rows
+}  // namespace jq
