@@ -45,8 +45,6 @@ using mm::unpack2;
 constexpr int NT = 16, N = 32;       // rows of x, columns
 constexpr int RANGES = 8;
 constexpr int MAX_WEIGHTS = 3;
-constexpr int GROUPS = 2, FOLD = 8, THREADS = (4 + FOLD + 4 * GROUPS) * 32;
-constexpr int C = NT / (FOLD / 4);   // columns (rows of x) of a fold warp
 constexpr int STEP = N * 32;         // bytes of 16 k of the image: [8 k][8 columns][8 rows of 16 bytes]
 constexpr int IMAGE = 17 * STEP;     // of a unit: 256 k, then the sums of x over its runs of 32, twice, as 16 more k
 constexpr int MAX_RAW = 6, MAX_IMG = 6, OPERANDS = 3, MAX_ACC = 4, FACTORS = 8;
@@ -113,6 +111,9 @@ __device__ __forceinline__ bool wait_all(volatile int* abort_flag, const Args& p
     i = 0;
     return ((__all_sync(0xffffffffu, ready[i++]) || mm::wait_warp(phases.bar, phases.parity, abort_flag, p, phases.code)) && ...);
 }
+
+__device__ __forceinline__ void ld(float (&r)[8], uint32_t addr) { mm::ld_tmem8(r, addr); }
+__device__ __forceinline__ void ld(float (&r)[16], uint32_t addr) { mm::ld_tmem16(r, addr); }
 
 // ---- the formats -------------------------------------------------------------------------------------------------------------------
 // PARTS: operand values per weight; MINS: the sums of x have a part (what is the same for 32 weights, the middle of the quants and the min: 8 more columns
@@ -341,15 +342,19 @@ struct Shape {
     static constexpr int UNIT_Q = 128 * F::ROW, UNIT_A = 128 * F::AUX, UNIT = UNIT_Q + UNIT_A;
     static constexpr int A_COLS = 128 + (F::MINS ? 8 : 0);
     static constexpr int ACC = F::MINS ? 2 : 4, ACC_COLS = ACC * (N + (F::MINS ? NT : 0));  // accumulators
+    static_assert(F::ACCS / F::HALVES == 1 || ACC == 2, "");
     static_assert(ACC_COLS + OPERANDS * A_COLS <= 512, "tensor memory");
+    static constexpr int GROUPS = 2, FOLD = F::HALVES == 1 ? 8 : 4, THREADS = (4 + FOLD + 4 * GROUPS) * 32;  // warps that make weights (groups of four), that add up
+    static constexpr int C = NT / (FOLD / 4);  // columns (rows of x) of a fold warp
 };
 constexpr int TAIL = FACTORS * 128 * 8 + 4 * 1024 + 1024;  // factors, the fold warps' scales of x, barriers
 constexpr int part_bytes(int ksplit) { return ksplit > 1 ? RANGES / ksplit * NT * 512 : 0; }
 
 template <int TYPE>
-__global__ void __launch_bounds__(THREADS, 1) rows_kernel(const __grid_constant__ Args p) {
+__global__ void __launch_bounds__((Shape<TYPE>::THREADS), 1) rows_kernel(const __grid_constant__ Args p) {
     using F = Rw<TYPE>;
     using S = Shape<TYPE>;
+    constexpr int GROUPS = S::GROUPS, FOLD = S::FOLD, THREADS = S::THREADS, C = S::C;
     extern __shared__ uint8_t smem_unaligned[];
     const uint32_t base = (tc::smem_u32(smem_unaligned) + 127u) & ~127u;  // sums of this thread block's ranges (ksplit > 1), then the rings
     const uint32_t img0 = base + (uint32_t)(p.ksplit > 1 ? RANGES / p.ksplit * NT * 512 : 0), raw0 = img0 + (uint32_t)(p.img * IMAGE), fac0 = raw0 + (uint32_t)(p.raw * S::UNIT);
@@ -458,65 +463,72 @@ __global__ void __launch_bounds__(THREADS, 1) rows_kernel(const __grid_constant_
             }
         }
     } else if (warp == 1) {
-        // ---- MMAs: an operand's in one go (an election between them costs as much as several) --------------------------------------------
-        int a = 0, s = 0, buf = 0;
+        // ---- MMAs: an operand's in one go (an election between them costs as much as several). What the next operand needs is asked for before they are
+        // issued: an answer takes 200 clocks, with those of all polls together, and by then it is mostly yes.
+        constexpr int BUFS = F::ACCS / F::HALVES, STEPS = 16 / F::HALVES;  // accumulators and steps of 16 k of an operand
+        const int turns = (p.ftiles - cluster_id + clusters - 1) / clusters * (u1 - u0) * F::HALVES;
+        int a = 0, s = 0, buf = 0, half = 0;
         uint32_t pa = 0, ps = 0, pb = 1;
-        for (int ft = cluster_id; ft < p.ftiles && ok; ft += clusters) {
-            for (int u = u0; u < u1 && ok; u++) {
-                const uint32_t img = desc(img0 + (uint32_t)(s * IMAGE));
+        bool ready = false;
+        for (int t = 0; t < turns; t++) {
+            uint32_t d[BUFS], d_bar[BUFS], dm = 0;
+            Phase free[BUFS];
 #pragma unroll
-                for (int half = 0; half < F::HALVES; half++) {
-                    constexpr int BUFS = F::ACCS / F::HALVES, STEPS = 16 / F::HALVES;  // accumulators and steps of 16 k of an operand
-                    uint32_t d[BUFS], d_bar[BUFS], dm = 0;
-                    Phase free[BUFS];
-#pragma unroll
-                    for (int i = 0; i < BUFS; i++) {
-                        d[i] = tmem + (uint32_t)(buf * N);
-                        dm = tmem_m + (uint32_t)(buf * NT);
-                        d_bar[i] = acc_full + 8 * buf;
-                        free[i] = Phase{acc_free + 8 * buf, pb, 5};
-                        if (++buf == S::ACC) {
-                            buf = 0;
-                            pb ^= 1;
-                        }
-                    }
-                    if (!(ok = wait_all(abort_flag, p, Phase{img_full + 8 * s, ps, 3}, Phase{full_a + 8 * a, pa, 2}, free[0], free[BUFS - 1]))) {
-                        break;
-                    }
-                    tc::fence_after_sync();
-                    const uint32_t ta = tmem_a + (uint32_t)(a * S::A_COLS), bd = img + (uint32_t)(half * STEPS * (STEP >> 4)), a_bar = free_a + 8 * a, s_bar = img_free + 8 * s;
-                    if (elect_one()) {
-#pragma unroll
-                        for (int i = 0; i < STEPS; i++) {
-                            const int b = i / (STEPS / BUFS);
-                            mma(d[b], ta + 8 * i, bd + i * (STEP >> 4), ID_N, i % (STEPS / BUFS) == 0 ? 0u : 1u);  // hi x (hi | lo)
-                            if constexpr (F::PARTS == 2) {
-                                mma(d[b] + NT, ta + 64 + 8 * i, bd + i * (STEP >> 4), ID_NT, 1u);  // lo x hi, beside the other small products
-                            }
-                            if (F::MINS && half == F::HALVES - 1 && i == STEPS - 1) {
-                                mma(dm, ta + 128, img + 16 * (STEP >> 4) + (NT * 16 >> 4), ID_NT, 0u);
-                                mma(dm, ta + 128, img + 16 * (STEP >> 4), ID_NT, 1u);
-                            }
-                            if ((i + 1) % (STEPS / BUFS) == 0) {
-                                tc::umma_commit(d_bar[b]);
-                            }
-                        }
-                        tc::umma_commit(a_bar);
-                        if (half == F::HALVES - 1) {
-                            tc::umma_commit(s_bar);
-                        }
-                    }
-                    __syncwarp();
-                    if (++a == OPERANDS) {
-                        a = 0;
-                        pa ^= 1;
-                    }
-                }
-                if (++s == p.img) {
-                    s = 0;
-                    ps ^= 1;
+            for (int i = 0; i < BUFS; i++) {
+                d[i] = tmem + (uint32_t)(buf * N);
+                dm = tmem_m + (uint32_t)(buf * NT);
+                d_bar[i] = acc_full + 8 * buf;
+                free[i] = Phase{acc_free + 8 * buf, pb, 5};
+                if (++buf == S::ACC) {
+                    buf = 0;
+                    pb ^= 1;
                 }
             }
+            if (!__all_sync(0xffffffffu, ready) &&
+                !(ok = wait_all(abort_flag, p, Phase{full_a + 8 * a, pa, 2}, Phase{img_full + 8 * s, ps, 3}, free[0], free[BUFS - 1]))) {
+                break;
+            }
+            tc::fence_after_sync();
+            const uint32_t img = desc(img0 + (uint32_t)(s * IMAGE)), ta = tmem_a + (uint32_t)(a * S::A_COLS), bd = img + (uint32_t)(half * STEPS * (STEP >> 4));
+            const uint32_t a_bar = free_a + 8 * a, s_bar = img_free + 8 * s;
+            const bool last = F::HALVES == 1 || half == 1;
+            if (++a == OPERANDS) {
+                a = 0;
+                pa ^= 1;
+            }
+            if (last && ++s == p.img) {
+                s = 0;
+                ps ^= 1;
+            }
+            half = last ? 0 : 1;
+            ready = tc::mbar_test(full_a + 8 * a, pa);
+            ready = tc::mbar_test(img_full + 8 * s, ps) && ready;
+            ready = tc::mbar_test(acc_free + 8 * buf, pb) && ready;
+            if constexpr (BUFS == 2) {  // (all of them)
+                ready = tc::mbar_test(acc_free + 8 * (buf + 1), pb) && ready;
+            }
+            if (elect_one()) {
+#pragma unroll
+                for (int i = 0; i < STEPS; i++) {
+                    const int b = i / (STEPS / BUFS);
+                    mma(d[b], ta + 8 * i, bd + i * (STEP >> 4), ID_N, i % (STEPS / BUFS) == 0 ? 0u : 1u);  // hi x (hi | lo)
+                    if constexpr (F::PARTS == 2) {
+                        mma(d[b] + NT, ta + 64 + 8 * i, bd + i * (STEP >> 4), ID_NT, 1u);  // lo x hi, beside the other small products
+                    }
+                    if (F::MINS && i == STEPS - 1 && last) {
+                        mma(dm, ta + 128, img + 16 * (STEP >> 4) + (NT * 16 >> 4), ID_NT, 0u);
+                        mma(dm, ta + 128, img + 16 * (STEP >> 4), ID_NT, 1u);
+                    }
+                    if ((i + 1) % (STEPS / BUFS) == 0) {
+                        tc::umma_commit(d_bar[b]);
+                    }
+                }
+                tc::umma_commit(a_bar);
+                if (last) {
+                    tc::umma_commit(s_bar);
+                }
+            }
+            __syncwarp();
         }
     } else if (warp >= 4 + FOLD) {
         // ---- weights -------------------------------------------------------------------------------------------------------------------
@@ -618,11 +630,11 @@ __global__ void __launch_bounds__(THREADS, 1) rows_kernel(const __grid_constant_
                     }
                     tc::fence_after_sync();
                     float hi[C], lo[C], mn[C];
-                    mm::ld_tmem8(hi, tmem + lanes + (uint32_t)(buf * N + c0));
-                    mm::ld_tmem8(lo, tmem + lanes + (uint32_t)(buf * N + NT + c0));
+                    ld(hi, tmem + lanes + (uint32_t)(buf * N + c0));
+                    ld(lo, tmem + lanes + (uint32_t)(buf * N + NT + c0));
                     const bool mins = F::MINS && acc == F::ACCS - 1;
                     if (mins) {
-                        mm::ld_tmem8(mn, tmem_m + lanes + (uint32_t)(buf * NT + c0));
+                        ld(mn, tmem_m + lanes + (uint32_t)(buf * NT + c0));
                     }
                     mm::ld_tmem_done();
                     tc::fence_before_sync();

@@ -11,8 +11,8 @@ namespace rows {
 template <int TYPE>
 size_t configure(Args& a) {
     using S = Shape<TYPE>;
-    const int room = 227 * 1024 - 128 - TAIL - part_bytes(a.ksplit), step = Rw<TYPE>::HALVES == 1 ? GROUPS : 1;
-    a.raw = 2;
+    const int room = 227 * 1024 - 128 - TAIL - part_bytes(a.ksplit), step = Rw<TYPE>::HALVES == 1 ? S::GROUPS : 1;
+    a.raw = step == 1 ? 2 : step;
     a.img = 2;
     while (a.raw + step <= MAX_RAW && (a.raw + step) * S::UNIT + 3 * IMAGE <= room) {
         a.raw += step;
@@ -35,7 +35,7 @@ int launch_format(Args& a, int ctas, cudaStream_t s) {
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas);
-    cfg.blockDim = dim3(THREADS);
+    cfg.blockDim = dim3(Shape<TYPE>::THREADS);
     cfg.dynamicSmemBytes = configure<TYPE>(a);
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
