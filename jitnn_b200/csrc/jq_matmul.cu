@@ -130,7 +130,7 @@ static bool configure(int type, bool fp32, bool bwd, int nt, int ksplit, Args& a
     const Facts f = facts(type, fp32, bwd, plan.nmax);
     // sums of a CTA's virtual ranges (instances for 16 rows of x), kept apart from the rings, which are still in use
     a.part_bytes = fp32 && !bwd && nt <= 16 && ksplit > 1 ? VIRTUAL / ksplit * nt * 512 : 0;
-    const int at = a_bytes(bwd), bt = f.b_tiles * tile_bytes(fp32, nt), rb = unit_bytes(type), room = 227 * 1024 - 1024 - TAIL_BYTES - a.part_bytes;
+    const int at = a_bytes(bwd), bt = f.b_tiles * tile_bytes(fp32, nt), rb = unit_bytes(type), tail = TAIL_BYTES + f.scales, room = 227 * 1024 - 1024 - tail - a.part_bytes;
     // tensor memory: as many accumulators as fit beside the groups' operands; operands behind them
     a.cols = f.columns * nt;
     a.bufs = fp32 ? MAX_BUFS : 2;
@@ -170,7 +170,7 @@ static bool configure(int type, bool fp32, bool bwd, int nt, int ksplit, Args& a
     while (a.tmem < a.bufs * a.cols + (bwd ? 0 : a.sa * f.a_cols)) {
         a.tmem *= 2;
     }
-    plan.smem = (size_t)(room - left) + a.part_bytes + TAIL_BYTES + 1024;
+    plan.smem = (size_t)(room - left) + a.part_bytes + tail + 1024;
     return true;
 }
 

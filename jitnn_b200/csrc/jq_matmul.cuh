@@ -66,6 +66,8 @@ struct Shape {
     // 4e-7 to 2.4e-6.
     static constexpr int ACC = BWD ? 1 : (TYPE == JQ_TYPE_Q4_K && JOINED && TURN == 4 ? 4 : 2), ACCS = CHUNKS / ACC;
     static constexpr bool PAIRED = FP32 && !BWD && !JOINED;
+    static constexpr int AHEAD = BWD && !JOINED ? 8 : 1;                // units whose scales of x the fold fetches at a time
+    static constexpr int SCALES = 8 * 2 * 64 * 4 * AHEAD;               // bytes for them
     static constexpr int OPERANDS = PAIRED ? 2 / TURN + 2 : GROUPS;     // to have at least
     static_assert(!FP32 || PAIRED || TURN % ACC == 0, "");
 };
@@ -295,7 +297,7 @@ __host__ __device__ constexpr int raw_bytes() {
 }
 __host__ __device__ inline int a_bytes(bool bwd) { return bwd ? 2 * A_TILE : 0; }  // the forward product's weights go to tensor memory
 __host__ __device__ inline int tile_bytes(bool fp32, int nt) { return (fp32 ? 2 * nt : nt) * 128; }
-constexpr int TAIL_BYTES = FACTORS * 128 * 4 + 8 * 2 * 64 * 4 + 1024;  // row factors, the fold warps' scales, barriers
+constexpr int TAIL_BYTES = FACTORS * 128 * 4 + 1024;  // row factors, barriers
 
 // NMAX: largest tile of rows of x an FP32 instance adds up in registers.
 template <int TYPE, bool FP32, bool BWD, int NMAX>
@@ -316,7 +318,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
     const uint32_t tile_st = (uint32_t)tile_bytes(FP32, nt), a_st = (uint32_t)a_bytes(BWD), b_st = (uint32_t)BT * tile_st;
     const uint32_t a0 = base + (uint32_t)p.part_bytes, b0 = a0 + (uint32_t)SA * a_st, raw0 = b0 + (uint32_t)SB * b_st;
     const uint32_t fac0 = raw0 + (uint32_t)R * raw_bytes<TYPE>();
-    const uint32_t scl0 = fac0 + FACTORS * 128 * 4, full_a = scl0 + 8 * 2 * 64 * 4, free_a = full_a + 8 * MAX_A, full_b = free_a + 8 * MAX_A, free_b = full_b + 8 * MAX_B;
+    const uint32_t scl0 = fac0 + FACTORS * 128 * 4, full_a = scl0 + W::SCALES, free_a = full_a + 8 * MAX_A, full_b = free_a + 8 * MAX_A, free_b = full_b + 8 * MAX_B;
     const uint32_t raw_full = free_b + 8 * MAX_B, raw_read = raw_full + 8 * MAX_RAW;
     const uint32_t acc_full = raw_read + 8 * MAX_RAW, acc_empty = acc_full + 8 * MAX_BUFS, fac_full = acc_empty + 8 * MAX_BUFS, max_full = fac_full + 8 * FACTORS, slot_s = max_full + 64;
     uint8_t* const generic = smem_unaligned + (slot_s - tc::smem_u32(smem_unaligned));
@@ -928,29 +930,34 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                     }
                     slot = virt - range * (VIRTUAL / p.ksplit);
                 }
-                // the scales of a unit's columns: fetched by the lanes a unit ahead, read back as broadcasts
-                const uint32_t scl = scl0 + (uint32_t)(warp - 3 - 4 * G) * (8u * C32);
-                const float* xs = p.xscale + (int64_t)u0 * p.xstride + t0 + c0;
-                float next[(C + 31) / 32];
+                // The scales of a unit's columns: fetched by the lanes AHEAD units at a time, read back as broadcasts. (A load takes up to 2000 clocks while the
+                // weights stream: one unit ahead, the backward form's units waited for it: Q4_K 32000 x 4096, 128 rows 147 us, now 138; 4096 x 4096
+                // 28.5 and 27.2. The forward forms do not wait for it.)
+                constexpr int AHEAD = W::AHEAD, NEXT = (C * AHEAD + 31) / 32;
+                const uint32_t scl = scl0 + (uint32_t)(warp - 3 - 4 * G) * (8u * C32 * AHEAD);
+                float next[NEXT];
+                auto fetch = [&](int u) {
 #pragma unroll
-                for (int i = 0; i < (C + 31) / 32; i++) {
-                    next[i] = lane + 32 * i < cols ? __ldg(xs + lane + 32 * i) : 0.0f;
-                }
+                    for (int i = 0; i < NEXT; i++) {
+                        const int on = AHEAD > 1 ? i : 0, col = AHEAD > 1 ? lane : lane + 32 * i;  // (AHEAD > 1: 32 columns)
+                        next[i] = col < cols && u + on < u1 ? __ldg(p.xscale + (int64_t)(u + on) * p.xstride + t0 + c0 + col) : 0.0f;
+                    }
+                };
+                fetch(u0);
                 for (int u = u0; u < u1; u++, chunk++) {
-                    const uint32_t sb = scl + (uint32_t)(chunk & 1) * (4u * C32);
-                    __syncwarp();
+                    const int step = (u - u0) % AHEAD, block = (u - u0) / AHEAD & 1;
+                    const uint32_t sb = scl + (uint32_t)((block * AHEAD + step) * C32) * 4u;
+                    if (step == 0) {
+                        __syncwarp();
 #pragma unroll
-                    for (int i = 0; i < (C + 31) / 32; i++) {
-                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(sb + (uint32_t)(lane + 32 * i) * 4u), "f"(next[i]) : "memory");
-                    }
-                    xs += p.xstride;
-                    if (u + 1 < u1) {
-#pragma unroll
-                        for (int i = 0; i < (C + 31) / 32; i++) {
-                            next[i] = lane + 32 * i < cols ? __ldg(xs + lane + 32 * i) : 0.0f;
+                        for (int i = 0; i < NEXT; i++) {
+                            asm volatile("st.shared.f32 [%0], %1;" ::"r"(sb + (uint32_t)(lane + 32 * i) * 4u), "f"(next[i]) : "memory");
                         }
+                        if (u + AHEAD < u1) {
+                            fetch(u + AHEAD);
+                        }
+                        __syncwarp();
                     }
-                    __syncwarp();
                     if (!(ok = wait_warp<true>(fac_full + 8 * (chunk & (FACTORS - 1)), (uint32_t)(chunk / FACTORS) & 1u, abort_flag, p, 6))) {
                         break;
                     }

@@ -17,13 +17,13 @@ struct Plan {
 // What the host has to know of an instance's Shape.
 struct Facts {
     int groups, turn, turns, a_cols, b_tiles, columns;  // columns: accumulator columns per row of x
-    int operands;
+    int operands, scales;
     bool owned, ext, paired;
 };
 template <int TYPE, bool FP32, bool BWD, int NMAX>
 constexpr Facts facts_of() {
     using W = Shape<TYPE, FP32, BWD, NMAX>;
-    return Facts{W::GROUPS, W::TURN, W::TURNS, W::A_COLS, W::B_TILES, W::JOINED ? 2 : 1, W::OPERANDS, W::OWNED, W::EXT, W::PAIRED};
+    return Facts{W::GROUPS, W::TURN, W::TURNS, W::A_COLS, W::B_TILES, W::JOINED ? 2 : 1, W::OPERANDS, W::SCALES, W::OWNED, W::EXT, W::PAIRED};
 }
 template <int TYPE>
 Facts facts_format(bool fp32, bool bwd, int nmax) {
