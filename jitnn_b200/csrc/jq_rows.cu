@@ -1,4 +1,4 @@
-// Host side of the rows kernel (jq_rows.cuh): the image of x, the choice of ranges, the launches.
+// Host side of the rows kernel (jq_rows.cuh): the image of x, the choice of launches.
 #include "jq_rows_launch.cuh"
 
 namespace jq {
@@ -78,32 +78,59 @@ __global__ void __launch_bounds__(128) image_kernel(const float* __restrict__ x,
 // 4 or 8).
 static int clusters_of(int ks) { return ks == 1 ? 148 : (ks == 2 ? 74 : (ks == 4 ? 33 : 15)); }
 
-// Thread blocks that share a tile's ranges of k.
-static int ranges_for(int ftiles, int units, double unit_ns) {
+// What a unit takes a thread block in nanoseconds, measured on 32000 x 4096.
+static double unit_ns(int type) { return type == JQ_TYPE_Q4_K ? 630.0 : (type == JQ_TYPE_Q5_K ? 940.0 : (type == JQ_TYPE_Q4_0 ? 1040.0 : 1170.0)); }
+
+// A product's tiles in up to three launches, each with its own number of thread blocks per tile: whole waves first, then what is left, which alone would
+// leave most of the chip idle for a whole contraction, with its contraction split over clusters (57344 x 8192: 448 tiles are three waves and four
+// tiles: 85.5 us in one launch, 71.7 in two). The launch behind starts where SMs become free; GAP_NS is its own start.
+constexpr int MAX_PARTS = 3;
+constexpr double GAP_NS = 2500.0;
+struct Parts {
+    int count;
+    int tiles[MAX_PARTS], ksplit[MAX_PARTS];
+};
+static double cut(int tiles, int units, double unit, int most, Parts& out) {
     double best = 1e30;
-    int best_ks = 1;
-    for (int ks = 1; ks <= 8; ks *= 2) {
-        const int slots = clusters_of(ks), waves = (ftiles + slots - 1) / slots;
-        if (ks > 1 && (units < 2 * ks || waves > 1)) {
-            break;
+    for (int ks = 1; ks <= 8 && (ks == 1 || units >= 2 * ks); ks *= 2) {
+        const int slots = clusters_of(ks), waves = (tiles + slots - 1) / slots;
+        auto cost_of = [&](int w) { return w * (((units + ks - 1) / ks) * unit + 1700.0) + (ks > 1 ? 1600.0 : 0.0); };
+        if (ks == 1 || waves == 1) {
+            const double cost = cost_of(waves);
+            if (cost < best) {
+                best = cost;
+                out.count = 1;
+                out.tiles[0] = tiles;
+                out.ksplit[0] = ks;
+            }
         }
-        const double cost = waves * (((units + ks - 1) / ks) * unit_ns + 1700.0) + (ks > 1 ? 1600.0 : 0.0);
-        if (cost < best) {
-            best = cost;
-            best_ks = ks;
+        const int whole = ks == 1 ? tiles / slots : 1, front = whole * slots;
+        if (most > 1 && front > 0 && front < tiles) {
+            Parts rest;
+            const double cost = cost_of(whole) + GAP_NS + cut(tiles - front, units, unit, most - 1, rest);
+            if (cost < best) {
+                best = cost;
+                out.count = 1 + rest.count;
+                out.tiles[0] = front;
+                out.ksplit[0] = ks;
+                for (int i = 0; i < rest.count; i++) {
+                    out.tiles[1 + i] = rest.tiles[i];
+                    out.ksplit[1 + i] = rest.ksplit[i];
+                }
+            }
         }
     }
-    return best_ks;
+    return best;
 }
 
-static int launch_any(int type, Args& a, int ctas, cudaStream_t s) {
+static int launch_any(int type, Args& a, int ctas, bool after, cudaStream_t s) {
     switch (type) {
-        case JQ_TYPE_Q4_K: return launch_q4_k(a, ctas, s);
-        case JQ_TYPE_Q5_K: return launch_q5_k(a, ctas, s);
-        case JQ_TYPE_Q6_K: return launch_q6_k(a, ctas, s);
-        case JQ_TYPE_Q8_0: return launch_q8_0(a, ctas, s);
-        case JQ_TYPE_Q4_0: return launch_q4_0(a, ctas, s);
-        case JQ_TYPE_Q4_1: return launch_q4_1(a, ctas, s);
+        case JQ_TYPE_Q4_K: return launch_q4_k(a, ctas, after, s);
+        case JQ_TYPE_Q5_K: return launch_q5_k(a, ctas, after, s);
+        case JQ_TYPE_Q6_K: return launch_q6_k(a, ctas, after, s);
+        case JQ_TYPE_Q8_0: return launch_q8_0(a, ctas, after, s);
+        case JQ_TYPE_Q4_0: return launch_q4_0(a, ctas, after, s);
+        case JQ_TYPE_Q4_1: return launch_q4_1(a, ctas, after, s);
         default: return fail(JQ_ERR_UNSUPPORTED, "rows product: type %d has no kernel", type);
     }
 }
@@ -168,12 +195,18 @@ int launch_rows(const View* vs, int count, const float* x, const float* up, int 
         a.scales = scales;
         a.bias = i == 0 ? bias : nullptr;
         a.units = units;
-        a.ftiles = end;
         a.m = m;
-        a.ksplit = ranges_for(end, units, vs[i].type == JQ_TYPE_Q4_K ? 450.0 : 700.0);
         a.status = status;
         a.wait_clocks = (long long)g_opt_wait_limit_us.load(std::memory_order_relaxed) * 2000;  // about 2 GHz
-        rc = launch_any(vs[i].type, a, a.ksplit > 1 ? end * a.ksplit : (end < 148 ? end : 148), s);
+        Parts parts;
+        cut(end, units, unit_ns(vs[i].type), MAX_PARTS, parts);
+        for (int c = 0, at = 0; c < parts.count && rc == JQ_OK; c++) {
+            a.first_ft = at;
+            a.ftiles = at += parts.tiles[c];
+            a.ksplit = parts.ksplit[c];
+            a.followed = c + 1 < parts.count;
+            rc = launch_any(vs[i].type, a, a.ksplit > 1 ? parts.tiles[c] * a.ksplit : (parts.tiles[c] < 148 ? parts.tiles[c] : 148), c > 0, s);
+        }
     }
     return rc;
 }

@@ -58,7 +58,9 @@ struct Args {
     const uint8_t* image;     // [units][IMAGE]
     const float* scales;      // [units][NT]
     const float* bias;        // of the first weight, or null
-    int units, ftiles, m;
+    int units, m;
+    int first_ft, ftiles;     // this launch's tiles: the first, and the one behind the last
+    int followed;             // another launch of the same product is behind
     int ksplit;               // thread blocks that share a tile's ranges
     int raw, img;             // ring depths
     int* status;
@@ -350,7 +352,10 @@ struct Shape {
 constexpr int TAIL = FACTORS * 128 * 8 + 4 * 1024 + 1024;  // factors, the fold warps' scales of x, barriers
 constexpr int part_bytes(int ksplit) { return ksplit > 1 ? RANGES / ksplit * NT * 512 : 0; }
 
-template <int TYPE>
+// AFTER: another launch of the same product is in front. A product may be cut by tiles into several launches, which read and write nothing of each
+// other's: the one behind starts as SMs become free, without waiting for the one in front, once that one knows that x's image is complete. It ends
+// after it, though, so whoever waits for the last waits for all.
+template <int TYPE, bool AFTER>
 __global__ void __launch_bounds__((Shape<TYPE>::THREADS), 1) rows_kernel(const __grid_constant__ Args p) {
     using F = Rw<TYPE>;
     using S = Shape<TYPE>;
@@ -404,7 +409,9 @@ __global__ void __launch_bounds__((Shape<TYPE>::THREADS), 1) rows_kernel(const _
         mm::cluster_sync();
     }
     tc::fence_after_sync();
-    asm volatile("griddepcontrol.launch_dependents;");
+    if (AFTER || !p.followed) {
+        asm volatile("griddepcontrol.launch_dependents;");
+    }
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     const uint32_t tmem_m = tmem + S::ACC * N, tmem_a = tmem + S::ACC_COLS;
 
@@ -419,7 +426,7 @@ __global__ void __launch_bounds__((Shape<TYPE>::THREADS), 1) rows_kernel(const _
         if (lane == 0) {
             int r = 0;
             uint32_t ph = 1;
-            for (int ft = cluster_id; ft < p.ftiles && ok; ft += clusters) {
+            for (int ft = p.first_ft + cluster_id; ft < p.ftiles && ok; ft += clusters) {
                 int ft0;
                 const int w = weight_of(ft, ft0);
                 const int64_t first = (int64_t)(ft - ft0) * p.units;
@@ -445,10 +452,13 @@ __global__ void __launch_bounds__((Shape<TYPE>::THREADS), 1) rows_kernel(const _
     } else if (warp == 2) {
         // ---- the image ---------------------------------------------------------------------------------------------------------------
         if (lane == 0) {
-            asm volatile("griddepcontrol.wait;" ::: "memory");  // the kernel in front writes it
+            if constexpr (!AFTER) {
+                asm volatile("griddepcontrol.wait;" ::: "memory");  // the kernel in front writes it
+                asm volatile("griddepcontrol.launch_dependents;");
+            }
             int s = 0;
             uint32_t ph = 1;
-            for (int ft = cluster_id; ft < p.ftiles && ok; ft += clusters) {
+            for (int ft = p.first_ft + cluster_id; ft < p.ftiles && ok; ft += clusters) {
                 for (int u = u0; u < u1; u++) {
                     if (!(ok = mm::wait<true>(img_free + 8 * s, ph, abort_flag, p, 3))) {
                         break;
@@ -466,7 +476,7 @@ __global__ void __launch_bounds__((Shape<TYPE>::THREADS), 1) rows_kernel(const _
         // ---- MMAs: an operand's in one go (an election between them costs as much as several). What the next operand needs is asked for before they are
         // issued: an answer takes 200 clocks, with those of all polls together, and by then it is mostly yes.
         constexpr int BUFS = F::ACCS / F::HALVES, STEPS = 16 / F::HALVES;  // accumulators and steps of 16 k of an operand
-        const int turns = (p.ftiles - cluster_id + clusters - 1) / clusters * (u1 - u0) * F::HALVES;
+        const int turns = (p.ftiles - p.first_ft - cluster_id + clusters - 1) / clusters * (u1 - u0) * F::HALVES;
         int a = 0, s = 0, buf = 0, half = 0;
         uint32_t pa = 0, ps = 0, pb = 1;
         bool ready = false;
@@ -534,7 +544,7 @@ __global__ void __launch_bounds__((Shape<TYPE>::THREADS), 1) rows_kernel(const _
         // ---- weights -------------------------------------------------------------------------------------------------------------------
         const int group = (warp - 4 - FOLD) >> 2, row = (warp & 3) * 32 + lane;
         const uint32_t to0 = tmem_a + ((uint32_t)((warp & 3) * 32) << 16);
-        const int units = (p.ftiles - cluster_id + clusters - 1) / clusters * (u1 - u0);
+        const int units = (p.ftiles - p.first_ft - cluster_id + clusters - 1) / clusters * (u1 - u0);
         // One operand per unit: the groups take units in turn, and places in the ring of raw units too (its depth is even), so no group tests a barrier
         // that is a turn of the ring behind. Two: each group makes its half of every unit.
         constexpr bool OWN = F::HALVES == 1;
@@ -569,7 +579,9 @@ __global__ void __launch_bounds__((Shape<TYPE>::THREADS), 1) rows_kernel(const _
         }
     } else if (warp >= 4) {
         // ---- sums ----------------------------------------------------------------------------------------------------------------------
-        asm volatile("griddepcontrol.wait;" ::: "memory");  // x's scales; and y may be read by the kernel in front
+        if constexpr (!AFTER) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");  // x's scales; and y may be read by the kernel in front
+        }
         const int lane_row = (warp & 3) * 32 + lane;
         const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
         const int c0 = (warp - 4) / 4 * C;  // this warp's columns
@@ -588,7 +600,7 @@ __global__ void __launch_bounds__((Shape<TYPE>::THREADS), 1) rows_kernel(const _
         };
         const bool keep = u1 - u0 <= 16;  // (a short contraction's stay for the next tile)
         fetch(u0);
-        for (int ft = cluster_id; ft < p.ftiles && ok; ft += clusters) {
+        for (int ft = p.first_ft + cluster_id; ft < p.ftiles && ok; ft += clusters) {
             f2 sum[C / 2], total[C / 2];
 #pragma unroll
             for (int i = 0; i < C / 2; i++) {
@@ -600,7 +612,7 @@ __global__ void __launch_bounds__((Shape<TYPE>::THREADS), 1) rows_kernel(const _
             }
             int v_end = (int)((int64_t)(v + 1) * p.units / RANGES);
             for (int u = u0; u < u1; u++, chunk++) {
-                if (((u - u0) & 15) == 0 && (!keep || ft == cluster_id)) {
+                if (((u - u0) & 15) == 0 && (!keep || ft == p.first_ft + cluster_id)) {
                     __syncwarp();
 #pragma unroll
                     for (int i = 0; i < NEXT; i++) {
@@ -718,8 +730,8 @@ __global__ void __launch_bounds__((Shape<TYPE>::THREADS), 1) rows_kernel(const _
         mm::cluster_sync();  // the sums of all ranges are there
         if (*abort_flag == 0) {
             int ft0;
-            const int w = weight_of(cluster_id, ft0);
-            const int64_t f0 = (int64_t)(cluster_id - ft0) * 128, n = mm::pick(p.n, w);
+            const int ft = p.first_ft + cluster_id, w = weight_of(ft, ft0);
+            const int64_t f0 = (int64_t)(ft - ft0) * 128, n = mm::pick(p.n, w);
             float* const y = mm::pick(p.y, w);
             const int per = RANGES / p.ksplit;
             // columns range, range + ksplit, ... of the tile; a thread adds up one row's eight ranges
@@ -747,6 +759,9 @@ __global__ void __launch_bounds__((Shape<TYPE>::THREADS), 1) rows_kernel(const _
         }
         __syncthreads();
         mm::cluster_sync();  // no thread block ends while others read its sums
+    }
+    if (AFTER && threadIdx.x == 0) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
     }
     if (warp == 1) {
         tc::fence_after_sync();

@@ -23,9 +23,9 @@ size_t configure(Args& a) {
     return (size_t)(128 + TAIL + part_bytes(a.ksplit) + a.raw * S::UNIT + a.img * IMAGE);
 }
 
-template <int TYPE>
-int launch_format(Args& a, int ctas, cudaStream_t s) {
-    auto kernel = rows_kernel<TYPE>;
+template <int TYPE, bool AFTER>
+int launch_instance(Args& a, int ctas, cudaStream_t s) {
+    auto kernel = rows_kernel<TYPE, AFTER>;
     static std::atomic<uint64_t> configured{0};  // the opt-in for large dynamic shared memory is per device
     int dev = 0;
     JQ_CUDA(cudaGetDevice(&dev));
@@ -52,12 +52,17 @@ int launch_format(Args& a, int ctas, cudaStream_t s) {
     return JQ_OK;
 }
 
-int launch_q4_k(Args& a, int ctas, cudaStream_t s);
-int launch_q5_k(Args& a, int ctas, cudaStream_t s);
-int launch_q6_k(Args& a, int ctas, cudaStream_t s);
-int launch_q8_0(Args& a, int ctas, cudaStream_t s);
-int launch_q4_0(Args& a, int ctas, cudaStream_t s);
-int launch_q4_1(Args& a, int ctas, cudaStream_t s);
+template <int TYPE>
+int launch_format(Args& a, int ctas, bool after, cudaStream_t s) {
+    return after ? launch_instance<TYPE, true>(a, ctas, s) : launch_instance<TYPE, false>(a, ctas, s);
+}
+
+int launch_q4_k(Args& a, int ctas, bool after, cudaStream_t s);
+int launch_q5_k(Args& a, int ctas, bool after, cudaStream_t s);
+int launch_q6_k(Args& a, int ctas, bool after, cudaStream_t s);
+int launch_q8_0(Args& a, int ctas, bool after, cudaStream_t s);
+int launch_q4_0(Args& a, int ctas, bool after, cudaStream_t s);
+int launch_q4_1(Args& a, int ctas, bool after, cudaStream_t s);
 
 }  // namespace rows
 }  // namespace jq
