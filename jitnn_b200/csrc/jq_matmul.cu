@@ -124,13 +124,11 @@ static Facts facts(int type, bool fp32, bool bwd, int nmax) {
 static bool configure(int type, bool fp32, bool bwd, int nt, int ksplit, Args& a, Plan& plan) {
     plan.fp32 = fp32;
     plan.bwd = bwd;
-    plan.nmax = !fp32 ? (nt <= 128 ? 128 : 256) : (nt <= 16 && !bwd ? 16 : (nt <= 32 ? 32 : 128));
+    plan.nmax = !fp32 ? (nt <= 128 ? 128 : 256) : (nt <= 32 ? 32 : 128);
     a.nt = nt;
     a.ksplit = ksplit;
     const Facts f = facts(type, fp32, bwd, plan.nmax);
-    // sums of a CTA's virtual ranges (instances for 16 rows of x), kept apart from the rings, which are still in use
-    a.part_bytes = fp32 && !bwd && nt <= 16 && ksplit > 1 ? VIRTUAL / ksplit * nt * 512 : 0;
-    const int at = a_bytes(bwd), bt = f.b_tiles * tile_bytes(fp32, nt), rb = unit_bytes(type), tail = TAIL_BYTES + f.scales, room = 227 * 1024 - 1024 - tail - a.part_bytes;
+    const int at = a_bytes(bwd), bt = f.b_tiles * tile_bytes(fp32, nt), rb = unit_bytes(type), tail = TAIL_BYTES + f.scales, room = 227 * 1024 - 1024 - tail;
     // tensor memory: as many accumulators as fit beside the groups' operands; operands behind them
     a.cols = f.columns * nt;
     a.bufs = fp32 ? MAX_BUFS : 2;
@@ -170,7 +168,7 @@ static bool configure(int type, bool fp32, bool bwd, int nt, int ksplit, Args& a
     while (a.tmem < a.bufs * a.cols + (bwd ? 0 : a.sa * f.a_cols)) {
         a.tmem *= 2;
     }
-    plan.smem = (size_t)(room - left) + a.part_bytes + tail + 1024;
+    plan.smem = (size_t)(room - left) + tail + 1024;
     return true;
 }
 
@@ -184,7 +182,7 @@ static double unit_ns(int type, bool fp32, bool bwd, int nt) {
         return nt <= 128 ? 950.0 : 350.0 + 4.5 * ((nt + 63) / 64 * 64);  // (a tile of 208 or 240 is no faster than one of 256)
     }
     if (nt <= 32) {
-        return one_part(type) ? (nt <= 16 ? 950.0 : 1270.0) : 1430.0;
+        return one_part(type) ? 1270.0 : 1430.0;
     }
     const double t = one_part(type) ? 1330.0 + 6.5 * nt : 1450.0 + 8.6 * nt;
     return one_part(type) || t > 1960.0 ? t : 1960.0;
@@ -201,7 +199,7 @@ static double choose(int type, bool fp32, bool bwd, int64_t ftiles, int units, i
     int last_nt = 0;
     for (int tt = (m + nmax - 1) / nmax; tt <= (m + nmax - 1) / nmax + 6; tt++) {
         const int nt = ((m + tt - 1) / tt + 15) / 16 * 16;
-        if (nt == last_nt) {
+        if (nt == last_nt || (fp32 && !bwd && nt <= 16)) {  // (16 rows of x are the rows kernel's)
             continue;
         }
         last_nt = nt;
@@ -239,9 +237,8 @@ static double choose(int type, bool fp32, bool bwd, int64_t ftiles, int units, i
 }
 
 // A product may be cut by features into up to three launches, each with its own tiles: whole waves first, then what is left, which alone would
-// leave most of the chip idle for a whole contraction, with its contraction split over clusters. (57344 x 8192, 16 rows: 448 tiles are three
-// waves and four tiles: 107.4 us in one launch, 92.2 in two. Q4_K 11008 x 4096, 200 rows: 63.3 and 56.5; backward 4096 x 11008, 128 rows: 67.9
-// and 57.9.) The launch behind waits for the one in front, fills and drains: GAP_NS, measured at 5 to 7 us. Finding the cut takes 10 to 35 us.
+// leave most of the chip idle for a whole contraction, with its contraction split over clusters. (Q4_K 11008 x 4096, 200 rows: 63.3 us in one launch,
+// 56.5 in two; backward 4096 x 11008, 128 rows: 67.9 and 57.9.) The launch behind waits for the one in front, fills and drains: GAP_NS, measured at 5 to 7 us. Finding the cut takes 10 to 35 us.
 constexpr int MAX_PARTS = 3;
 constexpr double GAP_NS = 7000.0;
 struct Part {
@@ -456,9 +453,9 @@ int launch_matmul_f32_multi(const View* vs, int count, const float* x, int64_t m
     return mm::product_f32(vs, count, false, x, nullptr, m, nullptr, ys, s);
 }
 
-// More than 16 rows of x always: the weight is read once for all of them. Up to 16 rows take the same time as one (Q4_K 32000 x 4096: 32 us, Q6_K
-// 45, the others 44, Q4_K 4096 x 4096 12), so the line lies where the decode kernels need another pass: Q4_K and Q5_K take up to eight rows in
-// one (25 us), Q6_K four (34), the 32-element formats two (24 and 16). It must not depend on the number of output rows, and neither do
+// More than 16 rows of x always: the weight is read once for all of them. Up to 16 rows (the rows kernel's) take the same time as one (Q4_K
+// 32000 x 4096: 25 us, Q5_K 35, Q6_K 42, the others 37 to 44, Q4_K 4096 x 4096 9.5), so the line lies where the decode kernels need another pass: Q4_K and Q5_K take up to eight rows in
+// one (24 and 26 us; 7.8 and 8.0), Q6_K four (34), the 32-element formats two (24 and 16). It must not depend on the number of output rows, and neither do
 // the sums, so a row shard gives bitwise the outputs of the whole weight. Where the decode kernels decline (k no multiple of 256, or too
 // wide) there is only the CUDA-core kernel besides, whose time grows with rows x k: with 4096 output rows it meets the matrix kernel near
 // rows k = 4096 for Q8_0 (k = 1056: 16.4 us at 4 rows against 17.4; 2080: 16.4 at 2 rows and 24.6 at 4 against 19.2) and near 2048 for Q4_0 and

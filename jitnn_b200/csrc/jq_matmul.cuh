@@ -25,8 +25,9 @@
 // order. Grid: one cluster per tile and range, or, without ranges, as many CTAs as the GPU has SMs walking the tiles.
 //
 // What bounds it: the tensor pipe for BF16 tiles of 200 and more rows of x (1.5 us per unit at 256, the measured rate of a dense BF16 product). Below
-// that a BF16 unit takes 0.95 us whatever the number of rows. FP32, one unit: 0.95 us for 17 MMAs (Q4_K, up to 16 rows), 1.4 for 32 (two parts,
-// up to 32 rows), 1.3 us + 6.5 ns a row for 34 (Q4_K), which is 80 to 110 clocks an MMA and what the hand-over of an accumulator takes besides.
+// that a BF16 unit takes 0.95 us whatever the number of rows. FP32, one unit: 1.4 us for 32 MMAs (two parts,
+// up to 32 rows), 1.3 us + 6.5 ns a row for 34 (Q4_K). That is not the tensor pipe (an MMA of up to 32 columns whose weights lie in tensor memory takes
+// 16 clocks) but the instructions of the roles and their hand-overs; the FP32 product of up to 16 rows has a kernel of its own (jq_rows.cuh).
 //
 // Every wait is bounded: one that runs out records a code, raises the CTA's abort flag and all roles fall through to the exit.
 #pragma once
@@ -49,7 +50,7 @@ __host__ __device__ constexpr bool one_part(int type) { return type == JQ_TYPE_Q
 template <int TYPE, bool FP32, bool BWD, int NMAX>
 struct Shape {
     static constexpr bool JOINED = FP32 && NMAX <= 32;
-    static constexpr int TURN = BWD ? 1 : (!FP32 ? (NMAX <= 128 ? 4 : 1) : (!JOINED ? (one_part(TYPE) ? 2 : 1) : (NMAX <= 16 && one_part(TYPE) ? 4 : 2)));
+    static constexpr int TURN = BWD ? 1 : (!FP32 ? (NMAX <= 128 ? 4 : 1) : (JOINED || one_part(TYPE) ? 2 : 1));
     static constexpr int GROUPS = FP32 && !JOINED ? 2 : (BWD || (!FP32 && NMAX > 128) ? 4 : 3), FOLD = FP32 && !JOINED ? 16 : 4, THREADS = (3 + 4 * GROUPS + FOLD) * 32;
     static constexpr int CHUNKS = BWD ? 2 : 4;                           // chunks of 64 of the contraction in a unit
     static constexpr int TURNS = CHUNKS / TURN;
@@ -60,11 +61,9 @@ struct Shape {
     static constexpr bool OWNED = TURNS == 1;                           // a raw unit is one group's own
     // FP32: ACC chunks' products go into one accumulator before the fold adds it up. The tensor core cuts every sum off towards zero, so the error
     // grows with the MMAs that add to an accumulator of full size. Products with a lo part are small: they go first (PAIRED: two chunks' operands
-    // and activation tiles are waited for and used together) or into columns of their own (JOINED); then 4 (backward), 8 or 16 are left.
-    // Relative to the result's norm at k = 4096: 1.5e-7 (backward) and 1.8 to 2.3e-7 with 4 and 8; 3.0e-7, which is what the decode kernels
-    // have, with 16 (Q4_K up to 16 rows, whose second hand-over a unit would take 11 % longer). All products of 256 terms as they come left
-    // 4e-7 to 2.4e-6.
-    static constexpr int ACC = BWD ? 1 : (TYPE == JQ_TYPE_Q4_K && JOINED && TURN == 4 ? 4 : 2), ACCS = CHUNKS / ACC;
+    // and activation tiles are waited for and used together) or into columns of their own (JOINED); then 4 (backward) or 8 are left.
+    // Relative to the result's norm at k = 4096: 1.5e-7 (backward) and 1.8 to 2.3e-7. All products of 256 terms as they come left 4e-7 to 2.4e-6.
+    static constexpr int ACC = BWD ? 1 : 2, ACCS = CHUNKS / ACC;
     static constexpr bool PAIRED = FP32 && !BWD && !JOINED;
     static constexpr int AHEAD = BWD && !JOINED ? 8 : 1;                // units whose scales of x the fold fetches at a time
     static constexpr int SCALES = 8 * 2 * 64 * 4 * AHEAD;               // bytes for them
@@ -75,7 +74,6 @@ constexpr int A_TILE = 128 * 128;  // 128 rows of 128 bytes
 constexpr int MAX_A = 6, MAX_B = 12, MAX_RAW = 6;
 constexpr int MAX_BUFS = 4;
 constexpr int FACTORS = 8;   // units whose factors the fold may still need, see where they are written
-constexpr int VIRTUAL = 8;   // ranges of the contraction whose sums are added up in order, whatever the cluster (instances for 16 rows of x)
 
 constexpr int MAX_WEIGHTS = 3;
 
@@ -94,7 +92,6 @@ struct Args {
     int ttiles, nt;   // tiles of nt rows of x
     int m;
     int ksplit;
-    int part_bytes;   // shared memory for the sums of this CTA's virtual ranges
     int sa, sb, raw;  // ring depths: weight operands, activation tiles, raw units
     int cols;         // tensor-memory columns of one accumulator
     int bufs;         // accumulators: as many as fit, up to MAX_BUFS
@@ -308,7 +305,6 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
     static_assert(FP32 || !BWD, "the backward product is FP32");
     constexpr bool HALF = FP32 && !BWD;  // weights by half arithmetic, see there
     constexpr bool EXT = W::EXT, JOINED = W::JOINED, OWNED = W::OWNED;
-    constexpr bool CANON = HALF && NMAX <= 16;  // sums depend on k alone, not on how many CTAs share it
     constexpr int G = W::GROUPS, TURN = W::TURN, TURNS = W::TURNS, A_COLS = W::A_COLS, BT = W::B_TILES;
     static_assert(!HALF || (W::PARTS == H::TILES && EXT == H::EXT), "");
     constexpr int X_UNIT = BWD ? 128 : 256 + (EXT ? 16 : 0);  // columns of the activations per unit
@@ -316,7 +312,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
     const uint32_t base = (tc::smem_u32(smem_unaligned) + 1023u) & ~1023u;  // swizzled tiles start on 1024-byte boundaries
     const int SA = p.sa, SB = p.sb, R = p.raw, nt = p.nt;
     const uint32_t tile_st = (uint32_t)tile_bytes(FP32, nt), a_st = (uint32_t)a_bytes(BWD), b_st = (uint32_t)BT * tile_st;
-    const uint32_t a0 = base + (uint32_t)p.part_bytes, b0 = a0 + (uint32_t)SA * a_st, raw0 = b0 + (uint32_t)SB * b_st;
+    const uint32_t a0 = base, b0 = a0 + (uint32_t)SA * a_st, raw0 = b0 + (uint32_t)SB * b_st;
     const uint32_t fac0 = raw0 + (uint32_t)R * raw_bytes<TYPE>();
     const uint32_t scl0 = fac0 + FACTORS * 128 * 4, full_a = scl0 + W::SCALES, free_a = full_a + 8 * MAX_A, full_b = free_a + 8 * MAX_A, free_b = full_b + 8 * MAX_B;
     const uint32_t raw_full = free_b + 8 * MAX_B, raw_read = raw_full + 8 * MAX_RAW;
@@ -774,7 +770,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                             // The unit's factors for the fold, into a ring of FACTORS units. This operand's slot is free, so what it held SA
                             // operands ago went through the tensor core, into an accumulator that the fold had emptied: the fold has
                             // finished the accumulator `bufs` before that one, and with it the unit eight before this one as
-                            // SA TURN / ACC + bufs <= 7 ACCS + 1 (at most 6 + 4 and 15; Q4_K up to 16 rows 3 + 4 and 8).
+                            // SA TURN / ACC + bufs <= 7 ACCS + 1 (at most 6 + 4 and 15).
                             const uint32_t fa = fac0 + (uint32_t)(at_unit & (FACTORS - 1)) * 512u;
                             if constexpr (!BWD) {
                                 asm volatile("st.shared.u32 [%0], %1;" ::"r"(fa + 4u * (uint32_t)row0), "r"(unit_factor) : "memory");
@@ -913,22 +909,10 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
             };
             if constexpr (FP32) {
                 constexpr int C = NMAX / PARTS, C32 = C < 32 ? 32 : C;  // columns per thread
-                f2 sum[C / 2], total[CANON ? C / 2 : 1];
+                f2 sum[C / 2];
 #pragma unroll
                 for (int i = 0; i < C / 2; i++) {
                     sum[i] = 0;
-                    if constexpr (CANON) {
-                        total[i] = 0;
-                    }
-                }
-                // CANON: the end of the virtual range that unit u0 belongs to; its sum is added to the total, or kept apart for the cluster
-                int virt = 0, slot = 0;
-                auto virt_end = [&](int v) { return (int)((int64_t)(v + 1) * p.units / VIRTUAL); };
-                if constexpr (CANON) {
-                    while (virt < VIRTUAL - 1 && virt_end(virt) <= u0) {
-                        virt++;
-                    }
-                    slot = virt - range * (VIRTUAL / p.ksplit);
                 }
                 // The scales of a unit's columns: fetched by the lanes AHEAD units at a time, read back as broadcasts. (A load takes up to 2000 clocks while the
                 // weights stream: one unit ahead, the backward form's units waited for it: Q4_K 32000 x 4096, 128 rows 147 us, now 138; 4096 x 4096
@@ -1000,45 +984,9 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                     if (!ok) {
                         break;
                     }
-                    if constexpr (CANON) {
-                        if (u + 1 == virt_end(virt)) {
-                            if (p.ksplit > 1) {
-#pragma unroll
-                                for (int i = 0; i < C / 2; i++) {
-                                    float a, b;
-                                    unpack2(sum[i], a, b);
-                                    const uint32_t to = base + (uint32_t)(((slot * nt + c0 + 2 * i) * 128 + lane_row) * 4);
-                                    asm volatile("st.shared.f32 [%0], %1;" ::"r"(to), "f"(a) : "memory");
-                                    asm volatile("st.shared.f32 [%0], %1;" ::"r"(to + 512u), "f"(b) : "memory");
-                                }
-                            } else {
-#pragma unroll
-                                for (int i = 0; i < C / 2; i++) {
-                                    total[i] = add2(total[i], sum[i]);
-                                }
-                            }
-#pragma unroll
-                            for (int i = 0; i < C / 2; i++) {
-                                sum[i] = 0;
-                            }
-                            do {
-                                virt++;
-                                slot++;
-                            } while (virt < VIRTUAL - 1 && virt_end(virt) <= u + 1);
-                        }
-                    }
                 }
                 if (!ok) {
                     break;
-                }
-                if constexpr (CANON) {
-                    if (p.ksplit > 1) {
-                        continue;  // (one tile per cluster)
-                    }
-#pragma unroll
-                    for (int i = 0; i < C / 2; i++) {
-                        sum[i] = total[i];
-                    }
                 }
                 // (the last accumulator is complete: every tile in shared memory is used up and may hold the partial tile)
 #pragma unroll
@@ -1084,7 +1032,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
         cluster_sync();  // partial tiles are complete
     }
     if (p.ksplit > 1 && *abort_flag == 0) {
-        // columns range, range + ksplit, .. of the tile: the (virtual) ranges' sums in order
+        // columns range, range + ksplit, .. of the tile: the ranges' sums in order
         const int ft = p.first_ft + cluster_id / p.ttiles, t0 = (cluster_id % p.ttiles) * nt;
         int ft0;
         const int wi = weight_of(p, ft, ft0);
@@ -1093,20 +1041,19 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
         const float* const bias = wi == 0 ? p.bias : nullptr;
         const int mine = (nt - range + p.ksplit - 1) / p.ksplit * 32;  // pieces of four features of a column
         constexpr int BATCH = 2, MOST = 4;  // pieces and ranges in flight: another CTA's memory is most of a microsecond away
-        const int parts = CANON ? VIRTUAL : p.ksplit, per_cta = parts / p.ksplit;
         for (int i0 = threadIdx.x; i0 < mine; i0 += BATCH * W::THREADS) {
             float4 sum[BATCH];
 #pragma unroll
             for (int j = 0; j < BATCH; j++) {
                 sum[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             }
-            for (int g0 = 0; g0 < parts; g0 += MOST) {
+            for (int g0 = 0; g0 < p.ksplit; g0 += MOST) {
                 float4 v[MOST][BATCH];
 #pragma unroll
                 for (int g = 0; g < MOST; g++) {
                     const int part = g0 + g;
-                    const bool there = part < parts && (!CANON || (int64_t)part * p.units / VIRTUAL < (int64_t)(part + 1) * p.units / VIRTUAL);
-                    const uint32_t from = map_rank(base + (uint32_t)(part % per_cta * nt * 512), (uint32_t)(there ? part / per_cta : 0));
+                    const bool there = part < p.ksplit;
+                    const uint32_t from = map_rank(base, (uint32_t)(there ? part : 0));
 #pragma unroll
                     for (int j = 0; j < BATCH; j++) {
                         const int i = i0 + j * W::THREADS, col = range + (i >> 5) * p.ksplit;

@@ -33,7 +33,7 @@ Facts facts_format(bool fp32, bool bwd, int nmax) {
     if (bwd) {
         return nmax <= 32 ? facts_of<TYPE, true, true, 32>() : facts_of<TYPE, true, true, 128>();
     }
-    return nmax <= 16 ? facts_of<TYPE, true, false, 16>() : (nmax <= 32 ? facts_of<TYPE, true, false, 32>() : facts_of<TYPE, true, false, 128>());
+    return nmax <= 32 ? facts_of<TYPE, true, false, 32>() : facts_of<TYPE, true, false, 128>();
 }
 
 template <int TYPE, bool FP32, bool BWD, int NMAX>
@@ -73,9 +73,7 @@ int launch_format(const Plan& plan, const Args& args, const CUtensorMap& map, cu
     if (plan.bwd) {
         return plan.nmax <= 32 ? launch_instance<TYPE, true, true, 32>(plan, args, map, s) : launch_instance<TYPE, true, true, 128>(plan, args, map, s);
     }
-    return plan.nmax <= 16   ? launch_instance<TYPE, true, false, 16>(plan, args, map, s)
-           : plan.nmax <= 32 ? launch_instance<TYPE, true, false, 32>(plan, args, map, s)
-                             : launch_instance<TYPE, true, false, 128>(plan, args, map, s);
+    return plan.nmax <= 32 ? launch_instance<TYPE, true, false, 32>(plan, args, map, s) : launch_instance<TYPE, true, false, 128>(plan, args, map, s);
 }
 
 int launch_q4_k(const Plan& plan, const Args& args, const CUtensorMap& map, cudaStream_t s);
