@@ -742,18 +742,15 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                         for (int j = 0; j < TURN; j++) {
                             raw[j] = D::load(uq, row, c0 + j);
                         }
-                        if (OWNED || turn + G >= TURNS) {
-                            // This warp has read all it needs of the unit once the values are in registers. Program order alone does not see to that: the
-                            // arrival overtook loads whose values were used later, and the next unit was copied over what they had yet to read (backward,
-                            // 11008 x 4096 Q4_0, 128 rows: wrong weights in 179 of 200 calls). A vote on a word of every load waits for them.
-                            uint32_t seen = D::seen(head);
-#pragma unroll
-                            for (int j = 0; j < TURN; j++) {
-                                seen ^= words_seen(raw[j]);
-                            }
-                            if (__any_sync(0xffffffffu, seen == 0x9E3779B9u)) {
-                                __threadfence_block();  // (nothing more to wait for)
-                            }
+                        // This warp has read all it needs of the unit once its loads are done. Program order alone does not see to that: with an arrival right
+                        // behind loads whose values are used later, the next unit was copied over what they had yet to read (backward, 11008 x 4096
+                        // Q4_0, 128 rows: wrong weights in 179 of 200 calls). FP32 forward gives the unit back when its values have gone to tensor
+                        // memory; the others, which use theirs behind another wait, behind a fence. (A vote on a word of every load, in all forms:
+                        // Q8_0 11008 x 4096, 200 rows 65.7 us, now 63.8; Q4_K 57.6 and 57.4; BF16 Q4_K 512 rows 46.1 and 45.3; backward Q6_K 4096 x 4096,
+                        // 128 rows 28.4 and 27.9. Only Q4_1 was faster with it: 300 rows 92.2 and 92.9.)
+                        const bool done = OWNED || turn + G >= TURNS;
+                        if (!HALF && done) {
+                            tc::reads_before_refill();
                             if (lane == 0) {
                                 tc::mbar_arrive(raw_read + 8 * r);
                             }
@@ -823,6 +820,12 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                                     uint32_t v[8];
                                     H::ext(head, v);
                                     st_tmem8(to + TURN * 32 * W::PARTS, v);
+                                }
+                            }
+                            if (HALF && done) {
+                                __syncwarp();
+                                if (lane == 0) {
+                                    tc::mbar_arrive(raw_read + 8 * r);
                                 }
                             }
                             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -920,12 +923,14 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                 constexpr int AHEAD = W::AHEAD, NEXT = (C * AHEAD + 31) / 32;
                 const uint32_t scl = scl0 + (uint32_t)(warp - 3 - 4 * G) * (8u * C32 * AHEAD);
                 float next[NEXT];
+                const float* xs = p.xscale + (int64_t)u0 * p.xstride + t0 + c0 + lane;  // of the units that are fetched next
                 auto fetch = [&](int u) {
 #pragma unroll
                     for (int i = 0; i < NEXT; i++) {
-                        const int on = AHEAD > 1 ? i : 0, col = AHEAD > 1 ? lane : lane + 32 * i;  // (AHEAD > 1: 32 columns)
-                        next[i] = col < cols && u + on < u1 ? __ldg(p.xscale + (int64_t)(u + on) * p.xstride + t0 + c0 + col) : 0.0f;
+                        const int on = AHEAD > 1 ? i : 0, off = AHEAD > 1 ? 0 : 32 * i;  // (AHEAD > 1: 32 columns)
+                        next[i] = lane + off < cols && (AHEAD == 1 || u + on < u1) ? __ldg(xs + (int64_t)on * p.xstride + off) : 0.0f;
                     }
+                    xs += (int64_t)AHEAD * p.xstride;
                 };
                 fetch(u0);
                 for (int u = u0; u < u1; u++, chunk++) {

@@ -59,19 +59,6 @@ __device__ __forceinline__ uint32_t max_half8(const uint4& v) {
     return max(m & 0xffffu, m >> 16);
 }
 
-// A word that depends on every 16-byte load of v.
-template <typename T>
-__device__ __forceinline__ uint32_t words_seen(const T& v) {
-    static_assert(sizeof(T) % 16 == 0, "");
-    const uint4* const w = reinterpret_cast<const uint4*>(&v);
-    uint32_t x = w[0].x;
-#pragma unroll
-    for (int i = 1; i < (int)(sizeof(T) / 16); i++) {
-        x ^= w[i].x;
-    }
-    return x;
-}
-
 // Words of the scales and mins of sub-blocks 4 (c >> 1) .. + 3 (GgufKernels.java:74-83), one byte each.
 __device__ __forceinline__ void scale_min_words(const uint4& h, int c, uint32_t& sc, uint32_t& mn) {
     const uint32_t high_sc = (h.w & 0x0f0f0f0fu) | ((h.y >> 2) & 0x30303030u), high_mn = ((h.w >> 4) & 0x0f0f0f0fu) | ((h.z >> 2) & 0x30303030u);
@@ -104,7 +91,6 @@ struct DqK45 {
         }
         return r;
     }
-    __device__ static __forceinline__ uint32_t seen(const Head& r) { return Q5 ? r.h.x ^ r.hi[0].x ^ r.hi[1].x : r.h.x; }
     __device__ static __forceinline__ Raw load(uint32_t uq, int row, int c) {
         const uint32_t at = uq + (uint32_t)row * ROW + (Q5 ? 48 : 16) + 32 * c;
         return Raw{{lds16(at), lds16(at + 16)}};
@@ -179,7 +165,6 @@ struct Dq<JQ_TYPE_Q6_K> {
         r.d = __half2float(__ushort_as_half(d));
         return r;
     }
-    __device__ static __forceinline__ uint32_t seen(const Head& r) { return r.sv.x ^ __float_as_uint(r.d); }
     __device__ static __forceinline__ Raw load(uint32_t uq, int row, int c) {
         const uint32_t l = uq + (uint32_t)row * ROW + 64 * (c >> 1), h = uq + (uint32_t)row * ROW + 128 + 32 * (c >> 1);
         return Raw{{lds16(l), lds16(l + 16)}, {lds16(l + 32), lds16(l + 48)}, {lds16(h), lds16(h + 16)}};
@@ -227,7 +212,6 @@ struct Dq<JQ_TYPE_Q8_0> {
     };
     __device__ static __forceinline__ int piece(int part, int run) { return 4 * part + 2 * run; }
     __device__ static __forceinline__ Head head(uint32_t, uint32_t ua, int row) { return Head{lds16(ua + 16u * (uint32_t)row)}; }
-    __device__ static __forceinline__ uint32_t seen(const Head& r) { return r.d.x; }
     __device__ static __forceinline__ Raw load(uint32_t uq, int row, int c) {
         const uint32_t base = uq + (uint32_t)row * ROW;
         return Raw{{lds16(base + 16 * swizzle_piece(4 * c, row)), lds16(base + 16 * swizzle_piece(4 * c + 1, row)), lds16(base + 16 * swizzle_piece(4 * c + 2, row)),
@@ -279,7 +263,6 @@ struct DqN {
         }
         return r;
     }
-    __device__ static __forceinline__ uint32_t seen(const Head& r) { return HAS_MIN ? r.d.x ^ r.d2.x : r.d.x; }
     __device__ static __forceinline__ Raw load(uint32_t uq, int row, int c) {
         const uint32_t base = uq + (uint32_t)row * ROW;
         return Raw{{lds16(base + 16 * swizzle_piece(2 * c, row)), lds16(base + 16 * swizzle_piece(2 * c + 1, row))}};

@@ -70,6 +70,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
 }
 
+// Between a warp's reads of shared memory and the arrival that lets the copy engine fill it again. A barrier among the lanes orders their loads
+// against each other's, not against the copy engine, and a load whose value is used later may be made behind the arrival; the fence between
+// the proxies orders them.
+__device__ __forceinline__ void reads_before_refill() {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+}
+
 // One contiguous run of bytes (a multiple of 16, both addresses 16-byte aligned) from global into shared memory.
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)

@@ -236,7 +236,9 @@ def test_error_is_no_larger_than_the_decode_kernels(t):
 @pytest.mark.parametrize("t,n,k,m,kind", [("Q4_0", 11008, 4096, 128, "backward"), ("Q8_0", 11008, 4096, 128, "backward"), ("Q5_K", 11008, 4096, 128, "backward"),
                                           ("Q6_K", 11008, 4096, 128, "backward"), ("Q4_1", 11008, 4096, 100, "backward"), ("Q4_K", 11008, 4096, 128, "backward"),
                                           ("Q8_0", 4096, 4096, 512, "bf16"), ("Q6_K", 4096, 4096, 512, "bf16"), ("Q4_K", 11008, 4096, 200, "forward"),
-                                          ("Q8_0", 11008, 4096, 16, "forward")])
+                                          ("Q8_0", 11008, 4096, 16, "forward"), ("Q4_0", 11008, 4096, 24, "forward"), ("Q5_K", 11008, 4096, 32, "forward"),
+                                          ("Q6_K", 11008, 4096, 100, "forward"), ("Q8_0", 11008, 4096, 200, "forward"), ("Q4_1", 11008, 4096, 300, "forward"),
+                                          ("Q4_K", 4096, 11008, 100, "bf16"), ("Q5_K", 11008, 4096, 300, "bf16")])
 def test_repeated_calls_give_the_same_bits(t, n, k, m, kind):
     w, _ = weight(t, n, k, seed=2)
     x = torch.randn(m, n if kind == "backward" else k, generator=torch.Generator().manual_seed(4)).cuda()
