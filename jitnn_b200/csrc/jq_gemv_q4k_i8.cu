@@ -517,7 +517,9 @@ __global__ void __launch_bounds__(NW * 32, OCC) gemv_q4k_i8_kernel(View v, Secon
             const int my_tile = (int)blockIdx.x + ti * (int)gridDim.x;
             const uint8_t* blk = xd_lane + (size_t)warp * C::PB;
             for (int j = 0; j < nb; j++) {
-                __syncwarp();  // every lane is done reading the slot that is requested next
+                // Every lane is done with the slot that is requested next: its values have been multiplied in compute(), in front of this point, and it is
+                // this warp that makes the request. (A proxy fence or a request that needs the last products would wait longer: 32000 x 4096 14.24 -> 14.43 and 14.57 us.)
+                __syncwarp();
                 issue();
                 if (!gave_up) {
                     // the copy of this step has landed (bounded: the clock, not the number of polls)

@@ -334,7 +334,9 @@ __global__ void __launch_bounds__(THREADS, OCC) gemv_q6k_i8_kernel(View v, const
         for (int ti = 0; ti < my_tiles; ti++) {
             const int my_tile = (int)blockIdx.x + ti * (int)gridDim.x;
             for (int b = warp; b < len; b += WARPS) {
-                __syncwarp();  // every lane is done reading the slot that is requested next
+                // Every lane is done with the slot that is requested next: its values have been multiplied in compute(), in front of this point, and it is
+                // this warp that makes the request. (A proxy fence or a vote that needs the last products would wait longer: 32000 x 4096 21.83 -> 22.08 and 22.07 us.)
+                __syncwarp();
                 issue();
                 if (!gave_up) {
                     // the copies of this step have landed (bounded: the clock, not the number of polls)

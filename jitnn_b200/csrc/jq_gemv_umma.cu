@@ -879,7 +879,7 @@ __global__ void __launch_bounds__(Roles<MR>::THREADS, 1) gemv_umma_kernel(const 
                 c[m] = fmaf(d, q, -(dmin * msum[m]));
             }
             if constexpr (!RES) {
-                __syncwarp();
+                tc::reads_before_refill();  // the weights and sums of x (aux)
                 if (lane == 0) {
                     tc::mbar_arrive(empty_x(xs));
                 }
