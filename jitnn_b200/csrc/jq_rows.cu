@@ -1,4 +1,5 @@
-// Host side of the rows kernel (jq_rows.cuh): the image of x, the choice of launches.
+// Host side of the rows kernel (jq_rows.cuh): the image of x, the launches (their choice: jq_rows_cut.cuh).
+#include "jq_rows_cut.cuh"
 #include "jq_rows_launch.cuh"
 
 namespace jq {
@@ -72,55 +73,6 @@ __global__ void __launch_bounds__(128) image_kernel(const float* __restrict__ x,
     if (lane == 0) {
         scales[(int64_t)u * NT + row] = bad ? __uint_as_float(0x7fc00000u) : __uint_as_float((e - 9u) << 23);
     }
-}
-
-// Clusters of ks thread blocks that run at a time, one thread block per SM (cudaOccupancyMaxActiveClusters; the SMs of a GPC are not all a multiple of
-// 4 or 8).
-static int clusters_of(int ks) { return ks == 1 ? 148 : (ks == 2 ? 74 : (ks == 4 ? 33 : 15)); }
-
-// What a unit takes a thread block in nanoseconds, measured on 32000 x 4096.
-static double unit_ns(int type) { return type == JQ_TYPE_Q4_K ? 630.0 : (type == JQ_TYPE_Q5_K ? 940.0 : (type == JQ_TYPE_Q4_0 ? 1040.0 : 1170.0)); }
-
-// A product's tiles in up to three launches, each with its own number of thread blocks per tile: whole waves first, then what is left, which alone would
-// leave most of the chip idle for a whole contraction, with its contraction split over clusters (57344 x 8192: 448 tiles are three waves and four
-// tiles: 85.5 us in one launch, 71.7 in two). The launch behind starts where SMs become free; GAP_NS is its own start.
-constexpr int MAX_PARTS = 3;
-constexpr double GAP_NS = 2500.0;
-struct Parts {
-    int count;
-    int tiles[MAX_PARTS], ksplit[MAX_PARTS];
-};
-static double cut(int tiles, int units, double unit, int most, Parts& out) {
-    double best = 1e30;
-    for (int ks = 1; ks <= 8 && (ks == 1 || units >= 2 * ks); ks *= 2) {
-        const int slots = clusters_of(ks), waves = (tiles + slots - 1) / slots;
-        auto cost_of = [&](int w) { return w * (((units + ks - 1) / ks) * unit + 1700.0) + (ks > 1 ? 1600.0 : 0.0); };
-        if (ks == 1 || waves == 1) {
-            const double cost = cost_of(waves);
-            if (cost < best) {
-                best = cost;
-                out.count = 1;
-                out.tiles[0] = tiles;
-                out.ksplit[0] = ks;
-            }
-        }
-        const int whole = ks == 1 ? tiles / slots : 1, front = whole * slots;
-        if (most > 1 && front > 0 && front < tiles) {
-            Parts rest;
-            const double cost = cost_of(whole) + GAP_NS + cut(tiles - front, units, unit, most - 1, rest);
-            if (cost < best) {
-                best = cost;
-                out.count = 1 + rest.count;
-                out.tiles[0] = front;
-                out.ksplit[0] = ks;
-                for (int i = 0; i < rest.count; i++) {
-                    out.tiles[1 + i] = rest.tiles[i];
-                    out.ksplit[1 + i] = rest.ksplit[i];
-                }
-            }
-        }
-    }
-    return best;
 }
 
 static int launch_any(int type, Args& a, int ctas, bool after, cudaStream_t s) {

@@ -16,9 +16,11 @@ pytestmark = pytest.mark.gpu
 
 REL = 1e-5
 
-# one row of W; a second tile's first row; one unit of k, fewer units than ranges, no multiple of the ranges; k over 2, 4 and 8 thread blocks; one wave
-# and one tile, three launches (148 + 74 + rest) and a short contraction whose scales of x stay from tile to tile
-SHAPES = [(1, 256, 9), (129, 512, 16), (128, 2816, 10), (4096, 4096, 13), (1024, 8192, 16), (2000, 16384, 9), (19000, 2048, 12), (30000, 1024, 16)]
+# One row of W; a second tile's first row; one unit of k, fewer units than ranges, no multiple of the ranges; few tiles with k over 8, 4 and 2 thread blocks;
+# two waves of whole tiles whose scales of x stay from tile to tile; whole tiles and what is left in two launches; a cluster launch in front of another.
+# (test_rows_plan.py has the launches of each.)
+SHAPES = [(1, 256, 9), (129, 512, 16), (128, 2816, 10), (4096, 4096, 13), (1024, 8192, 16), (2000, 16384, 9), (19000, 2048, 12), (30000, 1024, 16),
+          (6400, 4096, 12), (18950, 2560, 10), (23200, 3584, 15), (9500, 8192, 11), (4300, 14080, 14)]
 
 
 @pytest.mark.parametrize("n,k,m", SHAPES)
