@@ -8,7 +8,7 @@ import pytest
 
 from conftest import LINEAR_TYPES, ROOT
 from oracle.oracle import TYPES
-from test_gpu_rows import SHAPES
+from test_gpu_rows import SHAPES, THREE_LAUNCHES, TWO_LAUNCHES
 
 CALL = """
 #include "jq_rows_cut.cuh"
@@ -44,14 +44,14 @@ def plan(tmp_path_factory):
 PLANS = {
     (1, 256): [(1, 1)], (129, 512): [(2, 1)], (128, 2816): [(1, 4)], (4096, 4096): [(32, 4)], (1024, 8192): [(8, 8)], (2000, 16384): [(16, 4)],
     (19000, 2048): [(148, 1), (1, 4)], (30000, 1024): [(235, 1)], (6400, 4096): [(50, 2)], (18950, 2560): [(148, 1), (1, 4)],
-    (23200, 3584): [(148, 1), (34, 2)], (9500, 8192): [(74, 2), (1, 8)], (4300, 14080): [(33, 4), (1, 8)],
+    (23200, 3584): [(148, 1), (34, 2)], (9500, 8192): [(74, 2), (1, 8)], (4300, 14080): [(33, 4), (1, 8)], (28500, 11264): [(148, 1), (74, 2), (1, 8)],
 }
 PLANS_Q4_K = {(19000, 2048): [(149, 1)], (4300, 14080): [(34, 2)]}
 
 
 @pytest.mark.parametrize("t", LINEAR_TYPES)
 def test_launches_of_the_tested_shapes(plan, t):
-    for n, k, _ in SHAPES:
+    for n, k in [s[:2] for s in SHAPES] + [TWO_LAUNCHES, THREE_LAUNCHES]:
         want = PLANS_Q4_K.get((n, k), PLANS[n, k]) if t == "Q4_K" else PLANS[n, k]
         assert plan(t, n, k) == want, (n, k)
 
