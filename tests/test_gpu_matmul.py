@@ -1,4 +1,5 @@
-"""The tensor-core matrix kernel (FP32 products with many rows of x, and the input gradient) where its tiles, ranges and rings end.
+"""The tensor-core matrix kernel (FP32 products with many rows of x, and the input gradient) where its tiles, ranges and rings end, and the values
+that are hard on it and, with up to 16 rows of x, on the rows kernel.
 
 The reference is the product of the oracle's dequantised weights in double. Both operands of the kernel keep 22 significant bits (2^-22 each),
 and sums of at most 272 terms are taken in FP32 by the tensor core before they are added up in FP32 registers: 3e-7 of the result's norm or
@@ -53,8 +54,8 @@ def test_backward(t, n, k, m):
     close(Gguf.linearBackward(g, w), g.double() @ wd)
 
 
-# products cut by features into several launches, each with its own tiles: 150 tiles for 9 rows (two more than a wave), 86 x 2 for 200 rows, and the
-# backward form, with an even and an odd first tile of features
+# products cut by features into several launches, each with its own tiles: 150 tiles for 9 rows (two more than a wave; the rows kernel), 86 x 2 for 200 rows,
+# and the backward form, with an even and an odd first tile of features
 @pytest.mark.parametrize("t,n,k,m,bwd", [("Q4_K", 19100, 8192, 9, False), ("Q6_K", 19100, 8192, 9, False), ("Q4_K", 11000, 4096, 200, False),
                                          ("Q6_K", 11000, 4096, 500, False), ("Q8_0", 4096, 11008, 128, True), ("Q4_K", 16384, 5120, 128, True)])
 def test_cut_by_features(t, n, k, m, bwd):
@@ -68,8 +69,8 @@ def test_cut_by_features(t, n, k, m, bwd):
         close(Gguf.linear(x, w, b), x.double() @ wd.T + b.double())
 
 
-# up to 16 rows the sums are taken in eight ranges of k whatever the number of thread blocks that share it: a row shard, whose k is split over a
-# larger cluster, gives bitwise the outputs of the whole weight. k: fewer units than ranges, more, and not a multiple
+# up to 16 rows (the rows kernel) the sums are taken in eight ranges of k whatever the number of thread blocks that share it: a row shard, whose k is
+# split over a larger cluster, gives bitwise the outputs of the whole weight. k: fewer units than ranges, more, and not a multiple
 @pytest.mark.parametrize("k", [768, 2048, 2816, 11008])
 @pytest.mark.parametrize("t", LINEAR_TYPES)
 def test_row_shards_are_bitwise_equal(t, k):
@@ -85,11 +86,12 @@ def test_row_shards_are_bitwise_equal(t, k):
     close(y, x.double() @ wd.T)
 
 
-# 32-element formats: k that does not fill a step of 256, or not even a multiple of 4 x 32
+# 32-element formats: k that does not fill a step of 256, or not even a multiple of 4 x 32 (13 rows: the rows kernel where rows x k is large enough)
+@pytest.mark.parametrize("m", [20, 13])
 @pytest.mark.parametrize("k", [32, 96, 224, 288, 1056])
 @pytest.mark.parametrize("t", ["Q8_0", "Q4_0", "Q4_1"])
-def test_partial_steps(t, k):
-    n, m = 150, 20
+def test_partial_steps(t, k, m):
+    n = 150
     w, wd = weight(t, n, k, seed=k)
     g = torch.Generator().manual_seed(k)
     x, gy = torch.randn(m, k, generator=g).cuda(), torch.randn(m, n, generator=g).cuda()
@@ -97,9 +99,10 @@ def test_partial_steps(t, k):
     close(Gguf.linearBackward(gy, w), gy.double() @ wd)
 
 
-def test_wide_ranges():
+@pytest.mark.parametrize("m", [64, 13])
+def test_wide_ranges(m):
     """Scales and mins of very different sizes within a row's block and across rows, zero and subnormal scales, x over 80 powers of two."""
-    n, k, m = 256, 512, 64
+    n, k = 256, 512
     for t in LINEAR_TYPES:
         block = {"Q8_0": 34, "Q4_0": 18, "Q4_1": 20, "Q4_K": 144, "Q5_K": 176, "Q6_K": 210}[t]
         fields = {"Q8_0": [0], "Q4_0": [0], "Q4_1": [0, 2], "Q4_K": [0, 2], "Q5_K": [0, 2], "Q6_K": [208]}[t]
@@ -176,10 +179,11 @@ def k_scales(sc, mn):
 
 # mins far above the scales beside sub-blocks whose min is 0 or 1: every weight keeps its own 22 bits. All quants of a sub-block are equal and x is
 # positive, so an error of a weight does not average out. ratio = dmin / d, 0: d is zero
+@pytest.mark.parametrize("m", [20, 13])
 @pytest.mark.parametrize("ratio", [30.0, 900.0, 1001.0, 1100.0, 20000.0, 1.0e6, 0.0])
 @pytest.mark.parametrize("t", ["Q4_K", "Q5_K"])
-def test_mins_far_above_the_scales(t, ratio):
-    n, k, m = 64, 512, 20
+def test_mins_far_above_the_scales(t, ratio, m):
+    n, k = 64, 512
     block, quants = {"Q4_K": (144, 16), "Q5_K": (176, 16)}[t]
     d = 0.0 if ratio == 0.0 else (2.0 ** -14 if ratio > 30000 else 2.0 ** -9)
     dmin = float(np.float16(d * ratio if ratio else 0.37))
@@ -208,6 +212,37 @@ def test_mins_far_above_the_scales(t, ratio):
         y, ref = Gguf.linear(part, w).double(), part.double() @ wd.T
         # 2^-22 of the two parts of each weight, 2^-22 of x, and what the tensor cores cut off: some 2^-23 a step
         assert float(((y - ref).abs() / (part.double() @ size.T + 1e-30)).max()) <= 2e-6, (sub, ratio)
+    assert device_status(0) == 0
+
+
+# Q4_1: one min far above the others of the same 256, and x in one block of 32 at a time, so that the large min does not hide the others: what is the same
+# for a block (8 d + min) goes as two halves under one power of two for all eight, which keep 22 bits of each down to 2^-17 of the largest
+@pytest.mark.parametrize("m", [20, 13])
+@pytest.mark.parametrize("ratio", [30.0, 1000.0, 30000.0])
+def test_one_min_far_above_the_others(ratio, m):
+    n, k = 64, 512
+    parts = np.empty((n, k // 32))  # of a block's weights: d q + min
+
+    def edit(raw):
+        rng = np.random.default_rng(int(ratio))
+        for row, blocks in enumerate(raw.reshape(n, k // 32, 20)):
+            mins = rng.uniform(0.5, 1.0, k // 32) * 2.0 ** -9
+            mins[row % 8::8] *= ratio
+            mins = mins.astype(np.float16)
+            blocks[:, 0:2] = np.full(k // 32, 2.0 ** -9, np.float16).view(np.uint8).reshape(-1, 2)
+            blocks[:, 2:4] = mins.view(np.uint8).reshape(-1, 2)
+            blocks[:, 4:] = 0xff if row % 2 == 0 else 0x77
+            parts[row] = 2.0 ** -9 * (15 if row % 2 == 0 else 7) + mins.astype(np.float64)
+
+    w, wd = weight("Q4_1", n, k, 3, edit)
+    assert bool((wd == torch.from_numpy(np.repeat(parts, 32, axis=1)).cuda()).all())  # all weights of a block are the same
+    x = torch.rand(m, k, generator=torch.Generator().manual_seed(9)).cuda() + 0.5
+    for block in range(k // 32):
+        part = torch.zeros_like(x)
+        part[:, 32 * block:32 * block + 32] = x[:, 32 * block:32 * block + 32]
+        y, ref = Gguf.linear(part, w).double(), part.double() @ wd.T
+        # as above: 2^-22 of the two parts of each weight, 2^-22 of x, and what the tensor cores cut off
+        assert float(((y - ref).abs() / ref).max()) <= 2e-6, (block, ratio)
     assert device_status(0) == 0
 
 
