@@ -453,19 +453,22 @@ int launch_matmul_f32_multi(const View* vs, int count, const float* x, int64_t m
     return mm::product_f32(vs, count, false, x, nullptr, m, nullptr, ys, s);
 }
 
-// More than 16 rows of x always: the weight is read once for all of them. Up to 16 rows (the rows kernel's) take the same time as one (Q4_K
-// 32000 x 4096: 25 us, Q5_K 35, Q6_K 42, the others 37 to 44, Q4_K 4096 x 4096 9.5), so the line lies where the decode kernels need another pass: Q4_K and Q5_K take up to eight rows in
-// one (24 and 26 us; 7.8 and 8.0), Q6_K four (34), the 32-element formats two (24 and 16). It must not depend on the number of output rows, and neither do
-// the sums, so a row shard gives bitwise the outputs of the whole weight. Where the decode kernels decline (k no multiple of 256, or too
-// wide) there is only the CUDA-core kernel besides, whose time grows with rows x k: with 4096 output rows it meets the matrix kernel near
-// rows k = 4096 for Q8_0 (k = 1056: 16.4 us at 4 rows against 17.4; 2080: 16.4 at 2 rows and 24.6 at 4 against 19.2) and near 2048 for Q4_0 and
-// Q4_1 (1056: 16.4 at 2 rows and 32.8 at 4 against 17.4; 2080: 16.4 at one row against 17.4).
+// More than 16 rows of x always: the weight is read once for all of them. Up to 16 rows (the rows kernel's) take the same time as one, so the line lies
+// where the decode kernels need another pass. Measured with 4096 and 32000 output rows, k = 4096, last row count in front of the line / first behind it / the
+// rows kernel, us: Q4_K (8 rows in a pass) 6.9 / 11.2 / 9.0 and 24.3 / 38.8 / 24.4; Q5_K 7.2 / 12.5 / 10.6 and 26.5 / 43.8 / 34.9; Q6_K (4) 8.2 / 14.4 / 11.5
+// and 33.9 / 55.3 / 41.2; the 32-element formats (2; the third pass) Q8_0 10.0 / 14.4 / 12.0 and 47.4 / 70.5 / 41.6, Q4_0 9.1 / 13.5 / 10.6 and 31.8 / 45.2 / 37.2,
+// Q4_1 9.6 / 14.6 / 11.1 and 33.2 / 48.7 / 43.1. K-quants with k = 1024 alike: Q4_K 5.0 / 7.2 / 5.7 and 15.1 / 21.6 / 9.9, Q5_K 5.2 / 7.4 / 7.0 and 15.6 / 23.1 / 11.9.
+// The line must not depend on the number of output rows, and neither do the sums, so a row shard gives bitwise the outputs of the whole weight.
+// Where the decode kernels decline (k no multiple of 256, or too wide) there is only the CUDA-core kernel besides, whose time grows with rows x k and
+// with the output rows. At 4096 of them the rows kernel is the faster one from a little less on than the lines below say: Q8_0 k = 288 from 5 rows (5.6 us
+// against 5.2), 1056 from 3 (9.2, 8.4), 2080 from 2 (11.1, 10.0); Q4_0 and Q4_1 288 from 3 (7.4, 5.1), 1056 from 2 (10.7, 8.1), 2080 from one (10.6, 9.4).
+// In front of the lines a call needs no scratch buffer, so that a program may capture one that it has not made before.
 bool matmul_takes(const View& v, int64_t rows) {
     if (rows > 16) {
         return true;
     }
     if (v.type == JQ_TYPE_Q4_K || v.type == JQ_TYPE_Q5_K) {
-        return rows >= (v.k <= 1024 ? 12 : 9);
+        return rows >= 9;
     }
     if (v.type == JQ_TYPE_Q6_K) {
         return rows >= 5;

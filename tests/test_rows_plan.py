@@ -1,12 +1,16 @@
-"""How the rows kernel's tiles go into launches (jitnn_b200/csrc/jq_rows_cut.cuh), without a GPU: the shapes of its GPU tests reach every kind of plan."""
+"""How the rows kernel's tiles go into launches (jitnn_b200/csrc/jq_rows_cut.cuh), without a GPU but for the last test: the shapes of its GPU tests reach
+every kind of plan."""
 import ctypes
 import os
 import shutil
 import subprocess
 
 import pytest
+import torch
 
+import jitnn_b200
 from conftest import LINEAR_TYPES, ROOT
+from jitnn_b200 import Gguf, Tensor, synth
 from oracle.oracle import TYPES
 from test_gpu_rows import SHAPES, THREE_LAUNCHES, TWO_LAUNCHES
 
@@ -64,3 +68,18 @@ def test_launches_hold_every_tile_once_and_fit_the_chip(plan, t):
             assert 1 <= len(parts) <= 3 and sum(tiles for tiles, _ in parts) == (n + 127) // 128
             for tiles, ks in parts:
                 assert tiles > 0 and (ks == 1 or (ks in (2, 4, 8) and tiles * ks <= 148 and (k + 255) // 256 >= 2 * ks))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("t", LINEAR_TYPES)
+def test_the_tested_shapes_are_the_rows_kernels(t):
+    """x's image and the launches of the plan: no shape goes to the decode kernels instead (32-element formats, Q6_K: from 5 rows on, Q4_K and Q5_K: from 9)."""
+    L = jitnn_b200.load()
+    for n, k, m in SHAPES:
+        raw = synth.random_valid_blocks(t, n, k, seed=1).numpy().reshape(-1)
+        w, x = Tensor.quantized(t, raw, n, k), torch.zeros(m, k, device="cuda")
+        before = L.jq_launch_count()
+        Gguf.linear(x, w)
+        want = PLANS_Q4_K.get((n, k), PLANS[n, k]) if t == "Q4_K" else PLANS[n, k]
+        assert L.jq_launch_count() - before == 1 + len(want), (n, k, m)
+        w.release()
