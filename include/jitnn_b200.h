@@ -119,9 +119,9 @@ JQ_API int jq_dequantize(const jq_weight* w, float* dst, int dst_mem, void* stre
  * non-finite outputs (Q4_K, Q5_K: NaN in every output of that row of x). Stands in for Gguf.linear(x, w, bias) (ops/Gguf.java:76-98) and
  * Quant.linear / F.linearQ8 (ops/Quant.java:66-80): any m >= 0 (leading axes of x flattened by the
  * caller as ops/Gguf.java:86-93 does), bias may be NULL. Rows are dispatched like the reference
- * dispatches them (ops/Gguf.java:90): few rows to the fused dequantise-GEMV kernels, more (from 5 to 12 on, by format;
- * always above 16) to the tensor-core matrix kernel, which takes x and the weights as sums of two half-precision numbers (22 significant bits, relative to the largest
- * magnitude of a 256-element block) and adds up in FP32 (errors of 2e-7 to 3e-7 of the result's norm, the decode kernels' own),
+ * dispatches them (ops/Gguf.java:90): few rows to the fused dequantise-GEMV kernels, more to the tensor cores (from 5 to 12 rows on, by format, the
+ * rows kernel; always above 16 the matrix kernel), which take x and the weights as sums of two half-precision numbers (22 significant bits, relative to the largest
+ * magnitude of a 256-element block) and add up in FP32 (errors of 1.3e-7 to 2.4e-7 of the result's norm; the decode kernels' are 2.8e-7 to 3.2e-7),
  * unless the bfloat16 prefill path is selected with jq_set_option. `mem` says where x, bias and y live (all three alike); with JQ_MEM_DEVICE they must
  * be 16-byte aligned and `stream` is the CUDA stream (cudaStream_t, NULL = default stream).
  */
@@ -220,12 +220,12 @@ JQ_API int jq_quantize_q8_0(int device, const float* x, int64_t count, void* blo
  *   "decoder_fused"     zero: the decoder's single-token step uses the general kernels (one per operator) instead of the
  *                       fused ones that hand activations to the next linear as its activation image.
  *   "gemv_tcgen05"      which Q4_K and Q5_K decode GEMVs run on the tcgen05 GEMV (1 to 16 rows of x in one pass over the weights)
- *                       instead of the mma.sync one (up to 8 rows) and the matrix kernel (more). 0 (default): the shapes the
+ *                       instead of the mma.sync one (up to 8 rows) and the rows kernel (more). 0 (default): the shapes the
  *                       mma.sync kernel declines; 1: all; 2: none.
  *   "wait_limit_us"     microseconds after which a kernel's wait for its own copies and tensor-core work gives up (default 2 000 000,
- *                       in the matrix kernel counted from the end of the kernel in front): the call returns JQ_ERR_TIMEOUT or
- *                       jq_device_status reports a code (1 to 8 matrix kernel, 24 and 25 decode GEMVs, 64 + role tcgen05
- *                       GEMV), its outputs are undefined.
+ *                       in the matrix and the rows kernel counted from the end of the kernel in front): the call returns JQ_ERR_TIMEOUT
+ *                       or jq_device_status reports a code (1 to 8 matrix and rows kernel, 24 and 25 decode GEMVs, 64 + role
+ *                       tcgen05 GEMV), its outputs are undefined.
  */
 JQ_API int jq_set_option(const char* name, int64_t value);
 JQ_API int jq_get_option(const char* name, int64_t* value);

@@ -334,8 +334,8 @@ std::atomic<int64_t> g_opt_gemv_generic{0};
 std::atomic<int64_t> g_opt_decoder_graph{1};
 std::atomic<int64_t> g_opt_decoder_fused{1};
 
-// Whether a product with m rows of x goes to the matrix kernel in FP32 (under option gemv_tcgen05 = 1 up to 16 rows of Q4_K and Q5_K go to the
-// tcgen05 GEMV).
+// Whether a product with m rows of x goes to the matrix kernel in FP32 or, with up to 16 rows, to the rows kernel (under option gemv_tcgen05 = 1 up to 16
+// rows of Q4_K and Q5_K go to the tcgen05 GEMV).
 static bool to_matrix_kernel(const jq_weight* w, int64_t m) {
     return g_opt_gemv_generic.load() == 0 && matmul_takes(view_of(w), m) && !(m <= 16 && gemv_umma_takes(w->type, w->k, (int)m));
 }

@@ -80,7 +80,7 @@ constexpr int MAX_WEIGHTS = 3;
 struct Args {
     // Up to three weights of one format and k, whose tiles of features follow one another. Linears on one x (q, k and v; gate and up) leave
     // the chip partly idle one by one: 32 or 86 tiles of features on 148 SMs, each launch with a fill and a drain. Together: prompt of 512
-    // tokens, 8 layers of the 7B width, 2529 -> 2437 us; 16 sequences at the 70B width, 626 -> 588 us.
+    // tokens, 8 layers of the 7B width, 2529 -> 2437 us.
     const uint8_t* q[MAX_WEIGHTS];
     const uint8_t* aux[MAX_WEIGHTS];
     float* y[MAX_WEIGHTS];

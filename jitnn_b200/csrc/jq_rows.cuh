@@ -15,8 +15,10 @@
 // operand; a unit's part of the image is one contiguous copy. An accumulator holds 256 (two-part formats and Q5_K: 128) terms before its sums are
 // added up in registers, rounded to nearest: the tensor core cuts sums off towards zero.
 //
-// Roles: warp 0 brings in raw units, warp 2 the image, one bulk copy each; warp 1 issues the MMAs; warps 4 .. 11 add up (a warp may only read its
-// quarter of tensor memory's lanes; two share it, eight rows of x each); warps 12 .. 19 are two groups that turn raw units into operands in tensor memory (three of them), thread = row of W.
+// Roles: warp 0 brings in raw units, warp 2 the image, one bulk copy each; warp 1 issues the MMAs; warps 4 .. 3 + FOLD add up (a warp may only read its
+// quarter of tensor memory's lanes); the eight behind them are two groups that turn raw units into operands in tensor memory (three of them), thread =
+// row of W. Formats with one operand a unit (Q4_K, Q5_K): FOLD = 8, two warps share a quarter, eight rows of x each, and the groups take units in turn;
+// 640 threads. With two (Q6_K and the 32-element formats): FOLD = 4, a warp has its quarter's 16 rows of x, and each group makes its half of every unit; 512.
 //
 // k is cut into eight ranges whatever the grid is; a range's units are added up in order, then the ranges. So a row shard gives bitwise what the whole
 // weight gives, and a cluster of 2, 4 or 8 thread blocks may share the ranges (their sums meet through distributed shared memory) where there

@@ -195,9 +195,8 @@ def test_full_width_decoder(layers, dim, heads, kv_heads, hidden, formats, fused
 
 @pytest.mark.parametrize("layers,dim,heads,kv_heads,hidden", [(2, 4096, 32, 32, 11008), (1, 8192, 64, 8, 28672)])
 def test_full_width_decoder_twelve_tokens_per_call(layers, dim, heads, kv_heads, hidden):
-    """Twelve tokens in one call at the benchmark's widths, all Q4_K: from eleven rows on the linears whose weights have enough rows
-    go through the tcgen05 GEMV in one pass, wq / wk / wv and w1 / w3 as one launch each on one activation image, weights of few
-    128-row tiles with k cut into ranges; the others through the mma.sync kernel in two passes. Against the oracle, token by token."""
+    """Twelve tokens in one call at the benchmark's widths, all Q4_K: every linear goes through the rows kernel, wq / wk / wv and w1 / w3 together on one
+    image of x (at the 70B widths in two launches each, the one behind without a wait for the image). Against the oracle, token by token."""
     all_q4k = {"wv": "Q4_K", "w2": "Q4_K", "output": "Q4_K"}
     cfg = llama_oracle.Config(layers=layers, dim=dim, heads=heads, kv_heads=kv_heads, hidden=hidden, vocab=32000, max_seq=16)
     weights = llama_oracle.random_model(cfg, seed=dim // 32, formats=all_q4k)

@@ -6,7 +6,8 @@ hanging anything: two peer buffers are allocated on the same device as "rank 0" 
 ever calls. Its exchange stores its slice into its own y and, as marked words, into the other buffer's staging area, then waits
 for rank 1's words in its own staging area, which nothing writes: the wait gives up after its limit (option "peer_wait_us",
 0.4 s by default), records 32 + 1 and the kernel returns.
-The matrix kernel's waits run out by themselves under a limit of a microsecond ("wait_limit_us"): its first accumulator takes longer.
+The waits of the matrix kernel and of the rows kernel (9 rows of x, a decoder's 16 sequences) run out by themselves under a limit of a microsecond
+("wait_limit_us"): their first accumulator takes longer.
 After a timeout the ranks' exchange numbers on those buffers are out of step: the buffers are to be freed and allocated anew
 (jq_peer_free / jq_peer_alloc), which is what the test does before it checks that the device still works.
 """
@@ -140,7 +141,7 @@ def gives_up(call):
 
 
 def test_the_matrix_kernel_gives_up(short_waits):
-    """Host calls report their own waits, and nobody else's; calls with device memory leave a code for jq_device_status."""
+    """Host calls report their own waits, and nobody else's; calls with device memory leave a code for jq_device_status. (Nine rows: the rows kernel.)"""
     L = short_waits
     n, k, m = 11008, 4096, 200
     w = Tensor.quantized("Q4_0", synth.random_valid_blocks("Q4_0", n, k, seed=2).numpy().reshape(-1), n, k)
