@@ -453,11 +453,12 @@ int launch_matmul_f32_multi(const View* vs, int count, const float* x, int64_t m
     return mm::product_f32(vs, count, false, x, nullptr, m, nullptr, ys, s);
 }
 
-// More than 16 rows of x always: the weight is read once for all of them. Up to 16 rows (the rows kernel's) take the same time as one, so the line lies
-// where the decode kernels need another pass. Measured with 4096 and 32000 output rows, k = 4096, last row count in front of the line / first behind it / the
-// rows kernel, us: Q4_K (8 rows in a pass) 6.9 / 11.2 / 9.0 and 24.3 / 38.8 / 24.4; Q5_K 7.2 / 12.5 / 10.6 and 26.5 / 43.8 / 34.9; Q6_K (4) 8.2 / 14.4 / 11.5
-// and 33.9 / 55.3 / 41.2; the 32-element formats (2; the third pass) Q8_0 10.0 / 14.4 / 12.0 and 47.4 / 70.5 / 41.6, Q4_0 9.1 / 13.5 / 10.6 and 31.8 / 45.2 / 37.2,
-// Q4_1 9.6 / 14.6 / 11.1 and 33.2 / 48.7 / 43.1. K-quants with k = 1024 alike: Q4_K 5.0 / 7.2 / 5.7 and 15.1 / 21.6 / 9.9, Q5_K 5.2 / 7.4 / 7.0 and 15.6 / 23.1 / 11.9.
+// More than 16 rows of x always: the weight is read once for all of them. Up to 16 rows (the rows kernel's) take the time of 8 or of 16, so the line lies where
+// the decode kernels need another pass. Measured with 4096 and 32000 output rows, k = 4096, last row count in front of the line / first behind it / the
+// rows kernel, us: Q4_K (8 rows in a pass) 6.9 / 11.2 / 9.0 and 24.3 / 38.8 / 24.4; Q5_K 7.2 / 12.5 / 10.6 and 26.5 / 43.8 / 33.4; Q6_K (4) 7.6 / 14.4 / 9.4
+// and 33.8 / 55.3 / 32.1; the 32-element formats (2) Q8_0 4.7 / 9.2 / 8.4 and 23.4 / 46.8 / 25.7, Q4_0 4.6 / 8.8 / 8.2 and 16.2 / 31.1 / 23.8, Q4_1 4.4 / 8.6 / 8.8
+// and 17.0 / 32.8 / 27.7. With k = 1024 alike: Q4_K 5.0 / 7.2 / 5.7 and 15.1 / 21.6 / 9.9, Q8_0 with 1024 output rows 3.1 / 5.8 / 5.9. (Q4_K from 3 to 8 rows, both us,
+// the decode kernel 6.8 and 25.0, the rows kernel 8.0 and 21.8: that crosses with the number of output rows.)
 // The line must not depend on the number of output rows, and neither do the sums, so a row shard gives bitwise the outputs of the whole weight.
 // Where the decode kernels decline (k no multiple of 256, or too wide) there is only the CUDA-core kernel besides, whose time grows with rows x k and
 // with the output rows. At 4096 of them the rows kernel is the faster one from a little less on than the lines below say: Q8_0 k = 288 from 5 rows (5.6 us
@@ -474,7 +475,7 @@ bool matmul_takes(const View& v, int64_t rows) {
         return rows >= 5;
     }
     if (gemv_blk32_i8_scratch_bytes(v.type, v.k, rows < 2 ? 1 : 2) > 0) {
-        return rows >= 5;
+        return rows >= (v.k <= 28672 ? 3 : 5);  // (a wider k's image of x may need a larger scratch buffer than calls with one or two rows have left)
     }
     return rows * v.k >= (v.type == JQ_TYPE_Q8_0 ? 4096 : 2048);
 }

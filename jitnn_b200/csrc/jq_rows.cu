@@ -7,10 +7,12 @@ namespace rows {
 
 // x [m, k] FP32 (or silu(x) * up) -> per 256-wide step of k its image (jq_rows.cuh) and a scale per row: the row's 256 values times a power of two that
 // brings the largest to [2^9, 2^10), hi = that rounded to half precision, lo = the rest rounded to half precision: 22 significant bits for
-// everything down to 2^-13 of the largest. A row's 256 that hold a NaN or an Inf get the scale NaN, which reaches every output of that row. One
+// everything down to 2^-13 of the largest. NT: 8 or 16 rows. A row's 256 that hold a NaN or an Inf get the scale NaN, which reaches every output of that row. One
 // warp per row and step, eight values a lane; rows from m on are zeros. Memory bound: 4 bytes read and 4.5 written (to L2) a value.
+template <int NT>
 __global__ void __launch_bounds__(128) image_kernel(const float* __restrict__ x, const float* __restrict__ up, int m, int64_t k, int units, uint8_t* __restrict__ image,
                                                     float* __restrict__ scales, int vec) {
+    constexpr int N = 2 * NT, STEP = step_bytes(NT);
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int64_t task = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -56,7 +58,7 @@ __global__ void __launch_bounds__(128) image_kernel(const float* __restrict__ x,
         sum += (h.x + l.x) + (h.y + l.y);
     }
     // lane = step of 16 and half of it; columns row (hi) and NT + row (lo), 128 bytes per eight columns
-    uint8_t* const unit = image + (int64_t)u * IMAGE;
+    uint8_t* const unit = image + (int64_t)u * image_bytes(NT);
     const int col = (row >> 3) * 128 + (row & 7) * 16;
     uint8_t* const to = unit + (lane >> 1) * STEP + (lane & 1) * (N * 16) + col;
     *reinterpret_cast<uint4*>(to) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
@@ -87,7 +89,10 @@ static int launch_any(int type, Args& a, int ctas, bool after, cudaStream_t s) {
     }
 }
 
-constexpr int SLOT = 8;  // scratch: image and scales
+// Scratch for image and scales. Up to four rows the slot is that of the decode kernels' images, so that a program that has made a call with one or two rows may
+// capture one with three or four (matmul_takes sends no wider k here than the slot's least size holds).
+constexpr int SLOT = 8;
+constexpr int slot_of(int m) { return m < 5 ? 0 : SLOT; }
 
 }  // namespace rows
 
@@ -101,12 +106,13 @@ int launch_rows(const View* vs, int count, const float* x, const float* up, int 
     uint8_t* image = nullptr;
     int rc = status_word(&status);
     if (rc == JQ_OK) {
-        rc = scratch_for_slot(s, SLOT, (size_t)units * (IMAGE + NT * sizeof(float)), &image);
+        rc = scratch_for_slot(s, slot_of(m), (size_t)units * (image_bytes(m < 5 ? 8 : MAX_NT) + MAX_NT * sizeof(float)), &image);
     }
     if (rc != JQ_OK) {
         return rc;
     }
-    float* const scales = reinterpret_cast<float*>(image + (size_t)units * IMAGE);
+    const int nt = m <= 8 ? 8 : 16;
+    float* const scales = reinterpret_cast<float*>(image + (size_t)units * image_bytes(nt));
     {
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
@@ -115,10 +121,10 @@ int launch_rows(const View* vs, int count, const float* x, const float* up, int 
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         cfg.stream = s;
-        cfg.gridDim = dim3((unsigned)((int64_t)units * NT / 4));
+        cfg.gridDim = dim3((unsigned)((int64_t)units * nt / 4));
         cfg.blockDim = dim3(128);
         const int vec = k % 4 == 0 && (((uintptr_t)x | (uintptr_t)up) & 15) == 0;
-        JQ_CUDA(cudaLaunchKernelEx(&cfg, image_kernel, x, up, m, k, units, image, scales, vec));
+        JQ_CUDA(cudaLaunchKernelEx(&cfg, nt == 8 ? image_kernel<8> : image_kernel<16>, x, up, m, k, units, image, scales, vec));
         count_launch();
     }
     for (int i = 0; i < count && rc == JQ_OK; i++) {

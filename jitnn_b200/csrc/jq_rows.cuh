@@ -1,24 +1,29 @@
 // The rows kernel: y[m, n] = x[m, k] . W[n, k]^T (+ bias) in FP32 for up to 16 rows of x on the 5th-generation tensor cores, every weight read once.
 //
 // What bounds it. At 6.5 TB/s an SM gets a unit of 128 rows x 256 k of Q4_K (18 KB) in 770 clocks. The tensor core needs 270 of them: an MMA of 128
-// weights' rows x 32 columns x 16 k whose weights lie in tensor memory takes 16 clocks. What is scarce is instructions: a unit is 64 KB of halves to
+// weights' rows x 32 columns x 16 k whose weights lie in tensor memory takes 16 clocks, one of 16 columns 9. What is scarce is instructions: a unit is 64 KB of halves to
 // be made by the warps, and with 1050 instructions per scheduler and unit, a fifth of the time without the next instruction at hand (long unrolled
-// code of five roles), the same product as an instance of the matrix kernel (jq_matmul.cuh) took 1800 clocks a unit. So the roles here are small loops,
-// and the weights are made with as few instructions as there are:
+// code of five roles), the same product as an instance of the matrix kernel (jq_matmul.cuh) took 1800 clocks a unit. So the weights are made with as few
+// instructions as there are:
 // * A quant in the low bits of a half IS the subnormal half q 2^-24: 1.1 logic operations a pair and one fused multiply-add that
 //   multiplies by the scale and takes off the middle of the quants' range, exactly (Q4_K, Q5_K: (q - 8) scale <= 1008 is a half). Bits 4 .. 7
 //   stay in place, as 16 q. The pairs are values 0 and 2, 1 and 3 of four; x's image has the same order.
 // * d and dmin go to the sums: the mins, times the sums of x over 32 values, have columns of their own in tensor memory.
-// * Formats whose products do not fit a half (Q6_K 13 bits, 32-element formats 15 to 18) have two: hi = scale q rounded, lo = the rest, exact.
+// * Where quant x scale does not fit a half (Q6_K 13 bits, 32-element formats 15 to 18) the operand is the quants alone, and every scale has an accumulator of
+//   its own: its 16 or 32 k times hi and lo of x, which the warps that add up multiply by the scale. Before, such a weight was two halves, hi = scale q rounded
+//   and lo = the rest: two instructions a pair and twice the stores to tensor memory more, for 16 (8) multiply-adds a row and 8 columns. 32000 x 4096, 8 and 16 rows, us:
+//   Q6_K 41.4 -> 32.2 and 42.0 -> 38.2, Q8_0 41.9 -> 26.0 and 42.4 -> 30.3, Q4_0 37.6 -> 23.9 and 38.4 -> 28.9, Q4_1 43.6 -> 27.9 and 44.6 -> 35.0; and the error
+//   against 64 bits, 2.0e-7 of the norm, is 1.1e-7, as a sum of 16 or 32 terms is all that the tensor core cuts off. Q6_K is still bound by its
+//   instructions (1180 per scheduler and unit with 8 rows, 0.55 of the issue slots; four groups of warps that make weights in place of two: 33.2).
 //
-// x is split into halves hi + lo, 22 bits a value, times a power of two per row and 256 values (image_kernel in jq_rows.cu): 16 + 16 columns of one B
-// operand; a unit's part of the image is one contiguous copy. An accumulator holds 256 (two-part formats and Q5_K: 128) terms before its sums are
-// added up in registers, rounded to nearest: the tensor core cuts sums off towards zero.
+// x is split into halves hi + lo, 22 bits a value, times a power of two per row and 256 values (image_kernel in jq_rows.cu): NT + NT columns of one B
+// operand, NT = 8 or 16 rows of x; a unit's part of the image is one contiguous copy, 8.5 or 17 KB. An accumulator of both hi and lo holds 256 (Q5_K: 128)
+// terms before its sums are added up in registers, rounded to nearest: the tensor core cuts sums off towards zero.
 //
-// Roles: warp 0 brings in raw units, warp 2 the image, one bulk copy each; warp 1 issues the MMAs; warps 4 .. 3 + FOLD add up (a warp may only read its
-// quarter of tensor memory's lanes); the eight behind them are two groups that turn raw units into operands in tensor memory (three of them), thread =
-// row of W. Formats with one operand a unit (Q4_K, Q5_K): FOLD = 8, two warps share a quarter, eight rows of x each, and the groups take units in turn;
-// 640 threads. With two (Q6_K and the 32-element formats): FOLD = 4, a warp has its quarter's 16 rows of x, and each group makes its half of every unit; 512.
+// Roles: warp 0 brings in raw units, warp 2 the image, one bulk copy each; warp 1 issues the MMAs; warps 4 .. 3 + FOLD add up, eight columns each (a warp may only
+// read its quarter of tensor memory's lanes): four with NT = 8, eight with 16; the eight behind them are two groups that turn raw units into operands in
+// tensor memory, thread = row of W. Q4_K, Q5_K: an operand is a unit, the groups take units in turn. The others: an operand is half a unit's k, and each group
+// makes its half of every unit. (The fold's loop over halves and the makers' loops are unrolled: as loops they were 3 to 6 % slower.)
 //
 // k is cut into eight ranges whatever the grid is; a range's units are added up in order, then the ranges. So a row shard gives bitwise what the whole
 // weight gives, and a cluster of 2, 4 or 8 thread blocks may share the ranges (their sums meet through distributed shared memory) where there
@@ -44,12 +49,12 @@ using mm::mul2;
 using mm::pack2;
 using mm::unpack2;
 
-constexpr int NT = 16, N = 32;       // rows of x, columns
 constexpr int RANGES = 8;
 constexpr int MAX_WEIGHTS = 3;
-constexpr int STEP = N * 32;         // bytes of 16 k of the image: [8 k][8 columns][8 rows of 16 bytes]
-constexpr int IMAGE = 17 * STEP;     // of a unit: 256 k, then the sums of x over its runs of 32, twice, as 16 more k
-constexpr int MAX_RAW = 6, MAX_IMG = 6, OPERANDS = 3, MAX_ACC = 4, FACTORS = 8;
+constexpr int MAX_NT = 16;           // NT: rows of x that an instance takes, 8 or 16; 2 NT columns
+__host__ __device__ constexpr int step_bytes(int nt) { return 2 * nt * 32; }         // 16 k of the image: [8 k][8 columns][8 rows of 16 bytes]
+__host__ __device__ constexpr int image_bytes(int nt) { return 17 * step_bytes(nt); }  // a unit: 256 k, then the sums of x over its runs of 32, twice, as 16 more k
+constexpr int MAX_RAW = 6, MAX_IMG = 6, MAX_OPERANDS = 4, MAX_ACC = 4, MAX_FACTORS = 8;
 
 struct Args {
     const uint8_t* q[MAX_WEIGHTS];
@@ -57,7 +62,7 @@ struct Args {
     float* y[MAX_WEIGHTS];
     int64_t n[MAX_WEIGHTS];
     int ft_end[MAX_WEIGHTS];  // tiles of 128 rows up to and including each weight
-    const uint8_t* image;     // [units][IMAGE]
+    const uint8_t* image;     // [units][image_bytes]
     const float* scales;      // [units][NT]
     const float* bias;        // of the first weight, or null
     int units, m;
@@ -104,9 +109,8 @@ __device__ __forceinline__ void mma(uint32_t d, uint32_t a, uint32_t b, uint32_t
         "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "r"((128u >> 4) | (1u << 14))  // 128 bytes between groups of 8 columns
         : "memory");
 }
-__device__ __forceinline__ uint32_t desc(uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | ((uint32_t)(N * 16) >> 4 << 16); }  // between the two halves of a step
-constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(128 >> 4) << 24);
-constexpr uint32_t ID_N = IDESC | ((uint32_t)(N >> 3) << 17), ID_NT = IDESC | ((uint32_t)(NT >> 3) << 17);
+__device__ __forceinline__ uint32_t desc(uint32_t addr, int n) { return ((addr & 0x3FFFFu) >> 4) | ((uint32_t)(n * 16) >> 4 << 16); }  // between the two halves of a step
+constexpr uint32_t idesc(int n) { return (1u << 4) | ((uint32_t)(128 >> 4) << 24) | ((uint32_t)(n >> 3) << 17); }
 
 constexpr uint32_t dup(uint32_t half_bits) { return half_bits * 0x10001u; }
 
@@ -128,12 +132,12 @@ __device__ __forceinline__ bool wait_all(volatile int* abort_flag, const Args& p
 }
 
 __device__ __forceinline__ void ld(float (&r)[8], uint32_t addr) { mm::ld_tmem8(r, addr); }
-__device__ __forceinline__ void ld(float (&r)[16], uint32_t addr) { mm::ld_tmem16(r, addr); }
 
 // ---- the formats -------------------------------------------------------------------------------------------------------------------
-// PARTS: operand values per weight; MINS: the sums of x have a part (what is the same for 32 weights, the middle of the quants and the min: 8 more columns
-// of an operand, the eight values' hi parts and lo parts, whose products have an accumulator of their own); HALVES: operands per unit; ACCS: accumulators per unit.
-// make(): operand `half` of the row's unit into this lane's columns from `to` on, and (with the first) what the fold multiplies the sums by into `fac`.
+// HALVES: operands per unit, each of 128 columns / HALVES; GROUP: consecutive k with one scale that the fold multiplies by, 0 where the scales are in the
+// operand; MINS: the sums of x have a part (what is the same for 32 weights, the middle of the quants and the min: 8 more columns of an operand, the eight
+// values' hi parts and lo parts, whose products have an accumulator of their own); ACCS: accumulators per unit, without GROUP.
+// make(): operand `half` of the row's unit into this lane's columns from `to` on, and what the fold multiplies the sums by into `fac`.
 template <int TYPE>
 struct Rw;
 
@@ -153,7 +157,7 @@ __device__ __forceinline__ float sums_part(const float (&e)[8], float bound, uin
 // Q4_K and Q5_K: values scale (q - mid) 2^-14.
 template <bool FIVE>
 struct RwK45 {
-    static constexpr int ROW = FIVE ? 176 : 144, AUX = 0, PARTS = 1, HALVES = 1, ACCS = FIVE ? 2 : 1;
+    static constexpr int ROW = FIVE ? 176 : 144, AUX = 0, HALVES = 1, GROUP = 0, ACCS = FIVE ? 2 : 1;
     static constexpr bool MINS = true;
     __device__ static __forceinline__ void make(uint32_t uq, uint32_t, int row, int, uint32_t to, uint32_t fac) {
         const uint32_t at = uq + (uint32_t)(row * ROW);
@@ -218,96 +222,70 @@ struct Rw<JQ_TYPE_Q4_K> : RwK45<false> {};
 template <>
 struct Rw<JQ_TYPE_Q5_K> : RwK45<true> {};
 
-// hi and lo of the products of two pairs of quants
-__device__ __forceinline__ void product(uint32_t q, uint32_t s, uint32_t& hi, uint32_t& lo) {
-    hi = hmul2(q, s);
-    lo = hfma2(q, s, hi ^ 0x80008000u);
-}
-
+// The other formats' products of quant and scale do not fit a half: the operand is the quants alone, and the sums over the k of one scale come out of the
+// tensor core one by one. fac: the scales of the half's groups (bytes or halves in .x and .y), .z what else the fold multiplies by.
 template <>
 struct Rw<JQ_TYPE_Q6_K> {
-    static constexpr int ROW = 208, AUX = 2, PARTS = 2, HALVES = 2, ACCS = 2;
+    static constexpr int ROW = 208, AUX = 2, HALVES = 2, GROUP = 16, ACCS = 2;
     static constexpr bool MINS = false;
     __device__ static __forceinline__ void make(uint32_t uq, uint32_t ua, int row, int half, uint32_t to, uint32_t fac) {
         const uint32_t at = uq + (uint32_t)(row * ROW), l = at + 64u * (uint32_t)half, h = at + 128u + 32u * (uint32_t)half;
         const uint32_t s0 = lds4(at + 192u + 8u * (uint32_t)half) ^ 0x80808080u, s1 = lds4(at + 196u + 8u * (uint32_t)half) ^ 0x80808080u;
         const uint32_t dw = lds4(ua + 4u * (uint32_t)(row >> 1));
-        if (half == 0) {
-            sts_pair(fac, half_bits_to_float((row & 1) != 0 ? dw >> 16 : dw), 0.0f);
-        }
-#pragma unroll 1
+        mm::sts16(fac, s0, s1, __float_as_uint(half_bits_to_float((row & 1) != 0 ? dw >> 16 : dw)), 0u);
+#pragma unroll
         for (int p = 0; p < 2; p++) {  // bytes 16 p .. 16 p + 15 of the half's runs of 32
             const uint4 qa = lds16(l + 16u * (uint32_t)p), qb = lds16(l + 32u + 16u * (uint32_t)p), qh = lds16(h + 16u * (uint32_t)p);
             const uint32_t wa[4] = {qa.x, qa.y, qa.z, qa.w}, wb[4] = {qb.x, qb.y, qb.z, qb.w}, wh[4] = {qh.x, qh.y, qh.z, qh.w};
-            // runs 0 .. 3: low nibbles of a and b, high nibbles of a and b; their scales are bytes p, p + 2, p + 4, p + 6
+            uint32_t q[4][8];  // runs 0 .. 3: low nibbles of a and b, high nibbles of a and b
+#pragma unroll
+            for (int x = 0; x < 4; x++) {
+#pragma unroll
+                for (int odd = 0; odd < 2; odd++) {
+                    const uint32_t a = wa[x] >> (8 * odd), b = wb[x] >> (8 * odd), t = wh[x] >> (8 * odd), t2 = t << 2, t4 = t << 4;
+                    const int i = 2 * x + odd;  // 1024 + q, and 1024 + 16 q; minus 32
+                    q[0][i] = hadd2(and_or(a, 0x000F000Fu, and_or(t4, 0x00300030u, 0x64006400u)), 0xE420E420u);
+                    q[1][i] = hadd2(and_or(b, 0x000F000Fu, and_or(t2, 0x00300030u, 0x64006400u)), 0xE420E420u);
+                    q[2][i] = hfma2(and_or(a, 0x00F000F0u, and_or(t4, 0x03000300u, 0x64006400u)), 0x2C002C00u, 0xD600D600u);
+                    q[3][i] = hfma2(and_or(b, 0x00F000F0u, and_or(t2, 0x03000300u, 0x64006400u)), 0x2C002C00u, 0xD600D600u);
+                }
+            }
 #pragma unroll
             for (int run = 0; run < 4; run++) {
-                const uint32_t pick = 0x4040u + 0x0101u * (uint32_t)(2 * (run & 1) + p);
-                const uint32_t s = hadd2(__byte_perm(run < 2 ? s0 : s1, 0x64646464u, pick), 0xE480E480u);  // 1024 + 128 + scale
-                uint32_t hi[8], lo[8];
-#pragma unroll
-                for (int x = 0; x < 4; x++) {
-#pragma unroll
-                    for (int odd = 0; odd < 2; odd++) {
-                        const uint32_t v = (run & 1 ? wb[x] : wa[x]) >> (8 * odd), b = wh[x] >> (8 * odd);
-                        uint32_t q;  // 1024 + q, and 1024 + 16 q; minus 32
-                        if (run < 2) {
-                            q = hadd2(and_or(v, 0x000F000Fu, and_or(run == 0 ? b << 4 : b << 2, 0x00300030u, 0x64006400u)), 0xE420E420u);
-                        } else {
-                            q = hfma2(and_or(v, 0x00F000F0u, and_or(run == 2 ? b << 4 : b << 2, 0x03000300u, 0x64006400u)), 0x2C002C00u, 0xD600D600u);
-                        }
-                        product(q, s, hi[2 * x + odd], lo[2 * x + odd]);
-                    }
-                }
-                const uint32_t col = to + (uint32_t)(16 * run) + 8u * (uint32_t)p;
-                mm::st_tmem8(col, hi);
-                mm::st_tmem8(col + 64, lo);
+                mm::st_tmem8(to + (uint32_t)(16 * run) + 8u * (uint32_t)p, q[run]);
             }
         }
     }
 };
 
-// The 32-element formats: block scales d' = d 2^-e in [2^4, 2^5) at the largest of the row's eight; the fold multiplies by 2^e.
 template <int TYPE>
 struct Rw32 {
     static constexpr bool Q8 = TYPE == JQ_TYPE_Q8_0, MINS = TYPE == JQ_TYPE_Q4_1;
-    static constexpr int ROW = Q8 ? 256 : 128, AUX = MINS ? 32 : 16, PARTS = 2, HALVES = 2, ACCS = 2;
+    static constexpr int ROW = Q8 ? 256 : 128, AUX = MINS ? 32 : 16, HALVES = 2, GROUP = 32, ACCS = 2;
     __device__ static __forceinline__ void make(uint32_t uq, uint32_t ua, int row, int half, uint32_t to, uint32_t fac) {
         const uint32_t at = uq + (uint32_t)(row * ROW), au = ua + (uint32_t)(row * AUX);
-        const uint4 d0 = lds16(au), d1 = MINS ? lds16(au + 16) : d0;
-        uint32_t ds[4];  // the eight d
         if constexpr (MINS) {
-            ds[0] = __byte_perm(d0.x, d0.y, 0x5410), ds[1] = __byte_perm(d0.z, d0.w, 0x5410), ds[2] = __byte_perm(d1.x, d1.y, 0x5410), ds[3] = __byte_perm(d1.z, d1.w, 0x5410);
-        } else {
-            ds[0] = d0.x, ds[1] = d0.y, ds[2] = d0.z, ds[3] = d0.w;
-        }
-        const uint32_t e = mm::scale_exponent(mm::max_half8(make_uint4(ds[0], ds[1], ds[2], ds[3])));
-        const float inv = __uint_as_float((258u - e) << 23);  // 2^(4 + 127 - e)
-        // (the second half's group knows the sums' part, the first half's has to know its factor)
-        float bound = 0.0f;
-        if constexpr (MINS) {
-            const uint32_t a[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
-            float c[8];  // 8 d + m
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                c[i] = fmaf(8.0f, half_bits_to_float(a[i]), half_bits_to_float(a[i] >> 16));
-                bound = fmaxf(bound, fabsf(c[i]));
-            }
+            const uint4 d0 = lds16(au), d1 = lds16(au + 16);
+            uint32_t f1 = 0;
             if (half == 1) {
-                sums_part(c, bound, to + 128);
+                const uint32_t a[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+                float c[8], bound = 0.0f;  // 8 d + m
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    c[i] = fmaf(8.0f, half_bits_to_float(a[i]), half_bits_to_float(a[i] >> 16));
+                    bound = fmaxf(bound, fabsf(c[i]));
+                }
+                f1 = __float_as_uint(sums_part(c, bound, to + 64));
             }
+            const uint4 d = half ? d1 : d0;
+            mm::sts16(fac, __byte_perm(d.x, d.y, 0x5410), __byte_perm(d.z, d.w, 0x5410), f1, 0u);
+        } else {
+            const uint4 d = lds16(au);
+            mm::sts16(fac, half ? d.z : d.x, half ? d.w : d.y, 0u, 0u);
         }
-        if (half == 0) {
-            const uint32_t ex = min(max(__float_as_uint(bound) >> 23, 40u), 250u);
-            sts_pair(fac, __uint_as_float((e - 4u) << 23), __uint_as_float((ex - 13u) << 23));
-        }
-        const uint32_t dp[2] = {half ? ds[2] : ds[0], half ? ds[3] : ds[1]};
-#pragma unroll 1
+#pragma unroll
         for (int b = 0; b < 4; b++) {  // blocks of 32 of the half
-            const uint32_t dw = b < 2 ? dp[0] : dp[1];
-            const uint32_t s = mm::h2_dup(half_bits_to_float((b & 1) != 0 ? dw >> 16 : dw) * inv);
-            const uint32_t col = to + 16u * (uint32_t)b;
-            uint32_t hi[8], lo[8];
+            uint32_t v[16];
             if constexpr (Q8) {
 #pragma unroll
                 for (int c = 0; c < 2; c++) {
@@ -316,30 +294,23 @@ struct Rw32 {
 #pragma unroll
                     for (int x = 0; x < 4; x++) {
                         const uint32_t u = w[x] ^ 0x80808080u;  // q + 128 under 0x64: 1024 + that
-                        product(hadd2(__byte_perm(u, 0x64646464u, 0x4240), 0xE480E480u), s, hi[2 * x], lo[2 * x]);
-                        product(hadd2(__byte_perm(u, 0x64646464u, 0x4341), 0xE480E480u), s, hi[2 * x + 1], lo[2 * x + 1]);
+                        v[8 * c + 2 * x] = hadd2(__byte_perm(u, 0x64646464u, 0x4240), 0xE480E480u);
+                        v[8 * c + 2 * x + 1] = hadd2(__byte_perm(u, 0x64646464u, 0x4341), 0xE480E480u);
                     }
-                    mm::st_tmem8(col + 8u * (uint32_t)c, hi);
-                    mm::st_tmem8(col + 8u * (uint32_t)c + 64u, lo);
                 }
             } else {
                 const uint4 q = lds16(at + 16u * (uint32_t)swizzle_piece(4 * half + b, row));
                 const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-                for (int c = 0; c < 2; c++) {  // low nibbles, high nibbles: 1024 + q, 1024 + 16 q; minus 8
-#pragma unroll
-                    for (int x = 0; x < 4; x++) {
-#pragma unroll
-                        for (int odd = 0; odd < 2; odd++) {
-                            const uint32_t v = w[x] >> (8 * odd);
-                            const uint32_t n = c == 0 ? hadd2(and_or(v, 0x000F000Fu, 0x64006400u), 0xE408E408u) : hfma2(and_or(v, 0x00F000F0u, 0x64006400u), 0x2C002C00u, 0xD480D480u);
-                            product(n, s, hi[2 * x + odd], lo[2 * x + odd]);
-                        }
-                    }
-                    mm::st_tmem8(col + 8u * (uint32_t)c, hi);
-                    mm::st_tmem8(col + 8u * (uint32_t)c + 64u, lo);
+                for (int x = 0; x < 4; x++) {  // low nibbles, high nibbles: 1024 + q, 1024 + 16 q; minus 8
+                    const uint32_t u = w[x] >> 8;
+                    v[2 * x] = hadd2(and_or(w[x], 0x000F000Fu, 0x64006400u), 0xE408E408u);
+                    v[2 * x + 1] = hadd2(and_or(u, 0x000F000Fu, 0x64006400u), 0xE408E408u);
+                    v[8 + 2 * x] = hfma2(and_or(w[x], 0x00F000F0u, 0x64006400u), 0x2C002C00u, 0xD480D480u);
+                    v[8 + 2 * x + 1] = hfma2(and_or(u, 0x00F000F0u, 0x64006400u), 0x2C002C00u, 0xD480D480u);
                 }
             }
+            st_tmem16(to + 16u * (uint32_t)b, v);
         }
     }
 };
@@ -350,38 +321,47 @@ struct Rw<JQ_TYPE_Q4_0> : Rw32<JQ_TYPE_Q4_0> {};
 template <>
 struct Rw<JQ_TYPE_Q4_1> : Rw32<JQ_TYPE_Q4_1> {};
 
-// Tensor memory: accumulators (32 columns each, then 16 each for the mins' sums), behind them the operands.
-template <int TYPE>
+// Tensor memory: slots of accumulators, then those of the mins' sums (16 columns each), behind them the operands. Without GROUP a slot is one
+// accumulator of N columns, hi and lo; with it, the accumulators of an operand's groups, 16 columns each: an MMA with the hi columns and one with the lo
+// columns of x add to the same. (An MMA of 128 rows has at least 16 columns: with NT = 8 the upper eight are whatever lies behind in the image, and not read.)
+template <int TYPE, int NT>
 struct Shape {
     using F = Rw<TYPE>;
     static constexpr int UNIT_Q = 128 * F::ROW, UNIT_A = 128 * F::AUX, UNIT = UNIT_Q + UNIT_A;
-    static constexpr int A_COLS = 128 + (F::MINS ? 8 : 0);
-    static constexpr int ACC = F::MINS ? 2 : 4, ACC_COLS = ACC * (N + (F::MINS ? NT : 0));  // accumulators
-    static_assert(F::ACCS / F::HALVES == 1 || ACC == 2, "");
-    static_assert(ACC_COLS + OPERANDS * A_COLS <= 512, "tensor memory");
-    static constexpr int GROUPS = 2, FOLD = F::HALVES == 1 ? 8 : 4, THREADS = (4 + FOLD + 4 * GROUPS) * 32;  // warps that make weights (groups of four), that add up
-    static constexpr int C = NT / (FOLD / 4);  // columns (rows of x) of a fold warp
+    static constexpr int N = 2 * NT, STEP = step_bytes(NT), IMAGE = image_bytes(NT);
+    static constexpr bool GROUPED = F::GROUP > 0;
+    static constexpr int A_COLS = 128 / F::HALVES + (F::MINS ? 8 : 0), OPERANDS = GROUPED ? 4 : 3;
+    static constexpr int PER_HALF = GROUPED ? 128 / F::GROUP : 0;  // groups of an operand
+    static constexpr int SLOT = GROUPED ? 16 * PER_HALF : N, ACC = !GROUPED || F::GROUP == 16 ? 2 : (F::MINS ? 3 : 4), MIN_ACC = F::MINS ? 2 : 0;
+    static constexpr int ACC_COLS = ACC * SLOT + MIN_ACC * 16;
+    static_assert(ACC_COLS + OPERANDS * A_COLS <= 512 && OPERANDS <= MAX_OPERANDS && ACC <= MAX_ACC, "tensor memory");
+    static constexpr int FACTORS = GROUPED ? 4 : 8, FAC_HALF = GROUPED ? 2048 : 1024, FAC = GROUPED ? 2 * FAC_HALF : FAC_HALF;  // units whose factors are kept, bytes
+        static constexpr int GROUPS = 2, FOLD = NT / 2, THREADS = (4 + FOLD + 4 * GROUPS) * 32;  // warps that make weights (groups of four), that add up
+    static constexpr int C = 8;  // columns (rows of x) of a fold warp
+    static constexpr int SCALES = FOLD * 16 * C * 4;  // bytes of the fold warps' scales of x
+    static constexpr int TAIL = FACTORS * FAC + SCALES + 1024;  // and barriers
 };
-constexpr int TAIL = FACTORS * 128 * 8 + 4 * 1024 + 1024;  // factors, the fold warps' scales of x, barriers
-constexpr int part_bytes(int ksplit) { return ksplit > 1 ? RANGES / ksplit * NT * 512 : 0; }
+constexpr int part_bytes(int ksplit, int nt) { return ksplit > 1 ? RANGES / ksplit * nt * 512 : 0; }
 
 // AFTER: another launch of the same product is in front. A product may be cut by tiles into several launches, which read and write nothing of each
 // other's: the one behind starts as SMs become free, without waiting for the one in front, once that one knows that x's image is complete. It ends
 // after it, though, so whoever waits for the last waits for all. What it reads of the image kernel's work is in L2 by then (that kernel had ended before the
 // launch in front let this one start), and it reads it there: the image by bulk copies, the scales past L1. (Past L1 in every launch: Q4_K 32000 x 4096, 16
 // rows 24.6 -> 25.2 us, as eight warps of every SM read the same lines.)
-template <int TYPE, bool AFTER>
-__global__ void __launch_bounds__((Shape<TYPE>::THREADS), 1) rows_kernel(const __grid_constant__ Args p) {
+template <int TYPE, int NT, bool AFTER>
+__global__ void __launch_bounds__((Shape<TYPE, NT>::THREADS), 1) rows_kernel(const __grid_constant__ Args p) {
     using F = Rw<TYPE>;
-    using S = Shape<TYPE>;
-    constexpr int GROUPS = S::GROUPS, FOLD = S::FOLD, THREADS = S::THREADS, C = S::C;
+    using S = Shape<TYPE, NT>;
+    constexpr int GROUPS = S::GROUPS, FOLD = S::FOLD, THREADS = S::THREADS, C = S::C, N = S::N, STEP = S::STEP, IMAGE = S::IMAGE;
+    constexpr int OPERANDS = S::OPERANDS, FACTORS = S::FACTORS;
+    constexpr bool GROUPED = S::GROUPED;
     extern __shared__ uint8_t smem_unaligned[];
     const uint32_t base = (tc::smem_u32(smem_unaligned) + 127u) & ~127u;  // sums of this thread block's ranges (ksplit > 1), then the rings
     const uint32_t img0 = base + (uint32_t)(p.ksplit > 1 ? RANGES / p.ksplit * NT * 512 : 0), raw0 = img0 + (uint32_t)(p.img * IMAGE), fac0 = raw0 + (uint32_t)(p.raw * S::UNIT);
-    const uint32_t scl0 = fac0 + FACTORS * 128 * 8, bars = scl0 + 4 * 1024;
+    const uint32_t scl0 = fac0 + FACTORS * S::FAC, bars = scl0 + S::SCALES;
     const uint32_t img_full = bars, img_free = img_full + 8 * MAX_IMG, raw_full = img_free + 8 * MAX_IMG, raw_free = raw_full + 8 * MAX_RAW;
-    const uint32_t full_a = raw_free + 8 * MAX_RAW, free_a = full_a + 8 * OPERANDS, acc_full = free_a + 8 * OPERANDS, acc_free = acc_full + 8 * MAX_ACC;
-    const uint32_t fac_full = acc_free + 8 * MAX_ACC, slot_s = fac_full + 8 * FACTORS;
+    const uint32_t full_a = raw_free + 8 * MAX_RAW, free_a = full_a + 8 * MAX_OPERANDS, acc_full = free_a + 8 * MAX_OPERANDS, acc_free = acc_full + 8 * MAX_ACC;
+    const uint32_t fac_full = acc_free + 8 * MAX_ACC, slot_s = fac_full + 8 * MAX_FACTORS;
     uint8_t* const generic = smem_unaligned + (slot_s - tc::smem_u32(smem_unaligned));
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(generic);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(generic + 4);
@@ -408,7 +388,7 @@ __global__ void __launch_bounds__((Shape<TYPE>::THREADS), 1) rows_kernel(const _
             tc::mbar_init(acc_full + 8 * i, 1);
             tc::mbar_init(acc_free + 8 * i, FOLD);
         }
-        for (int i = 0; i < FACTORS; i++) {
+        for (int i = 0; i < MAX_FACTORS; i++) {
             tc::mbar_init(fac_full + 8 * i, 4);
         }
         *abort_flag = 0;
@@ -428,7 +408,7 @@ __global__ void __launch_bounds__((Shape<TYPE>::THREADS), 1) rows_kernel(const _
         asm volatile("griddepcontrol.launch_dependents;");
     }
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
-    const uint32_t tmem_m = tmem + S::ACC * N, tmem_a = tmem + S::ACC_COLS;
+    const uint32_t tmem_m = tmem + S::ACC * S::SLOT, tmem_a = tmem + S::ACC_COLS;
 
     auto weight_of = [&](int ft, int& ft0) {
         const int w = ft < p.ft_end[0] ? 0 : (ft < p.ft_end[1] ? 1 : 2);
@@ -490,7 +470,7 @@ __global__ void __launch_bounds__((Shape<TYPE>::THREADS), 1) rows_kernel(const _
     } else if (warp == 1) {
         // ---- MMAs: an operand's in one go (an election between them costs as much as several). What the next operand needs is asked for before they are
         // issued: an answer takes 200 clocks, with those of all polls together, and by then it is mostly yes.
-        constexpr int BUFS = F::ACCS / F::HALVES, STEPS = 16 / F::HALVES;  // accumulators and steps of 16 k of an operand
+        constexpr int BUFS = F::ACCS / F::HALVES, STEPS = 16 / F::HALVES;  // slots of accumulators and steps of 16 k of an operand
         const int turns = (p.ftiles - p.first_ft - cluster_id + clusters - 1) / clusters * (u1 - u0) * F::HALVES;
         int a = 0, s = 0, buf = 0, half = 0;
         uint32_t pa = 0, ps = 0, pb = 1;
@@ -500,8 +480,8 @@ __global__ void __launch_bounds__((Shape<TYPE>::THREADS), 1) rows_kernel(const _
             Phase free[BUFS];
 #pragma unroll
             for (int i = 0; i < BUFS; i++) {
-                d[i] = tmem + (uint32_t)(buf * N);
-                dm = tmem_m + (uint32_t)(buf * NT);
+                d[i] = tmem + (uint32_t)(buf * S::SLOT);
+                dm = tmem_m + 16u * (uint32_t)(GROUPED ? (t >> 1) & 1 : buf);
                 d_bar[i] = acc_full + 8 * buf;
                 free[i] = Phase{acc_free + 8 * buf, pb, 5};
                 if (++buf == S::ACC) {
@@ -514,7 +494,7 @@ __global__ void __launch_bounds__((Shape<TYPE>::THREADS), 1) rows_kernel(const _
                 break;
             }
             tc::fence_after_sync();
-            const uint32_t img = desc(img0 + (uint32_t)(s * IMAGE)), ta = tmem_a + (uint32_t)(a * S::A_COLS), bd = img + (uint32_t)(half * STEPS * (STEP >> 4));
+            const uint32_t img = desc(img0 + (uint32_t)(s * IMAGE), N), ta = tmem_a + (uint32_t)(a * S::A_COLS), bd = img + (uint32_t)(half * STEPS * (STEP >> 4));
             const uint32_t a_bar = free_a + 8 * a, s_bar = img_free + 8 * s;
             const bool last = F::HALVES == 1 || half == 1;
             if (++a == OPERANDS) {
@@ -533,19 +513,35 @@ __global__ void __launch_bounds__((Shape<TYPE>::THREADS), 1) rows_kernel(const _
                 ready = tc::mbar_test(acc_free + 8 * (buf + 1), pb) && ready;
             }
             if (elect_one()) {
+                auto sums_of_x = [&]() {  // times the lo columns, then the hi columns
+                    mma(dm, ta + 128 / F::HALVES, img + 16 * (STEP >> 4) + NT, idesc(16), 0u);
+                    mma(dm, ta + 128 / F::HALVES, img + 16 * (STEP >> 4), idesc(16), 1u);
+                };
+                if constexpr (GROUPED) {
+                    constexpr int KS = F::GROUP / 16;  // steps of a group
 #pragma unroll
-                for (int i = 0; i < STEPS; i++) {
-                    const int b = i / (STEPS / BUFS);
-                    mma(d[b], ta + 8 * i, bd + i * (STEP >> 4), ID_N, i % (STEPS / BUFS) == 0 ? 0u : 1u);  // hi x (hi | lo)
-                    if constexpr (F::PARTS == 2) {
-                        mma(d[b] + NT, ta + 64 + 8 * i, bd + i * (STEP >> 4), ID_NT, 1u);  // lo x hi, beside the other small products
+                    for (int g = 0; g < S::PER_HALF; g++) {
+#pragma unroll
+                        for (int i = 0; i < 2 * KS; i++) {  // lo first, while the accumulator is small
+                            const int step = g * KS + i % KS;
+                            mma(d[0] + 16 * g, ta + 8 * step, bd + step * (STEP >> 4) + (i < KS ? NT : 0), idesc(16), i == 0 ? 0u : 1u);
+                        }
                     }
-                    if (F::MINS && i == STEPS - 1 && last) {
-                        mma(dm, ta + 128, img + 16 * (STEP >> 4) + (NT * 16 >> 4), ID_NT, 0u);
-                        mma(dm, ta + 128, img + 16 * (STEP >> 4), ID_NT, 1u);
+                    if (F::MINS && last) {
+                        sums_of_x();
                     }
-                    if ((i + 1) % (STEPS / BUFS) == 0) {
-                        tc::umma_commit(d_bar[b]);
+                    tc::umma_commit(d_bar[0]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < STEPS; i++) {
+                        const int b = i / (STEPS / BUFS);
+                        mma(d[b], ta + 8 * i, bd + i * (STEP >> 4), idesc(N), i % (STEPS / BUFS) == 0 ? 0u : 1u);  // (hi | lo)
+                        if (F::MINS && i == STEPS - 1) {
+                            sums_of_x();
+                        }
+                        if ((i + 1) % (STEPS / BUFS) == 0) {
+                            tc::umma_commit(d_bar[b]);
+                        }
                     }
                 }
                 tc::umma_commit(a_bar);
@@ -560,30 +556,29 @@ __global__ void __launch_bounds__((Shape<TYPE>::THREADS), 1) rows_kernel(const _
         const int group = (warp - 4 - FOLD) >> 2, row = (warp & 3) * 32 + lane;
         const uint32_t to0 = tmem_a + ((uint32_t)((warp & 3) * 32) << 16);
         const int units = (p.ftiles - p.first_ft - cluster_id + clusters - 1) / clusters * (u1 - u0);
-        // One operand per unit: the groups take units in turn, and places in the ring of raw units too (its depth is even), so no group tests a barrier
-        // that is a turn of the ring behind. Two: each group makes its half of every unit.
-        constexpr bool OWN = F::HALVES == 1;
-        int r = OWN ? group : 0, o = group;
+        // A group makes one operand (half) of every TAKE-th unit. Without halves the places in the ring of raw units go in turn too (its depth is even), so no
+        // group tests a barrier that is a turn of the ring behind.
+        constexpr int TAKE = GROUPS / F::HALVES;
+        const int half = group % F::HALVES;
+        int r = group / F::HALVES, o = group;
         uint32_t pr = 0, po = 1;
-        for (int unit = OWN ? group : 0; unit < units; unit += OWN ? GROUPS : 1) {
+        for (int unit = r; unit < units; unit += TAKE) {
             if (!(ok = wait_all(abort_flag, p, Phase{raw_full + 8 * r, pr, 6}, Phase{free_a + 8 * o, po, 1}))) {
                 break;
             }
             tc::fence_after_sync();
-            const int half = OWN ? 0 : group;
-            const uint32_t uq = raw0 + (uint32_t)(r * S::UNIT), fac = fac0 + (uint32_t)((unit & (FACTORS - 1)) * 1024 + row * 8);
+            const int slot = unit & (FACTORS - 1);
+            const uint32_t uq = raw0 + (uint32_t)(r * S::UNIT), fac = fac0 + (uint32_t)(slot * S::FAC + half * S::FAC_HALF + row * (GROUPED ? 16 : 8));
             F::make(uq, uq + S::UNIT_Q, row, half, to0 + (uint32_t)(o * S::A_COLS), fac);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             tc::fence_before_sync();
             __syncwarp();
             if (lane == 0) {
                 tc::mbar_arrive(full_a + 8 * o);
-                if (half == 0) {
-                    tc::mbar_arrive(fac_full + 8 * (unit & (FACTORS - 1)));
-                }
+                tc::mbar_arrive(fac_full + 8 * (slot * F::HALVES + half));
                 tc::mbar_arrive(raw_free + 8 * r);  // (all that was read of the unit has been used)
             }
-            if ((r += OWN ? GROUPS : 1) >= p.raw) {
+            if ((r += TAKE) >= p.raw) {
                 r -= p.raw;
                 pr ^= 1;
             }
@@ -644,26 +639,10 @@ __global__ void __launch_bounds__((Shape<TYPE>::THREADS), 1) rows_kernel(const _
                 for (int j = 0; j < C / 4; j++) {
                     x4[j] = lds16(xs + 16u * (uint32_t)j);
                 }
-                if (!(ok = wait_all(abort_flag, p, Phase{fac_full + 8 * (chunk & (FACTORS - 1)), (uint32_t)(chunk / FACTORS) & 1u, 6}, Phase{acc_full + 8 * buf, pb, 4}))) {
-                    break;
-                }
-                float f0, f1;
-                asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(f0), "=f"(f1) : "r"(fac0 + (uint32_t)((chunk & (FACTORS - 1)) * 1024 + lane_row * 8)));
-                const f2 ff0 = pack2(f0, f0), ff1 = pack2(f1, f1);
-#pragma unroll
-                for (int acc = 0; acc < F::ACCS; acc++) {
-                    if (acc > 0 && !(ok = mm::wait_warp<true>(acc_full + 8 * buf, pb, abort_flag, p, 4))) {
-                        break;
-                    }
-                    tc::fence_after_sync();
-                    float hi[C], lo[C], mn[C];
-                    ld(hi, tmem + lanes + (uint32_t)(buf * N + c0));
-                    ld(lo, tmem + lanes + (uint32_t)(buf * N + NT + c0));
-                    const bool mins = F::MINS && acc == F::ACCS - 1;
-                    if (mins) {
-                        ld(mn, tmem_m + lanes + (uint32_t)(buf * NT + c0));
-                    }
-                    mm::ld_tmem_done();
+                const int slot = chunk & (FACTORS - 1);
+                const uint32_t fac_phase = (uint32_t)(chunk / FACTORS) & 1u;
+                f2 t[C / 2];  // the unit's sums
+                auto took = [&]() {  // a slot's sums are in registers
                     tc::fence_before_sync();
                     __syncwarp();
                     if (lane == 0) {
@@ -673,21 +652,107 @@ __global__ void __launch_bounds__((Shape<TYPE>::THREADS), 1) rows_kernel(const _
                         buf = 0;
                         pb ^= 1;
                     }
+                };
+                if constexpr (GROUPED) {
+                    uint4 fc;
 #pragma unroll
-                    for (int j = 0; j < C / 4; j++) {
-                        const f2 sc[2] = {pack2(__uint_as_float(x4[j].x), __uint_as_float(x4[j].y)), pack2(__uint_as_float(x4[j].z), __uint_as_float(x4[j].w))};
+                    for (int i = 0; i < C / 2; i++) {
+                        t[i] = 0;
+                    }
 #pragma unroll
-                        for (int i = 2 * j; i < 2 * j + 2; i++) {
-                            f2 t = mul2(add2(pack2(hi[2 * i], hi[2 * i + 1]), pack2(lo[2 * i], lo[2 * i + 1])), ff0);
-                            if (mins) {
-                                t = fma2(pack2(mn[2 * i], mn[2 * i + 1]), ff1, t);
+                    for (int half = 0; half < 2; half++) {
+                        if (!(ok = wait_all(abort_flag, p, Phase{fac_full + 8 * (slot * 2 + half), fac_phase, 6}, Phase{acc_full + 8 * buf, pb, 4}))) {
+                            break;
+                        }
+                        tc::fence_after_sync();
+                        fc = lds16(fac0 + (uint32_t)(slot * S::FAC + half * S::FAC_HALF + lane_row * 16));
+                        float mn[C];
+#pragma unroll
+                        for (int part = 0; part < S::PER_HALF / 4; part++) {
+                            float v[4][C];
+#pragma unroll
+                            for (int g = 0; g < 4; g++) {
+                                ld(v[g], tmem + lanes + (uint32_t)(buf * S::SLOT + 16 * (4 * part + g) + c0));
                             }
-                            sum[i] = fma2(t, sc[i & 1], sum[i]);
+                            if (F::MINS && half == 1) {
+                                ld(mn, tmem_m + lanes + (uint32_t)((chunk & 1) * 16 + c0));
+                            }
+                            mm::ld_tmem_done();
+                            if (part == S::PER_HALF / 4 - 1) {
+                                took();
+                            }
+                            const uint32_t w = part == 0 ? fc.x : fc.y;
+#pragma unroll
+                            for (int g = 0; g < 4; g++) {
+                                float sc;
+                                if constexpr (F::GROUP == 16) {  // a byte + 128 in the mantissa of 2^23
+                                    sc = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540u + (uint32_t)g)) - 8388736.0f;
+                                } else {
+                                    const uint32_t bits = g < 2 ? fc.x : fc.y;
+                                    sc = half_bits_to_float(g % 2 != 0 ? bits >> 16 : bits);
+                                }
+                                const f2 s2 = pack2(sc, sc);
+#pragma unroll
+                                for (int i = 0; i < C / 2; i++) {
+                                    const f2 e = pack2(v[g][2 * i], v[g][2 * i + 1]);
+                                    t[i] = fma2(e, s2, t[i]);
+                                }
+                            }
+                        }
+                        if (F::MINS && half == 1) {
+                            const f2 f = pack2(__uint_as_float(fc.z), __uint_as_float(fc.z));
+#pragma unroll
+                            for (int i = 0; i < C / 2; i++) {
+                                t[i] = fma2(pack2(mn[2 * i], mn[2 * i + 1]), f, t[i]);
+                            }
+                        }
+                    }
+                    if constexpr (F::GROUP == 16) {
+                        const f2 f = pack2(__uint_as_float(fc.z), __uint_as_float(fc.z));
+#pragma unroll
+                        for (int i = 0; i < C / 2; i++) {
+                            t[i] = mul2(t[i], f);
+                        }
+                    }
+                } else {
+                    if (!(ok = wait_all(abort_flag, p, Phase{fac_full + 8 * slot, fac_phase, 6}, Phase{acc_full + 8 * buf, pb, 4}))) {
+                        break;
+                    }
+                    float f0, f1;
+                    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(f0), "=f"(f1) : "r"(fac0 + (uint32_t)(slot * S::FAC + lane_row * 8)));
+                    const f2 ff0 = pack2(f0, f0), ff1 = pack2(f1, f1);
+#pragma unroll
+                    for (int acc = 0; acc < F::ACCS; acc++) {
+                        if (acc > 0 && !(ok = mm::wait_warp<true>(acc_full + 8 * buf, pb, abort_flag, p, 4))) {
+                            break;
+                        }
+                        tc::fence_after_sync();
+                        float hi[C], lo[C], mn[C];
+                        ld(hi, tmem + lanes + (uint32_t)(buf * N + c0));
+                        ld(lo, tmem + lanes + (uint32_t)(buf * N + NT + c0));
+                        const bool mins = acc == F::ACCS - 1;
+                        if (mins) {
+                            ld(mn, tmem_m + lanes + (uint32_t)(buf * 16 + c0));
+                        }
+                        mm::ld_tmem_done();
+                        took();
+#pragma unroll
+                        for (int i = 0; i < C / 2; i++) {
+                            const f2 e = add2(pack2(hi[2 * i], hi[2 * i + 1]), pack2(lo[2 * i], lo[2 * i + 1]));
+                            t[i] = acc == 0 ? mul2(e, ff0) : fma2(e, ff0, t[i]);
+                            if (mins) {
+                                t[i] = fma2(pack2(mn[2 * i], mn[2 * i + 1]), ff1, t[i]);
+                            }
                         }
                     }
                 }
                 if (!ok) {
                     break;
+                }
+#pragma unroll
+                for (int j = 0; j < C / 4; j++) {
+                    sum[2 * j] = fma2(t[2 * j], pack2(__uint_as_float(x4[j].x), __uint_as_float(x4[j].y)), sum[2 * j]);
+                    sum[2 * j + 1] = fma2(t[2 * j + 1], pack2(__uint_as_float(x4[j].z), __uint_as_float(x4[j].w)), sum[2 * j + 1]);
                 }
                 if (u + 1 == v_end) {  // the end of a range
                     const int slot = v - range * (RANGES / p.ksplit);

@@ -10,8 +10,9 @@ namespace rows {
 // 4 or 8).
 inline int clusters_of(int ks) { return ks == 1 ? 148 : (ks == 2 ? 74 : (ks == 4 ? 33 : 15)); }
 
-// What a unit takes a thread block in nanoseconds, measured on 32000 x 4096.
-inline double unit_ns(int type) { return type == JQ_TYPE_Q4_K ? 630.0 : (type == JQ_TYPE_Q5_K ? 940.0 : (type == JQ_TYPE_Q4_0 ? 1040.0 : 1170.0)); }
+// What a unit takes a thread block in nanoseconds, 16 rows of x, measured on 32000 x 4096. Q4_0 and Q8_0 take 720 and 770, a little less than is said here,
+// and 8 rows of x a fifth less throughout: that would move a tile or two of shapes at a wave's edge from one launch to another, which gained nothing.
+inline double unit_ns(int type) { return type == JQ_TYPE_Q4_K ? 630.0 : (type == JQ_TYPE_Q5_K ? 870.0 : (type == JQ_TYPE_Q4_0 || type == JQ_TYPE_Q8_0 ? 830.0 : (type == JQ_TYPE_Q4_1 ? 915.0 : 1010.0))); }
 
 // A product's tiles in up to three launches, each with its own number of thread blocks per tile: whole waves first, then what is left, which alone would
 // leave most of the chip idle for a whole contraction, with its contraction split over clusters (57344 x 8192: 448 tiles are three waves and four

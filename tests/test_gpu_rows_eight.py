@@ -1,0 +1,96 @@
+"""The rows kernel with up to 8 rows of x, and the formats whose scales its sums are multiplied by, where they can go wrong.
+
+The reference is the product of the oracle's dequantised weights in double. x keeps 22 significant bits, products are exact, sums of at most 256 terms
+are taken by the tensor core: 2e-7 of the result's norm on ordinary weights, and 1e-5 leaves room for cancellation.
+"""
+import numpy as np
+import pytest
+import torch
+
+import jitnn_b200
+from conftest import LINEAR_TYPES
+from jitnn_b200 import Gguf, Tensor, device_status, synth
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+REL = 1e-5
+GROUPED = ["Q6_K", "Q8_0", "Q4_0", "Q4_1"]
+# One row of W; a second tile's first row; fewer units than ranges; clusters of 2, 4 and 8; two waves; two launches.
+SHAPES = [(1, 256), (129, 512), (128, 2816), (1024, 8192), (4096, 4096), (6400, 4096), (19000, 2048), (9500, 8192)]
+
+
+def product(t, n, k, seed):
+    raw = synth.random_valid_blocks(t, n, k, seed=seed).numpy().reshape(-1)
+    return raw, Tensor.quantized(t, raw, n, k), torch.from_numpy(oracle.dequantize(t, raw).reshape(n, k)).cuda().double()
+
+
+@pytest.mark.parametrize("n,k", SHAPES)
+@pytest.mark.parametrize("t", GROUPED)
+def test_up_to_eight_rows(t, n, k):
+    raw, w, wd = product(t, n, k, n)
+    b = torch.randn(n, generator=torch.Generator().manual_seed(n)).cuda()
+    for m in (3, 5, 8):
+        x = torch.randn(m, k, generator=torch.Generator().manual_seed(m)).cuda()
+        ref = x.double() @ wd.T + b.double()
+        y = Gguf.linear(x, w, b)
+        assert float((y.double() - ref).norm() / ref.norm()) <= REL
+        for _ in range(5):
+            assert torch.equal(Gguf.linear(x, w, b), y)
+        if n > 128:  # a row shard gives the bits of the whole weight, whatever its launches are
+            shard = Tensor.quantized(t, raw, n, k, rows=(0, n // 3))
+            assert torch.equal(Gguf.linear(x, shard, b[:n // 3]), y[:, :n // 3])
+            shard.release()
+    assert device_status(0) == 0
+
+
+@pytest.mark.parametrize("m", [8, 16])
+@pytest.mark.parametrize("t", GROUPED)
+def test_scales_of_every_size(t, m):
+    """Block scales from the smallest subnormal half to the largest half, side by side; each row of W is held against its own size."""
+    n, k = 200, 1024
+    raw = synth.random_valid_blocks(t, n, k, seed=5).numpy().reshape(n, -1).copy()
+    size = {"Q6_K": 210, "Q8_0": 34, "Q4_0": 18, "Q4_1": 20}[t]
+    blocks = raw.reshape(-1, size)
+    d = np.exp2(np.random.default_rng(2).uniform(-24, 15.9, blocks.shape[0])).astype(np.float16)
+    for at in {"Q6_K": [208], "Q8_0": [0], "Q4_0": [0], "Q4_1": [0, 2]}[t]:
+        blocks[:, at:at + 2] = d.view(np.uint8).reshape(-1, 2)
+    raw = raw.reshape(-1)
+    w, wd = Tensor.quantized(t, raw, n, k), torch.from_numpy(oracle.dequantize(t, raw).reshape(n, k)).cuda().double()
+    x = torch.randn(m, k, generator=torch.Generator().manual_seed(3)).cuda()
+    y, ref, size = Gguf.linear(x, w).double(), x.double() @ wd.T, (x.double() ** 2) @ (wd ** 2).T
+    assert float(((y - ref).abs() / size.sqrt()).max()) <= REL
+
+
+@pytest.mark.parametrize("t", LINEAR_TYPES)
+def test_nan_and_inf_reach_their_rows_alone(t):
+    n, k, m = 300, 1024, 8
+    _, w, wd = product(t, n, k, 3)
+    x = torch.randn(m, k, generator=torch.Generator().manual_seed(1)).cuda()
+    x[2, 17], x[7, 1000] = float("nan"), float("inf")
+    x[4] = 0.0
+    y = Gguf.linear(x, w)
+    bad = ~torch.isfinite(y)
+    assert bool(bad[2].all()) and bool(bad[7].all()) and bool((y[4] == 0).all())
+    rows = [r for r in range(m) if r not in (2, 7)]
+    ref = x[rows].double() @ wd.T
+    assert float((y[rows].double() - ref).norm() / ref.norm()) <= REL
+
+
+@pytest.mark.parametrize("t", ["Q8_0", "Q4_0", "Q4_1"])
+def test_three_rows_are_captured_after_a_call_with_one(t):
+    """The row count at which the kernel changes needs no scratch buffer that a call with one row has not left."""
+    n, k = 512, 28672
+    _, w, _ = product(t, n, k, 4)
+    stream = torch.cuda.Stream()
+    x = torch.randn(4, k, generator=torch.Generator().manual_seed(1)).cuda()
+    want = Gguf.linear(x, w)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        Gguf.linear(x[:1], w)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        y = Gguf.linear(x, w)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
