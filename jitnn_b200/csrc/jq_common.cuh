@@ -183,10 +183,10 @@ int decoder_peer_status(int* status);
 size_t q6k_image_bytes_one_row(int64_t k);
 int launch_gemv_q6k_i8_imaged(const View& v, const uint8_t* image, const float* bias, float* y, cudaStream_t s, bool* handled);
 // The same for Q6_K, rows <= 4.
-int launch_gemv_q6k_i8(const View& v, const float* x, int rows, const float* bias, float* y, cudaStream_t s, uint8_t* image, bool* handled);
+int launch_gemv_q6k_i8(const View& v, const float* x, int rows, const float* bias, float* y, cudaStream_t s, uint8_t* image, bool* handled, bool x_remote);
 size_t gemv_q6k_i8_scratch_bytes(int64_t k, int rows);
 // The same for Q8_0, Q4_0 and Q4_1 (jq_gemv_blk32_i8.cu): rows <= 2, k a multiple of 256.
-int launch_gemv_blk32_i8(const View& v, const float* x, int rows, const float* bias, float* y, cudaStream_t s, uint8_t* image, bool* handled);
+int launch_gemv_blk32_i8(const View& v, const float* x, int rows, const float* bias, float* y, cudaStream_t s, uint8_t* image, bool* handled, bool x_remote);
 size_t gemv_blk32_i8_scratch_bytes(int type, int64_t k, int rows);
 
 // Scratch memory of at least `bytes` on the current device, private to work enqueued on `s` (one buffer per

@@ -118,11 +118,11 @@ int launch_gemv(const View& v, const float* x, int rows, const float* bias, floa
     }
     if (v.type == JQ_TYPE_Q6_K && rows <= 4 && g_opt_gemv_generic.load(std::memory_order_relaxed) == 0) {
         bool handled = false;
-        const size_t need = gemv_q6k_i8_scratch_bytes(v.k, rows);
+        const size_t need = gemv_q6k_i8_scratch_bytes(v.k, rows);  // (asked for also where the kernel makes the image itself: later calls find the buffer)
         uint8_t* image = nullptr;
         int rc = need > 0 ? scratch_for(s, need, &image) : JQ_OK;
         if (rc == JQ_OK) {
-            rc = launch_gemv_q6k_i8(v, x, rows, bias, y, s, image, &handled);
+            rc = launch_gemv_q6k_i8(v, x, rows, bias, y, s, image, &handled, x_remote);
         }
         if (rc != JQ_OK || handled) {
             return rc;
@@ -135,7 +135,7 @@ int launch_gemv(const View& v, const float* x, int rows, const float* bias, floa
             uint8_t* image = nullptr;
             int rc = scratch_for(s, need, &image);
             if (rc == JQ_OK) {
-                rc = launch_gemv_blk32_i8(v, x, rows, bias, y, s, image, &handled);
+                rc = launch_gemv_blk32_i8(v, x, rows, bias, y, s, image, &handled, x_remote);
             }
             if (rc != JQ_OK || handled) {
                 return rc;

@@ -3,7 +3,8 @@
 //
 // The scheme of the Q4_K kernel (jq_gemv_q4k_i8.cu) with what these formats need. The activations become an image
 // first: per 256 values of k a power-of-two scale, 22-bit fixed point, three signed base-256 digits laid out as B
-// fragments of mma.sync.m16n8k32, column 3m + i = digit i of row m of x (one warp per 256 values, image_kernel).
+// fragments of mma.sync.m16n8k32, column 3m + i = digit i of row m of x (one warp per 256 values, in a kernel of its own or
+// in the GEMV's warps that need it).
 // The GEMV kernel streams 16 rows x 256 k at a time (8 blocks per row) through a per-warp cp.async ring:
 //   Q8_0  the int8 quants are the A operand as they are (s8 x s8 -> s32), read with one ldmatrix per block;
 //   Q4_0  one AND / one shift + AND per four weights widen the nibbles (u8 x s8); the offset, -8 * sum(x over the block),
@@ -20,6 +21,7 @@
 // (row shards are bitwise equal to the whole weight). Quant and scale planes are separate on the device (jq_formats.cuh), in tiled
 // order, so that a step is one contiguous run of each; its rows are stored swizzled by (row & 7), so that ldmatrix's eight row
 // reads fall into different banks.
+#include "jq_digits.cuh"
 #include "jq_formats.cuh"
 
 namespace jq {
@@ -92,23 +94,20 @@ struct Img {
     static_assert(PB % 16 == 0, "the image is copied in 16-byte pieces");
 };
 
-// One warp per (256 values of k, row of x). Lane = (block lane / 4, tt = lane % 4): the values 4tt..4tt+3 and
-// 16+4tt..16+4tt+3 of the block, which are the k-slots of that lane in the MMA's B fragment when the A fragment holds
-// the block's 32 quants in their natural order.
-constexpr int PREP_WARPS = 4;
+// Lane = (block lane / 4, tt = lane % 4) of 256 values of x: the values 4tt..4tt+3 and 16+4tt..16+4tt+3 of the block, which are the k-slots of that lane in the
+// MMA's B fragment when the A fragment holds the block's 32 quants in their natural order.
+__device__ __forceinline__ void load_x(const float* x256, int lane, float (&xv)[8]) {
+    const float* xb = x256 + (lane >> 2) * 32 + 4 * (lane & 3);
+    const float4 lo = *reinterpret_cast<const float4*>(xb), hi = *reinterpret_cast<const float4*>(xb + 16);
+    xv[0] = lo.x; xv[1] = lo.y; xv[2] = lo.z; xv[3] = lo.w;
+    xv[4] = hi.x; xv[5] = hi.y; xv[6] = hi.z; xv[7] = hi.w;
+}
+
+// One warp makes the part of row m of x (given: it is one of the call's rows; else all zero) in the image of 256 values at `img` (global or shared memory).
 template <int MT>
-__global__ void __launch_bounds__(PREP_WARPS * 32) blk32_image_kernel(const float* __restrict__ x, int rows, int64_t k, uint8_t* __restrict__ image) {
+__device__ __forceinline__ void build_image(const float (&xv)[8], bool given, int m, uint8_t* img, int lane) {
     using I = Img<MT>;
-    asm volatile("griddepcontrol.launch_dependents;");  // the GEMV kernel may start requesting weights now
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // x is complete, and the GEMV before this one is done with the scratch image
-    const int lane = threadIdx.x & 31;
-    const int pair = blockIdx.x * PREP_WARPS + (threadIdx.x >> 5);
-    const int b = pair / MT, m = pair % MT;
-    if (b >= (int)(k >> 8)) {
-        return;
-    }
     const int blk = lane >> 2, tt = lane & 3;
-    uint8_t* img = image + (size_t)b * I::PB;
     uint2* xd = reinterpret_cast<uint2*>(img);
     float* xs = reinterpret_cast<float*>(img + I::XD);
     float* tab = reinterpret_cast<float*>(img + I::XD + I::XS);
@@ -119,69 +118,46 @@ __global__ void __launch_bounds__(PREP_WARPS * 32) blk32_image_kernel(const floa
             xs[j * 8 + lane] = 0.0f;
         }
     }
-    float xv[8];
-    if (m < rows) {
-        const float* xb = x + (int64_t)m * k + (int64_t)b * 256 + blk * 32 + 4 * tt;
-        const float4 lo = __ldg(reinterpret_cast<const float4*>(xb)), hi = __ldg(reinterpret_cast<const float4*>(xb + 16));
-        xv[0] = lo.x; xv[1] = lo.y; xv[2] = lo.z; xv[3] = lo.w;
-        xv[4] = hi.x; xv[5] = hi.y; xv[6] = hi.z; xv[7] = hi.w;
-    } else {
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            xv[i] = 0.0f;
-        }
-    }
-    float am = 0.0f;
-    bool bad = false;  // a NaN or an Inf among the values: the column weights become NaN and with them every output of this row of x
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        am = fmaxf(am, fabsf(xv[i]));
-        bad = bad || (__float_as_uint(xv[i]) & 0x7f800000u) == 0x7f800000u;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
-    }
-    bad = __any_sync(0xffffffffu, bad);
-    // s = 2^floor(log2(amax)): the largest |x| / s of the 256 values lies in [1, 2)
-    uint32_t e = __float_as_uint(am) & 0x7f800000u;
-    e = e < 0x0c000000u ? 0x0c000000u : (e > 0x7e800000u ? 0x7e800000u : e);  // keeps 2^21 / s and s * 2^-21 normal
-    const float inv = __uint_as_float(0x7f000000u - e + (21u << 23));           // 2^21 / s: |X| <= 2^22
-    int X[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        X[i] = __float2int_rn(xv[i] * inv);
-    }
+    bool bad;  // the column weights then become NaN and with them every output of this row of x
+    const uint32_t e = image_exponent(xv, 0x0c000000u, bad);
+    uint32_t dw[3][2];
+    image_digits(xv, e, dw);
 #pragma unroll
     for (int dgt = 0; dgt < 3; dgt++) {
-        uint32_t w0 = 0, w1 = 0;
-        int sum = 0;
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int d = dgt == 2 ? X[i] : (int)(int8_t)(X[i] & 0xff);  // signed low byte
-            X[i] = (X[i] - d) >> 8;
-            sum += d;
-            if (i < 4) {
-                w0 |= (uint32_t)(d & 0xff) << (8 * i);
-            } else {
-                w1 |= (uint32_t)(d & 0xff) << (8 * (i - 4));
-            }
-        }
+        int sum = digit_sum(dw[dgt]);
         const int col = 3 * m + dgt;
-        xd[((((size_t)(blk >> 1)) * I::COLS + col) * 4 + tt) * 2 + (blk & 1)] = make_uint2(w0, w1);
+        xd[((((size_t)(blk >> 1)) * I::COLS + col) * 4 + tt) * 2 + (blk & 1)] = make_uint2(dw[dgt][0], dw[dgt][1]);
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);
         sum += __shfl_xor_sync(0xffffffffu, sum, 2);
         if (tt == 0) {
             xs[blk * 8 + col] = (float)sum;  // |sum| <= 32 * 128: exact
         }
         if (lane == 0) {
-            tab[col] = m >= rows ? 0.0f : (bad ? __uint_as_float(0x7fc00000u) : __uint_as_float(e + ((uint32_t)(8 * dgt) << 23) - (21u << 23)));  // s * 2^(8 dgt - 21)
+            tab[col] = !given ? 0.0f : (bad ? __uint_as_float(0x7fc00000u) : __uint_as_float(e + ((uint32_t)(8 * dgt) << 23) - (21u << 23)));  // s * 2^(8 dgt - 21)
         }
     }
 }
 
-template <int TYPE, int MT, int STAGES>
-__global__ void __launch_bounds__(THREADS, 2) gemv_blk32_i8_kernel(View v, const uint8_t* __restrict__ image, int rows, const float* __restrict__ bias,
+// One warp per (256 values of k, row of x).
+constexpr int PREP_WARPS = 4;
+template <int MT>
+__global__ void __launch_bounds__(PREP_WARPS * 32) blk32_image_kernel(const float* x, int rows, int64_t k, uint8_t* __restrict__ image) {
+    asm volatile("griddepcontrol.launch_dependents;");  // the GEMV kernel may start requesting weights now
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // x is complete, and the GEMV before this one is done with the scratch image
+    const int pair = blockIdx.x * PREP_WARPS + (threadIdx.x >> 5);
+    const int b = pair / MT, m = pair % MT;
+    if (b < (int)(k >> 8)) {
+        float xv[8] = {};
+        if (m < rows) {
+            load_x(x + (int64_t)m * k + (int64_t)b * 256, threadIdx.x & 31, xv);
+        }
+        build_image<MT>(xv, m < rows, m, image + (size_t)b * Img<MT>::PB, threadIdx.x & 31);
+    }
+}
+
+// FROM_X: no image in memory, every warp makes that of the 256-blocks that it multiplies itself, straight from x.
+template <int TYPE, int MT, int STAGES, bool FROM_X>
+__global__ void __launch_bounds__(THREADS, 2) gemv_blk32_i8_kernel(View v, const uint8_t* __restrict__ image, const float* x, int rows, const float* __restrict__ bias,
                                                                    float* __restrict__ y, int tiles) {
     using G = Geo<TYPE>;
     using I = Img<MT>;
@@ -227,8 +203,35 @@ __global__ void __launch_bounds__(THREADS, 2) gemv_blk32_i8_kernel(View v, const
         issue();  // the first weights are on their way before the activation image is complete
     }
 
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // the image kernel has finished
-    {
+    if constexpr (FROM_X) {
+        asm volatile("griddepcontrol.launch_dependents;");  // (in the place of the image kernel's)
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the kernel in front, the image kernel or that which writes x, has finished
+    if constexpr (FROM_X) {
+        constexpr int TWO = 2;  // blocks whose values are on their way at a time
+        for (int j = 0; j < nb; j += TWO) {
+            float xv[TWO][MT][8] = {};
+#pragma unroll
+            for (int i = 0; i < TWO; i++) {
+#pragma unroll
+                for (int m = 0; m < MT; m++) {
+                    if (j + i < nb && m < rows) {
+                        load_x(x + (int64_t)m * v.k + (int64_t)(warp + NW * (j + i)) * 256, lane, xv[i][m]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < TWO; i++) {
+#pragma unroll
+                for (int m = 0; m < MT; m++) {
+                    if (j + i < nb) {
+                        build_image<MT>(xv[i][m], m < rows, m, img + (size_t)(warp + NW * (j + i)) * I::PB, lane);
+                    }
+                }
+            }
+        }
+        __syncwarp();  // nobody else reads them
+    } else {
         const uint32_t img_s = (uint32_t)__cvta_generic_to_shared(img);
         const int chunks = (int)((size_t)KB * I::PB / 16);
         for (int c = tid; c < chunks; c += THREADS) {
@@ -388,55 +391,56 @@ bool image_fits(int64_t k, int rows) {
     return (rows == 1 ? smem_bytes<TYPE, 1>((int)(k / 256)) : smem_bytes<TYPE, 2>((int)(k / 256))) <= SMEM_MAX;
 }
 
-template <int TYPE, int MT>
-int run(const View& v, const float* x, int rows, const float* bias, float* y, cudaStream_t s, uint8_t* image, bool* handled) {
+// The GEMV builds the image itself for up to this many values of x: four blocks a warp. Every thread block then makes all of it, redundant work that grows with
+// them; x in host memory is never read once per thread block. Replayed from a graph, image kernel / built here, us: one row, 4096 x 4096 Q8_0 4.6 / 3.7, Q4_0 4.4 /
+// 3.9, Q4_1 4.4 / 4.0; 1024 x 1024 2.8 / 1.8; 32000 x 4096 23.3 / 21.9, 15.8 / 13.6, 16.6 / 14.6; one row of 8192 (4096 x 8192) 7.2 / 7.1, 5.9 / 6.1, 6.4 / 6.4; two rows of
+// 4096 (4096 x 4096) 4.6 / 4.7, 4.6 / 4.8, 4.6 / 4.8, at most 7.2 / 8.0 (11008 x 4096, Q4_0). A call that is launched, not replayed, saves 2 us of host time besides,
+// and that is the longer of the two for most of these.
+constexpr int64_t FROM_X = 8192;
+
+template <int TYPE, int MT, bool FROM_X>
+int run(const View& v, const float* x, int rows, const float* bias, float* y, cudaStream_t s, uint8_t* image) {
     constexpr int STAGES = stages_of(TYPE);
+    auto kernel = gemv_blk32_i8_kernel<TYPE, MT, STAGES, FROM_X>;
     const int KB = (int)(v.k / 256);
     const int tiles = (int)((v.n + 15) / 16);
     const size_t smem = smem_bytes<TYPE, MT>(KB);
     // two CTAs per SM, or one where the image of the whole k leaves no room for two (Q8_0, one row of x: from k = 11008 on)
     const int per_sm = smem > SMEM_MAX / 2 - 1024 ? 1 : 2;
-    *handled = true;
     static std::atomic<uint64_t> configured{0};  // the opt-in for large dynamic shared memory is per device
     int dev = 0;
     JQ_CUDA(cudaGetDevice(&dev));
     if ((configured.load() >> (dev & 63) & 1) == 0) {
-        JQ_CUDA(cudaFuncSetAttribute(gemv_blk32_i8_kernel<TYPE, MT, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
+        JQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
         configured.fetch_or((uint64_t)1 << (dev & 63));
     }
-    // launched programmatically as well: it is scheduled while the kernel before it still runs (it waits for that kernel
-    // before touching memory) and lets the GEMV behind it be scheduled at once
-    cudaLaunchConfig_t icfg = {};
-    cudaLaunchAttribute iattr[1];
-    iattr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    iattr[0].val.programmaticStreamSerializationAllowed = 1;
-    icfg.attrs = iattr;
-    icfg.numAttrs = 1;
-    icfg.stream = s;
-    icfg.gridDim = dim3((unsigned)((KB * MT + PREP_WARPS - 1) / PREP_WARPS));
-    icfg.blockDim = dim3(PREP_WARPS * 32);
-    JQ_CUDA(cudaLaunchKernelEx(&icfg, blk32_image_kernel<MT>, x, rows, (int64_t)v.k, image));
-    count_launch();
-    const int grid = tiles < sm_count() * per_sm ? tiles : sm_count() * per_sm;
+    // launched programmatically: a kernel is scheduled while the one before it still runs (it waits for that one before touching what it
+    // writes) and lets the one behind it be scheduled at once
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // may start while the image kernel runs
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    JQ_CUDA(cudaLaunchKernelEx(&cfg, gemv_blk32_i8_kernel<TYPE, MT, STAGES>, v, (const uint8_t*)image, rows, bias, y, tiles));
+    cfg.stream = s;
+    if (!FROM_X) {
+        cfg.gridDim = dim3((unsigned)((KB * MT + PREP_WARPS - 1) / PREP_WARPS));
+        cfg.blockDim = dim3(PREP_WARPS * 32);
+        JQ_CUDA(cudaLaunchKernelEx(&cfg, blk32_image_kernel<MT>, x, rows, (int64_t)v.k, image));
+        count_launch();
+    }
+    cfg.gridDim = dim3((unsigned)(tiles < sm_count() * per_sm ? tiles : sm_count() * per_sm));
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = smem;
+    JQ_CUDA(cudaLaunchKernelEx(&cfg, kernel, v, (const uint8_t*)image, x, rows, bias, y, tiles));
     count_launch();
     return JQ_OK;
 }
 
 template <int TYPE>
-int by_rows(const View& v, const float* x, int rows, const float* bias, float* y, cudaStream_t s, uint8_t* image, bool* handled) {
-    if (rows == 1) return run<TYPE, 1>(v, x, rows, bias, y, s, image, handled);
-    return run<TYPE, 2>(v, x, rows, bias, y, s, image, handled);
+int by_rows(const View& v, const float* x, int rows, const float* bias, float* y, cudaStream_t s, uint8_t* image, bool from_x) {
+    if (rows == 1) return from_x ? run<TYPE, 1, true>(v, x, rows, bias, y, s, image) : run<TYPE, 1, false>(v, x, rows, bias, y, s, image);
+    return from_x ? run<TYPE, 2, true>(v, x, rows, bias, y, s, image) : run<TYPE, 2, false>(v, x, rows, bias, y, s, image);
 }
 
 }  // namespace
@@ -454,16 +458,18 @@ size_t gemv_blk32_i8_scratch_bytes(int type, int64_t k, int rows) {
 
 // Q8_0, Q4_0, Q4_1 with rows in [1, 2] and k a multiple of 256, on a weight whose planes are padded by 16 rows.
 // *handled = false leaves the call to another kernel.
-int launch_gemv_blk32_i8(const View& v, const float* x, int rows, const float* bias, float* y, cudaStream_t s, uint8_t* image, bool* handled) {
+int launch_gemv_blk32_i8(const View& v, const float* x, int rows, const float* bias, float* y, cudaStream_t s, uint8_t* image, bool* handled, bool x_remote) {
     *handled = false;
     if (gemv_blk32_i8_scratch_bytes(v.type, v.k, rows) == 0 || v.n == 0 || v.aux == nullptr || image == nullptr ||
         (int64_t)16 * (v.k / 256) * 256 >= ((int64_t)1 << 31)) {
         return JQ_OK;
     }
+    *handled = true;
+    const bool from_x = rows * v.k <= FROM_X && !x_remote;
     switch (v.type) {
-        case JQ_TYPE_Q8_0: return by_rows<JQ_TYPE_Q8_0>(v, x, rows, bias, y, s, image, handled);
-        case JQ_TYPE_Q4_0: return by_rows<JQ_TYPE_Q4_0>(v, x, rows, bias, y, s, image, handled);
-        default: return by_rows<JQ_TYPE_Q4_1>(v, x, rows, bias, y, s, image, handled);
+        case JQ_TYPE_Q8_0: return by_rows<JQ_TYPE_Q8_0>(v, x, rows, bias, y, s, image, from_x);
+        case JQ_TYPE_Q4_0: return by_rows<JQ_TYPE_Q4_0>(v, x, rows, bias, y, s, image, from_x);
+        default: return by_rows<JQ_TYPE_Q4_1>(v, x, rows, bias, y, s, image, from_x);
     }
 }
 

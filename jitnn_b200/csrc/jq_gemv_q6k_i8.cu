@@ -113,8 +113,9 @@ __global__ void __launch_bounds__(PREP_WARPS * 32) q6k_activation_image_kernel(c
 }
 
 // ---- the GEMV ---------------------------------------------------------------------------------------------------
-template <int MT, int STAGES, int OCC>
-__global__ void __launch_bounds__(THREADS, OCC) gemv_q6k_i8_kernel(View v, const uint8_t* __restrict__ image, int rows,
+// FROM_X: no image in memory, every warp makes that of the super-blocks that it multiplies itself, straight from x (one slice).
+template <int MT, int STAGES, int OCC, bool FROM_X>
+__global__ void __launch_bounds__(THREADS, OCC) gemv_q6k_i8_kernel(View v, const uint8_t* __restrict__ image, const float* x, int rows,
                                                                   const float* __restrict__ bias, float* __restrict__ y, int tiles,
                                                                   int KS, int max_tiles, long long wait_clocks, int* status) {
     // KS = super-blocks of k per slice: the activation image of one slice is resident in shared memory at a time;
@@ -309,7 +310,31 @@ __global__ void __launch_bounds__(THREADS, OCC) gemv_q6k_i8_kernel(View v, const
         if (sl > 0) {
             __syncthreads();  // every warp is done with the previous slice
         }
-        if (nslices == 1) {
+        if constexpr (FROM_X) {
+            constexpr int TWO = 2;  // super-blocks whose values are on their way at a time
+            for (int b = warp; b < KB; b += TWO * WARPS) {
+                float xv[TWO][MT][8] = {};
+#pragma unroll
+                for (int i = 0; i < TWO; i++) {
+#pragma unroll
+                    for (int m = 0; m < MT; m++) {
+                        if (b + i * WARPS < KB && m < rows) {
+                            q6k::load_x(x + (int64_t)m * v.k + (int64_t)(b + i * WARPS) * 256, lane, xv[i][m]);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < TWO; i++) {
+#pragma unroll
+                    for (int m = 0; m < MT; m++) {
+                        if (b + i * WARPS < KB) {
+                            build_image<MT>(xv[i][m], m < rows, m, img + (size_t)(b + i * WARPS) * C::PB, lane);
+                        }
+                    }
+                }
+            }
+            __syncwarp();
+        } else if (nslices == 1) {
             // one slice: a warp only ever reads the image of its own super-blocks, so it fetches just those and waits for
             // nobody else (the wait also covers the weight stages requested so far, which it needs next anyway)
             constexpr int CH = (int)(C::PB / 16);
@@ -413,6 +438,8 @@ __global__ void __launch_bounds__(THREADS, OCC) gemv_q6k_i8_kernel(View v, const
     }
 }
 
+constexpr int64_t FROM_X_VALUES = 8192;
+
 int g_sms = 0;
 int sm_count() {
     if (g_sms == 0) {
@@ -426,13 +453,13 @@ int sm_count() {
     return g_sms;
 }
 
-template <int MT, int STAGES, int OCC>
-int launch(const View& v, const uint8_t* image, int rows, const float* bias, float* y, cudaStream_t s, int KS, int grid, int max_tiles, size_t smem) {
+template <int MT, int STAGES, int OCC, bool FROM_X>
+int launch(const View& v, const uint8_t* image, const float* x, int rows, const float* bias, float* y, cudaStream_t s, int KS, int grid, int max_tiles, size_t smem) {
     static std::atomic<uint64_t> configured{0};  // the opt-in for large dynamic shared memory is per device
     int dev = 0;
     JQ_CUDA(cudaGetDevice(&dev));
     if ((configured.load() >> (dev & 63) & 1) == 0) {
-        JQ_CUDA(cudaFuncSetAttribute(gemv_q6k_i8_kernel<MT, STAGES, OCC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
+        JQ_CUDA(cudaFuncSetAttribute(gemv_q6k_i8_kernel<MT, STAGES, OCC, FROM_X>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
         configured.fetch_or((uint64_t)1 << (dev & 63));
     }
     const int tiles = (int)((v.n + 15) / 16);
@@ -452,7 +479,7 @@ int launch(const View& v, const uint8_t* image, int rows, const float* bias, flo
     if (rc != JQ_OK) {
         return rc;
     }
-    JQ_CUDA(cudaLaunchKernelEx(&cfg, gemv_q6k_i8_kernel<MT, STAGES, OCC>, v, image, rows, bias, y, tiles, KS, max_tiles, wait_clocks, status));
+    JQ_CUDA(cudaLaunchKernelEx(&cfg, gemv_q6k_i8_kernel<MT, STAGES, OCC, FROM_X>, v, image, x, rows, bias, y, tiles, KS, max_tiles, wait_clocks, status));
     count_launch();
     return JQ_OK;
 }
@@ -465,7 +492,7 @@ size_t smem_bytes(int KS, int stages, bool sliced, int max_tiles) {
 }
 
 template <int MT>
-int run(const View& v, const float* x, int rows, const float* bias, float* y, cudaStream_t s, uint8_t* image, bool* handled) {
+int run(const View& v, const float* x, int rows, const float* bias, float* y, cudaStream_t s, uint8_t* image, bool* handled, bool x_remote = false) {
     const int KB = (int)(v.k / 256);
     const int tiles = (int)((v.n + 15) / 16);
     // Candidate shapes, best first: (CTAs per SM, ring stages); two CTAs per SM with three stages measured best. The slice length KS is a function of MT and k only (so
@@ -506,6 +533,16 @@ int run(const View& v, const float* x, int rows, const float* bias, float* y, cu
         return JQ_OK;
     }
     *handled = true;
+    if constexpr (MT <= 2) {
+        // Up to FROM_X_VALUES values of x, four super-blocks a warp: the GEMV builds the image itself (every thread block makes all of it, redundant work that grows with
+        // them; x in host memory is never read once per thread block). Replayed from a graph, image kernel / built here, us: one row,
+        // 1024 x 1024 3.2 / 2.0, 4096 x 4096 5.6 / 4.5, 32000 x 4096 21.8 / 20.3, 4096 x 8192 8.2 / 8.1; two rows, 4096 x 2048 4.6 / 3.7, 4096 x 4096 5.6 / 5.9, 32000 x 4096 22.1 / 22.0. A
+        // launched call saves 2 us of host time besides.
+        if (x != nullptr && rows * v.k <= FROM_X_VALUES && !x_remote && !sliced) {
+            return stages == 3 ? launch<MT, 3, 2, true>(v, image, x, rows, bias, y, s, KS, grid, max_tiles, smem)
+                               : launch<MT, 2, 2, true>(v, image, x, rows, bias, y, s, KS, grid, max_tiles, smem);
+        }
+    }
     if (x != nullptr) {  // else the image is already in `image` (written by a kernel earlier in the stream)
         // launched programmatically as well: it is scheduled while the kernel before it still runs (it waits for that kernel
         // before touching memory) and lets the GEMV behind it be scheduled at once
@@ -521,8 +558,8 @@ int run(const View& v, const float* x, int rows, const float* bias, float* y, cu
         JQ_CUDA(cudaLaunchKernelEx(&icfg, q6k_activation_image_kernel<MT>, x, rows, (int64_t)v.k, image));
         count_launch();
     }
-    if (stages == 3) return launch<MT, 3, 2>(v, image, rows, bias, y, s, KS, grid, max_tiles, smem);
-    return launch<MT, 2, 2>(v, image, rows, bias, y, s, KS, grid, max_tiles, smem);
+    if (stages == 3) return launch<MT, 3, 2, false>(v, image, x, rows, bias, y, s, KS, grid, max_tiles, smem);
+    return launch<MT, 2, 2, false>(v, image, x, rows, bias, y, s, KS, grid, max_tiles, smem);
 }
 
 }  // namespace
@@ -540,13 +577,13 @@ size_t gemv_q6k_i8_scratch_bytes(int64_t k, int rows) {
 // Q6_K with rows in [1, 4] on a weight whose planes is padded by 16 rows. `image` is a scratch buffer of
 // gemv_q6k_i8_scratch_bytes(k, rows) bytes, 16-byte aligned, private to `s` until the GEMV kernel has run.
 // *handled = false leaves the call to another kernel.
-int launch_gemv_q6k_i8(const View& v, const float* x, int rows, const float* bias, float* y, cudaStream_t s, uint8_t* image, bool* handled) {
+int launch_gemv_q6k_i8(const View& v, const float* x, int rows, const float* bias, float* y, cudaStream_t s, uint8_t* image, bool* handled, bool x_remote) {
     *handled = false;
     if (v.type != JQ_TYPE_Q6_K || v.n == 0 || v.k == 0 || rows > 4 || image == nullptr || (int64_t)16 * (v.k / 256) * 208 >= ((int64_t)1 << 31)) {
         return JQ_OK;
     }
-    if (rows == 1) return run<1>(v, x, rows, bias, y, s, image, handled);
-    if (rows == 2) return run<2>(v, x, rows, bias, y, s, image, handled);
+    if (rows == 1) return run<1>(v, x, rows, bias, y, s, image, handled, x_remote);
+    if (rows == 2) return run<2>(v, x, rows, bias, y, s, image, handled, x_remote);
     return run<4>(v, x, rows, bias, y, s, image, handled);
 }
 

@@ -3,7 +3,7 @@
 // and SwiGLU kernels) include this to write the image directly instead of a float vector.
 #pragma once
 
-#include "jq_common.cuh"
+#include "jq_digits.cuh"
 
 namespace jq {
 namespace q4k {
@@ -53,45 +53,14 @@ __device__ __forceinline__ void build_image_from(const float (&xv)[8], bool pres
         tab[lane] = 0.0f;  // columns that hold no activation row
         tab[NG * 8 + lane] = 0.0f;
     }
-    // largest magnitude as an integer (NaN > Inf > every finite value in this order), so one comparison finds a value that is
-    // not finite: the column weights then become NaN and with them every output of this row of x
-    uint32_t amb = 0u;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        amb = max(amb, __float_as_uint(xv[i]) & 0x7fffffffu);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        amb = max(amb, __shfl_xor_sync(0xffffffffu, amb, o));
-    }
-    const bool bad = amb >= 0x7f800000u;
-    // s = 2^floor(log2(amax)): the largest |x| / s of the super-block lies in [1, 2)
-    uint32_t e = amb & 0x7f800000u;
-    e = e < 0x0d000000u ? 0x0d000000u : (e > 0x7e800000u ? 0x7e800000u : e);  // keeps 2^21 / s and s * 2^-25 normal
-    // 2^21 / s: |X| <= 2^22, so the top digit stays within a signed byte after the carries
-    const float inv = __uint_as_float(0x7f000000u - e + (21u << 23));
-    // X = rint(x * inv) lands in the mantissa of x * inv + 1.5 * 2^23 (the product is exact: inv is a power of two). With 128
-    // added at every byte position the three low bytes of Y = X + 0x808080 are the signed base-256 digits plus 128 each
-    // (X = d0 + 256 d1 + 65536 d2 with -128 <= d < 128 has exactly one such form), so digit = byte ^ 0x80.
-    uint32_t Y[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        Y[i] = __float_as_uint(fmaf(xv[i], inv, 12582912.0f)) - 0x4b400000u + 0x00808080u;
-    }
-    // bytes of four values side by side: [Y0.b, Y1.b, Y2.b, Y3.b] for b = 0, 1, 2
+    bool bad;  // the column weights then become NaN and with them every output of this row of x
+    const uint32_t e = image_exponent(xv, 0x0d000000u, bad);
     uint32_t dw[3][2];
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        const uint32_t t01 = __byte_perm(Y[4 * h], Y[4 * h + 1], 0x5140), t23 = __byte_perm(Y[4 * h + 2], Y[4 * h + 3], 0x5140);
-        const uint32_t h01 = __byte_perm(Y[4 * h], Y[4 * h + 1], 0x0062), h23 = __byte_perm(Y[4 * h + 2], Y[4 * h + 3], 0x0062);
-        dw[0][h] = __byte_perm(t01, t23, 0x5410) ^ 0x80808080u;
-        dw[1][h] = __byte_perm(t01, t23, 0x7632) ^ 0x80808080u;
-        dw[2][h] = __byte_perm(h01, h23, 0x5410) ^ 0x80808080u;
-    }
+    image_digits(xv, e, dw);
 #pragma unroll
     for (int dgt = 0; dgt < 3; dgt++) {
         const uint32_t w0 = dw[dgt][0], w1 = dw[dgt][1];
-        int sum = __dp4a((int)w0, 0x01010101, __dp4a((int)w1, 0x01010101, 0));  // the eight digits as signed bytes
+        int sum = digit_sum(dw[dgt]);
         const int col = C::qcol(m, dgt);
         xd[((((size_t)(sub >> 1) * NG + (col >> 3)) * NCOL + (col & 7)) * 4 + tt) * 2 + (sub & 1)] = make_uint2(w0, w1);
         // digit sum of the sub-block (its 4 octets sit in 4 consecutive lanes): sum = 128 hi + lo7, both fit a signed byte.

@@ -3,7 +3,7 @@
 // directly instead of a float vector.
 #pragma once
 
-#include "jq_common.cuh"
+#include "jq_digits.cuh"
 
 namespace jq {
 namespace q6k {
@@ -23,12 +23,19 @@ struct Cfg {
     static constexpr size_t PB = XD + XC + TAB;
 };
 
-// One warp turns the 256 values at xb (one super-block of k of row m of x; nullptr: a row beyond those of x, all zero)
-// into its part of the super-block's image at `img` (global or shared memory).
-// Lane L holds the 8 activations 8L .. 8L+7: they are k-slots 8 (L % 2) .. + 7 of scale group L / 2 (a group = 16
+// Lane L holds the 8 activations 8L .. 8L+7 of 256: they are k-slots 8 (L % 2) .. + 7 of scale group L / 2 (a group = 16
 // consecutive elements of the super-block).
+__device__ __forceinline__ void load_x(const float* xb, int lane, float (&xv)[8]) {
+    const float4* xp = reinterpret_cast<const float4*>(xb) + 2 * lane;
+    const float4 lo = xp[0], hi = xp[1];
+    xv[0] = lo.x; xv[1] = lo.y; xv[2] = lo.z; xv[3] = lo.w;
+    xv[4] = hi.x; xv[5] = hi.y; xv[6] = hi.z; xv[7] = hi.w;
+}
+
+// One warp turns the 256 values of one super-block of k of row m of x (not given: a row beyond those of x, all zero)
+// into its part of the super-block's image at `img` (global or shared memory).
 template <int MT>
-__device__ __forceinline__ void build_image(const float* xb, int m, uint8_t* img, int lane) {
+__device__ __forceinline__ void build_image(const float (&xv)[8], bool given, int m, uint8_t* img, int lane) {
     using C = Cfg<MT>;
     constexpr int NG = C::NG, NCOL = C::NCOL;
     const int grp = lane >> 1, half = lane & 1;
@@ -38,68 +45,37 @@ __device__ __forceinline__ void build_image(const float* xb, int m, uint8_t* img
     if (m == 0 && lane >= C::COLS && lane < NG * 8) {
         tab[lane] = 0.0f;  // columns that hold no activation row
     }
-    float xv[8];
-    if (xb != nullptr) {
-        const float4* xp = reinterpret_cast<const float4*>(xb) + 2 * lane;
-        const float4 lo = xp[0], hi = xp[1];
-        xv[0] = lo.x; xv[1] = lo.y; xv[2] = lo.z; xv[3] = lo.w;
-        xv[4] = hi.x; xv[5] = hi.y; xv[6] = hi.z; xv[7] = hi.w;
-    } else {
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            xv[i] = 0.0f;
-        }
-    }
-    float am = 0.0f;
-    bool bad = false;  // a NaN or an Inf among the values: the column weights become NaN and with them every output of this row of x
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        am = fmaxf(am, fabsf(xv[i]));
-        bad = bad || (__float_as_uint(xv[i]) & 0x7f800000u) == 0x7f800000u;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
-    }
-    bad = __any_sync(0xffffffffu, bad);
-    // s = 2^floor(log2(amax)): the largest |x| / s of the super-block lies in [1, 2)
-    uint32_t e = __float_as_uint(am) & 0x7f800000u;
-    e = e < 0x0c000000u ? 0x0c000000u : (e > 0x7e800000u ? 0x7e800000u : e);  // keeps 2^21 / s and s * 2^-21 normal
-    const float inv = __uint_as_float(0x7f000000u - e + (21u << 23));           // 2^21 / s: |X| <= 2^22
-    int X[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        X[i] = __float2int_rn(xv[i] * inv);
-    }
+    bool bad;  // the column weights then become NaN and with them every output of this row of x
+    const uint32_t e = image_exponent(xv, 0x0c000000u, bad);
+    uint32_t dw[3][2];
+    image_digits(xv, e, dw);
 #pragma unroll
     for (int dgt = 0; dgt < 3; dgt++) {
-        uint32_t w0 = 0, w1 = 0;
-        int sum = 0;
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int d = dgt == 2 ? X[i] : (int)(int8_t)(X[i] & 0xff);  // signed low byte
-            X[i] = (X[i] - d) >> 8;
-            sum += d;
-            if (i < 4) {
-                w0 |= (uint32_t)(d & 0xff) << (8 * i);
-            } else {
-                w1 |= (uint32_t)(d & 0xff) << (8 * (i - 4));
-            }
-        }
+        int sum = digit_sum(dw[dgt]);
         const int col = 3 * m + dgt;
         // lane slots 2 half and 2 half + 1 of this group's B fragment
         uint32_t* cell = xd + ((((size_t)(grp >> 2) * NG + (col >> 3)) * NCOL + (col & 7)) * 16) + (grp & 3);
-        cell[(2 * half) * 4] = w0;
-        cell[(2 * half + 1) * 4] = w1;
+        cell[(2 * half) * 4] = dw[dgt][0];
+        cell[(2 * half + 1) * 4] = dw[dgt][1];
         // -32 * (digit sum of the group's 16 elements): the row-independent part of sum (q - 32) x, the MMA's C operand
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);
         if (half == 0) {
             xc[((((size_t)(grp >> 1) * NG + (col >> 3)) * 4 + ((col & 7) >> 1)) * 2 + (grp & 1)) * 2 + (col & 1)] = -32 * sum;
         }
         if (lane == 0) {
-            tab[col] = xb == nullptr ? 0.0f : (bad ? __uint_as_float(0x7fc00000u) : __uint_as_float(e + ((uint32_t)(8 * dgt) << 23) - (21u << 23)));  // s * 2^(8 dgt - 21)
+            tab[col] = !given ? 0.0f : (bad ? __uint_as_float(0x7fc00000u) : __uint_as_float(e + ((uint32_t)(8 * dgt) << 23) - (21u << 23)));  // s * 2^(8 dgt - 21)
         }
     }
+}
+
+// The same from memory; nullptr: not given.
+template <int MT>
+__device__ __forceinline__ void build_image(const float* xb, int m, uint8_t* img, int lane) {
+    float xv[8] = {};
+    if (xb != nullptr) {
+        load_x(xb, lane, xv);
+    }
+    build_image<MT>(xv, xb != nullptr, m, img, lane);
 }
 
 }  // namespace q6k
