@@ -8,6 +8,7 @@ import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libjitnn_b200.so")
+FRONT_PATH = os.path.join(HERE, "_front.so")
 
 JQ_OK = 0
 JQ_ERR_INVALID, JQ_ERR_OOM, JQ_ERR_CUDA, JQ_ERR_NCCL, JQ_ERR_TIMEOUT, JQ_ERR_UNSUPPORTED = -1, -2, -3, -4, -5, -6
@@ -91,6 +92,18 @@ def load():
             fn.argtypes = args
         _lib = L
     return _lib
+
+
+def load_front(weight_class):
+    """The native front of calls on torch tensors (csrc/front.cpp), built against the torch it runs with; bound to the library's functions."""
+    import torch  # noqa: F401  (its libraries are what the module is linked to)
+    if not os.path.exists(FRONT_PATH):
+        raise ImportError("_front.so is not built: run `python -m jitnn_b200.build`; calls on torch tensors need it")
+    from . import _front
+    L = ctypes.CDLL(LIB_PATH)  # (the one that load() has)
+    names = ("jq_linear_f32", "jq_linear_bf16", "jq_linear_backward_f32", "jq_dequantize", "jq_quantize_q8_0")
+    _front.bind(weight_class, check, *(ctypes.cast(getattr(L, name), vp).value for name in names))
+    return _front
 
 
 def last_error():

@@ -1,4 +1,4 @@
-"""Builds ``libjitnn_b200.so`` in-tree with nvcc for sm_100a.
+"""Builds ``libjitnn_b200.so`` in-tree with nvcc for sm_100a, and ``_front.so``, the Python front of calls on torch tensors, with the C++ compiler.
 
     python -m jitnn_b200.build [--force] [--verbose]
 
@@ -16,6 +16,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "build")
 LIB = os.path.join(HERE, "libjitnn_b200.so")
+FRONT_SRC = os.path.join(CSRC, "front.cpp")
+FRONT = os.path.join(HERE, "_front.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -44,6 +46,23 @@ def _compile(src, obj, verbose, extra):
         sys.stderr.write(res.stdout + res.stderr)
 
 
+def build_front(force=False):
+    """Against the torch that is installed here, which is also the one it has to run with."""
+    if not force and os.path.exists(FRONT) and os.path.getmtime(FRONT) >= os.path.getmtime(FRONT_SRC):
+        return FRONT
+    import sysconfig
+    from importlib.util import find_spec
+    torch = os.path.dirname(find_spec("torch").origin)
+    cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc()))), "include")
+    cmd = [shutil.which("g++") or "c++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden"]
+    cmd += ["-I" + d for d in (os.path.join(torch, "include"), os.path.join(torch, "include", "torch", "csrc", "api", "include"), sysconfig.get_path("include"), cuda)]
+    cmd += [FRONT_SRC, "-o", FRONT, "-L" + os.path.join(torch, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("the build of _front.so failed:\n%s\n%s" % (res.stdout, res.stderr))
+    return FRONT
+
+
 def build(force=False, verbose=False, ptxas_info=False):
     os.makedirs(OBJ, exist_ok=True)
     sources = sorted(glob.glob(os.path.join(CSRC, "*.cu")))
@@ -58,8 +77,10 @@ def build(force=False, verbose=False, ptxas_info=False):
         if stale:
             jobs.append((src, obj))
     with concurrent.futures.ThreadPoolExecutor(max_workers=max(1, os.cpu_count() or 1)) as pool:
+        front = pool.submit(build_front, force)
         for f in [pool.submit(_compile, s, o, verbose or ptxas_info, extra) for s, o in jobs]:
             f.result()
+        front.result()
     if jobs or not os.path.exists(LIB):
         cmd = [nvcc(), "-shared", "-o", LIB] + objects + ["-gencode", "arch=compute_100a,code=sm_100a", "-cudart", "static"]
         res = subprocess.run(cmd, capture_output=True, text=True)

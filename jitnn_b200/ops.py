@@ -62,6 +62,7 @@ class Tensor:
 
     def __init__(self, handle, dtype, dims, device=0):
         self._h = handle
+        self._addr = handle.value if handle else 0  # for the native front; 0 once the tensor is released
         self._dtype = dtype
         self._dims = tuple(dims)
         self._device = device
@@ -134,7 +135,7 @@ class Tensor:
 
     def release(self):
         if self._h is not None:
-            h, self._h = self._h, None
+            h, self._h, self._addr = self._h, None, 0
             check(_lib.load().jq_weight_free(h))
 
     close = release
@@ -146,17 +147,19 @@ class Tensor:
             pass
 
 
-# Calls on torch tensors. A decode linear takes a few microseconds on the GPU, less than the host needs for an ordinary chain of torch calls
-# around it, so these paths ask each tensor for as little as the checks need, take torch's raw current stream, and leave making the
-# weight's device current to the library.
+# Calls on torch tensors. A decode linear takes a few microseconds on the GPU, less than the host needs for a chain of torch calls around it. So the plain
+# case, an ordinary contiguous tensor of the right type on the weight's device, is taken by native code as a whole (csrc/front.cpp), 4.0 us a call in place
+# of 7.4; it hands back None for everything else, which goes on here. It comes in with torch, on the first call with a torch tensor.
 _torch = None
+_front = None
 
 
 def _t():
-    global _torch
+    global _torch, _front
     if _torch is None:
         import torch
-        _torch = torch
+        front = _lib.load_front(Tensor)
+        _torch, _front = torch, front
     return _torch
 
 
@@ -271,22 +274,38 @@ class Gguf:
     @staticmethod
     def linear(x, w, bias=None):
         """y = x W^T + b, W [N, K] in a GGUF format, x FP32 [..., K]; b may be None."""
+        if _front is not None:
+            y = _front.linear(x, w, bias)
+            if y is not None:
+                return y
         return _linear(x, w, bias, "Gguf.linear")
 
     @staticmethod
     def dequantize(w, out=None):
+        if _front is not None:
+            y = _front.dequantize(w, out)
+            if y is not None:
+                return y
         return _dequantize(w, out)
 
     @staticmethod
     def linearBackward(g, w):
         """The input gradient of linear: gx [..., K] = g [..., N] . dequant(W) (ops/Gguf.java:208-212; the weight gets
         no gradient, the bias gradient is the column sum of g)."""
+        if _front is not None:
+            gx = _front.backward(g, w)
+            if gx is not None:
+                return gx
         return _linear_backward(g, w)
 
     @staticmethod
     def linearBf16(x, w, bias=None):
         """Prefill form: x bfloat16 [..., K] (a torch CUDA tensor, or a numpy uint16 array of bfloat16 bit patterns),
         y float32 [..., N]; dequantised weights rounded to bfloat16, tensor-core product, FP32 accumulation."""
+        if _front is not None:
+            y = _front.linear_bf16(x, w, bias)
+            if y is not None:
+                return y
         L = _lib.load()
         if not isinstance(w, Tensor):
             raise ValueError("Gguf.linearBf16: weight is not a quantised tensor")
@@ -331,6 +350,10 @@ class Quant:
     def linear(x, w, bias=None):
         if not isinstance(w, Tensor) or w.dtype() != DType.Q8_0:
             raise ValueError("Q8_0 linear: weight %s" % (w.dtype().name if isinstance(w, Tensor) else type(w)))
+        if _front is not None:
+            y = _front.linear(x, w, bias)
+            if y is not None:
+                return y
         return _linear(x, w, bias, "Quant.linear")
 
     @staticmethod
@@ -349,6 +372,10 @@ class Quant:
     @staticmethod
     def quantizeQ8Blocks(x, device=0):
         """FP32 values (last axis a multiple of 32) to raw Q8_0 block bytes (numpy uint8)."""
+        if _front is not None:
+            out = _front.quantize(x)
+            if out is not None:
+                return out
         L = _lib.load()
         if _is_torch(x):
             torch = _t()
