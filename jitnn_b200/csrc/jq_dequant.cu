@@ -102,14 +102,18 @@ template <>
 struct Four<JQ_TYPE_Q4_1> : FourN<JQ_TYPE_Q4_1> {};
 
 // A warp takes 256 values of ROWS rows: lane i the values 4 i .. and 128 + 4 i .. of each, so that every store of the warp is 512 contiguous
-// bytes; eight warps take neighbouring steps of k. Memory bound: the 4 output bytes per weight are 80 % and more of the traffic. (One
+// bytes; neighbouring warps take neighbouring steps of k. The weights are on their way before the kernel in front has ended (nothing writes them): Q6_K 4096 x 11008
+// 39.4 -> 36.5 us, 4096 x 4096 17.9 -> 15.3, 1024 x 1024 4.6 -> 2.8. Memory bound: the 4 output bytes per weight are 80 % and more of the traffic. (One
 // thread per 16 or 64 consecutive weights left stores of 16 bytes at strides of 64 to 256.)
 constexpr int ROWS = 4;
+constexpr int THREADS = 256;
 template <int TYPE>
-__global__ void __launch_bounds__(256) dequantize_kernel(View v, float* __restrict__ dst) {
+__global__ void __launch_bounds__(THREADS) dequantize_kernel(View v, float* __restrict__ dst, int steps) {
+    asm volatile("griddepcontrol.launch_dependents;");
     const int lane = threadIdx.x & 31;
-    const int64_t b = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5), r0 = (int64_t)blockIdx.y * ROWS;
-    if (b >= tiled_steps(v.k)) {
+    const uint32_t task = blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5);  // (warps that the last step of a row leaves idle would be every tenth at k = 11008)
+    const int64_t b = task % (uint32_t)steps, r0 = (int64_t)(task / (uint32_t)steps) * ROWS;
+    if (r0 >= v.n) {
         return;
     }
     Four<TYPE> f[ROWS][2];
@@ -121,6 +125,7 @@ __global__ void __launch_bounds__(256) dequantize_kernel(View v, float* __restri
             f[r][j].load(v, row, b, 128 * j + 4 * lane);
         }
     }
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // dst may be in use by the kernel in front
 #pragma unroll
     for (int r = 0; r < ROWS; r++) {
 #pragma unroll
@@ -134,59 +139,86 @@ __global__ void __launch_bounds__(256) dequantize_kernel(View v, float* __restri
 }
 
 // ---- formats that are dequantised only (no linear kernel): verbatim bytes ----
-__device__ __forceinline__ int u8(const uint8_t* w, int64_t at) { return w[at]; }
-__device__ __forceinline__ float f16(const uint8_t* w, int64_t at) {
-    return __half2float(__ushort_as_half((unsigned short)(w[at] | (w[at + 1] << 8))));
-}
-__device__ __forceinline__ int bit32(const uint8_t* w, int64_t at, int bit) { return (u8(w, at + bit / 8) >> (bit % 8)) & 1; }
+__device__ __forceinline__ uint32_t ld2(const uint8_t* p) { return __ldg(reinterpret_cast<const unsigned short*>(p)); }
+__device__ __forceinline__ uint32_t ld2x2(const uint8_t* p) { return ld2(p) | ld2(p + 2) << 16; }  // (where a block starts on an even address only)
+// Bits 0 .. 3 to bit 4 of four bytes.
+__device__ __forceinline__ uint32_t bits_to_bytes(uint32_t h) { return ((h & 15u) * 0x00204081u & 0x01010101u) << 4; }
 
-// kernels/GgufKernels.java:147-198 of the reference (Q5_0, Q5_1, Q2_K, Q3_K), one rounded float
-// operation per arithmetic step.
-__device__ __forceinline__ float extra_value(int type, const uint8_t* w, int64_t i) {
-    if (type == JQ_TYPE_Q5_0) {
-        int64_t base = (i / 32) * 22;
-        int e = (int)(i % 32);
-        int b = u8(w, base + 6 + e % 16);
-        int q = (e < 16 ? b & 15 : b >> 4) + 16 * bit32(w, base + 2, e);
-        return __fmul_rn((float)(q - 16), f16(w, base));
-    }
-    if (type == JQ_TYPE_Q5_1) {
-        int64_t base = (i / 32) * 24;
-        int e = (int)(i % 32);
-        int b = u8(w, base + 8 + e % 16);
-        int q = (e < 16 ? b & 15 : b >> 4) + 16 * bit32(w, base + 4, e);
-        return __fadd_rn(__fmul_rn((float)q, f16(w, base)), f16(w, base + 2));
-    }
-    if (type == JQ_TYPE_Q2_K) {
-        int64_t base = (i / 256) * 84;
-        int e = (int)(i % 256);
-        int n = e / 128, j = (e % 128) / 32, l = e % 32;
-        int sc = u8(w, base + n * 8 + j * 2 + l / 16);
-        int q = (u8(w, base + 16 + n * 32 + l) >> (2 * j)) & 3;
-        float a = __fmul_rn(__fmul_rn(f16(w, base + 80), (float)(sc & 15)), (float)q);
-        return __fsub_rn(a, __fmul_rn(f16(w, base + 82), (float)(sc >> 4)));
-    }
-    // Q3_K
-    int64_t base = (i / 256) * 110;
-    int e = (int)(i % 256);
-    int n = e / 128, j = (e % 128) / 32, l = e % 32;
-    int is = n * 8 + j * 2 + l / 16;
-    int q = (u8(w, base + 32 + n * 32 + l) >> (2 * j)) & 3;
-    int high = (u8(w, base + l) >> (4 * n + j)) & 1;
-    int64_t s = base + 96;
-    int low = is < 8 ? u8(w, s + is) & 15 : u8(w, s + is - 8) >> 4;
-    int hi2 = (u8(w, s + 8 + is % 4) >> (2 * (is / 4))) & 3;
-    int scale = low + 16 * hi2 - 32;
-    return __fmul_rn(__fmul_rn(f16(w, base + 108), (float)scale), (float)(q - (high == 1 ? 0 : 4)));
-}
-
-// Four consecutive values per thread (they share a block), so that stores are 16 bytes each.
+// Four consecutive values, which share a scale: kernels/GgufKernels.java:147-198 of the reference (Q5_0, Q5_1, Q2_K, Q3_K), one rounded float operation
+// per arithmetic step.
 template <int TYPE>
-__global__ void __launch_bounds__(256) dequantize_extra_kernel(const uint8_t* __restrict__ w, float* __restrict__ dst, int64_t count) {
-    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
-    if (i < count) {
-        *reinterpret_cast<float4*>(dst + i) = make_float4(extra_value(TYPE, w, i), extra_value(TYPE, w, i + 1), extra_value(TYPE, w, i + 2), extra_value(TYPE, w, i + 3));
+__device__ __forceinline__ float4 extra_values(const uint8_t* w, int64_t i) {
+    if constexpr (TYPE == JQ_TYPE_Q5_0) {
+        const uint8_t* p = w + (i >> 5) * 22;
+        const int e = (int)(i & 31);
+        const uint32_t q = ((ld2x2(p + 6 + (e & 15)) >> (e & 16 ? 4 : 0)) & 0x0f0f0f0fu) | bits_to_bytes(ld2x2(p + 2) >> e);
+        const float d = half_bits_to_float(ld2(p));
+        return make_float4(__fmul_rn(byte_float(q, 0) - 16.0f, d), __fmul_rn(byte_float(q, 1) - 16.0f, d), __fmul_rn(byte_float(q, 2) - 16.0f, d), __fmul_rn(byte_float(q, 3) - 16.0f, d));
+    } else if constexpr (TYPE == JQ_TYPE_Q5_1) {
+        const uint8_t* p = w + (i >> 5) * 24;
+        const int e = (int)(i & 31);
+        const uint32_t q = ((ld4(p + 8 + (e & 15)) >> (e & 16 ? 4 : 0)) & 0x0f0f0f0fu) | bits_to_bytes(ld4(p + 4) >> e), dm = ld4(p);
+        const float d = half_bits_to_float(dm), m = half_bits_to_float(dm >> 16);
+        return make_float4(__fadd_rn(__fmul_rn(byte_float(q, 0), d), m), __fadd_rn(__fmul_rn(byte_float(q, 1), d), m), __fadd_rn(__fmul_rn(byte_float(q, 2), d), m),
+                           __fadd_rn(__fmul_rn(byte_float(q, 3), d), m));
+    } else if constexpr (TYPE == JQ_TYPE_Q2_K) {
+        const uint8_t* p = w + (i >> 8) * 84;
+        const int n = (int)(i >> 7) & 1, j = (int)(i >> 5) & 3, l = (int)(i & 31);
+        const uint32_t sc = __ldg(p + n * 8 + j * 2 + (l >> 4)), q = (ld4(p + 16 + n * 32 + l) >> (2 * j)) & 0x03030303u, dm = ld4(p + 80);
+        const float d = __fmul_rn(half_bits_to_float(dm), (float)(sc & 15)), m = __fmul_rn(half_bits_to_float(dm >> 16), (float)(sc >> 4));
+        return make_float4(__fsub_rn(__fmul_rn(d, byte_float(q, 0)), m), __fsub_rn(__fmul_rn(d, byte_float(q, 1)), m), __fsub_rn(__fmul_rn(d, byte_float(q, 2)), m),
+                           __fsub_rn(__fmul_rn(d, byte_float(q, 3)), m));
+    } else {
+        const uint8_t* p = w + (i >> 8) * 110;
+        const int n = (int)(i >> 7) & 1, j = (int)(i >> 5) & 3, l = (int)(i & 31), is = n * 8 + j * 2 + (l >> 4);
+        // (quant) + 4 (its bit in the mask), minus 4
+        const uint32_t q = ((ld2x2(p + 32 + n * 32 + l) >> (2 * j)) & 0x03030303u) | ((ld2x2(p + l) >> (4 * n + j)) & 0x01010101u) << 2;
+        const int low = __ldg(p + 96 + (is & 7)), high = __ldg(p + 104 + (is & 3));
+        const int scale = (is < 8 ? low & 15 : low >> 4) + 16 * (high >> (2 * (is >> 2)) & 3) - 32;
+        const float d = __fmul_rn(half_bits_to_float(ld2(p + 108)), (float)scale);
+        return make_float4(__fmul_rn(d, byte_float(q, 0) - 4.0f), __fmul_rn(d, byte_float(q, 1) - 4.0f), __fmul_rn(d, byte_float(q, 2) - 4.0f), __fmul_rn(d, byte_float(q, 3) - 4.0f));
     }
+}
+
+// A warp's stores are 512 contiguous bytes; a thread has the loads of PIECES of them in flight. (With every value of its own, made from loads of single bytes,
+// instructions bound it: 4096 x 11008 Q5_0 71.7 us, Q5_1 74.0, Q2_K 86.4, Q3_K 112.8; now 42.9, 34.2, 34.6, 43.7, and 47 with one piece in flight; floor 30 to 33. Q5_0's and
+// Q3_K's blocks start on even addresses, so that four quants are two loads.)
+constexpr int PIECES = 2;
+template <int TYPE>
+__global__ void __launch_bounds__(THREADS) dequantize_extra_kernel(const uint8_t* __restrict__ w, float* __restrict__ dst, int64_t count) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    const int64_t i0 = ((int64_t)blockIdx.x * (PIECES * THREADS) + threadIdx.x) * 4;
+    float4 v[PIECES];
+#pragma unroll
+    for (int j = 0; j < PIECES; j++) {
+        const int64_t i = i0 + j * (THREADS * 4);
+        v[j] = extra_values<TYPE>(w, i < count ? i : 0);
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // dst may be in use by the kernel in front
+#pragma unroll
+    for (int j = 0; j < PIECES; j++) {
+        const int64_t i = i0 + j * (THREADS * 4);
+        if (i < count) {
+            *reinterpret_cast<float4*>(dst + i) = v[j];
+        }
+    }
+}
+
+// `ctas` thread blocks, launched programmatically.
+struct Config {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+};
+static Config& launch_config(int64_t ctas, cudaStream_t s) {
+    static thread_local Config c;
+    c.attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    c.attr[0].val.programmaticStreamSerializationAllowed = 1;
+    c.cfg.attrs = c.attr;
+    c.cfg.numAttrs = 1;
+    c.cfg.gridDim = dim3((unsigned)ctas);
+    c.cfg.blockDim = dim3(THREADS);
+    c.cfg.stream = s;
+    return c;
 }
 
 template <int TYPE>
@@ -195,9 +227,9 @@ static int run_extra(const View& v, float* dst, cudaStream_t s) {
     if (count == 0) {
         return JQ_OK;
     }
-    dequantize_extra_kernel<TYPE><<<(unsigned)((count / 4 + 255) / 256), 256, 0, s>>>(v.q, dst, count);
+    JQ_CUDA(cudaLaunchKernelEx(&launch_config((count / 4 + PIECES * THREADS - 1) / (PIECES * THREADS), s).cfg, dequantize_extra_kernel<TYPE>, (const uint8_t*)v.q, dst, count));
     count_launch();
-    return check_launch("dequantize_extra_kernel");
+    return JQ_OK;
 }
 
 template <int TYPE>
@@ -205,18 +237,18 @@ static int run(const View& v, float* dst, cudaStream_t s) {
     if (v.n == 0 || v.k == 0) {
         return JQ_OK;
     }
-    constexpr int64_t GROUP = 128 * 1024;  // rows per launch: a grid has at most 65535 rows of CTAs; a multiple of 128, so the tiles go on
+    constexpr int64_t GROUP = 128 * 1024;  // rows per launch, a multiple of 128, so the tiles go on: (at most 2^31 values) / 256 / ROWS tasks fit 32 bits
     const int64_t steps = tiled_steps(v.k);
     for (int64_t r0 = 0; r0 < v.n; r0 += GROUP) {
         View part = v;
         part.n = v.n - r0 < GROUP ? v.n - r0 : GROUP;
         part.q = v.q + tiled_index(r0, 0, steps) * (256 / Fmt<TYPE>::QK) * plane_q_bytes(TYPE);
         part.aux = v.aux == nullptr ? nullptr : v.aux + tiled_index(r0, 0, steps) * (256 / Fmt<TYPE>::QK) * plane_aux_bytes(TYPE);
-        const dim3 grid((unsigned)((steps + 7) / 8), (unsigned)((part.n + ROWS - 1) / ROWS));
-        dequantize_kernel<TYPE><<<grid, 256, 0, s>>>(part, dst + r0 * v.k);
+        const int64_t tasks = steps * ((part.n + ROWS - 1) / ROWS);
+        JQ_CUDA(cudaLaunchKernelEx(&launch_config((tasks + THREADS / 32 - 1) / (THREADS / 32), s).cfg, dequantize_kernel<TYPE>, part, dst + r0 * v.k, (int)steps));
         count_launch();
     }
-    return check_launch("dequantize_kernel");
+    return JQ_OK;
 }
 
 int launch_dequantize(const View& v, float* dst, cudaStream_t s) {
