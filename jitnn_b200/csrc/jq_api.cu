@@ -346,6 +346,16 @@ bool linear_takes_swiglu(const jq_weight* w, int64_t m) {
     return w->n > 0 && !(min_rows > 0 && m >= min_rows) && to_matrix_kernel(w, m);
 }
 
+// Whether these linears, on m rows of one x, all go to the rows kernel, whose image of x a kernel in front may then write.
+bool linears_take_rows(const jq_weight* const* ws, int count, int64_t m) {
+    const int64_t min_rows = g_prefill_min_rows.load();
+    bool rows = m <= 16 && !(min_rows > 0 && m >= min_rows);
+    for (int i = 0; i < count && rows; i++) {
+        rows = ws[i]->n > 0 && ws[i]->k == ws[0]->k && to_matrix_kernel(ws[i], m);
+    }
+    return rows;
+}
+
 // ---- linear on device pointers --------------------------------------------------------------------
 int linear_device(const jq_weight* w, const float* x, int64_t m, const float* bias, float* y, cudaStream_t s, bool x_remote) {
     View v = view_of(w);

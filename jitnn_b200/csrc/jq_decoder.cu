@@ -16,6 +16,7 @@
 #include "jq_prompt.cuh"
 #include "jq_q4k_image.cuh"
 #include "jq_q6k_image.cuh"
+#include "jq_rows_image.cuh"
 #include "jq_peer_device.cuh"
 
 namespace jq {
@@ -23,6 +24,7 @@ namespace jq {
 int linear_device(const jq_weight* w, const float* x, int64_t m, const float* bias, float* y, cudaStream_t s, bool x_remote = false);
 int linear_device_multi(const jq_weight* const* ws, int count, const float* x, int64_t m, float* const* ys, cudaStream_t s);
 bool linear_takes_swiglu(const jq_weight* w, int64_t m);
+bool linears_take_rows(const jq_weight* const* ws, int count, int64_t m);
 
 namespace {
 
@@ -107,9 +109,11 @@ __device__ __forceinline__ void store4(__nv_bfloat16* o, int64_t i, float4 v) {
 // all of its row's values in flight at once (128-bit loads) and keeps up to HOLD of them in registers for the second pass. 1024 threads a row
 // while each row can have an SM; with more rows 256 or 512, so that more of them are in flight at once.
 // Out: float, or bfloat16 for a linear that rounds its input to it.
-template <typename Out, int NORM_THREADS, int HOLD>
+// IMAGE: 8 or 16, the rows of the rows kernel's instance behind, whose image of x goes out in the place of the vector (its scales at `scales`; dim a multiple of 256,
+// which meets in shared memory): a launch less in front of every group of linears.
+template <typename Out, int NORM_THREADS, int HOLD, int IMAGE = 0>
 __global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ delta, const float* __restrict__ w,
-                                                                   float eps, Out* __restrict__ out, int dim) {
+                                                                   float eps, Out* __restrict__ out, int dim, float* scales) {
     asm volatile("griddepcontrol.launch_dependents;");  // launched programmatically, the kernel behind this one may be scheduled now ...
     const int nv = (dim & 3) == 0 ? dim >> 2 : 0;  // 128-bit pieces; a dim that is no multiple of 4 takes the scalar loops below
     float4 wv[HOLD];
@@ -122,7 +126,8 @@ __global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_kernel(float* __rest
     __shared__ float scratch[32];
     float* xr = x + (int64_t)blockIdx.x * dim;
     const float* dr = delta != nullptr ? delta + (int64_t)blockIdx.x * dim : nullptr;
-    Out* o = out + (int64_t)blockIdx.x * dim;
+    extern __shared__ __align__(16) float normed[];  // IMAGE: the row
+    Out* o = out + (IMAGE > 0 ? 0 : (int64_t)blockIdx.x * dim);
     float4 held[HOLD];
     float sq = 0.0f;
 #pragma unroll
@@ -155,11 +160,26 @@ __global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_kernel(float* __rest
     for (int h = 0; h < HOLD; h++) {
         const int i = threadIdx.x + h * NORM_THREADS;
         if (i < nv) {
-            store4(o, i, make_float4(held[h].x * inv * wv[h].x, held[h].y * inv * wv[h].y, held[h].z * inv * wv[h].z, held[h].w * inv * wv[h].w));
+            const float4 v = make_float4(held[h].x * inv * wv[h].x, held[h].y * inv * wv[h].y, held[h].z * inv * wv[h].z, held[h].w * inv * wv[h].w);
+            if constexpr (IMAGE > 0) {
+                store4(normed, i, v);
+            } else {
+                store4(o, i, v);
+            }
         }
     }
-    for (int i = rest + threadIdx.x; i < dim; i += NORM_THREADS) {
-        store1(o, i, xr[i] * inv * w[i]);
+    if constexpr (IMAGE > 0) {  // (the whole row is held)
+        __syncthreads();
+        const int lane = threadIdx.x & 31;
+        for (int u = threadIdx.x >> 5; u < dim / 256; u += NORM_THREADS / 32) {
+            const float4 a = reinterpret_cast<const float4*>(normed)[u * 64 + lane * 2], b = reinterpret_cast<const float4*>(normed)[u * 64 + lane * 2 + 1];
+            const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            rows::store_image<IMAGE>(v, u, blockIdx.x, reinterpret_cast<uint8_t*>(out), scales, lane);
+        }
+    } else {
+        for (int i = rest + threadIdx.x; i < dim; i += NORM_THREADS) {
+            store1(o, i, xr[i] * inv * w[i]);
+        }
     }
 }
 
@@ -302,39 +322,49 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_partial_kernel(const fl
     }
 }
 
-// The same for head sizes 64 and 128, all query heads that share a key/value head in one CTA: CTA (kv head, split, t) has its 64 keys and values
-// in registers (warp w keys 8w .. 8w + 7, a lane HD / 32 neighbouring dimensions of each) and goes through the group's query heads. With one CTA
+// The same for head sizes 64 and 128, all query heads that share a key/value head in one CTA: CTA (kv head, split, tokens) has its 64 keys and values
+// in registers (warp w keys 8w .. 8w + 7, a lane HD / 32 neighbouring dimensions of each) and goes through the group's query heads, of each of up to `take`
+// consecutive tokens of one sequence, which see the same keys (a batch's tokens do not: take 1). With one CTA
 // per query head, a group of eight read every cached byte eight times, and the dot products' shuffles, five per key, bound it (16 sequences of
-// 64 heads at position 256: 55 us). The warps go through up to GROUP_HEADS heads on their own and meet once for all of them: with a barrier and
+// 64 heads at position 256: 55 us); with one per token, a run of 14 tokens read the cache 14 times. The warps go through up to GROUP_HEADS heads on their own and meet once for all of them: with a barrier and
 // a merge for each head the kernel was a chain of those (587.5 us against 582.9 for a step of 16 sequences, 2 layers of the 70B width).
+// The call's own keys, from position pos0 on, come unrotated from k_new and v_new (row j - pos0 of consecutive tokens, row t of a batch); every CTA
+// rotates those it sees, and the queries, itself, and the one whose token a key is puts it into the cache, which nobody reads there in this launch.
+// (A kernel of its own for that took 3.5 us in front of this one.)
 constexpr int GROUP_THREADS = 256, GROUP_HEADS = 8;
-template <int HD>
-__global__ void __launch_bounds__(GROUP_THREADS) attention_group_kernel(const float* __restrict__ q, const float* __restrict__ k_cache,
-                                                                       const float* __restrict__ v_cache, float* __restrict__ part,
-                                                                       const int* __restrict__ pos0, int heads, int kv_heads, int splits, float scale,
-                                                                       int pos_step, int64_t tok_stride) {
+// MANY: take may be more than one.
+template <int HD, bool MANY>
+__global__ void __launch_bounds__(GROUP_THREADS, HD == 64 ? 3 : 2) attention_group_kernel(const float* __restrict__ q, const float* __restrict__ k_new, const float* __restrict__ v_new,
+                                                                       float* k_cache, float* v_cache, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+                                                                       float* __restrict__ part, const int* __restrict__ pos0, int heads, int kv_heads, int splits,
+                                                                       float scale, int pos_step, int64_t tok_stride, int tokens, int take) {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     static_assert(HD == 64 || HD == 128, "head sizes");
     constexpr int V = HD / 32;
     __shared__ __align__(16) float red[GROUP_HEADS][8][HD];
     __shared__ float stat[GROUP_HEADS][16];  // the warps' maxima, later their weights; their sums
-    const int kvh = blockIdx.x, sp = blockIdx.y, t = blockIdx.z, group = heads / kv_heads;
+    __shared__ __align__(16) float turned[GROUP_HEADS][HD];  // rotated queries
+    const int kvh = blockIdx.x, sp = blockIdx.y, group = heads / kv_heads;
+    const int t0 = MANY ? blockIdx.z * take : blockIdx.z, t1 = MANY ? min(t0 + take, tokens) : t0 + 1;  // tokens
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int keys = *pos0 + t * pos_step + 1, k0 = sp * ATT_CHUNK;
-    float* const out0 = part + (((int64_t)t * heads + (int64_t)kvh * group) * splits + sp) * (HD + 2);
-    const int64_t head_stride = (int64_t)splits * (HD + 2);
+    const int first = *pos0, keys = first + (t1 - 1) * pos_step + 1, k0 = sp * ATT_CHUNK;  // keys of the last token
+    const int items = (t1 - t0) * group;  // (token, query head)
+    auto token_of = [&](int item) { return MANY ? t0 + item / group : t0; };
+    auto head_of = [&](int item) { return kvh * group + (MANY ? item % group : item); };
+    auto result = [&](int item) { return part + (((int64_t)token_of(item) * heads + head_of(item)) * splits + sp) * (HD + 2); };
     if (k0 >= keys) {
-        for (int hh = tid; hh < group; hh += GROUP_THREADS) {
-            out0[hh * head_stride + HD] = -INFINITY;  // m
-            out0[hh * head_stride + HD + 1] = 0.0f;   // l
+        for (int item = tid; item < items; item += GROUP_THREADS) {
+            float* const out = result(item);
+            out[HD] = -INFINITY;  // m
+            out[HD + 1] = 0.0f;   // l
         }
         return;
     }
     const int cnt = keys - k0 < ATT_CHUNK ? keys - k0 : ATT_CHUNK;
     const int kv_dim = kv_heads * HD;
-    const float* kb = k_cache + t * tok_stride + (int64_t)(k0 + warp * 8) * kv_dim + kvh * HD + lane * V;
-    const float* vb = v_cache + t * tok_stride + (int64_t)(k0 + warp * 8) * kv_dim + kvh * HD + lane * V;
+    float* const kb = k_cache + t0 * tok_stride + (int64_t)(k0 + warp * 8) * kv_dim + kvh * HD + lane * V;
+    float* const vb = v_cache + t0 * tok_stride + (int64_t)(k0 + warp * 8) * kv_dim + kvh * HD + lane * V;
     auto get = [](const float* p, float (&r)[V]) {
         if constexpr (V == 4) {
             const float4 x = *reinterpret_cast<const float4*>(p);
@@ -352,25 +382,65 @@ __global__ void __launch_bounds__(GROUP_THREADS) attention_group_kernel(const fl
             kr[u][i] = vr[u][i] = 0.0f;
         }
         if (warp * 8 + u < cnt) {
-            get(kb + (int64_t)u * kv_dim, kr[u]);
-            get(vb + (int64_t)u * kv_dim, vr[u]);
+            const int own = k0 + warp * 8 + u - first;  // 0 and more: one of the call's own
+            const int64_t row = (int64_t)(pos_step != 0 ? own : t0) * kv_dim + kvh * HD + lane * V;
+            get(own < 0 ? kb + (int64_t)u * kv_dim : k_new + row, kr[u]);
+            get(own < 0 ? vb + (int64_t)u * kv_dim : v_new + row, vr[u]);
         }
     }
-    const float* qp = q + ((int64_t)t * heads + (int64_t)kvh * group) * HD + lane * V;
-    float qn[V];
-    get(qp, qn);
-    // after the halving exchange below a lane holds the score of key (lane >> 2), every key in four lanes
-    const int my_key = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
-    const bool seen = warp * 8 + my_key < cnt;
-    for (int hh = 0; hh < group; hh++) {
-        float qv[V];
+    // rotate-half: this lane's dimensions and those of the lane 16 further, the same angles
+    auto turn = [&](float (&x)[V], const float (&c)[V], const float (&s)[V]) {
 #pragma unroll
         for (int i = 0; i < V; i++) {
-            qv[i] = qn[i];
+            const float other = __shfl_xor_sync(0xffffffffu, x[i], 16);
+            x[i] = lane < 16 ? __fsub_rn(__fmul_rn(x[i], c[i]), __fmul_rn(other, s[i])) : __fadd_rn(__fmul_rn(other, s[i]), __fmul_rn(x[i], c[i]));
         }
-        if (hh + 1 < group) {
-            get(qp + (hh + 1) * HD, qn);
+    };
+    const int angle = (lane & 15) * V;
+    // the rotated queries of items base .. base + 7, one a warp
+    auto turn_queries = [&](int base) {
+        if (base + warp < items) {
+            const int t = token_of(base + warp);
+            const int64_t at = (int64_t)(first + t * pos_step) * (HD / 2) + angle;
+            float x[V], c[V], s[V];
+            get(q + ((int64_t)t * heads + head_of(base + warp)) * HD + lane * V, x);
+            get(cos_t + at, c);
+            get(sin_t + at, s);
+            turn(x, c, s);
+            if constexpr (V == 4) {
+                reinterpret_cast<float4*>(turned[warp])[lane] = make_float4(x[0], x[1], x[2], x[3]);
+            } else {
+                reinterpret_cast<float2*>(turned[warp])[lane] = make_float2(x[0], x[1]);
+            }
         }
+    };
+    turn_queries(0);
+    if (k0 + warp * 8 + 7 >= first) {
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int j = k0 + warp * 8 + u;
+            if (j >= first && j < keys) {
+                float c[V], s[V];
+                get(cos_t + (int64_t)j * (HD / 2) + angle, c);
+                get(sin_t + (int64_t)j * (HD / 2) + angle, s);
+                turn(kr[u], c, s);
+                if (pos_step == 0 || j - first >= t0) {
+#pragma unroll
+                    for (int i = 0; i < V; i++) {
+                        kb[(int64_t)u * kv_dim + i] = kr[u][i];
+                        vb[(int64_t)u * kv_dim + i] = vr[u][i];
+                    }
+                }
+            }
+        }
+    }
+    // after the halving exchange below a lane holds the score of key (lane >> 2), every key in four lanes
+    const int my_key = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+    __syncthreads();
+    for (int item = 0; item < items; item++) {
+        const int last = first + token_of(item) * pos_step - k0 - warp * 8;  // the warp's last key that the token sees
+        float qv[V];
+        get(turned[item % GROUP_HEADS] + lane * V, qv);
         float d[8];
 #pragma unroll
         for (int u = 0; u < 8; u++) {
@@ -397,13 +467,13 @@ __global__ void __launch_bounds__(GROUP_THREADS) attention_group_kernel(const fl
         }
         d[0] += __shfl_xor_sync(0xffffffffu, d[0], 2);
         d[0] += __shfl_xor_sync(0xffffffffu, d[0], 1);
-        const float sco = seen ? d[0] * scale : -INFINITY;
+        const float sco = my_key <= last ? d[0] * scale : -INFINITY;
         float mw = sco;
 #pragma unroll
         for (int o = 16; o >= 4; o >>= 1) {
             mw = fmaxf(mw, __shfl_xor_sync(0xffffffffu, mw, o));
         }
-        const float pj = mw == -INFINITY ? 0.0f : expf(sco - mw);  // 0 for the keys beyond the chunk's count
+        const float pj = mw == -INFINITY ? 0.0f : expf(sco - mw);  // 0 for the keys that the token does not see
         float lw = pj;
 #pragma unroll
         for (int o = 16; o >= 4; o >>= 1) {
@@ -419,10 +489,10 @@ __global__ void __launch_bounds__(GROUP_THREADS) attention_group_kernel(const fl
             const float w = __shfl_sync(0xffffffffu, pj, (u >> 2) * 16 + ((u >> 1) & 1) * 8 + (u & 1) * 4);
 #pragma unroll
             for (int i = 0; i < V; i++) {
-                acc[i] = fmaf(w, vr[u][i], acc[i]);
+                acc[i] = u <= last ? fmaf(w, vr[u][i], acc[i]) : acc[i];  // (a later token's value reaches nobody in front of it, whatever it holds)
             }
         }
-        const int at = hh % GROUP_HEADS;
+        const int at = item % GROUP_HEADS;
         if constexpr (V == 4) {
             reinterpret_cast<float4*>(red[at][warp])[lane] = make_float4(acc[0], acc[1], acc[2], acc[3]);
         } else {
@@ -432,13 +502,12 @@ __global__ void __launch_bounds__(GROUP_THREADS) attention_group_kernel(const fl
             stat[at][warp] = mw;
             stat[at][8 + warp] = lw;
         }
-        if (at < GROUP_HEADS - 1 && hh < group - 1) {
+        if (at < GROUP_HEADS - 1 && item < items - 1) {
             continue;
         }
-        // the 8 warps' results of heads hh - at .. hh, added up in warp order
+        // the 8 warps' results of items item - at .. item, added up in warp order
         __syncthreads();
-        float* const out = out0 + (hh - at) * head_stride;
-        if (tid < GROUP_HEADS * 8) {  // (whole warps; what lies in the places of heads beyond `at` goes nowhere)
+        if (tid < GROUP_HEADS * 8) {  // (whole warps; what lies in the places of items beyond `at` goes nowhere)
             const int w = tid & 7;
             float* const st = stat[tid >> 3];
             const float m = st[w];
@@ -447,7 +516,7 @@ __global__ void __launch_bounds__(GROUP_THREADS) attention_group_kernel(const fl
             for (int o = 4; o > 0; o >>= 1) {
                 M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
             }
-            const float wgt = expf(m - M);  // 0 for a warp without keys (warp 0 always has one)
+            const float wgt = m == -INFINITY ? 0.0f : expf(m - M);  // 0 for a warp without keys
             float l = wgt * st[8 + w];
 #pragma unroll
             for (int o = 4; o > 0; o >>= 1) {
@@ -455,8 +524,9 @@ __global__ void __launch_bounds__(GROUP_THREADS) attention_group_kernel(const fl
             }
             st[w] = wgt;
             if (w == 0 && (tid >> 3) <= at) {
-                out[(tid >> 3) * head_stride + HD] = M;
-                out[(tid >> 3) * head_stride + HD + 1] = l;
+                float* const out = result(item - at + (tid >> 3));
+                out[HD] = M;
+                out[HD + 1] = l;
             }
         }
         __syncthreads();
@@ -467,50 +537,86 @@ __global__ void __launch_bounds__(GROUP_THREADS) attention_group_kernel(const fl
             for (int wv = 0; wv < 8; wv++) {
                 sum = fmaf(stat[head][wv], red[head][wv][dd], sum);
             }
-            out[head * head_stride + dd] = sum;
+            result(item - at + head)[dd] = sum;
         }
-        if (hh < group - 1) {
-            __syncthreads();  // read by all before the next heads' results come
+        if (item < items - 1) {
+            turn_queries(item + 1);  // (all are done with the last eight since the first of these barriers)
+            __syncthreads();  // read by all before the next items' results come
         }
     }
 }
 
-// out[t, h, :] = sum_s exp(m_s - M) acc_s / sum_s exp(m_s - M) l_s over the splits of (t, h), in split order. The splits' maxima and sums are
-// read at once, one per thread; chunks without a visible key (those of a captured step beyond the position) have weight zero and are not read.
+// out[t, h, :] = sum_s exp(m_s - M) acc_s / sum_s exp(m_s - M) l_s over the splits of (t, h), in split order. A warp makes the weights of a head's splits, a lane a
+// split at a time; chunks without a visible key (those of a captured step beyond the position) have weight zero and are not read. (When every thread went
+// through the splits' exponentials by itself, 15 splits took 12.8 us.) A thread block takes 256 values of a token: IMAGE 0, they go to out; 8 or 16, they
+// become a step of the rows kernel's image.
 constexpr int MAX_SPLITS = 128;  // 8192 positions
-__global__ void attention_combine_kernel(const float* __restrict__ part, float* __restrict__ out, int heads, int head_dim, int stride_splits,
-                                         int splits) {
+template <int IMAGE>
+__global__ void __launch_bounds__(256) attention_combine_kernel(const float* __restrict__ part, float* out, int heads, int head_dim, int stride_splits, int splits, float* scales,
+                                                               int span) {
     asm volatile("griddepcontrol.launch_dependents;");  // launched programmatically, the kernel behind this one may be scheduled now ...
     asm volatile("griddepcontrol.wait;" ::: "memory");  // ... and this one touches memory only when the kernel before it has finished
     // stride_splits = chunks the partial buffer was laid out for, splits = chunks written by this call
-    __shared__ float wm[MAX_SPLITS], wl[MAX_SPLITS];
-    const int h = blockIdx.x, t = blockIdx.y;
-    const float* p = part + ((int64_t)t * heads + h) * stride_splits * (head_dim + 2);
-    for (int s = threadIdx.x; s < splits; s += blockDim.x) {
-        wm[s] = p[(int64_t)s * (head_dim + 2) + head_dim];
-        wl[s] = p[(int64_t)s * (head_dim + 2) + head_dim + 1];
-    }
-    __syncthreads();
-    float M = -INFINITY;
-    for (int s = 0; s < splits; s++) {
-        M = fmaxf(M, wm[s]);
-    }
-    float L = 0.0f;
-    for (int s = 0; s < splits; s++) {
-        if (wm[s] != -INFINITY) {
-            L = fmaf(expf(wm[s] - M), wl[s], L);
+    constexpr int HEADS = 10;  // that a thread block's `span` values belong to, at most: 256 values of heads of 32 and more, else eight heads
+    __shared__ float weight[HEADS][MAX_SPLITS], total[HEADS];
+    __shared__ __align__(16) float merged[256];
+    const int t = blockIdx.y, tid = threadIdx.x, lane = tid & 31, dim = heads * head_dim;
+    const int v0 = (int)blockIdx.x * span, v1 = min(v0 + span, dim), h0 = v0 / head_dim, here = (v1 - 1) / head_dim - h0 + 1;  // the first head, how many
+    const int64_t row = (int64_t)stride_splits * (head_dim + 2);
+    const float* const p = part + ((int64_t)t * heads + h0) * row;
+    for (int h = tid >> 5; h < here; h += 8) {
+        const float* const ph = p + h * row + head_dim;
+        float m[MAX_SPLITS / 32], M = -INFINITY, L = 0.0f;
+#pragma unroll
+        for (int i = 0; i < MAX_SPLITS / 32; i++) {
+            m[i] = 32 * i + lane < splits ? ph[(int64_t)(32 * i + lane) * (head_dim + 2)] : -INFINITY;
+            M = fmaxf(M, m[i]);
         }
-    }
-    for (int d = threadIdx.x; d < head_dim; d += blockDim.x) {
-        float acc = 0.0f;
-#pragma unroll 4
-        for (int s = 0; s < splits; s++) {
-            const float m = wm[s];
-            if (m != -INFINITY) {
-                acc = fmaf(expf(m - M), p[(int64_t)s * (head_dim + 2) + d], acc);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+        }
+#pragma unroll
+        for (int i = 0; i < MAX_SPLITS / 32; i++) {
+            if (32 * i + lane < splits) {
+                const float e = m[i] == -INFINITY ? -1.0f : expf(m[i] - M);  // -1: no visible key
+                weight[h][32 * i + lane] = e;
+                L = !(e < 0.0f) ? fmaf(e, ph[(int64_t)(32 * i + lane) * (head_dim + 2) + 1], L) : L;
             }
         }
-        out[((int64_t)t * heads + h) * head_dim + d] = acc / L;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            L += __shfl_xor_sync(0xffffffffu, L, o);
+        }
+        if (lane == 0) {
+            total[h] = L;
+        }
+    }
+    __syncthreads();
+    const int at = v0 + tid;
+    float v = 0.0f;
+    if (at < v1) {
+        const int h = at / head_dim - h0;
+        const float* const pd = p + h * row + at % head_dim;
+#pragma unroll 8
+        for (int s = 0; s < splits; s++) {
+            const float e = weight[h][s];
+            v = !(e < 0.0f) ? fmaf(e, pd[(int64_t)s * (head_dim + 2)], v) : v;
+        }
+        v /= total[h];
+    }
+    if constexpr (IMAGE == 0) {
+        if (at < v1) {
+            out[(int64_t)t * dim + at] = v;
+        }
+    } else {
+        merged[tid] = v;
+        __syncthreads();
+        if (tid < 32) {
+            const float4 a = reinterpret_cast<const float4*>(merged)[lane * 2], b = reinterpret_cast<const float4*>(merged)[lane * 2 + 1];
+            const float w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            rows::store_image<IMAGE>(w, blockIdx.x, t, reinterpret_cast<uint8_t*>(out), scales, lane);
+        }
     }
 }
 
@@ -961,15 +1067,31 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// The norm of up to 16 rows, each held by its thread block, as the rows kernel's image.
+constexpr int NORM_IMAGE_DIM = 11264;  // (a row in the shared memory that needs no opt-in)
+cudaError_t launch_add_rmsnorm_image(int rows, cudaStream_t s, float* x, const float* delta, const float* w, float eps, uint8_t* image, float* scales, int dim) {
+    auto kernel = rows <= 8 ? add_rmsnorm_kernel<float, 1024, 4, 8> : add_rmsnorm_kernel<float, 1024, 4, 16>;
+    return launch_pdl(kernel, dim3((unsigned)rows), dim3(1024), (size_t)dim * sizeof(float), s, true, x, delta, w, eps, reinterpret_cast<float*>(image), dim, scales);
+}
+
+// The attention's merged results of T tokens: to `out`, or (image not null) as the rows kernel's image.
+cudaError_t launch_combine(int T, int heads, int head_dim, int stride_splits, int splits, const float* part, float* out, uint8_t* image, float* scales, bool programmatic,
+                           cudaStream_t s) {
+    auto kernel = image == nullptr ? attention_combine_kernel<0> : (T <= 8 ? attention_combine_kernel<8> : attention_combine_kernel<16>);
+    const int span = head_dim >= 32 ? 256 : 8 * head_dim;
+    return launch_pdl(kernel, dim3((unsigned)((heads * head_dim + span - 1) / span), (unsigned)T), dim3(256), 0, s, programmatic, part,
+                      image == nullptr ? out : reinterpret_cast<float*>(image), heads, head_dim, stride_splits, splits, scales, span);
+}
+
 template <typename Out>
 cudaError_t launch_add_rmsnorm(int rows, cudaStream_t s, bool programmatic, float* x, const float* delta, const float* w, float eps, Out* out, int dim) {
     if (rows <= 148) {
-        return launch_pdl(add_rmsnorm_kernel<Out, 1024, 4>, dim3((unsigned)rows), dim3(1024), 0, s, programmatic, x, delta, w, eps, out, dim);
+        return launch_pdl(add_rmsnorm_kernel<Out, 1024, 4>, dim3((unsigned)rows), dim3(1024), 0, s, programmatic, x, delta, w, eps, out, dim, (float*)nullptr);
     }
     if (dim <= 4096) {
-        return launch_pdl(add_rmsnorm_kernel<Out, 256, 4>, dim3((unsigned)rows), dim3(256), 0, s, programmatic, x, delta, w, eps, out, dim);
+        return launch_pdl(add_rmsnorm_kernel<Out, 256, 4>, dim3((unsigned)rows), dim3(256), 0, s, programmatic, x, delta, w, eps, out, dim, (float*)nullptr);
     }
-    return launch_pdl(add_rmsnorm_kernel<Out, 512, 4>, dim3((unsigned)rows), dim3(512), 0, s, programmatic, x, delta, w, eps, out, dim);
+    return launch_pdl(add_rmsnorm_kernel<Out, 512, 4>, dim3((unsigned)rows), dim3(512), 0, s, programmatic, x, delta, w, eps, out, dim, (float*)nullptr);
 }
 
 // The same for a kernel whose whole grid is one thread-block cluster.
@@ -1556,19 +1678,25 @@ static int enqueue_forward_fused(jq_decoder* d, int max_keys, const TokenArgs* t
 
 static int enqueue_forward_sharded(jq_decoder* d, int T, int max_keys, const TokenArgs* ta, cudaStream_t s);
 
-// The general path's attention of T tokens over `splits_now` chunks of keys, into the decoder's partial results.
-static cudaError_t launch_attention(jq_decoder* d, int heads, int kv_heads, int T, int splits_now, const float* kc, const float* vc, float scale, int pos_step,
-                                    int64_t tok_stride, bool programmatic, cudaStream_t s) {
-    if (d->head_dim == 128) {
-        return launch_pdl(attention_group_kernel<128>, dim3(kv_heads, splits_now, T), dim3(GROUP_THREADS), 0, s, programmatic, d->q, kc, vc, d->att_part, d->pos, heads,
-                          kv_heads, d->splits, scale, pos_step, tok_stride);
+// The general path's attention of T tokens over `splits_now` chunks of keys, into the decoder's partial results, with the rotation of queries and keys and the
+// append to the cache: part of the kernel for head sizes 64 and 128, a launch in front of it for others.
+static cudaError_t launch_attention(jq_decoder* d, int heads, int kv_heads, int T, int splits_now, float* kc, float* vc, float scale, int pos_step, int64_t tok_stride,
+                                    bool programmatic, cudaStream_t s) {
+    count_launch(1);
+    if (d->head_dim == 128 || d->head_dim == 64) {
+        // consecutive tokens share keys: as many of them per thread block as leave two thread blocks for every SM
+        const int pairs = kv_heads * splits_now, parts = pairs >= 296 ? 1 : (296 + pairs - 1) / pairs, take = pos_step == 0 || parts >= T ? 1 : (T + parts - 1) / parts;
+        auto kernel = d->head_dim == 128 ? (take > 1 ? attention_group_kernel<128, true> : attention_group_kernel<128, false>)
+                                         : (take > 1 ? attention_group_kernel<64, true> : attention_group_kernel<64, false>);
+        return launch_pdl(kernel, dim3(kv_heads, splits_now, (T + take - 1) / take), dim3(GROUP_THREADS), 0, s, programmatic, d->q, d->k, d->v, kc, vc, d->cos_t, d->sin_t,
+                          d->att_part, d->pos, heads, kv_heads, d->splits, scale, pos_step, tok_stride, T, take);
     }
-    if (d->head_dim == 64) {
-        return launch_pdl(attention_group_kernel<64>, dim3(kv_heads, splits_now, T), dim3(GROUP_THREADS), 0, s, programmatic, d->q, kc, vc, d->att_part, d->pos, heads,
-                          kv_heads, d->splits, scale, pos_step, tok_stride);
-    }
-    return launch_pdl(attention_partial_kernel, dim3(heads, splits_now, T), dim3(ATT_THREADS), 0, s, programmatic, d->q, kc, vc, d->att_part, d->pos, heads, kv_heads,
-                      d->head_dim, d->splits, scale, pos_step, tok_stride);
+    const cudaError_t e = launch_pdl(rope_store_kernel, dim3(T, heads + 2 * kv_heads), dim3(d->head_dim / 2), 0, s, programmatic, d->q, d->k, d->v, kc, vc, d->cos_t, d->sin_t,
+                                     d->pos, heads, kv_heads, d->head_dim, pos_step, tok_stride);
+    count_launch(1);
+    return e != cudaSuccess ? e
+                            : launch_pdl(attention_partial_kernel, dim3(heads, splits_now, T), dim3(ATT_THREADS), 0, s, programmatic, d->q, kc, vc, d->att_part, d->pos, heads,
+                                         kv_heads, d->head_dim, d->splits, scale, pos_step, tok_stride);
 }
 
 // Enqueues the forward of T tokens on s. Tokens and position come either from kernel arguments (ta != nullptr) or, for
@@ -1615,6 +1743,41 @@ static int enqueue_forward(jq_decoder* d, int T, int max_keys, const TokenArgs* 
         if (rc == JQ_OK) pdl_err = launch_pdl(embed_kernel, dim3(T), dim3(256), 0, s, true, d->tokens, d->embed, d->x, dim, d->vocab);
         LAUNCHED("embed_kernel");
     }
+    auto CKL = [&](cudaError_t e, const char* name) {
+        if (rc == JQ_OK && e != cudaSuccess) {
+            rc = cuda_fail(e, name);
+        }
+    };
+    // linears of the rows kernel on an image that the kernel in front has written
+    auto ROWS = [&](const jq_weight* const* w, int count, float* const* ys) {
+        View vs[3];
+        for (int i = 0; i < count; i++) {
+            vs[i] = View{w[i]->q, w[i]->aux, w[i]->n, w[i]->k, w[i]->type};
+        }
+        if (rc == JQ_OK) {
+            rc = launch_rows(vs, count, nullptr, nullptr, T, nullptr, ys, s);
+        }
+    };
+    // x += delta, its norm, and the linears on that
+    auto NORMED = [&](const float* delta, const float* norm_w, const jq_weight* const* w, int count, float* const* ys) {
+        count_launch(1);
+        if (dim % 256 == 0 && dim <= NORM_IMAGE_DIM && linears_take_rows(w, count, T)) {
+            uint8_t* image = nullptr;
+            float* scales = nullptr;
+            rc = rc == JQ_OK ? rows_image(s, T, dim, &image, &scales) : rc;
+            if (rc == JQ_OK) {
+                CKL(launch_add_rmsnorm_image(T, s, d->x, delta, norm_w, d->eps, image, scales, dim), "add_rmsnorm_kernel");
+                ROWS(w, count, ys);
+            }
+            return;
+        }
+        if (rc == JQ_OK) {
+            CKL(launch_add_rmsnorm<float>(T, s, true, d->x, delta, norm_w, d->eps, d->xn, dim), "add_rmsnorm_kernel");
+        }
+        if (rc == JQ_OK) {
+            rc = count > 1 ? linear_device_multi(w, count, d->xn, T, ys, s) : linear_device(w[0], d->xn, T, nullptr, ys[0], s);
+        }
+    };
     const float scale = (float)(1.0 / std::sqrt((double)hd));
     // caches are [sequence][layer][position][kv_dim]; a call works on one sequence, or on one token of each of the first T
     const size_t seq_elems = (size_t)d->layers * d->max_seq * kv_dim, seq_base = (size_t)d->cur_seq * seq_elems;
@@ -1625,30 +1788,31 @@ static int enqueue_forward(jq_decoder* d, int T, int max_keys, const TokenArgs* 
         float* kc = d->k_cache + seq_base + (size_t)l * d->max_seq * kv_dim;
         float* vc = d->v_cache + seq_base + (size_t)l * d->max_seq * kv_dim;
         // attention block; the residual add of the previous block's feed-forward output is fused into this norm
-        if (rc == JQ_OK) pdl_err = launch_add_rmsnorm<float>(T, s, true, d->x, l == 0 ? nullptr : d->proj, d->norms + (size_t)(2 * l) * dim, d->eps, d->xn, dim);
-        LAUNCHED("add_rmsnorm_kernel");
-        {
-            float* const qkv[3] = {d->q, d->k, d->v};
-            if (rc == JQ_OK) rc = linear_device_multi(L, 3, d->xn, T, qkv, s);
-        }
+        float* const qkv[3] = {d->q, d->k, d->v};
+        NORMED(l == 0 ? nullptr : d->proj, d->norms + (size_t)(2 * l) * dim, L, 3, qkv);
         if (rc != JQ_OK) break;
-        if (rc == JQ_OK) pdl_err = launch_pdl(rope_store_kernel, dim3(T, d->heads + 2 * d->kv_heads), dim3(hd / 2), 0, s, true, d->q, d->k, d->v, kc, vc, d->cos_t, d->sin_t, d->pos, d->heads, d->kv_heads, hd, pos_step, tok_stride);
-        LAUNCHED("rope_store_kernel");
         // only the key chunks that can hold a position of this call are launched (all of them inside the captured graph)
         const int splits_now = (max_keys + ATT_CHUNK - 1) / ATT_CHUNK;
-        if (rc == JQ_OK) pdl_err = launch_attention(d, d->heads, d->kv_heads, T, splits_now, kc, vc, scale, pos_step, tok_stride, true, s);
-        LAUNCHED("attention_group_kernel");
-        if (rc == JQ_OK) pdl_err = launch_pdl(attention_combine_kernel, dim3(d->heads, T), dim3(hd < 128 ? hd : 128), 0, s, true, d->att_part, d->att, d->heads, hd, d->splits, splits_now);
-        LAUNCHED("attention_combine_kernel");
-        LIN(L[3], d->att, d->proj);
+        CKL(launch_attention(d, d->heads, d->kv_heads, T, splits_now, kc, vc, scale, pos_step, tok_stride, true, s), "attention_group_kernel");
+        {
+            uint8_t* image = nullptr;
+            float* scales = nullptr;
+            if (rc == JQ_OK && dim % 256 == 0 && hd >= 32 && 256 % hd == 0 && linears_take_rows(L + 3, 1, T)) {
+                rc = rows_image(s, T, dim, &image, &scales);
+            }
+            if (rc != JQ_OK) break;
+            count_launch(1);
+            CKL(launch_combine(T, d->heads, hd, d->splits, splits_now, d->att_part, d->att, image, scales, true, s), "attention_combine_kernel");
+            if (image != nullptr) {
+                ROWS(L + 3, 1, &d->proj);
+            } else {
+                LIN(L[3], d->att, d->proj);
+            }
+        }
         if (rc != JQ_OK) break;
         // feed-forward block
-        if (rc == JQ_OK) pdl_err = launch_add_rmsnorm<float>(T, s, true, d->x, d->proj, d->norms + (size_t)(2 * l + 1) * dim, d->eps, d->xn, dim);
-        LAUNCHED("add_rmsnorm_kernel");
-        {
-            float* const gu[2] = {d->gate, d->up};
-            if (rc == JQ_OK) rc = linear_device_multi(L + 4, 2, d->xn, T, gu, s);
-        }
+        float* const gu[2] = {d->gate, d->up};
+        NORMED(d->proj, d->norms + (size_t)(2 * l + 1) * dim, L + 4, 2, gu);
         if (rc != JQ_OK) break;
         if (linear_takes_swiglu(L[6], T)) {
             rc = launch_matmul_f32_swiglu(View{L[6]->q, L[6]->aux, L[6]->n, L[6]->k, L[6]->type}, d->gate, d->up, T, d->proj, s);
@@ -1660,9 +1824,7 @@ static int enqueue_forward(jq_decoder* d, int T, int max_keys, const TokenArgs* 
         }
     }
     if (rc == JQ_OK) {
-        if (rc == JQ_OK) pdl_err = launch_add_rmsnorm<float>(T, s, true, d->x, d->proj, d->norms + (size_t)(2 * d->layers) * dim, d->eps, d->xn, dim);
-        LAUNCHED("add_rmsnorm_kernel");
-        LIN(d->output, d->xn, d->logits);
+        NORMED(d->proj, d->norms + (size_t)(2 * d->layers) * dim, &d->output, 1, &d->logits);
     }
     if (rc == JQ_OK) {
         if (rc == JQ_OK) pdl_err = launch_pdl(argmax_split_kernel, dim3(ARGMAX_CTAS, T), dim3(256), 0, s, true, d->logits, d->vocab, d->argmax_v, d->argmax_i,
@@ -1816,16 +1978,12 @@ static int enqueue_forward_sharded(jq_decoder* d, int T, int max_keys, const Tok
             // the norm behind it finds the vector complete
             if (rc == JQ_OK) rc = peer_linear_q4k_imaged(L[3], shard_image(d, 5), dim, d->rank * dim_l, d->peer_buf, d->area[1], d->stage[1], d->rank, G, s, true, false);
         } else {
-            rope_store_kernel<<<dim3(T, heads + 2 * kv_heads), hd / 2, 0, s>>>(d->q, d->k, d->v, kc, vc, d->cos_t, d->sin_t, d->pos, heads, kv_heads, hd, pos_step,
-                                                                               tok_stride);
-            LAUNCHED("rope_store_kernel");
-            if (rc == JQ_OK) {
-                const cudaError_t e = launch_attention(d, heads, kv_heads, T, splits_now, kc, vc, scale, pos_step, tok_stride, false, s);
-                if (e != cudaSuccess) rc = cuda_fail(e, "attention_group_kernel");
+            cudaError_t e = launch_attention(d, heads, kv_heads, T, splits_now, kc, vc, scale, pos_step, tok_stride, false, s);
+            if (e == cudaSuccess) {
+                count_launch(1);
+                e = launch_combine(T, heads, hd, d->splits, splits_now, d->att_part, d->att, nullptr, nullptr, false, s);
             }
-            LAUNCHED("attention_group_kernel");
-            attention_combine_kernel<<<dim3(heads, T), hd < 128 ? hd : 128, 0, s>>>(d->att_part, d->att, heads, hd, d->splits, splits_now);
-            LAUNCHED("attention_combine_kernel");
+            if (rc == JQ_OK && e != cudaSuccess) rc = cuda_fail(e, "attention");
             GATHER(d->att, dim, dim_l, 0);
             PEER_LIN(L[3], A, dim, dim_l, 1);
         }

@@ -5,14 +5,11 @@
 namespace jq {
 namespace rows {
 
-// x [m, k] FP32 (or silu(x) * up) -> per 256-wide step of k its image (jq_rows.cuh) and a scale per row: the row's 256 values times a power of two that
-// brings the largest to [2^9, 2^10), hi = that rounded to half precision, lo = the rest rounded to half precision: 22 significant bits for
-// everything down to 2^-13 of the largest. NT: 8 or 16 rows. A row's 256 that hold a NaN or an Inf get the scale NaN, which reaches every output of that row. One
-// warp per row and step, eight values a lane; rows from m on are zeros. Memory bound: 4 bytes read and 4.5 written (to L2) a value.
+// x [m, k] FP32 (or silu(x) * up) -> its image (jq_rows_image.cuh), rows from m on zeros. One warp per row and 256-wide step of k, eight values a lane. Memory bound:
+// 4 bytes read and 4.5 written (to L2) a value.
 template <int NT>
 __global__ void __launch_bounds__(128) image_kernel(const float* __restrict__ x, const float* __restrict__ up, int m, int64_t k, int units, uint8_t* __restrict__ image,
                                                     float* __restrict__ scales, int vec) {
-    constexpr int N = 2 * NT, STEP = step_bytes(NT);
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int64_t task = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -38,43 +35,7 @@ __global__ void __launch_bounds__(128) image_kernel(const float* __restrict__ x,
             v[i] = (v[i] / (1.0f + expf(-v[i]))) * g;
         }
     }
-    uint32_t am = 0;  // the largest magnitude as bits: an Inf or a NaN is larger than any number
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        am = max(am, __float_as_uint(v[i]) & 0x7fffffffu);
-    }
-    am = __reduce_max_sync(0xffffffffu, am);
-    const bool bad = am >= 0x7f800000u;
-    uint32_t e = am >> 23;
-    e = e < 14u ? 14u : (e > 254u ? 254u : e);
-    const float f = __uint_as_float((263u - e) << 23);
-    uint32_t hi[4], lo[4];  // of four values 0 and 2, 1 and 3
-    float sum = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const float a = v[(i >> 1) * 4 + (i & 1)] * f, c = v[(i >> 1) * 4 + (i & 1) + 2] * f;
-        mm::split_pair(a, c, hi[i], lo[i]);
-        const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hi[i])), l = __half22float2(*reinterpret_cast<const __half2*>(&lo[i]));
-        sum += (h.x + l.x) + (h.y + l.y);
-    }
-    // lane = step of 16 and half of it; columns row (hi) and NT + row (lo), 128 bytes per eight columns
-    uint8_t* const unit = image + (int64_t)u * image_bytes(NT);
-    const int col = (row >> 3) * 128 + (row & 7) * 16;
-    uint8_t* const to = unit + (lane >> 1) * STEP + (lane & 1) * (N * 16) + col;
-    *reinterpret_cast<uint4*>(to) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-    *reinterpret_cast<uint4*>(to + NT * 16) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-    // the sums over runs of 32 (four lanes), up to 2^15, twice
-    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-    const __half sh = __float2half_rn(sum), sl = __float2half_rn(sum - __half2float(sh));
-    if ((lane & 3) == 0) {
-        __half* const run = reinterpret_cast<__half*>(unit + 16 * STEP + col) + (lane >> 2);
-        run[0] = run[N * 8] = sh;
-        run[NT * 8] = run[(N + NT) * 8] = sl;
-    }
-    if (lane == 0) {
-        scales[(int64_t)u * NT + row] = bad ? __uint_as_float(0x7fc00000u) : __uint_as_float((e - 9u) << 23);
-    }
+    store_image<NT>(v, u, row, image, scales, lane);
 }
 
 static int launch_any(int type, Args& a, int ctas, bool after, cudaStream_t s) {
@@ -96,24 +57,32 @@ constexpr int slot_of(int m) { return m < 5 ? 0 : SLOT; }
 
 }  // namespace rows
 
+// Where the image of m rows of x for the next product on `s` goes, for a kernel that writes it itself.
+int rows_image(cudaStream_t s, int m, int64_t k, uint8_t** image, float** scales) {
+    using namespace rows;
+    const size_t units = (size_t)tiled_steps(k);
+    const int rc = scratch_for_slot(s, slot_of(m), units * (image_bytes(m < 5 ? 8 : MAX_NT) + MAX_NT * sizeof(float)), image);
+    *scales = reinterpret_cast<float*>(*image + units * image_bytes(nt_of(m)));
+    return rc;
+}
+
 // ys[i] [rows, n_i] = x . W_i^T (+ bias for the first), x [rows, k] or silu(x) * up, for up to three weights of one k: one image, the weights of one
-// format in one launch.
+// format in one launch. x null: the kernel in front has written the image.
 int launch_rows(const View* vs, int count, const float* x, const float* up, int m, const float* bias, float* const* ys, cudaStream_t s) {
     using namespace rows;
     const int64_t k = vs[0].k;
-    const int units = (int)tiled_steps(k);
+    const int units = (int)tiled_steps(k), nt = nt_of(m);
     int* status = nullptr;
     uint8_t* image = nullptr;
+    float* scales = nullptr;
     int rc = status_word(&status);
     if (rc == JQ_OK) {
-        rc = scratch_for_slot(s, slot_of(m), (size_t)units * (image_bytes(m < 5 ? 8 : MAX_NT) + MAX_NT * sizeof(float)), &image);
+        rc = rows_image(s, m, k, &image, &scales);
     }
     if (rc != JQ_OK) {
         return rc;
     }
-    const int nt = m <= 8 ? 8 : 16;
-    float* const scales = reinterpret_cast<float*>(image + (size_t)units * image_bytes(nt));
-    {
+    if (x != nullptr) {
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -33,6 +33,7 @@
 #pragma once
 
 #include "jq_matmul.cuh"
+#include "jq_rows_image.cuh"
 
 namespace jq {
 namespace rows {
@@ -51,9 +52,6 @@ using mm::unpack2;
 
 constexpr int RANGES = 8;
 constexpr int MAX_WEIGHTS = 3;
-constexpr int MAX_NT = 16;           // NT: rows of x that an instance takes, 8 or 16; 2 NT columns
-__host__ __device__ constexpr int step_bytes(int nt) { return 2 * nt * 32; }         // 16 k of the image: [8 k][8 columns][8 rows of 16 bytes]
-__host__ __device__ constexpr int image_bytes(int nt) { return 17 * step_bytes(nt); }  // a unit: 256 k, then the sums of x over its runs of 32, twice, as 16 more k
 constexpr int MAX_RAW = 6, MAX_IMG = 6, MAX_OPERANDS = 4, MAX_ACC = 4, MAX_FACTORS = 8;
 
 struct Args {
