@@ -751,10 +751,18 @@ __global__ void __launch_bounds__(ATTF_THREADS, 3) attention_image_kernel(const 
     // The position was set before the first kernel of this step started, and the cached keys and values of earlier
     // positions by earlier steps: both are read before the wait for the kernel in front, so that a CTA scheduled while that
     // kernel still runs has its cache lines on the way.
-    const int h = blockIdx.x, sp = blockIdx.y, splits = gridDim.y;
+    const int h = blockIdx.x, sp = blockIdx.y;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int pos = *pos0, keys = pos + 1, k0 = sp * ATT_CHUNK;
+    const int splits = (keys + ATT_CHUNK - 1) / ATT_CHUNK;  // chunks with a visible key; thread blocks of others (a captured step reaches further) have nothing to do
     const int kv_dim = kv_heads * HD, group = heads / kv_heads, kvh = h / group;
+    if (sp >= splits) {
+        pdl_enter();
+        if constexpr (PEER) {
+            peer_publish(pi.flags, pi.rank, pi.world, false, nullptr, false);  // this CTA stored nothing to a peer
+        }
+        return;
+    }
     float* out = part + ((int64_t)h * stride_splits + sp) * (HD + 2);
     const int cnt = keys - k0 < ATT_CHUNK ? keys - k0 : ATT_CHUNK;
     // Warp w owns keys 8w .. 8w + 7 of the chunk, a lane four consecutive dimensions of each. The keys wait in registers, the values in shared
@@ -773,7 +781,7 @@ __global__ void __launch_bounds__(ATTF_THREADS, 3) attention_image_kernel(const 
         }
     }
     pdl_enter();
-    if (k0 < keys) {
+    {
         const bool has_new = pos < k0 + ATT_CHUNK;  // the new token's key and value belong to this chunk
         if (tid < HALF) {
             const float c = cos_t[pos * HALF + tid], s = sin_t[pos * HALF + tid];
@@ -802,34 +810,53 @@ __global__ void __launch_bounds__(ATTF_THREADS, 3) attention_image_kernel(const 
         __syncthreads();
         // this warp's scores, its own running maximum and sum of exponentials, and its weighted sum of values
         const float4 qv = reinterpret_cast<const float4*>(qs)[lane];
-        float sco[8], mw = -INFINITY;
+        float d[8];
 #pragma unroll
         for (int u = 0; u < 8; u++) {
-            const int j = warp * 8 + u;
-            if (k0 + j == pos) {
+            if (k0 + warp * 8 + u == pos) {
                 kreg[u] = reinterpret_cast<const float4*>(knew)[lane];
             }
-            float dot = fmaf(qv.x, kreg[u].x, fmaf(qv.y, kreg[u].y, fmaf(qv.z, kreg[u].z, qv.w * kreg[u].w)));
+            d[u] = fmaf(qv.x, kreg[u].x, fmaf(qv.y, kreg[u].y, fmaf(qv.z, kreg[u].z, qv.w * kreg[u].w)));
+        }
+        // eight sums over 32 lanes in nine shuffles: exchange halves of the keys, then sum the last two bits of the lane
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                dot += __shfl_xor_sync(0xffffffffu, dot, o);
-            }
-            sco[u] = j < cnt ? dot * scale : -INFINITY;
-            mw = fmaxf(mw, sco[u]);
+        for (int i = 0; i < 4; i++) {
+            const float mine = (lane & 16) ? d[i + 4] : d[i], other = (lane & 16) ? d[i] : d[i + 4];
+            d[i] = mine + __shfl_xor_sync(0xffffffffu, other, 16);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const float mine = (lane & 8) ? d[i + 2] : d[i], other = (lane & 8) ? d[i] : d[i + 2];
+            d[i] = mine + __shfl_xor_sync(0xffffffffu, other, 8);
+        }
+        {
+            const float mine = (lane & 4) ? d[1] : d[0], other = (lane & 4) ? d[0] : d[1];
+            d[0] = mine + __shfl_xor_sync(0xffffffffu, other, 4);
+        }
+        d[0] += __shfl_xor_sync(0xffffffffu, d[0], 2);
+        d[0] += __shfl_xor_sync(0xffffffffu, d[0], 1);
+        const int my_key = warp * 8 + ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);  // in four lanes each
+        const float sco = my_key < cnt ? d[0] * scale : -INFINITY;
+        float mw = sco;
+#pragma unroll
+        for (int o = 16; o >= 4; o >>= 1) {
+            mw = fmaxf(mw, __shfl_xor_sync(0xffffffffu, mw, o));
+        }
+        const float pk = mw == -INFINITY ? 0.0f : expf(sco - mw);  // 0 for the keys beyond the chunk's count
+        float lw = pk;
+#pragma unroll
+        for (int o = 16; o >= 4; o >>= 1) {
+            lw += __shfl_xor_sync(0xffffffffu, lw, o);
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
-        float lw = 0.0f;
         float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (mw != -INFINITY) {
 #pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const float pj = expf(sco[u] - mw);  // 0 for the keys beyond the chunk's count
-                lw += pj;
-                const int j = warp * 8 + u;
-                if (j < cnt) {
-                    const float4 vv = *reinterpret_cast<const float4*>(k0 + j == pos ? vnew + 4 * lane : &vs[j][4 * lane]);
-                    acc.x = fmaf(pj, vv.x, acc.x); acc.y = fmaf(pj, vv.y, acc.y); acc.z = fmaf(pj, vv.z, acc.z); acc.w = fmaf(pj, vv.w, acc.w);
-                }
+        for (int u = 0; u < 8; u++) {
+            const float pj = __shfl_sync(0xffffffffu, pk, (u >> 2) * 16 + ((u >> 1) & 1) * 8 + (u & 1) * 4);
+            const int j = warp * 8 + u;
+            if (j < cnt) {
+                const float4 vv = *reinterpret_cast<const float4*>(k0 + j == pos ? vnew + 4 * lane : &vs[j][4 * lane]);
+                acc.x = fmaf(pj, vv.x, acc.x); acc.y = fmaf(pj, vv.y, acc.y); acc.z = fmaf(pj, vv.z, acc.z); acc.w = fmaf(pj, vv.w, acc.w);
             }
         }
         reinterpret_cast<float4*>(red[warp])[lane] = acc;
@@ -859,16 +886,13 @@ __global__ void __launch_bounds__(ATTF_THREADS, 3) attention_image_kernel(const 
                 out[HD + 1] = l;
             }
         }
-    } else if (tid == 0) {
-        out[HD] = -INFINITY;  // no key of this chunk is visible yet
-        out[HD + 1] = 0.0f;
     }
     // ---- the last CTA of this pair of heads merges the chunks ---------------------------------------------------------------
-    __threadfence();
     __syncthreads();
     const int sb = h >> 1;  // 2 heads of 128 = one super-block of 256
     if (tid == 0) {
-        const int done = atomicAdd(&counters[sb], 1);
+        int done;  // what the thread block has stored (the barrier's cumulativity) is there for whoever counts behind it
+        asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(done) : "l"(&counters[sb]) : "memory");
         last_flag = done == 2 * splits - 1;
         if (last_flag) {
             counters[sb] = 0;  // every CTA of the pair has counted: ready for the next launch
@@ -881,10 +905,16 @@ __global__ void __launch_bounds__(ATTF_THREADS, 3) attention_image_kernel(const 
         }
         return;
     }
-    __threadfence();
     {
-        // Chunk maxima and sums first, then the weights exp(m - M), then the weighted sums with every load independent of
-        // the others (chunks without a visible key have weight zero and their partial sums are never used).
+        // Chunk maxima and sums and the first chunks' partial sums at once, then the weights exp(m - M), then the weighted sums.
+        constexpr int AT_ONCE = 12;
+        const int hsel = tid >> 7, d = tid & 127;
+        const float* p = part + (int64_t)(2 * sb + hsel) * stride_splits * (HD + 2) + d;
+        float early[AT_ONCE];
+#pragma unroll
+        for (int i = 0; i < AT_ONCE; i++) {
+            early[i] = i < splits ? __ldcg(p + (int64_t)i * (HD + 2)) : 0.0f;
+        }
         float* wm = red[0];  // [2 heads][splits <= 128]: m, later the weight
         float* wl = red[2];  // [2 heads][splits]: l
         for (int i = tid; i < 2 * splits; i += ATTF_THREADS) {
@@ -904,19 +934,24 @@ __global__ void __launch_bounds__(ATTF_THREADS, 3) attention_image_kernel(const 
             }
             for (int sidx = lane; sidx < splits; sidx += 32) {
                 const float m = wm[warp * 128 + sidx];
-                wm[warp * 128 + sidx] = m == -INFINITY ? 0.0f : expf(m - M);
+                wm[warp * 128 + sidx] = expf(m - M);
             }
         }
         __syncthreads();
-        const int hsel = tid >> 7, d = tid & 127;
-        const float* p = part + (int64_t)(2 * sb + hsel) * stride_splits * (HD + 2) + d;
         float L = 0.0f, acc = 0.0f;
-#pragma unroll 4
-        for (int sidx = 0; sidx < splits; sidx++) {
-            const float wgt = wm[hsel * 128 + sidx];
-            const float val = __ldcg(p + (int64_t)sidx * (HD + 2));
-            L = fmaf(wgt, wl[hsel * 128 + sidx], L);
-            acc = fmaf(wgt, wgt != 0.0f ? val : 0.0f, acc);
+#pragma unroll
+        for (int i = 0; i < AT_ONCE; i++) {
+            if (i < splits) {
+                const float wgt = wm[hsel * 128 + i];
+                L = fmaf(wgt, wl[hsel * 128 + i], L);
+                acc = fmaf(wgt, early[i], acc);
+            }
+        }
+#pragma unroll 8
+        for (int i = AT_ONCE; i < splits; i++) {
+            const float wgt = wm[hsel * 128 + i];
+            L = fmaf(wgt, wl[hsel * 128 + i], L);
+            acc = fmaf(wgt, __ldcg(p + (int64_t)i * (HD + 2)), acc);
         }
         outs[tid] = acc / L;
     }
