@@ -157,15 +157,18 @@ int launch_gemv_q4k_i8_multi(const View* vs, int count, const float* x, int rows
 // The same for one row of x whose activation image (jq_q4k_image.cuh) a kernel earlier in the stream has already written; a
 // second Q4_K weight with the same k can ride in the same launch.
 size_t q4k_image_bytes_one_row(int64_t k);
-// What a Q4_K GEMV of one row needs to make its activation image from RMSNorm(x + delta) itself. It also leaves x + delta in x_out (not x: other
-// thread blocks still read it) and, unless q6k is null, the Q6_K image of the normalised vector there (scratch: k floats).
+// What a GEMV of one row needs to make its activation image from RMSNorm(x + delta) itself. It also leaves x + delta in x_out (not x: other
+// thread blocks still read it).
 struct NormInput {
     const float *x, *delta, *w;
     float eps;
-    float *x_out, *scratch;
-    uint8_t* q6k;
+    float* x_out;  // receives x + delta; null where the launch in front does that
+    bool followed;  // a launch on the same input is behind, which does not wait for this one: it may start when this one knows that the input is complete
 };
 int launch_gemv_q4k_i8_normed(const View* vs, int count, const NormInput& norm, float* const* ys, cudaStream_t s, bool* handled);
+// The launch behind it, of one Q6_K weight: it starts as SMs become free and ends after the one in front.
+bool gemv_q6k_i8_normed_takes(const View& v);
+int launch_gemv_q6k_i8_normed(const View& v, const NormInput& norm, float* y, cudaStream_t s);
 int launch_gemv_q4k_i8_imaged(const View& v, const View* v2, const uint8_t* image, const float* bias, float* y, float* y2, cudaStream_t s, bool* handled,
                               const PeerOut* peer = nullptr, const View* v3 = nullptr, float* y3 = nullptr);
 // Status word of the waits a GEMV makes itself for a peer exchange (peer_wait_inline): 0 or 32 + rank, cleared by the call.

@@ -1644,15 +1644,20 @@ static int enqueue_forward_fused(jq_decoder* d, int max_keys, const TokenArgs* t
     const int splits_now = (max_keys + ATT_CHUNK - 1) / ATT_CHUNK;
     // The residual stream. A norm whose linears' first is Q4_K is made inside that launch, which leaves x + delta in the other buffer.
     float *x = d->x, *x_other = d->xn;
-    auto NORMED = [&](const float* norm_w, const jq_weight* const* w, int count, float* const* ys, uint8_t* q6k) {
+    auto NORMED = [&](const float* norm_w, const jq_weight* const* w, int count, float* const* ys, const View* behind, float* behind_y) {
         View vs[3];
         for (int i = 0; i < count; i++) {
             vs[i] = View{w[i]->q, w[i]->aux, w[i]->n, w[i]->k, w[i]->type};
         }
-        const NormInput in{x, d->proj, norm_w, d->eps, x_other, d->att, q6k};
+        NormInput in{x, d->proj, norm_w, d->eps, x_other, behind != nullptr};
         bool handled = false;
         if (rc == JQ_OK) {
             rc = launch_gemv_q4k_i8_normed(vs, count, in, ys, s, &handled);
+        }
+        if (rc == JQ_OK && handled && behind != nullptr) {
+            in.x_out = nullptr;
+            in.followed = false;
+            rc = launch_gemv_q6k_i8_normed(*behind, in, behind_y, s);
         }
         if (handled) {
             std::swap(x, x_other);
@@ -1667,10 +1672,8 @@ static int enqueue_forward_fused(jq_decoder* d, int max_keys, const TokenArgs* t
         float* vc = d->v_cache + seq_base + (size_t)l * d->max_seq * kv_dim;
         // attention block: x = embedding (first layer) or x += feed-forward output of the layer before; norm -> images
         const bool all_q4k = L[2]->type == JQ_TYPE_Q4_K;
-        if (l > 0 && NORMED(d->norms + (size_t)(2 * l) * dim, L, all_q4k ? 3 : 2, qkv, all_q4k ? nullptr : d->img_q6k)) {
-            if (!all_q4k) {
-                GEMV(L[2], d->v, nullptr, nullptr, s);
-            }
+        const View wv{L[2]->q, L[2]->aux, L[2]->n, L[2]->k, L[2]->type};
+        if (l > 0 && (all_q4k || gemv_q6k_i8_normed_takes(wv)) && NORMED(d->norms + (size_t)(2 * l) * dim, L, all_q4k ? 3 : 2, qkv, all_q4k ? nullptr : &wv, d->v)) {
         } else {
             CKL(launch_cluster_pdl(norm_image_kernel, norm_ctas, norm_block, norm_smem, s, l > 0 || first_programmatic, x, l == 0 ? nullptr : d->proj,
                                    l == 0 ? d->embed : nullptr, d->tokens, d->vocab, d->norms + (size_t)(2 * l) * dim, d->eps, dim,
@@ -1687,7 +1690,7 @@ static int enqueue_forward_fused(jq_decoder* d, int max_keys, const TokenArgs* t
         GEMV(L[3], d->proj, nullptr, nullptr, s);
         if (rc != JQ_OK) break;
         // feed-forward block
-        if (!NORMED(d->norms + (size_t)(2 * l + 1) * dim, L + 4, 2, gate_up, nullptr)) {
+        if (!NORMED(d->norms + (size_t)(2 * l + 1) * dim, L + 4, 2, gate_up, nullptr, nullptr)) {
             CKL(launch_cluster_pdl(norm_image_kernel, norm_ctas, norm_block, norm_smem, s, true, x, d->proj, nullptr, d->tokens, d->vocab,
                                    d->norms + (size_t)(2 * l + 1) * dim, d->eps, dim, images_for({L[4], L[5]}), (const uint32_t*)nullptr, 0),
                 "norm_image_kernel");

@@ -164,7 +164,9 @@ __global__ void __launch_bounds__(NW * 32, OCC) gemv_q4k_i8_kernel(View v, Secon
     constexpr int SLOT_BYTES = B::SLOT;
     constexpr uint32_t RING_BYTES = STAGES * SLOT_BYTES;
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    asm volatile("griddepcontrol.launch_dependents;");  // the kernel after this one may be scheduled as room becomes free
+    if (SRC != FROM_NORM || !norm.followed) {
+        asm volatile("griddepcontrol.launch_dependents;");  // the kernel after this one may be scheduled as room becomes free
+    }
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 #ifdef JQ_Q4K_TRACE
     int tslot = 0;
@@ -252,6 +254,9 @@ __global__ void __launch_bounds__(NW * 32, OCC) gemv_q4k_i8_kernel(View v, Secon
 
     // ---- x (or the image made from it) is complete once the kernel before this one has finished --------------------------
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (SRC == FROM_NORM && norm.followed) {
+        asm volatile("griddepcontrol.launch_dependents;");  // (the kernel after this one reads the same input and does not wait for it itself)
+    }
     QT(1);
     const uint32_t img_s = tc::smem_u32(img);
     bool peer_marks = false;  // the outputs travel as marked words (jq_peer_device.cuh) rather than behind a release
@@ -458,12 +463,6 @@ __global__ void __launch_bounds__(NW * 32, OCC) gemv_q4k_i8_kernel(View v, Secon
                         a[j][i] = a[j][i] * inv * norm_w[j][i];
                     }
                     q4k::build_image_from<MT>(a[j], true, 0, img + (size_t)b * C::PB, lane);
-                    if (keeps && norm.q6k != nullptr) {
-                        float4* const to = reinterpret_cast<float4*>(norm.scratch + b * 256) + 2 * lane;
-                        to[0] = make_float4(a[j][0], a[j][1], a[j][2], a[j][3]);
-                        to[1] = make_float4(a[j][4], a[j][5], a[j][6], a[j][7]);
-                        q6k::build_image<1>(norm.scratch + b * 256, 0, norm.q6k + (size_t)b * q6k::Cfg<1>::PB, lane);  // (a lane reads what it wrote)
-                    }
                 }
             }
             __syncwarp();

@@ -113,11 +113,21 @@ __global__ void __launch_bounds__(PREP_WARPS * 32) q6k_activation_image_kernel(c
 }
 
 // ---- the GEMV ---------------------------------------------------------------------------------------------------
-// FROM_X: no image in memory, every warp makes that of the super-blocks that it multiplies itself, straight from x (one slice).
-template <int MT, int STAGES, int OCC, bool FROM_X>
+// SRC: where the image comes from. FROM_X, FROM_NORM: no image in memory, every warp makes that of the super-blocks that it multiplies itself (one slice), straight from x,
+// or from the RMSNorm of norm.x + norm.delta, which every thread block makes in the order of the Q4_K kernel (jq_gemv_q4k_i8.cu).
+// FROM_NORM is the launch behind one of that kernel on the same input. It does not wait for it: that one has waited for the input, which is in L2, when it lets
+// this one start, and it is read there. So the weights of a Q6_K wv come in while wq|wk drains. It ends after it, so whoever waits for this one waits for both.
+enum Source { FROM_IMAGE, FROM_X, FROM_NORM };
+constexpr int NORM_MAX = 4;  // super-blocks a warp: k <= 8192
+__device__ __forceinline__ void load_l2(const float* p, int lane, float (&r)[8]) {
+    const float4 a = __ldcg(reinterpret_cast<const float4*>(p) + 2 * lane), b = __ldcg(reinterpret_cast<const float4*>(p) + 2 * lane + 1);
+    r[0] = a.x; r[1] = a.y; r[2] = a.z; r[3] = a.w;
+    r[4] = b.x; r[5] = b.y; r[6] = b.z; r[7] = b.w;
+}
+template <int MT, int STAGES, int OCC, int SRC>
 __global__ void __launch_bounds__(THREADS, OCC) gemv_q6k_i8_kernel(View v, const uint8_t* __restrict__ image, const float* x, int rows,
                                                                   const float* __restrict__ bias, float* __restrict__ y, int tiles,
-                                                                  int KS, int max_tiles, long long wait_clocks, int* status) {
+                                                                  int KS, int max_tiles, long long wait_clocks, int* status, NormInput norm) {
     // KS = super-blocks of k per slice: the activation image of one slice is resident in shared memory at a time;
     // with more than one slice the per-tile sums are carried in shared memory (max_tiles tiles per CTA).
     using C = Cfg<MT>;
@@ -192,7 +202,9 @@ __global__ void __launch_bounds__(THREADS, OCC) gemv_q6k_i8_kernel(View v, const
     }
 
     // ---- the activation image is complete once the kernel that writes it has finished ----------------------------
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if constexpr (SRC != FROM_NORM) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
     const uint32_t img_s = (uint32_t)__cvta_generic_to_shared(img);
 
     // ---- main loop ----------------------------------------------------------------------------------------------
@@ -310,7 +322,56 @@ __global__ void __launch_bounds__(THREADS, OCC) gemv_q6k_i8_kernel(View v, const
         if (sl > 0) {
             __syncthreads();  // every warp is done with the previous slice
         }
-        if constexpr (FROM_X) {
+        if constexpr (SRC == FROM_NORM) {
+            float a[NORM_MAX][8], sq = 0.0f;
+#pragma unroll
+            for (int j = 0; j < NORM_MAX; j++) {
+                const int b = warp + WARPS * j;
+                float dl[8] = {};
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    a[j][i] = 0.0f;
+                }
+                if (b < KB) {
+                    load_l2(norm.x + b * 256, lane, a[j]);
+                    load_l2(norm.delta + b * 256, lane, dl);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    a[j][i] += dl[i];
+                    sq = fmaf(a[j][i], a[j][i], sq);
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                sq += __shfl_xor_sync(0xffffffffu, sq, o);
+            }
+            float* const partial = red + WARPS * 16 * MT;  // (the half that the second tile is the first to use)
+            if (lane == 0) {
+                partial[warp] = sq;
+            }
+            __syncthreads();
+            float total = 0.0f;
+#pragma unroll
+            for (int i = 0; i < WARPS; i++) {
+                total += partial[i];
+            }
+            const float inv = 1.0f / sqrtf(total / (float)(int)v.k + norm.eps);
+#pragma unroll
+            for (int j = 0; j < NORM_MAX; j++) {
+                const int b = warp + WARPS * j;
+                if (b < KB) {
+                    float w[8];
+                    q6k::load_x(norm.w + b * 256, lane, w);
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        a[j][i] = a[j][i] * inv * w[i];
+                    }
+                    build_image<MT>(a[j], true, 0, img + (size_t)b * C::PB, lane);
+                }
+            }
+            __syncwarp();
+        } else if constexpr (SRC == FROM_X) {
             constexpr int TWO = 2;  // super-blocks whose values are on their way at a time
             for (int b = warp; b < KB; b += TWO * WARPS) {
                 float xv[TWO][MT][8] = {};
@@ -436,6 +497,9 @@ __global__ void __launch_bounds__(THREADS, OCC) gemv_q6k_i8_kernel(View v, const
             __nanosleep(1000);  // copies that may still be in flight land long before this millisecond is over
         }
     }
+    if (SRC == FROM_NORM && tid == 0) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
 }
 
 constexpr int64_t FROM_X_VALUES = 8192;
@@ -453,13 +517,14 @@ int sm_count() {
     return g_sms;
 }
 
-template <int MT, int STAGES, int OCC, bool FROM_X>
-int launch(const View& v, const uint8_t* image, const float* x, int rows, const float* bias, float* y, cudaStream_t s, int KS, int grid, int max_tiles, size_t smem) {
+template <int MT, int STAGES, int OCC, int SRC>
+int launch(const View& v, const uint8_t* image, const float* x, int rows, const float* bias, float* y, cudaStream_t s, int KS, int grid, int max_tiles, size_t smem,
+           const NormInput& norm = NormInput{}) {
     static std::atomic<uint64_t> configured{0};  // the opt-in for large dynamic shared memory is per device
     int dev = 0;
     JQ_CUDA(cudaGetDevice(&dev));
     if ((configured.load() >> (dev & 63) & 1) == 0) {
-        JQ_CUDA(cudaFuncSetAttribute(gemv_q6k_i8_kernel<MT, STAGES, OCC, FROM_X>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
+        JQ_CUDA(cudaFuncSetAttribute(gemv_q6k_i8_kernel<MT, STAGES, OCC, SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
         configured.fetch_or((uint64_t)1 << (dev & 63));
     }
     const int tiles = (int)((v.n + 15) / 16);
@@ -479,7 +544,7 @@ int launch(const View& v, const uint8_t* image, const float* x, int rows, const 
     if (rc != JQ_OK) {
         return rc;
     }
-    JQ_CUDA(cudaLaunchKernelEx(&cfg, gemv_q6k_i8_kernel<MT, STAGES, OCC, FROM_X>, v, image, x, rows, bias, y, tiles, KS, max_tiles, wait_clocks, status));
+    JQ_CUDA(cudaLaunchKernelEx(&cfg, gemv_q6k_i8_kernel<MT, STAGES, OCC, SRC>, v, image, x, rows, bias, y, tiles, KS, max_tiles, wait_clocks, status, norm));
     count_launch();
     return JQ_OK;
 }
@@ -539,8 +604,8 @@ int run(const View& v, const float* x, int rows, const float* bias, float* y, cu
         // 1024 x 1024 3.2 / 2.0, 4096 x 4096 5.6 / 4.5, 32000 x 4096 21.8 / 20.3, 4096 x 8192 8.2 / 8.1; two rows, 4096 x 2048 4.6 / 3.7, 4096 x 4096 5.6 / 5.9, 32000 x 4096 22.1 / 22.0. A
         // launched call saves 2 us of host time besides.
         if (x != nullptr && rows * v.k <= FROM_X_VALUES && !x_remote && !sliced) {
-            return stages == 3 ? launch<MT, 3, 2, true>(v, image, x, rows, bias, y, s, KS, grid, max_tiles, smem)
-                               : launch<MT, 2, 2, true>(v, image, x, rows, bias, y, s, KS, grid, max_tiles, smem);
+            return stages == 3 ? launch<MT, 3, 2, FROM_X>(v, image, x, rows, bias, y, s, KS, grid, max_tiles, smem)
+                               : launch<MT, 2, 2, FROM_X>(v, image, x, rows, bias, y, s, KS, grid, max_tiles, smem);
         }
     }
     if (x != nullptr) {  // else the image is already in `image` (written by a kernel earlier in the stream)
@@ -558,8 +623,8 @@ int run(const View& v, const float* x, int rows, const float* bias, float* y, cu
         JQ_CUDA(cudaLaunchKernelEx(&icfg, q6k_activation_image_kernel<MT>, x, rows, (int64_t)v.k, image));
         count_launch();
     }
-    if (stages == 3) return launch<MT, 3, 2, false>(v, image, x, rows, bias, y, s, KS, grid, max_tiles, smem);
-    return launch<MT, 2, 2, false>(v, image, x, rows, bias, y, s, KS, grid, max_tiles, smem);
+    if (stages == 3) return launch<MT, 3, 2, FROM_IMAGE>(v, image, x, rows, bias, y, s, KS, grid, max_tiles, smem);
+    return launch<MT, 2, 2, FROM_IMAGE>(v, image, x, rows, bias, y, s, KS, grid, max_tiles, smem);
 }
 
 }  // namespace
@@ -597,6 +662,16 @@ int launch_gemv_q6k_i8_imaged(const View& v, const uint8_t* image, const float* 
         return JQ_OK;
     }
     return run<1>(v, nullptr, 1, bias, y, s, const_cast<uint8_t*>(image), handled);
+}
+
+// Two thread blocks per SM, three ring stages and the image of the whole k.
+bool gemv_q6k_i8_normed_takes(const View& v) {
+    return v.type == JQ_TYPE_Q6_K && v.n > 0 && v.k > 0 && v.k <= NORM_MAX * WARPS * 256 && smem_bytes<1>((int)(v.k / 256), 3, false, 0) <= SMEM_MAX / 2 - 1024;
+}
+
+int launch_gemv_q6k_i8_normed(const View& v, const NormInput& norm, float* y, cudaStream_t s) {
+    const int KB = (int)(v.k / 256), tiles = (int)((v.n + 15) / 16), grid = tiles < 2 * sm_count() ? tiles : 2 * sm_count();
+    return launch<1, 3, 2, FROM_NORM>(v, nullptr, nullptr, 1, nullptr, y, s, KB, grid, (tiles + grid - 1) / grid, smem_bytes<1>(KB, 3, false, 0), norm);
 }
 
 }  // namespace jq
