@@ -334,12 +334,14 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_partial_kernel(const fl
 constexpr int GROUP_THREADS = 256, GROUP_HEADS = 8;
 // MANY: take may be more than one.
 template <int HD, bool MANY>
-__global__ void __launch_bounds__(GROUP_THREADS, HD == 64 ? 3 : 2) attention_group_kernel(const float* __restrict__ q, const float* __restrict__ k_new, const float* __restrict__ v_new,
+__global__ void __launch_bounds__(GROUP_THREADS, HD == 64 ? 3 : 2) attention_group_kernel(const float* q, const float* k_new, const float* v_new,
                                                                        float* k_cache, float* v_cache, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                                                                        float* __restrict__ part, const int* __restrict__ pos0, int heads, int kv_heads, int splits,
                                                                        float scale, int pos_step, int64_t tok_stride, int tokens, int take) {
     asm volatile("griddepcontrol.launch_dependents;");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // The position was set before the first kernel of this call started, and the cached keys and values of earlier positions by earlier calls: both are read before
+    // the wait for the kernel in front, so that a CTA scheduled while that kernel still runs has its cache lines on the way. (q, k_new and v_new are not: as
+    // read-only data their loads would be moved in front of it too.)
     static_assert(HD == 64 || HD == 128, "head sizes");
     constexpr int V = HD / 32;
     __shared__ __align__(16) float red[GROUP_HEADS][8][HD];
@@ -354,6 +356,7 @@ __global__ void __launch_bounds__(GROUP_THREADS, HD == 64 ? 3 : 2) attention_gro
     auto head_of = [&](int item) { return kvh * group + (MANY ? item % group : item); };
     auto result = [&](int item) { return part + (((int64_t)token_of(item) * heads + head_of(item)) * splits + sp) * (HD + 2); };
     if (k0 >= keys) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
         for (int item = tid; item < items; item += GROUP_THREADS) {
             float* const out = result(item);
             out[HD] = -INFINITY;  // m
@@ -381,11 +384,19 @@ __global__ void __launch_bounds__(GROUP_THREADS, HD == 64 ? 3 : 2) attention_gro
         for (int i = 0; i < V; i++) {
             kr[u][i] = vr[u][i] = 0.0f;
         }
-        if (warp * 8 + u < cnt) {
-            const int own = k0 + warp * 8 + u - first;  // 0 and more: one of the call's own
+        if (warp * 8 + u < cnt && k0 + warp * 8 + u < first) {
+            get(kb + (int64_t)u * kv_dim, kr[u]);
+            get(vb + (int64_t)u * kv_dim, vr[u]);
+        }
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+        const int own = k0 + warp * 8 + u - first;  // 0 and more: one of the call's own
+        if (warp * 8 + u < cnt && own >= 0) {
             const int64_t row = (int64_t)(pos_step != 0 ? own : t0) * kv_dim + kvh * HD + lane * V;
-            get(own < 0 ? kb + (int64_t)u * kv_dim : k_new + row, kr[u]);
-            get(own < 0 ? vb + (int64_t)u * kv_dim : v_new + row, vr[u]);
+            get(k_new + row, kr[u]);
+            get(v_new + row, vr[u]);
         }
     }
     // rotate-half: this lane's dimensions and those of the lane 16 further, the same angles
@@ -552,7 +563,7 @@ __global__ void __launch_bounds__(GROUP_THREADS, HD == 64 ? 3 : 2) attention_gro
 // become a step of the rows kernel's image.
 constexpr int MAX_SPLITS = 128;  // 8192 positions
 template <int IMAGE>
-__global__ void __launch_bounds__(256) attention_combine_kernel(const float* __restrict__ part, float* out, int heads, int head_dim, int stride_splits, int splits, float* scales,
+__global__ void __launch_bounds__(256) attention_combine_kernel(const float* part, float* out, int heads, int head_dim, int stride_splits, int splits, float* scales,
                                                                int span) {
     asm volatile("griddepcontrol.launch_dependents;");  // launched programmatically, the kernel behind this one may be scheduled now ...
     asm volatile("griddepcontrol.wait;" ::: "memory");  // ... and this one touches memory only when the kernel before it has finished
@@ -564,6 +575,15 @@ __global__ void __launch_bounds__(256) attention_combine_kernel(const float* __r
     const int v0 = (int)blockIdx.x * span, v1 = min(v0 + span, dim), h0 = v0 / head_dim, here = (v1 - 1) / head_dim - h0 + 1;  // the first head, how many
     const int64_t row = (int64_t)stride_splits * (head_dim + 2);
     const float* const p = part + ((int64_t)t * heads + h0) * row;
+    // the first chunks' values are on their way while the weights are made (a chunk without a visible key holds anything: not used)
+    constexpr int EARLY = 8;
+    const int at = v0 + tid, my_h = at < v1 ? at / head_dim - h0 : 0;
+    const float* const pd = p + my_h * row + at % head_dim;
+    float early[EARLY];
+#pragma unroll
+    for (int s = 0; s < EARLY; s++) {
+        early[s] = s < splits && at < v1 ? pd[(int64_t)s * (head_dim + 2)] : 0.0f;
+    }
     for (int h = tid >> 5; h < here; h += 8) {
         const float* const ph = p + h * row + head_dim;
         float m[MAX_SPLITS / 32], M = -INFINITY, L = 0.0f;
@@ -593,17 +613,19 @@ __global__ void __launch_bounds__(256) attention_combine_kernel(const float* __r
         }
     }
     __syncthreads();
-    const int at = v0 + tid;
     float v = 0.0f;
     if (at < v1) {
-        const int h = at / head_dim - h0;
-        const float* const pd = p + h * row + at % head_dim;
+#pragma unroll
+        for (int s = 0; s < EARLY; s++) {
+            const float e = s < splits ? weight[my_h][s] : -1.0f;
+            v = !(e < 0.0f) ? fmaf(e, early[s], v) : v;
+        }
 #pragma unroll 8
-        for (int s = 0; s < splits; s++) {
-            const float e = weight[h][s];
+        for (int s = EARLY; s < splits; s++) {
+            const float e = weight[my_h][s];
             v = !(e < 0.0f) ? fmaf(e, pd[(int64_t)s * (head_dim + 2)], v) : v;
         }
-        v /= total[h];
+        v /= total[my_h];
     }
     if constexpr (IMAGE == 0) {
         if (at < v1) {
