@@ -82,8 +82,11 @@ __global__ void set_tokens_kernel(TokenArgs a, int* __restrict__ tokens, int* __
     }
 }
 
+// Kernels behind a programmatic launch do not declare what the kernel in front writes __restrict__, nor read it as read-only data: such loads depend on nothing that
+// the wait for that kernel says it touches, and are moved in front of it.
+
 // x[t, :] = table[token[t], :]
-__global__ void embed_kernel(const int* __restrict__ tokens, const float* __restrict__ table, float* __restrict__ x, int dim, int vocab) {
+__global__ void embed_kernel(const int* tokens, const float* __restrict__ table, float* __restrict__ x, int dim, int vocab) {
     asm volatile("griddepcontrol.launch_dependents;");  // launched programmatically, the kernel behind this one may be scheduled now ...
     asm volatile("griddepcontrol.wait;" ::: "memory");  // ... and this one touches memory only when the kernel before it has finished
     int tok = tokens[blockIdx.x];
@@ -112,7 +115,7 @@ __device__ __forceinline__ void store4(__nv_bfloat16* o, int64_t i, float4 v) {
 // IMAGE: 8 or 16, the rows of the rows kernel's instance behind, whose image of x goes out in the place of the vector (its scales at `scales`; dim a multiple of 256,
 // which meets in shared memory): a launch less in front of every group of linears.
 template <typename Out, int NORM_THREADS, int HOLD, int IMAGE = 0>
-__global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ delta, const float* __restrict__ w,
+__global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_kernel(float* x, const float* delta, const float* __restrict__ w,
                                                                    float eps, Out* __restrict__ out, int dim, float* scales) {
     asm volatile("griddepcontrol.launch_dependents;");  // launched programmatically, the kernel behind this one may be scheduled now ...
     const int nv = (dim & 3) == 0 ? dim >> 2 : 0;  // 128-bit pieces; a dim that is no multiple of 4 takes the scalar loops below
@@ -193,7 +196,7 @@ __global__ void add_kernel(float* __restrict__ x, const float* __restrict__ delt
 
 // Rotate-half RoPE on the query heads (in place) and key heads, and the append of key and value to the cache.
 // grid (tokens, heads + 2 * kv_heads), head_dim / 2 threads.
-__global__ void rope_store_kernel(float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v, float* __restrict__ k_cache,
+__global__ void rope_store_kernel(float* q, const float* k, const float* v, float* __restrict__ k_cache,
                                   float* __restrict__ v_cache, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                                   const int* __restrict__ pos0, int heads, int kv_heads, int head_dim, int pos_step, int64_t tok_stride) {
     asm volatile("griddepcontrol.launch_dependents;");  // launched programmatically, the kernel behind this one may be scheduled now ...
@@ -235,8 +238,8 @@ __global__ void rope_store_kernel(float* __restrict__ q, const float* __restrict
 constexpr int ATT_CHUNK = 64;
 constexpr int ATT_THREADS = 128;
 
-__global__ void __launch_bounds__(ATT_THREADS) attention_partial_kernel(const float* __restrict__ q, const float* __restrict__ k_cache,
-                                                                        const float* __restrict__ v_cache, float* __restrict__ part,
+__global__ void __launch_bounds__(ATT_THREADS) attention_partial_kernel(const float* q, const float* k_cache,
+                                                                        const float* v_cache, float* __restrict__ part,
                                                                         const int* __restrict__ pos0, int heads, int kv_heads, int head_dim,
                                                                         int splits, float scale, int pos_step, int64_t tok_stride) {
     asm volatile("griddepcontrol.launch_dependents;");  // launched programmatically, the kernel behind this one may be scheduled now ...
@@ -644,7 +647,7 @@ __global__ void __launch_bounds__(256) attention_combine_kernel(const float* par
 
 // act = silu(gate) * up, four elements per thread
 template <typename Out>
-__global__ void __launch_bounds__(256) swiglu_kernel(const float* __restrict__ gate, const float* __restrict__ up, Out* __restrict__ act, int64_t count) {
+__global__ void __launch_bounds__(256) swiglu_kernel(const float* gate, const float* up, Out* __restrict__ act, int64_t count) {
     asm volatile("griddepcontrol.launch_dependents;");  // launched programmatically, the kernel behind this one may be scheduled now ...
     asm volatile("griddepcontrol.wait;" ::: "memory");  // ... and this one touches memory only when the kernel before it has finished
     auto one = [](float g, float u) { return (g / (1.0f + expf(-g))) * u; };
@@ -691,8 +694,8 @@ __device__ __forceinline__ void write_images(const float* block, int b, const Im
 // CTA takes dim / CTAs elements (whole super-blocks of 256), the sums of squares meet through distributed shared
 // memory (each CTA adds the partial sums of all CTAs in rank order, so all get the same total), and every CTA writes
 // the images of its own super-blocks. blockDim.x = elements per CTA / 4.
-__global__ void __launch_bounds__(1024) norm_image_kernel(float* __restrict__ x, const float* __restrict__ delta, const float* __restrict__ table,
-                                                          const int* __restrict__ token, int vocab, const float* __restrict__ w, float eps, int dim,
+__global__ void __launch_bounds__(1024) norm_image_kernel(float* x, const float* delta, const float* __restrict__ table,
+                                                          const int* token, int vocab, const float* __restrict__ w, float eps, int dim,
                                                           Images im, const uint32_t* wait_flags, int wait_world) {
     namespace cg = cooperative_groups;
     extern __shared__ __align__(16) float norm_xs[];  // this CTA's normalised elements
@@ -756,7 +759,7 @@ constexpr int ATTF_THREADS = 256;
 // PEER (a rank of the row-sharded decoder): heads are this rank's, the image block goes to the same place of every
 // rank's image area, and the CTA that finishes last of the whole grid raises this rank's flag on every rank.
 template <bool PEER>
-__global__ void __launch_bounds__(ATTF_THREADS, 3) attention_image_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
+__global__ void __launch_bounds__(ATTF_THREADS, 3) attention_image_kernel(const float* q, const float* k, const float* v,
                                                                        float* __restrict__ k_cache, float* __restrict__ v_cache,
                                                                        const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                                                                        const int* __restrict__ pos0, int heads, int kv_heads, int stride_splits, float scale,
@@ -996,7 +999,7 @@ __global__ void __launch_bounds__(ATTF_THREADS, 3) attention_image_kernel(const 
 // their stores to the other ranks (each announcement is a release at system scope).
 constexpr int SWIGLU_PEER_BLOCKS = 4;
 template <bool PEER>
-__global__ void __launch_bounds__(256) swiglu_image_kernel(const float* __restrict__ gate, const float* __restrict__ up, Images im, PeerImage pi, int blocks) {
+__global__ void __launch_bounds__(256) swiglu_image_kernel(const float* gate, const float* up, Images im, PeerImage pi, int blocks) {
     constexpr int PER_CTA = PEER ? SWIGLU_PEER_BLOCKS : 1;
     __shared__ __align__(16) float xs[PER_CTA][256];
     pdl_enter();
@@ -1028,7 +1031,7 @@ __global__ void __launch_bounds__(256) swiglu_image_kernel(const float* __restri
 // First index of the maximum (ops/Reduce.java:201) of each row (grid y), over ARGMAX_CTAS CTAs: each leaves its best (value,
 // index), the CTA of a row that finishes last picks among them.
 constexpr int ARGMAX_CTAS = 64;
-__global__ void __launch_bounds__(256) argmax_split_kernel(const float* __restrict__ logits, int vocab, float* __restrict__ best_v, int* __restrict__ best_i,
+__global__ void __launch_bounds__(256) argmax_split_kernel(const float* logits, int vocab, float* __restrict__ best_v, int* __restrict__ best_i,
                                                            int* __restrict__ counter, int* __restrict__ out) {
     __shared__ float bv[8];
     __shared__ int bi[8];

@@ -95,7 +95,7 @@ constexpr int PREP_WARPS = 4;
 __device__ int g_gemv_peer_status;  // 0, or 32 + rank once a GEMV's own wait for an exchange has given up
 
 template <int MT>
-__global__ void __launch_bounds__(PREP_WARPS * 32) q4k_activation_image_kernel(const float* __restrict__ x, int rows, int64_t k,
+__global__ void __launch_bounds__(PREP_WARPS * 32) q4k_activation_image_kernel(const float* x, int rows, int64_t k,
                                                                              uint8_t* __restrict__ image) {
     asm volatile("griddepcontrol.launch_dependents;");  // the GEMV kernel may start requesting weights now
     asm volatile("griddepcontrol.wait;" ::: "memory");  // x is complete, and the GEMV before this one is done with the scratch image
@@ -151,7 +151,7 @@ enum From { FROM_IMAGE, FROM_FLOATS, FROM_NORM };
 constexpr int NORM_MAX = 4;
 template <int MT, int STAGES, int NW, int OCC, bool Q5, bool PEER, From SRC>
 __global__ void __launch_bounds__(NW * 32, OCC) gemv_q4k_i8_kernel(View v, Second w2, const PeerOut* __restrict__ peerp, const uint8_t* __restrict__ image,
-                                                                  const float* __restrict__ xin, int rows, const float* __restrict__ bias, float* __restrict__ y,
+                                                                  const float* xin, int rows, const float* __restrict__ bias, float* __restrict__ y,
                                                                   int tiles, int KS, int max_tiles, long long wait_clocks, int* status, NormInput norm) {
     // Tiles 0 .. w2.first_tiles - 1 are rows of v, the tiles from w2.first_tiles on rows of the second weight w2 (same k,
     // same x, its own output), if there is one.

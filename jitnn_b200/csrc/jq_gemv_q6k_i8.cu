@@ -101,7 +101,7 @@ __device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {
 constexpr int PREP_WARPS = 4;
 
 template <int MT>
-__global__ void __launch_bounds__(PREP_WARPS * 32) q6k_activation_image_kernel(const float* __restrict__ x, int rows, int64_t k,
+__global__ void __launch_bounds__(PREP_WARPS * 32) q6k_activation_image_kernel(const float* x, int rows, int64_t k,
                                                                              uint8_t* __restrict__ image) {
     asm volatile("griddepcontrol.launch_dependents;");  // the GEMV kernel may start requesting weights now
     asm volatile("griddepcontrol.wait;" ::: "memory");  // x is complete, and the GEMV before this one is done with the scratch image

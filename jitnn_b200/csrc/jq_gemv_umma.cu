@@ -277,7 +277,7 @@ __device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {
 }
 
 template <int N>
-__global__ void __launch_bounds__(128) umma_activation_image_kernel(const float* __restrict__ x, int rows, int64_t k, uint8_t* __restrict__ image) {
+__global__ void __launch_bounds__(128) umma_activation_image_kernel(const float* x, int rows, int64_t k, uint8_t* __restrict__ image) {
     asm volatile("griddepcontrol.launch_dependents;");  // the GEMV may start asking for weights
     asm volatile("griddepcontrol.wait;" ::: "memory");  // x is complete, and the GEMV before this one is done with the image
     const int pair = blockIdx.x * 4 + (threadIdx.x >> 5);

@@ -18,7 +18,7 @@ namespace mm {
 // EXT: 16 more columns follow every 256, the sums over the eight runs of 32 values, twice (hi plane: their hi parts, lo plane: their lo
 // parts).
 template <int BLK, bool EXT>
-__global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ x, const float* __restrict__ up, int m, int64_t k, int per_row, uint4* __restrict__ planes,
+__global__ void __launch_bounds__(256) split_kernel(const float* x, const float* up, int m, int64_t k, int per_row, uint4* __restrict__ planes,
                                                     float* __restrict__ scales, int stride, int vec) {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -32,26 +32,26 @@ __global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ x,
     const float* src = x + (int64_t)row * k + i0;
     float v[8];
     if (vec && i0 + 8 <= k) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(src)), c = __ldg(reinterpret_cast<const float4*>(src) + 1);
+        const float4 a = *reinterpret_cast<const float4*>(src), c = *(reinterpret_cast<const float4*>(src) + 1);
         v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
         v[4] = c.x; v[5] = c.y; v[6] = c.z; v[7] = c.w;
     } else {
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            v[i] = i0 + i < k ? __ldg(src + i) : 0.0f;
+            v[i] = i0 + i < k ? src[i] : 0.0f;
         }
     }
     if (up != nullptr) {  // x is the gate of a feed-forward block
         const float* us = up + (src - x);
         float u[8];
         if (vec && i0 + 8 <= k) {
-            const float4 a = __ldg(reinterpret_cast<const float4*>(us)), c = __ldg(reinterpret_cast<const float4*>(us) + 1);
+            const float4 a = *reinterpret_cast<const float4*>(us), c = *(reinterpret_cast<const float4*>(us) + 1);
             u[0] = a.x; u[1] = a.y; u[2] = a.z; u[3] = a.w;
             u[4] = c.x; u[5] = c.y; u[6] = c.z; u[7] = c.w;
         } else {
 #pragma unroll
             for (int i = 0; i < 8; i++) {
-                u[i] = i0 + i < k ? __ldg(us + i) : 0.0f;
+                u[i] = i0 + i < k ? us[i] : 0.0f;
             }
         }
 #pragma unroll

@@ -287,6 +287,13 @@ __device__ __forceinline__ void run_to_smem(const f2 (&w)[8], uint32_t row_addr,
     }
 }
 
+// A scale of x or a bias, behind the wait for the kernel that writes it: not a read-only load, which might be moved in front of that wait.
+__device__ __forceinline__ float load_behind_wait(const float* p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+
 // Bytes of the parts of a CTA's shared memory.
 template <int TYPE>
 __host__ __device__ constexpr int raw_bytes() {
@@ -879,7 +886,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
             const int wi = weight_of(p, ft, ft0);
             const int64_t feature = (int64_t)(ft - ft0) * 128 + lane_row, features = pick(p.features, wi);
             const bool valid = feature < features;
-            const float bias = p.bias != nullptr && wi == 0 && valid ? __ldg(p.bias + feature) : 0.0f;
+            const float bias = p.bias != nullptr && wi == 0 && valid ? load_behind_wait(p.bias + feature) : 0.0f;
             // Columns c .. c + 7 of the tile are finished: to y, or (contraction split over the cluster) to this CTA's own partial tile
             // [column][128]. One warp per scheduler does this, so it is kept short: no test per value where the tile is whole.
             const int64_t row_bytes = features * 4;
@@ -928,7 +935,7 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
 #pragma unroll
                     for (int i = 0; i < NEXT; i++) {
                         const int on = AHEAD > 1 ? i : 0, off = AHEAD > 1 ? 0 : 32 * i;  // (AHEAD > 1: 32 columns)
-                        next[i] = lane + off < cols && (AHEAD == 1 || u + on < u1) ? __ldg(xs + (int64_t)on * p.xstride + off) : 0.0f;
+                        next[i] = lane + off < cols && (AHEAD == 1 || u + on < u1) ? load_behind_wait(xs + (int64_t)on * p.xstride + off) : 0.0f;
                     }
                     xs += (int64_t)AHEAD * p.xstride;
                 };

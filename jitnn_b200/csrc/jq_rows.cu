@@ -8,7 +8,7 @@ namespace rows {
 // x [m, k] FP32 (or silu(x) * up) -> its image (jq_rows_image.cuh), rows from m on zeros. One warp per row and 256-wide step of k, eight values a lane. Memory bound:
 // 4 bytes read and 4.5 written (to L2) a value.
 template <int NT>
-__global__ void __launch_bounds__(128) image_kernel(const float* __restrict__ x, const float* __restrict__ up, int m, int64_t k, int units, uint8_t* __restrict__ image,
+__global__ void __launch_bounds__(128) image_kernel(const float* x, const float* up, int m, int64_t k, int units, uint8_t* __restrict__ image,
                                                     float* __restrict__ scales, int vec) {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -20,18 +20,18 @@ __global__ void __launch_bounds__(128) image_kernel(const float* __restrict__ x,
     const int64_t i0 = (int64_t)u * 256 + lane * 8, at = (int64_t)row * k + i0;
     float v[8];
     if (row < m && vec && i0 + 8 <= k) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(x + at)), c = __ldg(reinterpret_cast<const float4*>(x + at) + 1);
+        const float4 a = *reinterpret_cast<const float4*>(x + at), c = *(reinterpret_cast<const float4*>(x + at) + 1);
         v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = c.x, v[5] = c.y, v[6] = c.z, v[7] = c.w;
     } else {
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            v[i] = row < m && i0 + i < k ? __ldg(x + at + i) : 0.0f;
+            v[i] = row < m && i0 + i < k ? x[at + i] : 0.0f;
         }
     }
     if (up != nullptr) {  // x is the gate of a feed-forward block
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            const float g = row < m && i0 + i < k ? __ldg(up + at + i) : 0.0f;
+            const float g = row < m && i0 + i < k ? up[at + i] : 0.0f;
             v[i] = (v[i] / (1.0f + expf(-v[i]))) * g;
         }
     }
