@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(PREP_WARPS * 32) blk32_image_kernel(const floa
 
 // FROM_X: no image in memory, every warp makes that of the 256-blocks that it multiplies itself, straight from x.
 template <int TYPE, int MT, int STAGES, bool FROM_X>
-__global__ void __launch_bounds__(THREADS, 2) gemv_blk32_i8_kernel(View v, const uint8_t* __restrict__ image, const float* x, int rows, const float* __restrict__ bias,
+__global__ void __launch_bounds__(THREADS, 2) gemv_blk32_i8_kernel(View v, const uint8_t* __restrict__ image, const float* x, int rows, const float* bias,
                                                                    float* __restrict__ y, int tiles) {
     using G = Geo<TYPE>;
     using I = Img<MT>;
@@ -321,6 +321,12 @@ __global__ void __launch_bounds__(THREADS, 2) gemv_blk32_i8_kernel(View v, const
     uint32_t cmp_slot = 0;
     for (int ti = 0; ti < my_tiles; ti++) {
         const int my_tile = (int)blockIdx.x + ti * (int)gridDim.x;
+        // the bias is on its way while the tile is multiplied: behind the sums it is a trip to memory, or across PCIe, that nothing hides
+        float ahead = 0.0f;
+        static_assert(16 * MT <= THREADS, "one result a thread");
+        if (bias != nullptr && tid < 16 * MT && (int64_t)my_tile * 16 + tid / MT < v.n) {
+            ahead = bias[(int64_t)my_tile * 16 + tid / MT];
+        }
         const uint8_t* blk = xd_lane + (size_t)warp * I::PB;
         for (int j = 0; j < nb; j++) {
             __syncwarp();                 // every lane is done reading the slot that is requested next
@@ -361,7 +367,7 @@ __global__ void __launch_bounds__(THREADS, 2) gemv_blk32_i8_kernel(View v, const
             constexpr int W = 16 * MT;
             const float sum = ((p[0] + p[W]) + (p[2 * W] + p[3 * W])) + ((p[4 * W] + p[5 * W]) + (p[6 * W] + p[7 * W]));
             if (m < rows && row < v.n) {
-                y[(int64_t)m * v.n + row] = sum + (bias != nullptr ? bias[row] : 0.0f);
+                y[(int64_t)m * v.n + row] = sum + ahead;
             }
         }
         parity ^= 1;

@@ -151,7 +151,7 @@ enum From { FROM_IMAGE, FROM_FLOATS, FROM_NORM };
 constexpr int NORM_MAX = 4;
 template <int MT, int STAGES, int NW, int OCC, bool Q5, bool PEER, From SRC>
 __global__ void __launch_bounds__(NW * 32, OCC) gemv_q4k_i8_kernel(View v, Second w2, const PeerOut* __restrict__ peerp, const uint8_t* __restrict__ image,
-                                                                  const float* xin, int rows, const float* __restrict__ bias, float* __restrict__ y,
+                                                                  const float* xin, int rows, const float* bias, float* __restrict__ y,
                                                                   int tiles, int KS, int max_tiles, long long wait_clocks, int* status, NormInput norm) {
     // Tiles 0 .. w2.first_tiles - 1 are rows of v, the tiles from w2.first_tiles on rows of the second weight w2 (same k,
     // same x, its own output), if there is one.
@@ -514,6 +514,12 @@ __global__ void __launch_bounds__(NW * 32, OCC) gemv_q4k_i8_kernel(View v, Secon
         }
         for (int ti = 0; ti < my_tiles; ti++) {
             const int my_tile = (int)blockIdx.x + ti * (int)gridDim.x;
+            // the bias is on its way while the tile is multiplied: behind the sums it is a trip to memory, or across PCIe, that nothing hides
+            float ahead = 0.0f;
+            static_assert(16 * MT <= THREADS, "one result a thread");
+            if (bias != nullptr && my_tile < w2.first_tiles && tid < 16 * MT && (int64_t)my_tile * 16 + tid / MT < v.n) {
+                ahead = bias[(int64_t)my_tile * 16 + tid / MT];
+            }
             const uint8_t* blk = xd_lane + (size_t)warp * C::PB;
             for (int j = 0; j < nb; j++) {
                 // Every lane is done with the slot that is requested next: its values have been multiplied in compute(), in front of this point, and it is
@@ -608,7 +614,7 @@ __global__ void __launch_bounds__(NW * 32, OCC) gemv_q4k_i8_kernel(View v, Secon
                 if (sl + 1 < nslices) {
                     carry[(size_t)ti * 16 * MT + o] = sum;
                 } else if (m < rows && row < n) {
-                    const float val = sum + (bias != nullptr && !second ? bias[row] : 0.0f);
+                    const float val = sum + ahead;
                     if constexpr (!PEER) {
                         yo[(int64_t)m * n + row] = val;
                     } else {

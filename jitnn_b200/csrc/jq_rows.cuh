@@ -609,6 +609,10 @@ __global__ void __launch_bounds__((Shape<TYPE, NT>::THREADS), 1) rows_kernel(con
         const bool keep = u1 - u0 <= 16;  // (a short contraction's stay for the next tile)
         fetch(u0);
         for (int ft = p.first_ft + cluster_id; ft < p.ftiles && ok; ft += clusters) {
+            int ft0;
+            const int w = weight_of(ft, ft0);
+            const int64_t row = (int64_t)(ft - ft0) * 128 + lane_row, n = mm::pick(p.n, w);
+            const float bias = w == 0 && p.bias != nullptr && row < n ? load_scale<AFTER>(p.bias + row) : 0.0f;  // (on its way while the tile is multiplied)
             f2 sum[C / 2], total[C / 2];
 #pragma unroll
             for (int i = 0; i < C / 2; i++) {
@@ -776,18 +780,14 @@ __global__ void __launch_bounds__((Shape<TYPE, NT>::THREADS), 1) rows_kernel(con
             if (!ok || p.ksplit > 1) {
                 break;  // (one tile per cluster)
             }
-            int ft0;
-            const int w = weight_of(ft, ft0);
-            const int64_t row = (int64_t)(ft - ft0) * 128 + lane_row, n = mm::pick(p.n, w);
             if (row < n) {
-                const float b = w == 0 && p.bias != nullptr ? __ldg(p.bias + row) : 0.0f;
                 float* at = mm::pick(p.y, w) + (int64_t)c0 * n + row;
 #pragma unroll
                 for (int i = 0; i < C; i++, at += n) {
                     float v[2];
                     unpack2(total[i / 2], v[0], v[1]);
                     if (c0 + i < p.m) {
-                        *at = v[i % 2] + b;
+                        *at = v[i % 2] + bias;
                     }
                 }
             }
