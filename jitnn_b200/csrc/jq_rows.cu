@@ -67,7 +67,8 @@ int rows_image(cudaStream_t s, int m, int64_t k, uint8_t** image, float** scales
 }
 
 // ys[i] [rows, n_i] = x . W_i^T (+ bias for the first), x [rows, k] or silu(x) * up, for up to three weights of one k: one image, the weights of one
-// format in one launch. x null: the kernel in front has written the image.
+// format in one launch. x null: the kernel in front has written the image. Only the first launch waits for it; the others, further tiles or another format, start as SMs
+// become free.
 int launch_rows(const View* vs, int count, const float* x, const float* up, int m, const float* bias, float* const* ys, cudaStream_t s) {
     using namespace rows;
     const int64_t k = vs[0].k;
@@ -96,6 +97,7 @@ int launch_rows(const View* vs, int count, const float* x, const float* up, int 
         JQ_CUDA(cudaLaunchKernelEx(&cfg, nt == 8 ? image_kernel<8> : image_kernel<16>, x, up, m, k, units, image, scales, vec));
         count_launch();
     }
+    bool after = false;
     for (int i = 0; i < count && rc == JQ_OK; i++) {
         // the weights of one format in one launch, with the first of them
         Args a = {};
@@ -125,14 +127,23 @@ int launch_rows(const View* vs, int count, const float* x, const float* up, int 
         a.m = m;
         a.status = status;
         a.wait_clocks = (long long)g_opt_wait_limit_us.load(std::memory_order_relaxed) * 2000;  // about 2 GHz
+        bool more = false;  // another format is behind
+        for (int j = i + 1; j < count; j++) {
+            bool fresh = true;
+            for (int h = 0; h < j; h++) {
+                fresh = fresh && vs[h].type != vs[j].type;
+            }
+            more = more || fresh;
+        }
         Parts parts;
         cut(end, units, unit_ns(vs[i].type), MAX_PARTS, parts);
         for (int c = 0, at = 0; c < parts.count && rc == JQ_OK; c++) {
             a.first_ft = at;
             a.ftiles = at += parts.tiles[c];
             a.ksplit = parts.ksplit[c];
-            a.followed = c + 1 < parts.count;
-            rc = launch_any(vs[i].type, a, a.ksplit > 1 ? parts.tiles[c] * a.ksplit : (parts.tiles[c] < 148 ? parts.tiles[c] : 148), c > 0, s);
+            a.followed = more || c + 1 < parts.count;
+            rc = launch_any(vs[i].type, a, a.ksplit > 1 ? parts.tiles[c] * a.ksplit : (parts.tiles[c] < 148 ? parts.tiles[c] : 148), after, s);
+            after = true;
         }
     }
     return rc;
