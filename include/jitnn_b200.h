@@ -119,9 +119,9 @@ JQ_API int jq_dequantize(const jq_weight* w, float* dst, int dst_mem, void* stre
  * non-finite outputs (Q4_K, Q5_K: NaN in every output of that row of x). Stands in for Gguf.linear(x, w, bias) (ops/Gguf.java:76-98) and
  * Quant.linear / F.linearQ8 (ops/Quant.java:66-80): any m >= 0 (leading axes of x flattened by the
  * caller as ops/Gguf.java:86-93 does), bias may be NULL. Rows are dispatched like the reference
- * dispatches them (ops/Gguf.java:90): few rows to the fused dequantise-GEMV kernels, more to the tensor cores (from 5 to 12 rows on, by format, the
- * rows kernel; always above 16 the matrix kernel), which take x and the weights as sums of two half-precision numbers (22 significant bits, relative to the largest
- * magnitude of a 256-element block) and add up in FP32 (errors of 1.3e-7 to 2.4e-7 of the result's norm; the decode kernels' are 2.8e-7 to 3.2e-7),
+ * dispatches them (ops/Gguf.java:90): few rows to the fused dequantise-GEMV kernels, more to the tensor cores (from 3 to 9 rows on, by format, the
+ * rows kernel; always above 16 the matrix kernel), which take x, and the weights where one does not hold them, as sums of two half-precision numbers (22 significant bits, relative to
+ * the largest magnitude of a 256-element block) and add up in FP32 (errors of 1.1e-7 to 2.6e-7 of the result's norm; the decode kernels' are 2.8e-7 to 3.2e-7),
  * unless the bfloat16 prefill path is selected with jq_set_option. `mem` says where x, bias and y live (all three alike); with JQ_MEM_DEVICE they must
  * be 16-byte aligned and `stream` is the CUDA stream (cudaStream_t, NULL = default stream).
  */

@@ -18,8 +18,9 @@ inline double unit_ns(int type) { return type == JQ_TYPE_Q4_K ? 630.0 : (type ==
 // leave most of the chip idle for a whole contraction, with its contraction split over clusters (57344 x 8192: 448 tiles are three waves and four
 // tiles: 85.5 us in one launch, 71.7 in two). The launch behind starts where SMs become free; GAP_NS is its own start.
 // The cost of a launch is its waves' units and 1700 ns a wave, for a cluster 1600 more, which are rounder than what 16 rows of x take, us: one wave of 8, 16 and 32
-// units 10.7, 15.5 and 25.7 (Q4_K) and 15.5, 24.7 and 43.3 (Q6_K), that is 5.4 and 6.2 beside the units, the image kernel in front among them; a second wave in
-// the same launch 0.3 beside its units; 16 units a thread block in clusters of 2, 4 and 8 2.6, 2.7 and 3.1 (Q4_K) and 1.7, 2.7 and 2.4 (Q6_K) more than alone.
+// units 10.7, 15.5 and 25.7 (Q4_K) and 15.5, 24.7 and 43.3 (Q6_K, when its weights were two halves each; 32 units take 38.2 now), that is 5.4 and 6.2 beside the
+// units, the image kernel in front among them; a second wave in the same launch 0.3 beside its units; 16 units a thread block in clusters of 2, 4 and 8 2.6, 2.7
+// and 3.1 (Q4_K) and 1.7, 2.7 and 2.4 (Q6_K) more than alone.
 constexpr int MAX_PARTS = 3;
 constexpr double GAP_NS = 2500.0;
 struct Parts {
