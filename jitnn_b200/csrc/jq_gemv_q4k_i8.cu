@@ -149,7 +149,7 @@ enum From { FROM_IMAGE, FROM_FLOATS, FROM_NORM };
 // only work is 16 KB, on a chain where every kernel takes more than four microseconds whatever its size (one token, 8 layers of the 7B width
 // at position 576: 530 -> 493 us). Up to NORM_MAX super-blocks a warp, that is k <= 8192; their values stay in registers.
 constexpr int NORM_MAX = 4;
-template <int MT, int STAGES, int NW, int OCC, bool Q5, bool PEER, From SRC>
+template <int MT, int STAGES, int NW, int OCC, bool Q5, bool PEER, From SRC, bool BIAS>
 __global__ void __launch_bounds__(NW * 32, OCC) gemv_q4k_i8_kernel(View v, Second w2, const PeerOut* __restrict__ peerp, const uint8_t* __restrict__ image,
                                                                   const float* xin, int rows, const float* bias, float* __restrict__ y,
                                                                   int tiles, int KS, int max_tiles, long long wait_clocks, int* status, NormInput norm) {
@@ -514,11 +514,15 @@ __global__ void __launch_bounds__(NW * 32, OCC) gemv_q4k_i8_kernel(View v, Secon
         }
         for (int ti = 0; ti < my_tiles; ti++) {
             const int my_tile = (int)blockIdx.x + ti * (int)gridDim.x;
-            // the bias is on its way while the tile is multiplied: behind the sums it is a trip to memory, or across PCIe, that nothing hides
+            // the bias is on its way while the tile is multiplied: behind the sums it is a trip to memory, or across PCIe, that nothing hides (4096 x 4096, one row, us:
+            // 4.07 there, 3.93 here; host arrays 29.7, 28.3). An instance of its own: the register and the tests cost calls without a bias 0.2 us a launch (eight shapes with
+            // one and eight rows 94.1, without them 92.2). Through shared memory by cp.async: 96.0.
             float ahead = 0.0f;
             static_assert(16 * MT <= THREADS, "one result a thread");
-            if (bias != nullptr && my_tile < w2.first_tiles && tid < 16 * MT && (int64_t)my_tile * 16 + tid / MT < v.n) {
-                ahead = bias[(int64_t)my_tile * 16 + tid / MT];
+            if constexpr (BIAS) {
+                if (bias != nullptr && my_tile < w2.first_tiles && tid < 16 * MT && (int64_t)my_tile * 16 + tid / MT < v.n) {
+                    ahead = bias[(int64_t)my_tile * 16 + tid / MT];
+                }
             }
             const uint8_t* blk = xd_lane + (size_t)warp * C::PB;
             for (int j = 0; j < nb; j++) {
@@ -665,11 +669,14 @@ int sm_count() {
 template <int MT, int STAGES, int NW, int OCC, bool Q5, bool PEER, From SRC>
 int launch(const View& v, const Second& w2, const PeerOut& peer, const uint8_t* image, const float* x, int rows, const float* bias, float* y, cudaStream_t s,
            int KS, int grid, int max_tiles, size_t smem, const NormInput& norm) {
+    constexpr bool CAN_BIAS = SRC != FROM_NORM, CAN_NONE = !PEER;  // (the exchange takes a bias or none in one instance)
+    const auto with_bias = gemv_q4k_i8_kernel<MT, STAGES, NW, OCC, Q5, PEER, SRC, CAN_BIAS>, without = gemv_q4k_i8_kernel<MT, STAGES, NW, OCC, Q5, PEER, SRC, !CAN_NONE>;
     static std::atomic<uint64_t> configured{0};  // the opt-in for large dynamic shared memory is per device
     int dev = 0;
     JQ_CUDA(cudaGetDevice(&dev));
     if ((configured.load() >> (dev & 63) & 1) == 0) {
-        JQ_CUDA(cudaFuncSetAttribute(gemv_q4k_i8_kernel<MT, STAGES, NW, OCC, Q5, PEER, SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
+        JQ_CUDA(cudaFuncSetAttribute(with_bias, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
+        JQ_CUDA(cudaFuncSetAttribute(without, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
         configured.fetch_or((uint64_t)1 << (dev & 63));
     }
     const int tiles = (int)((v.n + 15) / 16) + (w2.q != nullptr ? (int)((w2.n + 15) / 16) : 0) + (w2.q3 != nullptr ? (int)((w2.n3 + 15) / 16) : 0);
@@ -689,7 +696,7 @@ int launch(const View& v, const Second& w2, const PeerOut& peer, const uint8_t* 
     if (rc != JQ_OK) {
         return rc;
     }
-    JQ_CUDA(cudaLaunchKernelEx(&cfg, gemv_q4k_i8_kernel<MT, STAGES, NW, OCC, Q5, PEER, SRC>, v, w2, (const PeerOut*)(PEER ? peer.table : nullptr), image, x, rows,
+    JQ_CUDA(cudaLaunchKernelEx(&cfg, bias != nullptr ? with_bias : without, v, w2, (const PeerOut*)(PEER ? peer.table : nullptr), image, x, rows,
                                bias, y, tiles, KS, max_tiles, wait_clocks, status, norm));
     count_launch();
     return JQ_OK;
