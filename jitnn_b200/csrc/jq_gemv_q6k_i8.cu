@@ -670,14 +670,20 @@ int launch_gemv_q6k_i8_imaged(const View& v, const uint8_t* image, const float* 
     return run<1>(v, nullptr, 1, bias, y, s, const_cast<uint8_t*>(image), handled);
 }
 
-// Two thread blocks per SM, three ring stages and the image of the whole k.
+// Two thread blocks per SM with the image of the whole k, and three ring stages, or from k = 6656 on, where those leave no room for it, two. A step of 3 layers with
+// the norm kernel in front of wq|wk and wv, and this, us: k = 6656 314 and 305, 7168 330 and 322, 8192 429.5 and 428.3.
+static int normed_stages(int KB) { return smem_bytes<1>(KB, 3, false, 0) <= SMEM_MAX / 2 - 1024 ? 3 : 2; }
+
 bool gemv_q6k_i8_normed_takes(const View& v) {
-    return v.type == JQ_TYPE_Q6_K && v.n > 0 && v.k > 0 && v.k <= NORM_MAX * WARPS * 256 && smem_bytes<1>((int)(v.k / 256), 3, false, 0) <= SMEM_MAX / 2 - 1024;
+    return v.type == JQ_TYPE_Q6_K && v.n > 0 && v.k > 0 && v.k <= NORM_MAX * WARPS * 256 && smem_bytes<1>((int)(v.k / 256), 2, false, 0) <= SMEM_MAX / 2 - 1024;
 }
 
 int launch_gemv_q6k_i8_normed(const View& v, const NormInput& norm, float* y, cudaStream_t s) {
-    const int KB = (int)(v.k / 256), tiles = (int)((v.n + 15) / 16), grid = tiles < 2 * sm_count() ? tiles : 2 * sm_count();
-    return launch<1, 3, 2, FROM_NORM>(v, nullptr, nullptr, 1, nullptr, y, s, KB, grid, (tiles + grid - 1) / grid, smem_bytes<1>(KB, 3, false, 0), norm);
+    const int KB = (int)(v.k / 256), tiles = (int)((v.n + 15) / 16), grid = tiles < 2 * sm_count() ? tiles : 2 * sm_count(), max_tiles = (tiles + grid - 1) / grid;
+    const int stages = normed_stages(KB);
+    const size_t smem = smem_bytes<1>(KB, stages, false, 0);
+    return stages == 3 ? launch<1, 3, 2, FROM_NORM>(v, nullptr, nullptr, 1, nullptr, y, s, KB, grid, max_tiles, smem, norm)
+                       : launch<1, 2, 2, FROM_NORM>(v, nullptr, nullptr, 1, nullptr, y, s, KB, grid, max_tiles, smem, norm);
 }
 
 }  // namespace jq

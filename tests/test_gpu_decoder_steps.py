@@ -109,3 +109,39 @@ def test_norms_inside_and_in_front(dim, hidden):
     for a, b in zip(*out):
         assert np.abs(a - b).max() <= 1e-5 * np.abs(a).max()  # FP32 throughout, sums in other orders
     dec.close()
+
+
+# a Q6_K wv beside Q4_K wq and wk, which makes the norm itself: 20 super-blocks (no multiple of its eight warps), the first width with two ring stages in place
+# of three (26 super-blocks), the widest
+@pytest.mark.parametrize("dim,heads,hidden", [(5120, 40, 2048), (6656, 52, 2048), (8192, 64, 1024)])
+def test_a_q6k_wv_makes_its_own_norm(dim, heads, hidden):
+    """The fused single-token step against the general kernels; a layer with a Q6_K wv takes one launch more than one whose weights are all Q4_K."""
+    vocab, L = 512, jitnn_b200.load()
+    g = torch.Generator(device="cuda").manual_seed(dim)
+    launches = []
+    for fine in ("Q4_K", "Q6_K"):
+        def lin(n, k, t="Q4_K"):
+            return (t, synth.QUANTIZERS[t](torch.randn(n, k, generator=g, device="cuda") * 0.02).cpu().numpy().reshape(-1), n, k)
+
+        w = {"tok_embeddings": torch.randn(vocab, dim, generator=g, device="cuda").cpu().numpy(), "norm": np.ones(dim, np.float32), "output": lin(vocab, dim)}
+        for layer in range(2):
+            p = "layers.%d." % layer
+            w[p + "attention_norm"] = (1.0 + 0.1 * torch.randn(dim, generator=g, device="cuda")).cpu().numpy()
+            w[p + "ffn_norm"] = (1.0 + 0.1 * torch.randn(dim, generator=g, device="cuda")).cpu().numpy()
+            w.update({p + "wq": lin(dim, dim), p + "wk": lin(256, dim), p + "wv": lin(256, dim, fine), p + "wo": lin(dim, dim), p + "w1": lin(hidden, dim),
+                      p + "w3": lin(hidden, dim), p + "w2": lin(dim, hidden)})
+        dec = LlamaDecoder(2, dim, heads, 2, hidden, vocab, 8)
+        dec.load(w)
+        before = L.jq_launch_count()
+        fused = [np.array(dec.forward([1], 0)[0])]  # (the first step is issued kernel by kernel)
+        launches.append(L.jq_launch_count() - before)
+        fused += [np.array(dec.forward([7 * pos + 1], pos)[0]) for pos in (1, 2)]
+        L.jq_set_option(b"decoder_fused", 0)
+        try:
+            general = [np.array(dec.forward([7 * pos + 1], pos)[0]) for pos in range(3)]
+        finally:
+            L.jq_set_option(b"decoder_fused", 1)
+        for a, b in zip(general, fused):
+            assert np.abs(a - b).max() <= 1e-5 * np.abs(a).max()  # FP32 throughout, sums in other orders
+        dec.close()
+    assert launches[1] - launches[0] == 2
