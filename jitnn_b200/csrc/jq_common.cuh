@@ -185,6 +185,17 @@ int decoder_peer_status(int* status);
 // Q6_K for one row of x whose activation image (jq_q6k_image.cuh) a kernel earlier in the stream has written.
 size_t q6k_image_bytes_one_row(int64_t k);
 int launch_gemv_q6k_i8_imaged(const View& v, const uint8_t* image, const float* bias, float* y, cudaStream_t s, bool* handled);
+// Whether the GEMV of one or two rows of x in Q6_K or a 32-element format makes the image of x itself (the bits are those of the image kernel's). Every thread block then
+// makes all of it, so not for more than 8192 values (four blocks a warp), nor where x lies in host memory, which is read once. Up to 6144 values, up to 32 tiles of rows
+// and with more tiles than SMs it saves 0.3 to 1.6 us of the GPU's time and a launch of 1.6 us on the host. Between, thread blocks read the same values all at once with no
+// weights behind to hide it. Weights from device memory, inside / image kernel, us, replayed from a graph and (launched one after the other):
+//   one row of 8192, n = 1024    Q8_0 5.6 / 4.9 (5.6 / 5.7), Q4_0 5.3 / 4.3 (6.1 / 5.6), Q4_1 5.1 / 4.7 (6.2 / 5.6), Q6_K 6.3 / 6.9 (8.0 / 7.3)
+//                    n = 2048    Q8_0 6.1 / 5.6 (6.6 / 6.9), Q4_0 6.0 / 4.9 (6.3 / 5.7), Q4_1 6.0 / 5.5 (6.5 / 5.7), Q6_K 7.6 / 7.5 (8.2 / 8.4)
+//   two rows of 4096, n = 1024   Q8_0 4.4 / 3.9 (5.5 / 6.8), Q4_0 4.1 / 4.0 (3.8 / 5.5), Q4_1 4.0 / 3.5 (3.8 / 5.8), Q6_K 5.3 / 5.1 (5.5 / 5.9)
+//                    n = 2048    Q8_0 4.8 / 4.3 (5.2 / 5.7), Q4_0 4.5 / 3.8 (4.9 / 5.8), Q4_1 4.5 / 4.5 (4.9 / 5.7), Q6_K 5.7 / 5.3 (6.0 / 5.9)
+//   and on either side of that, one row of 8192: n = 256 Q8_0 4.5 / 4.6, Q6_K 5.2 / 5.9; n = 4096 Q8_0 7.7 / 8.4, Q6_K 7.9 / 8.2.
+// So one row of Q4_0 and Q4_1 has the image kernel there; one row of Q8_0, and two rows, have it where a graph is captured, whose replays cost the host nothing.
+bool gemv_image_inside(const View& v, int rows, bool x_remote, cudaStream_t s);
 // The same for Q6_K, rows <= 4.
 int launch_gemv_q6k_i8(const View& v, const float* x, int rows, const float* bias, float* y, cudaStream_t s, uint8_t* image, bool* handled, bool x_remote);
 size_t gemv_q6k_i8_scratch_bytes(int64_t k, int rows);

@@ -87,6 +87,24 @@ static int by_rows(const View& v, const float* x, int rows, const float* bias, f
     return run<TYPE, 16>(v, x, rows, bias, y, s);
 }
 
+bool gemv_image_inside(const View& v, int rows, bool x_remote, cudaStream_t s) {
+    const int64_t values = rows * v.k;
+    if (rows > 2 || values > 8192 || x_remote) {
+        return false;
+    }
+    if (values <= 6144 || v.n <= 32 * 16 || v.n > 148 * 16) {
+        return true;
+    }
+    if (rows == 1 && v.type != JQ_TYPE_Q8_0) {
+        return v.type == JQ_TYPE_Q6_K;
+    }
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &status) != cudaSuccess) {
+        cudaGetLastError();  // (the default stream while another is captured: the launch itself says so)
+    }
+    return status == cudaStreamCaptureStatusNone;
+}
+
 // rows in [1, 16].
 int launch_gemv(const View& v, const float* x, int rows, const float* bias, float* y, cudaStream_t s, bool x_remote) {
     if (v.n == 0) {

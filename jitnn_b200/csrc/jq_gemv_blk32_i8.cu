@@ -397,13 +397,6 @@ bool image_fits(int64_t k, int rows) {
     return (rows == 1 ? smem_bytes<TYPE, 1>((int)(k / 256)) : smem_bytes<TYPE, 2>((int)(k / 256))) <= SMEM_MAX;
 }
 
-// The GEMV builds the image itself for up to this many values of x: four blocks a warp. Every thread block then makes all of it, redundant work that grows with
-// them; x in host memory is never read once per thread block. Replayed from a graph, image kernel / built here, us: one row, 4096 x 4096 Q8_0 4.6 / 3.7, Q4_0 4.4 /
-// 3.9, Q4_1 4.4 / 4.0; 1024 x 1024 2.8 / 1.8; 32000 x 4096 23.3 / 21.9, 15.8 / 13.6, 16.6 / 14.6; one row of 8192 (4096 x 8192) 7.2 / 7.1, 5.9 / 6.1, 6.4 / 6.4; two rows of
-// 4096 (4096 x 4096) 4.6 / 4.7, 4.6 / 4.8, 4.6 / 4.8, at most 7.2 / 8.0 (11008 x 4096, Q4_0). A call that is launched, not replayed, saves 2 us of host time besides,
-// and that is the longer of the two for most of these.
-constexpr int64_t FROM_X = 8192;
-
 template <int TYPE, int MT, bool FROM_X>
 int run(const View& v, const float* x, int rows, const float* bias, float* y, cudaStream_t s, uint8_t* image) {
     constexpr int STAGES = stages_of(TYPE);
@@ -471,7 +464,7 @@ int launch_gemv_blk32_i8(const View& v, const float* x, int rows, const float* b
         return JQ_OK;
     }
     *handled = true;
-    const bool from_x = rows * v.k <= FROM_X && !x_remote;
+    const bool from_x = gemv_image_inside(v, rows, x_remote, s);
     switch (v.type) {
         case JQ_TYPE_Q8_0: return by_rows<JQ_TYPE_Q8_0>(v, x, rows, bias, y, s, image, from_x);
         case JQ_TYPE_Q4_0: return by_rows<JQ_TYPE_Q4_0>(v, x, rows, bias, y, s, image, from_x);

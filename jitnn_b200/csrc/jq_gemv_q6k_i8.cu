@@ -508,8 +508,6 @@ __global__ void __launch_bounds__(THREADS, OCC) gemv_q6k_i8_kernel(View v, const
     }
 }
 
-constexpr int64_t FROM_X_VALUES = 8192;
-
 int g_sms = 0;
 int sm_count() {
     if (g_sms == 0) {
@@ -605,11 +603,7 @@ int run(const View& v, const float* x, int rows, const float* bias, float* y, cu
     }
     *handled = true;
     if constexpr (MT <= 2) {
-        // Up to FROM_X_VALUES values of x, four super-blocks a warp: the GEMV builds the image itself (every thread block makes all of it, redundant work that grows with
-        // them; x in host memory is never read once per thread block). Replayed from a graph, image kernel / built here, us: one row,
-        // 1024 x 1024 3.2 / 2.0, 4096 x 4096 5.6 / 4.5, 32000 x 4096 21.8 / 20.3, 4096 x 8192 8.2 / 8.1; two rows, 4096 x 2048 4.6 / 3.7, 4096 x 4096 5.6 / 5.9, 32000 x 4096 22.1 / 22.0. A
-        // launched call saves 2 us of host time besides.
-        if (x != nullptr && rows * v.k <= FROM_X_VALUES && !x_remote && !sliced) {
+        if (x != nullptr && !sliced && gemv_image_inside(v, rows, x_remote, s)) {
             return stages == 3 ? launch<MT, 3, 2, FROM_X>(v, image, x, rows, bias, y, s, KS, grid, max_tiles, smem)
                                : launch<MT, 2, 2, FROM_X>(v, image, x, rows, bias, y, s, KS, grid, max_tiles, smem);
         }

@@ -1,4 +1,4 @@
-"""The decode GEMVs of Q6_K and the 32-element formats at the line between building x's image themselves and reading that of an image kernel.
+"""The decode GEMVs of Q6_K and the 32-element formats at the lines between building x's image themselves and reading that of an image kernel.
 
 Both make the same digits of x and sum in the same order, so that neighbours across the line differ by nothing but the launches. The reference is the product
 of the oracle's dequantised weights in double; x keeps 22 bits of the largest of its 256 neighbours, 4e-7 of what is added up on ordinary weights.
@@ -57,3 +57,34 @@ def test_x_of_every_size_and_of_the_kernel_in_front(t):
                 assert float((y[row].double() - ref[row]).abs().max()) <= 2.0 ** -124 * float(wd.abs().sum(1).max())
             else:
                 assert float((y[row].double() - ref[row]).norm() / ref[row].norm()) <= REL
+
+
+# the first and the last number of rows of W with which the rule looks at more than the values of x, and those beside them
+@pytest.mark.parametrize("n", [512, 513, 2368, 2369])
+@pytest.mark.parametrize("k,m", [(6144, 1), (3072, 2), (6400, 1), (3328, 2), (8192, 1), (4096, 2)])
+@pytest.mark.parametrize("t", ["Q6_K", "Q8_0", "Q4_1"])
+def test_the_image_kernel_between_few_and_many_rows(t, k, m, n):
+    """Which of the two routes a launched and a captured call take, and that all give the same bits."""
+    L = jitnn_b200.load()
+    raw = synth.random_valid_blocks(t, n, k, seed=k + n).numpy().reshape(-1)
+    w, wd = Tensor.quantized(t, raw, n, k), torch.from_numpy(oracle.dequantize(t, raw).reshape(n, k)).cuda().double()
+    x = torch.randn(m, k, generator=torch.Generator().manual_seed(m)).cuda()
+    between = m * k > 6144 and 512 < n <= 2368
+    stream = torch.cuda.Stream()
+    counts = []
+    with torch.cuda.stream(stream):
+        stream.wait_stream(torch.cuda.default_stream())
+        before = L.jq_launch_count()
+        y = Gguf.linear(x, w)
+        counts.append(L.jq_launch_count() - before)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        before = L.jq_launch_count()
+        z = Gguf.linear(x, w)
+        counts.append(L.jq_launch_count() - before)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert counts == [2 if between and m == 1 and t == "Q4_1" else 1, 2 if between and (m == 2 or t != "Q6_K") else 1]
+    assert torch.equal(y, z) and np.array_equal(Gguf.linear(x.cpu().numpy(), w), y.cpu().numpy())
+    ref, size = x.double() @ wd.T, ((x.double() ** 2) @ (wd ** 2).T).sqrt()
+    assert float(((y.double() - ref).abs() / size).max()) <= REL
