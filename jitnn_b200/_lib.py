@@ -4,11 +4,14 @@ The library is the product: there is no Python or CPU fallback. ``load()`` raise
 object has not been built (``python -m jitnn_b200.build``).
 """
 import ctypes
+import importlib.metadata
+import importlib.util
 import os
+import sys
+import warnings
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libjitnn_b200.so")
-FRONT_PATH = os.path.join(HERE, "_front.so")
 
 JQ_OK = 0
 JQ_ERR_INVALID, JQ_ERR_OOM, JQ_ERR_CUDA, JQ_ERR_NCCL, JQ_ERR_TIMEOUT, JQ_ERR_UNSUPPORTED = -1, -2, -3, -4, -5, -6
@@ -94,16 +97,33 @@ def load():
     return _lib
 
 
+def front_path():
+    """Where the native front of calls on torch tensors is (built from csrc/front.cpp), for this Python and the installed torch: it is compiled against both, and another's is not
+    loaded. None without torch."""
+    try:
+        torch = importlib.metadata.version("torch")
+    except importlib.metadata.PackageNotFoundError:
+        return None
+    return os.path.join(HERE, "_front.%s.torch-%s.so" % (sys.implementation.cache_tag, torch))
+
+
 def load_front(weight_class):
-    """The native front of calls on torch tensors (csrc/front.cpp), built against the torch it runs with; bound to the library's functions."""
+    """The native front, bound to the library's functions; None where there is none for this torch: the code in ops.py serves all its calls, a few microseconds slower."""
     import torch  # noqa: F401  (its libraries are what the module is linked to)
-    if not os.path.exists(FRONT_PATH):
-        raise ImportError("_front.so is not built: run `python -m jitnn_b200.build`; calls on torch tensors need it")
-    from . import _front
+    path = front_path()
+    if path is None or not os.path.exists(path):
+        return None
+    try:
+        spec = importlib.util.spec_from_file_location(__package__ + "._front", path)
+        front = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(front)
+    except ImportError as e:
+        warnings.warn("%s cannot be loaded (%s): calls on torch tensors go without it" % (os.path.basename(path), e))
+        return None
     L = ctypes.CDLL(LIB_PATH)  # (the one that load() has)
     names = ("jq_linear_f32", "jq_linear_bf16", "jq_linear_backward_f32", "jq_dequantize", "jq_quantize_q8_0")
-    _front.bind(weight_class, check, *(ctypes.cast(getattr(L, name), vp).value for name in names))
-    return _front
+    front.bind(weight_class, check, *(ctypes.cast(getattr(L, name), vp).value for name in names))
+    return front
 
 
 def last_error():

@@ -1,9 +1,10 @@
-"""Builds ``libjitnn_b200.so`` in-tree with nvcc for sm_100a, and ``_front.so``, the Python front of calls on torch tensors, with the C++ compiler.
+"""Builds ``libjitnn_b200.so`` in-tree with nvcc for sm_100a and, where a torch with CUDA is installed, the native front of Python's calls on torch tensors.
 
     python -m jitnn_b200.build [--force] [--verbose]
 
 Each ``csrc/*.cu`` is compiled to an object under ``csrc/build/`` (only when it or a header is
-newer than its object) and the objects are linked into ``jitnn_b200/libjitnn_b200.so``.
+newer than its object) and the objects are linked into ``jitnn_b200/libjitnn_b200.so``. The front (``csrc/front.cpp``) is a convenience of
+the Python binding: the library does not need it, and is built whatever becomes of it.
 """
 import concurrent.futures
 import glob
@@ -11,13 +12,16 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
+from importlib.util import find_spec
+
+from jitnn_b200 import _lib
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "build")
 LIB = os.path.join(HERE, "libjitnn_b200.so")
 FRONT_SRC = os.path.join(CSRC, "front.cpp")
-FRONT = os.path.join(HERE, "_front.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -47,20 +51,26 @@ def _compile(src, obj, verbose, extra):
 
 
 def build_front(force=False):
-    """Against the torch that is installed here, which is also the one it has to run with."""
-    if not force and os.path.exists(FRONT) and os.path.getmtime(FRONT) >= os.path.getmtime(FRONT_SRC):
-        return FRONT
-    import sysconfig
-    from importlib.util import find_spec
-    torch = os.path.dirname(find_spec("torch").origin)
+    """The front for this Python and the installed torch, whose versions its name carries; None where there is no torch with CUDA to build it against."""
+    front, spec = _lib.front_path(), find_spec("torch")
+    if front is None or spec is None or spec.origin is None:
+        return None
+    torch = os.path.dirname(spec.origin)
+    if not os.path.exists(os.path.join(torch, "lib", "libtorch_cuda.so")):
+        return None
+    if not force and os.path.exists(front) and os.path.getmtime(front) >= os.path.getmtime(FRONT_SRC):
+        return front
     cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc()))), "include")
     cmd = [shutil.which("g++") or "c++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden"]
     cmd += ["-I" + d for d in (os.path.join(torch, "include"), os.path.join(torch, "include", "torch", "csrc", "api", "include"), sysconfig.get_path("include"), cuda)]
-    cmd += [FRONT_SRC, "-o", FRONT, "-L" + os.path.join(torch, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"]
+    cmd += [FRONT_SRC, "-o", front, "-L" + os.path.join(torch, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
-        raise RuntimeError("the build of _front.so failed:\n%s\n%s" % (res.stdout, res.stderr))
-    return FRONT
+        raise RuntimeError("the build of %s failed:\n%s\n%s" % (os.path.basename(front), res.stdout, res.stderr))
+    for old in glob.glob(os.path.join(os.path.dirname(front), "_front*.so")):
+        if old != front:
+            os.remove(old)  # another torch's
+    return front
 
 
 def build(force=False, verbose=False, ptxas_info=False):
@@ -80,12 +90,15 @@ def build(force=False, verbose=False, ptxas_info=False):
         front = pool.submit(build_front, force)
         for f in [pool.submit(_compile, s, o, verbose or ptxas_info, extra) for s, o in jobs]:
             f.result()
-        front.result()
     if jobs or not os.path.exists(LIB):
         cmd = [nvcc(), "-shared", "-o", LIB] + objects + ["-gencode", "arch=compute_100a,code=sm_100a", "-cudart", "static"]
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError("link failed:\n%s\n%s" % (res.stdout, res.stderr))
+    try:
+        front.result()
+    except (RuntimeError, OSError) as e:
+        sys.stderr.write("%s\nCalls on torch tensors go without the native front.\n" % e)
     return LIB
 
 

@@ -149,7 +149,7 @@ class Tensor:
 
 # Calls on torch tensors. A decode linear takes a few microseconds on the GPU, less than the host needs for a chain of torch calls around it. So the plain
 # case, an ordinary contiguous tensor of the right type on the weight's device, is taken by native code as a whole (csrc/front.cpp), 4.0 us a call in place
-# of 7.4; it hands back None for everything else, which goes on here. It comes in with torch, on the first call with a torch tensor.
+# of 7.4; it hands back None for everything else, which goes on here, as all calls do where it is not built. It comes in with torch, on the first call with a torch tensor.
 _torch = None
 _front = None
 
