@@ -1097,14 +1097,14 @@ __global__ void __launch_bounds__((Shape<TYPE, FP32, BWD, NMAX>::THREADS), 1) ma
                 if (f + 4 <= features && ((uintptr_t)at & 15) == 0) {
                     float4 b = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     if (bias != nullptr) {
-                        b = make_float4(__ldg(bias + f), __ldg(bias + f + 1), __ldg(bias + f + 2), __ldg(bias + f + 3));
+                        b = make_float4(load_behind_wait(bias + f), load_behind_wait(bias + f + 1), load_behind_wait(bias + f + 2), load_behind_wait(bias + f + 3));
                     }
                     *reinterpret_cast<float4*>(at) = make_float4(one[0] + b.x, one[1] + b.y, one[2] + b.z, one[3] + b.w);
                 } else {
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
                         if (f + q < features) {
-                            at[q] = one[q] + (bias != nullptr ? __ldg(bias + f + q) : 0.0f);
+                            at[q] = one[q] + (bias != nullptr ? load_behind_wait(bias + f + q) : 0.0f);
                         }
                     }
                 }

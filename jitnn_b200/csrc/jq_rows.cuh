@@ -82,7 +82,7 @@ __device__ __forceinline__ uint32_t lds4(uint32_t at) {
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(at));
     return v;
 }
-// A scale of x, behind the wait for the kernel that writes it: not a read-only load, which might be moved in front of that wait. L2: from L2, past L1.
+// A scale of x or a bias, behind the wait for the kernel that writes it: not a read-only load, which might be moved in front of that wait. L2: from L2, past L1.
 template <bool L2>
 __device__ __forceinline__ float load_scale(const float* p) {
     float v;
@@ -812,9 +812,12 @@ __global__ void __launch_bounds__((Shape<TYPE, NT>::THREADS), 1) rows_kernel(con
             const int64_t f0 = (int64_t)(ft - ft0) * 128, n = mm::pick(p.n, w);
             float* const y = mm::pick(p.y, w);
             const int per = RANGES / p.ksplit;
+            static_assert(THREADS % 128 == 0, "a thread's columns are of the same row");
+            const int row = threadIdx.x & 127;
+            const float bias = w == 0 && p.bias != nullptr && f0 + row < n ? load_scale<AFTER>(p.bias + f0 + row) : 0.0f;
             // columns range, range + ksplit, ... of the tile; a thread adds up one row's eight ranges
             for (int i = threadIdx.x; i < NT / p.ksplit * 128; i += THREADS) {
-                const int col = range + (i >> 7) * p.ksplit, row = i & 127;
+                const int col = range + (i >> 7) * p.ksplit;
                 float e[RANGES];
 #pragma unroll
                 for (int g = 0; g < RANGES; g++) {
@@ -831,7 +834,7 @@ __global__ void __launch_bounds__((Shape<TYPE, NT>::THREADS), 1) rows_kernel(con
                     t += e[g];
                 }
                 if (f0 + row < n && col < p.m) {
-                    y[(int64_t)col * n + f0 + row] = t + (w == 0 && p.bias != nullptr ? __ldg(p.bias + f0 + row) : 0.0f);
+                    y[(int64_t)col * n + f0 + row] = t + bias;
                 }
             }
         }
