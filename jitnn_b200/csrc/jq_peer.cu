@@ -49,7 +49,7 @@ struct PeerTargets {
 
 // slice [m, n_slice] -> columns col0 .. of this rank's y [m, n_total] and, marked, of every other rank's staging area;
 // then the other ranks' columns from this rank's staging area into its y.
-__global__ void __launch_bounds__(256) peer_scatter_kernel(const float* __restrict__ slice, int64_t m, PeerOut po) {
+__global__ void __launch_bounds__(256) peer_scatter_kernel(const float* slice, int64_t m, PeerOut po) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t seq = peer_marks_seq(&po);
     const int64_t count = m * po.n_own;
