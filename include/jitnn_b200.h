@@ -122,7 +122,8 @@ JQ_API int jq_dequantize(const jq_weight* w, float* dst, int dst_mem, void* stre
  * dispatches them (ops/Gguf.java:90): few rows to the fused dequantise-GEMV kernels, more to the tensor cores (from 3 to 9 rows on, by format, the
  * rows kernel; always above 16 the matrix kernel), which take x, and the weights where one does not hold them, as sums of two half-precision numbers (22 significant bits, relative to
  * the largest magnitude of a 256-element block) and add up in FP32 (errors of 1.1e-7 to 2.6e-7 of the result's norm; the decode kernels' are 2.8e-7 to 3.2e-7),
- * unless the bfloat16 prefill path is selected with jq_set_option. `mem` says where x, bias and y live (all three alike); with JQ_MEM_DEVICE they must
+ * unless the bfloat16 prefill path is selected with jq_set_option. y may be x itself where n = k and k is a multiple
+ * of 256; apart from that y must not overlap x or bias, as some kernels read x while they store y. `mem` says where x, bias and y live (all three alike); with JQ_MEM_DEVICE they must
  * be 16-byte aligned and `stream` is the CUDA stream (cudaStream_t, NULL = default stream).
  */
 JQ_API int jq_linear_f32(const jq_weight* w, const float* x, int64_t m, const float* bias, float* y, int mem,

@@ -110,6 +110,8 @@ int launch_gemv(const View& v, const float* x, int rows, const float* bias, floa
     if (v.n == 0) {
         return JQ_OK;
     }
+    // y on x: the image kernel reads all of x before anything is stored, as for x in host memory
+    x_remote = x_remote || ((uintptr_t)x < (uintptr_t)(y + rows * v.n) && (uintptr_t)y < (uintptr_t)(x + rows * v.k));
     if (gemv_umma_takes(v.type, v.k, rows)) {
         // Q4_K, Q5_K: the tcgen05 kernel, one pass over the weights for up to 16 rows
         uint8_t* image = nullptr;

@@ -88,3 +88,20 @@ def test_the_image_kernel_between_few_and_many_rows(t, k, m, n):
     assert torch.equal(y, z) and np.array_equal(Gguf.linear(x.cpu().numpy(), w), y.cpu().numpy())
     ref, size = x.double() @ wd.T, ((x.double() ** 2) @ (wd ** 2).T).sqrt()
     assert float(((y.double() - ref).abs() / size).max()) <= REL
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 8, 16, 20])
+@pytest.mark.parametrize("t", ["Q4_K", "Q5_K", "Q6_K", "Q8_0", "Q4_0", "Q4_1"])
+def test_in_place(t, m):
+    """y on x with n = k: no thread block still reads x when another stores y. Products on a second stream let the call's thread blocks start one after the other."""
+    n = {1: 8192, 2: 4096}.get(m, 2048)  # (8192 values of x, which would become digits inside the GEMV)
+    w = Tensor.quantized(t, synth.random_valid_blocks(t, n, n, seed=m).numpy().reshape(-1), n, n)
+    L, x = jitnn_b200.load(), torch.randn(m, n, generator=torch.Generator().manual_seed(m)).cuda()
+    want, other, side = Gguf.linear(x, w), torch.randn(2048, 2048, device="cuda"), torch.cuda.Stream()
+    zs = [x.clone() for _ in range(50)]
+    torch.cuda.synchronize()
+    for z in zs:
+        with torch.cuda.stream(side):
+            torch.mm(other, other)
+        assert L.jq_linear_f32(w._handle(), z.data_ptr(), m, None, z.data_ptr(), 1, torch.cuda.current_stream().cuda_stream) == 0
+    assert all(torch.equal(z, want) for z in zs)
