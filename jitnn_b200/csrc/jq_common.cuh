@@ -208,6 +208,7 @@ size_t gemv_blk32_i8_scratch_bytes(int type, int64_t k, int rows);
 int scratch_for(cudaStream_t s, size_t bytes, uint8_t** out);
 // A second, third ... scratch buffer of the same (device, stream), for a caller that needs one while a kernel launcher uses slot 0.
 int scratch_for_slot(cudaStream_t s, int slot, size_t bytes, uint8_t** out);
+bool scratch_holds(cudaStream_t s, int slot, size_t bytes);
 
 // The same for words that kernels use as counters and leave at zero: a new allocation starts out zeroed (in stream order).
 int scratch_zeroed_for_slot(cudaStream_t s, int slot, size_t bytes, uint8_t** out);
@@ -263,7 +264,7 @@ int launch_matmul_f32_swiglu(const View& v, const float* gate, const float* up, 
 int launch_matmul_f32_multi(const View* vs, int count, const float* x, int64_t m, float* const* ys, cudaStream_t s);
 // The rows kernel (jq_rows.cu): the same for up to 16 rows of x (up: x is silu(x) * up).
 int launch_rows(const View* vs, int count, const float* x, const float* up, int m, const float* bias, float* const* ys, cudaStream_t s);
-int rows_image(cudaStream_t s, int m, int64_t k, uint8_t** image, float** scales);  // for a kernel that writes x's image itself: then x is null
+int rows_image(cudaStream_t s, int type, int m, int64_t k, uint8_t** image, float** scales);  // for a kernel that writes x's image itself: then x is null
 bool matmul_takes(const View& v, int64_t rows);  // where it is the fastest of the FP32 kernels
 bool prefill_supported(const View& v);
 int launch_prefill_bf16(const View& v, const uint16_t* x_bf16, int64_t m, const float* bias, float* y, cudaStream_t s);

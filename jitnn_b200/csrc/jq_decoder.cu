@@ -1827,7 +1827,7 @@ static int enqueue_forward(jq_decoder* d, int T, int max_keys, const TokenArgs* 
         if (dim % 256 == 0 && dim <= NORM_IMAGE_DIM && linears_take_rows(w, count, T)) {
             uint8_t* image = nullptr;
             float* scales = nullptr;
-            rc = rc == JQ_OK ? rows_image(s, T, dim, &image, &scales) : rc;
+            rc = rc == JQ_OK ? rows_image(s, w[0]->type, T, dim, &image, &scales) : rc;
             if (rc == JQ_OK) {
                 CKL(launch_add_rmsnorm_image(T, s, d->x, delta, norm_w, d->eps, image, scales, dim), "add_rmsnorm_kernel");
                 ROWS(w, count, ys);
@@ -1861,7 +1861,7 @@ static int enqueue_forward(jq_decoder* d, int T, int max_keys, const TokenArgs* 
             uint8_t* image = nullptr;
             float* scales = nullptr;
             if (rc == JQ_OK && dim % 256 == 0 && hd >= 32 && 256 % hd == 0 && linears_take_rows(L + 3, 1, T)) {
-                rc = rows_image(s, T, dim, &image, &scales);
+                rc = rows_image(s, L[3]->type, T, dim, &image, &scales);
             }
             if (rc != JQ_OK) break;
             count_launch(1);

@@ -475,7 +475,7 @@ bool matmul_takes(const View& v, int64_t rows) {
         return rows >= 5;
     }
     if (gemv_blk32_i8_scratch_bytes(v.type, v.k, rows < 2 ? 1 : 2) > 0) {
-        return rows >= (v.k <= 28672 ? 3 : 5);  // (a wider k's image of x may need a larger scratch buffer than calls with one or two rows have left)
+        return rows >= (v.k <= 28672 ? 3 : 5);  // (a wider k's image of x may not fit the scratch buffer that calls with one or two rows have left)
     }
     return rows * v.k >= (v.type == JQ_TYPE_Q8_0 ? 4096 : 2048);
 }

@@ -50,18 +50,23 @@ static int launch_any(int type, Args& a, int ctas, bool after, cudaStream_t s) {
     }
 }
 
-// Scratch for image and scales. Up to four rows the slot is that of the decode kernels' images, so that a program that has made a call with one or two rows may
-// capture one with three or four (matmul_takes sends no wider k here than the slot's least size holds).
-constexpr int SLOT = 8;
-constexpr int slot_of(int m) { return m < 5 ? 0 : SLOT; }
+// Scratch for image and scales: one slot, sized for 16 rows, so that a program that has made a call may capture one with another number of rows. For three and four
+// rows of a 32-element format with k a multiple of 256, up to 28672, the buffer of the decode kernels' images does as well, whose least size holds theirs: a call with one
+// or two rows, which has left that one, is enough in front of the capture too.
+constexpr int SLOT = 8, DECODE_SLOT = 0;
+static_assert((28672 / 256) * (image_bytes(8) + MAX_NT * sizeof(float)) <= (1 << 20), "the least size of a scratch buffer");
 
 }  // namespace rows
 
-// Where the image of m rows of x for the next product on `s` goes, for a kernel that writes it itself.
-int rows_image(cudaStream_t s, int m, int64_t k, uint8_t** image, float** scales) {
+// Where the image of m rows of x for the next product on `s` goes, whose first weight has that type, for a kernel that writes it itself. (Asked again it says the same.)
+int rows_image(cudaStream_t s, int type, int m, int64_t k, uint8_t** image, float** scales) {
     using namespace rows;
-    const size_t units = (size_t)tiled_steps(k);
-    const int rc = scratch_for_slot(s, slot_of(m), units * (image_bytes(m < 5 ? 8 : MAX_NT) + MAX_NT * sizeof(float)), image);
+    const size_t units = (size_t)tiled_steps(k), few = units * (image_bytes(8) + MAX_NT * sizeof(float)), any = units * (image_bytes(MAX_NT) + MAX_NT * sizeof(float));
+    bool decode = (m == 3 || m == 4) && k <= 28672 && gemv_blk32_i8_scratch_bytes(type, k, 1) > 0;
+    if (decode && !scratch_holds(s, DECODE_SLOT, few)) {
+        decode = !scratch_holds(s, SLOT, any) && gemv_blk32_i8_scratch_bytes(type, k, 2) > 0;
+    }
+    const int rc = scratch_for_slot(s, decode ? DECODE_SLOT : SLOT, decode ? few : any, image);
     *scales = reinterpret_cast<float*>(*image + units * image_bytes(nt_of(m)));
     return rc;
 }
@@ -78,7 +83,7 @@ int launch_rows(const View* vs, int count, const float* x, const float* up, int 
     float* scales = nullptr;
     int rc = status_word(&status);
     if (rc == JQ_OK) {
-        rc = rows_image(s, m, k, &image, &scales);
+        rc = rows_image(s, vs[0].type, m, k, &image, &scales);
     }
     if (rc != JQ_OK) {
         return rc;

@@ -94,3 +94,23 @@ def test_three_rows_are_captured_after_a_call_with_one(t):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(y, want)
+
+
+# k that is no multiple of 256, of which the decode kernels take no rows; k of which those of Q8_0 take one row but not two
+@pytest.mark.parametrize("t,k", [("Q8_0", 1056), ("Q4_0", 1056), ("Q8_0", 24576)])
+@pytest.mark.parametrize("first,then", [(8, 4), (4, 8), (16, 3)])
+def test_a_call_with_other_rows_leaves_the_scratch_for_a_capture(t, k, first, then):
+    n = 512
+    _, w, _ = product(t, n, k, 4)
+    stream = torch.cuda.Stream()
+    x = torch.randn(16, k, generator=torch.Generator().manual_seed(1)).cuda()
+    want = Gguf.linear(x[:then], w)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        Gguf.linear(x[:first], w)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        y = Gguf.linear(x[:then], w)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
