@@ -7,7 +7,7 @@
 namespace jq {
 
 // The exponent field of s = 2^floor(log2(largest magnitude of the warp's 256 values)), at least `least` (so that 2^21 / s and the smallest weight of
-// a digit stay normal); bad: a NaN or an Inf is among them. Magnitudes are compared as integers: NaN > Inf > every finite value.
+// a digit stay normal), at most that of the largest finite values: |x| / s < 2, on which the digits depend; bad: a NaN or an Inf is among them. Magnitudes are compared as integers: NaN > Inf > every finite value.
 __device__ __forceinline__ uint32_t image_exponent(const float (&xv)[8], uint32_t least, bool& bad) {
     uint32_t amb = 0u;
 #pragma unroll
@@ -17,7 +17,7 @@ __device__ __forceinline__ uint32_t image_exponent(const float (&xv)[8], uint32_
     amb = __reduce_max_sync(0xffffffffu, amb);
     bad = amb >= 0x7f800000u;
     const uint32_t e = amb & 0x7f800000u;
-    return e < least ? least : (e > 0x7e800000u ? 0x7e800000u : e);
+    return e < least ? least : (e > 0x7f000000u ? 0x7f000000u : e);
 }
 
 // dw[d][h]: digit d of values 4 h .. 4 h + 3, a signed byte each.

@@ -105,3 +105,22 @@ def test_in_place(t, m):
             torch.mm(other, other)
         assert L.jq_linear_f32(w._handle(), z.data_ptr(), m, None, z.data_ptr(), 1, torch.cuda.current_stream().cuda_stream) == 0
     assert all(torch.equal(z, want) for z in zs)
+
+
+@pytest.mark.parametrize("m", [1, 2])
+@pytest.mark.parametrize("t", ["Q4_K", "Q5_K", "Q6_K", "Q8_0", "Q4_0", "Q4_1"])
+def test_x_up_to_the_largest_float(t, m):
+    """Magnitudes from 2^127 to the largest float, with weights small enough for a finite result; made inside the GEMV, and by the image kernel (host arrays)."""
+    n, k = 64, 1024
+    raw = synth.random_valid_blocks(t, n, k, seed=2).numpy().reshape(-1).copy()
+    size, at = {"Q4_K": (144, [0, 2]), "Q5_K": (176, [0, 2]), "Q6_K": (210, [208]), "Q8_0": (34, [0]), "Q4_0": (18, [0]), "Q4_1": (20, [0, 2])}[t]
+    for a in at:
+        raw.reshape(-1, size)[:, a:a + 2] = np.array([2.0 ** -22], np.float16).view(np.uint8)
+    w, wd = Tensor.quantized(t, raw, n, k), torch.from_numpy(oracle.dequantize(t, raw).reshape(n, k)).cuda().double()
+    g = torch.Generator().manual_seed(m)
+    x = (torch.rand(m, k, generator=g) + 1.0) * 2.0 ** 127 * (torch.randint(0, 2, (m, k), generator=g) * 2 - 1)
+    x[0, 5] = torch.finfo(torch.float32).max
+    x = x.clamp(-torch.finfo(torch.float32).max, torch.finfo(torch.float32).max).cuda()
+    ref, of = x.double() @ wd.T, ((x.double() ** 2) @ (wd ** 2).T).sqrt()
+    for y in (Gguf.linear(x, w), torch.from_numpy(Gguf.linear(x.cpu().numpy(), w)).cuda()):
+        assert float(((y.double() - ref).abs() / of).max()) <= REL
