@@ -1550,9 +1550,19 @@ JQ_API int jq_decoder_set_embedding(jq_decoder* d, const float* host_table) {
     return e == cudaSuccess ? JQ_OK : cuda_fail(e, "jq_decoder_set_embedding");
 }
 
+// The thread blocks of norm_image_kernel's cluster: the most, up to 8, that get whole super-blocks each, four elements a thread; 0 where a thread block would get more than
+// 1024 threads (an odd number of super-blocks above 16, and the like).
+static int norm_image_ctas(int dim) {
+    int ctas = 8;
+    while (ctas > 1 && dim % (256 * ctas) != 0) {
+        ctas /= 2;
+    }
+    return dim % 256 == 0 && dim / ctas <= 4096 ? ctas : 0;
+}
+
 // Whether the single-token step can take the fused kernels: Q4_K / Q6_K linears, head_dim 128, sizes in whole super-blocks.
 static bool fused_step_possible(const jq_decoder* d) {
-    if (g_opt_decoder_fused.load() == 0 || d->world != 1 || d->head_dim != 128 || d->dim % 256 != 0 || d->hidden % 256 != 0 || d->dim > 32768) {
+    if (g_opt_decoder_fused.load() == 0 || d->world != 1 || d->head_dim != 128 || norm_image_ctas(d->dim) == 0 || d->hidden % 256 != 0) {
         return false;
     }
     for (const jq_weight* w : d->lin) {
@@ -1659,11 +1669,7 @@ static int enqueue_forward_fused(jq_decoder* d, int max_keys, const TokenArgs* t
     const int64_t tok_stride = d->cur_batch ? (int64_t)seq_elems : 0;
     (void)pos_step;
     (void)tok_stride;  // one token of one sequence here
-    // the norm kernel's cluster: the most CTAs (up to 8) that still get whole super-blocks each
-    int norm_ctas = 8;
-    while (norm_ctas > 1 && dim % (256 * norm_ctas) != 0) {
-        norm_ctas /= 2;
-    }
+    const int norm_ctas = norm_image_ctas(dim);
     const size_t norm_smem = (size_t)(dim / norm_ctas) * sizeof(float);
     const dim3 norm_block((unsigned)(dim / norm_ctas / 4));
     const int splits_now = (max_keys + ATT_CHUNK - 1) / ATT_CHUNK;
@@ -1937,17 +1943,14 @@ static int enqueue_forward_sharded(jq_decoder* d, int T, int max_keys, const Tok
     // step's norm kernel), and wq|wk and w1|w3 are one launch each: 19 launches per layer instead of 26. The norm's
     // sum of squares is then added in another order than the general kernel's, so results agree with the unsharded
     // decoder within rounding instead of bit for bit; option decoder_fused = 0 keeps the general kernels.
-    bool fused_in = T == 1 && g_opt_decoder_fused.load() != 0 && dim % 256 == 0 && dim <= 32768;
+    bool fused_in = T == 1 && g_opt_decoder_fused.load() != 0 && norm_image_ctas(dim) != 0;
     for (size_t i = 0; i < d->lin.size() && fused_in; i++) {
         const int slot = (int)(i % 7);
         if (slot != 3 && slot != 6 && d->lin[i]->type != JQ_TYPE_Q4_K && d->lin[i]->type != JQ_TYPE_Q6_K) {
             fused_in = false;
         }
     }
-    int norm_ctas = 8;
-    while (norm_ctas > 1 && dim % (256 * norm_ctas) != 0) {
-        norm_ctas /= 2;
-    }
+    const int norm_ctas = fused_in ? norm_image_ctas(dim) : 1;
     const size_t norm_smem = (size_t)(dim / norm_ctas) * sizeof(float);
     const dim3 norm_block((unsigned)(dim / norm_ctas / 4));
     // A peer linear whose flag wait has not been enqueued as a kernel: the norm that reads its output waits itself.

@@ -145,3 +145,17 @@ def test_a_q6k_wv_makes_its_own_norm(dim, heads, hidden):
             assert np.abs(a - b).max() <= 1e-5 * np.abs(a).max()  # FP32 throughout, sums in other orders
         dec.close()
     assert launches[1] - launches[0] == 2
+
+
+# an odd number of super-blocks: the last width whose norm one thread block makes, and the first that is too wide for it and goes to the general kernels
+@pytest.mark.parametrize("heads", [30, 42])
+def test_widths_of_an_odd_number_of_super_blocks(heads):
+    cfg = llama_oracle.Config(layers=1, dim=128 * heads, heads=heads, kv_heads=2, hidden=1024, vocab=512, max_seq=8)
+    dec = LlamaDecoder(cfg.layers, cfg.dim, cfg.heads, cfg.kv_heads, cfg.hidden, cfg.vocab, cfg.max_seq, cfg.eps, cfg.rope_base)
+    weights = llama_oracle.random_model(cfg, 3)
+    dec.load(weights)
+    ref = llama_oracle.Decoder(cfg, weights)
+    for pos in range(3):
+        want = ref.forward(7 * pos + 1, pos)
+        assert np.abs(dec.forward([7 * pos + 1], pos)[0][0] - want).max() <= 2e-4 * np.abs(want).max()
+    dec.close()
