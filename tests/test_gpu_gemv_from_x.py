@@ -38,7 +38,7 @@ def test_one_launch_up_to_the_line(t, k, m, n):
 
 @pytest.mark.parametrize("t", ["Q6_K", "Q8_0", "Q4_0", "Q4_1"])
 def test_x_of_every_size_and_of_the_kernel_in_front(t):
-    """Zeros, subnormals, the largest floats, ties of the fixed point, NaN and Inf, in x that the kernel in front of the call writes."""
+    """Zeros, subnormals, large floats, ties of the fixed point, NaN and Inf, in x that the kernel in front of the call writes."""
     n, k = 64, 1024
     raw = synth.random_valid_blocks(t, n, k, seed=2).numpy().reshape(-1)
     w, wd = Tensor.quantized(t, raw, n, k), torch.from_numpy(oracle.dequantize(t, raw).reshape(n, k)).cuda().double()
