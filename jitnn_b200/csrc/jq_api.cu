@@ -187,19 +187,19 @@ static int scratch_impl(cudaStream_t s, int slot, size_t bytes, bool zeroed, uin
     return JQ_OK;
 }
 
-// Whether a request of that size would find its buffer.
-bool scratch_holds(cudaStream_t s, int slot, size_t bytes) {
+// The buffer that a request of that size would find, or null where it would allocate.
+uint8_t* scratch_held(cudaStream_t s, int slot, size_t bytes) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) {
-        return false;
+        return nullptr;
     }
     std::lock_guard<std::mutex> lock(g_scratch_mu);
     for (const Scratch& sc : g_scratch) {
         if (sc.device == dev && sc.stream == s && sc.slot == slot) {
-            return sc.bytes >= bytes;
+            return sc.bytes >= bytes ? sc.buf : nullptr;
         }
     }
-    return false;
+    return nullptr;
 }
 
 // Frees the scratch of a stream that the library made itself and is about to destroy: nothing runs on it, and no graph that used it is left.

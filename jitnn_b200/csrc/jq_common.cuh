@@ -208,7 +208,7 @@ size_t gemv_blk32_i8_scratch_bytes(int type, int64_t k, int rows);
 int scratch_for(cudaStream_t s, size_t bytes, uint8_t** out);
 // A second, third ... scratch buffer of the same (device, stream), for a caller that needs one while a kernel launcher uses slot 0.
 int scratch_for_slot(cudaStream_t s, int slot, size_t bytes, uint8_t** out);
-bool scratch_holds(cudaStream_t s, int slot, size_t bytes);
+uint8_t* scratch_held(cudaStream_t s, int slot, size_t bytes);
 
 // The same for words that kernels use as counters and leave at zero: a new allocation starts out zeroed (in stream order).
 int scratch_zeroed_for_slot(cudaStream_t s, int slot, size_t bytes, uint8_t** out);

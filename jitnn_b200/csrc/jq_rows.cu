@@ -62,11 +62,15 @@ static_assert((28672 / 256) * (image_bytes(8) + MAX_NT * sizeof(float)) <= (1 <<
 int rows_image(cudaStream_t s, int type, int m, int64_t k, uint8_t** image, float** scales) {
     using namespace rows;
     const size_t units = (size_t)tiled_steps(k), few = units * (image_bytes(8) + MAX_NT * sizeof(float)), any = units * (image_bytes(MAX_NT) + MAX_NT * sizeof(float));
-    bool decode = (m == 3 || m == 4) && k <= 28672 && gemv_blk32_i8_scratch_bytes(type, k, 1) > 0;
-    if (decode && !scratch_holds(s, DECODE_SLOT, few)) {
-        decode = !scratch_holds(s, SLOT, any) && gemv_blk32_i8_scratch_bytes(type, k, 2) > 0;
+    const bool decode = (m == 3 || m == 4) && k <= 28672 && gemv_blk32_i8_scratch_bytes(type, k, 1) > 0;
+    int rc = JQ_OK;
+    *image = decode ? scratch_held(s, DECODE_SLOT, few) : nullptr;
+    if (*image == nullptr && decode && gemv_blk32_i8_scratch_bytes(type, k, 2) > 0) {
+        *image = scratch_held(s, SLOT, any);
+        rc = *image == nullptr ? scratch_for_slot(s, DECODE_SLOT, few, image) : JQ_OK;
+    } else if (*image == nullptr) {
+        rc = scratch_for_slot(s, SLOT, any, image);
     }
-    const int rc = scratch_for_slot(s, decode ? DECODE_SLOT : SLOT, decode ? few : any, image);
     *scales = reinterpret_cast<float*>(*image + units * image_bytes(nt_of(m)));
     return rc;
 }
