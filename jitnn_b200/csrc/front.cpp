@@ -1,7 +1,7 @@
 // The Python front of calls on torch CUDA tensors, in native code.
 //
-// A decode linear is done on the GPU in 2 to 5 us, and its launch takes the host 2.5; the checks, the new output tensor and the ctypes call took Python 5 more
-// (256 x 1024, one row of x: 7.4 us a call, of them new_empty 1.8 and ctypes 0.7; now 4.0). Here the whole call is one method of this module.
+// A decode linear is done on the GPU in 2 to 5 us, and its launch takes the host 2.5; the checks, the new output tensor and the ctypes call take Python 5 more
+// (256 x 1024, one row of x: 7.4 us a call, of them new_empty 1.8 and ctypes 0.7; with this module 4.0). Here the whole call is one method of this module.
 //
 // A method takes the plain case only: an ordinary strided, contiguous CUDA tensor (or parameter) with the weight's type, row length and device, while nothing
 // intercepts torch calls (function and dispatch modes, functorch transforms, tracing). For everything else, wrong arguments among it, it returns None

@@ -49,8 +49,8 @@ __device__ __forceinline__ float share_max(const float (&am)[8], int part) {
 
 // Eight threads per block of 32, four values each; the CTA's blocks are put together in shared memory and leave as 16-byte stores (a block
 // is 34 bytes, so nothing wider than two bytes is aligned by itself). Memory bound: 4 + 34/32 bytes per value. Each of the eight threads makes the scale of one
-// of their eight blocks: when each made all eight, a division and a reciprocal for every four values, those bound the kernel (4096 x 4096 20.6 us, now 15.4;
-// 4096 x 11008 45.1, now 35.2).
+// of their eight blocks: where each makes all eight, a division and a reciprocal for every four values, those bound the kernel (4096 x 4096 20.6 us against 15.4;
+// 4096 x 11008 45.1 against 35.2).
 __global__ void __launch_bounds__(THREADS) quantize_q8_0_kernel(const float* x, uint8_t* out, int64_t blocks, bool wide) {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");  // x is written, and out may be read, by the kernel in front

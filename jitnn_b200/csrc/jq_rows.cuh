@@ -10,10 +10,10 @@
 //   stay in place, as 16 q. The pairs are values 0 and 2, 1 and 3 of four; x's image has the same order.
 // * d and dmin go to the sums: the mins, times the sums of x over 32 values, have columns of their own in tensor memory.
 // * Where quant x scale does not fit a half (Q6_K 13 bits, 32-element formats 15 to 18) the operand is the quants alone, and every scale has an accumulator of
-//   its own: its 16 or 32 k times hi and lo of x, which the warps that add up multiply by the scale. Before, such a weight was two halves, hi = scale q rounded
-//   and lo = the rest: two instructions a pair and twice the stores to tensor memory more, for 16 (8) multiply-adds a row and 8 columns. 32000 x 4096, 8 and 16 rows, us:
-//   Q6_K 41.4 -> 32.2 and 42.0 -> 38.2, Q8_0 41.9 -> 26.0 and 42.4 -> 30.3, Q4_0 37.6 -> 23.9 and 38.4 -> 28.9, Q4_1 43.6 -> 27.9 and 44.6 -> 35.0; and the error
-//   against 64 bits, 2.0e-7 of the norm, is 1.1e-7, as a sum of 16 or 32 terms is all that the tensor core cuts off. Q6_K is still bound by its
+//   its own: its 16 or 32 k times hi and lo of x, which the warps that add up multiply by the scale, for 16 (8) multiply-adds a row and 8 columns. (As two halves,
+//   hi = scale q rounded and lo = the rest, a weight takes two instructions a pair and twice the stores to tensor memory more. 32000 x 4096, 8 and 16 rows, so and as quants,
+//   us: Q6_K 41.4, 42.0 and 32.2, 38.2; Q8_0 41.9, 42.4 and 26.0, 30.3; Q4_0 37.6, 38.4 and 23.9, 28.9; Q4_1 43.6, 44.6 and 27.9, 35.0; the error against 64 bits
+//   2.0e-7 of the norm and 1.1e-7, as a sum of 16 or 32 terms is all that the tensor core cuts off.) Q6_K is still bound by its
 //   instructions (1180 per scheduler and unit with 8 rows, 0.55 of the issue slots; four groups of warps that make weights in place of two: 33.2).
 //
 // x is split into halves hi + lo, 22 bits a value, times a power of two per row and 256 values (image_kernel in jq_rows.cu): NT + NT columns of one B
@@ -334,7 +334,7 @@ struct Shape {
     static constexpr int ACC_COLS = ACC * SLOT + MIN_ACC * 16;
     static_assert(ACC_COLS + OPERANDS * A_COLS <= 512 && OPERANDS <= MAX_OPERANDS && ACC <= MAX_ACC, "tensor memory");
     static constexpr int FACTORS = GROUPED ? 4 : 8, FAC_HALF = GROUPED ? 2048 : 1024, FAC = GROUPED ? 2 * FAC_HALF : FAC_HALF;  // units whose factors are kept, bytes
-        static constexpr int GROUPS = 2, FOLD = NT / 2, THREADS = (4 + FOLD + 4 * GROUPS) * 32;  // warps that make weights (groups of four), that add up
+    static constexpr int GROUPS = 2, FOLD = NT / 2, THREADS = (4 + FOLD + 4 * GROUPS) * 32;  // warps that make weights (groups of four), that add up
     static constexpr int C = 8;  // columns (rows of x) of a fold warp
     static constexpr int SCALES = FOLD * 16 * C * 4;  // bytes of the fold warps' scales of x
     static constexpr int TAIL = FACTORS * FAC + SCALES + 1024;  // and barriers

@@ -18,9 +18,9 @@ inline double unit_ns(int type) { return type == JQ_TYPE_Q4_K ? 630.0 : (type ==
 // leave most of the chip idle for a whole contraction, with its contraction split over clusters (57344 x 8192: 448 tiles are three waves and four
 // tiles: 85.5 us in one launch, 71.7 in two). The launch behind starts where SMs become free; GAP_NS is its own start.
 // The cost of a launch is its waves' units and 1700 ns a wave, for a cluster 1600 more, which are rounder than what 16 rows of x take, us: one wave of 8, 16 and 32
-// units 10.7, 15.5 and 25.7 (Q4_K) and 15.5, 24.7 and 43.3 (Q6_K, when its weights were two halves each; 32 units take 38.2 now), that is 5.4 and 6.2 beside the
-// units, the image kernel in front among them; a second wave in the same launch 0.3 beside its units; 16 units a thread block in clusters of 2, 4 and 8 2.6, 2.7
-// and 3.1 (Q4_K) and 1.7, 2.7 and 2.4 (Q6_K) more than alone.
+// units 10.9, 15.7 and 25.6 (Q4_K), 14.4, 22.4 and 38.2 (Q6_K) and 13.2, 19.0 and 30.6 (Q8_0), that is 0.62, 0.99 and 0.73 a unit and 5.7 to 7.3 beside the units,
+// the image kernel in front among them; a second wave of 16 in the same launch 10.5, 16.8 and 12.8; 16 units a thread block in clusters of 2, 4 and 8 2.5, 2.8 and 3.2
+// (Q4_K), 5.3, 3.0 and 2.6 (Q6_K) and 1.7, 2.1 and 2.7 (Q8_0) more than alone. (8 rows of x: Q6_K 0.86 a unit, Q8_0 0.74.)
 constexpr int MAX_PARTS = 3;
 constexpr double GAP_NS = 2500.0;
 struct Parts {
