@@ -210,6 +210,15 @@ int scratch_for(cudaStream_t s, size_t bytes, uint8_t** out);
 int scratch_for_slot(cudaStream_t s, int slot, size_t bytes, uint8_t** out);
 uint8_t* scratch_held(cudaStream_t s, int slot, size_t bytes);
 
+inline bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &status) != cudaSuccess) {
+        cudaGetLastError();  // (the default stream while another is captured: the launch itself says so)
+        return false;
+    }
+    return status != cudaStreamCaptureStatusNone;
+}
+
 // The same for words that kernels use as counters and leave at zero: a new allocation starts out zeroed (in stream order).
 int scratch_zeroed_for_slot(cudaStream_t s, int slot, size_t bytes, uint8_t** out);
 // For a stream of the library's own that is about to be destroyed.

@@ -98,11 +98,7 @@ bool gemv_image_inside(const View& v, int rows, bool x_remote, cudaStream_t s) {
     if (rows == 1 && v.type != JQ_TYPE_Q8_0) {
         return v.type == JQ_TYPE_Q6_K;
     }
-    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &status) != cudaSuccess) {
-        cudaGetLastError();  // (the default stream while another is captured: the launch itself says so)
-    }
-    return status == cudaStreamCaptureStatusNone;
+    return !capturing(s);
 }
 
 // rows in [1, 16].

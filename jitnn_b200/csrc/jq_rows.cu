@@ -50,9 +50,9 @@ static int launch_any(int type, Args& a, int ctas, bool after, cudaStream_t s) {
     }
 }
 
-// Scratch for image and scales: one slot, sized for 16 rows, so that a program that has made a call may capture one with another number of rows. For three and four
-// rows of a 32-element format with k a multiple of 256, up to 28672, the buffer of the decode kernels' images does as well, whose least size holds theirs: a call with one
-// or two rows, which has left that one, is enough in front of the capture too.
+// Scratch for image and scales: one slot, sized for 16 rows, so that a program that has made a call may capture one with another number of rows. Three and four rows of
+// which the decode kernels take two in a pass use the slot of those kernels' images, whose least size holds theirs, so that a call with one or two rows is enough in front of a
+// capture and the other way round. A capture that finds its slot too small takes the other one, for three and four rows of every k that fits there.
 constexpr int SLOT = 8, DECODE_SLOT = 0;
 static_assert((28672 / 256) * (image_bytes(8) + MAX_NT * sizeof(float)) <= (1 << 20), "the least size of a scratch buffer");
 
@@ -62,15 +62,12 @@ static_assert((28672 / 256) * (image_bytes(8) + MAX_NT * sizeof(float)) <= (1 <<
 int rows_image(cudaStream_t s, int type, int m, int64_t k, uint8_t** image, float** scales) {
     using namespace rows;
     const size_t units = (size_t)tiled_steps(k), few = units * (image_bytes(8) + MAX_NT * sizeof(float)), any = units * (image_bytes(MAX_NT) + MAX_NT * sizeof(float));
-    const bool decode = (m == 3 || m == 4) && k <= 28672 && gemv_blk32_i8_scratch_bytes(type, k, 1) > 0;
-    int rc = JQ_OK;
-    *image = decode ? scratch_held(s, DECODE_SLOT, few) : nullptr;
-    if (*image == nullptr && decode && gemv_blk32_i8_scratch_bytes(type, k, 2) > 0) {
-        *image = scratch_held(s, SLOT, any);
-        rc = *image == nullptr ? scratch_for_slot(s, DECODE_SLOT, few, image) : JQ_OK;
-    } else if (*image == nullptr) {
-        rc = scratch_for_slot(s, SLOT, any, image);
+    const bool either = (m == 3 || m == 4) && k <= 28672 && gemv_blk32_i8_scratch_bytes(type, k, 1) > 0, decode = either && gemv_blk32_i8_scratch_bytes(type, k, 2) > 0;
+    *image = either ? scratch_held(s, decode ? DECODE_SLOT : SLOT, decode ? few : any) : nullptr;
+    if (either && *image == nullptr && capturing(s)) {
+        *image = scratch_held(s, decode ? SLOT : DECODE_SLOT, decode ? any : few);
     }
+    const int rc = *image != nullptr ? JQ_OK : scratch_for_slot(s, decode ? DECODE_SLOT : SLOT, decode ? few : any, image);
     *scales = reinterpret_cast<float*>(*image + units * image_bytes(nt_of(m)));
     return rc;
 }
